@@ -528,6 +528,13 @@ int gcow_codec_tables4(const void** etab, const void** dtab, const void** epair,
   return 0;
 }
 
+// The tile kernels (tile_kernels.cu).
+int gcow_tile_usable(const int32_t* params, uint64_t blocks, int dim);
+int gcow_encode_tiles(const float* in, uint64_t nx, uint64_t ny, const int32_t* params, void* out, void* scratch,
+                      uint64_t* block_bits, void* stream);
+int gcow_decode_tiles(const void* in, float* out, uint64_t nx, uint64_t ny, const int32_t* params,
+                      const uint64_t* block_bits, int shift, void* stream);
+
 int gcow_codec_tables(const void** etab, const void** dtab) {
   const void *pair, *loop;
   return gcow_codec_tables4(etab, dtab, &pair, &loop);
@@ -576,7 +583,9 @@ int gcow_decode_1d_fixed(const void* in, float* out, uint64_t n, int maxbits, in
 }
 
 // Launch sequence of the generic encoder, shared by the entry point that takes the caller's scratch and the one
-// that uses the library's built-in array: slots -> per-block lengths -> prefix sum -> bit-offset scatter.
+// that uses the library's built-in array. One tile kernel where it applies (its scratch, 16 bytes per tile and 16
+// more, fits in what gcow_encode_generic_scratch_bytes asks for); blocks padded far beyond their longest code take
+// slots -> per-block lengths -> prefix sum -> bit-offset scatter.
 static int launch_encode_generic(const float* in, uint64_t nx, uint64_t ny, const ZfpParams& p, uint64_t blocks,
                                  uint64_t* out, uint64_t out_bytes, void* scratch, uint64_t* block_bits,
                                  cudaStream_t s) {
@@ -586,7 +595,9 @@ static int launch_encode_generic(const float* in, uint64_t nx, uint64_t ny, cons
   uint32_t* lens = (uint32_t*)(slots + wpb * blocks);
   uint64_t* tile_sums = (uint64_t*)((char*)lens + ((blocks * 4 + 7) & ~7ull));
   const uint64_t tiles = (blocks + kScanTile - 1) / kScanTile;
-  cudaMemsetAsync(out, 0, out_bytes, s);   // the scatter pass ORs into the stream
+  cudaMemsetAsync(out, 0, out_bytes, s);   // the scatter pass ORs into the stream, and callers find zeros after its end
+  const int32_t q[4] = {(int32_t)p.minbits, (int32_t)p.maxbits, (int32_t)p.maxprec, p.minexp};
+  if (gcow_tile_usable(q, blocks, dim)) return gcow_encode_tiles(in, nx, ny, q, out, scratch, block_bits, s);
   const int g = grid_for(blocks);
   if (dim == 1) encode_slots_kernel<1><<<g, kThreads, 0, s>>>(in, nx, ny, p, blocks, slots, lens);
   else encode_slots_kernel<2><<<g, kThreads, 0, s>>>(in, nx, ny, p, blocks, slots, lens);
@@ -632,6 +643,7 @@ int gcow_encode_fixed_direct(const float* in, uint64_t nx, uint64_t ny, const in
   if (!is_fixed_rate(p) || p.maxbits % 64) return -1;
   uint64_t blocks = ny ? num_blocks_2d(nx, ny) : num_blocks_1d(nx);
   if (!blocks) return 0;
+  if (gcow_tile_usable(params, blocks, ny ? 2 : 1)) return gcow_encode_tiles(in, nx, ny, params, out, nullptr, nullptr, stream);
   int g = grid_for(blocks);
   if (ny) encode_fixed_direct_kernel<2><<<g, kThreads, 0, s>>>(in, nx, ny, p, blocks, out);
   else encode_fixed_direct_kernel<1><<<g, kThreads, 0, s>>>(in, nx, ny, p, blocks, out);
@@ -646,6 +658,7 @@ int gcow_decode_generic(const uint64_t* in, float* out, uint64_t nx, uint64_t ny
   uint64_t blocks = ny ? num_blocks_2d(nx, ny) : num_blocks_1d(nx);
   if (!blocks) return 0;
   if (!block_bits && !is_fixed_rate(p)) return -2;
+  if (gcow_tile_usable(params, blocks, ny ? 2 : 1)) return gcow_decode_tiles(in, out, nx, ny, params, block_bits, shift, stream);
   int g = grid_for(blocks);
   if (ny) decode_generic_kernel<2><<<g, kThreads, 0, s>>>(in, out, nx, ny, p, blocks, block_bits, shift);
   else decode_generic_kernel<1><<<g, kThreads, 0, s>>>(in, out, nx, ny, p, blocks, block_bits, shift);

@@ -1,0 +1,521 @@
+// Block coders of the tile kernels (tile_kernels.cu): any mode, 1-D blocks of 4 and
+// 2-D blocks of 4x4, host + device.
+//
+// A block is coded into 32-bit words of its own ("slot", word j at slot[j * stride])
+// and read back from a window of 32-bit words at any bit position. Both use one
+// property of the embedded coder: after a plane, the running count n is one past the
+// highest coefficient that any plane so far has touched. A plane x therefore splits
+// at n into verbatim bits and a rest r = x >> n, and the code of the rest is a
+// function of r alone:
+//   r == 0                one 0 bit (nothing when n == N)
+//   otherwise, h = highest set bit of r:  a 1 bit, then the bits 0..h of r with a 1
+//   inserted after every one-bit, the last inserted one turned into a 0; when n + h
+//   is the last coefficient the final two bits are not sent (implied).
+// (sw/src/encode.c:279-339 is the serial form: group tests and unary runs.)
+#pragma once
+#include "zfp_block.cuh"
+
+namespace gcow {
+
+// The largest block the tile kernels take: the unpadded maximum of a 2-D block (9 header
+// bits + 15 group tests + 16 * 32 plane bits = 536), rounded up to words.
+constexpr uint32_t kTileMaxBlockBits = 544;
+
+// The rest of a plane, eight bits at a time: entry v != 0 holds the code of r = v (closing 0 included, as if more
+// coefficients followed), its length << 20 and the advance of n (h + 1) << 26. Entry 0 is the single 0 bit.
+constexpr int kRestTabSize = 256;
+GCOW_HD uint32_t make_rest_entry(uint32_t v) {
+  if (!v) return 1u << 20;
+  uint32_t code = 1, len = 1, h = 0;
+  for (uint32_t i = 0; i < 8; i++) if ((v >> i) & 1u) h = i;
+  for (uint32_t i = 0; i <= h; i++) {
+    const uint32_t b = (v >> i) & 1u;
+    code |= b << len;
+    len++;
+    if (b) code |= (i < h ? 1u : 0u) << len++;
+  }
+  return code | (len << 20) | ((h + 1) << 26);
+}
+// Its inverse: indexed by the next eight bits of the stream, from a group test on. Entry: the plane's rest (7 bits) |
+// bits used << 8 | advance of n << 16 when the rest ends within the eight bits, else 0.
+constexpr int kUnrestTabSize = 256;
+GCOW_HD uint32_t make_unrest_entry(uint32_t v) {
+  uint32_t r = 0, used = 0, n = 0;
+  for (;;) {
+    if (used >= 8) return 0;
+    const uint32_t test = (v >> used++) & 1u;
+    if (!test) return r | (used << 8) | (n << 16);
+    for (;;) {
+      if (used >= 8) return 0;
+      if ((v >> used++) & 1u) break;
+      n++;
+    }
+    r |= 1u << n++;
+  }
+}
+
+// v with every one-bit doubled ("1" -> "11"), 16 bits in, up to 32 out.
+GCOW_HD uint32_t double_ones16(uint32_t v) {
+  uint32_t r = 0, at = 0;
+  while (v) {
+    const uint32_t z = (uint32_t)ctz32(v);
+    at += z;
+    r |= 3u << at;
+    at += 2;
+    v >>= z;
+    v >>= 1;
+  }
+  return r;
+}
+
+GCOW_HD uint32_t popc32(uint32_t x) {
+#if defined(__CUDA_ARCH__)
+  return (uint32_t)__popc(x);
+#else
+  return (uint32_t)__builtin_popcount(x);
+#endif
+}
+GCOW_HD uint32_t funnel_l0(uint32_t v, uint32_t s) {   // the bits of v << s above bit 31, 0 <= s < 32
+#if defined(__CUDA_ARCH__)
+  return __funnelshift_l(v, 0u, s);
+#else
+  return s ? v >> (32 - s) : 0u;
+#endif
+}
+GCOW_HD uint32_t window32(uint32_t lo, uint32_t hi, uint32_t s) {   // low word of (hi:lo) >> s, 0 <= s < 32
+#if defined(__CUDA_ARCH__)
+  return __funnelshift_r(lo, hi, s);
+#else
+  return s ? (lo >> s) | (hi << (32 - s)) : lo;
+#endif
+}
+
+// Appends codes of up to 32 bits to a slot.
+struct SlotWriter {
+  uint32_t* at;        // next word
+  uint32_t stride;
+  uint32_t acc, fill;  // fill < 32 bits pending
+  uint32_t full;       // bits in completed words
+  GCOW_HD SlotWriter(uint32_t* slot, uint32_t s) : at(slot), stride(s), acc(0), fill(0), full(0) {}
+  // the header and z zero bits behind it, 0 <= z <= 32, as the first thing in the slot
+  GCOW_HD void begin(uint32_t head, uint32_t z) {
+    acc = head;
+    fill = kHeaderBits + z;
+    if (fill >= 32) flush(0);
+  }
+  GCOW_HD void flush(uint32_t next) {
+    *at = acc;
+    at += stride;
+    acc = next;
+    fill -= 32;
+    full += 32;
+  }
+  GCOW_HD void put(uint32_t code, uint32_t len) {       // len <= 32, code < 2^len
+    acc |= code << fill;
+    const uint32_t hi = funnel_l0(code, fill);
+    fill += len;
+    if (fill >= 32) flush(hi);
+  }
+  GCOW_HD uint32_t bits() const { return full + fill; }
+};
+
+// Ends a slot at `limit` bits (what lies past the budget is dropped) and returns its length.
+GCOW_HD uint32_t finish_slot(const SlotWriter& s, uint32_t* slot, uint32_t stride, uint32_t limit) {
+  uint32_t total = s.bits();
+  *s.at = s.acc;
+  if (total > limit) {
+    total = limit;
+    if (total & 31u) slot[(total >> 5) * stride] &= low_mask32(total & 31u);
+  }
+  return total;
+}
+
+// Cast of a block to integers relative to 2^(emax - 30). The clamping conversion (values out
+// of range, NaN) is only needed with a non-finite member or a vanishing maximum.
+template <int N>
+GCOW_HD void cast_block(int32_t* q, const float* f, int emax) {
+  const float scale = pow2f(30 - emax);
+  float s = 0;
+#pragma unroll
+  for (int i = 0; i < N; i++) s += scale * f[i];
+  if (emax >= -97 && fabsf(s) < (float)N * 2.0e9f) {       // false for NaN and infinity
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+#if defined(__CUDA_ARCH__)
+      q[i] = __float2int_rz(scale * f[i]);
+#else
+      q[i] = (int32_t)(scale * f[i]);
+#endif
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; i++) q[i] = trunc_to_i32(scale * f[i]);
+  }
+}
+template <int N>
+GCOW_HD int block_emax_fmax(const float* f) {              // block_emax with the hardware maximum (NaN members are skipped)
+  float m = 0;
+#pragma unroll
+  for (int i = 0; i < N; i++) m = fmaxf(m, fabsf(f[i]));
+  return scalar_exponent(m);
+}
+
+// ------------------------------------------------------------------- 1-D encoder
+// The planes below the leading all-zero ones are coded two per lookup for the first eight, a
+// last odd plane with the same table (the second plane masked away: an absent plane codes like a
+// zero plane minus that plane's own zero bits), and verbatim nibbles follow once n >= 3.
+GCOW_HD uint32_t encode_slot_1d(const float* f, const ZfpParams& p, const uint32_t* epair, const uint16_t* etab,
+                                uint32_t* slot, uint32_t stride) {
+  const int emax = block_emax_fmax<4>(f);
+  const uint32_t prec = block_precision(emax, p.maxprec, p.minexp, 1);
+  const uint32_t biased = prec ? (uint32_t)(emax + kEBias) : 0;
+  if (!biased) { *slot = 0; return 1; }
+  int32_t q[4];
+  uint32_t u[4];
+  cast_block<4>(q, f, emax);
+  fwd_lift(q[0], q[1], q[2], q[3]);
+#pragma unroll
+  for (int i = 0; i < 4; i++) u[i] = int2nb(q[i]);
+  const uint32_t planes = prec < 32u ? prec : 32u;
+  const uint32_t mm = u[0] | u[1] | u[2] | u[3];
+  uint32_t z = mm ? clz32(mm) : 32u;
+  if (z > planes) z = planes;
+  SlotWriter s(slot, stride);
+  s.begin(2u * biased + 1u, z);
+  uint32_t left = planes - z;
+  if (left && s.bits() < p.maxbits) {                      // z < 32
+    const uint32_t R = byte_perm(byte_perm(u[0] << z, u[1] << z, 0x0073), byte_perm(u[2] << z, u[3] << z, 0x0073), 0x5410);
+    // byte i = the next eight planes of coefficient i
+    uint32_t n = 0;
+    if (left >= 8) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const uint32_t e = epair[n * 256u + ((((R >> (6 - 2 * j)) & 0x03030303u) * 0x40100401u) >> 24)];
+        s.put(e & 0xffffu, (e >> 16) & 0xffu);
+        n += e >> 24;
+      }
+      left -= 8;
+      uint32_t k = 24 - z;                                 // planes k-1 .. k-left remain
+      while (left && s.bits() < p.maxbits) {
+        uint32_t T = plane_group8(u, k);
+        uint32_t cnt = left < 8 ? left : 8;
+        k -= cnt;
+        left -= cnt;
+        while (n < 3 && cnt) {                             // very smooth block: one plane per lookup
+          const uint32_t e = etab[n * 16 + (T & 15u)];
+          s.put(e & 0x7fu, (e >> 7) & 7u);
+          n = e >> 10;
+          T >>= 4;
+          cnt--;
+        }
+        s.put(T & low_mask32(4 * cnt), 4 * cnt);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        if (left > 2u * j) {
+          uint32_t g = (((R >> (6 - 2 * j)) & 0x03030303u) * 0x40100401u) >> 24;
+          const bool single = left == 2u * j + 1;
+          if (single) g &= 0xaau;
+          const uint32_t e = epair[n * 256u + g];
+          n += e >> 24;
+          uint32_t len = (e >> 16) & 0xffu;
+          if (single) len -= n < 4 ? n + 1 : 4u;
+          s.put(e & 0xffffu, len);
+        }
+      }
+    }
+  }
+  return finish_slot(s, slot, stride, p.maxbits);
+}
+
+// -------------------------------------------------------- 16 x 16 bit transposition
+// In: w[j] = row j in the low half, row j + 8 in the high half (j = 0..7). Out: w[j] = column j
+// in the low half, column j + 8 in the high half. The same function inverts itself.
+GCOW_HD uint32_t select_bits(uint32_t a, uint32_t b, uint32_t m) { return (a & m) | (b & ~m); }
+GCOW_HD void swap_quads(uint32_t* w, int a, int b, int s, uint32_t m) {
+  const uint32_t x = w[a], y = w[b];
+  w[a] = select_bits(x, y << s, m);
+  w[b] = select_bits(x >> s, y, m);
+}
+GCOW_HD void transpose16(uint32_t* w) {
+#pragma unroll
+  for (int j = 0; j < 8; j++) w[j] = byte_perm(w[j], 0, 0x3120);   // bytes: row j low, row j+8 low, row j high, row j+8 high
+#pragma unroll
+  for (int j = 0; j < 4; j++) swap_quads(w, j, j + 4, 4, 0x0f0f0f0fu);
+#pragma unroll
+  for (int j = 0; j < 8; j++) if (!(j & 2)) swap_quads(w, j, j + 2, 2, 0x33333333u);
+#pragma unroll
+  for (int j = 0; j < 8; j += 2) swap_quads(w, j, j + 1, 1, 0x55555555u);
+}
+// After the transposition the low half of w[j] is column j of rows 0..15 read as bytes: rows 0..7 in
+// byte 0, rows 8..15 in byte 1 - i.e. column j as a 16-bit word - and the high half is column j + 8.
+GCOW_HD void transpose16_inv(uint32_t* w) {
+#pragma unroll
+  for (int j = 0; j < 8; j += 2) swap_quads(w, j, j + 1, 1, 0x55555555u);
+#pragma unroll
+  for (int j = 0; j < 8; j++) if (!(j & 2)) swap_quads(w, j, j + 2, 2, 0x33333333u);
+#pragma unroll
+  for (int j = 0; j < 4; j++) swap_quads(w, j, j + 4, 4, 0x0f0f0f0fu);
+#pragma unroll
+  for (int j = 0; j < 8; j++) w[j] = byte_perm(w[j], 0, 0x3120);
+}
+
+// ------------------------------------------------------------------- 2-D encoder
+// Sixteen planes at a time: one bit-matrix transposition, then one code per plane. `rest` is the table of
+// make_rest_entry; only a rest of more than eight bits (the first planes of a noisy block) is worked out bit by bit.
+// kBudget: the block may have to be cut at maxbits.
+template <bool kBudget>
+GCOW_HD uint32_t encode_slot_2d(const float* f, const ZfpParams& p, const uint32_t* rest, uint32_t* slot, uint32_t stride) {
+  const int emax = block_emax_fmax<16>(f);
+  const uint32_t prec = block_precision(emax, p.maxprec, p.minexp, 2);
+  const uint32_t biased = prec ? (uint32_t)(emax + kEBias) : 0;
+  if (!biased) { *slot = 0; return 1; }
+  int32_t q[16];
+  uint32_t u[16];
+  cast_block<16>(q, f, emax);
+  Xform<2>::fwd(q);
+  fwd_reorder<2>(u, q);
+  uint32_t mm = 0;
+#pragma unroll
+  for (int i = 0; i < 16; i++) mm |= u[i];
+  const uint32_t planes = prec < 32u ? prec : 32u;
+  uint32_t z = mm ? clz32(mm) : 32u;
+  if (z > planes) z = planes;
+  SlotWriter s(slot, stride);
+  s.begin(2u * biased + 1u, z);
+  int left = (int)(planes - z);
+  uint32_t n = 0, zl = 1;                                   // zl: length of a plane without news, n + (n < 16)
+#pragma unroll 1
+  for (uint32_t sh = z; left > 0 && (!kBudget || s.bits() < p.maxbits); sh += 16, left -= 16) {
+    uint32_t w[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) w[j] = byte_perm(shl_sat(u[j], sh), shl_sat(u[j + 8], sh), 0x7632);   // the top halves
+    transpose16(w);
+#pragma unroll
+    for (int t = 0; t < 16; t++) {
+      if (t >= left) break;
+      const uint32_t x = t < 8 ? w[7 - t] >> 16 : w[15 - t] & 0xffffu;
+      const uint32_t r = x >> n;
+      uint32_t code = x, len = zl;
+      if (r) {
+        uint32_t c, adv;
+        if (r < 256u) {
+          const uint32_t e = rest[r];
+          c = e & 0xfffffu;
+          len = (e >> 20) & 0x3fu;
+          adv = e >> 26;
+        } else {
+          const uint32_t h = 31u - clz32(r), ones = popc32(r);
+          c = 1u | ((double_ones16(r) ^ (1u << (h + ones))) << 1);
+          len = h + ones + 2;
+          adv = h + 1;
+        }
+        if (n + adv == 16u) {                               // the last coefficient: its one-bit is implied, no closing test
+          len -= 2;
+          c &= low_mask32(len);
+        }
+        code = (x & ((1u << n) - 1u)) | (c << n);
+        len += n;
+        n += adv;
+        zl = n + (n < 16 ? 1u : 0u);
+      }
+      s.put(code, len);
+      if (kBudget && s.bits() >= p.maxbits) break;
+    }
+  }
+  return finish_slot(s, slot, stride, kBudget ? p.maxbits : 0xffffffffu);
+}
+
+// ---------------------------------------------------------------------- decoders
+// Window of 32-bit words read at any bit position; the caller guarantees two readable words after
+// the last one that holds bits of the block.
+struct WindowReader {
+  const uint32_t* w;   // the word after `hi`
+  uint32_t lo, hi, o;  // o < 32: position in lo
+  GCOW_HD WindowReader(const uint32_t* words, uint32_t pos) : w(words + (pos >> 5) + 2), o(pos & 31u) { lo = w[-2]; hi = w[-1]; }
+  GCOW_HD uint32_t peek() const { return window32(lo, hi, o); }
+  GCOW_HD void skip(uint32_t n) {                          // n <= 32
+    o += n;
+    if (o >= 32) {
+      lo = hi;
+      hi = *w++;
+      o -= 32;
+    }
+  }
+  GCOW_HD uint64_t get(uint32_t n) {                       // n <= 32
+    const uint32_t r = n ? peek() & low_mask32(n) : 0u;
+    skip(n);
+    return r;
+  }
+};
+
+// One block of 4 from a window. `rows`: rows n = 0..2 of the decoder loop table for a remaining budget of seven
+// bits or more, 128 entries each (plane | used << 8 | (n' * 4096) << 16).
+GCOW_HD void decode_window_1d(float* f, const ZfpParams& p, const uint32_t* rows, const uint32_t* words, uint32_t pos, int shift) {
+  WindowReader src(words, pos);
+  const uint32_t head = src.peek();
+  if (!(head & 1u)) {
+    f[0] = f[1] = f[2] = f[3] = 0;
+    return;
+  }
+  const int emax = (int)((head >> 1) & 0xffu) - kEBias;
+  const uint32_t prec = block_precision(emax, p.maxprec, p.minexp, 1);
+  uint32_t left = prec < 32u ? prec : 32u;                 // planes to come
+  const uint32_t kmin = 32 - left;
+  uint32_t bits = p.maxbits - kHeaderBits;                 // budget left
+  src.skip(kHeaderBits);
+  uint32_t n = 0;
+  uint32_t u[4] = {0, 0, 0, 0};
+  {                                                        // leading all-zero planes
+    const uint32_t S = src.peek();
+    uint32_t z = S ? (uint32_t)ctz32(S) : 32u;
+    if (z > left) z = left;
+    if (z > bits) z = bits;
+    src.skip(z);
+    bits -= z;
+    left -= z;
+  }
+  while (left && bits) {
+    const uint32_t k = kmin + left, cnt = left < 8 ? left : 8;
+    uint32_t T = 0, j = 0;
+    while (n < 3 && j < 4 * cnt && bits >= 7) {
+      const uint32_t e = rows[n * 128u + (src.peek() & 127u)];
+      const uint32_t used = (e >> 8) & 0xffu;
+      T |= (e & 15u) << j;
+      src.skip(used);
+      bits -= used;
+      n = e >> 28;
+      j += 4;
+    }
+    if (n >= 3 && j < 4 * cnt) {                           // verbatim nibbles
+      // A nibble cut by the budget after its first three bits: with n == 3 the missing bit is a group test that
+      // reads as 0, with n == 4 a verbatim bit that reads as 0 - the same nibble.
+      const uint32_t want = 4 * cnt - j, take = want < bits ? want : bits;
+      T |= (src.peek() & low_mask32(take)) << j;
+      src.skip(take);
+      bits -= take;
+      j = 4 * cnt;
+    }
+    if (T) deposit_group8(u, T, k);
+    if (j < 4 * cnt) {                                     // fewer than seven bits left and n < 3: the serial routine
+      decode_planes_from<4>(u, bits, kmin, k - j / 4, n, src);
+      break;
+    }
+    left -= cnt;
+  }
+  int32_t q[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) q[i] = nb2int(u[i]);
+  inv_lift(q[0], q[1], q[2], q[3]);
+  inv_cast<4>(f, q, emax, shift);
+}
+
+// One block of 4x4 from a window of 32-bit words starting at bit `pos`. Planes are collected as 16-bit words and
+// turned back into coefficients by the bit-matrix transposition. `unrest`: the table of make_unrest_entry.
+template <bool kBudget>
+GCOW_HD void decode_window_2d(float* f, const ZfpParams& p, const uint32_t* unrest, const uint32_t* words, uint32_t pos, int shift) {
+  WindowReader src(words, pos);
+  const uint32_t head = src.peek();
+  if (!(head & 1u)) {
+#pragma unroll
+    for (int j = 0; j < 16; j++) f[j] = 0;
+    return;
+  }
+  const int emax = (int)((head >> 1) & 0xffu) - kEBias;
+  const uint32_t prec = block_precision(emax, p.maxprec, p.minexp, 2);
+  const uint32_t planes = prec < 32u ? prec : 32u;
+  uint32_t bits = p.maxbits - kHeaderBits;                 // budget left
+  src.skip(kHeaderBits);
+  const uint32_t S = src.peek();
+  uint32_t z = S ? (uint32_t)ctz32(S) : 32u;
+  if (z > planes) z = planes;
+  if (kBudget && z > bits) z = bits;
+  src.skip(z);
+  if (kBudget) bits -= z;
+  int left = (int)(planes - z);
+  uint32_t u[16];
+#pragma unroll
+  for (int j = 0; j < 16; j++) u[j] = 0;
+  uint32_t n = 0, nmask = 0;
+#pragma unroll 1
+  for (uint32_t sh = z; left > 0 && (!kBudget || bits); sh += 16, left -= 16) {
+    uint32_t w[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) w[j] = 0;
+#pragma unroll
+    for (int t = 0; t < 16; t++) {
+      if (t >= left || (kBudget && !bits)) break;
+      uint32_t b = src.peek(), x, used;
+      if (!kBudget || bits >= 32) {
+        x = b & nmask;
+        used = n;
+        uint32_t e = b >> n;
+        if (n < 16) {
+          const uint32_t entry = unrest[e & 0xffu];
+          const uint32_t adv = entry >> 16;
+          if (entry && n + adv < 16) {
+            x |= (entry & 0x7fu) << n;
+            used += (entry >> 8) & 0xffu;
+            n += adv;
+          } else {                                         // a long rest, or one that reaches the last coefficient
+            used++;
+            while (e & 1u) {                               // a positive group test: zeros up to the next news, then the next test
+              e >>= 1;
+              const uint32_t c = e ? (uint32_t)ctz32(e) : 32u;
+              if (n + c >= 15u) {                          // the last coefficient's one-bit is implied
+                used += 15u - n;
+                x |= 0x8000u;
+                n = 16;
+                break;
+              }
+              x |= 1u << (n + c);
+              n += c + 1;
+              e = shr_sat(e, c + 1);
+              used += c + 2;
+            }
+          }
+          nmask = (1u << n) - 1u;
+        }
+        if (kBudget) bits -= used;
+      } else {                                             // the budget may end inside this plane: bit by bit
+        const uint32_t start = bits;
+        const uint32_t m = n < bits ? n : bits;
+        x = b & low_mask32(m);
+        b = shr_sat(b, m);
+        bits -= m;
+        while (bits && n < 16) {
+          bits--;
+          const uint32_t test = b & 1u;
+          b >>= 1;
+          if (!test) break;
+          while (bits && n < 15) {
+            bits--;
+            const uint32_t one = b & 1u;
+            b >>= 1;
+            if (one) break;
+            n++;
+          }
+          x += 1u << n;
+          n++;
+        }
+        nmask = (1u << n) - 1u;
+        used = start - bits;
+      }
+      src.skip(used);
+      if (t < 8) w[7 - t] |= x << 16; else w[15 - t] |= x;
+    }
+    transpose16_inv(w);
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      u[j] |= shr_sat(w[j] << 16, sh);
+      u[j + 8] |= shr_sat(w[j] & 0xffff0000u, sh);
+    }
+  }
+  int32_t q[16];
+  inv_reorder<2>(q, u);
+  Xform<2>::inv(q);
+  inv_cast<16>(f, q, emax, shift);
+}
+
+}  // namespace gcow

@@ -173,3 +173,25 @@ def test_gather_and_whole_block_stage_kernels():
     w = list(np.frombuffer(out.cpu().numpy().tobytes(), dtype=np.uint64)[:4])
     assert w == [7846959668108800257, 9092781915241025288, 1168152206201298680, 33031166]
     assert 192 < int(bits[0]) <= 256
+
+
+# Sizes around what one lane (4 or 1 blocks), one string (128 or 32 blocks) and one tile (1024 or 256 blocks) hold, and
+# several tiles; every mode the tile kernels take, with budgets that cut a code and that end on word boundaries or not.
+@pytest.mark.parametrize("dim,sizes", [(1, [1, 4, 127, 509, 512, 516, 4093, 4096, 4100, 70001]),
+                                       (2, [(1, 1), (4, 128), (7, 129), (40, 512), (129, 1023), (64, 2052), (33, 78)])])
+@pytest.mark.parametrize("how", [dict(tolerance=1e-6), dict(tolerance=1e-3), dict(tolerance=1e9), dict(precision=3), dict(precision=32),
+                                 dict(rate=2), dict(rate=3), dict(rate=12), dict(rate=20), dict(rate=33)],
+                         ids=lambda h: "%s-%g" % next(iter(h.items())))
+def test_tile_kernels_at_edges(dim, sizes, how):
+    rng = np.random.default_rng(7)
+    for sz in sizes:
+        n = sz if dim == 1 else sz[0] * sz[1]
+        noise = rng.standard_normal(n).astype(np.float32)
+        sparse = np.where(rng.random(n) < 0.7, np.float32(0), noise)
+        for x in (noise * 1e-3, np.cumsum(noise).astype(np.float32) * 1e-2, sparse, np.zeros(n, np.float32)):
+            t = torch.from_numpy(x if dim == 1 else x.reshape(sz))
+            cpu, gpu = (g.compress(v, dim=dim, return_index=True, **how) for v in (t, t.cuda()))
+            assert torch.equal(gpu.stream.cpu(), cpu.stream) and torch.equal(gpu.index.cpu(), cpu.index), sz
+            for shift in (0, 2):
+                a, b = g.decompress(cpu, shift=shift), g.decompress(gpu, shift=shift).cpu()
+                assert torch.equal(a.view(torch.int32), b.view(torch.int32)), sz
