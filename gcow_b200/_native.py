@@ -1,4 +1,4 @@
-"""ctypes access to the two native libraries (see build.py).
+"""Access to the native libraries (see build.py).
 
 ``cpu()`` is always available (built on demand with g++). ``cuda()`` returns the
 sm_100a kernel library; on a machine with a GPU a missing library is an error,
@@ -15,6 +15,7 @@ from . import build as _build
 _lock = threading.Lock()
 _cpu = None
 _cuda = None
+_ext = None
 
 u64, u32, i32, f64 = C.c_uint64, C.c_uint32, C.c_int, C.c_double
 ptr = C.c_void_p
@@ -84,3 +85,21 @@ def cuda() -> C.CDLL:
             _cuda_protos.declare(lib, _proto)
             _cuda = lib
     return _cuda
+
+
+def ext():
+    """The native host path (csrc/torch/gcow_ext.cpp): an extension module whose functions take tensors and launch."""
+    global _ext
+    if _ext is None:
+        cuda()                       # its kernels' library
+        import importlib.machinery
+        import importlib.util
+        path = str(_build.build_ext())
+        with _lock:
+            if _ext is None:
+                loader = importlib.machinery.ExtensionFileLoader("gcow_ext", path)
+                spec = importlib.util.spec_from_file_location("gcow_ext", path, loader=loader)
+                mod = importlib.util.module_from_spec(spec)
+                loader.exec_module(mod)
+                _ext = mod
+    return _ext

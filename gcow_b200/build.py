@@ -1,12 +1,14 @@
 """In-tree native build: plain g++/nvcc commands, no JIT cache.
 
-Two shared libraries are produced next to this file, under ``_lib/``:
+Three shared libraries are produced next to this file, under ``_lib/``:
 
 * ``libgcow_cpu.so``  – CPU oracle, host model of the flag protocol (g++ only).
 * ``libgcow_cuda.so`` – every sm_100a kernel plus its C launchers (nvcc).
+* ``gcow_ext.so``      – the host path of the CUDA calls as a CPython extension on
+  top of libtorch (g++); it calls the kernels through libgcow_cuda.so.
 
-Both export a C ABI and are loaded with ctypes, so building needs neither the
-PyTorch headers nor a GPU (nvcc cross-compiles). A content hash of the sources
+The first two export a C ABI and are loaded with ctypes; nothing needs a GPU to
+build (nvcc cross-compiles). A content hash of the sources
 is stored beside each library; an up-to-date library is never rebuilt, which is
 what lets a prebuilt tree run on a machine without recompiling.
 
@@ -42,7 +44,9 @@ CXX_FLAGS = ["-std=c++17", "-O2", "-fPIC", "-Wall", "-Wextra", "-pthread"]
 
 def _sources(kind: str) -> list[Path]:
     if kind == "cpu":
-        return sorted(p for p in CSRC.rglob("*.cpp") if "tests" not in p.parts)
+        return sorted(p for p in CSRC.rglob("*.cpp") if "tests" not in p.parts and "torch" not in p.parts)
+    if kind == "ext":
+        return sorted((CSRC / "torch").glob("*.cpp"))
     return sorted(CSRC.rglob("*.cu"))
 
 
@@ -172,6 +176,33 @@ def _build_cuda_locked(force, jobs, name, srcs, digest, nvcc) -> Path:
     return LIB / f"{name}.so"
 
 
+def build_ext(force: bool = False) -> Path:
+    """Build gcow_ext.so against the installed libtorch and CPython headers. It is linked to libgcow_cuda.so in its own
+    directory; libtorch's libraries are the ones that ``import torch`` has loaded."""
+    import sysconfig
+    import torch
+    LIB.mkdir(exist_ok=True)
+    name = "gcow_ext"
+    srcs = _sources("ext")
+    flags = ["-std=c++17", "-O2", "-fPIC", "-fvisibility=hidden", f"-DGCOW_TORCH_{torch.__version__.split('+')[0].replace('.', '_')}",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    digest = _digest(srcs, flags)
+    if not force and _up_to_date(name, digest):
+        return LIB / f"{name}.so"
+    with _build_lock():
+        if not force and _up_to_date(name, digest):
+            return LIB / f"{name}.so"
+        th = Path(torch.__file__).resolve().parent / "include"
+        cuda = Path(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc").resolve().parent.parent / "include"
+        inc = [f"-I{d}" for d in (th, th / "torch/csrc/api/include", sysconfig.get_path("include"), cuda)]
+        tmp = LIB / f"{name}.so.tmp{os.getpid()}"
+        _run(["g++", *flags, *inc, "-shared", *map(str, srcs), "-o", str(tmp), f"-L{LIB}", "-l:libgcow_cuda.so", "-Wl,-rpath,$ORIGIN",
+              f"-L{th.parent / 'lib'}", "-Wl,--no-as-needed", "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10_cuda", "-lc10"])
+        os.replace(tmp, LIB / f"{name}.so")
+        _replace_text(_stamp_path(name), json.dumps({"digest": digest}))
+    return LIB / f"{name}.so"
+
+
 def build_sanitizer_test(kind: str) -> Path:
     """Executable of csrc/tests/sanitize_main.cpp + the CPU sources under a sanitizer:
     kind = 'address' (with undefined-behaviour checks) or 'thread'."""
@@ -194,6 +225,7 @@ def build_sanitizer_test(kind: str) -> Path:
 def build_all(force: bool = False) -> None:
     build_cpu(force)
     build_cuda(force)
+    build_ext(force)
 
 
 if __name__ == "__main__":

@@ -15,8 +15,10 @@ the four expert parameters set by hand or by its accuracy setter
 from __future__ import annotations
 
 import ctypes as C
+import math
 import os
 from dataclasses import dataclass
+from functools import lru_cache
 from typing import Optional
 
 import torch
@@ -24,7 +26,6 @@ import torch
 from . import _native
 
 _NTHREADS = max(1, min(16, os.cpu_count() or 1))
-_FAST_BITS = (16, 32, 64, 128)
 
 
 @dataclass(frozen=True)
@@ -111,17 +112,23 @@ def compressed_nbytes(shape: tuple, params: ZfpParams) -> int:
     return ((bits + 63) // 64) * 8
 
 
+# The parameters of a rate, tolerance or precision are a fixed function of that number: a training loop asks for the same
+# ones on every call.
+_rate_params = lru_cache(maxsize=256)(ZfpParams.from_rate)
+_accuracy_params = lru_cache(maxsize=256)(ZfpParams.from_accuracy)
+_precision_params = lru_cache(maxsize=256)(ZfpParams.from_precision)
+
+
 def _resolve_params(rate, tolerance, precision, params, dim) -> ZfpParams:
-    given = [v is not None for v in (rate, tolerance, precision, params)]
-    if sum(given) != 1:
+    if (rate is not None) + (tolerance is not None) + (precision is not None) + (params is not None) != 1:
         raise ValueError("give exactly one of rate=, tolerance=, precision=, params=")
     if params is not None:
         return params
     if rate is not None:
-        return ZfpParams.from_rate(rate, dim)
+        return _rate_params(rate, dim)
     if tolerance is not None:
-        return ZfpParams.from_accuracy(tolerance)
-    return ZfpParams.from_precision(precision)
+        return _accuracy_params(tolerance)
+    return _precision_params(precision)
 
 
 def _check(err: int, what: str) -> None:
@@ -157,11 +164,15 @@ def compress(x: torch.Tensor, *, rate: float | None = None, tolerance: float | N
         raise ValueError("dim must be 1 or 2")
     p = _resolve_params(rate, tolerance, precision, params, dim)
     x = x.contiguous()
-    nx, ny = _nxny(shape)
-    blocks = _blocks(shape)
-    cap = max_compressed_nbytes(shape, p)
 
+    if x.is_cuda:
+        r = (_native._ext or _native.ext()).compress(x, p.minbits, p.maxbits, p.maxprec, p.minexp, dim, return_index)
+        if r is not None:
+            return Compressed(r[0], p, shape, r[1])
+    nx, ny = _nxny(shape)
     if not x.is_cuda:
+        blocks = _blocks(shape)
+        cap = max_compressed_nbytes(shape, p)
         out = torch.zeros(cap // 8, dtype=torch.int64)
         idx = torch.zeros(blocks + 1, dtype=torch.int64) if (return_index or not p.fixed_rate) else None
         nbytes = _native.cpu().gcow_oracle_compress(
@@ -170,37 +181,15 @@ def compress(x: torch.Tensor, *, rate: float | None = None, tolerance: float | N
         stream = out.view(torch.uint8)[:nbytes]
         return Compressed(stream, p, shape, idx if (return_index or not p.fixed_rate) else None)
 
+    # empty input, or blocks padded far beyond their longest code
     lib = _native.cuda()
+    blocks = _blocks(shape)
+    cap = max_compressed_nbytes(shape, p)
     with torch.cuda.device(x.device):
-        if dim == 1 and p.fixed_rate and p.maxbits in _FAST_BITS:
-            nbytes = compressed_nbytes(shape, p)
-            out = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
-            tail = blocks * p.maxbits // 8
-            if tail < nbytes:
-                out[tail:].zero_()
-            _check(lib.gcow_encode_1d_fixed(x.data_ptr(), nx, p.maxbits, out.data_ptr(), _stream_ptr()),
-                   "gcow_encode_1d_fixed")
-            return Compressed(out, p, shape, None)
-        if blocks and lib.gcow_tile_usable(p.as_c(), blocks, dim):
-            if p.fixed_rate:
-                out = torch.empty(compressed_nbytes(shape, p), dtype=torch.uint8, device=x.device)
-                idx = torch.empty(blocks + 1, dtype=torch.int64, device=x.device) if return_index else None
-                scratch = None
-            else:
-                out = torch.empty(cap, dtype=torch.uint8, device=x.device)
-                idx = torch.empty(blocks + 1, dtype=torch.int64, device=x.device)
-                scratch = torch.empty(lib.gcow_encode_tiles_scratch_bytes(p.as_c(), blocks, dim), dtype=torch.uint8,
-                                      device=x.device)
-            _check(lib.gcow_encode_tiles(x.data_ptr(), nx, ny, p.as_c(), out.data_ptr(),
-                                         scratch.data_ptr() if scratch is not None else None,
-                                         idx.data_ptr() if idx is not None else None, _stream_ptr()), "gcow_encode_tiles")
-            if p.fixed_rate:
-                return Compressed(out, p, shape, idx)
-            return Compressed(out[:((int(idx[-1].item()) + 63) // 64) * 8], p, shape, idx)
         scratch_bytes = lib.gcow_encode_generic_scratch_bytes(p.as_c(), blocks, dim)
         scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=x.device)
         out = torch.empty(cap, dtype=torch.uint8, device=x.device)
-        idx = torch.empty(blocks + 1, dtype=torch.int64, device=x.device)
+        idx = torch.zeros(blocks + 1, dtype=torch.int64, device=x.device)
         _check(lib.gcow_encode_generic(x.data_ptr(), nx, ny, p.as_c(), out.data_ptr(), cap,
                                        scratch.data_ptr(), idx.data_ptr(), _stream_ptr()),
                "gcow_encode_generic")
@@ -215,17 +204,21 @@ def compress(x: torch.Tensor, *, rate: float | None = None, tolerance: float | N
 def decompress(c: Compressed, out: torch.Tensor | None = None, *, shift: int = 0) -> torch.Tensor:
     """Inverse of :func:`compress`. ``shift`` divides every value by 2**shift
     exactly (used to average over a power-of-two number of ranks)."""
-    p, shape = c.params, tuple(c.shape)
-    nx, ny = _nxny(shape)
-    dev = c.stream.device
+    p, shape, stream = c.params, tuple(c.shape), c.stream
+    if out is not None and (out.dtype != torch.float32 or not out.is_contiguous() or out.numel() != math.prod(shape)):
+        raise ValueError("out must be a contiguous float32 tensor of the original size")
+    stream = stream.contiguous()
+    if stream.is_cuda and (out is None or out.is_cuda):
+        y = (_native._ext or _native.ext()).decompress(stream, c.index, p.minbits, p.maxbits, p.maxprec, p.minexp, shape, out, shift)
+        if y is not None:
+            return y
+    dev = stream.device
     if out is None:
         out = torch.empty(shape, dtype=torch.float32, device=dev)
-    if out.dtype != torch.float32 or not out.is_contiguous() or out.numel() != (nx * (ny or 1)):
-        raise ValueError("out must be a contiguous float32 tensor of the original size")
     if out.numel() == 0:
         return out
-    stream = c.stream.contiguous()
 
+    nx, ny = _nxny(shape)
     if not stream.is_cuda:
         buf = _padded_words(stream)
         _native.cpu().gcow_oracle_decompress(buf.data_ptr(), out.data_ptr(), nx, ny, p.as_c(), shift,
@@ -234,10 +227,6 @@ def decompress(c: Compressed, out: torch.Tensor | None = None, *, shift: int = 0
 
     lib = _native.cuda()
     with torch.cuda.device(dev):
-        if len(shape) == 1 and p.fixed_rate and p.maxbits in _FAST_BITS:
-            _check(lib.gcow_decode_1d_fixed(stream.data_ptr(), out.data_ptr(), nx, p.maxbits, shift,
-                                            _stream_ptr()), "gcow_decode_1d_fixed")
-            return out
         if not p.fixed_rate and c.index is None:
             # block offsets of a variable-rate stream are only known by walking
             # it; without an index that walk is serial, so it runs on the host

@@ -99,13 +99,15 @@ template <> struct CodeIO<128> {
 
 template <int BITS>
 __global__ void __launch_bounds__(kThreads)
-encode_1d_fixed_kernel(const float* __restrict__ in, uint64_t n, void* __restrict__ out, int aligned,
+encode_1d_fixed_kernel(const float* __restrict__ in, uint64_t n, void* __restrict__ out, int aligned, int pad_words16,
                        const uint16_t* __restrict__ tab, const uint32_t* __restrict__ pair_tab) {
   __shared__ __align__(16) uint32_t epair[kEncPairTabSize];
   load_pair_table(epair, pair_tab);
   __syncthreads();
   const LeanTables lt = {tab, nullptr, epair, nullptr};      // the plane-by-plane table is read from global memory (rare path)
   const uint64_t blocks = num_blocks_1d(n);
+  if (blockIdx.x == 0 && threadIdx.x < pad_words16)          // the stream's last 64-bit word
+    reinterpret_cast<uint16_t*>(out)[blocks * (BITS / 16) + threadIdx.x] = 0;
   for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < blocks;
        b += (uint64_t)gridDim.x * blockDim.x) {
     float f[4];
@@ -531,7 +533,7 @@ int gcow_codec_tables4(const void** etab, const void** dtab, const void** epair,
 // The tile kernels (tile_kernels.cu).
 int gcow_tile_usable(const int32_t* params, uint64_t blocks, int dim);
 int gcow_encode_tiles(const float* in, uint64_t nx, uint64_t ny, const int32_t* params, void* out, void* scratch,
-                      uint64_t* block_bits, void* stream);
+                      uint64_t* block_bits, uint64_t* total_out, void* stream);
 int gcow_decode_tiles(const void* in, float* out, uint64_t nx, uint64_t ny, const int32_t* params,
                       const uint64_t* block_bits, int shift, void* stream);
 
@@ -540,10 +542,7 @@ int gcow_codec_tables(const void** etab, const void** dtab) {
   return gcow_codec_tables4(etab, dtab, &pair, &loop);
 }
 
-// Fixed-rate 1-D encode; maxbits in {16, 32, 64, 128}. `out` holds
-// blocks*maxbits/8 bytes (caller rounds the buffer up to 8 bytes).
-int gcow_encode_1d_fixed(const float* in, uint64_t n, int maxbits, void* out, void* stream) {
-  cudaStream_t s = (cudaStream_t)stream;
+static int launch_encode_1d(const float* in, uint64_t n, int maxbits, void* out, bool pad, cudaStream_t s) {
   uint64_t blocks = num_blocks_1d(n);
   if (!blocks) return 0;
   int aligned = ((uintptr_t)in & 15) == 0;
@@ -552,14 +551,25 @@ int gcow_encode_1d_fixed(const float* in, uint64_t n, int maxbits, void* out, vo
   if (int rc = gcow_codec_tables4(&etp, &dtp, &ptp, &ltp)) return rc;
   const uint16_t* et = (const uint16_t*)etp;
   const uint32_t* pt = (const uint32_t*)ptp;
+  const int over = (int)(blocks * (uint64_t)maxbits % 64), pw = pad && over ? (64 - over) / 16 : 0;
   switch (maxbits) {
-    case 16: encode_1d_fixed_kernel<16><<<g, kThreads, 0, s>>>(in, n, out, aligned, et, pt); break;
-    case 32: encode_1d_fixed_kernel<32><<<g, kThreads, 0, s>>>(in, n, out, aligned, et, pt); break;
-    case 64: encode_1d_fixed_kernel<64><<<g, kThreads, 0, s>>>(in, n, out, aligned, et, pt); break;
-    case 128: encode_1d_fixed_kernel<128><<<g, kThreads, 0, s>>>(in, n, out, aligned, et, pt); break;
+    case 16: encode_1d_fixed_kernel<16><<<g, kThreads, 0, s>>>(in, n, out, aligned, pw, et, pt); break;
+    case 32: encode_1d_fixed_kernel<32><<<g, kThreads, 0, s>>>(in, n, out, aligned, pw, et, pt); break;
+    case 64: encode_1d_fixed_kernel<64><<<g, kThreads, 0, s>>>(in, n, out, aligned, pw, et, pt); break;
+    case 128: encode_1d_fixed_kernel<128><<<g, kThreads, 0, s>>>(in, n, out, aligned, pw, et, pt); break;
     default: return -1;
   }
   return (int)cudaGetLastError();
+}
+
+// Fixed-rate 1-D encode; maxbits in {16, 32, 64, 128}. `out` holds
+// blocks*maxbits/8 bytes (caller rounds the buffer up to 8 bytes).
+int gcow_encode_1d_fixed(const float* in, uint64_t n, int maxbits, void* out, void* stream) {
+  return launch_encode_1d(in, n, maxbits, out, false, (cudaStream_t)stream);
+}
+// The same with the stream's last 64-bit word zero padded; `out` holds that word.
+int gcow_encode_1d_stream(const float* in, uint64_t n, int maxbits, void* out, void* stream) {
+  return launch_encode_1d(in, n, maxbits, out, true, (cudaStream_t)stream);
 }
 
 int gcow_decode_1d_fixed(const void* in, float* out, uint64_t n, int maxbits, int shift, void* stream) {
@@ -597,7 +607,7 @@ static int launch_encode_generic(const float* in, uint64_t nx, uint64_t ny, cons
   const uint64_t tiles = (blocks + kScanTile - 1) / kScanTile;
   cudaMemsetAsync(out, 0, out_bytes, s);   // the scatter pass ORs into the stream, and callers find zeros after its end
   const int32_t q[4] = {(int32_t)p.minbits, (int32_t)p.maxbits, (int32_t)p.maxprec, p.minexp};
-  if (gcow_tile_usable(q, blocks, dim)) return gcow_encode_tiles(in, nx, ny, q, out, scratch, block_bits, s);
+  if (gcow_tile_usable(q, blocks, dim)) return gcow_encode_tiles(in, nx, ny, q, out, scratch, block_bits, nullptr, s);
   const int g = grid_for(blocks);
   if (dim == 1) encode_slots_kernel<1><<<g, kThreads, 0, s>>>(in, nx, ny, p, blocks, slots, lens);
   else encode_slots_kernel<2><<<g, kThreads, 0, s>>>(in, nx, ny, p, blocks, slots, lens);
@@ -643,7 +653,7 @@ int gcow_encode_fixed_direct(const float* in, uint64_t nx, uint64_t ny, const in
   if (!is_fixed_rate(p) || p.maxbits % 64) return -1;
   uint64_t blocks = ny ? num_blocks_2d(nx, ny) : num_blocks_1d(nx);
   if (!blocks) return 0;
-  if (gcow_tile_usable(params, blocks, ny ? 2 : 1)) return gcow_encode_tiles(in, nx, ny, params, out, nullptr, nullptr, stream);
+  if (gcow_tile_usable(params, blocks, ny ? 2 : 1)) return gcow_encode_tiles(in, nx, ny, params, out, nullptr, nullptr, nullptr, stream);
   int g = grid_for(blocks);
   if (ny) encode_fixed_direct_kernel<2><<<g, kThreads, 0, s>>>(in, nx, ny, p, blocks, out);
   else encode_fixed_direct_kernel<1><<<g, kThreads, 0, s>>>(in, nx, ny, p, blocks, out);

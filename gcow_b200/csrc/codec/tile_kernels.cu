@@ -288,7 +288,8 @@ constexpr int kPlaceUnits = 1024;
 
 template <int DIM>
 __global__ void __launch_bounds__(kTileThreads, DIM == 1 ? 4 : 5)
-place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restrict__ out, uint64_t* __restrict__ block_bits) {
+place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restrict__ out, uint64_t* __restrict__ block_bits,
+                     uint64_t* total_out) {
   constexpr int kPer = TileShape<DIM>::kPer, WB = TileShape<DIM>::kWarpBlocks;
   constexpr int kWords = DIM == 1 ? 8 : 3;                  // words per lane and step: a 1-D string is some 200 words, a 2-D one 70
   __shared__ unsigned long long s_sum[kTileWarps];
@@ -346,6 +347,11 @@ place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restric
       from += v[j];
     }
     __syncthreads();
+    // the caller's host thread waits for the stream's length: it gets it before the strings are moved
+    if (total_out && u0 + nu == units && tid == 0) {
+      *(volatile uint64_t*)total_out = base + all;
+      __threadfence_system();
+    }
 
     // The loads of a warp's next string are issued before the current one is written.
     struct Fetched { uint32_t w[kWords], len[kPer], q0, q1; } cur, nxt;
@@ -564,10 +570,49 @@ uint64_t gcow_encode_tiles_scratch_bytes(const int32_t* params, uint64_t blocks,
   return tile_scratch(p, blocks, dim).bytes;
 }
 
+// A word of pinned host memory of the calling thread, set to all ones: where an encode call leaves the stream's length for
+// the thread that made it. One per thread, given back when the thread ends.
+int gcow_host_word(uint64_t** word) {
+  struct Word {
+    uint64_t* p = nullptr;
+    ~Word() { if (p) (void)cudaFreeHost(p); }
+  };
+  static thread_local Word w;
+  if (!w.p) {
+    const cudaError_t e = cudaHostAlloc((void**)&w.p, 64, cudaHostAllocPortable | cudaHostAllocMapped);
+    if (e != cudaSuccess) { w.p = nullptr; return (int)e; }
+  }
+  *(volatile uint64_t*)w.p = ~0ull;
+  *word = w.p;
+  return 0;
+}
+
+// Waits until the device has written the word. The stream is asked now and then, so a launch that failed, or ended without
+// writing, ends the wait.
+int gcow_wait_host_word(volatile uint64_t* word, void* stream, uint64_t* value) {
+  for (;;) {
+    for (int i = 0; i < 512; i++) {
+      if ((*value = *word) != ~0ull) return 0;
+#if defined(__x86_64__)
+      __builtin_ia32_pause();
+#endif
+    }
+    const cudaError_t e = cudaStreamQuery((cudaStream_t)stream);
+    if (e == cudaSuccess) return (*value = *word) != ~0ull ? 0 : -1;
+    if (e != cudaErrorNotReady) return (int)e;
+  }
+}
+
+uint64_t gcow_max_stream_bytes(const int32_t* params, uint64_t blocks, int dim) {
+  const ZfpParams p = {(uint32_t)params[0], (uint32_t)params[1], (uint32_t)params[2], params[3]};
+  return max_output_bytes(p, blocks, dim);
+}
+
 // Encode without touching anything of `out` but the stream itself (its last word zero padded to 64 bits). `block_bits`
 // (blocks + 1, device) receives every block's start bit and the total; it may be null at fixed rate.
+// `total_out` (host memory that the device can write, or null): at variable rate also receives the total, early.
 int gcow_encode_tiles(const float* in, uint64_t nx, uint64_t ny, const int32_t* params, void* out, void* scratch,
-                      uint64_t* block_bits, void* stream) {
+                      uint64_t* block_bits, uint64_t* total_out, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   const ZfpParams p = {(uint32_t)params[0], (uint32_t)params[1], (uint32_t)params[2], params[3]};
   const int dim = ny ? 2 : 1;
@@ -603,8 +648,8 @@ int gcow_encode_tiles(const float* in, uint64_t nx, uint64_t ny, const int32_t* 
 #undef GCOW_ENCODE
   if (!fixed) {
     const uint32_t most = 148 * (dim == 1 ? 4 : 5), g = a.tiles < most ? a.tiles : most;
-    if (dim == 1) place_strings_kernel<1><<<g, kTileThreads, 0, s>>>(st, a, (uint32_t*)out, block_bits);
-    else place_strings_kernel<2><<<g, kTileThreads, 0, s>>>(st, a, (uint32_t*)out, block_bits);
+    if (dim == 1) place_strings_kernel<1><<<g, kTileThreads, 0, s>>>(st, a, (uint32_t*)out, block_bits, total_out);
+    else place_strings_kernel<2><<<g, kTileThreads, 0, s>>>(st, a, (uint32_t*)out, block_bits, total_out);
   }
   return (int)cudaGetLastError();
 }
