@@ -161,6 +161,7 @@ class CompressedAllReduce:
         self._peer_array = (C.c_void_p * 8)(*([C.c_void_p(p) for p in self.arena.peer_ptrs] +
                                                [C.c_void_p(0)] * (8 - len(self.arena.peer_ptrs))))
         self.status = torch.zeros(16, dtype=torch.int32, device=self.device)   # [0:8] record, [8] abort
+        self._status_addr, self._peer_addr = self.status.data_ptr(), C.addressof(self._peer_array)
         self.status_host = torch.zeros(16, dtype=torch.int32).pin_memory()
         self._lag_host = None          # check_lagged's two pinned slots, made on first use
         self.stamps = None
@@ -216,26 +217,22 @@ class CompressedAllReduce:
             raise TypeError("need a contiguous float32 CUDA tensor")
         out = x if out is None else out
         n = x.numel()
-        s = stream or torch.cuda.current_stream(self.device)
         if residual is not None and (residual.dtype != torch.float32 or residual.numel() != n or not residual.is_contiguous()
                                      or residual.device != x.device):
             raise TypeError("residual must be a contiguous float32 tensor of the input's size on the same device")
+        if out is not x and (out.dtype != torch.float32 or not out.is_contiguous() or out.numel() < n):
+            raise TypeError("out must be a contiguous float32 tensor of the input's size")
         for lo in range(0, n, self.max_numel):
-            hi = min(n, lo + self.max_numel)
-            self._launch(x.view(-1)[lo:hi], out.view(-1)[lo:hi], s, variant,
-                         residual.view(-1)[lo:hi] if residual is not None else None)
+            self._launch(x, out, lo, min(self.max_numel, n - lo), stream, variant, residual)
         return out
 
-    def _launch(self, x: torch.Tensor, out: torch.Tensor, s: torch.cuda.Stream, variant: str | None,
-                residual: torch.Tensor | None = None) -> None:
-        n = x.numel()
-        if n == 0:
-            return
+    def _launch(self, x: torch.Tensor, out: torch.Tensor, lo: int, n: int, stream: torch.cuda.Stream | None,
+                variant: str | None, residual: torch.Tensor | None = None) -> None:
         if self.header_only:
-            with torch.cuda.stream(s):
+            with torch.cuda.stream(stream or torch.cuda.current_stream(self.device)):
                 if residual is not None:          # everything is dropped: the residual keeps the whole input
-                    residual.add_(x)
-                out.zero_()
+                    residual.view(-1)[lo:lo + n].add_(x.view(-1)[lo:lo + n])
+                out.view(-1)[lo:lo + n].zero_()
             self.calls += 1
             self.bytes_in += n * 4
             return
@@ -250,12 +247,12 @@ class CompressedAllReduce:
         post = self._avg_scale
         if v == 3:
             err = self.lib.gcow_ar_launch_sparse(
-                x.data_ptr(), out.data_ptr(), n, self.rank, self.world, self.bits, self.ctas_for(n), shift,
+                x.data_ptr() + 4 * lo, out.data_ptr() + 4 * lo, n, self.rank, self.world, self.bits, self.ctas_for(n), shift,
                 C.c_float(post), self._peer_array, self.region_cap, self.epoch, int(self.cfg.timeout_ms) * 1_000_000,
                 self.status.data_ptr(), self.status[8:].data_ptr(),
                 self.stamps.data_ptr() if self.stamps is not None else None,
-                residual.data_ptr() if residual is not None else None, self.params.minexp,
-                self.wire_codes.data_ptr(), s.cuda_stream)
+                residual.data_ptr() + 4 * lo if residual is not None else None, self.params.minexp,
+                self.wire_codes.data_ptr(), (stream or torch.cuda.current_stream(self.device)).cuda_stream)
             if err:
                 raise RuntimeError(f"gcow_ar_launch_sparse failed: {err}")
             self.calls += 1
@@ -266,14 +263,10 @@ class CompressedAllReduce:
             return
         if v == 1 and shift:          # one-shot has no final decode to fold the shift into
             post, shift = post * 2.0 ** (-shift), 0
-        err = self.lib.gcow_ar_launch_ef(
-            x.data_ptr(), out.data_ptr(), n, self.rank, self.world, v, self.bits, self.ctas_for(n), shift,
-            C.c_float(post), self._peer_array, C.c_void_p(self.arena.mc_ptr), self.region_cap, self.epoch,
-            int(self.cfg.timeout_ms) * 1_000_000, self.status.data_ptr(), self.status[8:].data_ptr(),
-            self.stamps.data_ptr() if self.stamps is not None else None,
-            residual.data_ptr() if residual is not None else None, s.cuda_stream)
-        if err:
-            raise RuntimeError(f"gcow_ar_launch failed: {err}")
+        (_native._ext or _native.ext()).ar_launch(
+            x, out, residual, lo, n, stream.cuda_stream if stream is not None else None, self.rank, self.world, v, self.bits,
+            self.ctas_for(n), shift, post, self._peer_addr, self.arena.mc_ptr, self.region_cap, self.epoch & 0xffffffff,
+            int(self.cfg.timeout_ms) * 1_000_000, self._status_addr, self.stamps.data_ptr() if self.stamps is not None else 0)
         self.calls += 1
         self.bytes_in += n * 4
         cb = ((n + 3) // 4) * self.bits // 8

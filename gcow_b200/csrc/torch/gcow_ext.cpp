@@ -26,6 +26,10 @@ int gcow_encode_tiles(const float* in, uint64_t nx, uint64_t ny, const int32_t* 
                       uint64_t* block_bits, uint64_t* total_out, void* stream);
 int gcow_decode_tiles(const void* in, float* out, uint64_t nx, uint64_t ny, const int32_t* params,
                       const uint64_t* block_bits, int shift, void* stream);
+int gcow_ar_launch_ef(const float* in, float* out, uint64_t n, int rank, int world, int variant, int bits, int ctas, int shift,
+                      float postscale, void* const* arenas, void* mc_arena, uint64_t region_cap, uint32_t epoch,
+                      uint64_t timeout_ns, uint32_t* status, uint32_t* abort_flag, unsigned long long* stamps, float* residual,
+                      void* stream);
 uint64_t gcow_max_stream_bytes(const int32_t* params, uint64_t blocks, int dim);
 int gcow_host_word(uint64_t** word);
 int gcow_wait_host_word(volatile uint64_t* word, void* stream, uint64_t* value);
@@ -156,7 +160,35 @@ PyObject* decompress(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
+// ar_launch(x, out, residual or None, first, count, stream or None, rank, world, variant, bits, ctas, shift, postscale, arenas,
+//           mc_arena, region_cap, epoch, timeout_ns, status, stamps): one launch of the fused all-reduce over `count` values
+// from `first` on. Addresses are ints; `stream` is a cudaStream_t as int, None for the current stream.
+PyObject* ar_launch(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 20 && THPVariable_Check(args[0]) && THPVariable_Check(args[1]), "ar_launch: bad arguments");
+  const at::Tensor& x = THPVariable_Unpack(args[0]);
+  const at::Tensor& out = THPVariable_Unpack(args[1]);
+  uint64_t v[20];
+  for (int i = 3; i < 20; i++) {
+    if (i == 12 || (i == 5 && args[5] == Py_None)) continue;
+    v[i] = PyLong_AsUnsignedLongLong(args[i]);
+  }
+  const double post = PyFloat_AsDouble(args[12]);
+  if (PyErr_Occurred()) return nullptr;
+  const c10::cuda::CUDAGuard guard(x.device());
+  void* const stream = args[5] == Py_None ? c10::cuda::getCurrentCUDAStream(x.device().index()).stream() : (void*)v[5];
+  float* const res = args[2] == Py_None ? nullptr : THPVariable_Unpack(args[2]).mutable_data_ptr<float>() + v[3];
+  uint32_t* const status = (uint32_t*)v[18];
+  const int err = gcow_ar_launch_ef(x.const_data_ptr<float>() + v[3], out.mutable_data_ptr<float>() + v[3], v[4], (int)v[6], (int)v[7],
+                                    (int)v[8], (int)v[9], (int)v[10], (int)v[11], (float)post, (void* const*)v[13], (void*)v[14],
+                                    v[15], (uint32_t)v[16], v[17], status, status + 8, (unsigned long long*)v[19], res, stream);
+  TORCH_CHECK(err == 0, "gcow_ar_launch failed: ", err);
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef methods[] = {
+    {"ar_launch", (PyCFunction)(void (*)())ar_launch, METH_FASTCALL, nullptr},
     {"compress", (PyCFunction)(void (*)())compress, METH_FASTCALL, nullptr},
     {"decompress", (PyCFunction)(void (*)())decompress, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr},

@@ -43,6 +43,27 @@ def test_single_rank_equals_oracle(rate):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("rate", [4, 8, 16, 32])
+def test_single_rank_round_trip_views_and_feedback(rate):
+    """The one-rank kernel on bases that are not 16-byte aligned, a partial last block, and with error feedback."""
+    p = ZfpParams.from_rate(rate, 1)
+    ar = CompressedAllReduce(1 << 16, GcowConfig(rate=rate))
+    for n, off in ((1, 0), (4, 1), (257, 3), (1025, 1), (40003, 2)):
+        base = torch.from_numpy(gen(n, n + 4)).cuda()
+        x, out = base[off:off + n], torch.zeros(n + 4, device="cuda")[1:n + 1]
+        want = allreduce_oracle(x.cpu().numpy()[None], p, "oneshot", 0)
+        ar(x, out=out)
+        assert np.array_equal(out.cpu().numpy().view(np.uint32), want.view(np.uint32))
+        res = torch.from_numpy(gen(n + 1, n)).cuda()
+        total = (x + res).cpu().numpy()
+        want = allreduce_oracle(total[None], p, "oneshot", 0)
+        ar(x, out=out, residual=res)
+        assert np.array_equal(out.cpu().numpy().view(np.uint32), want.view(np.uint32))
+        assert np.array_equal(res.cpu().numpy(), total - want)
+    ar.check()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("cap,tol", [(4, 1e-2), (8, 1e-3), (16, 1e-6), (32, 1e-4)])
 def test_accuracy_mode_single_rank_equals_oracle(cap, tol):
     """Fixed accuracy with a bit cap (the sparse variant): bit-exact against the host model at the same four codec
