@@ -51,7 +51,7 @@ def _sources(kind: str) -> list[Path]:
 
 
 def _headers() -> list[Path]:
-    return sorted(list(CSRC.rglob("*.h")) + list(CSRC.rglob("*.cuh")))
+    return sorted(p for e in ("*.h", "*.cuh") for p in CSRC.rglob(e) if "torch" not in p.parts)
 
 
 def _digest(files: list[Path], flags: list[str]) -> str:
@@ -186,7 +186,7 @@ def build_ext(force: bool = False) -> Path:
     srcs = _sources("ext")
     flags = ["-std=c++17", "-O2", "-fPIC", "-fvisibility=hidden", f"-DGCOW_TORCH_{torch.__version__.split('+')[0].replace('.', '_')}",
              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
-    digest = _digest(srcs, flags)
+    digest = _digest(srcs + sorted((CSRC / "torch").glob("*.h")), flags)
     if not force and _up_to_date(name, digest):
         return LIB / f"{name}.so"
     with _build_lock():

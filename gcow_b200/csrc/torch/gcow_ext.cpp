@@ -17,6 +17,8 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Exceptions.h>
 
+#include "layers.h"
+
 extern "C" {
 int gcow_encode_1d_stream(const float* in, uint64_t n, int maxbits, void* out, void* stream);
 int gcow_decode_1d_fixed(const void* in, float* out, uint64_t n, int maxbits, int shift, void* stream);
@@ -197,4 +199,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "gcow_ext", "native host path of gc
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit_gcow_ext(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit_gcow_ext(void) {
+  PyObject* m = PyModule_Create(&module);
+  if (m && PyModule_AddFunctions(m, gcow_ext::layer_methods)) Py_CLEAR(m);
+  return m;
+}

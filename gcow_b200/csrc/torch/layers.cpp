@@ -1,0 +1,954 @@
+// The training layers' autograd functions: allocation, routing and launches of the tensor-core, normalisation and attention
+// kernels, forward and backward, without Python between them.
+//
+// One BERT layer is 12 function calls and about 35 launches; as Python autograd functions with ctypes launches that was
+// 1.1 ms of host time forward and backward, five times the device time of a small batch. The arithmetic, the kernels and
+// their order are those of the Python functions these replace (ops/kernels.py keeps the less used ones).
+#include "layers.h"
+
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <atomic>
+#include <cstdlib>
+#include <cstring>
+#include <mutex>
+
+extern "C" {
+int gcow_gemm2_max_pairs();
+int gcow_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, const float* bias,
+                    const void* residual, void* aux, int flags, uint32_t* error, int b_mn, void* stream);
+int gcow_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, const float* bias,
+                   const void* residual, int flags, uint32_t* error, int max_ctas, int a_mn, int b_mn, int tile_rows, void* stream);
+int gcow_gemm_bf16_aux(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, const float* bias,
+                       const void* residual, void* aux, int flags, uint32_t* error, int a_mn, int b_mn, int tile_rows, void* stream);
+int gcow_gemm_bf16_batched(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int batch,
+                           long long stride_a, long long stride_b, long long stride_c, const float* bias, const void* residual,
+                           int flags, uint32_t* error, int a_mn, int b_mn, int tile_rows, void* stream);
+int gcow_reduce_partials(const float* part, float* out, int parts, int64_t n, void* stream);
+int gcow_colsum_parts(int rows);
+int gcow_colsum(const void* g, float* part, float* out, int rows, int cols, int ld, void* stream);
+int gcow_layernorm_fwd(const void* x, const float* gamma, const float* beta, void* y, float* mean, float* rstd, int rows, int H,
+                       float eps, void* stream);
+int gcow_layernorm_bwd_parts(int rows);
+int gcow_layernorm_bwd(const void* dy, const void* x, const float* gamma, const float* mean, const float* rstd, void* dx,
+                       float* part, float* dgb, int rows, int H, void* stream);
+int gcow_attention_fwd(const void* qkv, void* out, float* lse, int B, int S, int H, int d, float scale, uint32_t* error, void* stream);
+int gcow_attention_bwd(const void* qkv, const void* out, const void* dout, const float* lse, float* delta, void* dqkv, int B, int S,
+                       int H, int d, float scale, uint32_t* error, void* stream);
+int gcow_softmax_fwd(const void* x, void* y, int64_t rows, int S, float scale, void* stream);
+int gcow_softmax_bwd(const void* dp, const void* p, void* ds, int64_t rows, int S, float scale, void* stream);
+int gcow_bn_parts(int64_t R, int C);
+int gcow_bn_fwd_train(const void* x, const void* residual, void* y, void* mask, const float* gamma, const float* beta, float* run_mean,
+                      float* run_var, float* stats, float* part, int64_t R, int C, float eps, float momentum, int relu, void* stream);
+int gcow_bn_bwd3(const void* dy, const void* dy2, const void* mask, const void* x, const float* gamma, const float* stats, void* dx,
+                 void* dres, float* dgamma, float* dbeta, float* part, int64_t R, int C, int relu, void* stream);
+int gcow_conv_fwd(const void* x, const void* w, void* y, const float* bias, int N, int Hin, int Win, int Ci, int Co, int kh, int kw,
+                  int pad_h, int pad_w, uint32_t* error, void* stream);
+int gcow_conv_fwd_strided(const void* x, const void* w, void* y, const float* bias, int N, int Hin, int Win, int Ci, int Co, int kh,
+                          int kw, int pad_h, int pad_w, int stride, uint32_t* error, void* stream);
+int gcow_conv_fwd_ws(const void* x, const void* w, void* y, const float* bias, int N, int H, int W, uint32_t* error, void* stream);
+int gcow_conv_fwd_halo(const void* x, const void* w, void* y, const float* bias, int N, int H, int W, int Ci, uint32_t* error,
+                       void* stream);
+int gcow_conv_ws_usable(int N, int H, int W);
+int gcow_conv_halo_usable(int N, int H, int W, int Ci);
+int gcow_conv_flip_weights(const void* w, void* wt, int Co, int kh, int kw, int Ci, void* stream);
+int gcow_conv_wgrad_ws_split(int N, int H, int W);
+int gcow_conv_wgrad_ws(const void* dy, const void* x, float* part, int N, int H, int W, uint32_t* error, void* stream);
+int gcow_conv_wgrad_halo_split(int N, int H, int W, int Ci, int Co);
+int gcow_conv_wgrad_halo(const void* dy, const void* x, float* part, int N, int H, int W, int Ci, int Co, uint32_t* error,
+                         void* stream);
+int gcow_conv_wgrad_split(int N, int Hin, int Win, int Ci, int Co, int kh, int kw, int pad_h, int pad_w);
+int gcow_conv_wgrad(const void* dy, const void* x, float* part, int N, int Hin, int Win, int Ci, int Co, int kh, int kw, int pad_h,
+                    int pad_w, uint32_t* error, void* stream);
+int gcow_conv_wgrad_split_strided(int N, int Hin, int Win, int Ci, int Co, int kh, int kw, int pad_h, int pad_w, int stride);
+int gcow_conv_wgrad_strided(const void* dy, const void* x, float* part, int N, int Hin, int Win, int Ci, int Co, int kh, int kw,
+                            int pad_h, int pad_w, int stride, uint32_t* error, void* stream);
+int gcow_conv_dgrad_1x1_s2(const void* dy, const void* wt, void* dx, int N, int Hin, int Win, int Ci, int Co, uint32_t* error,
+                           void* stream);
+int gcow_conv_dgrad_s2(const void* dy, const void* w, void* wp, void* dx, int N, int Hin, int Win, int Ci, int Co, uint32_t* error,
+                       void* stream);
+}
+
+namespace gcow_ext {
+
+using at::Tensor;
+using torch::autograd::variable_list;
+
+namespace {
+
+std::atomic<int64_t> g_launches{0}, g_view_hits{0};
+std::mutex g_error_mu;
+Tensor g_error[64];
+
+constexpr int kOutF32 = 1, kBias = 2, kGelu = 4, kResidual = 8, kAuxOut = 32, kGeluGrad = 64;
+
+void check(int err, const char* what) {
+  TORCH_CHECK(err == 0, what, " refused the call: ", err);
+}
+inline bool env_off(const char* name) {
+  const char* e = getenv(name);
+  return e && !strcmp(e, "0");
+}
+// The current stream of a tensor's device; the guard makes that device current.
+struct On {
+  c10::cuda::CUDAGuard guard;
+  void* stream;
+  uint32_t* error;
+  explicit On(const Tensor& t)
+      : guard(t.device()), stream(c10::cuda::getCurrentCUDAStream(t.device().index()).stream()),
+        error((uint32_t*)error_word(t.device().index()).mutable_data_ptr()) {}
+};
+inline Tensor empty(c10::IntArrayRef shape, at::ScalarType t, const Tensor& like) {
+  return at::detail::empty_cuda(shape, t, like.device(), std::nullopt);
+}
+inline Tensor empty_nhwc(int64_t N, int64_t C, int64_t H, int64_t W, const Tensor& like) {
+  return at::detail::empty_cuda({N, C, H, W}, at::kBFloat16, like.device(), at::MemoryFormat::ChannelsLast);
+}
+inline float* f32(const Tensor& t) { return t.defined() ? (float*)t.data_ptr() : nullptr; }
+inline void* raw(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+inline Tensor bf16_rows(const Tensor& t) {                  // contiguous bf16, copied only where it is not
+  return (t.scalar_type() == at::kBFloat16 ? t : t.to(at::kBFloat16)).contiguous();
+}
+inline Tensor float_vector(const Tensor& t) {
+  return !t.defined() ? t : (t.scalar_type() == at::kFloat ? t : t.to(at::kFloat)).contiguous();
+}
+inline Tensor nhwc_bf16(const Tensor& t) {
+  if (t.scalar_type() == at::kBFloat16 && t.is_contiguous(at::MemoryFormat::ChannelsLast)) return t;
+  return t.to(at::kBFloat16).contiguous(at::MemoryFormat::ChannelsLast);
+}
+
+// ------------------------------------------------------------------------ products
+bool pair_gemm_enabled() {
+  static const bool on = !env_off("GCOW_GEMM2") && gcow_gemm2_max_pairs() > 0;
+  return on;
+}
+
+struct GemmOpts {
+  Tensor bias, residual, pre_gelu_out, gelu_grad_of, out;
+  bool gelu = false, a_t = false, b_t = false, out_f32 = false;
+};
+
+// C[M,N] = op(A) op(B)^T with the epilogues of the tcgen05 kernels; the routing rule and its reasons are those of
+// ops/kernels.py::gemm_bf16.
+Tensor gemm(const Tensor& a, const Tensor& b, const GemmOpts& o, const On& on) {
+  const int64_t M = o.a_t ? a.size(1) : a.size(0), K = o.a_t ? a.size(0) : a.size(1);
+  const int64_t N = o.b_t ? b.size(1) : b.size(0), Kb = o.b_t ? b.size(0) : b.size(1);
+  TORCH_CHECK(K == Kb, "gemm: reduction lengths differ");
+  Tensor out = o.out.defined() ? o.out : empty({M, N}, o.out_f32 ? at::kFloat : at::kBFloat16, a);
+  const Tensor& aux = o.pre_gelu_out.defined() ? o.pre_gelu_out : o.gelu_grad_of;
+  int flags = (out.scalar_type() == at::kFloat ? kOutF32 : 0) | (o.bias.defined() ? kBias : 0) | (o.gelu ? kGelu : 0) |
+              (o.residual.defined() ? kResidual : 0);
+  if (aux.defined()) flags |= o.pre_gelu_out.defined() ? kAuxOut : kGeluGrad;
+  const int lda = (int)a.stride(0), ldb = (int)b.stride(0), ldc = (int)out.stride(0);
+  if (pair_gemm_enabled() && !o.a_t && !(flags & kOutF32) && K % 64 == 0 && K >= 512 && N % (o.b_t ? 64 : 32) == 0 && M >= 1024 &&
+      N >= 256 && lda % 8 == 0 && ldb % 8 == 0 && ldc % 8 == 0 && !(K >= 2048 && ((M + 255) / 256) * ((N + 255) / 256) >= 118)) {
+    const int err = gcow_gemm2_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, lda, ldb, ldc, f32(o.bias),
+                                    raw(o.residual), raw(aux), flags, on.error, o.b_t, on.stream);
+    if (err == 0) { g_launches++; return out; }
+    TORCH_CHECK(err == -2, "gcow_gemm2_bf16 refused the call: ", err);
+  }
+  if (aux.defined())
+    check(gcow_gemm_bf16_aux(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, lda, ldb, ldc, f32(o.bias),
+                             raw(o.residual), raw(aux), flags, on.error, o.a_t, o.b_t, 0, on.stream), "gcow_gemm_bf16_aux");
+  else
+    check(gcow_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, lda, ldb, ldc, f32(o.bias),
+                         raw(o.residual), flags, on.error, 0, o.a_t, o.b_t, 0, on.stream), "gcow_gemm_bf16");
+  g_launches++;
+  return out;
+}
+
+// Ordered sum of `parts` fp32 partial results into `out` (allocated when undefined).
+Tensor add_parts(const Tensor& part, int64_t parts, c10::IntArrayRef shape, Tensor out, const On& on) {
+  if (!out.defined()) out = empty(shape, at::kFloat, part);
+  check(gcow_reduce_partials(f32(part), f32(out), (int)parts, out.numel(), on.stream), "gcow_reduce_partials");
+  g_launches++;
+  return out;
+}
+
+// dW[N,K] = g^T x, fp32, the long reduction split into slabs whose products are added in order (ops/kernels.py::wgrad_gemm).
+Tensor wgrad(const Tensor& g, const Tensor& x, const Tensor& out, const On& on) {
+  const int64_t M = g.size(0), N = g.size(1), K = x.size(1);
+  const int64_t tiles = ((N + 127) / 128) * ((K + 255) / 256);
+  int64_t s = 1;
+  while (s < 64 && tiles * s * 2 <= 148 && M % (2 * s) == 0 && (M / (2 * s)) % 64 == 0 && M / (2 * s) >= 512) s *= 2;
+  if (s == 1 || g.stride(0) != N || x.stride(0) != K) {
+    GemmOpts o;
+    o.a_t = o.b_t = o.out_f32 = true;
+    o.out = out;
+    return gemm(g, x, o, on);
+  }
+  const Tensor part = empty({s, N, K}, at::kFloat, g);
+  const int64_t m = M / s;
+  check(gcow_gemm_bf16_batched(g.data_ptr(), x.data_ptr(), part.data_ptr(), (int)N, (int)K, (int)m, (int)N, (int)K, (int)K, (int)s,
+                               m * N, m * K, N * K, nullptr, nullptr, kOutF32, on.error, 1, 1, 0, on.stream), "gcow_gemm_bf16_batched");
+  g_launches++;
+  return add_parts(part, s, {N, K}, out, on);
+}
+
+Tensor colsum(const Tensor& g, const On& on) {
+  const int64_t rows = g.size(0), cols = g.size(1);
+  if (cols % 2 || g.stride(1) != 1 || g.stride(0) % 2) return g.to(at::kFloat).sum(0);
+  const Tensor part = empty({gcow_colsum_parts((int)rows) * cols}, at::kFloat, g), out = empty({cols}, at::kFloat, g);
+  check(gcow_colsum(g.data_ptr(), f32(part), f32(out), (int)rows, (int)cols, (int)g.stride(0), on.stream), "gcow_colsum");
+  g_launches += 2;
+  return out;
+}
+
+// ------------------------------------------------------- weights: bf16 copies, gradient targets
+PyObject* name_bf16() { static PyObject* s = PyUnicode_InternFromString("_gcow_bf16"); return s; }
+PyObject* name_version() { static PyObject* s = PyUnicode_InternFromString("_gcow_bf16_version"); return s; }
+PyObject* name_view() { static PyObject* s = PyUnicode_InternFromString("_gcow_grad_view"); return s; }
+
+// An attribute of a parameter object, or null (no error set) where there is none.
+PyObject* attr(PyObject* o, PyObject* name) {
+  PyObject* v = PyObject_GetAttr(o, name);
+  if (!v) PyErr_Clear();
+  return v;
+}
+
+// ops/kernels.py::bf16_weight
+Tensor bf16_weight(PyObject* obj) {
+  const Tensor& w = THPVariable_Unpack(obj);
+  PyObject* sh = attr(obj, name_bf16());
+  if (!sh || !THPVariable_Check(sh) || w.scalar_type() != at::kFloat || THPVariable_Unpack(sh).sizes() != w.sizes() ||
+      THPVariable_Unpack(sh).device() != w.device()) {
+    Py_XDECREF(sh);
+    const Tensor d = w.detach();
+    return d.scalar_type() == at::kBFloat16 ? d : d.to(at::kBFloat16);
+  }
+  Tensor copy = THPVariable_Unpack(sh);
+  Py_DECREF(sh);
+  PyObject* ver = attr(obj, name_version());
+  const long have = ver ? PyLong_AsLong(ver) : -1;
+  Py_XDECREF(ver);
+  PyErr_Clear();
+  const long now = (long)w._version();
+  if (have != now) {
+    at::NoGradGuard no_grad;
+    copy.copy_(w.detach());
+    PyObject* v = PyLong_FromLong(now);
+    if (PyObject_SetAttr(obj, name_version(), v)) PyErr_Clear();
+    Py_DECREF(v);
+  }
+  return copy;
+}
+
+// Where a weight's gradient may be written (ops/kernels.py::take_grad_view): taken at most once per step.
+Tensor take_grad_view(PyObject* obj) {
+  const Tensor& w = THPVariable_Unpack(obj);
+  if (w.scalar_type() != at::kFloat) return Tensor();
+  PyObject* v = attr(obj, name_view());
+  if (!v || v == Py_None || !THPVariable_Check(v)) { Py_XDECREF(v); return Tensor(); }
+  Tensor gv = THPVariable_Unpack(v);
+  Py_DECREF(v);
+  if (PyObject_SetAttr(obj, name_view(), Py_None)) PyErr_Clear();
+  if (gv.scalar_type() != at::kFloat || gv.sizes() != w.sizes() || gv.device() != w.device()) return Tensor();
+  return gv;
+}
+
+// A gradient target held by a backward function. `w` is the weight itself: its .grad tells whether gradients accumulate.
+struct Target { Tensor view, weight; };
+
+// The [rows, cols] fp32 matrix to write (undefined where there is none) and the tensor to return as the gradient.
+Tensor target_matrix(const Target& t, int64_t rows, int64_t cols, uintptr_t align, Tensor* result) {
+  if (!t.view.defined() || t.weight.grad().defined()) return Tensor();
+  const Tensor flat = t.view.dim() == 4 ? t.view.permute({0, 2, 3, 1}) : t.view;
+  if (!flat.is_contiguous() || flat.numel() != rows * cols || (uintptr_t)t.view.data_ptr() % align) return Tensor();
+  g_view_hits++;
+  *result = t.view.as_strided(t.view.sizes(), t.view.strides());
+  return flat.view({rows, cols});
+}
+
+// ---------------------------------------------------------------------- autograd nodes
+// A tensor kept for the backward pass: detached, with the version check that catches in-place writes in between.
+struct Kept {
+  Tensor t;
+  uint32_t version = 0;
+  void set(const Tensor& x) {
+    if (!x.defined()) return;
+    t = x.requires_grad() ? x.tensor_data() : x;            // shares the version counter
+    version = (uint32_t)x._version();
+  }
+  const Tensor& get() const {
+    TORCH_CHECK(t.defined(), "Trying to backward through the graph a second time, or to use a tensor that was freed by the first");
+    TORCH_CHECK((uint32_t)t._version() == version, "a tensor needed for gradient computation has been modified by an inplace operation");
+    return t;
+  }
+};
+
+// Backward nodes: `kept` holds the saved tensors, inputs are numbered in the order given to record().
+struct LayerNode : torch::autograd::Node {
+  Kept kept[6];
+  Target target[2];
+  void release_variables() override {
+    for (auto& k : kept) k.t.reset();
+    for (auto& t : target) { t.view.reset(); t.weight.reset(); }
+  }
+  bool wants(size_t i) { return task_should_compute_output(i); }
+  virtual variable_list grads(variable_list&& g) = 0;
+  variable_list apply(variable_list&& g) override {
+    at::NoGradGuard no_grad;
+    at::AutoDispatchBelowADInplaceOrView below;
+    return grads(std::move(g));
+  }
+};
+
+template <class N, class... In>
+std::shared_ptr<N> record(const In&... in) {
+  if (!at::GradMode::is_enabled() || !torch::autograd::compute_requires_grad(in...)) return nullptr;
+  std::shared_ptr<N> n(new N(), torch::autograd::deleteNode);
+  n->set_next_edges(torch::autograd::collect_next_edges(in...));
+  return n;
+}
+// Everything up to the history of the result runs below autograd.
+struct Below {
+  at::NoGradGuard no_grad;
+  at::AutoDispatchBelowADInplaceOrView below;
+};
+template <class N>
+PyObject* finish(Tensor out, const std::shared_ptr<N>& n) {
+  if (n) torch::autograd::set_history(out, n);
+  return THPVariable_Wrap(std::move(out));
+}
+inline Tensor arg(PyObject* o) { return o == Py_None ? Tensor() : THPVariable_Unpack(o); }   // None: undefined
+inline Tensor rows_of(const Tensor& x) { return bf16_rows(x.reshape({-1, x.size(-1)})); }
+inline Tensor as_rows(const Tensor& x) { return x.view({-1, x.size(-1)}); }
+inline std::vector<int64_t> with_last(const Tensor& x, int64_t last) {
+  std::vector<int64_t> s = x.sizes().vec();
+  s.back() = last;
+  return s;
+}
+
+// dW of a linear layer: into the trainer's target where there is one, else a new tensor.
+Tensor linear_wgrad(const Target& t, const Tensor& g, const Tensor& x, const On& on) {
+  Tensor result;
+  const Tensor flat = target_matrix(t, g.size(1), x.size(1), 16, &result);
+  if (flat.defined()) { wgrad(g, x, flat, on); return result; }
+  return wgrad(g, x, Tensor(), on);
+}
+
+// ---------------------------------------------------------------------- linear layers
+struct LinearNode : LayerNode {                             // inputs: x, w, b, residual
+  std::vector<int64_t> x_shape;
+  bool has_bias = false, has_res = false;
+  std::string name() const override { return "GcowLinearBackward"; }
+  variable_list grads(variable_list&& in) override {
+    variable_list out(4);
+    if (!in[0].defined()) return out;
+    const Tensor &xb = kept[0].get(), &wb = kept[1].get();
+    const On on(xb);
+    const Tensor g = rows_of(in[0]);
+    if (wants(0)) {                                         // dx[M,K] = g[M,N] W[N,K]: W is stored [reduction N][K]
+      GemmOpts o;
+      o.b_t = true;
+      o.out = empty(x_shape, at::kBFloat16, g);
+      Tensor full = o.out;
+      o.out = as_rows(full);
+      gemm(g, wb, o, on);
+      out[0] = std::move(full);
+    }
+    if (wants(1)) out[1] = linear_wgrad(target[0], g, xb, on);
+    if (has_bias && wants(2)) out[2] = colsum(g, on);
+    if (has_res && wants(3)) out[3] = in[0];
+    return out;
+  }
+};
+
+// linear(x, w, b or None, residual or None): x W^T + b (+ residual, in the epilogue)
+PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 4, "linear: bad arguments");
+  const Tensor x = arg(args[0]), w = arg(args[1]), b = arg(args[2]), r = arg(args[3]);
+  auto node = record<LinearNode>(x, w, b, r);
+  Tensor out;
+  {
+    Below below;
+    const On on(x);
+    const Tensor xb = rows_of(x), wb = bf16_weight(args[1]).contiguous();
+    out = empty(r.defined() ? r.sizes().vec() : with_last(x, w.size(0)), at::kBFloat16, x);
+    GemmOpts o;
+    o.bias = float_vector(b);
+    if (r.defined()) o.residual = rows_of(r);
+    o.out = as_rows(out);
+    gemm(xb, wb, o, on);
+    if (node) {
+      node->kept[0].set(xb);
+      node->kept[1].set(wb);
+      node->x_shape = x.sizes().vec();
+      node->has_bias = b.defined();
+      node->has_res = r.defined();
+      node->target[0] = {take_grad_view(args[1]), w};
+    }
+  }
+  return finish(std::move(out), node);
+  END_HANDLE_TH_ERRORS
+}
+
+struct FfnNode : LayerNode {                                // inputs: x, w1, b1, w2, b2
+  std::vector<int64_t> shape;
+  std::string name() const override { return "GcowFfnBackward"; }
+  variable_list grads(variable_list&& in) override {
+    variable_list out(5);
+    if (!in[0].defined()) return out;
+    const Tensor &xb = kept[0].get(), &w1b = kept[1].get(), &w2b = kept[2].get(), &pre = kept[3].get(), &act = kept[4].get();
+    const On on(xb);
+    const Tensor g = rows_of(in[0]);
+    GemmOpts o;
+    o.b_t = true;
+    o.gelu_grad_of = pre;
+    const Tensor dpre = gemm(g, w2b, o, on);                // (g W2) * GELU'(pre)
+    if (wants(3)) out[3] = linear_wgrad(target[1], g, act, on);
+    if (wants(4)) out[4] = colsum(g, on);
+    if (wants(0)) {
+      Tensor full = empty(shape, at::kBFloat16, g);
+      GemmOpts q;
+      q.b_t = true;
+      q.residual = g;
+      q.out = as_rows(full);
+      gemm(dpre, w1b, q, on);
+      out[0] = std::move(full);
+    }
+    if (wants(1)) out[1] = linear_wgrad(target[0], dpre, xb, on);
+    if (wants(2)) out[2] = colsum(dpre, on);
+    return out;
+  }
+};
+
+// ffn_residual(x, w1, b1, w2, b2): x + GELU(x W1^T + b1) W2^T + b2
+PyObject* ffn_residual(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 5, "ffn_residual: bad arguments");
+  const Tensor x = arg(args[0]), w1 = arg(args[1]), b1 = arg(args[2]), w2 = arg(args[3]), b2 = arg(args[4]);
+  auto node = record<FfnNode>(x, w1, b1, w2, b2);
+  Tensor out;
+  {
+    Below below;
+    const On on(x);
+    const Tensor xb = rows_of(x), w1b = bf16_weight(args[1]).contiguous(), w2b = bf16_weight(args[3]).contiguous();
+    GemmOpts o;
+    o.bias = float_vector(b1);
+    o.gelu = true;
+    o.pre_gelu_out = empty({xb.size(0), w1b.size(0)}, at::kBFloat16, x);
+    const Tensor act = gemm(xb, w1b, o, on);
+    out = empty(x.sizes(), at::kBFloat16, x);
+    GemmOpts q;
+    q.bias = float_vector(b2);
+    q.residual = xb;
+    q.out = as_rows(out);
+    gemm(act, w2b, q, on);
+    if (node) {
+      const Tensor all[5] = {xb, w1b, w2b, o.pre_gelu_out, act};
+      for (int i = 0; i < 5; i++) node->kept[i].set(all[i]);
+      node->shape = x.sizes().vec();
+      node->target[0] = {take_grad_view(args[1]), w1};
+      node->target[1] = {take_grad_view(args[3]), w2};
+    }
+  }
+  return finish(std::move(out), node);
+  END_HANDLE_TH_ERRORS
+}
+
+// ---------------------------------------------------------------------- LayerNorm
+struct LayerNormNode : LayerNode {                          // inputs: x, gamma, beta
+  std::vector<int64_t> shape;
+  at::ScalarType ptype = at::kFloat;
+  std::string name() const override { return "GcowLayerNormBackward"; }
+  variable_list grads(variable_list&& in) override {
+    variable_list out(3);
+    if (!in[0].defined()) return out;
+    const Tensor &xb = kept[0].get(), &g32 = kept[1].get(), &mean = kept[2].get(), &rstd = kept[3].get();
+    const On on(xb);
+    const int64_t rows = xb.size(0), H = xb.size(1);
+    const Tensor g = rows_of(in[0]);
+    Tensor dx = empty(shape, at::kBFloat16, xb);
+    const Tensor part = empty({gcow_layernorm_bwd_parts((int)rows) * 2 * H}, at::kFloat, xb), dgb = empty({2 * H}, at::kFloat, xb);
+    check(gcow_layernorm_bwd(g.data_ptr(), xb.data_ptr(), f32(g32), f32(mean), f32(rstd), dx.data_ptr(), f32(part), f32(dgb), (int)rows,
+                             (int)H, on.stream), "gcow_layernorm_bwd");
+    g_launches += 2;
+    out[0] = std::move(dx);
+    out[1] = dgb.narrow(0, 0, H).to(ptype);
+    out[2] = dgb.narrow(0, H, H).to(ptype);
+    return out;
+  }
+};
+
+PyObject* layernorm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {      // (x, gamma, beta, eps)
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 4, "layernorm: bad arguments");
+  const Tensor x = arg(args[0]), gamma = arg(args[1]), beta = arg(args[2]);
+  const double eps = PyFloat_AsDouble(args[3]);
+  if (PyErr_Occurred()) return nullptr;
+  auto node = record<LayerNormNode>(x, gamma, beta);
+  Tensor out;
+  {
+    Below below;
+    const On on(x);
+    const Tensor xb = rows_of(x), g32 = float_vector(gamma), b32 = float_vector(beta);
+    const int64_t rows = xb.size(0), H = xb.size(1);
+    out = empty(x.sizes(), at::kBFloat16, x);
+    const Tensor mean = empty({rows}, at::kFloat, x), rstd = empty({rows}, at::kFloat, x);
+    check(gcow_layernorm_fwd(xb.data_ptr(), f32(g32), f32(b32), out.data_ptr(), f32(mean), f32(rstd), (int)rows, (int)H, (float)eps,
+                             on.stream), "gcow_layernorm_fwd");
+    g_launches++;
+    if (node) {
+      const Tensor all[4] = {xb, g32, mean, rstd};
+      for (int i = 0; i < 4; i++) node->kept[i].set(all[i]);
+      node->shape = x.sizes().vec();
+      node->ptype = gamma.scalar_type();
+    }
+  }
+  return finish(std::move(out), node);
+  END_HANDLE_TH_ERRORS
+}
+
+// ---------------------------------------------------------------------- attention
+struct FusedAttentionNode : LayerNode {                     // input: qkv
+  float scale = 1;
+  std::string name() const override { return "GcowAttentionBackward"; }
+  variable_list grads(variable_list&& in) override {
+    variable_list out(1);
+    if (!in[0].defined() || !wants(0)) return out;
+    const Tensor &q = kept[0].get(), &o = kept[1].get(), &lse = kept[2].get();
+    const On on(q);
+    const int B = (int)q.size(0), S = (int)q.size(1), H = (int)q.size(3), D = (int)q.size(4);
+    const Tensor g = bf16_rows(in[0]);
+    Tensor dqkv = at::empty_like(q);
+    const Tensor delta = empty({B, H, S}, at::kFloat, q);
+    check(gcow_attention_bwd(q.data_ptr(), o.data_ptr(), g.data_ptr(), f32(lse), f32(delta), dqkv.data_ptr(), B, S, H, D, scale, on.error,
+                             on.stream), "gcow_attention_bwd");
+    g_launches += 3;
+    out[0] = std::move(dqkv);
+    return out;
+  }
+};
+
+PyObject* fused_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {   // (qkv [B, S, 3, H, 64], scale)
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 2, "fused_attention: bad arguments");
+  const Tensor qkv = arg(args[0]);
+  const double scale = PyFloat_AsDouble(args[1]);
+  if (PyErr_Occurred()) return nullptr;
+  auto node = record<FusedAttentionNode>(qkv);
+  Tensor out;
+  {
+    Below below;
+    const On on(qkv);
+    const int64_t B = qkv.size(0), S = qkv.size(1), H = qkv.size(3), D = qkv.size(4);
+    const Tensor q = bf16_rows(qkv);
+    out = empty({B, S, H * D}, at::kBFloat16, q);
+    const Tensor lse = empty({B, H, S}, at::kFloat, q);
+    check(gcow_attention_fwd(q.data_ptr(), out.data_ptr(), f32(lse), (int)B, (int)S, (int)H, (int)D, (float)scale, on.error, on.stream),
+          "gcow_attention_fwd");
+    g_launches++;
+    if (node) {
+      node->kept[0].set(q);
+      node->kept[1].set(out);
+      node->kept[2].set(lse);
+      node->scale = (float)scale;
+    }
+  }
+  return finish(std::move(out), node);
+  END_HANDLE_TH_ERRORS
+}
+
+// C[i] = op(A[i]) op(B[i])^T for contiguous [batch, rows, cols] operands
+Tensor bmm(const Tensor& a, const Tensor& b, bool a_t, bool b_t, const On& on) {
+  const int64_t batch = a.size(0), M = a_t ? a.size(2) : a.size(1), K = a_t ? a.size(1) : a.size(2), N = b_t ? b.size(2) : b.size(1);
+  Tensor out = empty({batch, M, N}, at::kBFloat16, a);
+  check(gcow_gemm_bf16_batched(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, (int)a.stride(1), (int)b.stride(1),
+                               (int)N, (int)batch, a.stride(0), b.stride(0), M * N, nullptr, nullptr, 0, on.error, a_t, b_t, 128, on.stream),
+        "gcow_gemm_bf16_batched");
+  g_launches++;
+  return out;
+}
+
+struct AttentionNode : LayerNode {                          // inputs: q, k, v
+  float scale = 1;
+  std::string name() const override { return "GcowUnfusedAttentionBackward"; }
+  variable_list grads(variable_list&& in) override {
+    variable_list out(3);
+    if (!in[0].defined()) return out;
+    const Tensor &q = kept[0].get(), &k = kept[1].get(), &v = kept[2].get(), &p = kept[3].get();
+    const On on(q);
+    const Tensor go = bf16_rows(in[0]);
+    out[2] = bmm(p, go, true, true, on);                    // P^T dO
+    const Tensor dp = bmm(go, v, false, false, on);         // dO V^T
+    const Tensor ds = at::empty_like(p);
+    check(gcow_softmax_bwd(dp.data_ptr(), p.data_ptr(), ds.data_ptr(), p.size(0) * p.size(1), (int)p.size(2), scale, on.stream),
+          "gcow_softmax_bwd");
+    g_launches++;
+    out[0] = bmm(ds, k, false, true, on);                   // dS K
+    out[1] = bmm(ds, q, true, true, on);                    // dS^T Q
+    return out;
+  }
+};
+
+PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {      // (q, k, v [batch * heads, S, D] bf16, scale)
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 4, "attention: bad arguments");
+  const Tensor q = arg(args[0]), k = arg(args[1]), v = arg(args[2]);
+  const double scale = PyFloat_AsDouble(args[3]);
+  if (PyErr_Occurred()) return nullptr;
+  auto node = record<AttentionNode>(q, k, v);
+  Tensor out;
+  {
+    Below below;
+    const On on(q);
+    const Tensor s = bmm(q, k, false, false, on), p = at::empty_like(s);
+    check(gcow_softmax_fwd(s.data_ptr(), p.data_ptr(), s.size(0) * s.size(1), (int)s.size(2), (float)scale, on.stream), "gcow_softmax_fwd");
+    g_launches++;
+    out = bmm(p, v, false, true, on);
+    if (node) {
+      const Tensor all[4] = {q, k, v, p};
+      for (int i = 0; i < 4; i++) node->kept[i].set(all[i]);
+      node->scale = (float)scale;
+    }
+  }
+  return finish(std::move(out), node);
+  END_HANDLE_TH_ERRORS
+}
+
+// ---------------------------------------------------------------------- convolutions (NHWC bf16)
+struct ConvShape { int N, C, H, W, Co, KH, KW, OH, OW, ph, pw; };
+
+bool conv_ws(const ConvShape& s) {
+  return s.C == 64 && s.Co == 64 && s.KH == 3 && s.KW == 3 && s.ph == 1 && s.pw == 1 && !env_off("GCOW_CONV_WS") &&
+         gcow_conv_ws_usable(s.N, s.H, s.W);
+}
+bool conv_halo(const ConvShape& s) {
+  return s.Co == 128 && s.KH == 3 && s.KW == 3 && s.ph == 1 && s.pw == 1 && !env_off("GCOW_CONV_HALO") &&
+         gcow_conv_halo_usable(s.N, s.H, s.W, s.C);
+}
+// The stride-1 forward kernel for these extents: weight-stationary or halo-tile where they apply, else the general one.
+void conv_forward(const Tensor& x, const Tensor& w, const Tensor& y, const Tensor& bias, const ConvShape& s, const On& on) {
+  if (conv_ws(s)) check(gcow_conv_fwd_ws(x.data_ptr(), w.data_ptr(), y.data_ptr(), f32(bias), s.N, s.H, s.W, on.error, on.stream), "gcow_conv_fwd_ws");
+  else if (conv_halo(s)) check(gcow_conv_fwd_halo(x.data_ptr(), w.data_ptr(), y.data_ptr(), f32(bias), s.N, s.H, s.W, s.C, on.error, on.stream), "gcow_conv_fwd_halo");
+  else check(gcow_conv_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), f32(bias), s.N, s.H, s.W, s.C, s.Co, s.KH, s.KW, s.ph, s.pw, on.error, on.stream), "gcow_conv_fwd");
+  g_launches++;
+}
+
+// The weight gradient [Co, KH * KW * C] from `parts` partial results that launch(float* part) writes.
+template <class Launch>
+Tensor conv_wgrad(const Target& t, const ConvShape& s, int parts, const Tensor& like, const On& on, Launch launch) {
+  const int64_t cols = (int64_t)s.KH * s.KW * s.C;
+  Tensor result;
+  const Tensor flat = target_matrix(t, s.Co, cols, 16, &result);
+  Tensor out = flat;
+  if (parts > 1) {
+    const Tensor part = empty({parts, s.Co, cols}, at::kFloat, like);
+    launch(f32(part));
+    out = add_parts(part, parts, {s.Co, cols}, flat, on);
+  } else {
+    if (!out.defined()) out = empty({s.Co, cols}, at::kFloat, like);
+    launch(f32(out));
+  }
+  g_launches++;
+  return flat.defined() ? result : out.view({s.Co, s.KH, s.KW, s.C}).permute({0, 3, 1, 2});
+}
+Tensor conv_bias_grad(const Tensor& gy, int Co, const On& on) { return colsum(gy.permute({0, 2, 3, 1}).reshape({-1, Co}), on); }
+
+struct ConvNode : LayerNode {                               // inputs: x, w, b
+  ConvShape s;
+  int kind = 0, halo_min_w = 15;                            // kind: 0 stride 1, 1 1x1 stride 2, 2 3x3 stride 2
+  bool has_bias = false;
+  std::string name() const override { return "GcowConvBackward"; }
+  variable_list grads(variable_list&& in) override {
+    variable_list out(3);
+    if (!in[0].defined()) return out;
+    const Tensor &x = kept[0].get(), &wr = kept[1].get();
+    const On on(x);
+    const Tensor gy = nhwc_bf16(in[0]);
+    const void* const g = gy.data_ptr();
+    if (wants(0)) {
+      Tensor gx = empty_nhwc(s.N, s.C, s.H, s.W, x);
+      if (kind == 2) {
+        const Tensor wp = empty({9 * (int64_t)s.C * s.Co}, at::kBFloat16, x);
+        check(gcow_conv_dgrad_s2(g, wr.data_ptr(), wp.data_ptr(), gx.data_ptr(), s.N, s.H, s.W, s.C, s.Co, on.error, on.stream), "gcow_conv_dgrad_s2");
+        g_launches += 5;
+      } else {
+        const Tensor wt = empty({s.C, s.KH, s.KW, s.Co}, at::kBFloat16, x);
+        check(gcow_conv_flip_weights(wr.data_ptr(), wt.data_ptr(), s.Co, s.KH, s.KW, s.C, on.stream), "gcow_conv_flip_weights");
+        g_launches++;
+        if (kind == 1) {
+          check(gcow_conv_dgrad_1x1_s2(g, wt.data_ptr(), gx.data_ptr(), s.N, s.H, s.W, s.C, s.Co, on.error, on.stream), "gcow_conv_dgrad_1x1_s2");
+          g_launches++;
+        } else {
+          const ConvShape back{s.N, s.Co, s.OH, s.OW, s.C, s.KH, s.KW, s.H, s.W, s.KH - 1 - s.ph, s.KW - 1 - s.pw};
+          conv_forward(gy, wt, gx, Tensor(), back, on);
+        }
+      }
+      out[0] = std::move(gx);
+    }
+    if (wants(1)) {
+      if (kind) {
+        const int parts = gcow_conv_wgrad_split_strided(s.N, s.H, s.W, s.C, s.Co, s.KH, s.KW, s.ph, s.pw, 2);
+        out[1] = conv_wgrad(target[0], s, parts, x, on, [&](float* part) {
+          check(gcow_conv_wgrad_strided(g, x.data_ptr(), part, s.N, s.H, s.W, s.C, s.Co, s.KH, s.KW, s.ph, s.pw, 2, on.error, on.stream), "gcow_conv_wgrad_strided");
+        });
+      } else {
+        // 64 -> 64 channels, 3x3, padding 1: the halo-tile kernel, when the image rows fit its slot pitch; channel counts
+        // that are multiples of 128, 3x3, padding 1, rows of at least halo_min_w pixels: the one with a CTA group per
+        // (filter row, 128 x 128 channels); else the general one (the line is explained in ops/kernels.py)
+        const int ws = conv_ws(s) && !env_off("GCOW_CONV_WS_WGRAD") ? gcow_conv_wgrad_ws_split(s.N, s.H, s.W) : 0;
+        const int halo = s.C % 128 == 0 && s.Co % 128 == 0 && s.KH == 3 && s.KW == 3 && s.ph == 1 && s.pw == 1 && s.W >= halo_min_w &&
+                         !env_off("GCOW_CONV_HALO_WGRAD") ? gcow_conv_wgrad_halo_split(s.N, s.H, s.W, s.C, s.Co) : 0;
+        const int parts = ws > 0 ? ws : halo > 0 ? halo : gcow_conv_wgrad_split(s.N, s.H, s.W, s.C, s.Co, s.KH, s.KW, s.ph, s.pw);
+        out[1] = conv_wgrad(target[0], s, parts, x, on, [&](float* part) {
+          if (ws > 0) check(gcow_conv_wgrad_ws(g, x.data_ptr(), part, s.N, s.H, s.W, on.error, on.stream), "gcow_conv_wgrad_ws");
+          else if (halo > 0) check(gcow_conv_wgrad_halo(g, x.data_ptr(), part, s.N, s.H, s.W, s.C, s.Co, on.error, on.stream), "gcow_conv_wgrad_halo");
+          else check(gcow_conv_wgrad(g, x.data_ptr(), part, s.N, s.H, s.W, s.C, s.Co, s.KH, s.KW, s.ph, s.pw, on.error, on.stream), "gcow_conv_wgrad");
+        });
+      }
+    }
+    if (has_bias && wants(2)) out[2] = conv_bias_grad(gy, s.Co, on);
+    return out;
+  }
+};
+
+// conv(x, w, b or None, kind, pad_h, pad_w, halo_min_w): implicit-GEMM convolutions; kind as in ConvNode
+PyObject* conv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 7, "conv: bad arguments");
+  const Tensor xin = arg(args[0]), w = arg(args[1]), b = arg(args[2]);
+  int v[4];
+  for (int i = 0; i < 4; i++) v[i] = (int)PyLong_AsLong(args[3 + i]);
+  if (PyErr_Occurred()) return nullptr;
+  auto node = record<ConvNode>(xin, w, b);
+  Tensor out;
+  {
+    Below below;
+    const On on(xin);
+    const Tensor x = nhwc_bf16(xin), wr = bf16_weight(args[1]).permute({0, 2, 3, 1}).contiguous(), bias = float_vector(b);   // [Co, kh, kw, Ci]
+    ConvShape s{(int)x.size(0), (int)x.size(1), (int)x.size(2), (int)x.size(3), (int)w.size(0), (int)w.size(2), (int)w.size(3), 0, 0, v[1], v[2]};
+    s.OH = v[0] ? (s.H - 1) / 2 + 1 : s.H + 2 * s.ph - s.KH + 1;
+    s.OW = v[0] ? (s.W - 1) / 2 + 1 : s.W + 2 * s.pw - s.KW + 1;
+    out = empty_nhwc(s.N, s.Co, s.OH, s.OW, x);
+    if (v[0]) {
+      check(gcow_conv_fwd_strided(x.data_ptr(), wr.data_ptr(), out.data_ptr(), f32(bias), s.N, s.H, s.W, s.C, s.Co, s.KH, s.KW, s.ph, s.pw, 2,
+                                  on.error, on.stream), "gcow_conv_fwd_strided");
+      g_launches++;
+    } else {
+      conv_forward(x, wr, out, bias, s, on);
+    }
+    if (node) {
+      node->kept[0].set(x);
+      node->kept[1].set(wr);
+      node->s = s;
+      node->kind = v[0];
+      node->halo_min_w = v[3];
+      node->has_bias = b.defined();
+      node->target[0] = {take_grad_view(args[1]), w};
+    }
+  }
+  return finish(std::move(out), node);
+  END_HANDLE_TH_ERRORS
+}
+
+struct Conv1x1Node : LayerNode {                            // inputs: x, w, b
+  int64_t N = 0, C = 0, H = 0, W = 0, Co = 0;
+  at::ScalarType wtype = at::kFloat;
+  bool has_bias = false;
+  std::string name() const override { return "GcowConv1x1Backward"; }
+  variable_list grads(variable_list&& in) override {
+    variable_list out(3);
+    if (!in[0].defined()) return out;
+    const Tensor &xm = kept[0].get(), &wb = kept[1].get();
+    const On on(xm);
+    const Tensor g = bf16_rows(in[0].permute({0, 2, 3, 1})).view({-1, Co});
+    if (wants(0)) {
+      GemmOpts o;
+      o.b_t = true;
+      out[0] = gemm(g, wb, o, on).view({N, H, W, C}).permute({0, 3, 1, 2});
+    }
+    if (wants(1)) {
+      Tensor result;
+      const Tensor flat = target_matrix(target[0], Co, C, 16, &result);
+      if (flat.defined()) { wgrad(g, xm, flat, on); out[1] = result; }
+      else out[1] = wgrad(g, xm, Tensor(), on).view({Co, C, 1, 1}).to(wtype).contiguous(at::MemoryFormat::ChannelsLast);
+    }
+    if (has_bias && wants(2)) out[2] = colsum(g, on);
+    return out;
+  }
+};
+
+PyObject* conv1x1(PyObject*, PyObject* const* args, Py_ssize_t nargs) {        // (x, w, b or None): a GEMM over the pixels
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 3, "conv1x1: bad arguments");
+  const Tensor x = arg(args[0]), w = arg(args[1]), b = arg(args[2]);
+  auto node = record<Conv1x1Node>(x, w, b);
+  Tensor out;
+  {
+    Below below;
+    const On on(x);
+    const int64_t N = x.size(0), C = x.size(1), H = x.size(2), W = x.size(3), Co = w.size(0);
+    const Tensor xm = bf16_rows(x.permute({0, 2, 3, 1})).view({-1, C}), wb = bf16_weight(args[1]).reshape({Co, C}).contiguous();
+    GemmOpts o;
+    o.bias = float_vector(b);
+    out = empty_nhwc(N, Co, H, W, x);
+    o.out = out.permute({0, 2, 3, 1}).view({-1, Co});
+    gemm(xm, wb, o, on);
+    if (node) {
+      node->kept[0].set(xm);
+      node->kept[1].set(wb);
+      node->N = N; node->C = C; node->H = H; node->W = W; node->Co = Co;
+      node->wtype = w.scalar_type();
+      node->has_bias = b.defined();
+      node->target[0] = {take_grad_view(args[1]), w};
+    }
+  }
+  return finish(std::move(out), node);
+  END_HANDLE_TH_ERRORS
+}
+
+// ---------------------------------------------------------------------- BatchNorm (+ add) (+ ReLU)
+struct BatchNormNode : LayerNode {                          // inputs: x, gamma, beta, residual; outputs: y and, forked, y again
+  int64_t R = 0, C = 0;
+  bool relu = false, has_res = false;
+  at::ScalarType ptype = at::kFloat;
+  std::string name() const override { return "GcowBatchNormBackward"; }
+  variable_list grads(variable_list&& in) override {
+    variable_list out(4);
+    Tensor gy = in[0], gy2 = in.size() > 1 ? in[1] : Tensor();
+    if (!gy.defined()) std::swap(gy, gy2);
+    if (!gy.defined()) return out;
+    const Tensor &x = kept[0].get(), &g32 = kept[1].get(), &stats = kept[2].get();
+    const Tensor mask = relu ? kept[3].get() : Tensor();
+    const On on(x);
+    gy = nhwc_bf16(gy);
+    if (gy2.defined()) gy2 = nhwc_bf16(gy2);
+    Tensor dx = empty_nhwc(x.size(0), C, x.size(2), x.size(3), x);
+    // the masked (summed) gradient: the residual input's gradient, and what the second sweep reads
+    Tensor dres;
+    if (has_res || gy2.defined()) dres = empty_nhwc(x.size(0), C, x.size(2), x.size(3), x);
+    const Tensor part = empty({(int64_t)gcow_bn_parts(R, (int)C) * 2 * C}, at::kFloat, x);
+    // dgamma and dbeta go straight into the two parameters' gradient tensors when the trainer pointed at them
+    Tensor dgamma, dbeta, flat_g = target_matrix(target[0], 1, C, 4, &dgamma), flat_b;
+    if (flat_g.defined()) flat_b = target_matrix(target[1], 1, C, 4, &dbeta);
+    float *pg, *pb;
+    if (flat_b.defined()) {
+      pg = f32(flat_g);
+      pb = f32(flat_b);
+    } else {
+      const Tensor dgb = empty({2 * C}, at::kFloat, x);
+      pg = f32(dgb);
+      pb = pg + C;
+      dgamma = dgb.narrow(0, 0, C);
+      dbeta = dgb.narrow(0, C, C);
+    }
+    check(gcow_bn_bwd3(gy.data_ptr(), raw(gy2), raw(mask), x.data_ptr(), f32(g32), f32(stats), dx.data_ptr(), raw(dres), pg, pb, f32(part),
+                       R, (int)C, relu, on.stream), "gcow_bn_bwd3");
+    g_launches += 3;
+    out[0] = std::move(dx);
+    out[1] = flat_b.defined() ? dgamma : dgamma.to(ptype);
+    out[2] = flat_b.defined() ? dbeta : dbeta.to(ptype);
+    if (has_res) out[3] = std::move(dres);
+    return out;
+  }
+};
+
+// batchnorm_act(x, gamma, beta, run_mean or None, run_var or None, residual or None, relu, momentum, eps, fork)
+PyObject* batchnorm_act(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 10, "batchnorm_act: bad arguments");
+  const Tensor x = arg(args[0]), gamma = arg(args[1]), beta = arg(args[2]), rm = arg(args[3]), rv = arg(args[4]), res = arg(args[5]);
+  const bool relu = PyObject_IsTrue(args[6]) == 1, fork = PyObject_IsTrue(args[9]) == 1;
+  const double momentum = PyFloat_AsDouble(args[7]), eps = PyFloat_AsDouble(args[8]);
+  if (PyErr_Occurred()) return nullptr;
+  auto node = record<BatchNormNode>(x, gamma, beta, res);
+  Tensor y, y2;
+  {
+    Below below;
+    const On on(x);
+    const int64_t C = x.size(1), R = x.size(0) * x.size(2) * x.size(3);
+    y = empty_nhwc(x.size(0), C, x.size(2), x.size(3), x);
+    const Tensor stats = empty({4 * C}, at::kFloat, x), part = empty({(int64_t)gcow_bn_parts(R, (int)C) * 2 * C}, at::kFloat, x);
+    const Tensor g32 = float_vector(gamma), b32 = float_vector(beta);
+    const Tensor mask = relu ? empty({R * C / 8}, at::kByte, x) : Tensor();
+    check(gcow_bn_fwd_train(x.data_ptr(), raw(res), y.data_ptr(), raw(mask), f32(g32), f32(b32), f32(rm), f32(rv), f32(stats), f32(part), R,
+                            (int)C, (float)eps, (float)momentum, relu, on.stream), "gcow_bn_fwd_train");
+    g_launches += 3;
+    if (node) {                                             // the ReLU bit mask stands in for y in the backward
+      node->kept[0].set(x);
+      node->kept[1].set(g32);
+      node->kept[2].set(stats);
+      node->kept[3].set(mask);
+      node->R = R; node->C = C;
+      node->relu = relu;
+      node->has_res = res.defined();
+      node->ptype = gamma.scalar_type();
+      if (gamma.scalar_type() == at::kFloat) {
+        node->target[0] = {take_grad_view(args[1]), gamma};
+        node->target[1] = {take_grad_view(args[2]), beta};
+      }
+    }
+    if (fork) {                                             // a second tensor on the same storage (not an autograd view of the first)
+      y2 = empty({0}, at::kBFloat16, x);
+      y2.set_(y.storage(), y.storage_offset(), y.sizes(), y.strides());
+    }
+  }
+  if (node) torch::autograd::set_history(y, node);
+  if (!fork) return THPVariable_Wrap(std::move(y));
+  if (node) torch::autograd::set_history(y2, node);
+  PyObject *a = THPVariable_Wrap(std::move(y)), *c = THPVariable_Wrap(std::move(y2));
+  PyObject* r = PyTuple_Pack(2, a, c);
+  Py_DECREF(a);
+  Py_DECREF(c);
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// ---------------------------------------------------------------------- bookkeeping
+PyObject* launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches.load()); }
+PyObject* view_hits(PyObject*, PyObject*) { return PyLong_FromLongLong(g_view_hits.load()); }
+PyObject* py_error_word(PyObject*, PyObject* index) {       // the kernels' error word of a device
+  HANDLE_TH_ERRORS
+  const long i = PyLong_AsLong(index);
+  if (PyErr_Occurred()) return nullptr;
+  return THPVariable_Wrap(error_word((int)i));
+  END_HANDLE_TH_ERRORS
+}
+PyObject* error_words(PyObject*, PyObject*) {               // those that exist
+  HANDLE_TH_ERRORS
+  PyObject* list = PyList_New(0);
+  std::lock_guard<std::mutex> lock(g_error_mu);
+  for (const Tensor& t : g_error) {
+    if (!t.defined()) continue;
+    PyObject* o = THPVariable_Wrap(t);
+    PyList_Append(list, o);
+    Py_DECREF(o);
+  }
+  return list;
+  END_HANDLE_TH_ERRORS
+}
+
+}  // namespace
+
+Tensor error_word(int device) {
+  TORCH_CHECK(device >= 0 && device < 64, "device index out of range");
+  std::lock_guard<std::mutex> lock(g_error_mu);
+  Tensor& t = g_error[device];
+  if (!t.defined()) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    t = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::Device(at::kCUDA, (at::DeviceIndex)device)));
+  }
+  return t;
+}
+
+#define GCOW_FAST(name) {#name, (PyCFunction)(void (*)())name, METH_FASTCALL, nullptr}
+PyMethodDef layer_methods[] = {
+    GCOW_FAST(linear), GCOW_FAST(ffn_residual), GCOW_FAST(layernorm), GCOW_FAST(fused_attention), GCOW_FAST(attention),
+    GCOW_FAST(conv), GCOW_FAST(conv1x1), GCOW_FAST(batchnorm_act),
+    {"launches", launches, METH_NOARGS, nullptr},
+    {"view_hits", view_hits, METH_NOARGS, nullptr},
+    {"error_word", py_error_word, METH_O, nullptr},
+    {"error_words", error_words, METH_NOARGS, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+
+}  // namespace gcow_ext

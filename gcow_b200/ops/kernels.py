@@ -18,17 +18,31 @@ OUT_F32, BIAS, GELU, RESIDUAL, ACCUMULATE, AUX_OUT, GELU_GRAD = 1, 2, 4, 8, 16, 
 
 
 def launch_count() -> int:
-    """How many compute kernels of this library were launched through this module."""
-    return _launches
+    """How many compute kernels of this library were launched through this module and the extension module's layers."""
+    return _launches + (_native._ext.launches() if _native._ext is not None else 0)
+
+
+_known: set = set()
 
 
 def _have(name: str) -> bool:
+    """Whether the CUDA library is here and exports ``name`` (asked once per name; a missing one is asked for again)."""
+    if name in _known:
+        return True
     if not _native.cuda_available():
         return False
     try:
-        return hasattr(_native.cuda(), name)
+        if hasattr(_native.cuda(), name):
+            _known.add(name)
+            return True
     except Exception:
-        return False
+        pass
+    return False
+
+
+def _layers():
+    """The extension module's layer functions (csrc/torch/layers.cpp)."""
+    return _native._ext or _native.ext()
 
 
 _arena: dict = {}
@@ -42,7 +56,7 @@ def _ws(tag: str, shape, dtype, device) -> torch.Tensor:
     n = 1
     for d in (shape if isinstance(shape, (tuple, list)) else (shape,)):
         n *= int(d)
-    key = (tag, dtype, device, torch.cuda.current_stream(device).cuda_stream)
+    key = (tag, dtype, device, _stream(device))
     buf = _arena.get(key)
     if buf is None or buf.numel() < n:
         buf = torch.empty(max(n, 1), dtype=dtype, device=device)
@@ -58,7 +72,7 @@ def workspace_bytes() -> int:
 def _error_word(device: torch.device) -> torch.Tensor:
     w = _err_words.get(device)
     if w is None:
-        w = torch.zeros(1, dtype=torch.int32, device=device)
+        w = _layers().error_word(device.index if device.index is not None else torch.cuda.current_device())
         _err_words[device] = w
     return w
 
@@ -72,7 +86,8 @@ def check_errors(device: torch.device | None = None, raise_on_error: bool = True
     """Read the error word of the compute kernels (synchronises). Raises KernelWaitAbandoned if a kernel gave up on
     an internal wait, or returns the code when ``raise_on_error`` is false. The word is cleared."""
     worst = 0
-    for dev, w in _err_words.items():
+    for w in _layers().error_words():
+        dev = w.device
         if device is not None and dev != device:
             continue
         code = int(w.item())
@@ -150,7 +165,7 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, bias: torch.Tensor | None = N
             a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
             bias.data_ptr() if bias is not None else None, residual.data_ptr() if residual is not None else None,
             aux.data_ptr() if aux is not None else None, flags, _error_word(a.device).data_ptr(), int(b_t),
-            torch.cuda.current_stream(a.device).cuda_stream)
+            _stream(a.device))
         if err == 0:
             _launches += 1
             return out
@@ -163,13 +178,13 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, bias: torch.Tensor | None = N
             a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
             bias.data_ptr() if bias is not None else None, residual.data_ptr() if residual is not None else None,
             aux.data_ptr(), flags, _error_word(a.device).data_ptr(), int(a_t), int(b_t), int(tile_rows),
-            torch.cuda.current_stream(a.device).cuda_stream)
+            _stream(a.device))
     else:
         err = _native.cuda().gcow_gemm_bf16(
             a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
             bias.data_ptr() if bias is not None else None, residual.data_ptr() if residual is not None else None,
             flags, _error_word(a.device).data_ptr(), max_ctas, int(a_t), int(b_t), int(tile_rows),
-            torch.cuda.current_stream(a.device).cuda_stream)
+            _stream(a.device))
     if err:
         raise RuntimeError(f"gcow_gemm_bf16 refused the call: {err}")
     _launches += 1
@@ -229,7 +244,7 @@ _grad_view_hits = 0
 
 def grad_view_hits() -> int:
     """How many weight gradients were written straight into the tensor the trainer pointed at (see take_grad_view)."""
-    return _grad_view_hits
+    return _grad_view_hits + (_native._ext.view_hits() if _native._ext is not None else 0)
 
 
 def wgrad_gemm(g: torch.Tensor, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -259,10 +274,6 @@ def wgrad_gemm(g: torch.Tensor, x: torch.Tensor, out: torch.Tensor | None = None
     return out
 
 
-def _gemm_ok(x2d: torch.Tensor, w: torch.Tensor) -> bool:
-    return x2d.is_cuda and x2d.shape[1] % 8 == 0 and w.shape[1] % 8 == 0 and x2d.shape[0] >= 64
-
-
 def _pad_rows(t: torch.Tensor, rows: int) -> torch.Tensor:
     if t.shape[0] == rows:
         return t
@@ -271,11 +282,10 @@ def _pad_rows(t: torch.Tensor, rows: int) -> torch.Tensor:
     return out
 
 
-class _LinearFn(torch.autograd.Function):
-    """y = x W^T + b with all three GEMMs (forward, dgrad, wgrad) on the tcgen05 kernel.
-    An output width that is not a multiple of 8 (e.g. a 30522-word vocabulary) is
-    padded internally: the result is a [.., N] view of a [M, N8] buffer whose pad
-    columns are zero-weighted."""
+class _PaddedLinearFn(torch.autograd.Function):
+    """y = x W^T + b for an output width that is not a multiple of 8 (e.g. a 30522-word vocabulary), padded internally:
+    the result is a [.., N] view of a [M, N8] buffer whose pad columns are zero-weighted. All three GEMMs (forward,
+    dgrad, wgrad) run on the tcgen05 kernel; the other widths are ``linear`` of the extension module."""
 
     @staticmethod
     def forward(ctx, x, w, b):
@@ -287,113 +297,31 @@ class _LinearFn(torch.autograd.Function):
         y = gemm_bf16(xb, wb, bias=bias)
         ctx.save_for_backward(xb, wb)
         ctx.meta = (x.shape, w.dtype, b is not None, N, N8)
-        ctx.grad_view = take_grad_view(w) if (N == N8 and w.dtype == torch.float32) else None
-        return y[:, :N].view(*x.shape[:-1], N) if N == N8 else y[:, :N].unflatten(0, x.shape[:-1])
+        return y[:, :N].unflatten(0, x.shape[:-1])
 
     @staticmethod
     def backward(ctx, gy):
         xb, wb = ctx.saved_tensors
         x_shape, w_dtype, has_bias, N, N8 = ctx.meta
         M = xb.shape[0]
-        g = gy.reshape(M, N) if gy.is_contiguous() or N == N8 else gy.flatten(0, -2)
+        g = gy.reshape(M, N) if gy.is_contiguous() else gy.flatten(0, -2)
         if (g.dtype == torch.bfloat16 and g.stride(1) == 1 and g.stride(0) == N8 and g.storage_offset() == 0
                 and g.untyped_storage().nbytes() >= M * N8 * 2):
             g = g.as_strided((M, N8), (N8, 1))          # the padded buffer itself (pad columns are zero)
         else:
-            g = g.to(torch.bfloat16)
-            if N != N8:
-                gp = torch.zeros((M, N8), dtype=torch.bfloat16, device=g.device)
-                gp[:, :N] = g
-                g = gp
-            else:
-                g = g.contiguous()
+            gp = torch.zeros((M, N8), dtype=torch.bfloat16, device=g.device)
+            gp[:, :N] = g
+            g = gp
         gx = gw = gb = None
         if ctx.needs_input_grad[0]:
             # dx[M,K] = g[M,N] @ W[N,K]: W is stored [reduction N][K], i.e. the B operand transposed
             gx = gemm_bf16(g, wb, b_t=True).view(x_shape)
         if ctx.needs_input_grad[1]:
             # dW[N,K] = g^T @ x: both g [M,N] and x [M,K] are stored [reduction M][rows]
-            flat, alias = _grad_target(ctx.grad_view, N, xb.shape[1])
-            if flat is not None:
-                wgrad_gemm(g, xb, out=flat)
-                gw = alias
-            else:
-                gw = wgrad_gemm(g, xb)[:N].to(w_dtype)
+            gw = wgrad_gemm(g, xb)[:N].to(w_dtype)
         if has_bias and ctx.needs_input_grad[2]:
             gb = colsum(g)[:N]
         return gx, gw, gb
-
-
-class _LinearResidualFn(torch.autograd.Function):
-    """y = r + x W^T + b with the residual added in the GEMM epilogue."""
-
-    @staticmethod
-    def forward(ctx, x, w, b, r):
-        xb = x.reshape(-1, x.shape[-1]).to(torch.bfloat16).contiguous()
-        wb = bf16_weight(w).contiguous()
-        rb = r.reshape(-1, r.shape[-1]).to(torch.bfloat16).contiguous()
-        y = gemm_bf16(xb, wb, bias=b.float().contiguous() if b is not None else None, residual=rb)
-        ctx.save_for_backward(xb, wb)
-        ctx.meta = (x.shape, r.shape, b is not None)
-        ctx.grad_view = take_grad_view(w)
-        return y.view(r.shape)
-
-    @staticmethod
-    def backward(ctx, gy):
-        xb, wb = ctx.saved_tensors
-        x_shape, r_shape, has_bias = ctx.meta
-        g = gy.reshape(-1, gy.shape[-1]).to(torch.bfloat16).contiguous()
-        gx = gw = gb = None
-        if ctx.needs_input_grad[0]:
-            gx = gemm_bf16(g, wb, b_t=True).view(x_shape)
-        if ctx.needs_input_grad[1]:
-            flat, alias = _grad_target(ctx.grad_view, wb.shape[0], wb.shape[1])
-            gw = wgrad_gemm(g, xb, out=flat)
-            if flat is not None:
-                gw = alias
-        if has_bias and ctx.needs_input_grad[2]:
-            gb = colsum(g)
-        return gx, gw, gb, (gy if ctx.needs_input_grad[3] else None)
-
-
-class _FfnResidualFn(torch.autograd.Function):
-    """y = x + GELU(x W1^T + b1) W2^T + b2 as two GEMMs forward and four backward, with every elementwise
-    step in a GEMM epilogue: bias + GELU (keeping the pre-activation), bias + residual, GELU' on the way
-    back, and the sum of the two gradient paths into x."""
-
-    @staticmethod
-    def forward(ctx, x, w1, b1, w2, b2):
-        xb = x.reshape(-1, x.shape[-1]).to(torch.bfloat16).contiguous()
-        w1b, w2b = bf16_weight(w1).contiguous(), bf16_weight(w2).contiguous()
-        M, F = xb.shape[0], w1b.shape[0]
-        pre = torch.empty((M, F), dtype=torch.bfloat16, device=xb.device)
-        act = gemm_bf16(xb, w1b, bias=b1.float().contiguous(), gelu=True, pre_gelu_out=pre)
-        y = gemm_bf16(act, w2b, bias=b2.float().contiguous(), residual=xb)
-        ctx.save_for_backward(xb, w1b, w2b, pre, act)
-        ctx.shape = x.shape
-        ctx.grad_views = (take_grad_view(w1), take_grad_view(w2))
-        return y.view(x.shape)
-
-    @staticmethod
-    def backward(ctx, gy):
-        xb, w1b, w2b, pre, act = ctx.saved_tensors
-        g = gy.reshape(-1, gy.shape[-1]).to(torch.bfloat16).contiguous()
-        dpre = gemm_bf16(g, w2b, b_t=True, gelu_grad_of=pre)                 # (g W2) * GELU'(pre)
-        gw1 = gw2 = None
-        if ctx.needs_input_grad[3]:
-            flat, alias = _grad_target(ctx.grad_views[1], w2b.shape[0], w2b.shape[1])
-            gw2 = wgrad_gemm(g, act, out=flat)
-            if flat is not None:
-                gw2 = alias
-        gb2 = colsum(g) if ctx.needs_input_grad[4] else None
-        gx = gemm_bf16(dpre, w1b, b_t=True, residual=g).view(ctx.shape) if ctx.needs_input_grad[0] else None
-        if ctx.needs_input_grad[1]:
-            flat, alias = _grad_target(ctx.grad_views[0], w1b.shape[0], w1b.shape[1])
-            gw1 = wgrad_gemm(dpre, xb, out=flat)
-            if flat is not None:
-                gw1 = alias
-        gb1 = colsum(dpre) if ctx.needs_input_grad[2] else None
-        return gx, gw1, gb1, gw2, gb2
 
 
 def fused_mlp_usable(x: torch.Tensor, *weights: torch.Tensor) -> bool:
@@ -404,26 +332,33 @@ def fused_mlp_usable(x: torch.Tensor, *weights: torch.Tensor) -> bool:
 
 
 def linear_residual(x, w, b, r):
-    return _LinearResidualFn.apply(x, w, b, r)
+    """r + x W^T + b with the residual added in the GEMM epilogue."""
+    return _layers().linear(x, w, b, r)
 
 
 def ffn_residual(x, w1, b1, w2, b2):
-    return _FfnResidualFn.apply(x, w1, b1, w2, b2)
+    """x + GELU(x W1^T + b1) W2^T + b2 as two GEMMs forward and four backward, with every elementwise step in a GEMM
+    epilogue: bias + GELU (keeping the pre-activation), bias + residual, GELU' on the way back, and the sum of the two
+    gradient paths into x."""
+    return _layers().ffn_residual(x, w1, b1, w2, b2)
 
 
 def gemm_usable(x: torch.Tensor, w: torch.Tensor) -> bool:
     if not (x.is_cuda and _have("gcow_gemm_bf16")):
         return False
-    x2 = x.reshape(-1, x.shape[-1])
-    return _gemm_ok(x2, w)
+    k = x.shape[-1]
+    return k % 8 == 0 and w.shape[1] % 8 == 0 and x.numel() >= 64 * k
 
 
 def linear(x, w, b):
-    return _LinearFn.apply(x, w, b)
+    """y = x W^T + b with all three GEMMs (forward, dgrad, wgrad) on the tcgen05 kernel."""
+    if w.shape[0] % 8 == 0:
+        return _layers().linear(x, w, b, None)
+    return _PaddedLinearFn.apply(x, w, b)
 
 
 def _stream(dev):
-    return torch.cuda.current_stream(dev).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(dev.index if dev.index is not None else torch.cuda.current_device())
 
 
 def _chk(err: int, what: str) -> None:
@@ -448,46 +383,6 @@ def colsum(g: torch.Tensor) -> torch.Tensor:
 
 
 # ------------------------------------------------------------------ 1x1 conv
-class _Conv1x1Fn(torch.autograd.Function):
-    """1x1 stride-1 convolution on channels-last activations as a GEMM:
-    [N*H*W, Cin] x [Cout, Cin]^T."""
-
-    @staticmethod
-    def forward(ctx, x, w, b):
-        N, C, H, W = x.shape
-        xm = x.permute(0, 2, 3, 1).reshape(-1, C)          # a view for channels-last input
-        if xm.dtype != torch.bfloat16 or not xm.is_contiguous():
-            xm = xm.to(torch.bfloat16).contiguous()
-        wb = bf16_weight(w).reshape(w.shape[0], C).contiguous()
-        y = gemm_bf16(xm, wb, bias=b.float().contiguous() if b is not None else None)
-        ctx.save_for_backward(xm, wb)
-        ctx.meta = (N, C, H, W, w.shape, w.dtype, b is not None)
-        ctx.grad_view = take_grad_view(w) if w.dtype == torch.float32 else None
-        return y.view(N, H, W, w.shape[0]).permute(0, 3, 1, 2)
-
-    @staticmethod
-    def backward(ctx, gy):
-        xm, wb = ctx.saved_tensors
-        N, C, H, W, wshape, wdtype, has_bias = ctx.meta
-        g = gy.permute(0, 2, 3, 1).reshape(-1, wshape[0])
-        if g.dtype != torch.bfloat16 or not g.is_contiguous():
-            g = g.to(torch.bfloat16).contiguous()
-        gx = gw = gb = None
-        if ctx.needs_input_grad[0]:
-            gx = gemm_bf16(g, wb, b_t=True).view(N, H, W, C).permute(0, 3, 1, 2)
-        if ctx.needs_input_grad[1]:
-            flat, alias = _grad_target(ctx.grad_view, wshape[0], C)
-            if flat is not None:
-                wgrad_gemm(g, xm, out=flat)
-                gw = alias
-            else:
-                gw = wgrad_gemm(g, xm)
-                gw = gw.view(wshape).to(wdtype).contiguous(memory_format=torch.channels_last)
-        if has_bias and ctx.needs_input_grad[2]:
-            gb = colsum(g)
-        return gx, gw, gb
-
-
 class _SubsampleFn(torch.autograd.Function):
     """x[:, :, ::s, ::s] of a channels-last bf16 tensor as a dense channels-last tensor (what a strided 1x1 convolution
     reads); the backward writes the gradient at the sampled pixels and zeros elsewhere in one kernel."""
@@ -532,47 +427,11 @@ def conv1x1_usable(x: torch.Tensor, w: torch.Tensor) -> bool:
 
 
 def conv1x1(x, w, b):
-    return _Conv1x1Fn.apply(x, w, b)
+    """1x1 stride-1 convolution on channels-last activations as a GEMM: [N*H*W, Cin] x [Cout, Cin]^T."""
+    return _layers().conv1x1(x, w, b)
 
 
 # ----------------------------------------------------------------- LayerNorm
-class _LayerNormFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, gamma, beta, eps):
-        global _launches
-        H = x.shape[-1]
-        xb = x.reshape(-1, H).to(torch.bfloat16).contiguous()
-        rows = xb.shape[0]
-        y = torch.empty_like(xb)
-        mean = torch.empty(rows, dtype=torch.float32, device=x.device)
-        rstd = torch.empty_like(mean)
-        g32, b32 = gamma.float().contiguous(), beta.float().contiguous()
-        _chk(_native.cuda().gcow_layernorm_fwd(xb.data_ptr(), g32.data_ptr(), b32.data_ptr(), y.data_ptr(),
-                                               mean.data_ptr(), rstd.data_ptr(), rows, H, eps, _stream(x.device)),
-             "gcow_layernorm_fwd")
-        _launches += 1
-        ctx.save_for_backward(xb, g32, mean, rstd)
-        ctx.shape, ctx.pdtype = x.shape, gamma.dtype
-        return y.view(x.shape)
-
-    @staticmethod
-    def backward(ctx, gy):
-        global _launches
-        xb, g32, mean, rstd = ctx.saved_tensors
-        rows, H = xb.shape
-        g = gy.reshape(rows, H).to(torch.bfloat16).contiguous()
-        lib = _native.cuda()
-        dx = torch.empty_like(xb)
-        parts = lib.gcow_layernorm_bwd_parts(rows)
-        part = _ws("ln_part", parts * 2 * H, torch.float32, xb.device)
-        dgb = torch.empty(2 * H, dtype=torch.float32, device=xb.device)
-        _chk(lib.gcow_layernorm_bwd(g.data_ptr(), xb.data_ptr(), g32.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
-                                    dx.data_ptr(), part.data_ptr(), dgb.data_ptr(), rows, H, _stream(xb.device)),
-             "gcow_layernorm_bwd")
-        _launches += 2
-        return dx.view(ctx.shape), dgb[:H].to(ctx.pdtype), dgb[H:].to(ctx.pdtype), None
-
-
 def layernorm_usable(x: torch.Tensor, mod) -> bool:
     H = x.shape[-1]
     return x.is_cuda and _have("gcow_layernorm_fwd") and H % 8 == 0 and H <= 4096 and \
@@ -580,7 +439,7 @@ def layernorm_usable(x: torch.Tensor, mod) -> bool:
 
 
 def layernorm(x, w, b, eps):
-    return _LayerNormFn.apply(x, w, b, eps)
+    return _layers().layernorm(x, w, b, eps)
 
 
 # ---------------------------------------------------------------------- GELU
@@ -684,78 +543,6 @@ def _nhwc_rows(x: torch.Tensor):
     return N * H * W, C
 
 
-class _BatchNormActFn(torch.autograd.Function):
-    """y = relu?(bn(x) (+ residual)) on channels-last bf16 tensors, training statistics.
-
-    With ``fork`` the result is returned twice, as two tensors on the same memory: a layer output that feeds two
-    consumers (the next block's first convolution and its identity branch) then gets its two gradients delivered
-    separately, and the first backward sweep adds them while it reads them - instead of autograd's addition kernel
-    (two reads and a write of the whole tensor) followed by a third read here."""
-
-    @staticmethod
-    def forward(ctx, x, gamma, beta, run_mean, run_var, residual, relu, momentum, eps, fork=False):
-        global _launches
-        R, C = _nhwc_rows(x)
-        lib = _native.cuda()
-        y = torch.empty_like(x, memory_format=torch.channels_last)
-        stats = torch.empty(4 * C, dtype=torch.float32, device=x.device)
-        part = _ws("bn_part", lib.gcow_bn_parts(R, C) * 2 * C, torch.float32, x.device)
-        g32, b32 = gamma.float().contiguous(), beta.float().contiguous()
-        mask = torch.empty(R * C // 8, dtype=torch.uint8, device=x.device) if relu else None
-        _chk(lib.gcow_bn_fwd_train(x.data_ptr(), residual.data_ptr() if residual is not None else None, y.data_ptr(),
-                                   mask.data_ptr() if mask is not None else None, g32.data_ptr(), b32.data_ptr(),
-                                   run_mean.data_ptr() if run_mean is not None else None,
-                                   run_var.data_ptr() if run_var is not None else None,
-                                   stats.data_ptr(), part.data_ptr(), R, C, eps, momentum, int(relu), _stream(x.device)),
-             "gcow_bn_fwd_train")
-        _launches += 3
-        ctx.save_for_backward(x, mask, g32, stats)      # the ReLU bit mask stands in for y in the backward
-        ctx.grad_views = (take_grad_view(gamma), take_grad_view(beta)) if gamma.dtype == torch.float32 else (None, None)
-        ctx.meta = (R, C, bool(relu), residual is not None, gamma.dtype)
-        if not fork:
-            return y
-        # a second tensor on the same storage (not an autograd view of the first)
-        y2 = torch.empty(0, dtype=y.dtype, device=y.device).set_(y.untyped_storage(), y.storage_offset(), y.size(), y.stride())
-        return y, y2
-
-    @staticmethod
-    def backward(ctx, gy, gy2=None):
-        global _launches
-        x, mask, g32, stats = ctx.saved_tensors
-        R, C, relu, has_res, pdtype = ctx.meta
-        lib = _native.cuda()
-        if gy is None:
-            gy, gy2 = gy2, None
-
-        def _cl(t):
-            if t.dtype != torch.bfloat16 or not t.is_contiguous(memory_format=torch.channels_last):
-                t = t.to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
-            return t
-        gy = _cl(gy)
-        gy2 = _cl(gy2) if gy2 is not None else None
-        dx = torch.empty_like(x, memory_format=torch.channels_last)
-        # the masked (summed) gradient: the residual input's gradient, and what the second sweep reads
-        dres = torch.empty_like(x, memory_format=torch.channels_last) if (has_res or gy2 is not None) else None
-        part = _ws("bn_part", lib.gcow_bn_parts(R, C) * 2 * C, torch.float32, x.device)
-        # dgamma and dbeta go straight into the two parameters' gradient tensors when the trainer pointed at them
-        fg, ag = _grad_target(ctx.grad_views[0], 1, C, align=4)
-        fb, ab = _grad_target(ctx.grad_views[1], 1, C, align=4) if fg is not None else (None, None)
-        if fb is not None and _have("gcow_bn_bwd3"):
-            dgamma, dbeta = ag, ab
-            pg, pb = fg.data_ptr(), fb.data_ptr()
-        else:
-            dgb = torch.empty(2 * C, dtype=torch.float32, device=x.device)
-            dgamma, dbeta = dgb[:C].to(pdtype), dgb[C:].to(pdtype)
-            pg, pb = dgb.data_ptr(), dgb.data_ptr() + 4 * C
-        _chk(lib.gcow_bn_bwd3(gy.data_ptr(), gy2.data_ptr() if gy2 is not None else None,
-                              mask.data_ptr() if mask is not None else None, x.data_ptr(), g32.data_ptr(),
-                              stats.data_ptr(), dx.data_ptr(),
-                              dres.data_ptr() if dres is not None else None, pg, pb, part.data_ptr(), R, C,
-                              int(relu), _stream(x.device)), "gcow_bn_bwd3")
-        _launches += 3
-        return dx, dgamma, dbeta, None, None, (dres if has_res else None), None, None, None, None
-
-
 def batchnorm_usable(x: torch.Tensor, mod, residual=None) -> bool:
     if not (x.is_cuda and x.dim() == 4 and x.dtype == torch.bfloat16 and _have("gcow_bn_fwd_train")):
         return False
@@ -768,8 +555,12 @@ def batchnorm_usable(x: torch.Tensor, mod, residual=None) -> bool:
 
 
 def batchnorm_act(x, mod, residual=None, relu=False, fork=False):
-    """Fused BN(+add)(+ReLU) using ``mod``'s parameters and running statistics. ``fork``: return the result as two
-    tensors on the same memory (see _BatchNormActFn)."""
+    """Fused BN(+add)(+ReLU) on channels-last bf16 tensors using ``mod``'s parameters and running statistics.
+
+    With ``fork`` the result is returned twice, as two tensors on the same memory: a layer output that feeds two
+    consumers (the next block's first convolution and its identity branch) then gets its two gradients delivered
+    separately, and the first backward sweep adds them while it reads them - instead of autograd's addition kernel
+    (two reads and a write of the whole tensor) followed by a third read here."""
     global _launches
     if mod.training or not mod.track_running_stats:
         if mod.training and mod.track_running_stats and mod.num_batches_tracked is not None:
@@ -779,7 +570,7 @@ def batchnorm_act(x, mod, residual=None, relu=False, fork=False):
         mom = mod.momentum if mod.momentum is not None else 0.1
         rm = mod.running_mean if (mod.training and mod.track_running_stats) else None
         rv = mod.running_var if (mod.training and mod.track_running_stats) else None
-        return _BatchNormActFn.apply(x, mod.weight, mod.bias, rm, rv, residual, relu, mom, mod.eps, fork)
+        return _layers().batchnorm_act(x, mod.weight, mod.bias, rm, rv, residual, relu, mom, mod.eps, fork)
     R, C = _nhwc_rows(x)
     y = torch.empty_like(x, memory_format=torch.channels_last)
     scratch = torch.empty(2 * C, dtype=torch.float32, device=x.device)
@@ -989,7 +780,10 @@ def conv_ws_usable(N, H, W, C, Co, KH, KW, pad_h, pad_w):
             and bool(_native.cuda().gcow_conv_ws_usable(N, H, W)))
 
 
-_HALO_WGRAD_MIN_W = 15      # narrowest image rows the halo-tile weight gradient is routed for
+# Narrowest image rows the halo-tile weight gradient of layers with multiples of 128 channels is routed for. Measured at
+# batch 256: 128 channels at 28 x 28 wins (layer 0.221 -> 0.189 ms), 256 channels at 14 x 14 ties with the general kernel,
+# 512 channels at 7 x 7 loses (slots of pitch 16 for rows of 7, 48 groups re-reading the tiles).
+_HALO_WGRAD_MIN_W = 15
 
 
 def conv_halo_usable(N, H, W, C, Co, KH, KW, pad_h, pad_w):
@@ -999,163 +793,6 @@ def conv_halo_usable(N, H, W, C, Co, KH, KW, pad_h, pad_w):
             and bool(_native.cuda().gcow_conv_halo_usable(N, H, W, C)))
 
 
-def _conv_fwd_s1(lib, x_ptr, w_ptr, y_ptr, bias_ptr, N, H, W, C, Co, KH, KW, pad_h, pad_w, err, st, what):
-    """Stride-1 forward kernel for these extents: the weight-stationary or halo-tile one where it applies, else the
-    general one."""
-    if conv_ws_usable(N, H, W, C, Co, KH, KW, pad_h, pad_w):
-        _chk(lib.gcow_conv_fwd_ws(x_ptr, w_ptr, y_ptr, bias_ptr, N, H, W, err, st), what + " (ws)")
-    elif conv_halo_usable(N, H, W, C, Co, KH, KW, pad_h, pad_w):
-        _chk(lib.gcow_conv_fwd_halo(x_ptr, w_ptr, y_ptr, bias_ptr, N, H, W, C, err, st), what + " (halo)")
-    else:
-        _chk(lib.gcow_conv_fwd(x_ptr, w_ptr, y_ptr, bias_ptr, N, H, W, C, Co, KH, KW, pad_h, pad_w, err, st), what)
-
-
-class _ConvIgemmFn(torch.autograd.Function):
-    """Stride-1 KxK convolution, channels-last bf16, as an implicit GEMM on the tcgen05 kernel
-    (csrc/ops/conv_tcgen05.cu): forward, data gradient (the same kernel on dY with the flipped
-    filter) and weight gradient (split over pixel ranges + ordered sum). No patch matrix."""
-
-    @staticmethod
-    def forward(ctx, x, w, b, pad_h, pad_w):
-        global _launches
-        N, C, H, W = x.shape
-        Co, _, KH, KW = w.shape
-        lib = _native.cuda()
-        if x.dtype != torch.bfloat16 or not x.is_contiguous(memory_format=torch.channels_last):
-            x = x.to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
-        wr = bf16_weight(w).permute(0, 2, 3, 1).contiguous()                                       # [Co, kh, kw, Ci]
-        OH, OW = H + 2 * pad_h - KH + 1, W + 2 * pad_w - KW + 1
-        y = torch.empty((N, Co, OH, OW), dtype=torch.bfloat16, device=x.device, memory_format=torch.channels_last)
-        bias = b.detach().float().contiguous() if b is not None else None
-        _conv_fwd_s1(lib, x.data_ptr(), wr.data_ptr(), y.data_ptr(), bias.data_ptr() if bias is not None else None,
-                     N, H, W, C, Co, KH, KW, pad_h, pad_w, _error_word(x.device).data_ptr(), _stream(x.device),
-                     "gcow_conv_fwd")
-        _launches += 1
-        ctx.save_for_backward(x, wr)
-        ctx.meta = (N, C, H, W, Co, KH, KW, OH, OW, pad_h, pad_w, b is not None)
-        ctx.grad_view = take_grad_view(w)
-        return y
-
-    @staticmethod
-    def backward(ctx, gy):
-        global _launches
-        x, wr = ctx.saved_tensors
-        N, C, H, W, Co, KH, KW, OH, OW, pad_h, pad_w, has_bias = ctx.meta
-        lib = _native.cuda()
-        if gy.dtype != torch.bfloat16 or not gy.is_contiguous(memory_format=torch.channels_last):
-            gy = gy.to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
-        dev, st, err = gy.device, _stream(gy.device), _error_word(gy.device).data_ptr()
-        gx = gw = gb = None
-        if ctx.needs_input_grad[0]:
-            wt = torch.empty((C, KH, KW, Co), dtype=torch.bfloat16, device=dev)
-            _chk(lib.gcow_conv_flip_weights(wr.data_ptr(), wt.data_ptr(), Co, KH, KW, C, st), "gcow_conv_flip_weights")
-            gx = torch.empty((N, C, H, W), dtype=torch.bfloat16, device=dev, memory_format=torch.channels_last)
-            _conv_fwd_s1(lib, gy.data_ptr(), wt.data_ptr(), gx.data_ptr(), None, N, OH, OW, Co, C, KH, KW,
-                         KH - 1 - pad_h, KW - 1 - pad_w, err, st, "gcow_conv_fwd (dgrad)")
-            _launches += 2
-        if ctx.needs_input_grad[1]:
-            # 64 -> 64 channels, 3x3, padding 1: the halo-tile kernel, when the image rows fit its slot pitch
-            ws_split = (lib.gcow_conv_wgrad_ws_split(N, H, W) if conv_ws_usable(N, H, W, C, Co, KH, KW, pad_h, pad_w)
-                        and os.environ.get("GCOW_CONV_WS_WGRAD", "1") != "0" and _have("gcow_conv_wgrad_ws") else 0)
-            # channel counts that are multiples of 128, 3x3, padding 1, rows of at least 15 pixels: the halo-tile kernel
-            # with one CTA group per (filter row, 128 x 128 channels). Measured at batch 256: 128 channels at 28 x 28 wins
-            # (layer 0.221 -> 0.189 ms), 256 channels at 14 x 14 ties with the general kernel, 512 channels at 7 x 7
-            # loses (slots of pitch 16 for rows of 7, 48 groups re-reading the tiles)
-            halo_split = (lib.gcow_conv_wgrad_halo_split(N, H, W, C, Co) if C % 128 == 0 and Co % 128 == 0 and KH == 3
-                          and KW == 3 and pad_h == 1 and pad_w == 1 and W >= _HALO_WGRAD_MIN_W
-                          and os.environ.get("GCOW_CONV_HALO_WGRAD", "1") != "0" and _have("gcow_conv_wgrad_halo") else 0)
-            split = (ws_split if ws_split > 0 else halo_split if halo_split > 0 else
-                     lib.gcow_conv_wgrad_split(N, H, W, C, Co, KH, KW, pad_h, pad_w))
-            flat, alias = _grad_target(ctx.grad_view, Co, KH * KW * C)
-            # the partial sums are scratch when an ordered sum follows; a single part IS the result
-            part = (_ws("conv_wgrad_part", (split, Co, KH * KW * C), torch.float32, dev) if split > 1 else
-                    (flat.unsqueeze(0) if flat is not None else torch.empty((1, Co, KH * KW * C), dtype=torch.float32, device=dev)))
-            if ws_split > 0:
-                _chk(lib.gcow_conv_wgrad_ws(gy.data_ptr(), x.data_ptr(), part.data_ptr(), N, H, W, err, st), "gcow_conv_wgrad_ws")
-            elif halo_split > 0:
-                _chk(lib.gcow_conv_wgrad_halo(gy.data_ptr(), x.data_ptr(), part.data_ptr(), N, H, W, C, Co, err, st),
-                     "gcow_conv_wgrad_halo")
-            else:
-                _chk(lib.gcow_conv_wgrad(gy.data_ptr(), x.data_ptr(), part.data_ptr(), N, H, W, C, Co, KH, KW, pad_h, pad_w,
-                                         err, st), "gcow_conv_wgrad")
-            _launches += 1
-            if split > 1:
-                out = flat if flat is not None else torch.empty((Co, KH * KW * C), dtype=torch.float32, device=dev)
-                _chk(lib.gcow_reduce_partials(part.data_ptr(), out.data_ptr(), split, out.numel(), st), "gcow_reduce_partials")
-                _launches += 1
-            else:
-                out = part[0]
-            # logical [Co, Ci, kh, kw], channels-last memory
-            gw = alias if flat is not None else out.view(Co, KH, KW, C).permute(0, 3, 1, 2)
-        if has_bias and ctx.needs_input_grad[2]:
-            gb = colsum(gy.permute(0, 2, 3, 1).reshape(-1, Co))
-        return gx, gw, gb, None, None
-
-
-class _Conv1x1Stride2Fn(torch.autograd.Function):
-    """1x1 convolution with stride 2 (the down-sampling shortcut of a ResNet stage) on the implicit-GEMM kernel with
-    one tap: forward and weight gradient read every second pixel through a tensor map with element strides, the input
-    gradient is one launch that stores to the sampled pixels of a zero-filled tensor. No subsampled copy of the input
-    and no scatter pass."""
-
-    @staticmethod
-    def forward(ctx, x, w, b):
-        global _launches
-        N, C, H, W = x.shape
-        Co = w.shape[0]
-        lib = _native.cuda()
-        if x.dtype != torch.bfloat16 or not x.is_contiguous(memory_format=torch.channels_last):
-            x = x.to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
-        wr = bf16_weight(w).reshape(Co, C).contiguous()                                             # [Co, Ci]
-        OH, OW = (H - 1) // 2 + 1, (W - 1) // 2 + 1
-        y = torch.empty((N, Co, OH, OW), dtype=torch.bfloat16, device=x.device, memory_format=torch.channels_last)
-        bias = b.detach().float().contiguous() if b is not None else None
-        _chk(lib.gcow_conv_fwd_strided(x.data_ptr(), wr.data_ptr(), y.data_ptr(), bias.data_ptr() if bias is not None else None,
-                                       N, H, W, C, Co, 1, 1, 0, 0, 2, _error_word(x.device).data_ptr(), _stream(x.device)),
-             "gcow_conv_fwd_strided")
-        _launches += 1
-        ctx.save_for_backward(x, wr)
-        ctx.meta = (N, C, H, W, Co, b is not None)
-        ctx.grad_view = take_grad_view(w)
-        return y
-
-    @staticmethod
-    def backward(ctx, gy):
-        global _launches
-        x, wr = ctx.saved_tensors
-        N, C, H, W, Co, has_bias = ctx.meta
-        lib = _native.cuda()
-        if gy.dtype != torch.bfloat16 or not gy.is_contiguous(memory_format=torch.channels_last):
-            gy = gy.to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
-        dev, st, err = gy.device, _stream(gy.device), _error_word(gy.device).data_ptr()
-        gx = gw = gb = None
-        if ctx.needs_input_grad[0]:
-            wt = torch.empty((C, Co), dtype=torch.bfloat16, device=dev)
-            _chk(lib.gcow_conv_flip_weights(wr.data_ptr(), wt.data_ptr(), Co, 1, 1, C, st), "gcow_conv_flip_weights")
-            gx = torch.empty((N, C, H, W), dtype=torch.bfloat16, device=dev, memory_format=torch.channels_last)
-            _chk(lib.gcow_conv_dgrad_1x1_s2(gy.data_ptr(), wt.data_ptr(), gx.data_ptr(), N, H, W, C, Co, err, st),
-                 "gcow_conv_dgrad_1x1_s2")
-            _launches += 2
-        if ctx.needs_input_grad[1]:
-            split = lib.gcow_conv_wgrad_split_strided(N, H, W, C, Co, 1, 1, 0, 0, 2)
-            flat, alias = _grad_target(ctx.grad_view, Co, C)
-            part = (_ws("conv_wgrad_part", (split, Co, C), torch.float32, dev) if split > 1 else
-                    (flat.unsqueeze(0) if flat is not None else torch.empty((1, Co, C), dtype=torch.float32, device=dev)))
-            _chk(lib.gcow_conv_wgrad_strided(gy.data_ptr(), x.data_ptr(), part.data_ptr(), N, H, W, C, Co, 1, 1, 0, 0, 2,
-                                             err, st), "gcow_conv_wgrad_strided")
-            _launches += 1
-            if split > 1:
-                out = flat if flat is not None else torch.empty((Co, C), dtype=torch.float32, device=dev)
-                _chk(lib.gcow_reduce_partials(part.data_ptr(), out.data_ptr(), split, out.numel(), st), "gcow_reduce_partials")
-                _launches += 1
-            else:
-                out = part[0]
-            gw = alias if flat is not None else out.view(Co, C, 1, 1)
-        if has_bias and ctx.needs_input_grad[2]:
-            gb = colsum(gy.permute(0, 2, 3, 1).reshape(-1, Co))
-        return gx, gw, gb
-
-
 def conv1x1_s2_usable(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Both channel counts whole 64-channel rows (the kernel's reduction rows forward, backward and in the weight gradient)."""
     return (x.is_cuda and x.dim() == 4 and _have("gcow_conv_dgrad_1x1_s2") and tuple(w.shape[2:]) == (1, 1)
@@ -1163,69 +800,11 @@ def conv1x1_s2_usable(x: torch.Tensor, w: torch.Tensor) -> bool:
 
 
 def conv1x1_s2(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor | None = None) -> torch.Tensor:
-    return _Conv1x1Stride2Fn.apply(x, w, b)
-
-
-class _ConvStride2Fn(torch.autograd.Function):
-    """3x3 convolution with stride 2 and padding 1 over even extents (the down-sampling layer of every ResNet stage)
-    on the implicit-GEMM kernel: the forward and the weight gradient read every second input pixel through a tensor
-    map with element strides; the input gradient is four stride-1 convolutions of dY, one per parity of the dX pixel,
-    with 1, 2, 2 and 4 of the nine taps. No patch matrix and no col2im scatter."""
-
-    @staticmethod
-    def forward(ctx, x, w, b):
-        global _launches
-        N, C, H, W = x.shape
-        Co = w.shape[0]
-        lib = _native.cuda()
-        if x.dtype != torch.bfloat16 or not x.is_contiguous(memory_format=torch.channels_last):
-            x = x.to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
-        wr = bf16_weight(w).permute(0, 2, 3, 1).contiguous()                                       # [Co, 3, 3, Ci]
-        y = torch.empty((N, Co, H // 2, W // 2), dtype=torch.bfloat16, device=x.device, memory_format=torch.channels_last)
-        bias = b.detach().float().contiguous() if b is not None else None
-        _chk(lib.gcow_conv_fwd_strided(x.data_ptr(), wr.data_ptr(), y.data_ptr(), bias.data_ptr() if bias is not None else None,
-                                       N, H, W, C, Co, 3, 3, 1, 1, 2, _error_word(x.device).data_ptr(), _stream(x.device)),
-             "gcow_conv_fwd_strided")
-        _launches += 1
-        ctx.save_for_backward(x, wr)
-        ctx.meta = (N, C, H, W, Co, b is not None)
-        ctx.grad_view = take_grad_view(w)
-        return y
-
-    @staticmethod
-    def backward(ctx, gy):
-        global _launches
-        x, wr = ctx.saved_tensors
-        N, C, H, W, Co, has_bias = ctx.meta
-        lib = _native.cuda()
-        if gy.dtype != torch.bfloat16 or not gy.is_contiguous(memory_format=torch.channels_last):
-            gy = gy.to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
-        dev, st, err = gy.device, _stream(gy.device), _error_word(gy.device).data_ptr()
-        gx = gw = gb = None
-        if ctx.needs_input_grad[0]:
-            wp = _ws("conv_s2_phase_w", (9 * C * Co,), torch.bfloat16, dev)
-            gx = torch.empty((N, C, H, W), dtype=torch.bfloat16, device=dev, memory_format=torch.channels_last)
-            _chk(lib.gcow_conv_dgrad_s2(gy.data_ptr(), wr.data_ptr(), wp.data_ptr(), gx.data_ptr(), N, H, W, C, Co, err, st),
-                 "gcow_conv_dgrad_s2")
-            _launches += 5
-        if ctx.needs_input_grad[1]:
-            split = lib.gcow_conv_wgrad_split_strided(N, H, W, C, Co, 3, 3, 1, 1, 2)
-            flat, alias = _grad_target(ctx.grad_view, Co, 9 * C)
-            part = (_ws("conv_wgrad_part", (split, Co, 9 * C), torch.float32, dev) if split > 1 else
-                    (flat.unsqueeze(0) if flat is not None else torch.empty((1, Co, 9 * C), dtype=torch.float32, device=dev)))
-            _chk(lib.gcow_conv_wgrad_strided(gy.data_ptr(), x.data_ptr(), part.data_ptr(), N, H, W, C, Co, 3, 3, 1, 1, 2,
-                                             err, st), "gcow_conv_wgrad_strided")
-            _launches += 1
-            if split > 1:
-                out = flat if flat is not None else torch.empty((Co, 9 * C), dtype=torch.float32, device=dev)
-                _chk(lib.gcow_reduce_partials(part.data_ptr(), out.data_ptr(), split, out.numel(), st), "gcow_reduce_partials")
-                _launches += 1
-            else:
-                out = part[0]
-            gw = alias if flat is not None else out.view(Co, 3, 3, C).permute(0, 3, 1, 2)
-        if has_bias and ctx.needs_input_grad[2]:
-            gb = colsum(gy.permute(0, 2, 3, 1).reshape(-1, Co))
-        return gx, gw, gb
+    """1x1 convolution with stride 2 (the down-sampling shortcut of a ResNet stage) on the implicit-GEMM kernel with
+    one tap: forward and weight gradient read every second pixel through a tensor map with element strides, the input
+    gradient is one launch that stores to the sampled pixels of a zero-filled tensor. No subsampled copy of the input
+    and no scatter pass."""
+    return _layers().conv(x, w, b, 1, 0, 0, _HALO_WGRAD_MIN_W)
 
 
 def conv_igemm_s2_usable(x: torch.Tensor, w: torch.Tensor, stride, padding, groups: int, dilation) -> bool:
@@ -1236,7 +815,11 @@ def conv_igemm_s2_usable(x: torch.Tensor, w: torch.Tensor, stride, padding, grou
 
 
 def conv_igemm_s2(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor | None = None) -> torch.Tensor:
-    return _ConvStride2Fn.apply(x, w, b)
+    """3x3 convolution with stride 2 and padding 1 over even extents (the down-sampling layer of every ResNet stage)
+    on the implicit-GEMM kernel: the forward and the weight gradient read every second input pixel through a tensor
+    map with element strides; the input gradient is four stride-1 convolutions of dY, one per parity of the dX pixel,
+    with 1, 2, 2 and 4 of the nine taps. No patch matrix and no col2im scatter."""
+    return _layers().conv(x, w, b, 2, 1, 1, _HALO_WGRAD_MIN_W)
 
 
 def conv_mode() -> str:
@@ -1322,7 +905,10 @@ def conv_igemm_usable(x: torch.Tensor, w: torch.Tensor, stride, padding, groups:
 
 
 def conv_igemm(x, w, b, padding):
-    return _ConvIgemmFn.apply(x, w, b, int(padding[0]), int(padding[1]))
+    """Stride-1 KxK convolution, channels-last bf16, as an implicit GEMM on the tcgen05 kernel
+    (csrc/ops/conv_tcgen05.cu): forward, data gradient (the same kernel on dY with the flipped
+    filter) and weight gradient (split over pixel ranges + ordered sum). No patch matrix."""
+    return _layers().conv(x, w, b, 0, int(padding[0]), int(padding[1]), _HALO_WGRAD_MIN_W)
 
 
 # ------------------------------------------------ batched GEMM and attention
@@ -1348,75 +934,6 @@ def bmm_bf16(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool =
     return out
 
 
-class _AttentionFn(torch.autograd.Function):
-    """Unfused multi-head self-attention on own kernels: batched QK^T GEMM, row softmax,
-    batched PV GEMM; the backward is five batched GEMMs and the softmax backward.
-    q, k, v: bf16 [batch*heads, S, D] contiguous."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, scale):
-        global _launches
-        lib = _native.cuda()
-        s = bmm_bf16(q, k)                                   # [BH, S, S] = Q K^T
-        p = torch.empty_like(s)
-        _chk(lib.gcow_softmax_fwd(s.data_ptr(), p.data_ptr(), s.shape[0] * s.shape[1], s.shape[2], scale,
-                                  _stream(q.device)), "gcow_softmax_fwd")
-        _launches += 1
-        o = bmm_bf16(p, v, b_t=True)                         # [BH, S, D] = P V   (V stored [S(red), D])
-        ctx.save_for_backward(q, k, v, p)
-        ctx.scale = scale
-        return o
-
-    @staticmethod
-    def backward(ctx, go):
-        global _launches
-        q, k, v, p = ctx.saved_tensors
-        go = go.to(torch.bfloat16).contiguous()
-        dv = bmm_bf16(p, go, a_t=True, b_t=True)             # P^T dO
-        dp = bmm_bf16(go, v)                                 # dO V^T
-        ds = torch.empty_like(p)
-        _chk(_native.cuda().gcow_softmax_bwd(dp.data_ptr(), p.data_ptr(), ds.data_ptr(), p.shape[0] * p.shape[1],
-                                             p.shape[2], ctx.scale, _stream(q.device)), "gcow_softmax_bwd")
-        _launches += 1
-        dq = bmm_bf16(ds, k, b_t=True)                       # dS K
-        dk = bmm_bf16(ds, q, a_t=True, b_t=True)             # dS^T Q
-        return dq, dk, dv, None
-
-
-class _FusedAttentionFn(torch.autograd.Function):
-    """Fused self-attention on the tcgen05 kernels of csrc/ops/attention_tcgen05.cu: packed qkv [B, S, 3, H, 64] in,
-    context [B, S, H*64] out; the backward recomputes the probabilities from the stored log-sum-exp and writes
-    the packed gradient [B, S, 3, H, 64]."""
-
-    @staticmethod
-    def forward(ctx, qkv, scale):
-        global _launches
-        B, S, _, H, D = qkv.shape
-        q = qkv if (qkv.dtype == torch.bfloat16 and qkv.is_contiguous()) else qkv.to(torch.bfloat16).contiguous()
-        out = torch.empty((B, S, H * D), dtype=torch.bfloat16, device=q.device)
-        lse = torch.empty((B, H, S), dtype=torch.float32, device=q.device)
-        _chk(_native.cuda().gcow_attention_fwd(q.data_ptr(), out.data_ptr(), lse.data_ptr(), B, S, H, D, scale,
-                                               _error_word(q.device).data_ptr(), _stream(q.device)), "gcow_attention_fwd")
-        _launches += 1
-        ctx.save_for_backward(q, out, lse)
-        ctx.scale = scale
-        return out
-
-    @staticmethod
-    def backward(ctx, go):
-        global _launches
-        q, out, lse = ctx.saved_tensors
-        B, S, _, H, D = q.shape
-        g = go if (go.dtype == torch.bfloat16 and go.is_contiguous()) else go.to(torch.bfloat16).contiguous()
-        dqkv = torch.empty_like(q)
-        delta = _ws("attn_delta", (B, H, S), torch.float32, q.device)
-        _chk(_native.cuda().gcow_attention_bwd(q.data_ptr(), out.data_ptr(), g.data_ptr(), lse.data_ptr(), delta.data_ptr(),
-                                               dqkv.data_ptr(), B, S, H, D, ctx.scale, _error_word(q.device).data_ptr(),
-                                               _stream(q.device)), "gcow_attention_bwd")
-        _launches += 3
-        return dqkv, None
-
-
 def fused_attention_usable(qkv: torch.Tensor) -> bool:
     """Head dimension 64 and a sequence length that is a multiple of 128, at most 512."""
     if not (qkv.is_cuda and qkv.dim() == 5 and _have("gcow_attention_fwd")):
@@ -1426,8 +943,9 @@ def fused_attention_usable(qkv: torch.Tensor) -> bool:
 
 
 def fused_attention(qkv: torch.Tensor) -> torch.Tensor:
-    """qkv: [B, S, 3, H, 64] -> context [B, S, H*64]."""
-    return _FusedAttentionFn.apply(qkv, 1.0 / (qkv.shape[-1] ** 0.5))
+    """qkv: [B, S, 3, H, 64] -> context [B, S, H*64] on the tcgen05 kernels of csrc/ops/attention_tcgen05.cu; the backward
+    recomputes the probabilities from the stored log-sum-exp and writes the packed gradient [B, S, 3, H, 64]."""
+    return _layers().fused_attention(qkv, 1.0 / (qkv.shape[-1] ** 0.5))
 
 
 def attention_mode() -> str:
@@ -1444,8 +962,9 @@ def attention_usable(qkv: torch.Tensor) -> bool:
 
 
 def attention(qkv: torch.Tensor) -> torch.Tensor:
-    """qkv: [B, S, 3, H, D] -> context [B, S, H*D]."""
+    """qkv: [B, S, 3, H, D] -> context [B, S, H*D], unfused: batched QK^T GEMM, row softmax, batched PV GEMM; the backward
+    is five batched GEMMs and the softmax backward."""
     B, S, _, H, D = qkv.shape
     t = qkv.to(torch.bfloat16).permute(2, 0, 3, 1, 4).contiguous().view(3, B * H, S, D)
-    o = _AttentionFn.apply(t[0], t[1], t[2], 1.0 / (D ** 0.5))
+    o = _layers().attention(t[0], t[1], t[2], 1.0 / (D ** 0.5))
     return o.view(B, H, S, D).permute(0, 2, 1, 3).reshape(B, S, H * D)
