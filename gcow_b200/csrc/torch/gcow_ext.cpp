@@ -144,6 +144,7 @@ PyObject* decompress(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const uint64_t* index = nullptr;
   if (!fixed) {
     if (args[1] == Py_None) Py_RETURN_NONE;
+    TORCH_CHECK_TYPE(THPVariable_Check(args[1]), "decompress: the index is no tensor");
     const at::Tensor& i = THPVariable_Unpack(args[1]);
     if (i.device() != s.device()) Py_RETURN_NONE;
     index = (const uint64_t*)i.const_data_ptr();

@@ -13,6 +13,7 @@
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
 
 #include <atomic>
 #include <cstdlib>
@@ -142,6 +143,10 @@ Tensor gemm(const Tensor& a, const Tensor& b, const GemmOpts& o, const On& on) {
   TORCH_CHECK(K == Kb, "gemm: reduction lengths differ");
   Tensor out = o.out.defined() ? o.out : empty({M, N}, o.out_f32 ? at::kFloat : at::kBFloat16, a);
   const Tensor& aux = o.pre_gelu_out.defined() ? o.pre_gelu_out : o.gelu_grad_of;
+  TORCH_CHECK(out.size(0) == M && out.size(1) == N, "gemm: the result has another shape than the product");
+  TORCH_CHECK(!o.bias.defined() || o.bias.numel() == N, "gemm: the bias has another length than the product's rows");
+  TORCH_CHECK(!o.residual.defined() || (o.residual.sizes() == out.sizes() && o.residual.strides() == out.strides()),
+              "gemm: the residual has another shape than the product");
   int flags = (out.scalar_type() == at::kFloat ? kOutF32 : 0) | (o.bias.defined() ? kBias : 0) | (o.gelu ? kGelu : 0) |
               (o.residual.defined() ? kResidual : 0);
   if (aux.defined()) flags |= o.pre_gelu_out.defined() ? kAuxOut : kGeluGrad;
@@ -266,29 +271,26 @@ Tensor target_matrix(const Target& t, int64_t rows, int64_t cols, uintptr_t alig
 }
 
 // ---------------------------------------------------------------------- autograd nodes
-// A tensor kept for the backward pass: detached, with the version check that catches in-place writes in between.
+// A tensor kept for the backward pass. SavedVariable runs the saved-tensor hooks in force (activation offload and
+// checkpointing work through them), catches in-place writes in between and breaks the cycle between a node and its output.
 struct Kept {
-  Tensor t;
-  uint32_t version = 0;
-  void set(const Tensor& x) {
-    if (!x.defined()) return;
-    t = x.requires_grad() ? x.tensor_data() : x;            // shares the version counter
-    version = (uint32_t)x._version();
-  }
-  const Tensor& get() const {
-    TORCH_CHECK(t.defined(), "Trying to backward through the graph a second time, or to use a tensor that was freed by the first");
-    TORCH_CHECK((uint32_t)t._version() == version, "a tensor needed for gradient computation has been modified by an inplace operation");
-    return t;
-  }
+  torch::autograd::SavedVariable saved;
+  void set(const Tensor& x, bool is_output = false) { saved = torch::autograd::SavedVariable(x, is_output); }
 };
 
 // Backward nodes: `kept` holds the saved tensors, inputs are numbered in the order given to record().
 struct LayerNode : torch::autograd::Node {
   Kept kept[6];
   Target target[2];
+  bool released = false;
   void release_variables() override {
-    for (auto& k : kept) k.t.reset();
+    for (auto& k : kept) k.saved.reset_data();
     for (auto& t : target) { t.view.reset(); t.weight.reset(); }
+    released = true;
+  }
+  Tensor get(int i) {
+    TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+    return kept[i].saved.unpack(shared_from_this());
   }
   bool wants(size_t i) { return task_should_compute_output(i); }
   virtual variable_list grads(variable_list&& g) = 0;
@@ -301,22 +303,32 @@ struct LayerNode : torch::autograd::Node {
 
 template <class N, class... In>
 std::shared_ptr<N> record(const In&... in) {
+  const Tensor* const all[] = {&in...};
+  for (const Tensor* t : all)
+    TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->_fw_grad(0).defined(), "forward-mode AD is not implemented for this layer function");
   if (!at::GradMode::is_enabled() || !torch::autograd::compute_requires_grad(in...)) return nullptr;
   std::shared_ptr<N> n(new N(), torch::autograd::deleteNode);
   n->set_next_edges(torch::autograd::collect_next_edges(in...));
   return n;
 }
-// Everything up to the history of the result runs below autograd.
+// Everything up to the history of the result runs without gradients, as in the forward of a Python function; views are
+// still tracked, so that a saved view of an input shares the input's version counter.
 struct Below {
   at::NoGradGuard no_grad;
-  at::AutoDispatchBelowADInplaceOrView below;
 };
 template <class N>
 PyObject* finish(Tensor out, const std::shared_ptr<N>& n) {
   if (n) torch::autograd::set_history(out, n);
   return THPVariable_Wrap(std::move(out));
 }
-inline Tensor arg(PyObject* o) { return o == Py_None ? Tensor() : THPVariable_Unpack(o); }   // None: undefined
+inline Tensor arg(PyObject* o) {                            // None: undefined
+  TORCH_CHECK_TYPE(o == Py_None || THPVariable_Check(o), "expected a tensor, got ", Py_TYPE(o)->tp_name);
+  return o == Py_None ? Tensor() : THPVariable_Unpack(o);
+}
+inline Tensor need(PyObject* o) {
+  TORCH_CHECK_TYPE(o != Py_None, "expected a tensor, got None");
+  return arg(o);
+}
 inline Tensor rows_of(const Tensor& x) { return bf16_rows(x.reshape({-1, x.size(-1)})); }
 inline Tensor as_rows(const Tensor& x) { return x.view({-1, x.size(-1)}); }
 inline std::vector<int64_t> with_last(const Tensor& x, int64_t last) {
@@ -341,7 +353,7 @@ struct LinearNode : LayerNode {                             // inputs: x, w, b, 
   variable_list grads(variable_list&& in) override {
     variable_list out(4);
     if (!in[0].defined()) return out;
-    const Tensor &xb = kept[0].get(), &wb = kept[1].get();
+    const Tensor xb = get(0), wb = get(1);
     const On on(xb);
     const Tensor g = rows_of(in[0]);
     if (wants(0)) {                                         // dx[M,K] = g[M,N] W[N,K]: W is stored [reduction N][K]
@@ -364,7 +376,7 @@ struct LinearNode : LayerNode {                             // inputs: x, w, b, 
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(nargs == 4, "linear: bad arguments");
-  const Tensor x = arg(args[0]), w = arg(args[1]), b = arg(args[2]), r = arg(args[3]);
+  const Tensor x = need(args[0]), w = need(args[1]), b = arg(args[2]), r = arg(args[3]);
   auto node = record<LinearNode>(x, w, b, r);
   Tensor out;
   {
@@ -396,7 +408,7 @@ struct FfnNode : LayerNode {                                // inputs: x, w1, b1
   variable_list grads(variable_list&& in) override {
     variable_list out(5);
     if (!in[0].defined()) return out;
-    const Tensor &xb = kept[0].get(), &w1b = kept[1].get(), &w2b = kept[2].get(), &pre = kept[3].get(), &act = kept[4].get();
+    const Tensor xb = get(0), w1b = get(1), w2b = get(2), pre = get(3), act = get(4);
     const On on(xb);
     const Tensor g = rows_of(in[0]);
     GemmOpts o;
@@ -424,7 +436,7 @@ struct FfnNode : LayerNode {                                // inputs: x, w1, b1
 PyObject* ffn_residual(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(nargs == 5, "ffn_residual: bad arguments");
-  const Tensor x = arg(args[0]), w1 = arg(args[1]), b1 = arg(args[2]), w2 = arg(args[3]), b2 = arg(args[4]);
+  const Tensor x = need(args[0]), w1 = need(args[1]), b1 = need(args[2]), w2 = need(args[3]), b2 = need(args[4]);
   auto node = record<FfnNode>(x, w1, b1, w2, b2);
   Tensor out;
   {
@@ -462,7 +474,7 @@ struct LayerNormNode : LayerNode {                          // inputs: x, gamma,
   variable_list grads(variable_list&& in) override {
     variable_list out(3);
     if (!in[0].defined()) return out;
-    const Tensor &xb = kept[0].get(), &g32 = kept[1].get(), &mean = kept[2].get(), &rstd = kept[3].get();
+    const Tensor xb = get(0), g32 = get(1), mean = get(2), rstd = get(3);
     const On on(xb);
     const int64_t rows = xb.size(0), H = xb.size(1);
     const Tensor g = rows_of(in[0]);
@@ -481,7 +493,7 @@ struct LayerNormNode : LayerNode {                          // inputs: x, gamma,
 PyObject* layernorm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {      // (x, gamma, beta, eps)
   HANDLE_TH_ERRORS
   TORCH_CHECK(nargs == 4, "layernorm: bad arguments");
-  const Tensor x = arg(args[0]), gamma = arg(args[1]), beta = arg(args[2]);
+  const Tensor x = need(args[0]), gamma = need(args[1]), beta = need(args[2]);
   const double eps = PyFloat_AsDouble(args[3]);
   if (PyErr_Occurred()) return nullptr;
   auto node = record<LayerNormNode>(x, gamma, beta);
@@ -514,7 +526,7 @@ struct FusedAttentionNode : LayerNode {                     // input: qkv
   variable_list grads(variable_list&& in) override {
     variable_list out(1);
     if (!in[0].defined() || !wants(0)) return out;
-    const Tensor &q = kept[0].get(), &o = kept[1].get(), &lse = kept[2].get();
+    const Tensor q = get(0), o = get(1), lse = get(2);
     const On on(q);
     const int B = (int)q.size(0), S = (int)q.size(1), H = (int)q.size(3), D = (int)q.size(4);
     const Tensor g = bf16_rows(in[0]);
@@ -531,7 +543,7 @@ struct FusedAttentionNode : LayerNode {                     // input: qkv
 PyObject* fused_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {   // (qkv [B, S, 3, H, 64], scale)
   HANDLE_TH_ERRORS
   TORCH_CHECK(nargs == 2, "fused_attention: bad arguments");
-  const Tensor qkv = arg(args[0]);
+  const Tensor qkv = need(args[0]);
   const double scale = PyFloat_AsDouble(args[1]);
   if (PyErr_Occurred()) return nullptr;
   auto node = record<FusedAttentionNode>(qkv);
@@ -548,12 +560,15 @@ PyObject* fused_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) { 
     g_launches++;
     if (node) {
       node->kept[0].set(q);
-      node->kept[1].set(out);
       node->kept[2].set(lse);
       node->scale = (float)scale;
     }
   }
-  return finish(std::move(out), node);
+  if (node) {
+    torch::autograd::set_history(out, node);
+    node->kept[1].set(out, true);
+  }
+  return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
 }
 
@@ -574,7 +589,7 @@ struct AttentionNode : LayerNode {                          // inputs: q, k, v
   variable_list grads(variable_list&& in) override {
     variable_list out(3);
     if (!in[0].defined()) return out;
-    const Tensor &q = kept[0].get(), &k = kept[1].get(), &v = kept[2].get(), &p = kept[3].get();
+    const Tensor q = get(0), k = get(1), v = get(2), p = get(3);
     const On on(q);
     const Tensor go = bf16_rows(in[0]);
     out[2] = bmm(p, go, true, true, on);                    // P^T dO
@@ -592,7 +607,7 @@ struct AttentionNode : LayerNode {                          // inputs: q, k, v
 PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {      // (q, k, v [batch * heads, S, D] bf16, scale)
   HANDLE_TH_ERRORS
   TORCH_CHECK(nargs == 4, "attention: bad arguments");
-  const Tensor q = arg(args[0]), k = arg(args[1]), v = arg(args[2]);
+  const Tensor q = need(args[0]), k = need(args[1]), v = need(args[2]);
   const double scale = PyFloat_AsDouble(args[3]);
   if (PyErr_Occurred()) return nullptr;
   auto node = record<AttentionNode>(q, k, v);
@@ -661,7 +676,7 @@ struct ConvNode : LayerNode {                               // inputs: x, w, b
   variable_list grads(variable_list&& in) override {
     variable_list out(3);
     if (!in[0].defined()) return out;
-    const Tensor &x = kept[0].get(), &wr = kept[1].get();
+    const Tensor x = get(0), wr = get(1);
     const On on(x);
     const Tensor gy = nhwc_bf16(in[0]);
     const void* const g = gy.data_ptr();
@@ -715,7 +730,7 @@ struct ConvNode : LayerNode {                               // inputs: x, w, b
 PyObject* conv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(nargs == 7, "conv: bad arguments");
-  const Tensor xin = arg(args[0]), w = arg(args[1]), b = arg(args[2]);
+  const Tensor xin = need(args[0]), w = need(args[1]), b = arg(args[2]);
   int v[4];
   for (int i = 0; i < 4; i++) v[i] = (int)PyLong_AsLong(args[3 + i]);
   if (PyErr_Occurred()) return nullptr;
@@ -758,7 +773,7 @@ struct Conv1x1Node : LayerNode {                            // inputs: x, w, b
   variable_list grads(variable_list&& in) override {
     variable_list out(3);
     if (!in[0].defined()) return out;
-    const Tensor &xm = kept[0].get(), &wb = kept[1].get();
+    const Tensor xm = get(0), wb = get(1);
     const On on(xm);
     const Tensor g = bf16_rows(in[0].permute({0, 2, 3, 1})).view({-1, Co});
     if (wants(0)) {
@@ -780,7 +795,7 @@ struct Conv1x1Node : LayerNode {                            // inputs: x, w, b
 PyObject* conv1x1(PyObject*, PyObject* const* args, Py_ssize_t nargs) {        // (x, w, b or None): a GEMM over the pixels
   HANDLE_TH_ERRORS
   TORCH_CHECK(nargs == 3, "conv1x1: bad arguments");
-  const Tensor x = arg(args[0]), w = arg(args[1]), b = arg(args[2]);
+  const Tensor x = need(args[0]), w = need(args[1]), b = arg(args[2]);
   auto node = record<Conv1x1Node>(x, w, b);
   Tensor out;
   {
@@ -817,8 +832,8 @@ struct BatchNormNode : LayerNode {                          // inputs: x, gamma,
     Tensor gy = in[0], gy2 = in.size() > 1 ? in[1] : Tensor();
     if (!gy.defined()) std::swap(gy, gy2);
     if (!gy.defined()) return out;
-    const Tensor &x = kept[0].get(), &g32 = kept[1].get(), &stats = kept[2].get();
-    const Tensor mask = relu ? kept[3].get() : Tensor();
+    const Tensor x = get(0), g32 = get(1), stats = get(2);
+    const Tensor mask = relu ? get(3) : Tensor();
     const On on(x);
     gy = nhwc_bf16(gy);
     if (gy2.defined()) gy2 = nhwc_bf16(gy2);
@@ -856,7 +871,7 @@ struct BatchNormNode : LayerNode {                          // inputs: x, gamma,
 PyObject* batchnorm_act(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(nargs == 10, "batchnorm_act: bad arguments");
-  const Tensor x = arg(args[0]), gamma = arg(args[1]), beta = arg(args[2]), rm = arg(args[3]), rv = arg(args[4]), res = arg(args[5]);
+  const Tensor x = need(args[0]), gamma = need(args[1]), beta = need(args[2]), rm = arg(args[3]), rv = arg(args[4]), res = arg(args[5]);
   const bool relu = PyObject_IsTrue(args[6]) == 1, fork = PyObject_IsTrue(args[9]) == 1;
   const double momentum = PyFloat_AsDouble(args[7]), eps = PyFloat_AsDouble(args[8]);
   if (PyErr_Occurred()) return nullptr;

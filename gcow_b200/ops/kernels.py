@@ -40,8 +40,48 @@ def _have(name: str) -> bool:
     return False
 
 
+class _TracedLayerFn(torch.autograd.Function):
+    """A layer function as one Python node of a ``torch.jit.trace`` graph: the tracer records Python functions and the
+    operators of torch, and would take the result of an extension function for a constant."""
+
+    @staticmethod
+    def forward(ctx, name, *args):
+        state = torch._C._get_tracing_state()
+        torch._C._set_tracing_state(None)
+        try:
+            with torch.enable_grad():
+                ctx.leaves = [a.detach().requires_grad_(need) if isinstance(a, torch.Tensor) else a
+                              for a, need in zip(args, ctx.needs_input_grad[1:])]
+                ctx.out = getattr(_native.ext(), name)(*ctx.leaves)
+            if isinstance(ctx.out, tuple):
+                return tuple(o.detach() for o in ctx.out)
+            return ctx.out.detach()
+        finally:
+            torch._C._set_tracing_state(state)
+
+    @staticmethod
+    def backward(ctx, *grads):
+        outs = ctx.out if isinstance(ctx.out, tuple) else (ctx.out,)
+        wanted = [i for i, a in enumerate(ctx.leaves) if isinstance(a, torch.Tensor) and a.requires_grad]
+        got = torch.autograd.grad(outs, [ctx.leaves[i] for i in wanted], grads)
+        res = [None] * (1 + len(ctx.leaves))
+        for i, g in zip(wanted, got):
+            res[1 + i] = g
+        return tuple(res)
+
+
+class _TracedLayers:
+    def __getattr__(self, name):
+        return lambda *args: _TracedLayerFn.apply(name, *args)
+
+
+_traced_layers = _TracedLayers()
+
+
 def _layers():
     """The extension module's layer functions (csrc/torch/layers.cpp)."""
+    if torch._C._get_tracing_state() is not None:
+        return _traced_layers
     return _native._ext or _native.ext()
 
 
@@ -72,7 +112,7 @@ def workspace_bytes() -> int:
 def _error_word(device: torch.device) -> torch.Tensor:
     w = _err_words.get(device)
     if w is None:
-        w = _layers().error_word(device.index if device.index is not None else torch.cuda.current_device())
+        w = (_native._ext or _native.ext()).error_word(device.index if device.index is not None else torch.cuda.current_device())
         _err_words[device] = w
     return w
 
@@ -86,7 +126,7 @@ def check_errors(device: torch.device | None = None, raise_on_error: bool = True
     """Read the error word of the compute kernels (synchronises). Raises KernelWaitAbandoned if a kernel gave up on
     an internal wait, or returns the code when ``raise_on_error`` is false. The word is cleared."""
     worst = 0
-    for w in _layers().error_words():
+    for w in _native.ext().error_words():
         dev = w.device
         if device is not None and dev != device:
             continue

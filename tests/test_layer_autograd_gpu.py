@@ -1,0 +1,111 @@
+"""The extension module's layer functions inside autograd: saved-tensor hooks, in-place checks, lifetimes, tracing."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _cases(weight_grad=True):
+    from gcow_b200.ops import kernels as K
+    from gcow_b200.ops import nn as gnn
+    torch.manual_seed(0)
+
+    def r(*s, dtype=torch.bfloat16):
+        return torch.randn(*s, device="cuda", dtype=dtype).requires_grad_(weight_grad or dtype == torch.bfloat16)
+
+    def nhwc(*s):
+        return torch.randn(*s, device="cuda", dtype=torch.bfloat16).to(memory_format=torch.channels_last).requires_grad_(True)
+    f = torch.float32
+    bn = gnn.BatchNorm2d(64).cuda().requires_grad_(weight_grad)
+    w, w1, w2 = r(64, 128, dtype=f), r(256, 128, dtype=f), r(128, 256, dtype=f)
+    b, b1, b2 = r(64, dtype=f), r(256, dtype=f), r(128, dtype=f)
+    gam, c1, c3 = r(128, dtype=f), r(64, 64, 1, 1, dtype=f), r(64, 64, 3, 3, dtype=f)
+    return {
+        "linear": (lambda x: K.linear(x, w, b), r(2, 64, 128)),
+        "ffn": (lambda x: K.ffn_residual(x, w1, b1, w2, b2), r(2, 64, 128)),
+        "layernorm": (lambda x: K.layernorm(x, gam, b2, 1e-5), r(2, 64, 128)),
+        "attention": (K.fused_attention, r(2, 128, 3, 2, 64)),
+        "conv1x1": (lambda x: K.conv1x1(x, c1, None), nhwc(2, 64, 8, 8)),
+        "conv3x3": (lambda x: K.conv_igemm(x, c3, None, (1, 1)), nhwc(2, 64, 8, 8)),
+        "batchnorm": (lambda x: K.batchnorm_act(x, bn, relu=True), nhwc(2, 64, 8, 8)),
+    }
+
+
+NAMES = ("linear", "ffn", "layernorm", "attention", "conv1x1", "conv3x3", "batchnorm")
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_saved_tensor_hooks(name):
+    """Everything kept for the backward pass goes through the hooks, so offload and checkpointing see it."""
+    fn, x = _cases()[name]
+    packed = []
+
+    def pack(t):
+        packed.append(t.numel())
+        return t.detach().cpu()
+    want = torch.autograd.grad(fn(x).float().square().sum(), x)[0]
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()):
+        y = fn(x)
+    assert packed
+    got = torch.autograd.grad(y.float().square().sum(), x)[0]
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_inplace_write_is_noticed(name):
+    fn, leaf = _cases()[name]
+    x = leaf * 1.0
+    y = fn(x)
+    with torch.no_grad():
+        x.mul_(2)
+    with pytest.raises(RuntimeError, match="in-?place"):
+        y.float().sum().backward()
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_graph_without_backward_is_freed(name):
+    fn, x = _cases()[name]
+    fn(x)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    for _ in range(3):
+        fn(x)
+    torch.cuda.synchronize()
+    assert torch.cuda.memory_allocated() == before
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_second_backward_and_transforms_are_refused(name):
+    fn, x = _cases()[name]
+    y = fn(x)
+    y.float().sum().backward()
+    with pytest.raises(RuntimeError, match="second time"):
+        y.backward(torch.ones_like(y))
+    import torch.autograd.forward_ad as fwd
+    with pytest.raises((NotImplementedError, RuntimeError)), fwd.dual_level():
+        fn(fwd.make_dual(x.detach(), torch.ones_like(x)))
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(fn)(x.detach()[None])
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_trace(name):
+    """A traced function computes from its input, forward and backward, and not from the tracing input's result."""
+    fn, x = _cases(False)[name]
+    traced = torch.jit.trace(fn, (x.detach(),), check_trace=False)
+    x2 = (x.detach() * 0.5 + 0.1).requires_grad_(True)
+    y, z = fn(x2), traced(x2)
+    assert torch.equal(y, z)
+    gy = torch.randn_like(y)
+    assert torch.equal(torch.autograd.grad(y, x2, gy)[0], torch.autograd.grad(z, x2, gy)[0])
+
+
+def test_wrong_arguments_are_refused():
+    from gcow_b200.ops import kernels as K
+    x, w = torch.randn(64, 128, device="cuda").bfloat16(), torch.randn(64, 128, device="cuda")
+    with pytest.raises(TypeError):
+        K.linear(x, w, "b")
+    with pytest.raises(RuntimeError):
+        K.linear(x, w, torch.zeros(32, device="cuda"))
+    with pytest.raises(RuntimeError):
+        K.linear_residual(x, w, None, torch.zeros(32, 64, device="cuda"))
