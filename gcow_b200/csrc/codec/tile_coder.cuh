@@ -184,16 +184,17 @@ GCOW_HD uint32_t encode_slot_1d(const float* f, const ZfpParams& p, const uint32
   s.begin(2u * biased + 1u, z);
   uint32_t left = planes - z;
   if (left && s.bits() < p.maxbits) {                      // z < 32
-    const uint32_t R = byte_perm(byte_perm(u[0] << z, u[1] << z, 0x0073), byte_perm(u[2] << z, u[3] << z, 0x0073), 0x5410);
+    const uint32_t m = pow2_factor(z);
+    const uint32_t R = byte_perm(byte_perm(u[0] * m, u[1] * m, 0x0073), byte_perm(u[2] * m, u[3] * m, 0x0073), 0x5410);
     // byte i = the next eight planes of coefficient i
     uint32_t n = 0;
     if (left >= 8) {
+      uint32_t e[4], prev = 0;
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const uint32_t e = epair[n * 256u + ((((R >> (6 - 2 * j)) & 0x03030303u) * 0x40100401u) >> 24)];
-        s.put(e & 0xffffu, (e >> 16) & 0xffu);
-        n += e >> 24;
-      }
+      for (int j = 0; j < 4; j++) prev = e[j] = pair_entry(epair, R, j, prev);
+      s.put(prepend_code(e[0], prepend_code(e[1], 0)), (e[0] + e[1]) & 63u);   // at most 28 bits
+      s.put(prepend_code(e[2], prepend_code(e[3], 0)), (e[2] + e[3]) & 63u);
+      n = (prev >> 8) & 0xffu;
       left -= 8;
       uint32_t k = 24 - z;                                 // planes k-1 .. k-left remain
       while (left && s.bits() < p.maxbits) {
@@ -211,17 +212,16 @@ GCOW_HD uint32_t encode_slot_1d(const float* f, const ZfpParams& p, const uint32
         s.put(T & low_mask32(4 * cnt), 4 * cnt);
       }
     } else {
+      uint32_t prev = 0;
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         if (left > 2u * j) {
-          uint32_t g = (((R >> (6 - 2 * j)) & 0x03030303u) * 0x40100401u) >> 24;
           const bool single = left == 2u * j + 1;
-          if (single) g &= 0xaau;
-          const uint32_t e = epair[n * 256u + g];
-          n += e >> 24;
-          uint32_t len = (e >> 16) & 0xffu;
+          prev = pair_entry(epair, single ? R & 0xaaaaaaaau : R, j, prev);
+          n = (prev >> 8) & 0xffu;
+          uint32_t len = prev & 31u;
           if (single) len -= n < 4 ? n + 1 : 4u;
-          s.put(e & 0xffffu, len);
+          s.put(prepend_code(prev, 0) & low_mask32(len), len);
         }
       }
     }

@@ -424,7 +424,7 @@ place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restric
 template <int DIM, bool BUDGET>
 __global__ void __launch_bounds__(kTileThreads)
 decode_tiles_kernel(const uint32_t* __restrict__ in, float* __restrict__ out, const TileArgs a,
-                    const uint64_t* __restrict__ block_bits, int shift, const uint32_t* __restrict__ loop_tab) {
+                    const uint64_t* __restrict__ block_bits, int shift, const uint16_t* __restrict__ plane_tab) {
   constexpr int kPer = TileShape<DIM>::kPer, WB = TileShape<DIM>::kWarpBlocks, NB = TileShape<DIM>::kBlocks;
   constexpr int kTabWords = DIM == 1 ? 384 : kUnrestTabSize;
   extern __shared__ __align__(16) uint32_t smem[];
@@ -432,7 +432,10 @@ decode_tiles_kernel(const uint32_t* __restrict__ in, float* __restrict__ out, co
   uint32_t* const words = smem + kTabWords + warp * a.warp_words;
   const uint32_t cap = a.slot_words;
   if (DIM == 1) {
-    for (int i = tid; i < 384; i += kTileThreads) smem[i] = loop_tab[((i >> 7) * 8 + 7) * 128 + (i & 127)];
+    for (int i = tid; i < 384; i += kTileThreads) {          // plane | used << 8 | n' << 28
+      const uint32_t e = plane_tab[((i >> 7) * 8 + 7) * 128 + (i & 127)];
+      smem[i] = (e & 15u) | (((e >> 4) & 7u) << 8) | ((e >> 7) << 28);
+    }
   } else {
     smem[tid] = make_unrest_entry((uint32_t)tid);
   }
@@ -676,7 +679,7 @@ int gcow_decode_tiles(const void* in, float* out, uint64_t nx, uint64_t ny, cons
   do {                                                                                                         \
     const int g = grid_of<&decode_tiles_kernel<D, B>>(smem, a.tiles, &err);                                    \
     if (err) return err;                                                                                       \
-    decode_tiles_kernel<D, B><<<g, kTileThreads, smem, s>>>((const uint32_t*)in, out, a, block_bits, shift, (const uint32_t*)lt); \
+    decode_tiles_kernel<D, B><<<g, kTileThreads, smem, s>>>((const uint32_t*)in, out, a, block_bits, shift, (const uint16_t*)dt); \
   } while (0)
   if (dim == 1) GCOW_DECODE(1, true);
   else if (budget_cuts(p, 2)) GCOW_DECODE(2, true);
