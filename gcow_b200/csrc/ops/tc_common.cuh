@@ -117,31 +117,64 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t saddr) {
   return d;
 }
 
-// GELU pieces for GEMM epilogues, where eight warps do the elementwise math of a whole tile and libm's erff
+// GELU for GEMM epilogues, where eight warps do the elementwise math of a whole tile and libm's erff
 // (a long dependent chain) would take longer than the tile's main loop. Phi(x) = 0.5 (1 + erf(x / sqrt 2)) from
 // the rational approximation erf(z) = 1 - (a1 t + ... + a5 t^5) exp(-z^2), t = 1 / (1 + p z) (Abramowitz &
 // Stegun 7.1.26, absolute error below 1.5e-7); exp(-z^2) = exp(-x^2 / 2) is also what the derivative needs.
-__device__ __forceinline__ void gelu_parts(float x, float& cdf, float& gauss) {
-  const float z = fabsf(x) * 0.70710678118654752f;
-  const float t = __fdividef(1.0f, fmaf(0.3275911f, z, 1.0f));
-  gauss = __expf(-0.5f * x * x);
-  float q = fmaf(1.061405429f, t, -1.453152027f);
-  q = fmaf(q, t, 1.421413741f);
-  q = fmaf(q, t, -0.284496736f);
-  q = fmaf(q, t, 0.254829592f);
-  q = 0.5f * q * t * gauss;
-  cdf = x >= 0.0f ? 1.0f - q : q;
+// Two elements per instruction (f32x2), constant factors folded into the coefficients, and the flushing forms of the
+// reciprocal (its argument is at least 1) and of the exponential (values below 2^-126 read as 0): the other forms
+// wrap each in a range test. 16384 x 4096 x 1024 product with bias and GELU: 146 -> 134 us, of 102 us without GELU.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r;
 }
-__device__ __forceinline__ float gelu_f(float x) {
-  float cdf, g;
-  gelu_parts(x, cdf, g);
-  return x * cdf;
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r;
 }
-// d/dx of x Phi(x) = Phi(x) + x phi(x)
-__device__ __forceinline__ float gelu_grad_f(float x) {
-  float cdf, g;
-  gelu_parts(x, cdf, g);
-  return fmaf(x * 0.3989422804014327f, g, cdf);
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r;
+}
+__device__ __forceinline__ float rcp_ftz(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float ex2_ftz(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+// Phi and exp(-x^2 / 2) of two values
+__device__ __forceinline__ void gelu_parts2(float x0, float x1, uint64_t x, uint64_t& cdf, uint64_t& gauss) {
+  constexpr float kP = 0.3275911f * 0.70710678118654752f;
+  float a, b;
+  unpack2(fma2(pack2(fabsf(x0), fabsf(x1)), pack2(kP, kP), pack2(1.0f, 1.0f)), a, b);
+  const uint64_t t = pack2(rcp_ftz(a), rcp_ftz(b));
+  constexpr float kE = -0.72134752044448170f;               // -log2(e) / 2
+  unpack2(mul2(mul2(x, x), pack2(kE, kE)), a, b);
+  gauss = pack2(ex2_ftz(a), ex2_ftz(b));
+  uint64_t q = fma2(t, pack2(0.5f * 1.061405429f, 0.5f * 1.061405429f), pack2(0.5f * -1.453152027f, 0.5f * -1.453152027f));
+  q = fma2(q, t, pack2(0.5f * 1.421413741f, 0.5f * 1.421413741f));
+  q = fma2(q, t, pack2(0.5f * -0.284496736f, 0.5f * -0.284496736f));
+  q = fma2(q, t, pack2(0.5f * 0.254829592f, 0.5f * 0.254829592f));
+  q = mul2(mul2(q, t), gauss);
+  float q0, q1;
+  unpack2(q, q0, q1);
+  unpack2(fma2(q, pack2(-1.0f, -1.0f), pack2(1.0f, 1.0f)), a, b);
+  cdf = pack2(x0 >= 0.0f ? a : q0, x1 >= 0.0f ? b : q1);
+}
+// v = GELU(v)
+__device__ __forceinline__ void gelu32(float (&v)[32]) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 2) {
+    const uint64_t x = pack2(v[j], v[j + 1]);
+    uint64_t cdf, gauss;
+    gelu_parts2(v[j], v[j + 1], x, cdf, gauss);
+    unpack2(mul2(x, cdf), v[j], v[j + 1]);
+  }
+}
+// v *= d/dx of x Phi(x) = Phi(x) + x phi(x)
+__device__ __forceinline__ void gelu_grad8(float* v, const float* s) {
+#pragma unroll
+  for (int j = 0; j < 8; j += 2) {
+    const uint64_t x = pack2(s[j], s[j + 1]);
+    uint64_t cdf, gauss;
+    gelu_parts2(s[j], s[j + 1], x, cdf, gauss);
+    const uint64_t d = fma2(mul2(x, pack2(0.3989422804014327f, 0.3989422804014327f)), gauss, cdf);
+    unpack2(mul2(pack2(v[j], v[j + 1]), d), v[j], v[j + 1]);
+  }
 }
 
 // Coalesced bf16 rows for epilogues. After tcgen05.ld a lane owns one row of the tile (32 consecutive columns),
@@ -175,6 +208,24 @@ __device__ __forceinline__ void warp_store_rows_bf16(uint8_t* stg, int lane, con
     if (ok) *reinterpret_cast<uint4*>(base + off + ch * 8) = x;
   }
   __syncwarp();
+}
+
+// A block that was fetched four lanes per row (row it * 8 + lane / 4, chunk lane & 3, in x[it]) into the staging buffer,
+// from where own_chunk() reads eight columns of the lane's own row. __syncwarp() after the last read.
+__device__ __forceinline__ void warp_place_rows(uint8_t* stg, int lane, const uint4 (&x)[4]) {
+#pragma unroll
+  for (int it = 0; it < 4; it++) *reinterpret_cast<uint4*>(stg + stage_offset(it * 8 + (lane >> 2), lane & 3)) = x[it];
+  __syncwarp();
+}
+__device__ __forceinline__ void own_chunk(const uint8_t* stg, int lane, int k, float (&x)[8]) {
+  const uint4 y = *reinterpret_cast<const uint4*>(stg + stage_offset(lane, k));
+  const __nv_bfloat162* yb = reinterpret_cast<const __nv_bfloat162*>(&y);
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    const float2 f = __bfloat1622float2(yb[e]);
+    x[2 * e] = f.x;
+    x[2 * e + 1] = f.y;
+  }
 }
 
 // out[j] (+)= the lane's own row of a bf16 tensor, fetched with the same coalesced pattern
