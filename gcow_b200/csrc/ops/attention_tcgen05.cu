@@ -12,13 +12,16 @@
 //            O = P V accumulates in the tensor-memory columns that S has vacated. exp(S - max)
 //            needs no running rescale because the whole row is present. Also stores the row's
 //            log2-sum-exp for the backward pass.
-//  backward  recomputes P from Q, K and the stored log-sum-exp.
-//     dK/dV  one CTA per (128 keys, head), loop over the query tiles: S and dP = dO V^T in tensor
-//            memory, P and dS = P (dP - delta) to shared memory in the MN-major layout so that
-//            P^T dO and dS^T Q need no transpose, dV and dK accumulate in tensor memory.
-//     dQ     one CTA per (128 queries, head), loop over the key tiles: same S, dP, dS, then
-//            dQ += dS K. Recomputing S and dP here instead of adding dQ with atomics keeps the
-//            gradients deterministic.
+//  backward  recomputes P from Q, K and the stored log-sum-exp, a 128 x 64 tile at a time.
+//     dK/dV  one CTA per (128 keys, head), loop over blocks of 64 queries: S^T = K Q^T and dP^T = V dO^T in
+//            tensor memory (one key per row, so lse and delta are per column, read from shared memory), P^T and
+//            dS^T = P^T (dP^T - delta) to shared memory as K-major operands, dV and dK accumulate in tensor memory.
+//     dQ     one CTA per (128 queries, head), loop over blocks of 64 keys: S, dP, dS, then dQ += dS K.
+//            Recomputing S and dP here instead of adding dQ with atomics keeps the gradients deterministic.
+//            The steps of one tile (products, exponentials, operands, products) follow one another, so what hides them
+//            is a second CTA on the SM: tiles of 64 keep a CTA within 256 tensor-memory columns and 113 KB of shared
+//            memory, where 128 x 128 tiles took 320 to 384 columns and 128 to 160 KB, one CTA per SM.
+//            512 x 32 sequences of 16 heads, both kernels and delta: 398 -> 337 us (dK/dV 206 -> 192, dQ 169 -> 133).
 //  delta = rowsum(dO * O) comes from a small elementwise kernel.
 //
 // 512 threads per CTA: four threads share an accumulator row (the four warps that may read a
@@ -42,6 +45,8 @@ constexpr int TILE = 128;             // rows of a query / key tile
 constexpr int TILE_BYTES = TILE * D * 2;   // 16 KB
 constexpr int MAX_S = 512;
 constexpr int NT = 512;               // threads per CTA: 4 column groups x 128 rows
+constexpr int STEP = 64;              // backward: queries / keys per loop step
+constexpr int STEP_BYTES = STEP * D * 2;   // 8 KB
 
 struct Params {
   __nv_bfloat16* out;      // forward: context [B][S][H][64]
@@ -90,30 +95,29 @@ __device__ __forceinline__ void store_kmajor32(uint8_t* tile, int row, int e0, c
     *reinterpret_cast<uint4*>(blk + sw128(row, j0 + j)) = o;
   }
 }
-// Store 32 consecutive values of this thread's row into an MN-major operand whose reduction index is the ROW
-// (this thread) and whose M/N index is the column: [k-block = row / 64][box = col / 64][row % 64][64 cols].
-__device__ __forceinline__ void store_mnmajor32(uint8_t* tile, int row, int c0, const float (&v)[32]) {
-  uint8_t* box = tile + (row >> 6) * 16384 + (c0 >> 6) * 8192;
-  const int r = row & 63, j0 = (c0 & 63) >> 3;
+// 16 values, elements e0..e0+15 of the row, of an operand with 64 elements per row.
+__device__ __forceinline__ void store_kmajor16(uint8_t* tile, int row, int e0, const float (&v)[16]) {
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
+  for (int j = 0; j < 2; j++) {
     uint4 o = make_uint4(pack2(v[8 * j], v[8 * j + 1]), pack2(v[8 * j + 2], v[8 * j + 3]),
                          pack2(v[8 * j + 4], v[8 * j + 5]), pack2(v[8 * j + 6], v[8 * j + 7]));
-    *reinterpret_cast<uint4*>(box + sw128(r, j0 + j)) = o;
+    *reinterpret_cast<uint4*>(tile + sw128(row, (e0 >> 3) + j)) = o;
   }
 }
 
+template <uint32_t COLS>
 __device__ __forceinline__ void tmem_alloc(Bars* bs, int warp) {
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bs->tmem_base)), "r"(512u) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bs->tmem_base)), "r"(COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
 }
+template <uint32_t COLS>
 __device__ __forceinline__ void tmem_free(uint32_t base, int warp) {
   if (warp == 0) {
     __syncwarp();
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(512u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(COLS) : "memory");
   }
 }
 // All MMAs issued by this thread have completed (bounded), so tensor memory and the operands may go.
@@ -152,7 +156,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
     bs->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  tmem_alloc(bs, warp);
+  tmem_alloc<512>(bs, warp);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -219,14 +223,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; j++) {
-          v[j] = exp2f(fmaf(__uint_as_float(ra[j]), p.scale_log2, -ms));
+          v[j] = ex2_ftz(fmaf(__uint_as_float(ra[j]), p.scale_log2, -ms));
           l += v[j];
         }
         store_kmajor32(sP, row, c0 * 32, v);
         if (two) {
 #pragma unroll
           for (int j = 0; j < 32; j++) {
-            v[j] = exp2f(fmaf(__uint_as_float(rb[j]), p.scale_log2, -ms));
+            v[j] = ex2_ftz(fmaf(__uint_as_float(rb[j]), p.scale_log2, -ms));
             l += v[j];
           }
           store_kmajor32(sP, row, (c0 + 1) * 32, v);
@@ -278,23 +282,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   if (tid == 0) drain(bs);
   tc_fence_before();
   __syncthreads();
-  tmem_free(tmem, warp);
+  tmem_free<512>(tmem, warp);
 }
 
-// delta[b][h][s] = sum_d dO[b][s][h][d] * O[b][s][h][d]; one thread per row.
+// delta[b][h][s] = sum_d dO[b][s][h][d] * O[b][s][h][d]; eight lanes per row, so that a warp reads whole lines (262 144
+// rows: 15 us, one thread per row took 24).
 __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ go,
                                   float* __restrict__ delta, int B, int S, int H) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;       // over b, s, h
-  if (i >= (size_t)B * S * H) return;
-  const int h = (int)(i % H);
-  const size_t bs = i / H;
-  const int s = (int)(bs % S), b = (int)(bs / S);
-  const uint4* po = reinterpret_cast<const uint4*>(o + i * D);
-  const uint4* pg = reinterpret_cast<const uint4*>(go + i * D);
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t i = t >> 3, rows = (size_t)B * S * H;                   // over b, s, h
+  const int part = (int)(t & 7);
   float acc = 0.0f;
-#pragma unroll
-  for (int k = 0; k < D / 8; k++) {
-    const uint4 x = po[k], y = pg[k];
+  if (i < rows) {
+    const uint4 x = reinterpret_cast<const uint4*>(o + i * D)[part], y = reinterpret_cast<const uint4*>(go + i * D)[part];
     const __nv_bfloat162* xb = reinterpret_cast<const __nv_bfloat162*>(&x);
     const __nv_bfloat162* yb = reinterpret_cast<const __nv_bfloat162*>(&y);
 #pragma unroll
@@ -303,33 +303,49 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
       acc = fmaf(a.x, c.x, fmaf(a.y, c.y, acc));
     }
   }
-  delta[((size_t)b * H + h) * S + s] = acc;
+#pragma unroll
+  for (int d = 1; d < 8; d <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+  if (i < rows && part == 0) {
+    const int h = (int)(i % H);
+    const size_t bs = i / H;
+    delta[((bs / S) * H + h) * S + bs % S] = acc;
+  }
 }
 
-// P and dS of one 128 x 128 tile from S (tensor-memory columns 0..127) and dP (columns 128..255): this thread's
-// row. WRITE_P: also emit P. MN: operands go to the MN-major layout (reduction over rows), else K-major.
-template <bool WRITE_P, bool MN>
-__device__ __forceinline__ void softmax_grad_tile(uint32_t lane_addr, int row, int c, float lse, float delta, const Params& p,
-                                                  uint8_t* sP, uint8_t* sdS) {
-  {                                          // this thread's 32-column chunk c of the row
-    uint32_t rs[32], rd[32];
-    tc_ld32(lane_addr + c * 32, rs);
-    tc_ld32(lane_addr + 128 + c * 32, rd);
-    tc_wait_ld();
-    float pv[32], ds[32];
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr) : "memory");
+}
+
+// P and dS of one 128 x 64 tile from S (tensor-memory columns 0..63) and dP (columns 64..127), this thread's row and
+// 16-column group c, as K-major operands. COLS: lse and delta belong to the columns (nlse / ndelta: their negatives for
+// this tile's columns in shared memory) and P is written too; else they are the row's (nlse[0], ndelta[0]).
+template <bool COLS>
+__device__ __forceinline__ void softmax_grad_tile(uint32_t lane_addr, int row, int c, const float* nlse, const float* ndelta,
+                                                  const Params& p, uint8_t* sP, uint8_t* sdS) {
+  uint32_t rs[16], rd[16];
+  tc_ld16(lane_addr + c * 16, rs);
+  tc_ld16(lane_addr + STEP + c * 16, rd);
+  tc_wait_ld();
+  float pv[16], ds[16];
+  const uint64_t sl = tc::pack2(p.scale_log2, p.scale_log2), sc = tc::pack2(p.scale, p.scale), one = tc::pack2(1.0f, 1.0f);
 #pragma unroll
-    for (int j = 0; j < 32; j++) {
-      pv[j] = exp2f(fmaf(__uint_as_float(rs[j]), p.scale_log2, -lse));
-      ds[j] = pv[j] * (__uint_as_float(rd[j]) - delta) * p.scale;
-    }
-    if (MN) {
-      if (WRITE_P) store_mnmajor32(sP, row, c * 32, pv);
-      store_mnmajor32(sdS, row, c * 32, ds);
-    } else {
-      if (WRITE_P) store_kmajor32(sP, row, c * 32, pv);
-      store_kmajor32(sdS, row, c * 32, ds);
-    }
+  for (int j = 0; j < 16; j += 2) {
+    const uint64_t nl = COLS ? *reinterpret_cast<const uint64_t*>(nlse + c * 16 + j) : tc::pack2(nlse[0], nlse[0]);
+    const uint64_t nd = COLS ? *reinterpret_cast<const uint64_t*>(ndelta + c * 16 + j) : tc::pack2(ndelta[0], ndelta[0]);
+    float a, b;
+    unpack2(fma2(tc::pack2(__uint_as_float(rs[j]), __uint_as_float(rs[j + 1])), sl, nl), a, b);
+    pv[j] = ex2_ftz(a);
+    pv[j + 1] = ex2_ftz(b);
+    const uint64_t d = fma2(tc::pack2(__uint_as_float(rd[j]), __uint_as_float(rd[j + 1])), one, nd);
+    unpack2(mul2(mul2(tc::pack2(pv[j], pv[j + 1]), d), sc), ds[j], ds[j + 1]);
   }
+  if (COLS) store_kmajor16(sP, row, c * 16, pv);
+  store_kmajor16(sdS, row, c * 16, ds);
 }
 
 // Write this thread's row of a 64-column fp32 accumulator (tensor-memory column `col`) as bf16 to `dst`.
@@ -350,22 +366,24 @@ __device__ __forceinline__ void store_acc_row(uint32_t lane_addr, int col, int c
 }
 
 // ------------------------------------------------------------------- backward: dK and dV
-__global__ void __launch_bounds__(NT, 1)
+__global__ void __launch_bounds__(NT, 2)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                      const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo, const Params p) {
   extern __shared__ uint8_t raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sK = base;                        // 16 KB each
   uint8_t* sV = sK + TILE_BYTES;
-  uint8_t* sQ = sV + TILE_BYTES;             // two buffers
-  uint8_t* sdO = sQ + 2 * TILE_BYTES;        // two buffers
-  uint8_t* sP = sdO + 2 * TILE_BYTES;        // 32 KB, MN-major
-  uint8_t* sdS = sP + 2 * TILE_BYTES;        // 32 KB, MN-major
-  Bars* bs = reinterpret_cast<Bars*>(sdS + 2 * TILE_BYTES);
+  uint8_t* sP = sV + TILE_BYTES;             // P^T, dS^T: [128 keys][64 queries]
+  uint8_t* sdS = sP + TILE_BYTES;
+  uint8_t* sQ = sdS + TILE_BYTES;            // two buffers of 8 KB each
+  uint8_t* sdO = sQ + 2 * STEP_BYTES;
+  float* nlse = reinterpret_cast<float*>(sdO + 2 * STEP_BYTES);      // -lse and -delta of every query
+  float* ndelta = nlse + MAX_S;
+  Bars* bs = reinterpret_cast<Bars*>(ndelta + MAX_S);
   const int tid = threadIdx.x, warp = tid >> 5;
   const int row = (warp & 3) * 32 + (tid & 31), cg = warp >> 2;
   const int k0 = blockIdx.x * TILE, h = blockIdx.y, b = blockIdx.z;
-  const int nq = p.S / TILE;
+  const int nq = p.S / STEP;
 
   if (tid == 0) {
     mbar_init(&bs->a, 1); mbar_init(&bs->c, 1); mbar_init(&bs->d, 1); mbar_init(&bs->drain, 1);
@@ -373,72 +391,72 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
     bs->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  tmem_alloc(bs, warp);
+  static_assert(MAX_S <= NT, "one query's statistics per thread");
+  if (tid < p.S) {
+    const size_t stat = ((size_t)b * p.H + h) * p.S + tid;
+    nlse[tid] = -p.lse[stat];
+    ndelta[tid] = -p.delta[stat];
+  }
+  tmem_alloc<256>(bs, warp);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bs->tmem_base;
   const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-  constexpr uint32_t COL_S = 0, COL_DV = 256, COL_DK = 320;      // dP sits at COL_S + 128
+  constexpr uint32_t COL_S = 0, COL_DV = 128, COL_DK = 192;      // dP^T sits at COL_S + 64
   bool ok = true;
 
   if (tid == 0) {
     mbar_expect_tx(&bs->a, 2 * TILE_BYTES);
     tma_load_4d(smem_u32(sK), &tk, smem_u32(&bs->a), 0, h, k0, b);
     tma_load_4d(smem_u32(sV), &tv, smem_u32(&bs->a), 0, h, k0, b);
-    mbar_expect_tx(&bs->e[0], 2 * TILE_BYTES);
+    mbar_expect_tx(&bs->e[0], 2 * STEP_BYTES);
     tma_load_4d(smem_u32(sQ), &tq, smem_u32(&bs->e[0]), 0, h, 0, b);
     tma_load_4d(smem_u32(sdO), &tdo, smem_u32(&bs->e[0]), 0, h, 0, b);
     ok = wait(bs, &bs->a, 0, p.error, 31);
   }
   for (int i = 0; i < nq; i++) {
     const int buf = i & 1;
-    uint8_t* q = sQ + buf * TILE_BYTES;
-    uint8_t* go = sdO + buf * TILE_BYTES;
+    uint8_t* q = sQ + buf * STEP_BYTES;
+    uint8_t* go = sdO + buf * STEP_BYTES;
     if (tid == 0 && ok) {
-      // the other buffer was last read by the MMAs of iteration i-1, whose completion (bar d) is awaited
-      // below before this point is reached again; start fetching tile i+1 into it now
-      if (i + 1 < nq) {
-        if (i >= 1) ok = wait(bs, &bs->d, (i - 1) & 1, p.error, 32);
-        if (ok) {
-          mbar_expect_tx(&bs->e[buf ^ 1], 2 * TILE_BYTES);
-          tma_load_4d(smem_u32(sQ + (buf ^ 1) * TILE_BYTES), &tq, smem_u32(&bs->e[buf ^ 1]), 0, h, (i + 1) * TILE, b);
-          tma_load_4d(smem_u32(sdO + (buf ^ 1) * TILE_BYTES), &tdo, smem_u32(&bs->e[buf ^ 1]), 0, h, (i + 1) * TILE, b);
-        }
-      }
-      ok = ok && wait(bs, &bs->e[buf], (i >> 1) & 1, p.error, 33);
+      // S and dP of this step right behind the products of the last one, whose end nothing here waits for
+      ok = wait(bs, &bs->e[buf], (i >> 1) & 1, p.error, 33);
       if (ok) {
         tc_fence_after();
-        mma_kk(tmem + COL_S, smem_u32(q), smem_u32(sK), TILE, false);            // S  = Q_i K_j^T
-        mma_kk(tmem + COL_S + 128, smem_u32(go), smem_u32(sV), TILE, false);     // dP = dO_i V_j^T
+        mma_kk(tmem + COL_S, smem_u32(sK), smem_u32(q), STEP, false);            // S^T  = K_j Q_i^T
+        mma_kk(tmem + COL_S + STEP, smem_u32(sV), smem_u32(go), STEP, false);    // dP^T = V_j dO_i^T
         tc_commit(&bs->c);
       }
+      // the other buffer was last read by the MMAs of step i-1; once they are done, block i+1 is fetched into it
+      if (ok && i + 1 < nq) {
+        if (i >= 1) ok = wait(bs, &bs->d, (i - 1) & 1, p.error, 32);
+        if (ok) {
+          mbar_expect_tx(&bs->e[buf ^ 1], 2 * STEP_BYTES);
+          tma_load_4d(smem_u32(sQ + (buf ^ 1) * STEP_BYTES), &tq, smem_u32(&bs->e[buf ^ 1]), 0, h, (i + 1) * STEP, b);
+          tma_load_4d(smem_u32(sdO + (buf ^ 1) * STEP_BYTES), &tdo, smem_u32(&bs->e[buf ^ 1]), 0, h, (i + 1) * STEP, b);
+        }
+      }
     }
-    const size_t stat = ((size_t)b * p.H + h) * p.S + i * TILE + row;
-    const float lse = p.lse[stat], delta = p.delta[stat];
-    ok = wait(bs, &bs->c, i & 1, p.error, 34);
+    ok = ok && wait(bs, &bs->c, i & 1, p.error, 34);
     // P / dS of iteration i-1 must have been consumed by its MMAs before they are overwritten
     if (i >= 1) ok = ok && wait(bs, &bs->d, (i - 1) & 1, p.error, 35);
     ok = __syncthreads_and(ok);
     if (!ok) break;
     tc_fence_after();
-    softmax_grad_tile<true, true>(lane_addr + COL_S, row, cg, lse, delta, p, sP, sdS);
+    softmax_grad_tile<true>(lane_addr + COL_S, row, cg, nlse + i * STEP, ndelta + i * STEP, p, sP, sdS);
     proxy_fence();
     tc_fence_before();
     __syncthreads();
     if (tid == 0) {
       tc_fence_after();
-      const uint32_t id = idesc_f16(D, true, true);                 // A = P^T / dS^T (MN-major), B = dO / Q as [q][d]
-      for (int kb = 0; kb < 2; kb++) {
-        const uint64_t dap = smem_desc_mn_sw128(smem_u32(sP + kb * 16384));
-        const uint64_t dad = smem_desc_mn_sw128(smem_u32(sdS + kb * 16384));
-        const uint64_t dbo = smem_desc_mn_sw128(smem_u32(go + kb * 8192));
-        const uint64_t dbq = smem_desc_mn_sw128(smem_u32(q + kb * 8192));
+      const uint32_t id = idesc_f16(D, false, true);                // A = P^T / dS^T (K-major), B = dO / Q as [q][d]
+      const uint64_t dap = smem_desc_sw128(smem_u32(sP)), dad = smem_desc_sw128(smem_u32(sdS));
+      const uint64_t dbo = smem_desc_mn_sw128(smem_u32(go)), dbq = smem_desc_mn_sw128(smem_u32(q));
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-          tc_mma(tmem + COL_DV, dap + (2048 >> 4) * k, dbo + (2048 >> 4) * k, id, (i | kb | k) != 0);
-          tc_mma(tmem + COL_DK, dad + (2048 >> 4) * k, dbq + (2048 >> 4) * k, id, (i | kb | k) != 0);
-        }
+      for (int k = 0; k < 4; k++) {
+        tc_mma(tmem + COL_DV, dap + 2 * k, dbo + (2048 >> 4) * k, id, (i | k) != 0);
+        tc_mma(tmem + COL_DK, dad + 2 * k, dbq + (2048 >> 4) * k, id, (i | k) != 0);
       }
       tc_commit(&bs->d);
     }
@@ -454,25 +472,25 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
   if (tid == 0) drain(bs);
   tc_fence_before();
   __syncthreads();
-  tmem_free(tmem, warp);
+  tmem_free<256>(tmem, warp);
 }
 
 // ------------------------------------------------------------------------ backward: dQ
-__global__ void __launch_bounds__(NT, 1)
+__global__ void __launch_bounds__(NT, 2)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                    const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo, const Params p) {
   extern __shared__ uint8_t raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = base;
   uint8_t* sdO = sQ + TILE_BYTES;
-  uint8_t* sK = sdO + TILE_BYTES;            // two buffers
-  uint8_t* sV = sK + 2 * TILE_BYTES;         // two buffers
-  uint8_t* sdS = sV + 2 * TILE_BYTES;        // 32 KB, K-major: [128 queries][128 keys] as two 64-key blocks
-  Bars* bs = reinterpret_cast<Bars*>(sdS + 2 * TILE_BYTES);
+  uint8_t* sdS = sdO + TILE_BYTES;           // [128 queries][64 keys]
+  uint8_t* sK = sdS + TILE_BYTES;            // two buffers of 8 KB each
+  uint8_t* sV = sK + 2 * STEP_BYTES;
+  Bars* bs = reinterpret_cast<Bars*>(sV + 2 * STEP_BYTES);
   const int tid = threadIdx.x, warp = tid >> 5;
   const int row = (warp & 3) * 32 + (tid & 31), cg = warp >> 2;
   const int q0 = blockIdx.x * TILE, h = blockIdx.y, b = blockIdx.z;
-  const int nkv = p.S / TILE;
+  const int nkv = p.S / STEP;
 
   if (tid == 0) {
     mbar_init(&bs->a, 1); mbar_init(&bs->c, 1); mbar_init(&bs->d, 1); mbar_init(&bs->drain, 1);
@@ -480,65 +498,62 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
     bs->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  tmem_alloc(bs, warp);
+  tmem_alloc<256>(bs, warp);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bs->tmem_base;
   const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-  constexpr uint32_t COL_S = 0, COL_DQ = 256;
+  constexpr uint32_t COL_S = 0, COL_DQ = 128;
   bool ok = true;
   const size_t stat = ((size_t)b * p.H + h) * p.S + q0 + row;
-  const float lse = p.lse[stat], delta = p.delta[stat];
+  const float nlse = -p.lse[stat], ndelta = -p.delta[stat];
 
   if (tid == 0) {
     mbar_expect_tx(&bs->a, 2 * TILE_BYTES);
     tma_load_4d(smem_u32(sQ), &tq, smem_u32(&bs->a), 0, h, q0, b);
     tma_load_4d(smem_u32(sdO), &tdo, smem_u32(&bs->a), 0, h, q0, b);
-    mbar_expect_tx(&bs->e[0], 2 * TILE_BYTES);
+    mbar_expect_tx(&bs->e[0], 2 * STEP_BYTES);
     tma_load_4d(smem_u32(sK), &tk, smem_u32(&bs->e[0]), 0, h, 0, b);
     tma_load_4d(smem_u32(sV), &tv, smem_u32(&bs->e[0]), 0, h, 0, b);
     ok = wait(bs, &bs->a, 0, p.error, 41);
   }
   for (int j = 0; j < nkv; j++) {
     const int buf = j & 1;
-    uint8_t* kt = sK + buf * TILE_BYTES;
-    uint8_t* vt = sV + buf * TILE_BYTES;
+    uint8_t* kt = sK + buf * STEP_BYTES;
+    uint8_t* vt = sV + buf * STEP_BYTES;
     if (tid == 0 && ok) {
-      if (j + 1 < nkv) {
-        if (j >= 1) ok = wait(bs, &bs->d, (j - 1) & 1, p.error, 42);      // K of tile j-1 is still read by its dQ MMAs
-        if (ok) {
-          mbar_expect_tx(&bs->e[buf ^ 1], 2 * TILE_BYTES);
-          tma_load_4d(smem_u32(sK + (buf ^ 1) * TILE_BYTES), &tk, smem_u32(&bs->e[buf ^ 1]), 0, h, (j + 1) * TILE, b);
-          tma_load_4d(smem_u32(sV + (buf ^ 1) * TILE_BYTES), &tv, smem_u32(&bs->e[buf ^ 1]), 0, h, (j + 1) * TILE, b);
-        }
-      }
-      ok = ok && wait(bs, &bs->e[buf], (j >> 1) & 1, p.error, 43);
+      ok = wait(bs, &bs->e[buf], (j >> 1) & 1, p.error, 43);                     // the order of the steps: as above
       if (ok) {
         tc_fence_after();
-        mma_kk(tmem + COL_S, smem_u32(sQ), smem_u32(kt), TILE, false);           // S  = Q_i K_j^T
-        mma_kk(tmem + COL_S + 128, smem_u32(sdO), smem_u32(vt), TILE, false);    // dP = dO_i V_j^T
+        mma_kk(tmem + COL_S, smem_u32(sQ), smem_u32(kt), STEP, false);           // S  = Q_i K_j^T
+        mma_kk(tmem + COL_S + STEP, smem_u32(sdO), smem_u32(vt), STEP, false);   // dP = dO_i V_j^T
         tc_commit(&bs->c);
       }
+      if (ok && j + 1 < nkv) {
+        if (j >= 1) ok = wait(bs, &bs->d, (j - 1) & 1, p.error, 42);             // K of block j-1 is still read by its dQ MMAs
+        if (ok) {
+          mbar_expect_tx(&bs->e[buf ^ 1], 2 * STEP_BYTES);
+          tma_load_4d(smem_u32(sK + (buf ^ 1) * STEP_BYTES), &tk, smem_u32(&bs->e[buf ^ 1]), 0, h, (j + 1) * STEP, b);
+          tma_load_4d(smem_u32(sV + (buf ^ 1) * STEP_BYTES), &tv, smem_u32(&bs->e[buf ^ 1]), 0, h, (j + 1) * STEP, b);
+        }
+      }
     }
-    ok = wait(bs, &bs->c, j & 1, p.error, 44);
+    ok = ok && wait(bs, &bs->c, j & 1, p.error, 44);
     if (j >= 1) ok = ok && wait(bs, &bs->d, (j - 1) & 1, p.error, 45);           // dS of tile j-1 consumed
     ok = __syncthreads_and(ok);
     if (!ok) break;
     tc_fence_after();
-    softmax_grad_tile<false, false>(lane_addr + COL_S, row, cg, lse, delta, p, nullptr, sdS);
+    softmax_grad_tile<false>(lane_addr + COL_S, row, cg, &nlse, &ndelta, p, nullptr, sdS);
     proxy_fence();
     tc_fence_before();
     __syncthreads();
     if (tid == 0) {
       tc_fence_after();
       const uint32_t id = idesc_f16(D, false, true);                // A = dS (K-major), B = K_j as [key][d] (MN-major)
-      for (int blk = 0; blk < 2; blk++) {
-        const uint64_t da = smem_desc_sw128(smem_u32(sdS + blk * TILE_BYTES));
-        const uint64_t db = smem_desc_mn_sw128(smem_u32(kt + blk * 8192));
+      const uint64_t da = smem_desc_sw128(smem_u32(sdS)), db = smem_desc_mn_sw128(smem_u32(kt));
 #pragma unroll
-        for (int k = 0; k < 4; k++) tc_mma(tmem + COL_DQ, da + 2 * k, db + (2048 >> 4) * k, id, (j | blk | k) != 0);
-      }
+      for (int k = 0; k < 4; k++) tc_mma(tmem + COL_DQ, da + 2 * k, db + (2048 >> 4) * k, id, (j | k) != 0);
       tc_commit(&bs->d);
     }
   }
@@ -552,13 +567,13 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant
   if (tid == 0) drain(bs);
   tc_fence_before();
   __syncthreads();
-  tmem_free(tmem, warp);
+  tmem_free<256>(tmem, warp);
 }
 
 // ------------------------------------------------------------------------------ host side
 // One of Q / K / V inside qkv [B][S][3][H][64] (which = 0, 1, 2), or a plain [B][S][H][64] tensor (which = -1):
-// dims {d, h, s, b}, box = 64 x 1 x 128 x 1 (128 rows of one head).
-static int make_map(CUtensorMap* map, const void* ptr, int B, int S, int H, int which) {
+// dims {d, h, s, b}, box = 64 x 1 x rows x 1 (that many rows of one head).
+static int make_map(CUtensorMap* map, const void* ptr, int B, int S, int H, int which, int rows) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return -10;
   const uint64_t row = (which >= 0 ? 3ull : 1ull) * H * D;          // elements between consecutive sequence positions
@@ -566,7 +581,7 @@ static int make_map(CUtensorMap* map, const void* ptr, int B, int S, int H, int 
   if ((uintptr_t)basep & 15) return -11;
   cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)S, (cuuint64_t)B};
   cuuint64_t strides[3] = {(cuuint64_t)D * 2, row * 2, row * 2 * (cuuint64_t)S};
-  cuuint32_t box[4] = {(cuuint32_t)D, 1, (cuuint32_t)TILE, 1};
+  cuuint32_t box[4] = {(cuuint32_t)D, 1, (cuuint32_t)rows, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<char*>(basep), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -579,8 +594,9 @@ static int make_map(CUtensorMap* map, const void* ptr, int B, int S, int H, int 
 }
 
 constexpr size_t kFwdSmem = TILE_BYTES * 13 + sizeof(Bars) + 1024;      // Q + 4 K + 4 V + 4 P
-constexpr size_t kBwdSmem = TILE_BYTES * 10 + sizeof(Bars) + 1024;      // K, V, 2 Q, 2 dO, P (2), dS (2)
-constexpr size_t kDqSmem = TILE_BYTES * 8 + sizeof(Bars) + 1024;        // Q, dO, 2 K, 2 V, dS (2)
+constexpr size_t kBwdSmem = TILE_BYTES * 4 + STEP_BYTES * 4 + MAX_S * 8 + sizeof(Bars) + 1024;      // K, V, P, dS, 2 Q, 2 dO, statistics
+constexpr size_t kDqSmem = TILE_BYTES * 3 + STEP_BYTES * 4 + sizeof(Bars) + 1024;                    // Q, dO, dS, 2 K, 2 V
+static_assert(kBwdSmem <= 112 * 1024 && kDqSmem <= 112 * 1024, "two CTAs per SM");
 
 static int check_shape(int B, int S, int H, int d) {
   if (d != D || S % TILE || S <= 0 || S > MAX_S || B <= 0 || H <= 0 || H > 65535 || B > 65535) return -1;
@@ -614,7 +630,7 @@ int gcow_attention_fwd(const void* qkv, void* out, float* lse, int B, int S, int
   set_attrs();
   CUtensorMap tq, tk, tv;
   int rc;
-  if ((rc = make_map(&tq, qkv, B, S, H, 0)) || (rc = make_map(&tk, qkv, B, S, H, 1)) || (rc = make_map(&tv, qkv, B, S, H, 2)))
+  if ((rc = make_map(&tq, qkv, B, S, H, 0, TILE)) || (rc = make_map(&tk, qkv, B, S, H, 1, TILE)) || (rc = make_map(&tv, qkv, B, S, H, 2, TILE)))
     return rc;
   Params p = {};
   p.out = (__nv_bfloat16*)out; p.lse = lse; p.B = B; p.S = S; p.H = H;
@@ -628,19 +644,20 @@ int gcow_attention_bwd(const void* qkv, const void* out, const void* dout, const
                        int B, int S, int H, int d, float scale, uint32_t* error, void* stream) {
   if (check_shape(B, S, H, d)) return -1;
   set_attrs();
-  CUtensorMap tq, tk, tv, tdo;
-  int rc;
-  if ((rc = make_map(&tq, qkv, B, S, H, 0)) || (rc = make_map(&tk, qkv, B, S, H, 1)) || (rc = make_map(&tv, qkv, B, S, H, 2)) ||
-      (rc = make_map(&tdo, dout, B, S, H, -1)))
-    return rc;
+  CUtensorMap tile[4], step[4];                              // Q, K, V, dO in boxes of TILE and of STEP rows
+  for (int i = 0; i < 4; i++) {
+    const void* const m = i < 3 ? qkv : dout;
+    int rc;
+    if ((rc = make_map(&tile[i], m, B, S, H, i < 3 ? i : -1, TILE)) || (rc = make_map(&step[i], m, B, S, H, i < 3 ? i : -1, STEP))) return rc;
+  }
   cudaStream_t st = (cudaStream_t)stream;
   const size_t rows = (size_t)B * S * H;
-  attn_delta_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, delta, B, S, H);
+  attn_delta_kernel<<<(unsigned)((rows * 8 + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, delta, B, S, H);
   Params p = {};
   p.lse = const_cast<float*>(lse); p.delta = delta; p.dqkv = (__nv_bfloat16*)dqkv; p.B = B; p.S = S; p.H = H;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.error = error;
-  attn_bwd_dkdv_kernel<<<dim3(S / TILE, H, B), NT, kBwdSmem, st>>>(tq, tk, tv, tdo, p);
-  attn_bwd_dq_kernel<<<dim3(S / TILE, H, B), NT, kDqSmem, st>>>(tq, tk, tv, tdo, p);
+  attn_bwd_dkdv_kernel<<<dim3(S / TILE, H, B), NT, kBwdSmem, st>>>(step[0], tile[1], tile[2], step[3], p);
+  attn_bwd_dq_kernel<<<dim3(S / TILE, H, B), NT, kDqSmem, st>>>(tile[0], step[1], step[2], tile[3], p);
   return (int)cudaGetLastError();
 }
 

@@ -1,0 +1,70 @@
+"""Epilogues of the CTA-pair GEMM and the fused attention against float64, at the edges of their tiles."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, b):
+    return ((a.double() - b).norm() / b.norm()).item()
+
+
+@pytest.mark.parametrize("M", [1024, 1025, 1100, 1279])
+@pytest.mark.parametrize("N", [256, 288, 320])
+def test_side_operands(M, N):
+    """Residual, GELU with its argument kept, GELU' and GELU' + residual. Rows that end inside a warp's 32 and inside a
+    tile, columns that end inside a warp's 128. One rounding to bf16 is at most 2^-9 of a value; the float32 sums are
+    far below that."""
+    from gcow_b200.ops import kernels as K
+    torch.manual_seed(M + N)
+    a = torch.randn(M, 512, device="cuda").bfloat16()
+    w = (torch.randn(N, 512, device="cuda") / 16).bfloat16()
+    bias = torch.randn(N, device="cuda")
+    x = torch.randn(M, N, device="cuda").bfloat16() * 2
+    p = a.double() @ w.double().T
+    xd = x.double()
+    cdf = 0.5 * (1 + torch.erf(xd / math.sqrt(2)))
+    dgelu = cdf + xd * torch.exp(-xd * xd / 2) / math.sqrt(2 * math.pi)
+    assert _rel(K.gemm_bf16(a, w, residual=x), p + xd) < 2 ** -9
+    assert _rel(K.gemm_bf16(a, w, gelu_grad_of=x), p * dgelu) < 2 ** -9
+    assert _rel(K.gemm_bf16(a, w, gelu_grad_of=x, residual=x), p * dgelu + xd) < 2 ** -9
+    pre = torch.empty_like(x)
+    y = K.gemm_bf16(a, w, bias=bias, gelu=True, pre_gelu_out=pre, residual=x)
+    z = p + bias.double()
+    assert _rel(pre, z) < 2 ** -9
+    assert _rel(y, z * 0.5 * (1 + torch.erf(z / math.sqrt(2))) + xd) < 2 ** -9
+
+
+def test_gelu_of_special_values():
+    """0, both infinities, NaN and the underflow range of exp(-x^2 / 2), through an identity weight, one value per row."""
+    from gcow_b200.ops import kernels as K
+    v = torch.tensor([0.0, 20.0, -20.0, 13.2, -13.2, -14.0, 1e-30, -1e-30, 3e38, -3e38], device="cuda").bfloat16()
+    x = torch.zeros(64, 64, device="cuda", dtype=torch.bfloat16)
+    x[:v.numel(), 0] = v
+    y = K.gemm_bf16(x, torch.eye(64, device="cuda", dtype=torch.bfloat16), gelu=True, out_dtype=torch.float32)[:v.numel(), 0].double()
+    d = v.double()
+    want = d * 0.5 * torch.erfc(-d / math.sqrt(2))
+    # |Phi| is off by at most 1.5e-7 / 2, and by two roundings
+    assert bool(((y - want).abs() <= d.abs() * 3e-7).all())
+    x[0, 0] = float("nan")
+    assert math.isnan(K.gemm_bf16(x, torch.eye(64, device="cuda", dtype=torch.bfloat16), gelu=True)[0, 0].item())
+
+
+@pytest.mark.parametrize("B,S,H", [(1, 128, 1), (2, 256, 3), (1, 384, 2), (3, 512, 4)])
+def test_attention(B, S, H):
+    """Forward and backward. Two roundings to bf16 on each path (P or dS, and the result): below 2^-8 of the norm."""
+    from gcow_b200.ops import kernels as K
+    torch.manual_seed(S)
+    qkv = torch.randn(B, S, 3, H, 64, device="cuda").bfloat16().requires_grad_(True)
+    o = K.fused_attention(qkv)
+    go = torch.randn_like(o)
+    o.backward(go)
+    r = qkv.detach().double().requires_grad_(True)
+    q, k, v = (r[:, :, i].permute(0, 2, 1, 3) for i in range(3))
+    ref = (torch.softmax(q @ k.transpose(-1, -2) / 8, -1) @ v).permute(0, 2, 1, 3).reshape(B, S, H * 64)
+    ref.backward(go.double())
+    assert _rel(o, ref.detach()) < 2 ** -8
+    for i in range(3):
+        assert _rel(qkv.grad[:, :, i], r.grad[:, :, i]) < 2 ** -8
