@@ -20,7 +20,7 @@
 #include <thread>
 #include <vector>
 
-#include "zfp_block.cuh"
+#include "tile_coder.cuh"
 
 namespace {
 
@@ -455,6 +455,27 @@ const gcow::LeanTables& host_lean_tables() {
   return h.t;
 }
 }  // namespace
+
+// The tile kernels' 1-D decoder against the plane-by-plane one on `blocks` blocks of `stride` words each (an even number),
+// starting `skip` bits in: the number of blocks decoded differently.
+int64_t gcow_window_decode_check(const uint32_t* words, uint64_t blocks, uint32_t stride, uint32_t skip, const int32_t* params) {
+  const gcow::LeanTables& lt = host_lean_tables();
+  const gcow::ZfpParams p = {(uint32_t)params[0], (uint32_t)params[1], (uint32_t)params[2], params[3]};
+  std::vector<uint32_t> tab(lt.dloop, lt.dloop + gcow::kTileRows);
+  tab.resize(gcow::kTileDecTab1);
+  for (uint32_t i = 0; i < 384; i++) reinterpret_cast<gcow::DecWindow*>(tab.data() + gcow::kTileRows)[i] = gcow::make_tile_row(lt.dtab, i);
+  int64_t bad = 0;
+  for (uint64_t b = 0; b < blocks; b++) {
+    float x[4], y[4];
+    gcow::decode_window_1d(x, p, tab.data(), lt.dtab, words + b * stride, skip, 1);
+    std::vector<uint64_t> w(stride / 2);
+    memcpy(w.data(), words + b * stride, stride * 4);
+    gcow::WordSrc src(w.data(), skip);
+    gcow::decode_block<1>(y, p, src, 1);
+    bad += memcmp(x, y, 16) != 0;
+  }
+  return bad;
+}
 
 // Fixed accuracy with a bit cap through the lean coders (as the sparse all-reduce kernel uses them) against the
 // definition path: out = D(E(x)) from the lean pair, and the return value counts the blocks whose result differs from

@@ -350,9 +350,18 @@ struct WindowReader {
   }
 };
 
-// One block of 4 from a window. `rows`: rows n = 0..2 of the decoder loop table for a remaining budget of seven
-// bits or more, 128 entries each (plane | used << 8 | (n' * 4096) << 16).
-GCOW_HD void decode_window_1d(float* f, const ZfpParams& p, const uint32_t* rows, const uint32_t* words, uint32_t pos, int shift) {
+// One block of 4 from a window. `tab`: the lean coder's decoder windows and nibble pairs, then at kTileRows one plane per
+// lookup in the same form (rows n = 0..2 of 128 entries, the next seven bits) for where a window would run past the last
+// plane or the budget; `dtab`: the decoder's budget table, for the last bits of a budget (may be global memory). Planes gather
+// in U, byte i those of coefficient i; once n >= 3 the rest is verbatim nibbles, two per lookup.
+constexpr int kTileRows = kDecTiny, kTileDecTab1 = kTileRows + 3 * 128 * 2;
+// Entry i (0..383) of the one-plane rows, from the decoder's budget table.
+GCOW_HD DecWindow make_tile_row(const uint16_t* dtab, uint32_t i) {
+  const uint32_t e = dtab[((i >> 7) * 8 + 7) * 128 + (i & 127)], n = e >> 7;
+  return {spread_nibble(e & 15u), ((e >> 4) & 7u) | (1u << 8) | ((n < 3 ? n : 3u) << 12)};
+}
+GCOW_HD void decode_window_1d(float* f, const ZfpParams& p, const uint32_t* tab, const uint16_t* dtab, const uint32_t* words,
+                              uint32_t pos, int shift) {
   WindowReader src(words, pos);
   const uint32_t head = src.peek();
   if (!(head & 1u)) {
@@ -360,49 +369,66 @@ GCOW_HD void decode_window_1d(float* f, const ZfpParams& p, const uint32_t* rows
     return;
   }
   const int emax = (int)((head >> 1) & 0xffu) - kEBias;
-  const uint32_t prec = block_precision(emax, p.maxprec, p.minexp, 1);
-  uint32_t left = prec < 32u ? prec : 32u;                 // planes to come
-  const uint32_t kmin = 32 - left;
+  const uint32_t prec = block_precision(emax, p.maxprec, p.minexp, 1), planes = prec < 32u ? prec : 32u;
   uint32_t bits = p.maxbits - kHeaderBits;                 // budget left
   src.skip(kHeaderBits);
-  uint32_t n = 0;
+  const uint32_t S = src.peek();                           // leading all-zero planes
+  uint32_t z = S ? (uint32_t)ctz32(S) : 32u;
+  if (z > planes) z = planes;
+  if (z > bits) z = bits;
+  src.skip(z);
+  bits -= z;
+  const uint32_t* const nib = tab + kDecNibbles;
   uint32_t u[4] = {0, 0, 0, 0};
-  {                                                        // leading all-zero planes
-    const uint32_t S = src.peek();
-    uint32_t z = S ? (uint32_t)ctz32(S) : 32u;
-    if (z > left) z = left;
-    if (z > bits) z = bits;
-    src.skip(z);
-    bits -= z;
-    left -= z;
-  }
-  while (left && bits) {
-    const uint32_t k = kmin + left, cnt = left < 8 ? left : 8;
-    uint32_t T = 0, j = 0;
-    while (n < 3 && j < 4 * cnt && bits >= 7) {
-      const uint32_t e = rows[n * 128u + (src.peek() & 127u)];
-      const uint32_t used = (e >> 8) & 0xffu;
-      T |= (e & 15u) << j;
+  uint32_t U = 0, held = 0, gone = z, row = 0;             // planes in U; planes above the next one; min(n, 3) * 4096
+  auto flush = [&]() {                                     // U to its place: the planes down to 32 - gone
+    const uint32_t m = pow2_factor(32u - gone);
+    u[0] += (U & 0xffu) * m; u[1] += ((U >> 8) & 0xffu) * m; u[2] += ((U >> 16) & 0xffu) * m; u[3] += (U >> 24) * m;
+    U = held = 0;
+  };
+  while (row != 0x3000u && gone < planes && bits) {
+    if (held > 3) flush();                                 // at most seven planes: the tail wants the bytes' top bits clear
+    const bool wide = planes - gone >= 4 && bits >= 9;     // a window holds at most four planes and nine bits
+    if (wide || bits >= 7) {
+      const uint32_t v = src.peek(), at = wide ? row + 8u * (v & 511u) : kTileRows * 4u + (row >> 2) + 8u * (v & 127u);
+      const DecWindow d = *reinterpret_cast<const DecWindow*>(reinterpret_cast<const char*>(tab) + at);
+      const uint32_t n = (d.meta >> 8) & 15u, used = d.meta & 31u;
+      U = (U << n) | d.u;
+      held += n;
+      gone += n;
       src.skip(used);
       bits -= used;
-      n = e >> 28;
-      j += 4;
+      row = d.meta & 0x3000u;
+    } else {                                               // the budget may end inside this plane
+      const uint32_t e = dtab[(((row >> 12) * 8 + bits) << 7) + (src.peek() & low_mask32(bits))], used = (e >> 4) & 7u, n = e >> 7;
+      U = 2 * U + (nib[e & 15u] >> 1);
+      held++;
+      gone++;
+      src.skip(used);
+      bits -= used;
+      row = (n < 3 ? n : 3u) << 12;
     }
-    if (n >= 3 && j < 4 * cnt) {                           // verbatim nibbles
-      // A nibble cut by the budget after its first three bits: with n == 3 the missing bit is a group test that
-      // reads as 0, with n == 4 a verbatim bit that reads as 0 - the same nibble.
-      const uint32_t want = 4 * cnt - j, take = want < bits ? want : bits;
-      T |= (src.peek() & low_mask32(take)) << j;
-      src.skip(take);
-      bits -= take;
-      j = 4 * cnt;
+  }
+  // A nibble cut by the budget after its first three bits: with n == 3 the missing bit is a group test that reads as 0,
+  // with n == 4 a verbatim bit that reads as 0 - the same nibble.
+  const uint32_t want = 4 * (planes - gone), tail = want < bits ? want : bits;
+  if (tail | U) {
+    const uint32_t t = src.peek() & low_mask32(tail);
+    const uint32_t W = ((nib[t & 255u] * 4u + nib[(t >> 8) & 255u]) * 4u + nib[(t >> 16) & 255u]) * 4u + nib[t >> 24];
+    const uint32_t m = gone < 24u ? pow2_factor(24u - gone) : 1u, r = gone < 24u ? 0u : gone - 24u;
+    u[0] += shr_sat(byte_perm_sx(W, U, 0xcc40) * m, r); u[1] += shr_sat(byte_perm_sx(W, U, 0xdd51) * m, r);
+    u[2] += shr_sat(byte_perm_sx(W, U, 0xee62) * m, r); u[3] += shr_sat(byte_perm_sx(W, U, 0xff73) * m, r);
+  }
+  if (tail > 32) {                                         // more than eight planes left: gone < 24
+    src.skip(32);
+    const uint32_t t = src.peek() & low_mask32(tail - 32), k = 24u - gone;
+    const uint32_t V = ((nib[t & 255u] * 4u + nib[(t >> 8) & 255u]) * 4u + nib[(t >> 16) & 255u]) * 4u + nib[t >> 24];
+    u[0] |= shr_sat(V << 24, 32u - k); u[1] |= shr_sat((V & 0xff00u) << 16, 32u - k);
+    u[2] |= shr_sat((V & 0xff0000u) << 8, 32u - k); u[3] |= shr_sat(V & 0xff000000u, 32u - k);
+    for (uint32_t done = 64, kk = k - 8; done < tail; done += 32, kk -= 8) {
+      src.skip(32);
+      deposit_group8(u, src.peek() & low_mask32(tail - done), kk);
     }
-    if (T) deposit_group8(u, T, k);
-    if (j < 4 * cnt) {                                     // fewer than seven bits left and n < 3: the serial routine
-      decode_planes_from<4>(u, bits, kmin, k - j / 4, n, src);
-      break;
-    }
-    left -= cnt;
   }
   int32_t q[4];
 #pragma unroll

@@ -419,3 +419,19 @@ def test_lean_coders_under_the_accuracy_rule(bits, tol):
         kept = np.abs(out).reshape(-1, 4).max(axis=1) > 0
         if kept.any() and bits == 128 and tol >= 1e-3 and np.abs(x).max() < 1:   # where the cap never cuts, the bound holds
             assert np.abs(out - x).max() <= tol
+
+
+@pytest.mark.parametrize("maxprec", [1, 3, 4, 8, 9, 16, 17, 31, 32])
+@pytest.mark.parametrize("maxbits", [9, 10, 17, 18, 31, 64, 105, 148])
+def test_window_decoder_of_the_tiles(maxprec, maxbits):
+    """The decoder of the 1-D tile kernel and the plane-by-plane one on arbitrary bits (which cut planes and runs at
+    every place), at every limit of planes and budget."""
+    rng = np.random.default_rng(maxprec * 1000 + maxbits)
+    words = rng.integers(0, 1 << 32, size=(20000, 12), dtype=np.uint64).astype(np.uint32)
+    words[::3] &= rng.integers(0, 1 << 32, size=words[::3].shape, dtype=np.uint64).astype(np.uint32)    # sparser planes
+    words[::7] &= rng.integers(0, 1 << 32, size=words[::7].shape, dtype=np.uint64).astype(np.uint32)
+    words[::5, 0] &= 0x3ff                                      # leading zero planes
+    for skip in (0, 5, 31):
+        words[1:, 0] |= np.uint32(1 << skip)                    # blocks that are not empty
+        par = ZfpParams(1, maxbits, maxprec, -1074)
+        assert lib.gcow_window_decode_check(words.ctypes.data, words.shape[0], words.shape[1], skip, par.as_c()) == 0
