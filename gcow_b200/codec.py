@@ -113,7 +113,8 @@ def compressed_nbytes(shape: tuple, params: ZfpParams) -> int:
 
 
 # The parameters of a rate, tolerance or precision are a fixed function of that number: a training loop asks for the same
-# ones on every call.
+# ones on every call. Looked up by the number itself, as a plain float or int: a tensor or an array that holds one can
+# change between two calls.
 _rate_params = lru_cache(maxsize=256)(ZfpParams.from_rate)
 _accuracy_params = lru_cache(maxsize=256)(ZfpParams.from_accuracy)
 _precision_params = lru_cache(maxsize=256)(ZfpParams.from_precision)
@@ -125,10 +126,10 @@ def _resolve_params(rate, tolerance, precision, params, dim) -> ZfpParams:
     if params is not None:
         return params
     if rate is not None:
-        return _rate_params(rate, dim)
+        return _rate_params(float(rate), int(dim))
     if tolerance is not None:
-        return _accuracy_params(tolerance)
-    return _precision_params(precision)
+        return _accuracy_params(float(tolerance))
+    return _precision_params(int(precision))
 
 
 def _check(err: int, what: str) -> None:

@@ -33,6 +33,21 @@ def words(b):
 
 
 # ---------------------------------------------------------------- parameters
+@pytest.mark.parametrize("make", [torch.tensor, np.array], ids=["tensor", "numpy"])
+def test_parameters_held_in_an_array_are_read_on_every_call(make):
+    """A rate, tolerance or precision that a program keeps in a 0-d array and changes in place between two calls."""
+    x = torch.from_numpy(np.random.default_rng(0).standard_normal(64).astype(np.float32))
+    tol, rate, prec = make(1e-1), make(8.0), make(8)
+    for t, r, q in ((1e-1, 8, 8), (1e-4, 16, 20), (1e-2, 4, 3)):
+        tol[()], rate[()], prec[()] = t, r, q
+        for how, held in ((dict(tolerance=t), dict(tolerance=tol)), (dict(rate=r), dict(rate=rate)),
+                          (dict(precision=q), dict(precision=prec))):
+            want, got = g.compress(x, **how), g.compress(x, **held)
+            # a float32 tensor holds 1e-4 as another number than a Python float does: the same power of two
+            assert got.params == want.params and torch.equal(got.stream, want.stream)
+        assert (g.decompress(g.compress(x, tolerance=tol)) - x).abs().max() <= t
+
+
 def test_params_modes():
     p = ZfpParams.from_accuracy(1e-3)
     assert (p.minbits, p.maxbits, p.maxprec, p.minexp) == (1, 16658, 64, -10)
