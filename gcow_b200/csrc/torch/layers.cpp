@@ -15,6 +15,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 
+#include <array>
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
@@ -277,10 +278,12 @@ struct Kept {
   torch::autograd::SavedVariable saved;
   void set(const Tensor& x, bool is_output = false) { saved = torch::autograd::SavedVariable(x, is_output); }
 };
+constexpr int kKeep = 6;
+using Saved = std::array<Tensor, kKeep>;                    // what a node kept, unpacked
 
 // Backward nodes: `kept` holds the saved tensors, inputs are numbered in the order given to record().
 struct LayerNode : torch::autograd::Node {
-  Kept kept[6];
+  Kept kept[kKeep];
   Target target[2];
   bool released = false;
   void release_variables() override {
@@ -288,16 +291,21 @@ struct LayerNode : torch::autograd::Node {
     for (auto& t : target) { t.view.reset(); t.weight.reset(); }
     released = true;
   }
-  Tensor get(int i) {
-    TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
-    return kept[i].saved.unpack(shared_from_this());
-  }
   bool wants(size_t i) { return task_should_compute_output(i); }
-  virtual variable_list grads(variable_list&& g) = 0;
+  // At least one of g is defined; `had`: the saved tensors.
+  virtual variable_list grads(variable_list&& g, const Saved& had) = 0;
   variable_list apply(variable_list&& g) override {
+    bool any = false;
+    for (const Tensor& t : g) any = any || t.defined();
+    if (!any) return variable_list(num_outputs());
+    TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+    // Before the guards: an unpack hook is the user's code, and a checkpoint's reruns the forward pass of its region, whose
+    // operators have to record their history.
+    Saved had;
+    for (int i = 0; i < kKeep; i++) had[i] = kept[i].saved.unpack(shared_from_this());
     at::NoGradGuard no_grad;
     at::AutoDispatchBelowADInplaceOrView below;
-    return grads(std::move(g));
+    return grads(std::move(g), had);
   }
 };
 
@@ -350,10 +358,9 @@ struct LinearNode : LayerNode {                             // inputs: x, w, b, 
   std::vector<int64_t> x_shape;
   bool has_bias = false, has_res = false;
   std::string name() const override { return "GcowLinearBackward"; }
-  variable_list grads(variable_list&& in) override {
+  variable_list grads(variable_list&& in, const Saved& had) override {
     variable_list out(4);
-    if (!in[0].defined()) return out;
-    const Tensor xb = get(0), wb = get(1);
+    const Tensor &xb = had[0], &wb = had[1];
     const On on(xb);
     const Tensor g = rows_of(in[0]);
     if (wants(0)) {                                         // dx[M,K] = g[M,N] W[N,K]: W is stored [reduction N][K]
@@ -405,10 +412,9 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 struct FfnNode : LayerNode {                                // inputs: x, w1, b1, w2, b2
   std::vector<int64_t> shape;
   std::string name() const override { return "GcowFfnBackward"; }
-  variable_list grads(variable_list&& in) override {
+  variable_list grads(variable_list&& in, const Saved& had) override {
     variable_list out(5);
-    if (!in[0].defined()) return out;
-    const Tensor xb = get(0), w1b = get(1), w2b = get(2), pre = get(3), act = get(4);
+    const Tensor &xb = had[0], &w1b = had[1], &w2b = had[2], &pre = had[3], &act = had[4];
     const On on(xb);
     const Tensor g = rows_of(in[0]);
     GemmOpts o;
@@ -471,10 +477,9 @@ struct LayerNormNode : LayerNode {                          // inputs: x, gamma,
   std::vector<int64_t> shape;
   at::ScalarType ptype = at::kFloat;
   std::string name() const override { return "GcowLayerNormBackward"; }
-  variable_list grads(variable_list&& in) override {
+  variable_list grads(variable_list&& in, const Saved& had) override {
     variable_list out(3);
-    if (!in[0].defined()) return out;
-    const Tensor xb = get(0), g32 = get(1), mean = get(2), rstd = get(3);
+    const Tensor &xb = had[0], &g32 = had[1], &mean = had[2], &rstd = had[3];
     const On on(xb);
     const int64_t rows = xb.size(0), H = xb.size(1);
     const Tensor g = rows_of(in[0]);
@@ -523,10 +528,9 @@ PyObject* layernorm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {      /
 struct FusedAttentionNode : LayerNode {                     // input: qkv
   float scale = 1;
   std::string name() const override { return "GcowAttentionBackward"; }
-  variable_list grads(variable_list&& in) override {
+  variable_list grads(variable_list&& in, const Saved& had) override {
     variable_list out(1);
-    if (!in[0].defined() || !wants(0)) return out;
-    const Tensor q = get(0), o = get(1), lse = get(2);
+    const Tensor &q = had[0], &o = had[1], &lse = had[2];
     const On on(q);
     const int B = (int)q.size(0), S = (int)q.size(1), H = (int)q.size(3), D = (int)q.size(4);
     const Tensor g = bf16_rows(in[0]);
@@ -586,10 +590,9 @@ Tensor bmm(const Tensor& a, const Tensor& b, bool a_t, bool b_t, const On& on) {
 struct AttentionNode : LayerNode {                          // inputs: q, k, v
   float scale = 1;
   std::string name() const override { return "GcowUnfusedAttentionBackward"; }
-  variable_list grads(variable_list&& in) override {
+  variable_list grads(variable_list&& in, const Saved& had) override {
     variable_list out(3);
-    if (!in[0].defined()) return out;
-    const Tensor q = get(0), k = get(1), v = get(2), p = get(3);
+    const Tensor &q = had[0], &k = had[1], &v = had[2], &p = had[3];
     const On on(q);
     const Tensor go = bf16_rows(in[0]);
     out[2] = bmm(p, go, true, true, on);                    // P^T dO
@@ -673,10 +676,9 @@ struct ConvNode : LayerNode {                               // inputs: x, w, b
   int kind = 0, halo_min_w = 15;                            // kind: 0 stride 1, 1 1x1 stride 2, 2 3x3 stride 2
   bool has_bias = false;
   std::string name() const override { return "GcowConvBackward"; }
-  variable_list grads(variable_list&& in) override {
+  variable_list grads(variable_list&& in, const Saved& had) override {
     variable_list out(3);
-    if (!in[0].defined()) return out;
-    const Tensor x = get(0), wr = get(1);
+    const Tensor &x = had[0], &wr = had[1];
     const On on(x);
     const Tensor gy = nhwc_bf16(in[0]);
     const void* const g = gy.data_ptr();
@@ -770,10 +772,9 @@ struct Conv1x1Node : LayerNode {                            // inputs: x, w, b
   at::ScalarType wtype = at::kFloat;
   bool has_bias = false;
   std::string name() const override { return "GcowConv1x1Backward"; }
-  variable_list grads(variable_list&& in) override {
+  variable_list grads(variable_list&& in, const Saved& had) override {
     variable_list out(3);
-    if (!in[0].defined()) return out;
-    const Tensor xm = get(0), wb = get(1);
+    const Tensor &xm = had[0], &wb = had[1];
     const On on(xm);
     const Tensor g = bf16_rows(in[0].permute({0, 2, 3, 1})).view({-1, Co});
     if (wants(0)) {
@@ -827,13 +828,12 @@ struct BatchNormNode : LayerNode {                          // inputs: x, gamma,
   bool relu = false, has_res = false;
   at::ScalarType ptype = at::kFloat;
   std::string name() const override { return "GcowBatchNormBackward"; }
-  variable_list grads(variable_list&& in) override {
+  variable_list grads(variable_list&& in, const Saved& had) override {
     variable_list out(4);
     Tensor gy = in[0], gy2 = in.size() > 1 ? in[1] : Tensor();
     if (!gy.defined()) std::swap(gy, gy2);
-    if (!gy.defined()) return out;
-    const Tensor x = get(0), g32 = get(1), stats = get(2);
-    const Tensor mask = relu ? get(3) : Tensor();
+    const Tensor &x = had[0], &g32 = had[1], &stats = had[2];
+    const Tensor& mask = had[3];
     const On on(x);
     gy = nhwc_bf16(gy);
     if (gy2.defined()) gy2 = nhwc_bf16(gy2);

@@ -109,3 +109,57 @@ def test_wrong_arguments_are_refused():
         K.linear(x, w, torch.zeros(32, device="cuda"))
     with pytest.raises(RuntimeError):
         K.linear_residual(x, w, None, torch.zeros(32, 64, device="cuda"))
+
+
+def _grads(net, x, run):
+    y = run(x)
+    y.backward(torch.ones_like(y))
+    out = [y.detach(), x.grad] + [p.grad for p in net.parameters()]
+    x.grad = None
+    net.zero_grad(set_to_none=True)
+    return out
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_checkpoint_recomputes_with_history(name):
+    """Non-reentrant checkpointing reruns the region from the layer function's unpacking: operators of torch in front of
+    it have to record their history there as in the first run."""
+    from torch.utils.checkpoint import checkpoint
+    fn, x = _cases()[name]
+
+    def region(t):
+        return fn(torch.tanh(t))
+    want = torch.autograd.grad(region(x).float().square().sum(), x)[0]
+    got = torch.autograd.grad(checkpoint(region, x, use_reentrant=False).float().square().sum(), x)[0]
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("S", [128, 72])
+def test_checkpoint_of_a_bert_layer(S):
+    """With the fused attention and with the unfused one."""
+    from torch.utils.checkpoint import checkpoint
+    from gcow_b200.models.bert import BertConfig, BertLayer
+    torch.manual_seed(1)
+    net = BertLayer(BertConfig(hidden=128, heads=2, ffn=512)).cuda()
+    x = torch.randn(2, S, 128, device="cuda").bfloat16().requires_grad_(True)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        want = _grads(net, x, net)
+        got = _grads(net, x, lambda t: checkpoint(net, t, use_reentrant=False))
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("stride", [1, 2])
+def test_checkpoint_of_a_resnet_block(stride):
+    from torch.utils.checkpoint import checkpoint
+    from gcow_b200.models.resnet import Bottleneck
+    from gcow_b200.ops import nn as gnn
+    torch.manual_seed(1)
+    down = torch.nn.Sequential(gnn.Conv2d(64, 256, 1, stride=stride, bias=False), gnn.BatchNorm2d(256))
+    net = Bottleneck(64, 64, stride, down).cuda().to(memory_format=torch.channels_last)
+    x = torch.randn(4, 64, 16, 16, device="cuda").bfloat16().to(memory_format=torch.channels_last).requires_grad_(True)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        want = _grads(net, x, net)
+        got = _grads(net, x, lambda t: checkpoint(net, t, use_reentrant=False))
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
