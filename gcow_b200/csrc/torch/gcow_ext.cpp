@@ -26,8 +26,8 @@ int gcow_tile_usable(const int32_t* params, uint64_t blocks, int dim);
 uint64_t gcow_encode_tiles_scratch_bytes(const int32_t* params, uint64_t blocks, int dim);
 int gcow_encode_tiles(const float* in, uint64_t nx, uint64_t ny, const int32_t* params, void* out, void* scratch,
                       uint64_t* block_bits, uint64_t* total_out, void* stream);
-int gcow_decode_tiles(const void* in, float* out, uint64_t nx, uint64_t ny, const int32_t* params,
-                      const uint64_t* block_bits, int shift, void* stream);
+int gcow_decode_generic(const uint64_t* in, float* out, uint64_t nx, uint64_t ny, const int32_t* params,
+                        const uint64_t* block_bits, int shift, void* stream);
 int gcow_ar_launch_ef(const float* in, float* out, uint64_t n, int rank, int world, int variant, int bits, int ctas, int shift,
                       float postscale, void* const* arenas, void* mc_arena, uint64_t region_cap, uint32_t epoch,
                       uint64_t timeout_ns, uint32_t* status, uint32_t* abort_flag, unsigned long long* stamps, float* residual,
@@ -157,7 +157,7 @@ PyObject* decompress(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (one_store)
     check(gcow_decode_1d_fixed(s.const_data_ptr(), out.mutable_data_ptr<float>(), nx, p[1], (int)shift, stream), "gcow_decode_1d_fixed");
   else
-    check(gcow_decode_tiles(s.const_data_ptr(), out.mutable_data_ptr<float>(), nx, ny, p, index, (int)shift, stream), "gcow_decode_tiles");
+    check(gcow_decode_generic((const uint64_t*)s.const_data_ptr(), out.mutable_data_ptr<float>(), nx, ny, p, index, (int)shift, stream), "gcow_decode_generic");
   if (args[7] != Py_None) return Py_NewRef(args[7]);
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS

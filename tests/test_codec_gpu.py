@@ -195,3 +195,24 @@ def test_tile_kernels_at_edges(dim, sizes, how):
             for shift in (0, 2):
                 a, b = g.decompress(cpu, shift=shift), g.decompress(gpu, shift=shift).cpu()
                 assert torch.equal(a.view(torch.int32), b.view(torch.int32)), sz
+
+
+@pytest.mark.parametrize("rate", [2.25, 2.5, 2.75, 3])
+def test_decode_of_short_blocks(rate):
+    """Blocks of 9 to 11 bits go to the kernel without staging, 12 bits and streams that are not word aligned to the tiles."""
+    rng = np.random.default_rng(3)
+    for n in (1, 5, 1021, 4096, 70001):
+        for x in (rng.standard_normal(n).astype(np.float32), np.cumsum(rng.standard_normal(n)).astype(np.float32),
+                  np.where(rng.random(n) < 0.9, 0, 1).astype(np.float32)):
+            cpu = g.compress(torch.from_numpy(x), rate=rate)
+            gpu = g.compress(dev(x), rate=rate)
+            assert torch.equal(gpu.stream.cpu(), cpu.stream)
+            held = torch.zeros(gpu.nbytes + 8, dtype=torch.uint8, device="cuda")
+            held[4:4 + gpu.nbytes] = gpu.stream
+            for shift in (0, 2):
+                want = g.decompress(cpu, shift=shift).view(torch.int32)
+                out = torch.zeros(n + 2, device="cuda")
+                got = g.decompress(gpu, out=out[1:n + 1], shift=shift)
+                assert torch.equal(got.cpu().view(torch.int32), want) and out[0] == 0 and out[n + 1] == 0
+                moved = Compressed(held[4:4 + gpu.nbytes], gpu.params, gpu.shape, None)
+                assert torch.equal(g.decompress(moved, shift=shift).cpu().view(torch.int32), want)
