@@ -97,8 +97,9 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128_16k(uint32_t saddr) {
   return d;
 }
 
-// B_MN: B is stored [K][N] (the data-gradient product dX = dY * W reads the weight matrix in place)
-template <bool B_MN>
+// B_MN: B is stored [K][N] (the data-gradient product dX = dY * W reads the weight matrix in place). SIDE: the epilogue reads
+// a residual or the argument of a GELU' factor.
+template <bool B_MN, bool SIDE>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const Params p) {
   extern __shared__ uint8_t smem_raw[];
@@ -202,7 +203,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     constexpr int COLS = BN / (EPI_WARPS / 4);
     constexpr int NCH = COLS / 32;
     const int col0 = (ew / 4) * COLS;
-    const __nv_bfloat16* const ahead = p.flags & kGeluGrad ? p.aux : p.flags & kResidual ? p.residual : nullptr;
+    [[maybe_unused]] const __nv_bfloat16* const ahead = p.flags & kGeluGrad ? p.aux : p.residual;
     uint8_t* stg = stage_base + ew * kStageWarpBytes;
     uint32_t t = 0;
     bool ok = true;
@@ -210,8 +211,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const int m0 = (tile % tiles_m) * BM + (int)rank * 128, n0 = (tile / tiles_m) * BN;
       const uint32_t acc = t & 1, aphase = (t >> 1) & 1;
       const int mw = m0 + q * 32;                         // the warp's first row
-      uint4 pf[4];
-      auto fetch = [&](int c) {                           // four lanes per row, as the staging helpers have it
+      [[maybe_unused]] uint4 pf[4];
+      [[maybe_unused]] auto fetch = [&](int c) {                           // four lanes per row, as the staging helpers have it
         const int n = n0 + col0 + c * 32 + (lane & 3) * 8;
 #pragma unroll
         for (int it = 0; it < 4; it++) {
@@ -220,7 +221,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           if (c < NCH && n < p.N && row < p.M) pf[it] = *reinterpret_cast<const uint4*>(ahead + (size_t)row * p.ldc + n);
         }
       };
-      if (ahead) fetch(0);
+      if (SIDE) fetch(0);
       ok = mbar_wait_abortable(&sm->abort, &sm->tmem_full[acc], aphase, p.error, 4);
       ok = __all_sync(0xffffffffu, ok);   // the tensor-memory loads below need the whole warp
       if (!ok) break;
@@ -231,7 +232,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       // What the epilogue reads besides the accumulator (the GELU's argument, else the residual) is fetched one block of
       // 32 columns ahead, the first block under the wait for the tile: read where it is used, every block stood for
       // its load's whole latency, and with two warps per scheduler nothing covered it (16384 x 4096 x 1024: with a
-      // residual 168 -> 126 us, times GELU' 237 -> 148 us, plain 100 us).
+      // residual 189 -> 144 us, times GELU' 247 -> 151 us, plain 95 us).
       auto process = [&](const uint32_t (&r)[32], int c) {
         const int n = n0 + col0 + c * 32;
         if (n >= p.N || mw >= p.M) return;                // warp-uniform; the launcher guarantees N % 32 == 0
@@ -245,7 +246,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         }
         if (p.flags & kAuxOut) warp_store_rows_bf16(stg, lane, v, p.aux, off, row_ok);
         if (p.flags & kGelu) gelu32(v);                    // not together with kGeluGrad
-        if (ahead) {
+        if (SIDE) {
           warp_place_rows(stg, lane, pf);
           fetch(c + 1);
 #pragma unroll
@@ -261,7 +262,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
           __syncwarp();
         }
-        if ((p.flags & kGeluGrad) && (p.flags & kResidual)) warp_load_rows_bf16<true>(stg, lane, p.residual, off, row_ok, v);
+        if (SIDE && (p.flags & kGeluGrad) && (p.flags & kResidual)) warp_load_rows_bf16<true>(stg, lane, p.residual, off, row_ok, v);
         warp_store_rows_bf16(stg, lane, v, p.C, off, row_ok);
       };
       uint32_t ra[32], rb[32];
@@ -324,6 +325,7 @@ static int make_map_mnfold(CUtensorMap* map, const void* ptr, uint64_t K, uint64
   return r == CUDA_SUCCESS ? 0 : -12;
 }
 
+using KernelFn = void (*)(CUtensorMap, CUtensorMap, Params);
 constexpr size_t kSmemBytes = (size_t)STAGES * STAGE_BYTES + sizeof(Smem) + 16 + (size_t)EPI_WARPS * kStageWarpBytes + 1024;
 
 }  // namespace gemm2
@@ -338,10 +340,12 @@ int gcow_gemm2_max_pairs() {
   static std::once_flag once;
   static int pairs = 0;
   std::call_once(once, [] {
-    if (cudaFuncSetAttribute(gemm2_bf16_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) != cudaSuccess ||
-        cudaFuncSetAttribute(gemm2_bf16_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) != cudaSuccess) {
-      cudaGetLastError();
-      return;
+    for (const KernelFn kernel : {gemm2_bf16_kernel<false, false>, gemm2_bf16_kernel<true, false>, gemm2_bf16_kernel<false, true>,
+                                  gemm2_bf16_kernel<true, true>}) {
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+      }
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2, 1, 1);
@@ -352,7 +356,7 @@ int gcow_gemm2_max_pairs() {
     attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
     cfg.attrs = &attr; cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm2_bf16_kernel<false>, &cfg) == cudaSuccess) pairs = n;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm2_bf16_kernel<false, false>, &cfg) == cudaSuccess) pairs = n;
     else cudaGetLastError();
   });
   return pairs;
@@ -396,8 +400,12 @@ int gcow_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   static const bool pdl = [] { const char* e = getenv("GCOW_PDL"); return !(e && e[0] == '0'); }();
   cfg.attrs = attr; cfg.numAttrs = pdl ? 2 : 1;
-  if (b_mn) return (int)cudaLaunchKernelEx(&cfg, gemm2_bf16_kernel<true>, ma, mb, p);
-  return (int)cudaLaunchKernelEx(&cfg, gemm2_bf16_kernel<false>, ma, mb, p);
+  // Its own instance for launches that read nothing besides the accumulator: the block fetched ahead costs 16 registers, for
+  // which the epilogue spilled (16384 x 4096 x 1024: plain 100 -> 95 us, bias 106 -> 97, bias and GELU 144 -> 128).
+  const bool side = flags & (kResidual | kGeluGrad);
+  const KernelFn kernel = b_mn ? (side ? gemm2_bf16_kernel<true, true> : gemm2_bf16_kernel<true, false>)
+                               : (side ? gemm2_bf16_kernel<false, true> : gemm2_bf16_kernel<false, false>);
+  return (int)cudaLaunchKernelEx(&cfg, kernel, ma, mb, p);
 }
 
 }  // extern "C"
