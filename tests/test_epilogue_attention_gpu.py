@@ -52,6 +52,12 @@ def test_gelu_of_special_values():
     assert math.isnan(K.gemm_bf16(x, torch.eye(64, device="cuda", dtype=torch.bfloat16), gelu=True)[0, 0].item())
 
 
+@pytest.mark.parametrize("B,S,H", [(37, 512, 1), (149, 128, 1), (25, 256, 3), (25, 384, 2), (38, 512, 1)])
+def test_attention_on_either_side_of_a_full_gpu(B, S, H):
+    """As below, with 148 CTAs (the last grid with long steps in the backward kernels) and a few more."""
+    test_attention(B, S, H)
+
+
 @pytest.mark.parametrize("B,S,H", [(1, 128, 1), (2, 256, 3), (1, 384, 2), (3, 512, 4)])
 def test_attention(B, S, H):
     """Forward and backward. Two roundings to bf16 on each path (P or dS, and the result): below 2^-8 of the norm."""
