@@ -149,9 +149,14 @@ def compress(x: torch.Tensor, *, rate: float | None = None, tolerance: float | N
     ``dim=1`` treats ``x`` as a flat vector cut into blocks of 4 (what the
     training study does with gradients); ``dim=2`` takes a 2-D tensor
     ``[ny, nx]`` cut into 4x4 blocks (the reference CPU/FPGA codec).
-    Variable-rate modes (tolerance / precision) on CUDA synchronise once to
-    learn the stream length; pass ``return_index=True`` to keep the per-block
-    bit offsets needed for a parallel decode.
+    Variable-rate modes (tolerance / precision) on CUDA wait for the length of
+    the stream, and for nothing else: ``stream`` and ``index`` (the per-block bit
+    offsets, always kept in these modes) are still being written when the call
+    returns, in the order of the current CUDA stream. As with any tensor, another
+    stream or library has to wait for that stream (``wait_stream``, an event or a
+    synchronisation) before it reads them; reading them on the same stream or
+    copying them to the host needs nothing. ``return_index=True`` asks for the
+    index at fixed rate too (1-D blocks of 16, 32, 64 or 128 bits have none).
     """
     if x.dtype != torch.float32:
         raise TypeError("the codec takes float32 input")

@@ -216,3 +216,20 @@ def test_decode_of_short_blocks(rate):
                 assert torch.equal(got.cpu().view(torch.int32), want) and out[0] == 0 and out[n + 1] == 0
                 moved = Compressed(held[4:4 + gpu.nbytes], gpu.params, gpu.shape, None)
                 assert torch.equal(g.decompress(moved, shift=shift).cpu().view(torch.int32), want)
+
+
+@pytest.mark.parametrize("dim,how", [(1, dict(tolerance=1e-6)), (1, dict(precision=20)), (2, dict(tolerance=1e-6))])
+def test_variable_rate_result_on_another_stream(dim, how):
+    """These modes wait for the length alone; the stream and its index are ready in the order of the CUDA stream that made
+    them, on which another stream has to wait."""
+    x = torch.randn(1 << 24, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    x = x.view(4096, -1) if dim == 2 else x
+    side = torch.cuda.Stream()
+    for _ in range(5):
+        c = g.compress(x, dim=dim, **how)
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            stream, index, y = c.stream.clone(), c.index.clone(), g.decompress(c)
+        torch.cuda.synchronize()
+        assert torch.equal(stream, c.stream) and torch.equal(index, c.index) and torch.equal(y, g.decompress(c))
+        assert c.nbytes == (int(index[-1]) + 63) // 64 * 8
