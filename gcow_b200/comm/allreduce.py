@@ -220,8 +220,8 @@ class CompressedAllReduce:
         if residual is not None and (residual.dtype != torch.float32 or residual.numel() != n or not residual.is_contiguous()
                                      or residual.device != x.device):
             raise TypeError("residual must be a contiguous float32 tensor of the input's size on the same device")
-        if out is not x and (out.dtype != torch.float32 or not out.is_contiguous() or out.numel() < n):
-            raise TypeError("out must be a contiguous float32 tensor of the input's size")
+        if out is not x and (out.dtype != torch.float32 or not out.is_contiguous() or out.numel() < n or out.device != x.device):
+            raise TypeError("out must be a contiguous float32 tensor of the input's size on the same device")
         for lo in range(0, n, self.max_numel):
             self._launch(x, out, lo, min(self.max_numel, n - lo), stream, variant, residual)
         return out

@@ -19,6 +19,7 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 
 extern "C" {
@@ -125,6 +126,23 @@ inline Tensor nhwc_bf16(const Tensor& t) {
   return t.to(at::kBFloat16).contiguous(at::MemoryFormat::ChannelsLast);
 }
 
+// ------------------------------------------------------------------------ operands
+// The kernels take bare pointers: every operand has to be where x is and as long as x says, or they would read and write
+// past its end.
+void on_device_of(const Tensor& x, std::initializer_list<const Tensor*> others) {
+  for (const Tensor* t : others)
+    TORCH_CHECK(!t->defined() || t->device() == x.device(), "expected every operand on ", x.device(), ", got one on ", t->device());
+}
+void length(const char* what, const Tensor& t, int64_t n) {
+  TORCH_CHECK(!t.defined() || t.numel() == n, what, " has ", t.numel(), " elements, expected ", n);
+}
+void matrix(const char* what, const Tensor& t, int64_t rows, int64_t cols) {
+  TORCH_CHECK(t.dim() == 2 && t.size(0) == rows && t.size(1) == cols, what, " has shape ", t.sizes(), ", expected [", rows, ", ", cols, "]");
+}
+void dims(const char* what, const Tensor& t, int64_t n) {
+  TORCH_CHECK(t.dim() == n, what, " has ", t.dim(), " dimensions, expected ", n);
+}
+
 // ------------------------------------------------------------------------ products
 bool pair_gemm_enabled() {
   static const bool on = !env_off("GCOW_GEMM2") && gcow_gemm2_max_pairs() > 0;
@@ -141,13 +159,21 @@ struct GemmOpts {
 Tensor gemm(const Tensor& a, const Tensor& b, const GemmOpts& o, const On& on) {
   const int64_t M = o.a_t ? a.size(1) : a.size(0), K = o.a_t ? a.size(0) : a.size(1);
   const int64_t N = o.b_t ? b.size(1) : b.size(0), Kb = o.b_t ? b.size(0) : b.size(1);
+  TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && a.stride(1) == 1 &&
+              b.stride(1) == 1, "gemm: the operands have to be bf16 matrices with contiguous rows");
   TORCH_CHECK(K == Kb, "gemm: reduction lengths differ");
   Tensor out = o.out.defined() ? o.out : empty({M, N}, o.out_f32 ? at::kFloat : at::kBFloat16, a);
   const Tensor& aux = o.pre_gelu_out.defined() ? o.pre_gelu_out : o.gelu_grad_of;
   TORCH_CHECK(out.size(0) == M && out.size(1) == N, "gemm: the result has another shape than the product");
-  TORCH_CHECK(!o.bias.defined() || o.bias.numel() == N, "gemm: the bias has another length than the product's rows");
-  TORCH_CHECK(!o.residual.defined() || (o.residual.sizes() == out.sizes() && o.residual.strides() == out.strides()),
-              "gemm: the residual has another shape than the product");
+  TORCH_CHECK(!o.bias.defined() || (o.bias.numel() == N && o.bias.scalar_type() == at::kFloat && o.bias.is_contiguous()),
+              "gemm: the bias has to be a float32 vector as long as the product's rows");
+  TORCH_CHECK(!o.residual.defined() || (o.residual.sizes() == out.sizes() && o.residual.strides() == out.strides() &&
+                                        o.residual.scalar_type() == out.scalar_type()),
+              "gemm: the residual has another shape or type than the product");
+  TORCH_CHECK(!(o.pre_gelu_out.defined() && o.gelu_grad_of.defined()), "gemm: one side tensor of the GELU at a time");
+  TORCH_CHECK(!aux.defined() || (aux.scalar_type() == at::kBFloat16 && aux.sizes() == out.sizes() && aux.strides() == out.strides()),
+              "gemm: the GELU's side tensor has another shape or type than the product");
+  on_device_of(a, {&b, &out, &o.bias, &o.residual, &aux});
   int flags = (out.scalar_type() == at::kFloat ? kOutF32 : 0) | (o.bias.defined() ? kBias : 0) | (o.gelu ? kGelu : 0) |
               (o.residual.defined() ? kResidual : 0);
   if (aux.defined()) flags |= o.pre_gelu_out.defined() ? kAuxOut : kGeluGrad;
@@ -384,6 +410,12 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(nargs == 4, "linear: bad arguments");
   const Tensor x = need(args[0]), w = need(args[1]), b = arg(args[2]), r = arg(args[3]);
+  TORCH_CHECK(x.dim() >= 1, "linear: the input has no dimensions");
+  on_device_of(x, {&w, &b, &r});
+  dims("linear: the weight", w, 2);
+  matrix("linear: the weight", w, w.size(0), x.size(-1));
+  length("linear: the bias", b, w.size(0));
+  TORCH_CHECK(!r.defined() || (r.dim() >= 1 && r.size(-1) == w.size(0)), "linear: the residual's rows have another length than the result's");
   auto node = record<LinearNode>(x, w, b, r);
   Tensor out;
   {
@@ -443,6 +475,13 @@ PyObject* ffn_residual(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(nargs == 5, "ffn_residual: bad arguments");
   const Tensor x = need(args[0]), w1 = need(args[1]), b1 = need(args[2]), w2 = need(args[3]), b2 = need(args[4]);
+  TORCH_CHECK(x.dim() >= 1, "ffn_residual: the input has no dimensions");
+  on_device_of(x, {&w1, &b1, &w2, &b2});
+  dims("ffn_residual: the first weight", w1, 2);
+  matrix("ffn_residual: the first weight", w1, w1.size(0), x.size(-1));
+  matrix("ffn_residual: the second weight", w2, x.size(-1), w1.size(0));
+  length("ffn_residual: the first bias", b1, w1.size(0));
+  length("ffn_residual: the second bias", b2, w2.size(0));
   auto node = record<FfnNode>(x, w1, b1, w2, b2);
   Tensor out;
   {
@@ -501,6 +540,10 @@ PyObject* layernorm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {      /
   const Tensor x = need(args[0]), gamma = need(args[1]), beta = need(args[2]);
   const double eps = PyFloat_AsDouble(args[3]);
   if (PyErr_Occurred()) return nullptr;
+  TORCH_CHECK(x.dim() >= 1, "layernorm: the input has no dimensions");
+  on_device_of(x, {&gamma, &beta});
+  length("layernorm: gamma", gamma, x.size(-1));
+  length("layernorm: beta", beta, x.size(-1));
   auto node = record<LayerNormNode>(x, gamma, beta);
   Tensor out;
   {
@@ -550,6 +593,8 @@ PyObject* fused_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) { 
   const Tensor qkv = need(args[0]);
   const double scale = PyFloat_AsDouble(args[1]);
   if (PyErr_Occurred()) return nullptr;
+  dims("fused_attention: the input", qkv, 5);
+  TORCH_CHECK(qkv.size(2) == 3, "fused_attention: expected [batch, positions, 3, heads, 64], got ", qkv.sizes());
   auto node = record<FusedAttentionNode>(qkv);
   Tensor out;
   {
@@ -613,6 +658,10 @@ PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {      /
   const Tensor q = need(args[0]), k = need(args[1]), v = need(args[2]);
   const double scale = PyFloat_AsDouble(args[3]);
   if (PyErr_Occurred()) return nullptr;
+  on_device_of(q, {&k, &v});
+  for (const Tensor* t : {&q, &k, &v})
+    TORCH_CHECK(t->dim() == 3 && t->sizes() == q.sizes() && t->scalar_type() == at::kBFloat16 && t->is_contiguous(),
+                "attention: expected three contiguous bf16 tensors [batch * heads, positions, dimensions] of one shape");
   auto node = record<AttentionNode>(q, k, v);
   Tensor out;
   {
@@ -736,6 +785,13 @@ PyObject* conv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   int v[4];
   for (int i = 0; i < 4; i++) v[i] = (int)PyLong_AsLong(args[3 + i]);
   if (PyErr_Occurred()) return nullptr;
+  on_device_of(xin, {&w, &b});
+  dims("conv: the input", xin, 4);
+  dims("conv: the weight", w, 4);
+  TORCH_CHECK(w.size(1) == xin.size(1), "conv: the weight has ", w.size(1), " input channels, the input ", xin.size(1));
+  TORCH_CHECK(v[0] == 0 || (v[0] == 1 ? w.size(2) == 1 && w.size(3) == 1 : w.size(2) == 3 && w.size(3) == 3),
+              "conv: the stride-2 kernels take filters of 1 x 1 and of 3 x 3");
+  length("conv: the bias", b, w.size(0));
   auto node = record<ConvNode>(xin, w, b);
   Tensor out;
   {
@@ -797,6 +853,10 @@ PyObject* conv1x1(PyObject*, PyObject* const* args, Py_ssize_t nargs) {        /
   HANDLE_TH_ERRORS
   TORCH_CHECK(nargs == 3, "conv1x1: bad arguments");
   const Tensor x = need(args[0]), w = need(args[1]), b = arg(args[2]);
+  on_device_of(x, {&w, &b});
+  dims("conv1x1: the input", x, 4);
+  length("conv1x1: the weight", w, w.size(0) * x.size(1));
+  length("conv1x1: the bias", b, w.size(0));
   auto node = record<Conv1x1Node>(x, w, b);
   Tensor out;
   {
@@ -875,6 +935,18 @@ PyObject* batchnorm_act(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const bool relu = PyObject_IsTrue(args[6]) == 1, fork = PyObject_IsTrue(args[9]) == 1;
   const double momentum = PyFloat_AsDouble(args[7]), eps = PyFloat_AsDouble(args[8]);
   if (PyErr_Occurred()) return nullptr;
+  on_device_of(x, {&gamma, &beta, &rm, &rv, &res});
+  dims("batchnorm_act: the input", x, 4);
+  for (const Tensor* t : {&x, &res})
+    TORCH_CHECK(!t->defined() || (t->sizes() == x.sizes() && t->scalar_type() == at::kBFloat16 && t->is_contiguous(at::MemoryFormat::ChannelsLast)),
+                "batchnorm_act: expected input and residual as channels-last bf16 tensors of one shape");
+  length("batchnorm_act: gamma", gamma, x.size(1));
+  length("batchnorm_act: beta", beta, x.size(1));
+  for (const Tensor* t : {&rm, &rv}) {
+    length("batchnorm_act: the running statistics", *t, x.size(1));
+    TORCH_CHECK(!t->defined() || (t->scalar_type() == at::kFloat && t->is_contiguous()),
+                "batchnorm_act: the running statistics have to be contiguous float32");
+  }
   auto node = record<BatchNormNode>(x, gamma, beta, res);
   Tensor y, y2;
   {

@@ -204,3 +204,14 @@ def test_late_peer_times_out_on_both_ranks_then_recovers():
     assert res["timed_out"] == [True, True] and res["recovered_bit_exact"] == [True, True]
     assert res["safe_mode_fallbacks"][0] > 0 and res["safe_mode_fallbacks"] == res["safe_mode_fallbacks"][::-1]
     assert res["replicas_equal"]
+
+
+@pytest.mark.gpu
+def test_out_that_does_not_fit_is_refused():
+    ar = CompressedAllReduce(1 << 12, GcowConfig(rate=8))
+    x = torch.ones(1000, device="cuda")
+    for out in (torch.empty(1000), torch.empty(999, device="cuda"), torch.empty(1000, device="cuda", dtype=torch.float64),
+                torch.empty(2000, device="cuda")[::2]):
+        with pytest.raises(TypeError):
+            ar(x, out=out)
+    assert torch.equal(ar(x, out=torch.empty(1000, device="cuda")), x)
