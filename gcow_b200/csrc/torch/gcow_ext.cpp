@@ -70,7 +70,7 @@ bool read_params(PyObject* const* args, int32_t* p) {
 PyObject* compress(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(nargs == 7 && THPVariable_Check(args[0]), "compress: bad arguments");
-  const at::Tensor& x = THPVariable_Unpack(args[0]);
+  const at::Tensor& x = gcow_ext::in_memory(THPVariable_Unpack(args[0]));
   int32_t p[4];
   if (!read_params(args + 1, p)) return nullptr;
   const long dim = PyLong_AsLong(args[5]);
@@ -127,7 +127,7 @@ PyObject* compress(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 PyObject* decompress(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(nargs == 9 && THPVariable_Check(args[0]) && PyTuple_Check(args[6]), "decompress: bad arguments");
-  const at::Tensor& s = THPVariable_Unpack(args[0]);
+  const at::Tensor& s = gcow_ext::in_memory(THPVariable_Unpack(args[0]));
   int32_t p[4];
   if (!read_params(args + 2, p)) return nullptr;
   const Py_ssize_t dim = PyTuple_GET_SIZE(args[6]);
@@ -145,14 +145,14 @@ PyObject* decompress(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (!fixed) {
     if (args[1] == Py_None) Py_RETURN_NONE;
     TORCH_CHECK_TYPE(THPVariable_Check(args[1]), "decompress: the index is no tensor");
-    const at::Tensor& i = THPVariable_Unpack(args[1]);
+    const at::Tensor& i = gcow_ext::in_memory(THPVariable_Unpack(args[1]));
     if (i.device() != s.device()) Py_RETURN_NONE;
     index = (const uint64_t*)i.const_data_ptr();
   }
-  const c10::cuda::CUDAGuard guard(s.device());
   at::Tensor out;
-  if (args[7] == Py_None) out = at::detail::empty_cuda(c10::IntArrayRef(shape, (size_t)dim), at::kFloat, s.device(), std::nullopt);
-  else out = THPVariable_Unpack(args[7]);
+  if (args[7] != Py_None) out = gcow_ext::in_memory(THPVariable_Unpack(args[7]));
+  const c10::cuda::CUDAGuard guard(s.device());
+  if (!out.defined()) out = at::detail::empty_cuda(c10::IntArrayRef(shape, (size_t)dim), at::kFloat, s.device(), std::nullopt);
   void* const stream = c10::cuda::getCurrentCUDAStream(s.device().index()).stream();
   if (one_store)
     check(gcow_decode_1d_fixed(s.const_data_ptr(), out.mutable_data_ptr<float>(), nx, p[1], (int)shift, stream), "gcow_decode_1d_fixed");
@@ -169,8 +169,8 @@ PyObject* decompress(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 PyObject* ar_launch(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(nargs == 20 && THPVariable_Check(args[0]) && THPVariable_Check(args[1]), "ar_launch: bad arguments");
-  const at::Tensor& x = THPVariable_Unpack(args[0]);
-  const at::Tensor& out = THPVariable_Unpack(args[1]);
+  const at::Tensor& x = gcow_ext::in_memory(THPVariable_Unpack(args[0]));
+  const at::Tensor& out = gcow_ext::in_memory(THPVariable_Unpack(args[1]));
   uint64_t v[20];
   for (int i = 3; i < 20; i++) {
     if (i == 12 || (i == 5 && args[5] == Py_None)) continue;
@@ -178,9 +178,11 @@ PyObject* ar_launch(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   }
   const double post = PyFloat_AsDouble(args[12]);
   if (PyErr_Occurred()) return nullptr;
+  at::Tensor residual;
+  if (args[2] != Py_None) residual = gcow_ext::in_memory(THPVariable_Unpack(args[2]));
   const c10::cuda::CUDAGuard guard(x.device());
   void* const stream = args[5] == Py_None ? c10::cuda::getCurrentCUDAStream(x.device().index()).stream() : (void*)v[5];
-  float* const res = args[2] == Py_None ? nullptr : THPVariable_Unpack(args[2]).mutable_data_ptr<float>() + v[3];
+  float* const res = residual.defined() ? residual.mutable_data_ptr<float>() + v[3] : nullptr;
   uint32_t* const status = (uint32_t*)v[18];
   const int err = gcow_ar_launch_ef(x.const_data_ptr<float>() + v[3], out.mutable_data_ptr<float>() + v[3], v[4], (int)v[6], (int)v[7],
                                     (int)v[8], (int)v[9], (int)v[10], (int)v[11], (float)post, (void* const*)v[13], (void*)v[14],

@@ -357,7 +357,7 @@ PyObject* finish(Tensor out, const std::shared_ptr<N>& n) {
 }
 inline Tensor arg(PyObject* o) {                            // None: undefined
   TORCH_CHECK_TYPE(o == Py_None || THPVariable_Check(o), "expected a tensor, got ", Py_TYPE(o)->tp_name);
-  return o == Py_None ? Tensor() : THPVariable_Unpack(o);
+  return o == Py_None ? Tensor() : in_memory(THPVariable_Unpack(o));
 }
 inline Tensor need(PyObject* o) {
   TORCH_CHECK_TYPE(o != Py_None, "expected a tensor, got None");
@@ -1021,7 +1021,9 @@ Tensor error_word(int device) {
   std::lock_guard<std::mutex> lock(g_error_mu);
   Tensor& t = g_error[device];
   if (!t.defined()) {
+    // below every dispatch mode: the word outlives a mode that would make it a tensor of its own kind
     at::AutoDispatchBelowADInplaceOrView below;
+    const c10::impl::ExcludeDispatchKeyGuard no_modes(c10::DispatchKeySet({c10::DispatchKey::Python, c10::DispatchKey::PythonTLSSnapshot}));
     t = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::Device(at::kCUDA, (at::DeviceIndex)device)));
   }
   return t;

@@ -73,3 +73,18 @@ def test_operands_that_do_not_fit_are_refused(ext, name, args, message):
 def test_operands_that_fit_get_as_far_as_the_device(ext, name, args):
     with pytest.raises(RuntimeError, match="(?i)cuda"):
         getattr(ext, name)(*args)
+
+
+def test_tensors_without_memory_are_refused(ext):
+    """A FakeTensor says it is on a GPU and has no address."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    with FakeTensorMode():
+        x, w, f = (torch.empty(64, 128, device="cuda", dtype=d) for d in (torch.bfloat16, torch.float32, torch.float32))
+        byte, index = torch.empty(512, device="cuda", dtype=torch.uint8), torch.empty(17, device="cuda", dtype=torch.int64)
+    for call in (lambda: ext.linear(x, w, None, None), lambda: ext.layernorm(x, f[0], f[0], 1e-5),
+                 lambda: ext.compress(f.view(-1), 32, 32, 64, -1074, 1, False), lambda: ext.compress(f, 1, 16658, 64, -10, 2, False),
+                 lambda: ext.decompress(byte, None, 32, 32, 64, -1074, (64,), None, 0),
+                 lambda: ext.decompress(torch.zeros(512, dtype=torch.uint8), None, 32, 32, 64, -1074, (64,), f.view(-1)[:64], 0),
+                 lambda: ext.ar_launch(f, f, None, 0, 64, None, *[0] * 6, 1.0, *[0] * 7)):
+        with pytest.raises(RuntimeError, match="FakeTensor"):
+            call()
