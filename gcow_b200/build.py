@@ -22,6 +22,7 @@ import fcntl
 import hashlib
 import json
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -176,6 +177,16 @@ def _build_cuda_locked(force, jobs, name, srcs, digest, nvcc) -> Path:
     return LIB / f"{name}.so"
 
 
+def _ext_flags() -> list[str]:
+    """Compiler flags of the extension module. The two names that nothing reads make its stamp that of one libtorch and one
+    interpreter: a module built for another of either does not load, or loads and misbehaves."""
+    import sysconfig
+    import torch
+    tag = re.sub(r"\W", "_", f"{torch.__version__}"), re.sub(r"\W", "_", f"{sysconfig.get_config_var('SOABI')}")
+    return ["-std=c++17", "-O2", "-fPIC", "-fvisibility=hidden", f"-DGCOW_TORCH_{tag[0]}", f"-DGCOW_PYTHON_{tag[1]}",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+
+
 def build_ext(force: bool = False) -> Path:
     """Build gcow_ext.so against the installed libtorch and CPython headers. It is linked to libgcow_cuda.so in its own
     directory; libtorch's libraries are the ones that ``import torch`` has loaded."""
@@ -184,8 +195,7 @@ def build_ext(force: bool = False) -> Path:
     LIB.mkdir(exist_ok=True)
     name = "gcow_ext"
     srcs = _sources("ext")
-    flags = ["-std=c++17", "-O2", "-fPIC", "-fvisibility=hidden", f"-DGCOW_TORCH_{torch.__version__.split('+')[0].replace('.', '_')}",
-             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    flags = _ext_flags()
     digest = _digest(srcs + sorted((CSRC / "torch").glob("*.h")), flags)
     if not force and _up_to_date(name, digest):
         return LIB / f"{name}.so"

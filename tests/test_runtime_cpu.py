@@ -49,3 +49,17 @@ def test_grad_target_respects_the_kernel_alignment():
     assert K._grad_target(taken, 1, 64, align=16) == (None, None)
     flat, alias = K._grad_target(taken, 1, 64, align=4)
     assert flat is not None and alias.shape == w.shape
+
+
+def test_extension_stamp_is_of_one_interpreter_and_one_libtorch(monkeypatch):
+    import sysconfig
+    from gcow_b200 import build
+    mine = build._ext_flags()
+    get = sysconfig.get_config_var
+    with monkeypatch.context() as m:
+        m.setattr(sysconfig, "get_config_var", lambda name: "cpython-399-x86_64-linux-gnu" if name == "SOABI" else get(name))
+        assert build._ext_flags() != mine
+    with monkeypatch.context() as m:
+        m.setattr(torch, "__version__", torch.__version__ + ".post1")
+        assert build._ext_flags() != mine
+    assert build._ext_flags() == mine
