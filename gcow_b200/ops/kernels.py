@@ -126,7 +126,7 @@ def check_errors(device: torch.device | None = None, raise_on_error: bool = True
     """Read the error word of the compute kernels (synchronises). Raises KernelWaitAbandoned if a kernel gave up on
     an internal wait, or returns the code when ``raise_on_error`` is false. The word is cleared."""
     worst = 0
-    for w in _native.ext().error_words():
+    for w in _native._ext.error_words() if _native._ext is not None else ():      # no module: no kernel has run
         dev = w.device
         if device is not None and dev != device:
             continue

@@ -63,3 +63,14 @@ def test_extension_stamp_is_of_one_interpreter_and_one_libtorch(monkeypatch):
         m.setattr(torch, "__version__", torch.__version__ + ".post1")
         assert build._ext_flags() != mine
     assert build._ext_flags() == mine
+
+
+def test_check_errors_needs_nothing_where_nothing_ran(monkeypatch):
+    """On a machine without the native libraries there is no error word, and no error."""
+    from gcow_b200 import _native
+
+    def missing():
+        raise RuntimeError("no library here")
+    monkeypatch.setattr(_native, "_ext", None)
+    monkeypatch.setattr(_native, "ext", missing)
+    assert K.check_errors() == 0 and K.check_errors(torch.device("cuda", 0)) == 0
