@@ -576,6 +576,7 @@ int gcow_codec_tables4(const void** etab, const void** dtab, const void** epair,
 
 // The tile kernels (tile_kernels.cu).
 int gcow_tile_usable(const int32_t* params, uint64_t blocks, int dim);
+uint64_t gcow_encode_tiles_scratch_bytes(const int32_t* params, uint64_t blocks, int dim);
 int gcow_encode_tiles(const float* in, uint64_t nx, uint64_t ny, const int32_t* params, void* out, void* scratch,
                       uint64_t* block_bits, uint64_t* total_out, void* stream);
 int gcow_decode_tiles(const void* in, float* out, uint64_t nx, uint64_t ny, const int32_t* params,
@@ -637,9 +638,8 @@ int gcow_decode_1d_fixed(const void* in, float* out, uint64_t n, int maxbits, in
 }
 
 // Launch sequence of the generic encoder, shared by the entry point that takes the caller's scratch and the one
-// that uses the library's built-in array. One tile kernel where it applies (its scratch, 16 bytes per tile and 16
-// more, fits in what gcow_encode_generic_scratch_bytes asks for); blocks padded far beyond their longest code take
-// slots -> per-block lengths -> prefix sum -> bit-offset scatter.
+// that uses the library's built-in array. The tile kernels where they apply; blocks padded far beyond their longest code
+// take slots -> per-block lengths -> prefix sum -> bit-offset scatter. The two lay the scratch out differently.
 static int launch_encode_generic(const float* in, uint64_t nx, uint64_t ny, const ZfpParams& p, uint64_t blocks,
                                  uint64_t* out, uint64_t out_bytes, void* scratch, uint64_t* block_bits,
                                  cudaStream_t s) {
@@ -666,14 +666,15 @@ static int launch_encode_generic(const float* in, uint64_t nx, uint64_t ny, cons
   return (int)cudaGetLastError();
 }
 
-// Scratch requirements of the generic encoder, in bytes, for `blocks` blocks.
-// Layout: slots (words_per_block * blocks u64) | lens (blocks u32, padded) |
-// tile sums (tiles u64).
+// Scratch requirements of the generic encoder, in bytes, for `blocks` blocks: enough for either layout. That of the slots
+// is slots (words_per_block * blocks u64) | lens (blocks u32, padded) | tile sums (tiles u64).
 uint64_t gcow_encode_generic_scratch_bytes(const int32_t* params, uint64_t blocks, int dim) {
   ZfpParams p = load_params(params);
   uint64_t wpb = (max_block_bits(p, dim) + 63) / 64;
   uint64_t tiles = (blocks + kScanTile - 1) / kScanTile;
-  return wpb * blocks * 8 + ((blocks * 4 + 7) & ~7ull) + tiles * 8 + 64;
+  const uint64_t slots = wpb * blocks * 8 + ((blocks * 4 + 7) & ~7ull) + tiles * 8 + 64;
+  const uint64_t strings = gcow_tile_usable(params, blocks, dim) ? gcow_encode_tiles_scratch_bytes(params, blocks, dim) : 0;
+  return slots > strings ? slots : strings;
 }
 
 // Generic encode (any mode, dim 1 or 2). `out` must hold max_output_bytes and

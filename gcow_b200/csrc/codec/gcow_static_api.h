@@ -10,10 +10,10 @@
 // cannot use gcow_encode_generic(), which needs a caller-allocated scratch area
 // sized by gcow_encode_generic_scratch_bytes().
 //
-// gcow_encode_generic_static() performs the same two-pass encode (per-block
-// slots, prefix sum of the block lengths, bit-offset scatter) but keeps its
-// scratch in a fixed array inside the library. Consequences the caller must
-// know:
+// gcow_encode_generic_static() performs the same encode (blocks coded into
+// scratch, their lengths summed up, the codes moved into place; in one kernel
+// and without scratch where the places are known) but keeps its scratch in a
+// fixed array inside the library. Consequences the caller must know:
 //   * Capacity is fixed: the scratch a call needs (the value
 //     gcow_encode_generic_scratch_bytes() would return) must not exceed
 //     gcow_encode_generic_static_capacity() = 8 MiB, e.g. up to about 109 000

@@ -343,11 +343,6 @@ struct WindowReader {
       o -= 32;
     }
   }
-  GCOW_HD uint64_t get(uint32_t n) {                       // n <= 32
-    const uint32_t r = n ? peek() & low_mask32(n) : 0u;
-    skip(n);
-    return r;
-  }
 };
 
 // One block of 4 from a window. `tab`: the lean coder's decoder windows and nibble pairs, then at kTileRows one plane per

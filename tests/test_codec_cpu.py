@@ -450,3 +450,21 @@ def test_window_decoder_of_the_tiles(maxprec, maxbits):
         words[1:, 0] |= np.uint32(1 << skip)                    # blocks that are not empty
         par = ZfpParams(1, maxbits, maxprec, -1074)
         assert lib.gcow_window_decode_check(words.ctypes.data, words.shape[0], words.shape[1], skip, par.as_c()) == 0
+
+
+def test_generic_scratch_holds_either_layout():
+    """The entry point that takes the caller's scratch goes through the slots or through the tile kernels."""
+    try:
+        cu = _native.cuda()
+    except Exception as e:
+        pytest.skip(f"CUDA library not loadable: {e}")
+    u64, i32, ptr = C.c_uint64, C.c_int, C.c_void_p
+    tiles = cu.gcow_encode_tiles_scratch_bytes
+    tiles.restype, tiles.argtypes = u64, [ptr, u64, i32]
+    cu.gcow_tile_usable.argtypes = [ptr, u64, i32]
+    for dim in (1, 2):
+        for p in [ZfpParams(1, 16658, prec, -1074) for prec in (0, 1, 2, 5, 32, 64)] + [ZfpParams(1, b, 64, -1074) for b in (9, 63, 64, 65, 160)]:
+            if not cu.gcow_tile_usable(p.as_c(), 1, dim):
+                continue
+            for blocks in (*range(1, 300), 1023, 1024, 1025, 1 << 20, (1 << 32) + 1):
+                assert tiles(p.as_c(), blocks, dim) <= cu.gcow_encode_generic_scratch_bytes(p.as_c(), blocks, dim)
