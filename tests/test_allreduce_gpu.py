@@ -215,3 +215,29 @@ def test_out_that_does_not_fit_is_refused():
         with pytest.raises(TypeError):
             ar(x, out=out)
     assert torch.equal(ar(x, out=torch.empty(1000, device="cuda")), x)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rate", [4, 8, 16, 32])
+def test_single_rank_feedback_with_a_partial_block(rate):
+    """The one-rank kernel against the resident one, which runs when phases are traced, bit for bit: values, residual, and
+    nothing past the end of either. The padding of the last block has no residual."""
+    plain, traced = (CompressedAllReduce(1 << 16, GcowConfig(rate=rate)) for _ in range(2))
+    traced.enable_tracing()
+    for n in (1, 2, 3, 257, 1026, 40003):
+        for off in (0, 1):
+            got = []
+            for ar in (plain, traced):
+                x, out, res = (torch.full((n + 8,), 7.0, device="cuda") for _ in range(3))
+                x[off:off + n] = torch.from_numpy(gen(n, n)).cuda()
+                res[off:off + n] = torch.from_numpy(gen(n + 1, n)).cuda() * 0.1
+                total = (x + res)[off:off + n]
+                ar(x[off:off + n], out=out[off:off + n], residual=res[off:off + n], variant="oneshot")
+                assert torch.equal(res[off:off + n], total - out[off:off + n])
+                for t in (out, res):
+                    assert bool((t[:off] == 7).all()) and bool((t[off + n:] == 7).all())
+                got.append((out, res))
+            for a, b in zip(*got):
+                assert torch.equal(a.view(torch.int32), b.view(torch.int32)), (n, off)
+    plain.check()
+    traced.check()
