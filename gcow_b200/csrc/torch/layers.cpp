@@ -89,7 +89,7 @@ std::atomic<int64_t> g_launches{0}, g_view_hits{0};
 std::mutex g_error_mu;
 Tensor g_error[64];
 
-constexpr int kOutF32 = 1, kBias = 2, kGelu = 4, kResidual = 8, kAuxOut = 32, kGeluGrad = 64;
+constexpr int kOutF32 = 1, kBias = 2, kGelu = 4, kResidual = 8, kAccumulate = 16, kAuxOut = 32, kGeluGrad = 64;
 
 void check(int err, const char* what) {
   TORCH_CHECK(err == 0, what, " refused the call: ", err);
@@ -144,6 +144,7 @@ void dims(const char* what, const Tensor& t, int64_t n) {
 }
 
 // ------------------------------------------------------------------------ products
+// Whether the device can co-schedule clusters of two CTAs with the pair kernel's shared memory, and GCOW_GEMM2 is not 0.
 bool pair_gemm_enabled() {
   static const bool on = !env_off("GCOW_GEMM2") && gcow_gemm2_max_pairs() > 0;
   return on;
@@ -151,20 +152,22 @@ bool pair_gemm_enabled() {
 
 struct GemmOpts {
   Tensor bias, residual, pre_gelu_out, gelu_grad_of, out;
-  bool gelu = false, a_t = false, b_t = false, out_f32 = false;
+  bool gelu = false, a_t = false, b_t = false, out_f32 = false, accumulate = false;
+  int max_ctas = 0, tile_rows = 0;       // of the one-CTA kernel; 0: chosen from the sizes
+  int pair = -1;                         // 1: the CTA-pair kernel wherever it can, 0: never, -1: by the rule below
 };
 
-// C[M,N] = op(A) op(B)^T with the epilogues of the tcgen05 kernels; the routing rule and its reasons are those of
-// ops/kernels.py::gemm_bf16.
+// C[M,N] = op(A) op(B)^T with the epilogues of the tcgen05 kernels.
 Tensor gemm(const Tensor& a, const Tensor& b, const GemmOpts& o, const On& on) {
-  const int64_t M = o.a_t ? a.size(1) : a.size(0), K = o.a_t ? a.size(0) : a.size(1);
-  const int64_t N = o.b_t ? b.size(1) : b.size(0), Kb = o.b_t ? b.size(0) : b.size(1);
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && a.stride(1) == 1 &&
               b.stride(1) == 1, "gemm: the operands have to be bf16 matrices with contiguous rows");
+  const int64_t M = o.a_t ? a.size(1) : a.size(0), K = o.a_t ? a.size(0) : a.size(1);
+  const int64_t N = o.b_t ? b.size(1) : b.size(0), Kb = o.b_t ? b.size(0) : b.size(1);
   TORCH_CHECK(K == Kb, "gemm: reduction lengths differ");
   Tensor out = o.out.defined() ? o.out : empty({M, N}, o.out_f32 ? at::kFloat : at::kBFloat16, a);
   const Tensor& aux = o.pre_gelu_out.defined() ? o.pre_gelu_out : o.gelu_grad_of;
-  TORCH_CHECK(out.size(0) == M && out.size(1) == N, "gemm: the result has another shape than the product");
+  TORCH_CHECK(out.dim() == 2 && out.size(0) == M && out.size(1) == N, "gemm: the result has another shape than the product");
+  TORCH_CHECK(out.scalar_type() == at::kFloat || out.scalar_type() == at::kBFloat16, "gemm: the result has to be float32 or bf16");
   TORCH_CHECK(!o.bias.defined() || (o.bias.numel() == N && o.bias.scalar_type() == at::kFloat && o.bias.is_contiguous()),
               "gemm: the bias has to be a float32 vector as long as the product's rows");
   TORCH_CHECK(!o.residual.defined() || (o.residual.sizes() == out.sizes() && o.residual.strides() == out.strides() &&
@@ -175,11 +178,16 @@ Tensor gemm(const Tensor& a, const Tensor& b, const GemmOpts& o, const On& on) {
               "gemm: the GELU's side tensor has another shape or type than the product");
   on_device_of(a, {&b, &out, &o.bias, &o.residual, &aux});
   int flags = (out.scalar_type() == at::kFloat ? kOutF32 : 0) | (o.bias.defined() ? kBias : 0) | (o.gelu ? kGelu : 0) |
-              (o.residual.defined() ? kResidual : 0);
+              (o.residual.defined() ? kResidual : 0) | (o.accumulate ? kAccumulate : 0);
   if (aux.defined()) flags |= o.pre_gelu_out.defined() ? kAuxOut : kGeluGrad;
   const int lda = (int)a.stride(0), ldb = (int)b.stride(0), ldc = (int)out.stride(0);
-  if (pair_gemm_enabled() && !o.a_t && !(flags & kOutF32) && K % 64 == 0 && K >= 512 && N % (o.b_t ? 64 : 32) == 0 && M >= 1024 &&
-      N >= 256 && lda % 8 == 0 && ldb % 8 == 0 && ldc % 8 == 0 && !(K >= 2048 && ((M + 255) / 256) * ((N + 255) / 256) >= 118)) {
+  // A large product with a short reduction goes to CTA pairs: two SMs per 256 x 256 tile have the one-CTA tile's traffic per
+  // flop and an overlapped epilogue as well. Long reductions stay on the one-CTA tile, and so do those below 512 (the 1x1
+  // convolutions of a ResNet), which the output stream bounds: the one-CTA kernel's TMA stores are 15 to 30 % faster there.
+  const bool can_pair = pair_gemm_enabled() && !o.a_t && !(flags & (kOutF32 | kAccumulate)) && !o.max_ctas && !o.tile_rows;
+  const bool by_rule = K % 64 == 0 && K >= 512 && N % (o.b_t ? 64 : 32) == 0 && M >= 1024 && N >= 256 && lda % 8 == 0 && ldb % 8 == 0 &&
+                       ldc % 8 == 0 && !(K >= 2048 && ((M + 255) / 256) * ((N + 255) / 256) >= 118);
+  if (can_pair && (o.pair < 0 ? by_rule : o.pair > 0)) {
     const int err = gcow_gemm2_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, lda, ldb, ldc, f32(o.bias),
                                     raw(o.residual), raw(aux), flags, on.error, o.b_t, on.stream);
     if (err == 0) { g_launches++; return out; }
@@ -187,10 +195,10 @@ Tensor gemm(const Tensor& a, const Tensor& b, const GemmOpts& o, const On& on) {
   }
   if (aux.defined())
     check(gcow_gemm_bf16_aux(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, lda, ldb, ldc, f32(o.bias),
-                             raw(o.residual), raw(aux), flags, on.error, o.a_t, o.b_t, 0, on.stream), "gcow_gemm_bf16_aux");
+                             raw(o.residual), raw(aux), flags, on.error, o.a_t, o.b_t, o.tile_rows, on.stream), "gcow_gemm_bf16_aux");
   else
     check(gcow_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, lda, ldb, ldc, f32(o.bias),
-                         raw(o.residual), flags, on.error, 0, o.a_t, o.b_t, 0, on.stream), "gcow_gemm_bf16");
+                         raw(o.residual), flags, on.error, o.max_ctas, o.a_t, o.b_t, o.tile_rows, on.stream), "gcow_gemm_bf16");
   g_launches++;
   return out;
 }
@@ -203,9 +211,16 @@ Tensor add_parts(const Tensor& part, int64_t parts, c10::IntArrayRef shape, Tens
   return out;
 }
 
-// dW[N,K] = g^T x, fp32, the long reduction split into slabs whose products are added in order (ops/kernels.py::wgrad_gemm).
+// dW[N,K] = g^T x, fp32, for g [M,N] and x [M,K], both stored with the reduction dimension M outermost. The result has few tiles
+// while M is long, so the rows are cut into `s` slabs that run as one batched launch and whose products are added in order: `s`
+// doubles while the tiles still fit one wave of 148 CTAs and a slab keeps at least 512 rows.
 Tensor wgrad(const Tensor& g, const Tensor& x, const Tensor& out, const On& on) {
+  TORCH_CHECK(g.dim() == 2 && x.dim() == 2 && g.size(0) == x.size(0) && g.scalar_type() == at::kBFloat16 && x.scalar_type() == at::kBFloat16 &&
+              g.stride(1) == 1 && x.stride(1) == 1, "wgrad: expected two bf16 matrices with contiguous rows, as many in each");
   const int64_t M = g.size(0), N = g.size(1), K = x.size(1);
+  TORCH_CHECK(!out.defined() || (out.dim() == 2 && out.size(0) == N && out.size(1) == K && out.scalar_type() == at::kFloat && out.is_contiguous()),
+              "wgrad: the result has to be a contiguous float32 matrix of the product's shape");
+  on_device_of(g, {&x, &out});
   const int64_t tiles = ((N + 127) / 128) * ((K + 255) / 256);
   int64_t s = 1;
   while (s < 64 && tiles * s * 2 <= 148 && M % (2 * s) == 0 && (M / (2 * s)) % 64 == 0 && M / (2 * s) >= 512) s *= 2;
@@ -223,9 +238,11 @@ Tensor wgrad(const Tensor& g, const Tensor& x, const Tensor& out, const On& on) 
   return add_parts(part, s, {N, K}, out, on);
 }
 
+// fp32 column sums of a bf16 matrix (bias gradient)
 Tensor colsum(const Tensor& g, const On& on) {
   const int64_t rows = g.size(0), cols = g.size(1);
   if (cols % 2 || g.stride(1) != 1 || g.stride(0) % 2) return g.to(at::kFloat).sum(0);
+  TORCH_CHECK(g.dim() == 2 && g.scalar_type() == at::kBFloat16, "colsum: expected a bf16 matrix");
   const Tensor part = empty({gcow_colsum_parts((int)rows) * cols}, at::kFloat, g), out = empty({cols}, at::kFloat, g);
   check(gcow_colsum(g.data_ptr(), f32(part), f32(out), (int)rows, (int)cols, (int)g.stride(0), on.stream), "gcow_colsum");
   g_launches += 2;
@@ -244,7 +261,7 @@ PyObject* attr(PyObject* o, PyObject* name) {
   return v;
 }
 
-// ops/kernels.py::bf16_weight
+// ops/kernels.py::bf16_weight, for the weights of the layers below
 Tensor bf16_weight(PyObject* obj) {
   const Tensor& w = THPVariable_Unpack(obj);
   PyObject* sh = attr(obj, name_bf16());
@@ -271,7 +288,11 @@ Tensor bf16_weight(PyObject* obj) {
   return copy;
 }
 
-// Where a weight's gradient may be written (ops/kernels.py::take_grad_view): taken at most once per step.
+// The float32 tensor this step's gradient of a weight may be written into, or none. A trainer that knows where the gradient
+// will end up (DDP's bucket view, i.e. last step's .grad) leaves it in the weight's _gcow_grad_view before it drops the
+// gradients; the first layer to use the weight in a forward pass takes it, so two uses of one weight never share it. The
+// weight-gradient kernels then write there and the backward returns an alias of that memory: autograd adopts it as the
+// weight's .grad and DDP, seeing its own bucket memory, copies nothing.
 Tensor take_grad_view(PyObject* obj) {
   const Tensor& w = THPVariable_Unpack(obj);
   if (w.scalar_type() != at::kFloat) return Tensor();
@@ -287,7 +308,8 @@ Tensor take_grad_view(PyObject* obj) {
 // A gradient target held by a backward function. `w` is the weight itself: its .grad tells whether gradients accumulate.
 struct Target { Tensor view, weight; };
 
-// The [rows, cols] fp32 matrix to write (undefined where there is none) and the tensor to return as the gradient.
+// The [rows, cols] fp32 matrix to write (undefined where there is none) and the tensor to return as the gradient. `align`: what
+// the writing kernel needs of the address (the GEMM and convolution epilogues store 16 bytes at a time).
 Tensor target_matrix(const Target& t, int64_t rows, int64_t cols, uintptr_t align, Tensor* result) {
   if (!t.view.defined() || t.weight.grad().defined()) return Tensor();
   const Tensor flat = t.view.dim() == 4 ? t.view.permute({0, 2, 3, 1}) : t.view;
@@ -621,12 +643,16 @@ PyObject* fused_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) { 
   END_HANDLE_TH_ERRORS
 }
 
-// C[i] = op(A[i]) op(B[i])^T for contiguous [batch, rows, cols] operands
-Tensor bmm(const Tensor& a, const Tensor& b, bool a_t, bool b_t, const On& on) {
+// C[i] = op(A[i]) op(B[i])^T for [batch, rows, cols] operands with contiguous rows
+Tensor bmm(const Tensor& a, const Tensor& b, bool a_t, bool b_t, const On& on, bool out_f32 = false) {
+  TORCH_CHECK(a.dim() == 3 && b.dim() == 3 && a.size(0) == b.size(0) && a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 &&
+              a.stride(2) == 1 && b.stride(2) == 1, "bmm: expected two bf16 batches of matrices with contiguous rows, as many in each");
   const int64_t batch = a.size(0), M = a_t ? a.size(2) : a.size(1), K = a_t ? a.size(1) : a.size(2), N = b_t ? b.size(2) : b.size(1);
-  Tensor out = empty({batch, M, N}, at::kBFloat16, a);
+  TORCH_CHECK(K == (b_t ? b.size(1) : b.size(2)), "bmm: reduction lengths differ");
+  on_device_of(a, {&b});
+  Tensor out = empty({batch, M, N}, out_f32 ? at::kFloat : at::kBFloat16, a);
   check(gcow_gemm_bf16_batched(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, (int)a.stride(1), (int)b.stride(1),
-                               (int)N, (int)batch, a.stride(0), b.stride(0), M * N, nullptr, nullptr, 0, on.error, a_t, b_t, 128, on.stream),
+                               (int)N, (int)batch, a.stride(0), b.stride(0), M * N, nullptr, nullptr, out_f32 ? kOutF32 : 0, on.error, a_t, b_t, 128, on.stream),
         "gcow_gemm_bf16_batched");
   g_launches++;
   return out;
@@ -684,10 +710,12 @@ PyObject* attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {      /
 // ---------------------------------------------------------------------- convolutions (NHWC bf16)
 struct ConvShape { int N, C, H, W, Co, KH, KW, OH, OW, ph, pw; };
 
+// 64 -> 64 channels, 3x3, stride 1, padding 1: the weight-stationary kernel (pixels as the MMA's N).
 bool conv_ws(const ConvShape& s) {
   return s.C == 64 && s.Co == 64 && s.KH == 3 && s.KW == 3 && s.ph == 1 && s.pw == 1 && !env_off("GCOW_CONV_WS") &&
          gcow_conv_ws_usable(s.N, s.H, s.W);
 }
+// Ci -> 128 channels, 3x3, stride 1, padding 1, tiles that fit the shared memory: the halo-tile kernel.
 bool conv_halo(const ConvShape& s) {
   return s.Co == 128 && s.KH == 3 && s.KW == 3 && s.ph == 1 && s.pw == 1 && !env_off("GCOW_CONV_HALO") &&
          gcow_conv_halo_usable(s.N, s.H, s.W, s.C);
@@ -990,6 +1018,92 @@ PyObject* batchnorm_act(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
+// ---------------------------------------------------------------------- the products and rules by themselves
+// gemm(a, b, bias, residual, gelu, out, out_f32, accumulate, max_ctas, a_t, b_t, tile_rows, pre_gelu_out, gelu_grad_of, pair)
+PyObject* py_gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 15, "gemm: bad arguments");
+  const Tensor a = need(args[0]), b = need(args[1]);
+  GemmOpts o;
+  o.bias = arg(args[2]);
+  o.residual = arg(args[3]);
+  o.gelu = PyObject_IsTrue(args[4]) == 1;
+  o.out = arg(args[5]);
+  o.out_f32 = PyObject_IsTrue(args[6]) == 1;
+  o.accumulate = PyObject_IsTrue(args[7]) == 1;
+  o.max_ctas = (int)PyLong_AsLong(args[8]);
+  o.a_t = PyObject_IsTrue(args[9]) == 1;
+  o.b_t = PyObject_IsTrue(args[10]) == 1;
+  o.tile_rows = (int)PyLong_AsLong(args[11]);
+  o.pre_gelu_out = arg(args[12]);
+  o.gelu_grad_of = arg(args[13]);
+  if (args[14] != Py_None) o.pair = PyObject_IsTrue(args[14]) == 1;
+  if (PyErr_Occurred()) return nullptr;
+  const On on(a);
+  return THPVariable_Wrap(gemm(a, b, o, on));
+  END_HANDLE_TH_ERRORS
+}
+PyObject* py_wgrad(PyObject*, PyObject* const* args, Py_ssize_t nargs) {       // (g, x, out or None)
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 3, "wgrad: bad arguments");
+  const Tensor g = need(args[0]), x = need(args[1]), out = arg(args[2]);
+  const On on(g);
+  return THPVariable_Wrap(wgrad(g, x, out, on));
+  END_HANDLE_TH_ERRORS
+}
+PyObject* py_bmm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {         // (a, b, a_t, b_t, out_f32)
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 5, "bmm: bad arguments");
+  const Tensor a = need(args[0]), b = need(args[1]);
+  const On on(a);
+  return THPVariable_Wrap(bmm(a, b, PyObject_IsTrue(args[2]) == 1, PyObject_IsTrue(args[3]) == 1, on, PyObject_IsTrue(args[4]) == 1));
+  END_HANDLE_TH_ERRORS
+}
+PyObject* py_colsum(PyObject*, PyObject* g) {
+  HANDLE_TH_ERRORS
+  const Tensor t = need(g);
+  at::NoGradGuard no_grad;
+  const On on(t);
+  return THPVariable_Wrap(colsum(t, on));
+  END_HANDLE_TH_ERRORS
+}
+PyObject* py_take_grad_view(PyObject*, PyObject* w) {                          // the view, or None
+  HANDLE_TH_ERRORS
+  need(w);
+  Tensor v = take_grad_view(w);
+  if (!v.defined()) Py_RETURN_NONE;
+  return THPVariable_Wrap(std::move(v));
+  END_HANDLE_TH_ERRORS
+}
+PyObject* py_grad_target(PyObject*, PyObject* const* args, Py_ssize_t nargs) { // (view, weight, rows, cols, align) -> (matrix, gradient)
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 5, "grad_target: bad arguments");
+  const Target t{need(args[0]), need(args[1])};
+  const int64_t rows = PyLong_AsLongLong(args[2]), cols = PyLong_AsLongLong(args[3]), align = PyLong_AsLongLong(args[4]);
+  if (PyErr_Occurred()) return nullptr;
+  TORCH_CHECK(align > 0, "grad_target: bad alignment");
+  Tensor result;
+  Tensor flat = target_matrix(t, rows, cols, (uintptr_t)align, &result);
+  if (!flat.defined()) return PyTuple_Pack(2, Py_None, Py_None);
+  PyObject *a = THPVariable_Wrap(std::move(flat)), *b = THPVariable_Wrap(std::move(result));
+  PyObject* r = a && b ? PyTuple_Pack(2, a, b) : nullptr;
+  Py_XDECREF(a);
+  Py_XDECREF(b);
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+// conv_rules(N, H, W, C, Co, KH, KW, pad_h, pad_w) -> (weight-stationary, halo-tile): which of the two stride-1 kernels apply
+PyObject* conv_rules(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 9, "conv_rules: bad arguments");
+  int v[9];
+  for (int i = 0; i < 9; i++) v[i] = (int)PyLong_AsLong(args[i]);
+  if (PyErr_Occurred()) return nullptr;
+  const ConvShape s{v[0], v[3], v[1], v[2], v[4], v[5], v[6], 0, 0, v[7], v[8]};
+  return PyTuple_Pack(2, conv_ws(s) ? Py_True : Py_False, conv_halo(s) ? Py_True : Py_False);
+  END_HANDLE_TH_ERRORS
+}
+
 // ---------------------------------------------------------------------- bookkeeping
 PyObject* launches(PyObject*, PyObject*) { return PyLong_FromLongLong(g_launches.load()); }
 PyObject* view_hits(PyObject*, PyObject*) { return PyLong_FromLongLong(g_view_hits.load()); }
@@ -1032,7 +1146,13 @@ Tensor error_word(int device) {
 #define GCOW_FAST(name) {#name, (PyCFunction)(void (*)())name, METH_FASTCALL, nullptr}
 PyMethodDef layer_methods[] = {
     GCOW_FAST(linear), GCOW_FAST(ffn_residual), GCOW_FAST(layernorm), GCOW_FAST(fused_attention), GCOW_FAST(attention),
-    GCOW_FAST(conv), GCOW_FAST(conv1x1), GCOW_FAST(batchnorm_act),
+    GCOW_FAST(conv), GCOW_FAST(conv1x1), GCOW_FAST(batchnorm_act), GCOW_FAST(conv_rules),
+    {"gemm", (PyCFunction)(void (*)())py_gemm, METH_FASTCALL, nullptr},
+    {"wgrad", (PyCFunction)(void (*)())py_wgrad, METH_FASTCALL, nullptr},
+    {"bmm", (PyCFunction)(void (*)())py_bmm, METH_FASTCALL, nullptr},
+    {"colsum", py_colsum, METH_O, nullptr},
+    {"take_grad_view", py_take_grad_view, METH_O, nullptr},
+    {"grad_target", (PyCFunction)(void (*)())py_grad_target, METH_FASTCALL, nullptr},
     {"launches", launches, METH_NOARGS, nullptr},
     {"view_hits", view_hits, METH_NOARGS, nullptr},
     {"error_word", py_error_word, METH_O, nullptr},

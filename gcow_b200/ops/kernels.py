@@ -5,16 +5,12 @@ alignment); callers fall back to PyTorch otherwise.
 """
 from __future__ import annotations
 
-import os
-
 import torch
 
 from .. import _native
 
 _launches = 0
 _err_words: dict = {}
-
-OUT_F32, BIAS, GELU, RESIDUAL, ACCUMULATE, AUX_OUT, GELU_GRAD = 1, 2, 4, 8, 16, 32, 64
 
 
 def launch_count() -> int:
@@ -160,12 +156,22 @@ def bf16_weight(w: torch.Tensor) -> torch.Tensor:
     return sh
 
 
+# The CTA-pair GEMM (cta_group::2): None: by the rule of csrc/torch/layers.cpp, unless GCOW_GEMM2=0; True: wherever the
+# kernel can; False: never.
+_pair_gemm = None
+
+
+def _out_type(dtype) -> None:
+    if dtype not in (torch.bfloat16, torch.float32):
+        raise TypeError("the products come in bf16 or float32")
+
+
 def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, bias: torch.Tensor | None = None,
               residual: torch.Tensor | None = None, gelu: bool = False, out_dtype=torch.bfloat16,
               out: torch.Tensor | None = None, accumulate: bool = False, max_ctas: int = 0,
               a_t: bool = False, b_t: bool = False, tile_rows: int = 0,
               pre_gelu_out: torch.Tensor | None = None, gelu_grad_of: torch.Tensor | None = None) -> torch.Tensor:
-    """C[M,N] = op(A) @ op(B)^T (+bias) (GELU) (+residual) on the tcgen05 kernel.
+    """C[M,N] = op(A) @ op(B)^T (+bias) (GELU) (+residual) on the tcgen05 kernels.
 
     ``pre_gelu_out`` (bf16 [M,N], with ``gelu``): also receives the value before the GELU, which its
     gradient needs. ``gelu_grad_of`` (bf16 [M,N]): the product is multiplied by GELU'(that tensor) before
@@ -175,143 +181,32 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, bias: torch.Tensor | None = N
     copy). b: bf16 [N,K] (or [K,N] with ``b_t``). Last dimension contiguous, leading
     dimensions multiples of 8. bias: fp32 [N]. residual/out: [M,N] of ``out_dtype``.
     ``tile_rows`` forces the 128- or 256-row tile (0: chosen from the problem size)."""
-    global _launches
-    assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.dim() == 2 and b.dim() == 2
-    assert a.stride(1) == 1 and b.stride(1) == 1
-    (K, M) = a.shape if a_t else a.shape[::-1]
-    (Kb, N) = b.shape if b_t else b.shape[::-1]
-    assert K == Kb, (a.shape, b.shape, a_t, b_t)
-    if out is None:
-        out = torch.empty((M, N), dtype=out_dtype, device=a.device)
-    flags = (OUT_F32 if out.dtype == torch.float32 else 0) | (BIAS if bias is not None else 0) | \
-        (GELU if gelu else 0) | (RESIDUAL if residual is not None else 0) | (ACCUMULATE if accumulate else 0)
-    if bias is not None:
-        assert bias.dtype == torch.float32 and bias.is_contiguous() and bias.numel() == N
-    if residual is not None:
-        assert residual.dtype == out.dtype and residual.stride() == out.stride()
-    aux = pre_gelu_out if pre_gelu_out is not None else gelu_grad_of
-    if aux is not None:
-        assert pre_gelu_out is None or gelu_grad_of is None
-        flags |= AUX_OUT if pre_gelu_out is not None else GELU_GRAD
-    if (_pair_gemm_enabled() and not a_t and out.dtype == torch.bfloat16 and not accumulate and max_ctas == 0
-            and tile_rows == 0 and K % 64 == 0 and K >= 512 and N % (64 if b_t else 32) == 0 and M >= 1024 and N >= 256
-            and a.stride(0) % 8 == 0 and b.stride(0) % 8 == 0 and out.stride(0) % 8 == 0
-            and not (K >= 2048 and -(-M // 256) * -(-N // 256) >= 118)):
-        # large product with a short reduction: the CTA-pair kernel (two SMs per 256 x 256 tile) has the one-CTA
-        # 256 x 256 tile's traffic per flop AND an overlapped epilogue; long reductions stay on the one-CTA tile, and
-        # so do reductions below 512 (the 1x1 convolutions of a ResNet), which are bound by the output stream: there
-        # the one-CTA kernel's TMA-store epilogue is 15-30 % faster
-        err = _native.cuda().gcow_gemm2_bf16(
-            a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
-            bias.data_ptr() if bias is not None else None, residual.data_ptr() if residual is not None else None,
-            aux.data_ptr() if aux is not None else None, flags, _error_word(a.device).data_ptr(), int(b_t),
-            _stream(a.device))
-        if err == 0:
-            _launches += 1
-            return out
-        if err != -2:
-            raise RuntimeError(f"gcow_gemm2_bf16 refused the call: {err}")
-    if aux is not None:
-        assert aux.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and aux.shape == out.shape
-        assert aux.stride() == out.stride() and N % 32 == 0 and max_ctas == 0
-        err = _native.cuda().gcow_gemm_bf16_aux(
-            a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
-            bias.data_ptr() if bias is not None else None, residual.data_ptr() if residual is not None else None,
-            aux.data_ptr(), flags, _error_word(a.device).data_ptr(), int(a_t), int(b_t), int(tile_rows),
-            _stream(a.device))
-    else:
-        err = _native.cuda().gcow_gemm_bf16(
-            a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
-            bias.data_ptr() if bias is not None else None, residual.data_ptr() if residual is not None else None,
-            flags, _error_word(a.device).data_ptr(), max_ctas, int(a_t), int(b_t), int(tile_rows),
-            _stream(a.device))
-    if err:
-        raise RuntimeError(f"gcow_gemm_bf16 refused the call: {err}")
-    _launches += 1
-    return out
-
-
-_pair_gemm = None
-
-
-def _pair_gemm_enabled() -> bool:
-    """The CTA-pair GEMM (cta_group::2) serves large products with a short reduction unless GCOW_GEMM2=0, provided
-    the device can co-schedule clusters of two CTAs with its shared-memory footprint."""
-    global _pair_gemm
-    if _pair_gemm is None:
-        import os
-        _pair_gemm = (os.environ.get("GCOW_GEMM2", "1") != "0" and _have("gcow_gemm2_bf16")
-                      and _native.cuda().gcow_gemm2_max_pairs() > 0)
-    return _pair_gemm
+    _out_type(out_dtype)
+    return (_native._ext or _native.ext()).gemm(a, b, bias, residual, gelu, out, out_dtype == torch.float32, accumulate, max_ctas,
+                                                a_t, b_t, tile_rows, pre_gelu_out, gelu_grad_of, _pair_gemm)
 
 
 def take_grad_view(w: torch.Tensor):
-    """The float32 tensor this step's gradient of ``w`` may be written into, or None. A trainer that knows where the
-    gradient will end up (DDP's bucket view, i.e. last step's ``w.grad``) leaves it in ``w._gcow_grad_view`` before it
-    drops the gradients; the first layer to use ``w`` in a forward pass takes it, so two uses of one weight never share
-    it. The weight-gradient kernels then write there and the backward returns an alias of that memory: autograd adopts
-    it as ``w.grad`` and DDP, seeing its own bucket memory, copies nothing."""
-    gv = getattr(w, "_gcow_grad_view", None)
-    if gv is None:
-        return None
-    w._gcow_grad_view = None
-    if gv.dtype != torch.float32 or gv.shape != w.shape or gv.device != w.device:
-        return None
-    return (gv, w)
+    """(tensor, w) for the float32 tensor that this step's gradient of ``w`` may be written into, or None: what a layer
+    takes from ``w._gcow_grad_view`` (csrc/torch/layers.cpp, take_grad_view)."""
+    gv = _native.ext().take_grad_view(w)
+    return None if gv is None else (gv, w)
 
 
 def _grad_target(taken, rows: int, cols: int, align: int = 16):
-    """(flat [rows, cols] view to write into, tensor to return as the gradient) or (None, None). ``align``: what the
-    writing kernel needs of the address (the GEMM and convolution epilogues store 16 bytes at a time)."""
-    if taken is None:
-        return None, None
-    gv, w = taken
-    if w.grad is not None:                       # gradients are being accumulated: that memory is in use
-        return None, None
-    flat = gv.permute(0, 2, 3, 1) if gv.dim() == 4 else gv
-    if not flat.is_contiguous() or flat.numel() != rows * cols:
-        return None, None
-    flat = flat.reshape(rows, cols)
-    if flat.data_ptr() != gv.data_ptr() or gv.data_ptr() % align:
-        return None, None
-    global _grad_view_hits
-    _grad_view_hits += 1
-    return flat, gv.as_strided(gv.shape, gv.stride())
-
-
-_grad_view_hits = 0
+    """(flat [rows, cols] view to write into, tensor to return as the gradient) or (None, None) (target_matrix there)."""
+    return (None, None) if taken is None else _native.ext().grad_target(*taken, rows, cols, align)
 
 
 def grad_view_hits() -> int:
     """How many weight gradients were written straight into the tensor the trainer pointed at (see take_grad_view)."""
-    return _grad_view_hits + (_native._ext.view_hits() if _native._ext is not None else 0)
+    return _native._ext.view_hits() if _native._ext is not None else 0
 
 
 def wgrad_gemm(g: torch.Tensor, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-    """dW[N, K] = g^T x for g [M, N], x [M, K] (both stored with the reduction dimension M outermost), fp32.
-    The output has few tiles while M is long, so the reduction is split across CTAs: the rows are cut into
-    ``s`` slabs that run as one batched launch, and the ``s`` partial products are added in a fixed order.
-    ``out`` (contiguous fp32 [N, K]): where the result goes."""
-    global _launches
-    M, N = g.shape
-    K = x.shape[1]
-    tiles = -(-N // 128) * -(-K // 256)
-    s = 1        # doubled while the tiles still fit one wave of 148 CTAs and a slab keeps at least 512 rows
-    while s < 64 and tiles * s * 2 <= 148 and M % (2 * s) == 0 and (M // (2 * s)) % 64 == 0 and M // (2 * s) >= 512:
-        s *= 2
-    if s == 1 or g.stride(0) != N or x.stride(0) != K:
-        return gemm_bf16(g, x, a_t=True, b_t=True, out_dtype=torch.float32, out=out)
-    lib = _native.cuda()
-    part = _ws("wgrad_part", (s, N, K), torch.float32, g.device)
-    err = lib.gcow_gemm_bf16_batched(
-        g.data_ptr(), x.data_ptr(), part.data_ptr(), N, K, M // s, N, K, K, s, (M // s) * N, (M // s) * K, N * K,
-        None, None, OUT_F32, _error_word(g.device).data_ptr(), 1, 1, 0, _stream(g.device))
-    _chk(err, "gcow_gemm_bf16_batched")
-    if out is None:
-        out = torch.empty((N, K), dtype=torch.float32, device=g.device)
-    _chk(lib.gcow_reduce_partials(part.data_ptr(), out.data_ptr(), s, N * K, _stream(g.device)), "gcow_reduce_partials")
-    _launches += 2
-    return out
+    """dW[N, K] = g^T x for g [M, N], x [M, K] (both stored with the reduction dimension M outermost), fp32, the long
+    reduction split across CTAs. ``out`` (contiguous fp32 [N, K]): where the result goes."""
+    return (_native._ext or _native.ext()).wgrad(g, x, out)
 
 
 def _pad_rows(t: torch.Tensor, rows: int) -> torch.Tensor:
@@ -408,18 +303,7 @@ def _chk(err: int, what: str) -> None:
 
 def colsum(g: torch.Tensor) -> torch.Tensor:
     """fp32 column sums of a bf16 [rows, cols] matrix (bias gradient)."""
-    global _launches
-    rows, cols = g.shape
-    lib = _native.cuda()
-    if cols % 2 or g.stride(1) != 1 or g.stride(0) % 2:
-        return g.float().sum(0)
-    parts = lib.gcow_colsum_parts(rows)
-    part = _ws("colsum_part", parts * cols, torch.float32, g.device)
-    out = torch.empty(cols, dtype=torch.float32, device=g.device)
-    _chk(lib.gcow_colsum(g.data_ptr(), part.data_ptr(), out.data_ptr(), rows, cols, g.stride(0), _stream(g.device)),
-         "gcow_colsum")
-    _launches += 2
-    return out
+    return (_native._ext or _native.ext()).colsum(g)
 
 
 # ------------------------------------------------------------------ 1x1 conv
@@ -815,9 +699,7 @@ def embed3(ids, type_ids, tok, pos, typ):
 # ------------------------------------------------ implicit-GEMM convolution (stride 1)
 def conv_ws_usable(N, H, W, C, Co, KH, KW, pad_h, pad_w):
     """64 -> 64 channels, 3x3, stride 1, padding 1: the weight-stationary kernel (pixels as the MMA's N) applies."""
-    return (C == 64 and Co == 64 and KH == 3 and KW == 3 and pad_h == 1 and pad_w == 1
-            and os.environ.get("GCOW_CONV_WS", "1") != "0" and _have("gcow_conv_fwd_ws")
-            and bool(_native.cuda().gcow_conv_ws_usable(N, H, W)))
+    return _native.ext().conv_rules(N, H, W, C, Co, KH, KW, pad_h, pad_w)[0]
 
 
 # Narrowest image rows the halo-tile weight gradient of layers with multiples of 128 channels is routed for. Measured at
@@ -828,9 +710,7 @@ _HALO_WGRAD_MIN_W = 15
 
 def conv_halo_usable(N, H, W, C, Co, KH, KW, pad_h, pad_w):
     """Ci -> 128 channels, 3x3, stride 1, padding 1, tiles that fit the shared memory: the halo-tile kernel applies."""
-    return (Co == 128 and KH == 3 and KW == 3 and pad_h == 1 and pad_w == 1
-            and os.environ.get("GCOW_CONV_HALO", "1") != "0" and _have("gcow_conv_fwd_halo")
-            and bool(_native.cuda().gcow_conv_halo_usable(N, H, W, C)))
+    return _native.ext().conv_rules(N, H, W, C, Co, KH, KW, pad_h, pad_w)[1]
 
 
 def conv1x1_s2_usable(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -956,22 +836,8 @@ def bmm_bf16(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool =
              out_dtype=torch.bfloat16) -> torch.Tensor:
     """Batched C[i] = op(A[i]) @ op(B[i])^T on the tcgen05 kernel. a, b: bf16 [batch, rows, cols]
     with contiguous matrices (row length and batch stride multiples of 8)."""
-    global _launches
-    assert a.dim() == 3 and b.dim() == 3 and a.shape[0] == b.shape[0]
-    assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.stride(2) == 1 and b.stride(2) == 1
-    batch = a.shape[0]
-    (K, M) = (a.shape[1], a.shape[2]) if a_t else (a.shape[2], a.shape[1])
-    (Kb, N) = (b.shape[1], b.shape[2]) if b_t else (b.shape[2], b.shape[1])
-    assert K == Kb
-    out = torch.empty((batch, M, N), dtype=out_dtype, device=a.device)
-    flags = OUT_F32 if out_dtype == torch.float32 else 0
-    err = _native.cuda().gcow_gemm_bf16_batched(
-        a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(1), b.stride(1), out.stride(1), batch,
-        a.stride(0), b.stride(0), out.stride(0), None, None, flags, _error_word(a.device).data_ptr(),
-        int(a_t), int(b_t), 128, _stream(a.device))
-    _chk(err, "gcow_gemm_bf16_batched")
-    _launches += 1
-    return out
+    _out_type(out_dtype)
+    return (_native._ext or _native.ext()).bmm(a, b, a_t, b_t, out_dtype == torch.float32)
 
 
 def fused_attention_usable(qkv: torch.Tensor) -> bool:

@@ -163,3 +163,66 @@ def test_checkpoint_of_a_resnet_block(stride):
         got = _grads(net, x, lambda t: checkpoint(net, t, use_reentrant=False))
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("name", ["linear", "ffn", "conv1x1", "conv3x3", "batchnorm"])
+def test_gradient_target(name):
+    """A weight gradient goes into the tensor left in _gcow_grad_view where that fits, once per step, and nowhere near it where
+    gradients accumulate, the address is not aligned or the layout differs."""
+    from gcow_b200.ops import kernels as K
+    fn, x = _cases()[name]
+    y = fn(x)
+    weights = [v for v in _leaves(y) if v is not x and v.dim() != 1 or name == "batchnorm" and v.dim() == 1]
+    for w in weights:
+        if w.dim() == 4:                                         # as a model in channels-last memory has them
+            w.data = w.data.to(memory_format=torch.channels_last)
+    fn(x).float().square().sum().backward()
+    want = [w.grad.clone() for w in weights]
+
+    def step(left):
+        for w, v in zip(weights, left):
+            w._gcow_grad_view = v
+        hits = K.grad_view_hits()
+        fn(x).float().square().sum().backward()
+        return K.grad_view_hits() - hits
+
+    def fresh():
+        for w in weights:
+            w.grad = None
+        return [torch.full_like(w, 7.0) for w in weights]
+    left = fresh()
+    assert step(left) == len(weights)
+    for w, v, g in zip(weights, left, want):
+        assert w.grad.data_ptr() == v.data_ptr() and torch.equal(w.grad, g)
+    left = [torch.full_like(w, 7.0) for w in weights]            # .grad is there: it has to be added to
+    assert step(left) == 0
+    for w, v, g in zip(weights, left, want):
+        assert torch.equal(w.grad, 2 * g) and bool((v == 7).all())
+    if name != "batchnorm":                                      # its kernel writes single floats
+        fresh()
+        held = [torch.full((w.numel() + 1,), 7.0, device="cuda") for w in weights]
+        left = [h[1:].as_strided(w.shape, w.stride()) for h, w in zip(held, weights)]
+        assert step(left) == 0
+        for w, h, g in zip(weights, held, want):
+            assert torch.equal(w.grad, g) and bool((h == 7).all())
+    left = fresh()
+    for w, v in zip(weights, left):
+        w._gcow_grad_view = v
+    hits = K.grad_view_hits()
+    (fn(x).float().square().sum() + fn(x).float().square().sum()).backward()
+    assert K.grad_view_hits() - hits <= len(weights)             # the second use of a weight has no target
+    for w, g in zip(weights, want):
+        assert torch.equal(w.grad, 2 * g)
+
+
+def _leaves(y):
+    seen, out, todo = set(), [], [y.grad_fn]
+    while todo:
+        f = todo.pop()
+        if f is None or f in seen:
+            continue
+        seen.add(f)
+        if hasattr(f, "variable"):
+            out.append(f.variable)
+        todo += [n for n, _ in f.next_functions]
+    return out
