@@ -6,10 +6,12 @@
 // store at computed bit offsets:
 //   * fixed rate, 1-D, 16/32/64/128 bits per block: table-driven coder, one
 //     aligned store per block, fully coalesced ("fast" kernels);
-//   * every other case (1-D odd rates such as the 9-bit floor, 2-D in any mode,
-//     fixed accuracy / precision): blocks are encoded into a scratch slot, the
-//     slot lengths are prefix-summed, and a second pass ORs each slot into the
-//     stream at its bit offset ("generic" kernels).
+//   * 2-D in any mode, fixed accuracy / precision, 1-D odd rates: the tile
+//     kernels (tile_kernels.cu);
+//   * blocks padded far beyond their longest code: encoded into a scratch slot
+//     each, the slot lengths prefix-summed, and a second pass ORs each slot into
+//     the stream at its bit offset; one thread per block decodes them, and 1-D
+//     blocks of up to 11 bits ("generic" kernels).
 // Array walk and partial edge blocks follow sw/src/zfp.c:31-56,79-103 and
 // sw/src/encode.c:41-88; per-stage debug kernels mirror hw/stages/*.cpp.
 #include <cuda_runtime.h>
