@@ -477,6 +477,49 @@ int64_t gcow_window_decode_check(const uint32_t* words, uint64_t blocks, uint32_
   return bad;
 }
 
+// The tile kernels' 2-D coders against the plane-by-plane ones: the number of blocks of 16 values that are coded to other bits,
+// write past their slot or decode to other values; `words`, if given, is instead read as blocks of `stride` words (an
+// even number) of arbitrary bits, starting `skip` bits in, and only decoded.
+int64_t gcow_tile_2d_check(const float* values, const uint32_t* words, uint64_t blocks, uint32_t stride, uint32_t skip, const int32_t* params) {
+  static const gcow::TwinTable twin;
+  static const gcow::RunTable run;
+  const gcow::ZfpParams p = {(uint32_t)params[0], (uint32_t)params[1], (uint32_t)params[2], params[3]};
+  const bool cuts = gcow::tile_budget_cuts(p, 2);
+  const uint32_t slot_words = gcow::tile_slot_words(p, 2);
+  int64_t bad = 0;
+  for (uint64_t b = 0; b < blocks; b++) {
+    uint64_t code[32] = {};
+    std::vector<uint32_t> window(64);
+    bool ok = true;
+    if (values) {
+      const float* f = values + 16 * b;
+      gcow::WordSink sink(code);
+      const uint32_t len = gcow::encode_block<2>(f, p, sink);
+      sink.finish();
+      std::vector<uint32_t> slot(slot_words + 8, 0xdeadbeefu);
+      const uint32_t got = cuts ? gcow::encode_slot_2d<true>(f, p, twin.v, slot.data(), 1) : gcow::encode_slot_2d<false>(f, p, twin.v, slot.data(), 1);
+      for (uint32_t i = slot_words; i < slot.size(); i++) ok = ok && slot[i] == 0xdeadbeefu;
+      ok = ok && (got < p.minbits ? p.minbits : got) == len;
+      for (uint32_t i = 0; ok && i < got; i++) ok = ((code[i >> 6] >> (i & 63)) & 1u) == ((slot[i >> 5] >> (i & 31)) & 1u);
+      for (uint32_t i = 0; i < 64; i++) window[i] = 0x9e3779b9u * (uint32_t)(b + i);           // what lies around a block
+      for (uint32_t i = 0; i < len; i++) {
+        uint32_t& w = window[(skip + i) >> 5];
+        w = (w & ~(1u << ((skip + i) & 31))) | (uint32_t)((code[i >> 6] >> (i & 63)) & 1u) << ((skip + i) & 31);
+      }
+    } else {
+      memcpy(window.data(), words + b * stride, stride * 4);
+    }
+    float x[16], y[16];
+    if (cuts) gcow::decode_window_2d<true>(x, p, run.v, window.data(), skip, 1); else gcow::decode_window_2d<false>(x, p, run.v, window.data(), skip, 1);
+    std::vector<uint64_t> w(32);
+    memcpy(w.data(), window.data(), 256);
+    gcow::WordSrc src(w.data(), skip);
+    gcow::decode_block<2>(y, p, src, 1);
+    bad += !ok || memcmp(x, y, 64) != 0;
+  }
+  return bad;
+}
+
 // Fixed accuracy with a bit cap through the lean coders (as the sparse all-reduce kernel uses them) against the
 // definition path: out = D(E(x)) from the lean pair, and the return value counts the blocks whose result differs from
 // decode_block(encode_block(x)) at {minbits 1, maxbits bits, maxprec 64, minexp}. 0 means they agree everywhere.

@@ -32,6 +32,9 @@ template <int DIM> struct TileShape {
   static constexpr int kPer = DIM == 1 ? 4 : 1, kWarpBlocks = 32 * kPer, kBlocks = kTileThreads * kPer;
 };
 
+__device__ const TwinTable d_twin{};
+__device__ const RunTable d_run{};
+
 struct TileArgs {
   uint64_t nx, ny, blocks;
   uint32_t bx, tiles;             // blocks per row of blocks (2-D); tiles
@@ -167,7 +170,7 @@ __global__ void __launch_bounds__(kTileThreads)
 encode_tiles_kernel(const float* __restrict__ in, const TileArgs a, uint32_t* __restrict__ out, uint64_t* __restrict__ block_bits,
                     const TileStrings st, const uint16_t* __restrict__ enc_tab, const uint32_t* __restrict__ pair_tab) {
   constexpr int kPer = TileShape<DIM>::kPer, WB = TileShape<DIM>::kWarpBlocks, NB = TileShape<DIM>::kBlocks;
-  constexpr int kTabWords = DIM == 1 ? kEncPairTabSize : kRestTabSize;
+  constexpr int kTabWords = DIM == 1 ? kEncPairTabSize : kTwinTabSize;
   extern __shared__ __align__(16) uint32_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // table | per warp: slots [slot_words][WB], lengths [WB], packed string [warp_words]
@@ -181,7 +184,7 @@ encode_tiles_kernel(const float* __restrict__ in, const TileArgs a, uint32_t* __
     for (int i = tid; i < kEncPairTabSize / 4; i += kTileThreads)
       reinterpret_cast<uint4*>(tab)[i] = reinterpret_cast<const uint4*>(pair_tab)[i];
   } else {
-    tab[tid] = make_rest_entry((uint32_t)tid);
+    if (tid < kTwinTabSize / 4) reinterpret_cast<uint4*>(tab)[tid] = reinterpret_cast<const uint4*>(d_twin.v)[tid];
   }
   __syncthreads();
   int turn = 0;
@@ -429,7 +432,7 @@ __global__ void __launch_bounds__(kTileThreads)
 decode_tiles_kernel(const uint32_t* __restrict__ in, float* __restrict__ out, const TileArgs a,
                     const uint64_t* __restrict__ block_bits, int shift, const uint16_t* __restrict__ plane_tab, const uint32_t* __restrict__ loop_tab) {
   constexpr int kPer = TileShape<DIM>::kPer, WB = TileShape<DIM>::kWarpBlocks, NB = TileShape<DIM>::kBlocks;
-  constexpr int kTabWords = DIM == 1 ? kTileDecTab1 : kUnrestTabSize;
+  constexpr int kTabWords = DIM == 1 ? kTileDecTab1 : kRunTabSize;
   extern __shared__ __align__(16) uint32_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t* const words = smem + kTabWords + warp * a.warp_words;
@@ -439,7 +442,7 @@ decode_tiles_kernel(const uint32_t* __restrict__ in, float* __restrict__ out, co
     for (int i = tid; i < kDecTiny / 4; i += kTileThreads)   // windows and nibble pairs
       reinterpret_cast<uint4*>(smem)[i] = reinterpret_cast<const uint4*>(loop_tab)[i];
   } else {
-    smem[tid] = make_unrest_entry((uint32_t)tid);
+    for (int i = tid; i < kRunTabSize / 4; i += kTileThreads) reinterpret_cast<uint4*>(smem)[i] = reinterpret_cast<const uint4*>(d_run.v)[i];
   }
   __syncthreads();
   for (uint32_t tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
@@ -503,18 +506,6 @@ TileArgs tile_args(const void* values, uint64_t nx, uint64_t ny, const ZfpParams
   return a;
 }
 
-// Words of one slot: the longest unpadded code, or what may have been emitted when the budget is found to be exceeded
-// (1-D: eight planes of at most seven bits at once, 2-D: one code of at most 32 bits), and one more written by the end.
-uint32_t slot_words_for(const ZfpParams& p, int dim) {
-  const uint32_t n = dim == 1 ? 4 : 16, prec = p.maxprec < 32 ? p.maxprec : 32;
-  const uint32_t natural = kHeaderBits + (n - 1) + n * prec;
-  const uint32_t past = p.maxbits + (dim == 1 ? 55 : 31);
-  return (natural <= p.maxbits || natural < past ? natural : past) / 32 + 1;
-}
-bool budget_cuts(const ZfpParams& p, int dim) {
-  const uint32_t n = dim == 1 ? 4 : 16, prec = p.maxprec < 32 ? p.maxprec : 32;
-  return kHeaderBits + (n - 1) + n * prec > p.maxbits;
-}
 // Words of a warp's packed string or window.
 uint32_t warp_words_for(const ZfpParams& p, int dim) {
   const uint32_t wb = dim == 1 ? TileShape<1>::kWarpBlocks : TileShape<2>::kWarpBlocks;
@@ -629,10 +620,10 @@ int gcow_encode_tiles(const float* in, uint64_t nx, uint64_t ny, const int32_t* 
   const void *et, *dt, *pt, *lt;
   if (int rc = gcow_codec_tables4(&et, &dt, &pt, &lt)) return rc;
   TileArgs a = tile_args(in, nx, ny, p, blocks, dim);
-  a.slot_words = slot_words_for(p, dim);
+  a.slot_words = tile_slot_words(p, dim);
   a.warp_words = round4(warp_words_for(p, dim) + kPackedPad);
   const uint32_t wb = dim == 1 ? TileShape<1>::kWarpBlocks : TileShape<2>::kWarpBlocks;
-  const uint32_t smem = ((dim == 1 ? kEncPairTabSize : kRestTabSize) + kTileWarps * (a.slot_words * wb + wb + a.warp_words)) * 4;
+  const uint32_t smem = ((dim == 1 ? kEncPairTabSize : kTwinTabSize) + kTileWarps * (a.slot_words * wb + wb + a.warp_words)) * 4;
   const TileScratch ts = tile_scratch(p, blocks, dim);
   char* const sp = (char*)(((uintptr_t)scratch + 15) & ~(uintptr_t)15);
   a.pitch = wb / 32 * max_block_bits(p, dim);
@@ -646,7 +637,7 @@ int gcow_encode_tiles(const float* in, uint64_t nx, uint64_t ny, const int32_t* 
     encode_tiles_kernel<D, F, B><<<g, kTileThreads, smem, s>>>(in, a, (uint32_t*)out, block_bits, st,         \
                                                                (const uint16_t*)et, (const uint32_t*)pt);      \
   } while (0)
-  const bool cuts = budget_cuts(p, dim);
+  const bool cuts = tile_budget_cuts(p, dim);
   if (dim == 1) { if (fixed) GCOW_ENCODE(1, true, true); else GCOW_ENCODE(1, false, true); }
   else if (fixed) { if (cuts) GCOW_ENCODE(2, true, true); else GCOW_ENCODE(2, true, false); }
   else { if (cuts) GCOW_ENCODE(2, false, true); else GCOW_ENCODE(2, false, false); }
@@ -675,7 +666,7 @@ int gcow_decode_tiles(const void* in, float* out, uint64_t nx, uint64_t ny, cons
   TileArgs a = tile_args(out, nx, ny, p, blocks, dim);
   a.slot_words = warp_words_for(p, dim) + 1;                 // window capacity: one more for the bits before the first block
   a.warp_words = round4(a.slot_words + kReadAhead);
-  const uint32_t smem = ((dim == 1 ? (uint32_t)kTileDecTab1 : (uint32_t)kUnrestTabSize) + kTileWarps * a.warp_words) * 4;
+  const uint32_t smem = ((dim == 1 ? (uint32_t)kTileDecTab1 : (uint32_t)kRunTabSize) + kTileWarps * a.warp_words) * 4;
   int err = 0;
 #define GCOW_DECODE(D, B)                                                                                      \
   do {                                                                                                         \
@@ -684,7 +675,7 @@ int gcow_decode_tiles(const void* in, float* out, uint64_t nx, uint64_t ny, cons
     decode_tiles_kernel<D, B><<<g, kTileThreads, smem, s>>>((const uint32_t*)in, out, a, block_bits, shift, (const uint16_t*)dt, (const uint32_t*)lt); \
   } while (0)
   if (dim == 1) GCOW_DECODE(1, true);
-  else if (budget_cuts(p, 2)) GCOW_DECODE(2, true);
+  else if (tile_budget_cuts(p, 2)) GCOW_DECODE(2, true);
   else GCOW_DECODE(2, false);
 #undef GCOW_DECODE
   return (int)cudaGetLastError();

@@ -452,6 +452,30 @@ def test_window_decoder_of_the_tiles(maxprec, maxbits):
         assert lib.gcow_window_decode_check(words.ctypes.data, words.shape[0], words.shape[1], skip, par.as_c()) == 0
 
 
+@pytest.mark.parametrize("par", [ZfpParams(1, 16658, 64, e) for e in (-1074, -30, -12, 0)] + [ZfpParams(1, 16658, q, -1074) for q in (1, 2, 15, 16, 17, 31, 32)]
+                         + [ZfpParams(b, b, 64, -1074) for b in (9, 10, 11, 12, 40, 41, 42, 43, 64, 128, 200, 256, 535, 544)], ids=str)
+def test_2d_coders_of_the_tiles(par):
+    """The 2-D coders of the tile kernels and the plane-by-plane ones: runs of planes that hold the first coefficient alone
+    (every length, none, cut by the budget), rests of up to 16 bits, arbitrary bits."""
+    rng = np.random.default_rng(par.maxbits + par.maxprec)
+    n = 4000
+    noise = rng.standard_normal((n, 16)).astype(np.float32)
+    scale = np.exp2(rng.integers(-28, 3, (n, 1))).astype(np.float32)
+    ramp = np.add.outer(np.arange(4), 2 * np.arange(4)).reshape(-1).astype(np.float32)
+    for x in (noise, 1 + noise * scale, np.repeat(noise[:, :1], 16, 1), noise[:, :1] + ramp * scale, np.where(noise > 1, noise, 0),
+              noise * np.exp2(rng.integers(-140, 120, (n, 16)))):
+        x = np.ascontiguousarray(x, dtype=np.float32)
+        for skip in (0, 31):
+            assert lib.gcow_tile_2d_check(x.ctypes.data, None, n, 0, skip, par.as_c()) == 0
+    w = rng.integers(0, 1 << 32, size=(n, 40), dtype=np.uint64).astype(np.uint32)
+    w[::3] &= rng.integers(0, 1 << 32, size=w[::3].shape, dtype=np.uint64).astype(np.uint32)
+    w[::4, :3] |= np.uint32(0x55555555)
+    w[1::4, :3] &= np.uint32(0x55555555)
+    for skip in (0, 5, 31):
+        w[1:, 0] |= np.uint32(1 << skip)                        # blocks that are not empty
+        assert lib.gcow_tile_2d_check(None, w.ctypes.data, n, w.shape[1], skip, par.as_c()) == 0
+
+
 def test_generic_scratch_holds_either_layout():
     """The entry point that takes the caller's scratch goes through the slots or through the tile kernels."""
     try:
