@@ -555,6 +555,34 @@ int64_t gcow_lean_accuracy_check(const float* data, uint64_t n, int bits, int mi
   return bad;
 }
 
+// The round trip that makes no code against encode_block / decode_block at `bits` bits per block: the number of blocks
+// whose values differ; *left receives how many of them it leaves to the coders. -1: bits not covered.
+int64_t gcow_roundtrip_check(const float* values, uint64_t blocks, int bits, uint64_t* left) {
+  const ZfpParams p = {(uint32_t)bits, (uint32_t)bits, 64, -1074};
+  int64_t bad = 0;
+  *left = 0;
+  for (uint64_t b = 0; b < blocks; b++) {
+    const float* f = values + 4 * b;
+    uint64_t code[4] = {};
+    gcow::WordSink sink(code);
+    gcow::encode_block<1>(f, p, sink);
+    sink.finish();
+    gcow::WordSrc src(code, 0);
+    float want[4], got[4];
+    gcow::decode_block<1>(want, p, src, 0);
+    memcpy(got, f, 16);
+    bool ok;
+    switch (bits) {
+      case 32: ok = gcow::roundtrip_block_1d_try<32>(got); break;
+      case 64: ok = gcow::roundtrip_block_1d_try<64>(got); break;
+      case 128: ok = gcow::roundtrip_block_1d_try<128>(got); break;
+      default: return -1;
+    }
+    if (ok) bad += memcmp(want, got, 16) != 0; else ++*left;
+  }
+  return bad;
+}
+
 int gcow_fast1d_compress(const float* data, uint64_t n, const int32_t* params, void* out) {
   ZfpParams p = load_params(params);
   uint16_t etab[gcow::kEncTabSize];

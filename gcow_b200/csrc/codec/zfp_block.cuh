@@ -1156,6 +1156,58 @@ GCOW_HD void decode_block_1d_lean(float* f, const LeanTables& t, const uint32_t 
   if (!decode_block_1d_try<BITS>(f, t, w, shift, kmin)) decode_block_1d_rest<BITS>(f, t, w, shift, kmin);
 }
 
+// The round trip D(E(f)) of a block of BITS bits without making the code: f becomes what decoding its code gives. What the
+// bit budget leaves of the coefficients has a closed form once n >= 3, where every plane takes four bits. Let top_i be the
+// highest bit of coefficients i..3 together: coefficient i is sent in every plane from top_i down, a coefficient i < 3
+// whose own highest bit is top_i costs one positive group test more, and every plane ends with a negative test until
+// coefficient 3 has been reached, from where on its own bit takes that place. So the planes 31..k cost
+//   C - 4 k,  C = (top_0 + 1) + (top_1 + 1) + (top_2 + 1) + #{i < 3: highest bit of coefficient i == top_i} + 32,
+// for every k <= top_2, and the bits that are left over (fewer than four) are the lowest coefficients' bits of plane k - 1.
+// No table, no branch.
+// False (f is not written) where the cut falls at or above top_2, or the exponent or a member is out of the ordinary.
+template <int BITS>
+GCOW_HD bool roundtrip_block_1d_try(float* f) {
+  constexpr int P = BITS - (int)kHeaderBits;
+  const uint32_t mb = f32_bits(fmaxf(fmaxf(fabsf(f[0]), fabsf(f[1])), fmaxf(fabsf(f[2]), fabsf(f[3]))));
+  const uint32_t ex = mb >> 23;                               // emax = ex - 126
+  const float scale = bits_f32(0x8d800000u - (mb & 0xff800000u));   // 2^(30 - emax)
+  const float p0 = scale * f[0], p1 = scale * f[1], p2 = scale * f[2], p3 = scale * f[3];
+  const bool ordinary = ex - 30u <= 224u && fabsf((p0 + p1) + (p2 + p3)) < 8.0e9f;     // the sum: a NaN member
+  int32_t q[4];
+#if defined(__CUDA_ARCH__)
+  q[0] = __float2int_rz(p0); q[1] = __float2int_rz(p1); q[2] = __float2int_rz(p2); q[3] = __float2int_rz(p3);
+#else
+  if (!ordinary) return false;                                // out of range for this conversion
+  q[0] = (int32_t)p0; q[1] = (int32_t)p1; q[2] = (int32_t)p2; q[3] = (int32_t)p3;
+#endif
+  fwd_lift(q[0], q[1], q[2], q[3]);
+  uint32_t u[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) u[i] = int2nb(q[i]);
+  const uint32_t m2 = u[2] | u[3], m1 = m2 | u[1], m0 = m1 | u[0];
+  const bool low = m2 != 0;                                   // top_2 exists
+#if defined(__CUDA_ARCH__)
+  const int l0 = __clz((int)m0), l1 = __clz((int)m1), l2 = __clz((int)m2);             // top_i = 31 - l_i
+#else
+  if (!low) return false;
+  const int l0 = (int)clz32(m0), l1 = (int)clz32(m1), l2 = (int)clz32(m2);
+#endif
+  // a coefficient holds the highest bit of a union when the rest of the union is smaller
+  const int own = (u[0] > (m0 ^ u[0])) + (u[1] > (m1 ^ u[1])) + (u[2] > (m2 ^ u[2]));
+  const int over = 128 + own - (l0 + l1 + l2) - P;            // C - P: bits too many with all planes sent
+  const int k = over > 0 ? (over + 3) >> 2 : 0, a = 4 * k - over;      // planes 31..k are whole; a: see above (any a > 3 with k == 0)
+  const bool ok = ordinary && low && k <= 31 - l2;
+  const uint32_t whole = shl_sat(0xffffffffu, (uint32_t)k), more = k > 0 ? whole | shl_sat(1u, (uint32_t)(k - 1)) : whole;
+#pragma unroll
+  for (int i = 0; i < 4; i++) q[i] = nb2int(u[i] & (i < 3 && i < a ? more : whole));
+  inv_lift(q[0], q[1], q[2], q[3]);
+  if (!ok) return false;
+  const float back = bits_f32((ex - 29u) << 23);              // 2^(emax - 30)
+#pragma unroll
+  for (int i = 0; i < 4; i++) f[i] = back * (float)q[i];
+  return true;
+}
+
 // Fixed accuracy with a bit cap (minexp from the tolerance, maxbits = BITS, minbits = 1): a block keeps the planes
 // 31 .. 32 - prec, prec = block_precision(emax, ., minexp, 1), as far as the cap allows. The embedded code of those
 // planes is a prefix of the fixed-rate code, so the fixed-rate encoder serves unchanged and the decoder only has to

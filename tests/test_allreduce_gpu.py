@@ -70,6 +70,27 @@ def test_single_rank_round_trip_views_and_feedback(rate):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("rate", [4, 8, 16, 32])
+@pytest.mark.parametrize("blocks", [148 * 8 * 256, 148 * 8 * 256 + 1, 5 * 148 * 8 * 256 - 3])
+def test_single_rank_round_trip_of_a_long_bucket(rate, blocks):
+    """More blocks than threads: two per thread and step, what is left of them, a partial one; noise, and stretches that the
+    kernel has to leave to the coders (smooth, zero, infinite, NaN)."""
+    n = 4 * blocks - 1
+    x = gen(blocks, n)
+    x[:n // 4] = np.cumsum(x[:n // 4])
+    x[n // 4:n // 3:5] = 0
+    x[n // 3:n // 2] = 0
+    x[n // 2::4099] = np.inf
+    x[n // 2 + 1::4097] = np.nan
+    x[-n // 8:] += 1
+    want = allreduce_oracle(x[None], ZfpParams.from_rate(rate, 1), "oneshot", 0)
+    ar = CompressedAllReduce(n, GcowConfig(rate=rate))
+    y = ar(torch.from_numpy(x).cuda()).cpu().numpy()
+    ar.check()
+    assert np.array_equal(y.view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("cap,tol", [(4, 1e-2), (8, 1e-3), (16, 1e-6), (32, 1e-4)])
 def test_accuracy_mode_single_rank_equals_oracle(cap, tol):
     """Fixed accuracy with a bit cap (the sparse variant): bit-exact against the host model at the same four codec

@@ -476,6 +476,26 @@ def test_2d_coders_of_the_tiles(par):
         assert lib.gcow_tile_2d_check(None, w.ctypes.data, n, w.shape[1], skip, par.as_c()) == 0
 
 
+@pytest.mark.parametrize("bits", [32, 64, 128])
+def test_roundtrip_without_a_code(bits):
+    """D(E(x)) in closed form against the coders, on data that is cut everywhere (inside a nibble, at the plane that brings the
+    third coefficient in, not at all) and on what it has to leave to them."""
+    rng = np.random.default_rng(bits)
+    n = 100000
+    noise = rng.standard_normal((n, 4))
+    odd = noise.copy()
+    odd[::3, 1] = np.inf
+    odd[1::3, 2] = np.nan
+    odd[2::3] *= 1e-40
+    left = C.c_uint64()
+    for name, x in dict(noise=noise * 1e-3, smooth=1 + noise * np.exp2(rng.integers(-28, 3, (n, 1))), uneven=noise * np.exp2(-rng.integers(0, 26, (n, 4))),
+                        magnitudes=noise * np.exp2(rng.integers(-140, 120, (n, 1))), sparse=np.where(noise > 1, noise, 0), zeros=noise * 0,
+                        same=np.repeat(noise[:, :1], 4, 1), odd=odd).items():
+        x = np.ascontiguousarray(x, dtype=np.float32)
+        assert lib.gcow_roundtrip_check(x.ctypes.data, n, bits, C.byref(left)) == 0, name
+        assert name != "noise" or left.value < n // 500
+
+
 def test_generic_scratch_holds_either_layout():
     """The entry point that takes the caller's scratch goes through the slots or through the tile kernels."""
     try:
