@@ -1,39 +1,34 @@
-// Fused multi-head self-attention on the 5th-generation tensor cores (sm_100a), head dimension 64,
-// sequence length a multiple of 128 up to 512, no mask, no dropout: forward and backward.
+// Fused multi-head self-attention on the 5th-generation tensor cores (sm_100a), head dimension 64, 72 to 512 positions (a
+// multiple of 8), no mask, no dropout: forward and backward.
 //
-// All three kernels read the packed projection qkv [B][S][3][H][64] (bf16) in place through 4-D
-// tensor maps {d, h, s, b} - a box is 128 sequence positions of one head, 128-byte rows with the
-// 128-byte swizzle - and write the context / gradients in the layouts the neighbouring GEMMs use
-// ([B][S][H][64] and [B][S][3][H][64]), so no transposed copy of Q, K or V exists.
+// All three kernels read the packed projection qkv [B][S][3][H][64] (bf16) in place through 4-D tensor maps {d, h, s, b} - a
+// box is 128 sequence positions of one head, 128-byte rows with the 128-byte swizzle - and write the context / gradients in
+// the layouts the neighbouring GEMMs use ([B][S][H][64] and [B][S][3][H][64]), so no transposed copy of Q, K or V exists.
 //
-//  forward   one CTA per (128 queries, head): S = Q K^T for ALL keys lands in tensor memory (up to
-//            512 fp32 columns, one row per thread), the row maximum and the exponentials are taken
-//            straight from there, P goes to shared memory as bf16 in the MMA's K-major layout and
-//            O = P V accumulates in the tensor-memory columns that S has vacated. exp(S - max)
-//            needs no running rescale because the whole row is present. Also stores the row's
+//  forward   a tile is 128 queries of a head; S = Q K^T comes in blocks of 128 keys. One thread per query takes the block's
+//            128 scores into registers (which frees their tensor-memory columns for the next block's product), their maximum
+//            and their exponentials, and puts P as bf16 into tensor memory, from where it is the A operand of O += P V. The
+//            running maximum is followed with a margin (kRescale), so O is hardly ever read back. Also stores the row's
 //            log2-sum-exp for the backward pass.
-//  backward  recomputes P from Q, K and the stored log-sum-exp, a 128 x 64 tile at a time (128 x 128 where the grid leaves
-//            each CTA an SM to itself).
-//     dK/dV  one CTA per (128 keys, head), loop over blocks of 64 queries: S^T = K Q^T and dP^T = V dO^T in
-//            tensor memory (one key per row, so lse and delta are per column, read from shared memory), P^T and
-//            dS^T = P^T (dP^T - delta) to shared memory as K-major operands, dV and dK accumulate in tensor memory.
-//     dQ     one CTA per (128 queries, head), loop over blocks of 64 keys: S, dP, dS, then dQ += dS K.
-//            Recomputing S and dP here instead of adding dQ with atomics keeps the gradients deterministic.
-//            The steps of one tile (products, exponentials, operands, products) follow one another, so what hides them
-//            is a second CTA on the SM: tiles of 64 keep a CTA within 256 tensor-memory columns and 113 KB of shared
-//            memory, where 128 x 128 tiles took 320 to 384 columns and 128 to 160 KB, one CTA per SM.
-//            512 x 32 sequences of 16 heads, both kernels and delta: 398 -> 337 us (dK/dV 206 -> 192, dQ 169 -> 133).
+//  backward  recomputes P from Q, K and the stored log-sum-exp, in blocks of 128 x 64, one row per thread as above.
+//     dK/dV  a tile is 128 keys, the loop runs over the queries: S^T = K Q^T and dP^T = V dO^T, so lse and delta belong to the
+//            columns; P^T and dS^T = P^T (dP^T - delta) are A operands in tensor memory of dV += P^T dO and dK += dS^T Q.
+//     dQ     a tile is 128 queries, the loop runs over the keys: S, dP, dS, then dQ += dS K. Recomputing S and dP here
+//            instead of adding dQ with atomics keeps the gradients deterministic.
 //  delta = rowsum(dO * O) comes from a small elementwise kernel.
 //
-// 512 threads per CTA: four threads share an accumulator row (the four warps that may read a
-// tensor-memory lane quarter each take a quarter of the columns), which is what hides the latency
-// of the exponentials; thread 0 issues the TMA loads and the MMAs. Every mbarrier wait is bounded: after a fixed number of polls the CTA records an error
-// code, leaves its loops, waits (bounded) for outstanding MMAs, frees its tensor memory and
-// returns. No load uses cluster multicast. The reference's models are CNNs
-// (hw/models/train_imagenet.py:199-202); this kernel serves the BERT configuration.
+// One persistent CTA per SM with two tiles in flight, A and B, 128 threads each: while one waits for its product the other
+// one's exponentials run. A warp per tile issues its products, another one the TMA loads; whole
+// sequences of the streamed operands (64 KB each) are held, and refilled for the next unit of work block by block as the
+// last product that reads a block completes.
+//
+// Every mbarrier wait is bounded: after a fixed number of polls the CTA records an error code, all roles leave their loops,
+// wait (bounded) for outstanding copies and MMAs, free the tensor memory and return. No load uses cluster multicast. The
+// reference's models are CNNs (hw/models/train_imagenet.py:199-202); these kernels serve the BERT configuration.
 #include <stdio.h>
 #include <mutex>
 
+#include "pdl.cuh"
 #include "tc_common.cuh"
 
 namespace gcow {
@@ -45,30 +40,14 @@ constexpr int D = 64;                 // head dimension: one 128-byte row
 constexpr int TILE = 128;             // rows of a query / key tile
 constexpr int TILE_BYTES = TILE * D * 2;   // 16 KB
 constexpr int MAX_S = 512;
-constexpr int NT = 512;               // threads per CTA: 4 column groups x 128 rows
-// Backward, by the queries / keys per loop step (64 or 128): bytes of a block of them, tensor-memory columns (S and dP of a
-// step, two accumulators), CTAs per SM.
-template <int STEP> struct Step {
-  static constexpr int BYTES = STEP * D * 2, COLS = STEP == 64 ? 256 : 512, CTAS = STEP == 64 ? 2 : 1;
-  static constexpr int PANELS = STEP / 64;   // of P and dS: [128 rows][64 columns], 16 KB each
-};
 
 struct Params {
-  __nv_bfloat16* out;      // forward: context [B][S][H][64]
   float* lse;              // [B][H][S] log2-sum-exp of the scaled scores
   const float* delta;      // backward: [B][H][S] rowsum(dO * O)
-  __nv_bfloat16* dqkv;     // backward: [B][S][3][H][64]
   int B, S, H;
   float scale_log2;        // softmax scale * log2(e)
   float scale;             // softmax scale
   uint32_t* error;
-};
-
-struct Bars {
-  uint64_t a, b, c, d, e[2], f[2], drain;
-  uint32_t tmem_base;
-  volatile uint32_t abort;
-  float red[4][TILE];      // per-row partial maxima / sums of the four column groups
 };
 
 __device__ __forceinline__ uint32_t idesc_f16(int n, bool a_mn, bool b_mn) {
@@ -77,217 +56,370 @@ __device__ __forceinline__ uint32_t idesc_f16(int n, bool a_mn, bool b_mn) {
          ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ bool wait(Bars* bs, uint64_t* bar, uint32_t parity, uint32_t* error, uint32_t code) {
-  return mbar_wait_abortable(&bs->abort, bar, parity, error, code);
-}
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&v);
 }
-// Byte offset of the 16-byte chunk holding elements 8j..8j+7 of row r in a [rows][64] bf16 tile with
-// 128-byte rows and the 128-byte swizzle (the layout TMA writes and the K-major descriptor reads).
-__device__ __forceinline__ uint32_t sw128(int r, int j) { return (uint32_t)(r * 128 + ((j ^ (r & 7)) << 4)); }
-
-// Store 32 consecutive fp32 values of this thread's row as bf16 into a K-major operand: the row has `64`
-// elements per 16 KB block, the 32 values are elements e0..e0+31 of the row (e0 a multiple of 32).
-__device__ __forceinline__ void store_kmajor32(uint8_t* tile, int row, int e0, const float (&v)[32]) {
-  uint8_t* blk = tile + (e0 >> 6) * TILE_BYTES;
-  const int j0 = (e0 & 63) >> 3;
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r; asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r;
+}
+// 32 fp32 values of a row as bf16 at elements e0.. of a 64-element row in the 128-byte swizzle that the TMA reads.
+__device__ __forceinline__ void store_row32(uint8_t* tile, int row, int e0, const float (&v)[32]) {
 #pragma unroll
   for (int j = 0; j < 4; j++) {
-    uint4 o = make_uint4(pack2(v[8 * j], v[8 * j + 1]), pack2(v[8 * j + 2], v[8 * j + 3]),
-                         pack2(v[8 * j + 4], v[8 * j + 5]), pack2(v[8 * j + 6], v[8 * j + 7]));
-    *reinterpret_cast<uint4*>(blk + sw128(row, j0 + j)) = o;
+    const uint4 o = make_uint4(pack2(v[8 * j], v[8 * j + 1]), pack2(v[8 * j + 2], v[8 * j + 3]),
+                               pack2(v[8 * j + 4], v[8 * j + 5]), pack2(v[8 * j + 6], v[8 * j + 7]));
+    *reinterpret_cast<uint4*>(tile + row * 128 + ((((e0 >> 3) + j) ^ (row & 7)) << 4)) = o;
   }
 }
-// 16 values, elements e0..e0+15 of the row, of an operand with 64 elements per row.
-__device__ __forceinline__ void store_kmajor16(uint8_t* tile, int row, int e0, const float (&v)[16]) {
-#pragma unroll
-  for (int j = 0; j < 2; j++) {
-    uint4 o = make_uint4(pack2(v[8 * j], v[8 * j + 1]), pack2(v[8 * j + 2], v[8 * j + 3]),
-                         pack2(v[8 * j + 4], v[8 * j + 5]), pack2(v[8 * j + 6], v[8 * j + 7]));
-    *reinterpret_cast<uint4*>(tile + sw128(row, (e0 >> 3) + j)) = o;
-  }
+__device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+        "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+        "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D += A B with A [128 x 16] in tensor memory: row r in lane r, two bf16 per column
+__device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
+}
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int x, int y, int z, int w) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+               ::"l"((uint64_t)map), "r"(src), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 
-template <uint32_t COLS>
-__device__ __forceinline__ void tmem_alloc(Bars* bs, int warp) {
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bs->tmem_base)), "r"(COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+// Work of a CTA: units of one or two tiles of 128 rows, A and B. kSingle: one tile each; kPair: two of one head (the last one
+// of an odd number stands alone); kHeads (up to 128 positions): one tile of each of two heads.
+enum UnitMode { kSingle, kPair, kHeads };
+struct Unit { int bh[2], q[2]; bool both; };
+__device__ __forceinline__ Unit unit_at(int u, int mode, int tiles, int heads) {
+  Unit r;
+  if (mode == kHeads) {
+    r.bh[0] = 2 * u; r.bh[1] = 2 * u + 1; r.q[0] = r.q[1] = 0; r.both = 2 * u + 1 < heads;
+  } else {
+    const int per = mode == kSingle ? tiles : (tiles + 1) / 2;
+    r.bh[0] = r.bh[1] = u / per;
+    r.q[0] = (u % per) * (mode == kSingle ? 1 : 2); r.q[1] = r.q[0] + 1;
+    r.both = mode == kPair && r.q[1] < tiles;
   }
-}
-template <uint32_t COLS>
-__device__ __forceinline__ void tmem_free(uint32_t base, int warp) {
-  if (warp == 0) {
-    __syncwarp();
-    tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(COLS) : "memory");
-  }
-}
-// All MMAs issued by this thread have completed (bounded), so tensor memory and the operands may go.
-__device__ __forceinline__ void drain(Bars* bs) {
-  tc_commit(&bs->drain);
-  for (uint32_t it = 0; it < kSpinLimit; it++) if (mbar_try_wait(&bs->drain, 0)) break;
+  return r;
 }
 
-// A [128 x 64k] K-major (rows x reduction) times B: 4 k-steps per 64 reduction elements.
-__device__ __forceinline__ void mma_kk(uint32_t d_tmem, uint32_t a_smem, uint32_t b_smem, int n, bool acc) {
-  const uint32_t id = idesc_f16(n, false, false);
-  const uint64_t da = smem_desc_sw128(a_smem), db = smem_desc_sw128(b_smem);
-#pragma unroll
-  for (int k = 0; k < 4; k++) tc_mma(d_tmem, da + 2 * k, db + 2 * k, id, acc || k);
+// The barriers of a CTA are numbered, and a role keeps the parities it waits for next in one word.
+//
+// What the issuing warps do per product decides the pace. As code of one thread alone, with the descriptors worked out where
+// they are used, a step of four to eight MMAs took it 1500 cycles (forward, B 32, S 512, 16 heads: 131 us): every operand of
+// an MMA is a uniform register, which a divergent thread has to fill one by one. So the whole warp runs the loop, all its
+// values are uniform, and one lane executes the MMAs, commits and copies alone (95 us). A wait that has nothing to wait for
+// still takes 200 cycles and an MMA 70 to 80, so each tile has a warp of its own.
+struct Phases {
+  uint32_t bits = 0;
+  __device__ __forceinline__ uint32_t next(int i) {
+    const uint32_t p = (bits >> i) & 1u;
+    bits ^= 1u << i;
+    return p;
+  }
+};
+// Waits (bounded) until the last copy that was issued on a barrier has landed: `next` has the parity of the one after it.
+__device__ __forceinline__ void landed(uint64_t* bar, uint32_t next) {
+  for (uint32_t it = 0; it < kSpinLimit; it++) if (mbar_try_wait(bar, next ^ 1u)) break;
 }
+__device__ __forceinline__ void drain(uint64_t* bar) {      // everything this thread has issued to the tensor core is done
+  tc_commit(bar);
+  for (uint32_t it = 0; it < kSpinLimit; it++) if (mbar_try_wait(bar, 0)) break;
+}
+__device__ __forceinline__ void tmem_alloc_all(uint32_t* slot) {
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(512u) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_free_all(uint32_t base) {
+  __syncwarp();
+  tc_fence_after();
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(512u) : "memory");
+}
+
+// Two groups of 128 threads that work on a row each, and one whose warps issue the products and the loads. A row's
+// thread holds 128 scores and their 64 packed probabilities (backward: 64 scores, probabilities and gradients each), more than
+// a third of an SM's registers allows (168 a thread): it takes what the third group gives up.
+constexpr int kThreads = 384, kLaunchRegs = 168;
+template <bool FWD> struct Regs { static constexpr int ROW = FWD ? 208 : 184, ISSUE = FWD ? 88 : 136; };
+static_assert(2 * Regs<true>::ROW + Regs<true>::ISSUE == 3 * kLaunchRegs && 2 * Regs<false>::ROW + Regs<false>::ISSUE == 3 * kLaunchRegs &&
+              kThreads * kLaunchRegs <= 65536, "setmaxnreg.inc waits for registers that must exist");
+template <bool FWD> __device__ __forceinline__ void regs_row() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Regs<FWD>::ROW)); }
+template <bool FWD> __device__ __forceinline__ void regs_issue() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Regs<FWD>::ISSUE)); }
 
 // ------------------------------------------------------------------------------ forward
-__global__ void __launch_bounds__(NT, 1)
-attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
-                const __grid_constant__ CUtensorMap tv, const Params p) {
+constexpr float kRescale = 8.0f;            // log2 units by which a running maximum may be out of date
+
+// Barriers, each for tile A and B or for the four blocks of keys. K and V blocks: full[2][4], free[2][4].
+enum FwdBar { kQFull = 0, kQFree = 2, kKvFull = 4, kKvFree = 12, kSFull = 20, kSFree = 22, kPFull = 24, kPv = 26, kFwdDrain = 28, kFwdBars = 30 };
+struct FwdBars {
+  uint64_t bar[kFwdBars];
+  uint32_t tmem_base;
+  volatile uint32_t abort;
+};
+
+__global__ void __launch_bounds__(kThreads, 1)
+attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
+                const __grid_constant__ CUtensorMap to, const Params p, int units, int mode) {
   extern __shared__ uint8_t raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* sQ = base;                       // 16 KB
-  uint8_t* sK = sQ + TILE_BYTES;            // S/128 tiles; P of the first 256 keys overwrites it
-  uint8_t* sV = sK + 4 * TILE_BYTES;
-  uint8_t* sP1 = sV + 4 * TILE_BYTES;       // P of keys 256..511
-  Bars* bs = reinterpret_cast<Bars*>(sP1 + 4 * TILE_BYTES);
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int row = (warp & 3) * 32 + (tid & 31), cg = warp >> 2;      // accumulator row, column group 0..3
-  const int q0 = blockIdx.x * TILE, h = blockIdx.y, b = blockIdx.z;
-  const int nk = p.S, ntile = nk / TILE;
-  const int half0 = nk < 256 ? nk : 256, half1 = nk - half0;
+  uint8_t* const sQ = base;                  // A, B
+  uint8_t* const sO = sQ + 2 * TILE_BYTES;   // 4 KB per softmax warp
+  uint8_t* const sK = sO + 2 * TILE_BYTES;   // blocks of 128 keys
+  uint8_t* const sV = sK + 4 * TILE_BYTES;
+  FwdBars* const bs = reinterpret_cast<FwdBars*>(sV + 4 * TILE_BYTES);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // warp: uniform
+  const int tiles = (p.S + TILE - 1) / TILE, heads = p.B * p.H;
+  const int blocks = tiles;                  // blocks of 128 keys; the last one may be partial: its copy fills up with zeros
+  const int u0 = (int)((long long)units * blockIdx.x / gridDim.x), u1 = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
 
   if (tid == 0) {
-    mbar_init(&bs->a, 1); mbar_init(&bs->b, 1); mbar_init(&bs->c, 1); mbar_init(&bs->d, 1); mbar_init(&bs->drain, 1);
+    // 4: the warps of a tile; keys and values that two tiles share are free when both have used them
+    for (int i = 0; i < kFwdBars; i++) mbar_init(&bs->bar[i], i >= kSFree && i < kPv ? 4 : i >= kKvFree && i < kSFull && mode == kPair ? 2 : 1);
     bs->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  tmem_alloc<512>(bs, warp);
+  if (warp == 0) tmem_alloc_all(&bs->tmem_base);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bs->tmem_base;
-  const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-  bool ok = true;
+  pdl_trigger();
+  pdl_wait();
+  // columns: S of A, B (128 each), P of A, B (64 each), O of A, B (64 each)
+  auto col_s = [&](int x) { return tmem + x * 128; };
+  auto col_p = [&](int x) { return tmem + 256 + x * 64; };
+  auto col_o = [&](int x) { return tmem + 384 + x * 64; };
 
-  if (tid == 0) {
-    mbar_expect_tx(&bs->a, TILE_BYTES + nk * 128);
-    tma_load_4d(smem_u32(sQ), &tq, smem_u32(&bs->a), 0, h, q0, b);
-    for (int t = 0; t < ntile; t++) tma_load_4d(smem_u32(sK + t * TILE_BYTES), &tk, smem_u32(&bs->a), 0, h, t * TILE, b);
-    mbar_expect_tx(&bs->b, nk * 128);
-    for (int t = 0; t < ntile; t++) tma_load_4d(smem_u32(sV + t * TILE_BYTES), &tv, smem_u32(&bs->b), 0, h, t * TILE, b);
-    ok = wait(bs, &bs->a, 0, p.error, 21);
-    if (ok) {
-      tc_fence_after();
-      mma_kk(tmem, smem_u32(sQ), smem_u32(sK), half0, false);                       // S[:, 0:half0]
-      if (half1) mma_kk(tmem + 256, smem_u32(sQ), smem_u32(sK + 2 * TILE_BYTES), half1, false);
-      tc_commit(&bs->c);
-    }
-  }
-  ok = wait(bs, &bs->c, 0, p.error, 22);
-  ok = __syncthreads_and(ok);
-  if (ok) {
-    tc_fence_after();
-    // pass 1: row maximum over every key; this thread scans its quarter of the columns
-    float m = -INFINITY;
-    {
-      // tensor-memory loads two chunks ahead of the arithmetic
-      const int c0 = cg * (nk / 128), c1 = (cg + 1) * (nk / 128);
-      uint32_t ra[32], rb[32];
-      tc_ld32(lane_addr + c0 * 32, ra);
-      for (int c = c0; c < c1; c += 2) {
-        tc_wait_ld();
-        if (c + 1 < c1) tc_ld32(lane_addr + (c + 1) * 32, rb);
-#pragma unroll
-        for (int j = 0; j < 32; j++) m = fmaxf(m, __uint_as_float(ra[j]));
-        if (c + 1 < c1) {
-          tc_wait_ld();
-          if (c + 2 < c1) tc_ld32(lane_addr + (c + 2) * 32, ra);
-#pragma unroll
-          for (int j = 0; j < 32; j++) m = fmaxf(m, __uint_as_float(rb[j]));
+  if (warp >= 8) {
+    regs_issue<true>();
+    Phases ph;
+    bool ok = true;
+    auto wait = [&](int i, uint32_t code) {
+      ok = __all_sync(0xffffffffu, mbar_wait_abortable(&bs->abort, &bs->bar[i], ph.next(i), p.error, code)) && ok;
+    };
+    if (warp == 10) {                                        // ---- loads
+      uint32_t issued = 0, landing = 0;                      // by barrier: a copy has been issued; the parity after it
+      for (int u = u0; u < u1 && ok; u++) {
+        const Unit un = unit_at(u, mode, tiles, heads);
+        const int nx = un.both ? 2 : 1, nk = mode == kHeads ? nx : blocks;   // key blocks held: those of the head, or one of each
+        // Q of A, the first keys, Q of B, the other keys, the values
+#pragma unroll 1
+        for (int n = 0; n < nx + 2 * nk && ok; n++) {
+          const bool is_q = n == 0 || (n == 2 && nx == 2);
+          const int kv = n - 1 - (n > 2 && nx == 2), x = n >> 1, is_v = kv >= nk, i = is_v ? kv - nk : kv;
+          const int full = is_q ? kQFull + x : kKvFull + 4 * is_v + i, empty = is_q ? kQFree + x : kKvFree + 4 * is_v + i;
+          const int bh = is_q ? un.bh[x] : mode == kHeads ? un.bh[i] : un.bh[0];
+          const int row = is_q ? un.q[x] * TILE : mode == kHeads ? 0 : i * TILE;
+          uint8_t* const dst = is_q ? sQ + x * TILE_BYTES : (is_v ? sV : sK) + i * TILE_BYTES;
+          if ((issued >> full) & 1u) wait(empty, 21);
+          if (!ok) break;
+          const int b = bh / p.H, h = bh - b * p.H;
+          if (lane == 0) {
+            mbar_expect_tx(&bs->bar[full], TILE_BYTES);
+            tma_load_4d(smem_u32(dst), is_q ? &tq : is_v ? &tv : &tk, smem_u32(&bs->bar[full]), 0, h, row, b);
+          }
+          issued |= 1u << full;
+          landing ^= 1u << full;
         }
       }
+      // nothing may be in flight when the CTA ends (there is something to wait for only after a wait gave up)
+#pragma unroll 1
+      for (int i = 0; i < kKvFree; i++) if ((issued >> i) & 1u) landed(&bs->bar[i], (landing >> i) & 1u);
+    } else if (warp < 10) {                                  // ---- products, warp 8: of tile A, 9: of tile B
+      const int x = warp - 8;
+      bool held = false;                                     // S has been written before
+      const uint32_t id_qk = idesc_f16(TILE, false, false), id_pv = idesc_f16(D, false, true);
+      const uint64_t dq = smem_desc_sw128(smem_u32(sQ + x * TILE_BYTES)), dk = smem_desc_sw128(smem_u32(sK)), dv = smem_desc_mn_sw128(smem_u32(sV));
+      const bool apart = mode == kHeads;                     // each tile has its own keys
+      for (int u = u0; u < u1 && ok; u++) {
+        const Unit un = unit_at(u, mode, tiles, heads);
+        if (x && !un.both) {                                 // nothing to do but to let go of what the other tile is given
+          if (mode == kPair)
+#pragma unroll 1
+            for (int i = 0; i < 2 * blocks && ok; i++) {
+              const int op = i < blocks ? i : 4 + i - blocks;
+              wait(kKvFull + op, 22);
+              if (ok && lane == 0) mbar_arrive(&bs->bar[kKvFree + op]);
+              __syncwarp();
+            }
+          continue;
+        }
+        // step j: S of block j, then O of block j - 1
+#pragma unroll 1
+        for (int j = 0; j <= blocks && ok; j++) {
+          if (j < blocks) {
+            const int i = apart ? x : j;
+            if (j == 0) wait(kQFull + x, 23);
+            wait(kKvFull + i, 24);
+            if (held) wait(kSFree + x, 25);
+            held = true;
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t db = dk + i * (uint64_t)(TILE_BYTES >> 4);
+            if (lane == 0) {
+#pragma unroll
+              for (int k = 0; k < 4; k++) tc_mma(col_s(x), dq + 2 * k, db + 2 * k, id_qk, k != 0);
+              tc_commit(&bs->bar[kSFull + x]);
+              tc_commit(&bs->bar[kKvFree + i]);
+              if (j == blocks - 1) tc_commit(&bs->bar[kQFree + x]);
+            }
+            __syncwarp();
+          }
+          if (j > 0) {
+            const int i = apart ? x : j - 1;
+            wait(kKvFull + 4 + i, 26);
+            wait(kPFull + x, 27);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t db = dv + i * (uint64_t)(TILE_BYTES >> 4);
+            if (lane == 0) {
+#pragma unroll
+              for (int k = 0; k < 8; k++) tc_mma_ts(col_o(x), col_p(x) + 8 * k, db + (2048 >> 4) * k, id_pv, k != 0 || j != 1);
+              tc_commit(&bs->bar[kPv + x]);
+              tc_commit(&bs->bar[kKvFree + 4 + i]);
+            }
+            __syncwarp();
+          }
+        }
+      }
+      if (lane == 0) drain(&bs->bar[kFwdDrain + x]);
     }
-    bs->red[cg][row] = m;
-    __syncthreads();
-    m = fmaxf(fmaxf(bs->red[0][row], bs->red[1][row]), fmaxf(bs->red[2][row], bs->red[3][row]));
-    __syncthreads();                        // red is reused for the row sums below
-    const float ms = m * p.scale_log2;
-    float l = 0.0f;
-    // pass 2: exponentials, row sum, P as bf16 in the A-operand layout; then O += P V for that half
-    for (int hf = 0; hf < 2; hf++) {      // same trip count for every thread: the loop body holds barriers
-      const int keys = hf ? half1 : half0;
-      if (!keys) break;
-      uint8_t* sP = hf ? sP1 : sK;
-      {
-        // this thread's one or two chunks of the half: both loads are issued before the first is used
-        const int c0 = cg * (keys / 128), two = keys / 128 == 2;
-        uint32_t ra[32], rb[32];
-        tc_ld32(lane_addr + hf * 256 + c0 * 32, ra);
-        if (two) tc_ld32(lane_addr + hf * 256 + (c0 + 1) * 32, rb);
+  } else {
+    // ---- softmax and output: one query per thread
+    regs_row<true>();
+    const int x = warp >> 2, row = tid & 127;
+    // the whole warp goes on or gives up: what follows is collective
+    Phases ph;
+    auto wait_all = [&](int i, uint32_t code) {
+      return __all_sync(0xffffffffu, mbar_wait_abortable(&bs->abort, &bs->bar[i], ph.next(i), p.error, code)) != 0;
+    };
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+    uint8_t* const stage = sO + warp * (32 * 128);           // the warp's 32 rows
+    bool ok = true;
+    for (int u = u0; u < u1 && ok; u++) {
+      const Unit un = unit_at(u, mode, tiles, heads);
+      if (x == 1 && !un.both) continue;
+      float m = 0.0f;
+      uint64_t l2 = 0, l2b = 0;
+      for (int j = 0; j < blocks; j++) {
+        if (!(ok = ok && wait_all(kSFull + x, 28))) break;
+        tc_fence_after();
+        uint32_t s[4][32];
+#pragma unroll
+        for (int c = 0; c < 4; c++) tc_ld32(col_s(x) + lanes + c * 32, s[c]);
         tc_wait_ld();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bs->bar[kSFree + x]);
+        if (j == blocks - 1 && p.S < blocks * TILE) {        // keys that do not exist
+          const int valid = p.S - j * TILE;
+#pragma unroll
+          for (int c = 0; c < 4; c++)
+#pragma unroll
+            for (int i = 0; i < 32; i++) if (c * 32 + i >= valid) s[c][i] = 0xff800000u;   // -inf
+        }
+        float bm[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          bm[c] = fmaxf(__uint_as_float(s[c][0]), __uint_as_float(s[c][1]));
+#pragma unroll
+          for (int i = 2; i < 32; i += 2) bm[c] = max3(bm[c], __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
+        }
+        const float top = max3(fmaxf(bm[0], bm[1]), bm[2], bm[3]);
+        // The running maximum follows only where it has fallen kRescale behind: probabilities up to 2^kRescale are as exact
+        // as those up to 1, and O hardly ever has to be read back.
+        float keep = 1.0f;
+        if (j == 0) m = fmaxf(top, -1e30f);                  // finite: a block of -inf does not decide the row
+        else if ((top - m) * p.scale_log2 > kRescale) {
+          keep = ex2_ftz((m - top) * p.scale_log2);
+          m = top;
+        }
+        const float ms = m * p.scale_log2;
+        const uint64_t sl = tc::pack2(p.scale_log2, p.scale_log2), nm = tc::pack2(-ms, -ms);
+        if (j) {
+          const uint64_t k2 = tc::pack2(keep, keep);
+          l2 = mul2(l2, k2);
+          l2b = mul2(l2b, k2);
+        }
+        uint32_t pk[64];
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            float a, b;
+            unpack2(fma2(tc::pack2(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), sl, nm), a, b);
+            a = ex2_ftz(a);
+            b = ex2_ftz(b);
+            if (i & 2) l2 = add2(l2, tc::pack2(a, b)); else l2b = add2(l2b, tc::pack2(a, b));
+            pk[c * 16 + i / 2] = pack2(a, b);
+          }
+        if (j) {
+          if (!(ok = ok && wait_all(kPv + x, 29))) break;   // P of the last block has been read, O holds it
+          tc_fence_after();
+          if (__any_sync(0xffffffffu, keep != 1.0f)) {
+            uint32_t o[32];
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+              tc_ld32(col_o(x) + lanes + c * 32, o);
+              tc_wait_ld();
+#pragma unroll
+              for (int i = 0; i < 32; i++) o[i] = __float_as_uint(__uint_as_float(o[i]) * keep);
+              tc_st32(col_o(x) + lanes + c * 32, o);
+            }
+          }
+        }
+        tc_st32(col_p(x) + lanes, pk);
+        tc_st32(col_p(x) + lanes + 32, pk + 32);
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bs->bar[kPFull + x]);
+      }
+      ok = ok && wait_all(kPv + x, 30);
+      if (!ok) break;
+      tc_fence_after();
+      float la, lb, lc, ld;
+      unpack2(l2, la, lb);
+      unpack2(l2b, lc, ld);
+      const float l = (la + lb) + (lc + ld), inv = 1.0f / l;
+      uint32_t o[2][32];
+      tc_ld32(col_o(x) + lanes, o[0]);
+      tc_ld32(col_o(x) + lanes + 32, o[1]);
+      tc_wait_ld();
+      if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the last store has read the staging rows
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
         float v[32];
 #pragma unroll
-        for (int j = 0; j < 32; j++) {
-          v[j] = ex2_ftz(fmaf(__uint_as_float(ra[j]), p.scale_log2, -ms));
-          l += v[j];
-        }
-        store_kmajor32(sP, row, c0 * 32, v);
-        if (two) {
-#pragma unroll
-          for (int j = 0; j < 32; j++) {
-            v[j] = ex2_ftz(fmaf(__uint_as_float(rb[j]), p.scale_log2, -ms));
-            l += v[j];
-          }
-          store_kmajor32(sP, row, (c0 + 1) * 32, v);
-        }
+        for (int i = 0; i < 32; i++) v[i] = __uint_as_float(o[c][i]) * inv;
+        store_row32(stage, lane, c * 32, v);
       }
+      if (un.q[x] * TILE + row < p.S) p.lse[(size_t)un.bh[x] * p.S + un.q[x] * TILE + row] = m * p.scale_log2 + log2f(l);
       proxy_fence();
-      tc_fence_before();
-      __syncthreads();
-      if (tid == 0) {
-        if (hf == 0 && ok) ok = wait(bs, &bs->b, 0, p.error, 23);
-        if (ok) {
-          tc_fence_after();
-          const uint32_t id = idesc_f16(D, false, true);
-          for (int blk = 0; blk < keys / 64; blk++) {
-            const uint64_t da = smem_desc_sw128(smem_u32(sP + blk * TILE_BYTES));
-            const uint64_t db = smem_desc_mn_sw128(smem_u32(sV + (hf * 256 + blk * 64) * 128));
-#pragma unroll
-            for (int k = 0; k < 4; k++) tc_mma(tmem, da + 2 * k, db + (2048 >> 4) * k, id, (hf | blk | k) != 0);
-          }
-          if (hf == 1 || !half1) tc_commit(&bs->d);
-        }
-      }
+      __syncwarp();
+      const int r0 = un.q[x] * TILE + (warp & 3) * 32;       // the map clips a partial block's rows
+      if (lane == 0 && r0 < p.S) tma_store_4d(&to, smem_u32(stage), 0, un.bh[x] % p.H, r0, un.bh[x] / p.H);
     }
-    bs->red[cg][row] = l;
-    ok = ok && wait(bs, &bs->d, 0, p.error, 24);
-    ok = __syncthreads_and(ok);
-    if (ok) {
-      tc_fence_after();
-      l = (bs->red[0][row] + bs->red[1][row]) + (bs->red[2][row] + bs->red[3][row]);
-      const float inv = 1.0f / l;
-      const size_t orow = (((size_t)b * p.S + q0 + row) * p.H + h) * D;
-      if (cg < 2) {                          // 64 output columns: column groups 0 and 1 take 32 each
-        const int c = cg;
-        uint32_t r[32];
-        tc_ld32(lane_addr + c * 32, r);
-        tc_wait_ld();
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          uint4 o = make_uint4(pack2(__uint_as_float(r[8 * j]) * inv, __uint_as_float(r[8 * j + 1]) * inv),
-                               pack2(__uint_as_float(r[8 * j + 2]) * inv, __uint_as_float(r[8 * j + 3]) * inv),
-                               pack2(__uint_as_float(r[8 * j + 4]) * inv, __uint_as_float(r[8 * j + 5]) * inv),
-                               pack2(__uint_as_float(r[8 * j + 6]) * inv, __uint_as_float(r[8 * j + 7]) * inv));
-          *reinterpret_cast<uint4*>(p.out + orow + c * 32 + j * 8) = o;
-        }
-      }
-      if (cg == 0) p.lse[((size_t)b * p.H + h) * p.S + q0 + row] = ms + log2f(l);
-    }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
-  if (tid == 0) drain(bs);
   tc_fence_before();
   __syncthreads();
-  tmem_free<512>(tmem, warp);
+  if (warp == 0) tmem_free_all(tmem);
 }
 
 // delta[b][h][s] = sum_d dO[b][s][h][d] * O[b][s][h][d]; eight lanes per row, so that a warp reads whole lines (262 144
@@ -317,282 +449,324 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
   }
 }
 
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr) : "memory");
-}
+// ------------------------------------------------------------------------------ backward
+// Barriers, each for tile A and B, for the two operands of the sequence's four blocks, or for two units' statistics.
+enum BwdBar { kAFull = 0, kAFree = 2, kBFull = 4, kBFree = 12, kStatFull = 16, kStatFree = 18, kSAt = 20, kSGone = 22, kDpAt = 24, kDpGone = 26,
+              kReady = 28, kAcc = 30, kBwdBars = 32 };
+struct BwdBars {
+  uint64_t bar[kBwdBars], drain[2];
+  uint32_t tmem_base;
+  volatile uint32_t abort;
+};
 
-// P and dS of one 128 x STEP tile from S (tensor-memory columns 0..STEP-1) and dP (the STEP columns behind), this thread's row
-// and 16-column group c of each 64-column panel, as K-major operands. COLS: lse and delta belong to the columns (nlse / ndelta: their negatives for
-// this tile's columns in shared memory) and P is written too; else they are the row's (nlse[0], ndelta[0]).
-template <bool COLS, int STEP>
-__device__ __forceinline__ void softmax_grad_tile(uint32_t lane_addr, int row, int c, const float* nlse, const float* ndelta,
-                                                  const Params& p, uint8_t* sP, uint8_t* sdS) {
-  const uint64_t sl = tc::pack2(p.scale_log2, p.scale_log2), sc = tc::pack2(p.scale, p.scale), one = tc::pack2(1.0f, 1.0f);
-#pragma unroll
-  for (int h = 0; h < Step<STEP>::PANELS; h++) {
-    const int col = h * 64 + c * 16;
-    uint32_t rs[16], rd[16];
-    tc_ld16(lane_addr + col, rs);
-    tc_ld16(lane_addr + STEP + col, rd);
-    tc_wait_ld();
-    float pv[16], ds[16];
-#pragma unroll
-    for (int j = 0; j < 16; j += 2) {
-      const uint64_t nl = COLS ? *reinterpret_cast<const uint64_t*>(nlse + col + j) : tc::pack2(nlse[0], nlse[0]);
-      const uint64_t nd = COLS ? *reinterpret_cast<const uint64_t*>(ndelta + col + j) : tc::pack2(ndelta[0], ndelta[0]);
-      float a, b;
-      unpack2(fma2(tc::pack2(__uint_as_float(rs[j]), __uint_as_float(rs[j + 1])), sl, nl), a, b);
-      pv[j] = ex2_ftz(a);
-      pv[j + 1] = ex2_ftz(b);
-      const uint64_t d = fma2(tc::pack2(__uint_as_float(rd[j]), __uint_as_float(rd[j + 1])), one, nd);
-      unpack2(mul2(mul2(tc::pack2(pv[j], pv[j + 1]), d), sc), ds[j], ds[j + 1]);
-    }
-    if (COLS) store_kmajor16(sP + h * TILE_BYTES, row, c * 16, pv);
-    store_kmajor16(sdS + h * TILE_BYTES, row, c * 16, ds);
-  }
-}
-
-// Write this thread's row of a 64-column fp32 accumulator (tensor-memory column `col`) as bf16 to `dst`.
-__device__ __forceinline__ void store_acc_row(uint32_t lane_addr, int col, int c, __nv_bfloat16* dst) {
-  {                                          // chunk c (0 or 1) of the 64 columns
-    uint32_t r[32];
-    tc_ld32(lane_addr + col + c * 32, r);
-    tc_wait_ld();
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      uint4 o = make_uint4(pack2(__uint_as_float(r[8 * j]), __uint_as_float(r[8 * j + 1])),
-                           pack2(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3])),
-                           pack2(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5])),
-                           pack2(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7])));
-      *reinterpret_cast<uint4*>(dst + c * 32 + j * 8) = o;
-    }
-  }
-}
-
-// ------------------------------------------------------------------- backward: dK and dV
-template <int STEP>
-__global__ void __launch_bounds__(NT, Step<STEP>::CTAS)
-attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
-                     const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo, const Params p) {
-  constexpr int STEP_BYTES = Step<STEP>::BYTES, PANELS = Step<STEP>::PANELS;
+// KV = true: a tile is 128 keys, the loop runs over blocks of 64 queries: S^T = K Q^T, dP^T = V dO^T, dV += P^T dO, dK += dS^T Q.
+// KV = false: a tile is 128 queries, the loop runs over blocks of 64 keys: S = Q K^T, dP = dO V^T, dQ += dS K.
+// a1, a2: the tile's operands (K, V or Q, dO); b1, b2: those of the whole sequence (Q, dO or K, V); to1, to2: dV, dK or -, dQ.
+template <bool KV>
+__global__ void __launch_bounds__(kThreads, 1)
+attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__ CUtensorMap ta2, const __grid_constant__ CUtensorMap tb1,
+                const __grid_constant__ CUtensorMap tb2, const __grid_constant__ CUtensorMap to1, const __grid_constant__ CUtensorMap to2,
+                const Params p, int units, int mode) {
+  constexpr int STEP = 64, STEP_BYTES = STEP * D * 2;
   extern __shared__ uint8_t raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* sK = base;                        // 16 KB each
-  uint8_t* sV = sK + TILE_BYTES;
-  uint8_t* sP = sV + TILE_BYTES;             // P^T, dS^T: panels of [128 keys][64 queries]
-  uint8_t* sdS = sP + PANELS * TILE_BYTES;
-  uint8_t* sQ = sdS + PANELS * TILE_BYTES;   // two buffers each
-  uint8_t* sdO = sQ + 2 * STEP_BYTES;
-  float* nlse = reinterpret_cast<float*>(sdO + 2 * STEP_BYTES);      // -lse and -delta of every query
-  float* ndelta = nlse + MAX_S;
-  Bars* bs = reinterpret_cast<Bars*>(ndelta + MAX_S);
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int row = (warp & 3) * 32 + (tid & 31), cg = warp >> 2;
-  const int k0 = blockIdx.x * TILE, h = blockIdx.y, b = blockIdx.z;
-  const int nq = p.S / STEP;
+  uint8_t* const sA = base;                  // [tile A, B][a1, a2]
+  uint8_t* const sB1 = sA + 4 * TILE_BYTES;  // the sequence, 128 rows per slot
+  uint8_t* const sB2 = sB1 + 4 * TILE_BYTES;
+  uint8_t* const sO = sB2 + 4 * TILE_BYTES;  // 2 KB per row warp
+  float* const stats = reinterpret_cast<float*>(sO + TILE_BYTES);      // KV: [2][-lse, -delta][MAX_S], the units in turn
+  BwdBars* const bs = reinterpret_cast<BwdBars*>(stats + 4 * MAX_S);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // warp: uniform
+  const int tiles = (p.S + TILE - 1) / TILE, heads = p.B * p.H;
+  const int u0 = (int)((long long)units * blockIdx.x / gridDim.x), u1 = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
+  const int nb = (p.S + STEP - 1) / STEP;
 
   if (tid == 0) {
-    mbar_init(&bs->a, 1); mbar_init(&bs->c, 1); mbar_init(&bs->d, 1); mbar_init(&bs->drain, 1);
-    mbar_init(&bs->e[0], 1); mbar_init(&bs->e[1], 1);
+    // 4: the warps of a tile, 8: all row warps, 32: the warp that fetches statistics; a sequence that two tiles share is free
+    // when both have used it
+    for (int i = 0; i < kBwdBars; i++) {
+      const int pair = i & ~1;
+      mbar_init(&bs->bar[i], pair == kSGone || pair == kDpGone || pair == kReady ? 4 : pair == kStatFree ? 8 : pair == kStatFull ? 32
+                             : i >= kBFree && i < kStatFull && mode == kPair ? 2 : 1);
+    }
+    mbar_init(&bs->drain[0], 1); mbar_init(&bs->drain[1], 1);
     bs->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  static_assert(MAX_S <= NT, "one query's statistics per thread");
-  if (tid < p.S) {
-    const size_t stat = ((size_t)b * p.H + h) * p.S + tid;
-    nlse[tid] = -p.lse[stat];
-    ndelta[tid] = -p.delta[stat];
-  }
-  tmem_alloc<Step<STEP>::COLS>(bs, warp);
+  if (warp == 0) tmem_alloc_all(&bs->tmem_base);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bs->tmem_base;
-  const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-  constexpr uint32_t COL_S = 0, COL_DV = 2 * STEP, COL_DK = COL_DV + D;      // dP^T sits at COL_S + STEP
-  bool ok = true;
+  pdl_trigger();
+  pdl_wait();
+  // Columns of a tile: S 64, dP 64, two accumulators of 64. P and dS (32 each, bf16) take dP's place once it has been read; with
+  // one accumulator dS has a place of its own, and dP can be refilled at once.
+  auto col = [&](int x) { return tmem + x * 256; };
+  constexpr uint32_t DP = 64, P_AT = 64, DS_AT = KV ? 96 : 128, ACC1 = 128, ACC2 = 192;
 
-  if (tid == 0) {
-    mbar_expect_tx(&bs->a, 2 * TILE_BYTES);
-    tma_load_4d(smem_u32(sK), &tk, smem_u32(&bs->a), 0, h, k0, b);
-    tma_load_4d(smem_u32(sV), &tv, smem_u32(&bs->a), 0, h, k0, b);
-    mbar_expect_tx(&bs->e[0], 2 * STEP_BYTES);
-    tma_load_4d(smem_u32(sQ), &tq, smem_u32(&bs->e[0]), 0, h, 0, b);
-    tma_load_4d(smem_u32(sdO), &tdo, smem_u32(&bs->e[0]), 0, h, 0, b);
-    ok = wait(bs, &bs->a, 0, p.error, 31);
-  }
-  for (int i = 0; i < nq; i++) {
-    const int buf = i & 1;
-    uint8_t* q = sQ + buf * STEP_BYTES;
-    uint8_t* go = sdO + buf * STEP_BYTES;
-    if (tid == 0 && ok) {
-      // S and dP of this step right behind the products of the last one, whose end nothing here waits for
-      ok = wait(bs, &bs->e[buf], (i >> 1) & 1, p.error, 33);
-      if (ok) {
+  if (warp >= 8) {
+    regs_issue<false>();
+    Phases ph;
+    bool ok = true;
+    auto wait = [&](int i, uint32_t code) {
+      ok = __all_sync(0xffffffffu, mbar_wait_abortable(&bs->abort, &bs->bar[i], ph.next(i), p.error, code)) && ok;
+    };
+    if (warp == 10) {                                        // ---- loads
+      uint32_t issued = 0, landing = 0;                      // by barrier: a copy has been issued; the parity after it
+      for (int u = u0; u < u1 && ok; u++) {
+        const Unit un = unit_at(u, mode, tiles, heads);
+        const int nx = un.both ? 2 : 1, slots = mode == kHeads ? nx : tiles;
+        // the operands of A, the first block of the sequence, the operands of B, the other blocks; two copies each
+#pragma unroll 1
+        for (int n = 0; n < 2 * (nx + slots) && ok; n++) {
+          const int which = n & 1, m = n >> 1;
+          const bool is_a = m == 0 || (m == 2 && nx == 2);
+          const int x = m >> 1, i = m - 1 - (m > 2 && nx == 2);
+          const int full = is_a ? kAFull + x : kBFull + 4 * which + i;
+          const int bh = is_a ? un.bh[x] : mode == kHeads ? un.bh[i] : un.bh[0];
+          const int row = is_a ? un.q[x] * TILE : mode == kHeads ? 0 : i * TILE;
+          uint8_t* const dst = is_a ? sA + (2 * x + which) * TILE_BYTES : (which ? sB2 : sB1) + i * TILE_BYTES;
+          if (!which && ((issued >> full) & 1u)) wait(is_a ? kAFree + x : kBFree + i, 31);
+          if (!ok) break;
+          const int b = bh / p.H, h = bh - b * p.H;
+          const bool arms = !is_a || !which;                 // one barrier for both operands of a tile
+          if (lane == 0) {
+            if (arms) mbar_expect_tx(&bs->bar[full], is_a ? 2 * TILE_BYTES : TILE_BYTES);
+            tma_load_4d(smem_u32(dst), is_a ? (which ? &ta2 : &ta1) : (which ? &tb2 : &tb1), smem_u32(&bs->bar[full]), 0, h, row, b);
+          }
+          if (arms) landing ^= 1u << full;
+          issued |= 1u << full;
+        }
+      }
+      // nothing may be in flight when the CTA ends (there is something to wait for only after a wait gave up)
+#pragma unroll 1
+      for (int i = 0; i < kBFree; i++) if ((i < kAFree || i >= kBFull) && ((issued >> i) & 1u)) landed(&bs->bar[i], (landing >> i) & 1u);
+    } else if (warp < 10) {                                  // ---- products, warp 8: of tile A, 9: of tile B
+      const int x = warp - 8;
+      bool s_held = false, dp_held = false;                  // S, dP has been written before
+      const uint32_t id_s = idesc_f16(STEP, false, false), id_acc = idesc_f16(D, false, true), tm = col(x);
+      const uint64_t da1 = smem_desc_sw128(smem_u32(sA + 2 * x * TILE_BYTES)), da2 = smem_desc_sw128(smem_u32(sA + (2 * x + 1) * TILE_BYTES));
+      const bool apart = mode == kHeads;                     // each tile has its own sequence
+      const int first = apart ? x * TILE_BYTES : 0;
+      const uint64_t db1 = smem_desc_sw128(smem_u32(sB1 + first)), db2 = smem_desc_sw128(smem_u32(sB2 + first));
+      const uint64_t dm1 = smem_desc_mn_sw128(smem_u32(sB1 + first)), dm2 = smem_desc_mn_sw128(smem_u32(sB2 + first));
+      for (int u = u0; u < u1 && ok; u++) {
+        const Unit un = unit_at(u, mode, tiles, heads);
+        if (x && !un.both) {                                 // nothing to do but to let go of what the other tile is given
+          if (mode == kPair)
+#pragma unroll 1
+            for (int i = 0; i < tiles && ok; i++) {
+              wait(kBFull + i, 32);
+              wait(kBFull + 4 + i, 32);
+              if (ok && lane == 0) mbar_arrive(&bs->bar[kBFree + i]);
+              __syncwarp();
+            }
+          continue;
+        }
+        // Round i: S of block i (and dP, where that has a place of its own), then the accumulators of block i - 1 (and dP of
+        // block i, which takes the place of what they have read).
+        auto dp_mma = [&](int i) {
+          const uint64_t db = db2 + i * (uint64_t)(STEP_BYTES >> 4);
+          if (!(i & 1)) wait(kBFull + 4 + (apart ? x : i >> 1), 36);
+          if (!KV && dp_held) wait(kDpGone + x, 37);
+          dp_held = true;
+          if (!ok) return;
+          tc_fence_after();
+          if (lane == 0) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) tc_mma(tm + DP, da2 + 2 * k, db + 2 * k, id_s, k != 0);
+            tc_commit(&bs->bar[kDpAt + x]);
+            if (i == nb - 1) tc_commit(&bs->bar[kAFree + x]);
+          }
+          __syncwarp();
+        };
+#pragma unroll 1
+        for (int i = 0; i <= nb && ok; i++) {
+          if (i < nb) {
+            const uint64_t db = db1 + i * (uint64_t)(STEP_BYTES >> 4);
+            if (i == 0) wait(kAFull + x, 33);
+            if (!(i & 1)) wait(kBFull + (apart ? x : i >> 1), 34);
+            if (s_held) wait(kSGone + x, 35);
+            s_held = true;
+            if (!ok) break;
+            tc_fence_after();
+            if (lane == 0) {
+#pragma unroll
+              for (int k = 0; k < 4; k++) tc_mma(tm, da1 + 2 * k, db + 2 * k, id_s, k != 0);
+              tc_commit(&bs->bar[kSAt + x]);
+            }
+            __syncwarp();
+            if (!KV) dp_mma(i);
+          }
+          if (i > 0) {
+            const uint64_t off = (i - 1) * (uint64_t)(STEP_BYTES >> 4), d1 = dm1 + off, d2 = dm2 + off;
+            wait(kReady + x, 38);
+            if (!ok) break;
+            tc_fence_after();
+            if (lane == 0) {
+#pragma unroll
+              for (int k = 0; k < 4; k++) {
+                if (KV) tc_mma_ts(tm + ACC1, tm + P_AT + 8 * k, d2 + (2048 >> 4) * k, id_acc, k != 0 || i != 1);
+                tc_mma_ts(tm + ACC2, tm + DS_AT + 8 * k, d1 + (2048 >> 4) * k, id_acc, k != 0 || i != 1);
+              }
+              tc_commit(&bs->bar[kAcc + x]);
+              if (!(i & 1) || i == nb) tc_commit(&bs->bar[kBFree + (apart ? x : (i - 1) >> 1)]);
+            }
+            __syncwarp();
+          }
+          if (KV && i < nb) dp_mma(i);
+        }
+      }
+      if (lane == 0) drain(&bs->drain[x]);
+    } else if (KV && warp == 11) {                           // ---- statistics of the queries
+      for (int u = u0, n = 0; u < u1 && ok; u++, n++) {
+        const Unit un = unit_at(u, mode, tiles, heads);
+        if (n >= 2) wait(kStatFree + (n & 1), 39);
+        if (!ok) break;
+        float* const st = stats + (n & 1) * 2 * MAX_S;
+        // kHeads: one head's rows per 128. A query that does not exist has no probabilities (its rows of Q and dO are zeros).
+        const int rows = mode == kHeads ? (un.both ? 2 * TILE : TILE) : tiles * TILE;
+        for (int r = lane; r < rows; r += 32) {
+          const int head = mode == kHeads ? un.bh[r >> 7] : un.bh[0], q = mode == kHeads ? r & (TILE - 1) : r;
+          const bool there = q < p.S;
+          st[r] = there ? -p.lse[(size_t)head * p.S + q] : -INFINITY;
+          st[MAX_S + r] = there ? -p.delta[(size_t)head * p.S + q] : 0.0f;
+        }
+        mbar_arrive(&bs->bar[kStatFull + (n & 1)]);
+      }
+    }
+  } else {
+    // ---- gradients of the scores, results: one row of the tile per thread
+    regs_row<false>();
+    const int x = warp >> 2, row = tid & 127;
+    // the whole warp goes on or gives up: what follows is collective
+    Phases ph;
+    auto wait_all = [&](int i, uint32_t code) {
+      return __all_sync(0xffffffffu, mbar_wait_abortable(&bs->abort, &bs->bar[i], ph.next(i), p.error, code)) != 0;
+    };
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+    uint8_t* const stage = sO + warp * kStageWarpBytes;
+    bool ok = true;
+    const uint64_t sl = tc::pack2(p.scale_log2, p.scale_log2), sc = tc::pack2(p.scale, p.scale);
+    for (int u = u0, n = 0; u < u1 && ok; u++, n++) {
+      const Unit un = unit_at(u, mode, tiles, heads);
+      const float* st = stats + (n & 1) * 2 * MAX_S + (mode == kHeads && x ? TILE : 0);
+      uint64_t nl = 0, nd = 0;
+      if (KV) {
+        if (!(ok = wait_all(kStatFull + (n & 1), 40))) break;
+      } else if ((x == 0 || un.both) && un.q[x] * TILE + row < p.S) {   // rows past the end give values that nothing stores
+        const size_t at = (size_t)un.bh[x] * p.S + un.q[x] * TILE + row;
+        const float l = -p.lse[at], d = -p.delta[at];
+        nl = tc::pack2(l, l);
+        nd = tc::pack2(d, d);
+      }
+      if (x == 0 || un.both) {
+        for (int i = 0; i < nb; i++) {
+          if (!(ok = wait_all(kSAt + x, 41))) break;
+          tc_fence_after();
+          uint32_t s[2][32];
+          tc_ld32(col(x) + lanes, s[0]);
+          tc_ld32(col(x) + lanes + 32, s[1]);
+          tc_wait_ld();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bs->bar[kSGone + x]);
+          uint32_t pk[32], dk[32];
+          float pv[64];
+#pragma unroll
+          for (int c = 0; c < 2; c++)
+#pragma unroll
+            for (int e = 0; e < 32; e += 4) {
+              uint64_t l0 = nl, l1 = nl;
+              if (KV) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(st + i * STEP + c * 32 + e);
+                l0 = v.x; l1 = v.y;
+              }
+              float* const o = pv + c * 32 + e;
+              unpack2(fma2(tc::pack2(__uint_as_float(s[c][e]), __uint_as_float(s[c][e + 1])), sl, l0), o[0], o[1]);
+              unpack2(fma2(tc::pack2(__uint_as_float(s[c][e + 2]), __uint_as_float(s[c][e + 3])), sl, l1), o[2], o[3]);
+#pragma unroll
+              for (int k = 0; k < 4; k++) o[k] = ex2_ftz(o[k]);
+              if (KV) {
+                pk[c * 16 + e / 2] = pack2(o[0], o[1]);
+                pk[c * 16 + e / 2 + 1] = pack2(o[2], o[3]);
+              }
+            }
+          if (!(ok = wait_all(kDpAt + x, 42))) break;
+          tc_fence_after();
+          tc_ld32(col(x) + DP + lanes, s[0]);
+          tc_ld32(col(x) + DP + lanes + 32, s[1]);
+          tc_wait_ld();
+          if (!KV) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bs->bar[kDpGone + x]);
+          }
+#pragma unroll
+          for (int c = 0; c < 2; c++)
+#pragma unroll
+            for (int e = 0; e < 32; e += 4) {
+              uint64_t d0 = nd, d1 = nd;
+              if (KV) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(st + MAX_S + i * STEP + c * 32 + e);
+                d0 = v.x; d1 = v.y;
+              }
+              const float* const o = pv + c * 32 + e;
+              float a, b;
+              unpack2(mul2(mul2(tc::pack2(o[0], o[1]), add2(tc::pack2(__uint_as_float(s[c][e]), __uint_as_float(s[c][e + 1])), d0)), sc), a, b);
+              dk[c * 16 + e / 2] = pack2(a, b);
+              unpack2(mul2(mul2(tc::pack2(o[2], o[3]), add2(tc::pack2(__uint_as_float(s[c][e + 2]), __uint_as_float(s[c][e + 3])), d1)), sc), a, b);
+              dk[c * 16 + e / 2 + 1] = pack2(a, b);
+            }
+          if (i) {                                           // the last block's P and dS have been read
+            if (!(ok = wait_all(kAcc + x, 43))) break;
+            tc_fence_after();
+          }
+          if (KV) tc_st32(col(x) + P_AT + lanes, pk);
+          tc_st32(col(x) + DS_AT + lanes, dk);
+          tc_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bs->bar[kReady + x]);
+        }
+        ok = ok && wait_all(kAcc + x, 44);
+        if (!ok) break;
         tc_fence_after();
-        mma_kk(tmem + COL_S, smem_u32(sK), smem_u32(q), STEP, false);            // S^T  = K_j Q_i^T
-        mma_kk(tmem + COL_S + STEP, smem_u32(sV), smem_u32(go), STEP, false);    // dP^T = V_j dO_i^T
-        tc_commit(&bs->c);
-      }
-      // the other buffer was last read by the MMAs of step i-1; once they are done, block i+1 is fetched into it
-      if (ok && i + 1 < nq) {
-        if (i >= 1) ok = wait(bs, &bs->d, (i - 1) & 1, p.error, 32);
-        if (ok) {
-          mbar_expect_tx(&bs->e[buf ^ 1], 2 * STEP_BYTES);
-          tma_load_4d(smem_u32(sQ + (buf ^ 1) * STEP_BYTES), &tq, smem_u32(&bs->e[buf ^ 1]), 0, h, (i + 1) * STEP, b);
-          tma_load_4d(smem_u32(sdO + (buf ^ 1) * STEP_BYTES), &tdo, smem_u32(&bs->e[buf ^ 1]), 0, h, (i + 1) * STEP, b);
+        const int h = un.bh[x] % p.H, b = un.bh[x] / p.H, r0 = un.q[x] * TILE + (warp & 3) * 32;
+#pragma unroll
+        for (int c = KV ? 0 : 2; c < 4; c++) {               // dV, then dK or dQ; 32 columns at a time
+          uint32_t a[32];
+          tc_ld32(col(x) + ACC1 + lanes + c * 32, a);
+          tc_wait_ld();
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          __syncwarp();
+#pragma unroll
+          for (int k = 0; k < 4; k++)
+            *reinterpret_cast<uint4*>(stage + stage_offset(lane, k)) =
+                make_uint4(pack2(__uint_as_float(a[8 * k]), __uint_as_float(a[8 * k + 1])), pack2(__uint_as_float(a[8 * k + 2]), __uint_as_float(a[8 * k + 3])),
+                           pack2(__uint_as_float(a[8 * k + 4]), __uint_as_float(a[8 * k + 5])), pack2(__uint_as_float(a[8 * k + 6]), __uint_as_float(a[8 * k + 7])));
+          proxy_fence();
+          __syncwarp();
+          if (lane == 0 && r0 < p.S) tma_store_4d(c < 2 ? &to1 : &to2, smem_u32(stage), (c & 1) * 32, h, r0, b);
         }
       }
-    }
-    ok = ok && wait(bs, &bs->c, i & 1, p.error, 34);
-    // P / dS of iteration i-1 must have been consumed by its MMAs before they are overwritten
-    if (i >= 1) ok = ok && wait(bs, &bs->d, (i - 1) & 1, p.error, 35);
-    ok = __syncthreads_and(ok);
-    if (!ok) break;
-    tc_fence_after();
-    softmax_grad_tile<true, STEP>(lane_addr + COL_S, row, cg, nlse + i * STEP, ndelta + i * STEP, p, sP, sdS);
-    proxy_fence();
-    tc_fence_before();
-    __syncthreads();
-    if (tid == 0) {
-      tc_fence_after();
-      const uint32_t id = idesc_f16(D, false, true);                // A = P^T / dS^T (K-major), B = dO / Q as [q][d]
-#pragma unroll
-      for (int h = 0; h < PANELS; h++) {
-        const uint64_t dap = smem_desc_sw128(smem_u32(sP + h * TILE_BYTES)), dad = smem_desc_sw128(smem_u32(sdS + h * TILE_BYTES));
-        const uint64_t dbo = smem_desc_mn_sw128(smem_u32(go + h * 8192)), dbq = smem_desc_mn_sw128(smem_u32(q + h * 8192));
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          tc_mma(tmem + COL_DV, dap + 2 * k, dbo + (2048 >> 4) * k, id, (i | h | k) != 0);
-          tc_mma(tmem + COL_DK, dad + 2 * k, dbq + (2048 >> 4) * k, id, (i | h | k) != 0);
-        }
+      if (KV) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bs->bar[kStatFree + (n & 1)]);
       }
-      tc_commit(&bs->d);
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
-  ok = ok && wait(bs, &bs->d, (nq - 1) & 1, p.error, 36);
-  ok = __syncthreads_and(ok);
-  if (ok) {
-    tc_fence_after();
-    const size_t orow = ((((size_t)b * p.S + k0 + row) * 3) * p.H + h) * D;     // [b][s][which][h][d], which = 0
-    // column groups 0, 1: the two halves of dK's row; 2, 3: of dV's row
-    store_acc_row(lane_addr, cg < 2 ? COL_DK : COL_DV, cg & 1, p.dqkv + orow + (size_t)(cg < 2 ? 1 : 2) * p.H * D);
-  }
-  if (tid == 0) drain(bs);
   tc_fence_before();
   __syncthreads();
-  tmem_free<Step<STEP>::COLS>(tmem, warp);
-}
-
-// ------------------------------------------------------------------------ backward: dQ
-template <int STEP>
-__global__ void __launch_bounds__(NT, Step<STEP>::CTAS)
-attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
-                   const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo, const Params p) {
-  constexpr int STEP_BYTES = Step<STEP>::BYTES, PANELS = Step<STEP>::PANELS;
-  extern __shared__ uint8_t raw[];
-  uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* sQ = base;
-  uint8_t* sdO = sQ + TILE_BYTES;
-  uint8_t* sdS = sdO + TILE_BYTES;           // panels of [128 queries][64 keys]
-  uint8_t* sK = sdS + PANELS * TILE_BYTES;   // two buffers each
-  uint8_t* sV = sK + 2 * STEP_BYTES;
-  Bars* bs = reinterpret_cast<Bars*>(sV + 2 * STEP_BYTES);
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int row = (warp & 3) * 32 + (tid & 31), cg = warp >> 2;
-  const int q0 = blockIdx.x * TILE, h = blockIdx.y, b = blockIdx.z;
-  const int nkv = p.S / STEP;
-
-  if (tid == 0) {
-    mbar_init(&bs->a, 1); mbar_init(&bs->c, 1); mbar_init(&bs->d, 1); mbar_init(&bs->drain, 1);
-    mbar_init(&bs->e[0], 1); mbar_init(&bs->e[1], 1);
-    bs->abort = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  tmem_alloc<Step<STEP>::COLS>(bs, warp);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = bs->tmem_base;
-  const uint32_t lane_addr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-  constexpr uint32_t COL_S = 0, COL_DQ = 2 * STEP;
-  bool ok = true;
-  const size_t stat = ((size_t)b * p.H + h) * p.S + q0 + row;
-  const float nlse = -p.lse[stat], ndelta = -p.delta[stat];
-
-  if (tid == 0) {
-    mbar_expect_tx(&bs->a, 2 * TILE_BYTES);
-    tma_load_4d(smem_u32(sQ), &tq, smem_u32(&bs->a), 0, h, q0, b);
-    tma_load_4d(smem_u32(sdO), &tdo, smem_u32(&bs->a), 0, h, q0, b);
-    mbar_expect_tx(&bs->e[0], 2 * STEP_BYTES);
-    tma_load_4d(smem_u32(sK), &tk, smem_u32(&bs->e[0]), 0, h, 0, b);
-    tma_load_4d(smem_u32(sV), &tv, smem_u32(&bs->e[0]), 0, h, 0, b);
-    ok = wait(bs, &bs->a, 0, p.error, 41);
-  }
-  for (int j = 0; j < nkv; j++) {
-    const int buf = j & 1;
-    uint8_t* kt = sK + buf * STEP_BYTES;
-    uint8_t* vt = sV + buf * STEP_BYTES;
-    if (tid == 0 && ok) {
-      ok = wait(bs, &bs->e[buf], (j >> 1) & 1, p.error, 43);                     // the order of the steps: as above
-      if (ok) {
-        tc_fence_after();
-        mma_kk(tmem + COL_S, smem_u32(sQ), smem_u32(kt), STEP, false);           // S  = Q_i K_j^T
-        mma_kk(tmem + COL_S + STEP, smem_u32(sdO), smem_u32(vt), STEP, false);   // dP = dO_i V_j^T
-        tc_commit(&bs->c);
-      }
-      if (ok && j + 1 < nkv) {
-        if (j >= 1) ok = wait(bs, &bs->d, (j - 1) & 1, p.error, 42);             // K of block j-1 is still read by its dQ MMAs
-        if (ok) {
-          mbar_expect_tx(&bs->e[buf ^ 1], 2 * STEP_BYTES);
-          tma_load_4d(smem_u32(sK + (buf ^ 1) * STEP_BYTES), &tk, smem_u32(&bs->e[buf ^ 1]), 0, h, (j + 1) * STEP, b);
-          tma_load_4d(smem_u32(sV + (buf ^ 1) * STEP_BYTES), &tv, smem_u32(&bs->e[buf ^ 1]), 0, h, (j + 1) * STEP, b);
-        }
-      }
-    }
-    ok = ok && wait(bs, &bs->c, j & 1, p.error, 44);
-    if (j >= 1) ok = ok && wait(bs, &bs->d, (j - 1) & 1, p.error, 45);           // dS of tile j-1 consumed
-    ok = __syncthreads_and(ok);
-    if (!ok) break;
-    tc_fence_after();
-    softmax_grad_tile<false, STEP>(lane_addr + COL_S, row, cg, &nlse, &ndelta, p, nullptr, sdS);
-    proxy_fence();
-    tc_fence_before();
-    __syncthreads();
-    if (tid == 0) {
-      tc_fence_after();
-      const uint32_t id = idesc_f16(D, false, true);                // A = dS (K-major), B = K_j as [key][d] (MN-major)
-#pragma unroll
-      for (int h = 0; h < PANELS; h++) {
-        const uint64_t da = smem_desc_sw128(smem_u32(sdS + h * TILE_BYTES)), db = smem_desc_mn_sw128(smem_u32(kt + h * 8192));
-#pragma unroll
-        for (int k = 0; k < 4; k++) tc_mma(tmem + COL_DQ, da + 2 * k, db + (2048 >> 4) * k, id, (j | h | k) != 0);
-      }
-      tc_commit(&bs->d);
-    }
-  }
-  ok = ok && wait(bs, &bs->d, (nkv - 1) & 1, p.error, 46);
-  ok = __syncthreads_and(ok);
-  if (ok) {
-    tc_fence_after();
-    const size_t orow = ((((size_t)b * p.S + q0 + row) * 3) * p.H + h) * D;
-    if (cg < 2) store_acc_row(lane_addr, COL_DQ, cg, p.dqkv + orow);
-  }
-  if (tid == 0) drain(bs);
-  tc_fence_before();
-  __syncthreads();
-  tmem_free<Step<STEP>::COLS>(tmem, warp);
+  if (warp == 0) tmem_free_all(tmem);
 }
 
 // ------------------------------------------------------------------------------ host side
 // One of Q / K / V inside qkv [B][S][3][H][64] (which = 0, 1, 2), or a plain [B][S][H][64] tensor (which = -1):
-// dims {d, h, s, b}, box = 64 x 1 x rows x 1 (that many rows of one head).
-static int make_map(CUtensorMap* map, const void* ptr, int B, int S, int H, int which, int rows) {
+// dims {d, h, s, b}, box = cols x 1 x rows x 1 (that many rows of one head); 32 columns in the 64-byte swizzle.
+static int make_map(CUtensorMap* map, const void* ptr, int B, int S, int H, int which, int rows, int cols = D) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return -10;
   const uint64_t row = (which >= 0 ? 3ull : 1ull) * H * D;          // elements between consecutive sequence positions
@@ -600,10 +774,10 @@ static int make_map(CUtensorMap* map, const void* ptr, int B, int S, int H, int 
   if ((uintptr_t)basep & 15) return -11;
   cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)S, (cuuint64_t)B};
   cuuint64_t strides[3] = {(cuuint64_t)D * 2, row * 2, row * 2 * (cuuint64_t)S};
-  cuuint32_t box[4] = {(cuuint32_t)D, 1, (cuuint32_t)rows, 1};
+  cuuint32_t box[4] = {(cuuint32_t)cols, 1, (cuuint32_t)rows, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<char*>(basep), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, cols == D ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     fprintf(stderr, "gcow attention: cuTensorMapEncodeTiled failed with CUresult %d (B %d S %d H %d which %d)\n", (int)r, B, S, H, which);
@@ -612,16 +786,24 @@ static int make_map(CUtensorMap* map, const void* ptr, int B, int S, int H, int 
   return 0;
 }
 
-constexpr size_t kFwdSmem = TILE_BYTES * 13 + sizeof(Bars) + 1024;      // Q + 4 K + 4 V + 4 P
-template <int STEP> constexpr size_t kBwdSmem =                            // K, V, P, dS, 2 Q, 2 dO, statistics
-    TILE_BYTES * (2 + 2 * Step<STEP>::PANELS) + Step<STEP>::BYTES * 4 + MAX_S * 8 + sizeof(Bars) + 1024;
-template <int STEP> constexpr size_t kDqSmem =                             // Q, dO, dS, 2 K, 2 V
-    TILE_BYTES * (2 + Step<STEP>::PANELS) + Step<STEP>::BYTES * 4 + sizeof(Bars) + 1024;
-static_assert(kBwdSmem<64> <= 112 * 1024 && kDqSmem<64> <= 112 * 1024, "two CTAs per SM");
-static_assert(kBwdSmem<128> <= 227 * 1024 && kDqSmem<128> <= 227 * 1024, "one CTA per SM");
+constexpr size_t kFwdSmem = TILE_BYTES * 12 + sizeof(FwdBars) + 1024;   // 2 Q, 2 O, 4 K, 4 V
+constexpr size_t kBwdSmem = TILE_BYTES * 13 + MAX_S * 16 + sizeof(BwdBars) + 1024;   // a1, a2 of both tiles, b1, b2, staging, statistics
+static_assert(kFwdSmem <= 227 * 1024 && kBwdSmem <= 227 * 1024, "one CTA per SM");
 
+// Two tiles per CTA share the sequence's operands, and each keeps the arithmetic units busy while the other one waits for a
+// product; where there are no more tiles than SMs each has an SM to itself.
+static int plan_units(int B, int S, int H, int* mode, int* units) {
+  const long long heads = (long long)B * H, tiles = (S + TILE - 1) / TILE;
+  *mode = heads * tiles <= 148 ? kSingle : tiles == 1 ? kHeads : kPair;
+  const long long n = *mode == kSingle ? heads * tiles : *mode == kHeads ? (heads + 1) / 2 : heads * ((tiles + 1) / 2);
+  if (n > 0x7fffffff) return -1;
+  *units = (int)n;
+  return 0;
+}
+
+// Up to 64 positions the 128-row tiles are mostly empty.
 static int check_shape(int B, int S, int H, int d) {
-  if (d != D || S % TILE || S <= 0 || S > MAX_S || B <= 0 || H <= 0 || H > 65535 || B > 65535) return -1;
+  if (d != D || S % 8 || S <= 64 || S > MAX_S || B <= 0 || H <= 0 || H > 65535 || B > 65535) return -1;
   return 0;
 }
 
@@ -629,30 +811,9 @@ static void set_attrs() {
   static std::once_flag once;
   std::call_once(once, [] {
     cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem);
-    cudaFuncSetAttribute(attn_bwd_dkdv_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwdSmem<64>);
-    cudaFuncSetAttribute(attn_bwd_dkdv_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwdSmem<128>);
-    cudaFuncSetAttribute(attn_bwd_dq_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDqSmem<64>);
-    cudaFuncSetAttribute(attn_bwd_dq_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDqSmem<128>);
+    cudaFuncSetAttribute(attn_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwdSmem);
+    cudaFuncSetAttribute(attn_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwdSmem);
   });
-}
-
-// The backward kernels; STEP as in Step.
-template <int STEP>
-static int launch_bwd(const void* qkv, const void* out, const void* dout, float* delta, const Params& p, cudaStream_t st) {
-  CUtensorMap tile[4], step[4];                              // Q, K, V, dO in boxes of TILE and of STEP rows
-  for (int i = 0; i < 4; i++) {
-    const void* const m = i < 3 ? qkv : dout;
-    int rc;
-    if ((rc = make_map(&tile[i], m, p.B, p.S, p.H, i < 3 ? i : -1, TILE))) return rc;
-    if (STEP == TILE) step[i] = tile[i];
-    else if ((rc = make_map(&step[i], m, p.B, p.S, p.H, i < 3 ? i : -1, STEP))) return rc;
-  }
-  const size_t rows = (size_t)p.B * p.S * p.H;
-  attn_delta_kernel<<<(unsigned)((rows * 8 + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, delta, p.B, p.S, p.H);
-  const dim3 grid(p.S / TILE, p.H, p.B);
-  attn_bwd_dkdv_kernel<STEP><<<grid, NT, kBwdSmem<STEP>, st>>>(step[0], tile[1], tile[2], step[3], p);
-  attn_bwd_dq_kernel<STEP><<<grid, NT, kDqSmem<STEP>, st>>>(tile[0], step[1], step[2], tile[3], p);
-  return (int)cudaGetLastError();
 }
 
 }  // namespace attn
@@ -662,7 +823,7 @@ using namespace gcow::attn;
 
 extern "C" {
 
-// 1 if the fused kernels cover this problem (head dimension 64, S a multiple of 128 up to 512).
+// 1 if the fused kernels cover this problem (head dimension 64, S a multiple of 8 from 72 to 512).
 int gcow_attention_supported(int B, int S, int H, int d) { return check_shape(B, S, H, d) == 0; }
 
 // out[B][S][H][64] = softmax(scale * Q K^T) V per head, qkv [B][S][3][H][64] bf16; lse [B][H][S] fp32 receives the
@@ -671,14 +832,16 @@ int gcow_attention_fwd(const void* qkv, void* out, float* lse, int B, int S, int
                        uint32_t* error, void* stream) {
   if (check_shape(B, S, H, d)) return -1;
   set_attrs();
-  CUtensorMap tq, tk, tv;
-  int rc;
-  if ((rc = make_map(&tq, qkv, B, S, H, 0, TILE)) || (rc = make_map(&tk, qkv, B, S, H, 1, TILE)) || (rc = make_map(&tv, qkv, B, S, H, 2, TILE)))
+  int mode, units, rc;
+  if (plan_units(B, S, H, &mode, &units)) return -1;
+  CUtensorMap tq, tk, tv, to;
+  if ((rc = make_map(&tq, qkv, B, S, H, 0, TILE)) || (rc = make_map(&tk, qkv, B, S, H, 1, TILE)) || (rc = make_map(&tv, qkv, B, S, H, 2, TILE)) ||
+      (rc = make_map(&to, out, B, S, H, -1, 32)))
     return rc;
   Params p = {};
-  p.out = (__nv_bfloat16*)out; p.lse = lse; p.B = B; p.S = S; p.H = H;
+  p.lse = lse; p.B = B; p.S = S; p.H = H;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.error = error;
-  attn_fwd_kernel<<<dim3(S / TILE, H, B), NT, kFwdSmem, (cudaStream_t)stream>>>(tq, tk, tv, p);
+  gcow::launch_dependent(attn_fwd_kernel, dim3(units < 148 ? units : 148), dim3(kThreads), kFwdSmem, (cudaStream_t)stream, tq, tk, tv, to, p, units, mode);
   return (int)cudaGetLastError();
 }
 
@@ -688,13 +851,22 @@ int gcow_attention_bwd(const void* qkv, const void* out, const void* dout, const
   if (check_shape(B, S, H, d)) return -1;
   set_attrs();
   cudaStream_t st = (cudaStream_t)stream;
+  int mode, units, rc;
+  if (plan_units(B, S, H, &mode, &units)) return -1;
+  CUtensorMap in[4], dq, dk, dv;                             // Q, K, V, dO
+  for (int i = 0; i < 4; i++)
+    if ((rc = make_map(&in[i], i < 3 ? qkv : dout, B, S, H, i < 3 ? i : -1, TILE))) return rc;
+  if ((rc = make_map(&dq, dqkv, B, S, H, 0, 32, 32)) || (rc = make_map(&dk, dqkv, B, S, H, 1, 32, 32)) || (rc = make_map(&dv, dqkv, B, S, H, 2, 32, 32)))
+    return rc;
   Params p = {};
-  p.lse = const_cast<float*>(lse); p.delta = delta; p.dqkv = (__nv_bfloat16*)dqkv; p.B = B; p.S = S; p.H = H;
+  p.lse = const_cast<float*>(lse); p.delta = delta; p.B = B; p.S = S; p.H = H;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.error = error;
-  // Two CTAs per SM hide one another's chain of steps, but only where there are more CTAs than SMs; with fewer, each has an SM
-  // to itself and half as many steps are the shorter chain. 512 positions, 128 CTAs: 38.6 us with steps of 64, 29.9 with 128;
-  // 192 CTAs: 48.4 and 55.4 (128 positions, 148 CTAs or fewer: 18.1 and 16.3).
-  return (long long)(S / TILE) * H * B <= 148 ? launch_bwd<128>(qkv, out, dout, delta, p, st) : launch_bwd<64>(qkv, out, dout, delta, p, st);
+  const size_t rows = (size_t)B * S * H;
+  attn_delta_kernel<<<(unsigned)((rows * 8 + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, delta, B, S, H);
+  const dim3 grid(units < 148 ? units : 148);
+  gcow::launch_dependent(attn_bwd_kernel<true>, grid, dim3(kThreads), kBwdSmem, st, in[1], in[2], in[0], in[3], dv, dk, p, units, mode);
+  gcow::launch_dependent(attn_bwd_kernel<false>, grid, dim3(kThreads), kBwdSmem, st, in[0], in[3], in[1], in[2], dq, dq, p, units, mode);
+  return (int)cudaGetLastError();
 }
 
 }  // extern "C"

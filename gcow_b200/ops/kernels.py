@@ -841,7 +841,7 @@ def bmm_bf16(a: torch.Tensor, b: torch.Tensor, *, a_t: bool = False, b_t: bool =
 
 
 def fused_attention_usable(qkv: torch.Tensor) -> bool:
-    """Head dimension 64 and a sequence length that is a multiple of 128, at most 512."""
+    """Head dimension 64 and a sequence length that is a multiple of 8, from 72 to 512."""
     if not (qkv.is_cuda and qkv.dim() == 5 and _have("gcow_attention_fwd")):
         return False
     B, S, three, H, D = qkv.shape
@@ -856,8 +856,8 @@ def fused_attention(qkv: torch.Tensor) -> torch.Tensor:
 
 def attention_mode() -> str:
     """GCOW_ATTENTION=lib sends self-attention to PyTorch's scaled_dot_product_attention (the comparison arm);
-    by default the own backend uses the fused tcgen05 kernels where they apply (head dimension 64, sequence a
-    multiple of 128 up to 512) and batched tcgen05 GEMMs with softmax kernels elsewhere."""
+    by default the own backend uses the fused tcgen05 kernels where they apply (head dimension 64, 72 to 512
+    positions) and batched tcgen05 GEMMs with softmax kernels elsewhere."""
     import os
     return os.environ.get("GCOW_ATTENTION", "own")
 

@@ -74,3 +74,45 @@ def test_attention(B, S, H):
     assert _rel(o, ref.detach()) < 2 ** -8
     for i in range(3):
         assert _rel(qkv.grad[:, :, i], r.grad[:, :, i]) < 2 ** -8
+
+
+@pytest.mark.parametrize("B,S,H", [(99, 128, 3), (331, 128, 1), (120, 384, 2), (80, 512, 2), (75, 256, 4)])
+def test_attention_with_several_units_per_cta(B, S, H):
+    """Two tiles per unit (of one head, of two heads, the last one alone) and more units than SMs."""
+    test_attention(B, S, H)
+
+
+@pytest.mark.parametrize("B,S,H", [(1, 72, 1), (3, 120, 1), (150, 120, 1), (2, 136, 3), (80, 192, 2), (40, 200, 3), (5, 320, 2), (60, 384 - 8, 1),
+                                   (70, 392, 2), (33, 504, 3)])
+def test_attention_of_sequences_that_end_inside_a_tile(B, S, H):
+    """Partial last blocks of keys and queries: of every kind of unit, an odd number of 64-row steps, a block of eight rows;
+    and what lies behind the last sequence is not used."""
+    from gcow_b200.ops import kernels as K
+    test_attention(B, S, H)
+    held = torch.full((B * S + 128, 3, H, 64), 7.0, device="cuda").bfloat16()
+    qkv = held[:B * S].view(B, S, 3, H, 64)
+    qkv.copy_(torch.randn(B, S, 3, H, 64, device="cuda"))
+    held[B * S:] = float("nan")
+    assert torch.isfinite(K.fused_attention(qkv)).all()
+
+
+@pytest.mark.parametrize("S", [256, 512])
+@pytest.mark.parametrize("order", [1, -1])
+def test_attention_when_the_row_maximum_moves_between_key_blocks(S, order):
+    """Keys that grow, or shrink, by a factor of four per 128 positions: the forward pass follows the row maximum by more than
+    the margin it allows itself, or never. Two roundings to bf16, as above."""
+    from gcow_b200.ops import kernels as K
+    torch.manual_seed(S)
+    qkv = torch.randn(5, S, 3, 2, 64, device="cuda")
+    grow = 4.0 ** (order * torch.arange(S // 128, device="cuda")).repeat_interleave(128)
+    qkv[:, :, 1] *= grow.view(1, S, 1, 1)
+    qkv = qkv.bfloat16().requires_grad_(True)
+    o = K.fused_attention(qkv)
+    go = torch.randn_like(o)
+    o.backward(go)
+    r = qkv.detach().double()
+    q, k, v = (r[:, :, i].permute(0, 2, 1, 3) for i in range(3))
+    w = torch.softmax(q @ k.transpose(-1, -2) / 8, -1)
+    assert _rel(o, (w @ v).permute(0, 2, 1, 3).reshape(5, S, 128)) < 2 ** -8
+    dv = w.transpose(-1, -2) @ go.double().view(5, S, 2, 64).permute(0, 2, 1, 3)
+    assert _rel(qkv.grad[:, :, 2], dv.permute(0, 2, 1, 3)) < 2 ** -8
