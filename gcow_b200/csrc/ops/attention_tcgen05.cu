@@ -158,6 +158,10 @@ template <bool FWD> struct Regs { static constexpr int ROW = FWD ? 208 : 184, IS
 static_assert(2 * Regs<true>::ROW + Regs<true>::ISSUE == 3 * kLaunchRegs && 2 * Regs<false>::ROW + Regs<false>::ISSUE == 3 * kLaunchRegs &&
               kThreads * kLaunchRegs <= 65536, "setmaxnreg.inc waits for registers that must exist");
 template <bool FWD> __device__ __forceinline__ void regs_row() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Regs<FWD>::ROW)); }
+// In step, both tiles want the exponential units at the same time and leave them idle at the same time: B starts this late.
+__device__ __forceinline__ void stagger(int x) {
+  if (x) for (const long long from = clock64(); clock64() - from < 1200;) {}
+}
 template <bool FWD> __device__ __forceinline__ void regs_issue() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Regs<FWD>::ISSUE)); }
 
 // ------------------------------------------------------------------------------ forward
@@ -241,7 +245,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
       for (int i = 0; i < kKvFree; i++) if ((issued >> i) & 1u) landed(&bs->bar[i], (landing >> i) & 1u);
     } else if (warp < 10) {                                  // ---- products, warp 8: of tile A, 9: of tile B
       const int x = warp - 8;
-      bool held = false;                                     // S has been written before
+      bool held = false, ahead = false;                      // S has been written before; this unit's first S has been issued
       const uint32_t id_qk = idesc_f16(TILE, false, false), id_pv = idesc_f16(D, false, true);
       const uint64_t dq = smem_desc_sw128(smem_u32(sQ + x * TILE_BYTES)), dk = smem_desc_sw128(smem_u32(sK)), dv = smem_desc_mn_sw128(smem_u32(sV));
       const bool apart = mode == kHeads;                     // each tile has its own keys
@@ -258,42 +262,43 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
             }
           continue;
         }
-        // step j: S of block j, then O of block j - 1
+        auto qk = [&](int j) {
+          const int i = apart ? x : j;
+          if (j == 0) wait(kQFull + x, 23);
+          wait(kKvFull + i, 24);
+          if (held) wait(kSFree + x, 25);
+          held = true;
+          if (!ok) return;
+          tc_fence_after();
+          const uint64_t db = dk + i * (uint64_t)(TILE_BYTES >> 4);
+          if (lane == 0) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) tc_mma(col_s(x), dq + 2 * k, db + 2 * k, id_qk, k != 0);
+            tc_commit(&bs->bar[kSFull + x]);
+            tc_commit(&bs->bar[kKvFree + i]);
+            if (j == blocks - 1) tc_commit(&bs->bar[kQFree + x]);
+          }
+          __syncwarp();
+        };
+        // step j: S of block j, then O of block j - 1; the next unit's first S comes before this one's last O
+        if (!ahead) qk(0);
+        ahead = u + 1 < u1 && (!x || unit_at(u + 1, mode, tiles, heads).both);
 #pragma unroll 1
-        for (int j = 0; j <= blocks && ok; j++) {
-          if (j < blocks) {
-            const int i = apart ? x : j;
-            if (j == 0) wait(kQFull + x, 23);
-            wait(kKvFull + i, 24);
-            if (held) wait(kSFree + x, 25);
-            held = true;
-            if (!ok) break;
-            tc_fence_after();
-            const uint64_t db = dk + i * (uint64_t)(TILE_BYTES >> 4);
-            if (lane == 0) {
+        for (int j = 1; j <= blocks && ok; j++) {
+          if (j < blocks || ahead) qk(j < blocks ? j : 0);
+          const int i = apart ? x : j - 1;
+          wait(kKvFull + 4 + i, 26);
+          wait(kPFull + x, 27);
+          if (!ok) break;
+          tc_fence_after();
+          const uint64_t db = dv + i * (uint64_t)(TILE_BYTES >> 4);
+          if (lane == 0) {
 #pragma unroll
-              for (int k = 0; k < 4; k++) tc_mma(col_s(x), dq + 2 * k, db + 2 * k, id_qk, k != 0);
-              tc_commit(&bs->bar[kSFull + x]);
-              tc_commit(&bs->bar[kKvFree + i]);
-              if (j == blocks - 1) tc_commit(&bs->bar[kQFree + x]);
-            }
-            __syncwarp();
+            for (int k = 0; k < 8; k++) tc_mma_ts(col_o(x), col_p(x) + 8 * k, db + (2048 >> 4) * k, id_pv, k != 0 || j != 1);
+            tc_commit(&bs->bar[kPv + x]);
+            tc_commit(&bs->bar[kKvFree + 4 + i]);
           }
-          if (j > 0) {
-            const int i = apart ? x : j - 1;
-            wait(kKvFull + 4 + i, 26);
-            wait(kPFull + x, 27);
-            if (!ok) break;
-            tc_fence_after();
-            const uint64_t db = dv + i * (uint64_t)(TILE_BYTES >> 4);
-            if (lane == 0) {
-#pragma unroll
-              for (int k = 0; k < 8; k++) tc_mma_ts(col_o(x), col_p(x) + 8 * k, db + (2048 >> 4) * k, id_pv, k != 0 || j != 1);
-              tc_commit(&bs->bar[kPv + x]);
-              tc_commit(&bs->bar[kKvFree + 4 + i]);
-            }
-            __syncwarp();
-          }
+          __syncwarp();
         }
       }
       if (lane == 0) drain(&bs->bar[kFwdDrain + x]);
@@ -310,6 +315,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     uint8_t* const stage = sO + warp * (32 * 128);           // the warp's 32 rows
     bool ok = true;
+    stagger(x);
     for (int u = u0; u < u1 && ok; u++) {
       const Unit un = unit_at(u, mode, tiles, heads);
       if (x == 1 && !un.both) continue;
