@@ -18,7 +18,7 @@
 //  delta = rowsum(dO * O) comes from a small elementwise kernel.
 //
 // One persistent CTA per SM with two tiles in flight, A and B, 128 threads each: while one waits for its product the other
-// one's exponentials run. A warp per tile issues its products, another one the TMA loads; whole
+// one's exponentials run. A warp per tile issues its products (two in the backward pass), another one the TMA loads; whole
 // sequences of the streamed operands (64 KB each) are held, and refilled for the next unit of work block by block as the
 // last product that reads a block completes.
 //
@@ -119,6 +119,11 @@ __device__ __forceinline__ Unit unit_at(int u, int mode, int tiles, int heads) {
 
 // The barriers of a CTA are numbered, and a role keeps the parities it waits for next in one word.
 //
+// B 32, S 512, 16 heads: forward 123 us with one tile in flight and the probabilities through shared memory, now 64 (0.54
+// PFLOP/s; the 134 M exponentials take 29 at 16 a clock and SM); backward 327, now 225 (delta 15, the rest 0.57 PFLOP/s;
+// 251 with one issuing warp per tile in the backward pass, 242 before dQ could start beside dK/dV). One sequence of 512:
+// backward 35 us, now 30.
+//
 // What the issuing warps do per product decides the pace. As code of one thread alone, with the descriptors worked out where
 // they are used, a step of four to eight MMAs took it 1500 cycles (forward, B 32, S 512, 16 heads: 131 us): every operand of
 // an MMA is a uniform register, which a divergent thread has to fill one by one. So the whole warp runs the loop, all its
@@ -153,16 +158,17 @@ __device__ __forceinline__ void tmem_free_all(uint32_t base) {
 // Two groups of 128 threads that work on a row each, and one whose warps issue the products and the loads. A row's
 // thread holds 128 scores and their 64 packed probabilities (backward: 64 scores, probabilities and gradients each), more than
 // a third of an SM's registers allows (168 a thread): it takes what the third group gives up.
-constexpr int kThreads = 384, kLaunchRegs = 168;
-template <bool FWD> struct Regs { static constexpr int ROW = FWD ? 208 : 184, ISSUE = FWD ? 88 : 136; };
-static_assert(2 * Regs<true>::ROW + Regs<true>::ISSUE == 3 * kLaunchRegs && 2 * Regs<false>::ROW + Regs<false>::ISSUE == 3 * kLaunchRegs &&
-              kThreads * kLaunchRegs <= 65536, "setmaxnreg.inc waits for registers that must exist");
-template <bool FWD> __device__ __forceinline__ void regs_row() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Regs<FWD>::ROW)); }
+// The backward pass has two groups of the latter, 512 threads of 128 registers.
+template <bool FWD> struct Shape {
+  static constexpr int THREADS = FWD ? 384 : 512, REGS = FWD ? 168 : 128, ROW = FWD ? 208 : 184, ISSUE = FWD ? 88 : 72;
+  static_assert(2 * ROW + (THREADS / 128 - 2) * ISSUE == THREADS / 128 * REGS && THREADS * REGS <= 65536, "setmaxnreg.inc waits for registers that must exist");
+};
 // In step, both tiles want the exponential units at the same time and leave them idle at the same time: B starts this late.
 __device__ __forceinline__ void stagger(int x) {
   if (x) for (const long long from = clock64(); clock64() - from < 1200;) {}
 }
-template <bool FWD> __device__ __forceinline__ void regs_issue() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Regs<FWD>::ISSUE)); }
+template <bool FWD> __device__ __forceinline__ void regs_issue() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Shape<FWD>::ISSUE)); }
+template <bool FWD> __device__ __forceinline__ void regs_row() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Shape<FWD>::ROW)); }
 
 // ------------------------------------------------------------------------------ forward
 constexpr float kRescale = 8.0f;            // log2 units by which a running maximum may be out of date
@@ -175,7 +181,7 @@ struct FwdBars {
   volatile uint32_t abort;
 };
 
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(Shape<true>::THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
                 const __grid_constant__ CUtensorMap to, const Params p, int units, int mode) {
   extern __shared__ uint8_t raw[];
@@ -432,6 +438,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
 // rows: 15 us, one thread per row took 24).
 __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ go,
                                   float* __restrict__ delta, int B, int S, int H) {
+  pdl_trigger();
+  pdl_wait();
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t i = t >> 3, rows = (size_t)B * S * H;                   // over b, s, h
   const int part = (int)(t & 7);
@@ -457,10 +465,10 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __n
 
 // ------------------------------------------------------------------------------ backward
 // Barriers, each for tile A and B, for the two operands of the sequence's four blocks, or for two units' statistics.
-enum BwdBar { kAFull = 0, kAFree = 2, kBFull = 4, kBFree = 12, kStatFull = 16, kStatFree = 18, kSAt = 20, kSGone = 22, kDpAt = 24, kDpGone = 26,
-              kReady = 28, kAcc = 30, kBwdBars = 32 };
+enum BwdBar { kAFull = 0, kAFree = 2, kBFull = 4, kBFree = 12, kStatFull = 16, kStatFree = 18, kSAt = 20, kSGone = 22, kDpAt = 24,
+              kReady = 26, kAcc = 28, kBwdBars = 30 };
 struct BwdBars {
-  uint64_t bar[kBwdBars], drain[2];
+  uint64_t bar[kBwdBars], drain[4];
   uint32_t tmem_base;
   volatile uint32_t abort;
 };
@@ -469,7 +477,7 @@ struct BwdBars {
 // KV = false: a tile is 128 queries, the loop runs over blocks of 64 keys: S = Q K^T, dP = dO V^T, dQ += dS K.
 // a1, a2: the tile's operands (K, V or Q, dO); b1, b2: those of the whole sequence (Q, dO or K, V); to1, to2: dV, dK or -, dQ.
 template <bool KV>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(Shape<false>::THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__ CUtensorMap ta2, const __grid_constant__ CUtensorMap tb1,
                 const __grid_constant__ CUtensorMap tb2, const __grid_constant__ CUtensorMap to1, const __grid_constant__ CUtensorMap to2,
                 const Params p, int units, int mode) {
@@ -489,13 +497,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
 
   if (tid == 0) {
     // 4: the warps of a tile, 8: all row warps, 32: the warp that fetches statistics; a sequence that two tiles share is free
-    // when both have used it
+    // when both have used it, a tile's operands when each warp that reads them has
     for (int i = 0; i < kBwdBars; i++) {
       const int pair = i & ~1;
-      mbar_init(&bs->bar[i], pair == kSGone || pair == kDpGone || pair == kReady ? 4 : pair == kStatFree ? 8 : pair == kStatFull ? 32
-                             : i >= kBFree && i < kStatFull && mode == kPair ? 2 : 1);
+      mbar_init(&bs->bar[i], pair == kSGone || pair == kReady ? 4 : pair == kStatFree ? 8 : pair == kStatFull ? 32
+                             : (KV && pair == kAFree) || (i >= kBFree && i < kStatFull && mode == kPair) ? 2 : 1);
     }
-    mbar_init(&bs->drain[0], 1); mbar_init(&bs->drain[1], 1);
+    for (int i = 0; i < 4; i++) mbar_init(&bs->drain[i], 1);
     bs->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -504,8 +512,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bs->tmem_base;
+  // The two kernels read the same and write apart, so dQ need not wait for dK/dV: that one lets it start when what both read is
+  // there. A grid that leaves SMs idle, and the end of every grid, is filled so. dQ ends only after dK/dV, for what follows it.
+  if (KV) pdl_wait();
   pdl_trigger();
-  pdl_wait();
   // Columns of a tile: S 64, dP 64, two accumulators of 64. P and dS (32 each, bf16) take dP's place once it has been read; with
   // one accumulator dS has a place of its own, and dP can be refilled at once.
   auto col = [&](int x) { return tmem + x * 256; };
@@ -518,7 +528,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
     auto wait = [&](int i, uint32_t code) {
       ok = __all_sync(0xffffffffu, mbar_wait_abortable(&bs->abort, &bs->bar[i], ph.next(i), p.error, code)) && ok;
     };
-    if (warp == 10) {                                        // ---- loads
+    if (warp == 12) {                                        // ---- loads
       uint32_t issued = 0, landing = 0;                      // by barrier: a copy has been issued; the parity after it
       for (int u = u0; u < u1 && ok; u++) {
         const Unit un = unit_at(u, mode, tiles, heads);
@@ -548,84 +558,97 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
       // nothing may be in flight when the CTA ends (there is something to wait for only after a wait gave up)
 #pragma unroll 1
       for (int i = 0; i < kBFree; i++) if ((i < kAFree || i >= kBFull) && ((issued >> i) & 1u)) landed(&bs->bar[i], (landing >> i) & 1u);
-    } else if (warp < 10) {                                  // ---- products, warp 8: of tile A, 9: of tile B
-      const int x = warp - 8;
-      bool s_held = false, dp_held = false;                  // S, dP has been written before
+    } else if (warp < 12) {
+      // ---- products: warps 8, 9 issue S (with dP, where that has a place of its own) of tiles A, B, warps 10, 11 the accumulators
+      // (and dP, where it takes the place of what they have read)
+      const int x = warp & 1;
+      const bool scores = warp < 10, apart = mode == kHeads; // apart: each tile has its own sequence
       const uint32_t id_s = idesc_f16(STEP, false, false), id_acc = idesc_f16(D, false, true), tm = col(x);
       const uint64_t da1 = smem_desc_sw128(smem_u32(sA + 2 * x * TILE_BYTES)), da2 = smem_desc_sw128(smem_u32(sA + (2 * x + 1) * TILE_BYTES));
-      const bool apart = mode == kHeads;                     // each tile has its own sequence
       const int first = apart ? x * TILE_BYTES : 0;
       const uint64_t db1 = smem_desc_sw128(smem_u32(sB1 + first)), db2 = smem_desc_sw128(smem_u32(sB2 + first));
       const uint64_t dm1 = smem_desc_mn_sw128(smem_u32(sB1 + first)), dm2 = smem_desc_mn_sw128(smem_u32(sB2 + first));
+      constexpr uint64_t kStep = STEP_BYTES >> 4;
+      bool held = false;                                     // S has been written before
       for (int u = u0; u < u1 && ok; u++) {
         const Unit un = unit_at(u, mode, tiles, heads);
         if (x && !un.both) {                                 // nothing to do but to let go of what the other tile is given
-          if (mode == kPair)
+          if (mode == kPair && (scores || KV))
 #pragma unroll 1
-            for (int i = 0; i < tiles && ok; i++) {
-              wait(kBFull + i, 32);
-              wait(kBFull + 4 + i, 32);
-              if (ok && lane == 0) mbar_arrive(&bs->bar[kBFree + i]);
-              __syncwarp();
+            for (int i = 0; i < tiles && ok; i++) {          // each warp waits for what it waits for in the other units
+              if (scores) wait(kBFull + i, 32);
+              if (scores != KV) {
+                wait(kBFull + 4 + i, 32);
+                if (ok && lane == 0) mbar_arrive(&bs->bar[kBFree + i]);
+                __syncwarp();
+              }
             }
           continue;
         }
-        // Round i: S of block i (and dP, where that has a place of its own), then the accumulators of block i - 1 (and dP of
-        // block i, which takes the place of what they have read).
-        auto dp_mma = [&](int i) {
-          const uint64_t db = db2 + i * (uint64_t)(STEP_BYTES >> 4);
-          if (!(i & 1)) wait(kBFull + 4 + (apart ? x : i >> 1), 36);
-          if (!KV && dp_held) wait(kDpGone + x, 37);
-          dp_held = true;
-          if (!ok) return;
-          tc_fence_after();
-          if (lane == 0) {
-#pragma unroll
-            for (int k = 0; k < 4; k++) tc_mma(tm + DP, da2 + 2 * k, db + 2 * k, id_s, k != 0);
-            tc_commit(&bs->bar[kDpAt + x]);
-            if (i == nb - 1) tc_commit(&bs->bar[kAFree + x]);
-          }
-          __syncwarp();
-        };
+        if (scores) {
 #pragma unroll 1
-        for (int i = 0; i <= nb && ok; i++) {
-          if (i < nb) {
-            const uint64_t db = db1 + i * (uint64_t)(STEP_BYTES >> 4);
+          for (int i = 0; i < nb && ok; i++) {
+            const int sl = apart ? x : i >> 1;
             if (i == 0) wait(kAFull + x, 33);
-            if (!(i & 1)) wait(kBFull + (apart ? x : i >> 1), 34);
-            if (s_held) wait(kSGone + x, 35);
-            s_held = true;
-            if (!ok) break;
-            tc_fence_after();
-            if (lane == 0) {
-#pragma unroll
-              for (int k = 0; k < 4; k++) tc_mma(tm, da1 + 2 * k, db + 2 * k, id_s, k != 0);
-              tc_commit(&bs->bar[kSAt + x]);
+            if (!(i & 1)) {
+              wait(kBFull + sl, 34);
+              if (!KV) wait(kBFull + 4 + sl, 34);
             }
-            __syncwarp();
-            if (!KV) dp_mma(i);
-          }
-          if (i > 0) {
-            const uint64_t off = (i - 1) * (uint64_t)(STEP_BYTES >> 4), d1 = dm1 + off, d2 = dm2 + off;
-            wait(kReady + x, 38);
+            if (held) wait(kSGone + x, 35);
+            held = true;
             if (!ok) break;
             tc_fence_after();
+            const uint64_t b1 = db1 + i * kStep, b2 = db2 + i * kStep;
             if (lane == 0) {
 #pragma unroll
               for (int k = 0; k < 4; k++) {
-                if (KV) tc_mma_ts(tm + ACC1, tm + P_AT + 8 * k, d2 + (2048 >> 4) * k, id_acc, k != 0 || i != 1);
-                tc_mma_ts(tm + ACC2, tm + DS_AT + 8 * k, d1 + (2048 >> 4) * k, id_acc, k != 0 || i != 1);
+                tc_mma(tm, da1 + 2 * k, b1 + 2 * k, id_s, k != 0);
+                if (!KV) tc_mma(tm + DP, da2 + 2 * k, b2 + 2 * k, id_s, k != 0);
               }
-              tc_commit(&bs->bar[kAcc + x]);
-              if (!(i & 1) || i == nb) tc_commit(&bs->bar[kBFree + (apart ? x : (i - 1) >> 1)]);
+              tc_commit(&bs->bar[kSAt + x]);
+              if (i == nb - 1) tc_commit(&bs->bar[kAFree + x]);
             }
             __syncwarp();
           }
-          if (KV && i < nb) dp_mma(i);
+        } else {
+          if (KV) wait(kAFull + x, 36);
+#pragma unroll 1
+          for (int i = 0; i <= nb && ok; i++) {
+            const int sl = apart ? x : i >> 1;
+            if (i > 0) {
+              const uint64_t b1 = dm1 + (i - 1) * kStep, b2 = dm2 + (i - 1) * kStep;
+              wait(kReady + x, 37);
+              if (!ok) break;
+              tc_fence_after();
+              if (lane == 0) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                  if (KV) tc_mma_ts(tm + ACC1, tm + P_AT + 8 * k, b2 + (2048 >> 4) * k, id_acc, k != 0 || i != 1);
+                  tc_mma_ts(tm + ACC2, tm + DS_AT + 8 * k, b1 + (2048 >> 4) * k, id_acc, k != 0 || i != 1);
+                }
+                tc_commit(&bs->bar[kAcc + x]);
+                if (!(i & 1) || i == nb) tc_commit(&bs->bar[kBFree + (apart ? x : (i - 1) >> 1)]);
+              }
+              __syncwarp();
+            }
+            if (KV && i < nb) {
+              if (!(i & 1)) wait(kBFull + 4 + sl, 38);
+              if (!ok) break;
+              tc_fence_after();
+              const uint64_t b2 = db2 + i * kStep;
+              if (lane == 0) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) tc_mma(tm + DP, da2 + 2 * k, b2 + 2 * k, id_s, k != 0);
+                tc_commit(&bs->bar[kDpAt + x]);
+                if (i == nb - 1) tc_commit(&bs->bar[kAFree + x]);
+              }
+              __syncwarp();
+            }
+          }
         }
       }
-      if (lane == 0) drain(&bs->drain[x]);
-    } else if (KV && warp == 11) {                           // ---- statistics of the queries
+      if (lane == 0) drain(&bs->drain[warp - 8]);
+    } else if (KV && warp == 13) {                           // ---- statistics of the queries
       for (int u = u0, n = 0; u < u1 && ok; u++, n++) {
         const Unit un = unit_at(u, mode, tiles, heads);
         if (n >= 2) wait(kStatFree + (n & 1), 39);
@@ -654,6 +677,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     uint8_t* const stage = sO + warp * kStageWarpBytes;
     bool ok = true;
+    stagger(x);
     const uint64_t sl = tc::pack2(p.scale_log2, p.scale_log2), sc = tc::pack2(p.scale, p.scale);
     for (int u = u0, n = 0; u < u1 && ok; u++, n++) {
       const Unit un = unit_at(u, mode, tiles, heads);
@@ -671,9 +695,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
         for (int i = 0; i < nb; i++) {
           if (!(ok = wait_all(kSAt + x, 41))) break;
           tc_fence_after();
-          uint32_t s[2][32];
+          uint32_t s[2][32], dp[2][32];
           tc_ld32(col(x) + lanes, s[0]);
           tc_ld32(col(x) + lanes + 32, s[1]);
+          if (!KV) {                                         // dP comes with S
+            tc_ld32(col(x) + DP + lanes, dp[0]);
+            tc_ld32(col(x) + DP + lanes + 32, dp[1]);
+          }
           tc_wait_ld();
           tc_fence_before();
           __syncwarp();
@@ -699,15 +727,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
                 pk[c * 16 + e / 2 + 1] = pack2(o[2], o[3]);
               }
             }
-          if (!(ok = wait_all(kDpAt + x, 42))) break;
-          tc_fence_after();
-          tc_ld32(col(x) + DP + lanes, s[0]);
-          tc_ld32(col(x) + DP + lanes + 32, s[1]);
-          tc_wait_ld();
-          if (!KV) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bs->bar[kDpGone + x]);
+          if (KV) {
+            if (!(ok = wait_all(kDpAt + x, 42))) break;
+            tc_fence_after();
+            tc_ld32(col(x) + DP + lanes, dp[0]);
+            tc_ld32(col(x) + DP + lanes + 32, dp[1]);
+            tc_wait_ld();
           }
 #pragma unroll
           for (int c = 0; c < 2; c++)
@@ -720,9 +745,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
               }
               const float* const o = pv + c * 32 + e;
               float a, b;
-              unpack2(mul2(mul2(tc::pack2(o[0], o[1]), add2(tc::pack2(__uint_as_float(s[c][e]), __uint_as_float(s[c][e + 1])), d0)), sc), a, b);
+              unpack2(mul2(mul2(tc::pack2(o[0], o[1]), add2(tc::pack2(__uint_as_float(dp[c][e]), __uint_as_float(dp[c][e + 1])), d0)), sc), a, b);
               dk[c * 16 + e / 2] = pack2(a, b);
-              unpack2(mul2(mul2(tc::pack2(o[2], o[3]), add2(tc::pack2(__uint_as_float(s[c][e + 2]), __uint_as_float(s[c][e + 3])), d1)), sc), a, b);
+              unpack2(mul2(mul2(tc::pack2(o[2], o[3]), add2(tc::pack2(__uint_as_float(dp[c][e + 2]), __uint_as_float(dp[c][e + 3])), d1)), sc), a, b);
               dk[c * 16 + e / 2 + 1] = pack2(a, b);
             }
           if (i) {                                           // the last block's P and dS have been read
@@ -767,6 +792,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_free_all(tmem);
+  if (!KV) pdl_wait();
 }
 
 // ------------------------------------------------------------------------------ host side
@@ -797,10 +823,10 @@ constexpr size_t kBwdSmem = TILE_BYTES * 13 + MAX_S * 16 + sizeof(BwdBars) + 102
 static_assert(kFwdSmem <= 227 * 1024 && kBwdSmem <= 227 * 1024, "one CTA per SM");
 
 // Two tiles per CTA share the sequence's operands, and each keeps the arithmetic units busy while the other one waits for a
-// product; where there are no more tiles than SMs each has an SM to itself.
-static int plan_units(int B, int S, int H, int* mode, int* units) {
+// product; where there are no more tiles than SMs (two kernels share them in the backward pass) each has an SM to itself.
+static int plan_units(int B, int S, int H, int sms, int* mode, int* units) {
   const long long heads = (long long)B * H, tiles = (S + TILE - 1) / TILE;
-  *mode = heads * tiles <= 148 ? kSingle : tiles == 1 ? kHeads : kPair;
+  *mode = heads * tiles <= sms ? kSingle : tiles == 1 ? kHeads : kPair;
   const long long n = *mode == kSingle ? heads * tiles : *mode == kHeads ? (heads + 1) / 2 : heads * ((tiles + 1) / 2);
   if (n > 0x7fffffff) return -1;
   *units = (int)n;
@@ -839,7 +865,7 @@ int gcow_attention_fwd(const void* qkv, void* out, float* lse, int B, int S, int
   if (check_shape(B, S, H, d)) return -1;
   set_attrs();
   int mode, units, rc;
-  if (plan_units(B, S, H, &mode, &units)) return -1;
+  if (plan_units(B, S, H, 148, &mode, &units)) return -1;
   CUtensorMap tq, tk, tv, to;
   if ((rc = make_map(&tq, qkv, B, S, H, 0, TILE)) || (rc = make_map(&tk, qkv, B, S, H, 1, TILE)) || (rc = make_map(&tv, qkv, B, S, H, 2, TILE)) ||
       (rc = make_map(&to, out, B, S, H, -1, 32)))
@@ -847,7 +873,7 @@ int gcow_attention_fwd(const void* qkv, void* out, float* lse, int B, int S, int
   Params p = {};
   p.lse = lse; p.B = B; p.S = S; p.H = H;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.error = error;
-  gcow::launch_dependent(attn_fwd_kernel, dim3(units < 148 ? units : 148), dim3(kThreads), kFwdSmem, (cudaStream_t)stream, tq, tk, tv, to, p, units, mode);
+  gcow::launch_dependent(attn_fwd_kernel, dim3(units < 148 ? units : 148), dim3(Shape<true>::THREADS), kFwdSmem, (cudaStream_t)stream, tq, tk, tv, to, p, units, mode);
   return (int)cudaGetLastError();
 }
 
@@ -858,7 +884,7 @@ int gcow_attention_bwd(const void* qkv, const void* out, const void* dout, const
   set_attrs();
   cudaStream_t st = (cudaStream_t)stream;
   int mode, units, rc;
-  if (plan_units(B, S, H, &mode, &units)) return -1;
+  if (plan_units(B, S, H, 148 / 2, &mode, &units)) return -1;
   CUtensorMap in[4], dq, dk, dv;                             // Q, K, V, dO
   for (int i = 0; i < 4; i++)
     if ((rc = make_map(&in[i], i < 3 ? qkv : dout, B, S, H, i < 3 ? i : -1, TILE))) return rc;
@@ -868,10 +894,10 @@ int gcow_attention_bwd(const void* qkv, const void* out, const void* dout, const
   p.lse = const_cast<float*>(lse); p.delta = delta; p.B = B; p.S = S; p.H = H;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.error = error;
   const size_t rows = (size_t)B * S * H;
-  attn_delta_kernel<<<(unsigned)((rows * 8 + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, delta, B, S, H);
+  gcow::launch_dependent(attn_delta_kernel, dim3((unsigned)((rows * 8 + 255) / 256)), dim3(256), 0, st, (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, delta, B, S, H);
   const dim3 grid(units < 148 ? units : 148);
-  gcow::launch_dependent(attn_bwd_kernel<true>, grid, dim3(kThreads), kBwdSmem, st, in[1], in[2], in[0], in[3], dv, dk, p, units, mode);
-  gcow::launch_dependent(attn_bwd_kernel<false>, grid, dim3(kThreads), kBwdSmem, st, in[0], in[3], in[1], in[2], dq, dq, p, units, mode);
+  gcow::launch_dependent(attn_bwd_kernel<true>, grid, dim3(Shape<false>::THREADS), kBwdSmem, st, in[1], in[2], in[0], in[3], dv, dk, p, units, mode);
+  gcow::launch_dependent(attn_bwd_kernel<false>, grid, dim3(Shape<false>::THREADS), kBwdSmem, st, in[0], in[3], in[1], in[2], dq, dq, p, units, mode);
   return (int)cudaGetLastError();
 }
 
