@@ -34,19 +34,40 @@ constexpr int CHUNK_BYTES = 128 * 64 * 2;             // 128 rows x 128 bytes
 constexpr int OPER_BYTES = 2 * CHUNK_BYTES;           // one CTA's half of an operand, one stage
 constexpr int STAGE_BYTES = 2 * OPER_BYTES;           // 64 KB
 constexpr int STAGES = 3;
-constexpr int EPI_WARPS = 8, THREADS = 64 + 32 * EPI_WARPS;
+// Epilogue warps: eight, or sixteen for a GELU, whose arithmetic two warps per scheduler leave half of the issue slots to
+// (bias, GELU and its argument kept: 16384 x 4096 x 1024 142 -> 129 us, x 3072 110 -> 97, x 1024 44 -> 36; with a residual
+// sixteen are slower, 144 and 156, and plain 95 and 98).
+template <bool WIDE> struct Epilogue { static constexpr int WARPS = WIDE ? 16 : 8, THREADS = 64 + 32 * WARPS; };
 constexpr uint32_t TMEM_COLS = 512;
 
-enum Flags : int { kBias = 2, kGelu = 4, kResidual = 8, kAuxOut = 32, kGeluGrad = 64 };
+enum Flags : int { kOutF32 = 1, kBias = 2, kGelu = 4, kResidual = 8, kAuxOut = 32, kGeluGrad = 64 };
 
 struct Params {
-  __nv_bfloat16* C;
+  __nv_bfloat16* C;        // float* with kOutF32
   const float* bias;
   const __nv_bfloat16* residual;
   __nv_bfloat16* aux;
   int M, N, K, ldc, flags;
+  int whole, items;        // items of work: `whole` 256 x 256 tiles (of every slice), then halves of 256 x 128
+  int slice_blocks;        // stages per slice of the reduction
+  size_t slice_stride;     // elements from one slice's result to the next
   uint32_t* error;
 };
+
+// An item of work: a tile, or the left or right half of one, over a slice of the reduction.
+struct Item { int m0, n0, kb0, kb1, slice; bool half; };
+template <bool SLICES> __device__ __forceinline__ Item item_at(const Params& p, int i, int tiles_m, int tiles, int kblocks) {
+  Item r;
+  r.half = i >= p.whole;
+  const int j = r.half ? (i - p.whole) >> 1 : i;
+  r.slice = SLICES ? j / tiles : 0;
+  const int tile = r.half ? p.whole + j : j - r.slice * tiles;
+  r.m0 = (tile % tiles_m) * BM;
+  r.n0 = (tile / tiles_m) * BN + (r.half ? ((i - p.whole) & 1) * (BN / 2) : 0);
+  r.kb0 = SLICES ? r.slice * p.slice_blocks : 0;
+  r.kb1 = SLICES && r.kb0 + p.slice_blocks < kblocks ? r.kb0 + p.slice_blocks : kblocks;
+  return r;
+}
 
 struct Smem {
   uint64_t full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], drain;
@@ -97,21 +118,24 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128_16k(uint32_t saddr) {
   return d;
 }
 
-// B_MN: B is stored [K][N] (the data-gradient product dX = dY * W reads the weight matrix in place). SIDE: the epilogue reads
+// B_MN: B is stored [K][N] (the data-gradient product dX = dY * W reads the weight matrix in place); A_MN: A is stored [K][M]
+// (with B_MN the weight gradient, which reads both in place). SIDE: the epilogue reads
 // a residual or the argument of a GELU' factor.
-template <bool B_MN, bool SIDE>
-__global__ void __launch_bounds__(THREADS, 1)
-gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const Params p) {
+template <bool A_MN, bool B_MN, bool SIDE, bool WIDE>
+__global__ void __launch_bounds__(Epilogue<WIDE>::THREADS, 1)
+gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                  const __grid_constant__ CUtensorMap tmap_bh, const Params p) {
+  constexpr int EPI_WARPS = Epilogue<WIDE>::WARPS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   Smem* sm = reinterpret_cast<Smem*>(base + STAGES * STAGE_BYTES);
   uint8_t* stage_base = reinterpret_cast<uint8_t*>(((uintptr_t)(sm + 1) + 15) & ~(uintptr_t)15);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp: uniform
   const uint32_t rank = cluster_rank();               // 0: issues the MMAs and owns full / tmem_empty
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int tiles_m = (p.M + BM - 1) / BM, tiles_n = (p.N + BN - 1) / BN;
-  const int num_tiles = tiles_m * tiles_n;
+  const int tiles = tiles_m * tiles_n;
   const int kblocks = (p.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
@@ -140,16 +164,19 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     if (lane == 0) {
       uint32_t s = 0, phase = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += pairs) {
-        const int m0 = (tile % tiles_m) * BM + (int)rank * 128, n0 = (tile / tiles_m) * BN + (int)rank * 128;
-        for (int kb = 0; kb < kblocks; kb++) {
+      for (int i = pair; i < p.items && ok; i += pairs) {
+        const Item it = item_at<A_MN>(p, i, tiles_m, tiles, kblocks);
+        const int m0 = it.m0 + (int)rank * 128, n0 = it.n0 + (int)rank * (it.half ? 64 : 128);
+        const CUtensorMap* const map_b = it.half ? &tmap_bh : &tmap_b;
+        for (int kb = it.kb0; kb < it.kb1; kb++) {
           if (!(ok = mbar_wait_abortable(&sm->abort, &sm->empty[s], phase ^ 1, p.error, 1))) break;
-          if (rank == 0) mbar_expect_tx(&sm->full[s], 2 * STAGE_BYTES);
+          if (rank == 0) mbar_expect_tx(&sm->full[s], 2 * (it.half ? OPER_BYTES + OPER_BYTES / 2 : STAGE_BYTES));
           const uint32_t bar = map_to_cta(smem_u32(&sm->full[s]), 0);
           uint8_t* st = base + s * STAGE_BYTES;
-          tma_load_3d_pair(smem_u32(st), &tmap_a, bar, 0, m0, kb * 2);
-          if (B_MN) tma_load_3d_pair(smem_u32(st + OPER_BYTES), &tmap_b, bar, 0, kb * BK, n0 / 64);
-          else tma_load_3d_pair(smem_u32(st + OPER_BYTES), &tmap_b, bar, 0, n0, kb * 2);
+          if (A_MN) tma_load_3d_pair(smem_u32(st), &tmap_a, bar, 0, kb * BK, m0 / 64);
+          else tma_load_3d_pair(smem_u32(st), &tmap_a, bar, 0, m0, kb * 2);
+          if (B_MN) tma_load_3d_pair(smem_u32(st + OPER_BYTES), map_b, bar, 0, kb * BK, n0 / 64);
+          else tma_load_3d_pair(smem_u32(st + OPER_BYTES), map_b, bar, 0, n0, kb * 2);
           if (++s == STAGES) { s = 0; phase ^= 1; }
         }
       }
@@ -160,65 +187,78 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer (CTA 0 only)
-    if (lane == 0 && rank == 0) {
-      // instruction descriptor: fp32 accumulate, bf16 x bf16, K-major operands, N 256, M 256 (128 rows per CTA)
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)B_MN << 16) | ((uint32_t)(BN >> 3) << 17) |
-                             ((uint32_t)(BM >> 4) << 24);
+    if (rank == 0) {                                    // the warp keeps together, so that every operand is uniform; one lane issues
+      // instruction descriptor: fp32 accumulate, bf16 x bf16, operand major-ness, M 256 (128 rows per CTA), N 256 or 128
+      const uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)A_MN << 15) | ((uint32_t)B_MN << 16) | ((uint32_t)(BM >> 4) << 24);
       uint32_t s = 0, phase = 0, t = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += pairs, t++) {
+      auto wait = [&](uint64_t* bar, uint32_t parity, uint32_t code) {
+        return __all_sync(0xffffffffu, mbar_wait_abortable(&sm->abort, bar, parity, p.error, code)) != 0;
+      };
+      for (int i = pair; i < p.items && ok; i += pairs, t++) {
+        const Item it = item_at<A_MN>(p, i, tiles_m, tiles, kblocks);
+        const uint32_t idesc = idesc0 | ((uint32_t)((it.half ? BN / 2 : BN) >> 3) << 17), chunk_b = it.half ? CHUNK_BYTES / 2 : CHUNK_BYTES;
         const uint32_t acc = t & 1, aphase = (t >> 1) & 1;
-        if (!(ok = mbar_wait_abortable(&sm->abort, &sm->tmem_empty[acc], aphase ^ 1, p.error, 2))) break;
+        if (!(ok = wait(&sm->tmem_empty[acc], aphase ^ 1, 2))) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < kblocks; kb++) {
-          if (!(ok = mbar_wait_abortable(&sm->abort, &sm->full[s], phase, p.error, 3))) break;
+        for (int kb = it.kb0; kb < it.kb1; kb++) {
+          if (!(ok = wait(&sm->full[s], phase, 3))) break;
           tc_fence_after();
           const uint32_t sa = smem_u32(base + s * STAGE_BYTES), sb = sa + OPER_BYTES;
+          const uint32_t eb0 = map_to_cta(smem_u32(&sm->empty[s]), 0), eb1 = map_to_cta(smem_u32(&sm->empty[s]), 1);
+          if (lane == 0) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; k++) {
-            const uint32_t off = (k >> 2) * CHUNK_BYTES + (k & 3) * 32;     // 64-wide chunk, then 32 bytes per K step
-            // MN-major B: 16 K-rows of 128 bytes per step, 128 rows contiguous within a column group
-            const uint64_t db = B_MN ? smem_desc_mn_sw128_16k(sb + k * 2048) : smem_desc_sw128(sb + off);
-            tc_mma_pair(d_tmem, smem_desc_sw128(sa + off), db, idesc, (kb | k) != 0);
+            for (int k = 0; k < BK / UMMA_K; k++) {
+              const uint32_t in = (k & 3) * 32;                               // 64-wide chunk, then 32 bytes per K step
+              // MN-major: 16 K-rows of 128 bytes per step, 128 rows contiguous within a column group
+              const uint64_t da = A_MN ? smem_desc_mn_sw128_16k(sa + k * 2048) : smem_desc_sw128(sa + (k >> 2) * CHUNK_BYTES + in);
+              const uint64_t db = B_MN ? smem_desc_mn_sw128_16k(sb + k * 2048) : smem_desc_sw128(sb + (k >> 2) * chunk_b + in);
+              tc_mma_pair(d_tmem, da, db, idesc, kb != it.kb0 || k);
+            }
+            tc_commit_pair(eb0);
+            tc_commit_pair(eb1);
           }
-          const uint32_t eb = smem_u32(&sm->empty[s]);
-          tc_commit_pair(map_to_cta(eb, 0));
-          tc_commit_pair(map_to_cta(eb, 1));
+          __syncwarp();
           if (++s == STAGES) { s = 0; phase ^= 1; }
         }
-        if (ok) {
+        if (ok && lane == 0) {
           const uint32_t fb = smem_u32(&sm->tmem_full[acc]);
           tc_commit_pair(map_to_cta(fb, 0));
           tc_commit_pair(map_to_cta(fb, 1));
         }
+        __syncwarp();
       }
       // drain: everything issued by this thread has finished before tensor memory is freed
-      tc_commit_pair(map_to_cta(smem_u32(&sm->drain), 0));
-      for (uint32_t it = 0; it < kSpinLimit; it++) if (mbar_try_wait(&sm->drain, 0)) break;
+      if (lane == 0) {
+        tc_commit_pair(map_to_cta(smem_u32(&sm->drain), 0));
+        for (uint32_t it = 0; it < kSpinLimit; it++) if (mbar_try_wait(&sm->drain, 0)) break;
+      }
     }
   } else {
     // ----------------------------------------------------------------- epilogue (both CTAs, own 128 rows)
     const int q = warp & 3, ew = warp - 2;
-    constexpr int COLS = BN / (EPI_WARPS / 4);
-    constexpr int NCH = COLS / 32;
-    const int col0 = (ew / 4) * COLS;
+    constexpr int GROUPS = EPI_WARPS / 4;               // of columns
+    const bool wide_bias = ((uintptr_t)p.bias & 15) == 0;
     [[maybe_unused]] const __nv_bfloat16* const ahead = p.flags & kGeluGrad ? p.aux : p.residual;
     uint8_t* stg = stage_base + ew * kStageWarpBytes;
     uint32_t t = 0;
     bool ok = true;
-    for (int tile = pair; tile < num_tiles && ok; tile += pairs, t++) {
-      const int m0 = (tile % tiles_m) * BM + (int)rank * 128, n0 = (tile / tiles_m) * BN;
+    for (int i = pair; i < p.items && ok; i += pairs, t++) {
+      const Item it = item_at<A_MN>(p, i, tiles_m, tiles, kblocks);
+      const int m0 = it.m0 + (int)rank * 128, n0 = it.n0;
+      const int cols = (it.half ? BN / 2 : BN) / GROUPS, chunks = cols / 32, col0 = (ew / 4) * cols;   // this warp's
       const uint32_t acc = t & 1, aphase = (t >> 1) & 1;
       const int mw = m0 + q * 32;                         // the warp's first row
+      // four lanes per row, as the staging helpers have it
       [[maybe_unused]] uint4 pf[4];
-      [[maybe_unused]] auto fetch = [&](int c) {                           // four lanes per row, as the staging helpers have it
+      [[maybe_unused]] auto fetch = [&](int c) {
         const int n = n0 + col0 + c * 32 + (lane & 3) * 8;
 #pragma unroll
-        for (int it = 0; it < 4; it++) {
-          const int row = mw + it * 8 + (lane >> 2);
-          pf[it] = make_uint4(0, 0, 0, 0);
-          if (c < NCH && n < p.N && row < p.M) pf[it] = *reinterpret_cast<const uint4*>(ahead + (size_t)row * p.ldc + n);
+        for (int j = 0; j < 4; j++) {
+          const int row = mw + j * 8 + (lane >> 2);
+          pf[j] = make_uint4(0, 0, 0, 0);
+          if (c < chunks && n < p.N && row < p.M) pf[j] = *reinterpret_cast<const uint4*>(ahead + (size_t)row * p.ldc + n);
         }
       };
       if (SIDE) fetch(0);
@@ -240,9 +280,25 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; j++) v[j] = __uint_as_float(r[j]);
-        if (p.flags & kBias) {
+        if constexpr (A_MN) {                              // a weight gradient, fp32
+          if (row_ok) {
+            float* const o = reinterpret_cast<float*>(p.C) + it.slice * p.slice_stride + off;
 #pragma unroll
-          for (int j = 0; j < 32; j++) v[j] += __ldg(p.bias + n + j);
+            for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+          }
+          return;
+        }
+        if (p.flags & kBias) {
+          if (wide_bias) {                                 // n is a multiple of 32
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              const float4 b = __ldg(reinterpret_cast<const float4*>(p.bias + n + j));
+              v[j] += b.x; v[j + 1] += b.y; v[j + 2] += b.z; v[j + 3] += b.w;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; j++) v[j] += __ldg(p.bias + n + j);
+          }
         }
         if (p.flags & kAuxOut) warp_store_rows_bf16(stg, lane, v, p.aux, off, row_ok);
         if (p.flags & kGelu) gelu32(v);                    // not together with kGeluGrad
@@ -265,16 +321,18 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         if (SIDE && (p.flags & kGeluGrad) && (p.flags & kResidual)) warp_load_rows_bf16<true>(stg, lane, p.residual, off, row_ok, v);
         warp_store_rows_bf16(stg, lane, v, p.C, off, row_ok);
       };
+      // tensor-memory loads one block ahead of the arithmetic (sixteen warps hide them from one another)
       uint32_t ra[32], rb[32];
       tc_ld32(taddr, ra);
 #pragma unroll 1
-      for (int c = 0; c < NCH; c += 2) {
+      for (int c = 0; c < chunks; c += 2) {
         tc_wait_ld();
-        if (c + 1 < NCH) tc_ld32(taddr + (c + 1) * 32, rb);
+        if (!WIDE && c + 1 < chunks) tc_ld32(taddr + (c + 1) * 32, rb);
         process(ra, c);
-        if (c + 1 < NCH) {
+        if (c + 1 < chunks) {
+          if (WIDE) tc_ld32(taddr + (c + 1) * 32, rb);
           tc_wait_ld();
-          if (c + 2 < NCH) tc_ld32(taddr + (c + 2) * 32, ra);
+          if (!WIDE && c + 2 < chunks) tc_ld32(taddr + (c + 2) * 32, ra);
           process(rb, c + 1);
         }
       }
@@ -295,14 +353,14 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   }
 }
 
-// K-major matrix [rows][K] (K a multiple of 64) as {64, rows, K / 64}; box = 64 x 128 rows x 2 chunks (32 KB).
-static int make_map_kfold(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t K, uint64_t ld) {
+// K-major matrix [rows][K] (K a multiple of 64) as {64, rows, K / 64}; box = 64 x 128 rows x 2 chunks (32 KB; half a tile: 64 rows).
+static int make_map_kfold(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t K, uint64_t ld, uint32_t box_rows = 128) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return -10;
   if (((uintptr_t)ptr & 15) || (ld * 2) % 16 || K % 64) return -11;
   cuuint64_t dims[3] = {64, rows, K / 64};
   cuuint64_t strides[2] = {ld * 2, 128};
-  cuuint32_t box[3] = {64, 128, 2};
+  cuuint32_t box[3] = {64, box_rows, 2};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -310,14 +368,14 @@ static int make_map_kfold(CUtensorMap* map, const void* ptr, uint64_t rows, uint
   return r == CUDA_SUCCESS ? 0 : -12;
 }
 
-// MN-major matrix [K][cols] (cols a multiple of 64) as {64, K, cols / 64}; box = 64 x 128 K-rows x 2 column groups (32 KB).
-static int make_map_mnfold(CUtensorMap* map, const void* ptr, uint64_t K, uint64_t cols, uint64_t ld) {
+// MN-major matrix [K][cols] (cols a multiple of 64) as {64, K, cols / 64}; box = 64 x 128 K-rows x 2 column groups (32 KB; half a tile: one).
+static int make_map_mnfold(CUtensorMap* map, const void* ptr, uint64_t K, uint64_t cols, uint64_t ld, uint32_t groups = 2) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return -10;
   if (((uintptr_t)ptr & 15) || (ld * 2) % 16 || cols % 64) return -11;
   cuuint64_t dims[3] = {64, K, cols / 64};
   cuuint64_t strides[2] = {ld * 2, 128};
-  cuuint32_t box[3] = {64, 128, 2};
+  cuuint32_t box[3] = {64, 128, groups};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -325,8 +383,32 @@ static int make_map_mnfold(CUtensorMap* map, const void* ptr, uint64_t K, uint64
   return r == CUDA_SUCCESS ? 0 : -12;
 }
 
-using KernelFn = void (*)(CUtensorMap, CUtensorMap, Params);
-constexpr size_t kSmemBytes = (size_t)STAGES * STAGE_BYTES + sizeof(Smem) + 16 + (size_t)EPI_WARPS * kStageWarpBytes + 1024;
+using KernelFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, Params);
+constexpr size_t kSmemBytes = (size_t)STAGES * STAGE_BYTES + sizeof(Smem) + 16 + (size_t)Epilogue<true>::WARPS * kStageWarpBytes + 1024;
+
+static KernelFn pick(bool b_mn, bool side, bool wide) {
+  if (side) return b_mn ? gemm2_bf16_kernel<false, true, true, false> : gemm2_bf16_kernel<false, false, true, false>;
+  if (wide) return b_mn ? gemm2_bf16_kernel<false, true, false, true> : gemm2_bf16_kernel<false, false, false, true>;
+  return b_mn ? gemm2_bf16_kernel<false, true, false, false> : gemm2_bf16_kernel<false, false, false, false>;
+}
+
+static int launch(KernelFn kernel, int threads, int max_pairs, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mh,
+                  const Params& p, void* stream) {
+  const int pairs = p.items < max_pairs ? p.items : max_pairs;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * pairs, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = kSmemBytes;
+  cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  static const bool pdl = [] { const char* e = getenv("GCOW_PDL"); return !(e && e[0] == '0'); }();
+  cfg.attrs = attr; cfg.numAttrs = pdl ? 2 : 1;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, ma, mb, mh, p);
+}
 
 }  // namespace gemm2
 }  // namespace gcow
@@ -340,8 +422,8 @@ int gcow_gemm2_max_pairs() {
   static std::once_flag once;
   static int pairs = 0;
   std::call_once(once, [] {
-    for (const KernelFn kernel : {gemm2_bf16_kernel<false, false>, gemm2_bf16_kernel<true, false>, gemm2_bf16_kernel<false, true>,
-                                  gemm2_bf16_kernel<true, true>}) {
+    for (const KernelFn kernel : {pick(false, false, false), pick(false, true, false), pick(false, false, true), pick(true, false, false),
+                                  pick(true, true, false), pick(true, false, true), (KernelFn)gemm2_bf16_kernel<true, true, false, false>}) {
       if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) != cudaSuccess) {
         cudaGetLastError();
         return;
@@ -349,14 +431,14 @@ int gcow_gemm2_max_pairs() {
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2, 1, 1);
-    cfg.blockDim = dim3(THREADS, 1, 1);
+    cfg.blockDim = dim3(Epilogue<true>::THREADS, 1, 1);
     cfg.dynamicSmemBytes = kSmemBytes;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
     cfg.attrs = &attr; cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm2_bf16_kernel<false, false>, &cfg) == cudaSuccess) pairs = n;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm2_bf16_kernel<false, false, false, true>, &cfg) == cudaSuccess) pairs = n;
     else cudaGetLastError();
   });
   return pairs;
@@ -383,29 +465,66 @@ int gcow_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
   rc = b_mn ? make_map_mnfold(&mb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb)
             : make_map_kfold(&mb, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb);
   if (rc) return rc;
-  Params p;
+  Params p = {};
   p.C = (__nv_bfloat16*)C; p.bias = bias; p.residual = (const __nv_bfloat16*)residual; p.aux = (__nv_bfloat16*)aux;
   p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.flags = flags; p.error = error;
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  const int pairs = tiles < max_pairs ? tiles : max_pairs;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * pairs, 1, 1);
-  cfg.blockDim = dim3(THREADS, 1, 1);
-  cfg.dynamicSmemBytes = kSmemBytes;
-  cfg.stream = (cudaStream_t)stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  static const bool pdl = [] { const char* e = getenv("GCOW_PDL"); return !(e && e[0] == '0'); }();
-  cfg.attrs = attr; cfg.numAttrs = pdl ? 2 : 1;
-  // Its own instance for launches that read nothing besides the accumulator: the block fetched ahead costs 16 registers, for
-  // which the epilogue spilled (16384 x 4096 x 1024: plain 100 -> 95 us, bias 106 -> 97, bias and GELU 144 -> 128).
-  const bool side = flags & (kResidual | kGeluGrad);
-  const KernelFn kernel = b_mn ? (side ? gemm2_bf16_kernel<true, true> : gemm2_bf16_kernel<true, false>)
-                               : (side ? gemm2_bf16_kernel<false, true> : gemm2_bf16_kernel<false, false>);
-  return (int)cudaLaunchKernelEx(&cfg, kernel, ma, mb, p);
+  // A last round of tiles that would leave half of the pairs idle is cut into halves of 128 columns, one for every pair (16384 x
+  // 1024 x 1024 is 3.46 rounds of 74: with a residual 43 -> 40 us, times GELU' 45 -> 41, plain 28 both ways).
+  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN), rest = tiles % max_pairs;
+  p.whole = rest && 2 * rest <= max_pairs ? tiles - rest : tiles;
+  p.items = p.whole + 2 * (tiles - p.whole);
+  CUtensorMap mh = mb;
+  if (p.items > p.whole) {
+    rc = b_mn ? make_map_mnfold(&mh, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, 1)
+              : make_map_kfold(&mh, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 64);
+    if (rc) return rc;
+  }
+  // Its own instance for launches that read nothing besides the accumulator: the blocks fetched ahead cost registers, for
+  // which the epilogue spilled (16384 x 4096 x 1024: plain 100 -> 95 us, bias 106 -> 97).
+  const bool side = flags & (kResidual | kGeluGrad), wide = !side && (flags & kGelu);
+  const KernelFn kernel = pick(b_mn, side, wide);
+  return launch(kernel, wide ? Epilogue<true>::THREADS : Epilogue<false>::THREADS, max_pairs, ma, mb, mh, p, stream);
+}
+
+// How many slices of the reduction gcow_gemm2_wgrad cuts an M x N result over K rows into; 0: not taken (an operand narrower
+// than a tile, or no cluster launches). Fewer tiles than pairs leave the others idle, and every further slice costs a pass
+// over an M x N partial result: the count that a model of the two puts lowest, in stages of 128 rows (0.83 us). 16384
+// rows to 1024 x 4096 122 -> 113 us, 4096 x 1024 116 -> 104, 1024 x 1024 48 -> 45; 50176 rows to 1024 x 256 40 -> 37, 12544 to 2048 x 512 38 -> 34.
+int gcow_gemm2_wgrad_slices(int M, int N, int K) {
+  const int max_pairs = gcow_gemm2_max_pairs();
+  if (max_pairs <= 0 || M < 256 || N < 256 || M % 64 || N % 64 || K < 1024) return 0;
+  const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+  const int kblocks = (K + BK - 1) / BK;
+  int best = 1;
+  double least = 1e30;
+  for (int s = 1; s <= 64 && kblocks / s >= 4; s++) {
+    const int per = (kblocks + s - 1) / s;
+    if ((s - 1) * per >= kblocks) continue;                  // an empty slice
+    const double cost = (double)((tiles * s + max_pairs - 1) / max_pairs) * (per + 6) + (s > 1 ? s * (double)M * N * 8 / 5e6 / 0.83 : 0.0);
+    if (cost < least) { least = cost; best = s; }
+  }
+  return best;
+}
+
+// parts[slice][M][N] fp32 = A^T B over the slice's rows, A [K][M], B [K][N] bf16 with contiguous rows: the weight gradient of a
+// linear layer. `slices` as gcow_gemm2_wgrad_slices has it.
+int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, int M, int N, int K, int lda, int ldb, int slices, uint32_t* error, void* stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || slices <= 0 || M % 64 || N % 64 || lda % 8 || ldb % 8 || ((uintptr_t)parts & 15)) return -2;
+  const int max_pairs = gcow_gemm2_max_pairs();
+  if (max_pairs <= 0) return -2;
+  CUtensorMap ma, mb;
+  int rc = make_map_mnfold(&ma, A, (uint64_t)K, (uint64_t)M, (uint64_t)lda);
+  if (!rc) rc = make_map_mnfold(&mb, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb);
+  if (rc) return rc;
+  Params p = {};
+  p.C = (__nv_bfloat16*)parts;
+  p.M = M; p.N = N; p.K = K; p.ldc = N; p.flags = kOutF32; p.error = error;
+  const int kblocks = (K + BK - 1) / BK;
+  p.slice_blocks = (kblocks + slices - 1) / slices;
+  if ((slices - 1) * p.slice_blocks >= kblocks) return -2;   // an empty slice would leave its part unwritten
+  p.whole = p.items = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * slices;
+  p.slice_stride = (size_t)M * N;
+  return launch(gemm2_bf16_kernel<true, true, false, false>, Epilogue<false>::THREADS, max_pairs, ma, mb, mb, p, stream);
 }
 
 }  // extern "C"

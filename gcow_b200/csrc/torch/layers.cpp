@@ -24,6 +24,9 @@
 
 extern "C" {
 int gcow_gemm2_max_pairs();
+int gcow_gemm2_wgrad_slices(int M, int N, int K);
+int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, int M, int N, int K, int lda, int ldb, int slices, uint32_t* error,
+                     void* stream);
 int gcow_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, const float* bias,
                     const void* residual, void* aux, int flags, uint32_t* error, int b_mn, void* stream);
 int gcow_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, const float* bias,
@@ -181,12 +184,14 @@ Tensor gemm(const Tensor& a, const Tensor& b, const GemmOpts& o, const On& on) {
               (o.residual.defined() ? kResidual : 0) | (o.accumulate ? kAccumulate : 0);
   if (aux.defined()) flags |= o.pre_gelu_out.defined() ? kAuxOut : kGeluGrad;
   const int lda = (int)a.stride(0), ldb = (int)b.stride(0), ldc = (int)out.stride(0);
-  // A large product with a short reduction goes to CTA pairs: two SMs per 256 x 256 tile have the one-CTA tile's traffic per
-  // flop and an overlapped epilogue as well. Long reductions stay on the one-CTA tile, and so do those below 512 (the 1x1
-  // convolutions of a ResNet), which the output stream bounds: the one-CTA kernel's TMA stores are 15 to 30 % faster there.
+  // A large product goes to CTA pairs: two SMs per 256 x 256 tile have the one-CTA tile's traffic per flop and an overlapped
+  // epilogue as well. Long reductions with nothing but a bias behind them stay on the one-CTA tile, whose main loop is a little
+  // faster (8192^3 682 us, pairs 730; 16384 x 1024 x 4096 plain 107 and 112, with a residual 137
+  // and 122), and so do those below 512 (the 1x1 convolutions of a ResNet), which the output stream bounds: the one-CTA
+  // kernel's TMA stores are 15 to 30 % faster there.
   const bool can_pair = pair_gemm_enabled() && !o.a_t && !(flags & (kOutF32 | kAccumulate)) && !o.max_ctas && !o.tile_rows;
   const bool by_rule = K % 64 == 0 && K >= 512 && N % (o.b_t ? 64 : 32) == 0 && M >= 1024 && N >= 256 && lda % 8 == 0 && ldb % 8 == 0 &&
-                       ldc % 8 == 0 && !(K >= 2048 && ((M + 255) / 256) * ((N + 255) / 256) >= 118);
+                       ldc % 8 == 0 && !(K >= 2048 && ((M + 255) / 256) * ((N + 255) / 256) >= 118 && !(flags & (kGelu | kResidual | kGeluGrad)));
   if (can_pair && (o.pair < 0 ? by_rule : o.pair > 0)) {
     const int err = gcow_gemm2_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, lda, ldb, ldc, f32(o.bias),
                                     raw(o.residual), raw(aux), flags, on.error, o.b_t, on.stream);
@@ -221,6 +226,16 @@ Tensor wgrad(const Tensor& g, const Tensor& x, const Tensor& out, const On& on) 
   TORCH_CHECK(!out.defined() || (out.dim() == 2 && out.size(0) == N && out.size(1) == K && out.scalar_type() == at::kFloat && out.is_contiguous()),
               "wgrad: the result has to be a contiguous float32 matrix of the product's shape");
   on_device_of(g, {&x, &out});
+  const int slices = pair_gemm_enabled() && M <= 0x7fffffff && N <= 0x7fffffff && K <= 0x7fffffff && g.stride(0) % 8 == 0 && x.stride(0) % 8 == 0 &&
+                             !((uintptr_t)g.data_ptr() & 15) && !((uintptr_t)x.data_ptr() & 15) && !(out.defined() && ((uintptr_t)out.data_ptr() & 15))
+                         ? gcow_gemm2_wgrad_slices((int)N, (int)K, (int)M) : 0;
+  if (slices > 0) {                                          // CTA pairs, which cut the rows themselves
+    const Tensor to = slices == 1 && out.defined() ? out : empty({slices, N, K}, at::kFloat, g);
+    check(gcow_gemm2_wgrad(g.data_ptr(), x.data_ptr(), f32(to), (int)N, (int)K, (int)M, (int)g.stride(0), (int)x.stride(0), slices, on.error, on.stream),
+          "gcow_gemm2_wgrad");
+    g_launches++;
+    return slices > 1 ? add_parts(to, slices, {N, K}, out, on) : out.defined() ? out : to.view({N, K});
+  }
   const int64_t tiles = ((N + 127) / 128) * ((K + 255) / 256);
   int64_t s = 1;
   while (s < 64 && tiles * s * 2 <= 148 && M % (2 * s) == 0 && (M / (2 * s)) % 64 == 0 && M / (2 * s) >= 512) s *= 2;
