@@ -456,8 +456,8 @@ const gcow::LeanTables& host_lean_tables() {
 }
 }  // namespace
 
-// The tile kernels' 1-D decoder against the plane-by-plane one on `blocks` blocks of `stride` words each (an even number),
-// starting `skip` bits in: the number of blocks decoded differently.
+// The tile kernels' 1-D decoders against the plane-by-plane one on `blocks` blocks of `stride` words each (an even number),
+// starting `skip` bits in: the number of blocks that either of them decodes differently.
 int64_t gcow_window_decode_check(const uint32_t* words, uint64_t blocks, uint32_t stride, uint32_t skip, const int32_t* params) {
   const gcow::LeanTables& lt = host_lean_tables();
   const gcow::ZfpParams p = {(uint32_t)params[0], (uint32_t)params[1], (uint32_t)params[2], params[3]};
@@ -473,6 +473,43 @@ int64_t gcow_window_decode_check(const uint32_t* words, uint64_t blocks, uint32_
     gcow::WordSrc src(w.data(), skip);
     gcow::decode_block<1>(y, p, src, 1);
     bad += memcmp(x, y, 16) != 0;
+    if (!gcow::tile_budget_cuts(p, 1) && gcow::decode_code_1d(x, p, tab.data(), words + b * stride, skip, 1)) bad += memcmp(x, y, 16) != 0;
+  }
+  return bad;
+}
+
+// The tile kernels' 1-D encoder against the plane-by-plane one: the number of blocks of 4 values coded differently; *serial
+// receives how many of them it left to its serial form.
+int64_t gcow_tile_1d_check(const float* values, uint64_t blocks, const int32_t* params, uint64_t* serial) {
+  const gcow::LeanTables& lt = host_lean_tables();
+  const gcow::ZfpParams p = {(uint32_t)params[0], (uint32_t)params[1], (uint32_t)params[2], params[3]};
+  const uint32_t slot_words = gcow::tile_slot_words(p, 1);
+  int64_t bad = 0;
+  *serial = 0;
+  for (uint64_t b = 0; b < blocks; b++) {
+    const float* f = values + 4 * b;
+    uint64_t code[16] = {}, got[16] = {};
+    gcow::WordSink sink(code), out(got);
+    const uint32_t len = gcow::encode_block<1>(f, p, sink);
+    sink.finish();
+    uint32_t bits, w[4];
+    bool ok = true;
+    if (!gcow::tile_budget_cuts(p, 1) && gcow::encode_code_1d(f, p, lt.epair, w, bits)) {
+      for (uint32_t i = 0; i < 4; i++) {
+        const uint32_t here = bits < 32 * i ? 0 : bits - 32 * i < 32 ? bits - 32 * i : 32;
+        ok = ok && (here == 32 || !(w[i] >> here));          // nothing past the code
+        out.put(w[i] & gcow::low_mask32(here), here);
+      }
+    } else {
+      ++*serial;
+      std::vector<uint32_t> slot(slot_words + 8, 0xdeadbeefu);
+      bits = gcow::encode_slot_1d(f, p, lt.epair, lt.etab, slot.data(), 1);
+      for (uint32_t i = slot_words; i < slot.size(); i++) ok = ok && slot[i] == 0xdeadbeefu;
+      for (uint32_t i = 0; i < bits; i += 32) out.put(slot[i / 32] & gcow::low_mask32(bits - i), bits - i < 32 ? bits - i : 32);
+    }
+    out.finish();
+    if (bits < p.minbits) bits = p.minbits;
+    bad += !ok || bits != len || memcmp(code, got, sizeof(code)) != 0;
   }
   return bad;
 }

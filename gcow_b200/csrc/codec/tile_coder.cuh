@@ -247,6 +247,86 @@ GCOW_HD uint32_t encode_slot_1d(const float* f, const ZfpParams& p, const uint32
   return finish_slot(s, slot, stride, p.maxbits);
 }
 
+// 64 bits to bit `at` of w, past what it holds; what leaves the 128 bits falls off.
+GCOW_HD void append64(uint32_t (&w)[4], uint32_t at, uint32_t lo, uint32_t hi) {
+  const uint32_t a = lo << (at & 31u), b = funnel_l(lo, hi, at), c = funnel_l0(hi, at & 31u);
+  if (at >> 5 == 1u) { w[1] |= a; w[2] |= b; w[3] |= c; }   // ordinary data
+  else if (at < 32u) { w[0] |= a; w[1] |= b; w[2] |= c; }
+  else if (at < 96u) { w[2] |= a; w[3] |= b; }
+  else if (at < 128u) w[3] |= a;
+}
+// The same code in registers, hardly a branch on ordinary data: the first eight planes behind the leading zeros two per lookup,
+// the next eight likewise while n < 3, then verbatim nibbles. w: the code from bit 0, zeros past its `length`. False where the
+// serial form above has to do it: a non-finite or tiny maximum, a NaN member, more than sixteen planes with n < 3 or
+// sixteen verbatim ones, a code of more than 128 bits. No budget: the block's code must not reach maxbits.
+GCOW_HD bool encode_code_1d(const float* f, const ZfpParams& p, const uint32_t* epair, uint32_t (&w)[4], uint32_t& length) {
+  const uint32_t mb = f32_bits(fmaxf(fmaxf(fabsf(f[0]), fabsf(f[1])), fmaxf(fabsf(f[2]), fabsf(f[3])))), ex = mb >> 23;
+  const float scale = bits_f32(0x8d800000u - (mb & 0xff800000u));   // 2^(30 - emax), emax = ex - 126; used with 29 <= ex <= 254
+  const float p0 = scale * f[0], p1 = scale * f[1], p2 = scale * f[2], p3 = scale * f[3];
+  bool ok = ex - 29u <= 225u && fabsf((p0 + p1) + (p2 + p3)) < 8.0e9f;              // the sum: a NaN member
+  int32_t q[4];
+#if defined(__CUDA_ARCH__)
+  q[0] = __float2int_rz(p0); q[1] = __float2int_rz(p1); q[2] = __float2int_rz(p2); q[3] = __float2int_rz(p3);
+#else
+  if (ok) { q[0] = (int32_t)p0; q[1] = (int32_t)p1; q[2] = (int32_t)p2; q[3] = (int32_t)p3; }
+  else q[0] = q[1] = q[2] = q[3] = 0;                                               // out of range for this conversion
+#endif
+  fwd_lift(q[0], q[1], q[2], q[3]);
+  uint32_t u[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) u[i] = int2nb(q[i]);
+  const uint32_t prec = block_precision((int)ex - 126, p.maxprec, p.minexp, 1), planes = prec < 32u ? prec : 32u;
+  const uint32_t mm = u[0] | u[1] | u[2] | u[3];
+  uint32_t z = mm ? clz32(mm) : 32u;
+  if (z > planes) z = planes;
+  const uint32_t left = planes - z, first = left < 8u ? left : 8u;
+  ok = ok && z < 23u;                                       // the header's shift
+  // A plane that the block does not have codes like a zero plane, min(n + 1, 4) zeros, which are taken off again.
+  auto planes8 = [&](uint32_t at, uint32_t here, uint32_t prev, uint32_t& lo, uint32_t& hi, uint32_t& bits) {
+    const uint32_t m = pow2_factor(at);
+    const uint32_t R = byte_perm(byte_perm(u[0] * m, u[1] * m, 0x0073), byte_perm(u[2] * m, u[3] * m, 0x0073), 0x5410) &
+                       (((0xff00u >> here) & 0xffu) * 0x01010101u);
+    uint32_t e[4], sum = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) sum += prev = e[j] = pair_entry(epair, R, j, prev);
+    lo = hi = 0;
+#pragma unroll
+    for (int j = 3; j >= 0; j--) {
+      hi = funnel_l(lo, hi, e[j]);
+      lo = prepend_code(e[j], lo);
+    }
+    const uint32_t n = (prev >> 8) & 0xffu;
+    bits = (sum & 0xffu) - (8u - here) * (n < 4u ? n + 1u : 4u);
+    return prev;
+  };
+  uint32_t lo, hi, bits;
+  uint32_t prev = planes8(z, first, 0, lo, hi, bits);
+  const uint32_t s = kHeaderBits + z;
+  const bool none = planes == 0 || mb == 0;                 // the block is a single 0 bit
+  w[0] = none ? 0u : (2u * ex + 3u) | (lo << (s & 31u));    // flag bit + biased exponent (emax + 127 = ex + 1)
+  w[1] = none ? 0u : funnel_l(lo, hi, s);
+  w[2] = none ? 0u : funnel_l0(hi, s & 31u);
+  w[3] = 0;
+  length = none ? 1u : s + bits;
+  uint32_t k = 24u - z, rest = none ? 0u : left - first;    // planes k-1 .. k-rest remain
+  if (rest && ((prev >> 8) & 0xffu) < 3u) {
+    const uint32_t next = rest < 8u ? rest : 8u;
+    prev = planes8(z + 8u, next, prev & 0xff00u, lo, hi, bits);
+    append64(w, length, lo, hi);
+    length += bits;
+    rest -= next;
+    k -= 8u;
+    ok = ok && (!rest || ((prev >> 8) & 0xffu) >= 3u);
+  }
+  if (rest) {                                               // verbatim nibbles
+    const uint32_t t0 = plane_group8(u, k) & low_mask32(4u * rest);
+    const uint32_t t1 = rest > 8u ? plane_group8(u, k - 8u) & low_mask32(4u * rest - 32u) : 0u;
+    append64(w, length, t0, t1);
+    length += 4u * rest;
+  }
+  return (ok && rest <= 16u && length <= 128u) || none;
+}
+
 // -------------------------------------------------------- 16 x 16 bit transposition
 // In: w[j] = row j in the low half, row j + 8 in the high half (j = 0..7). Out: w[j] = column j
 // in the low half, column j + 8 in the high half. The same function inverts itself.
@@ -455,6 +535,69 @@ GCOW_HD void decode_window_1d(float* f, const ZfpParams& p, const uint32_t* tab,
   for (int i = 0; i < 4; i++) q[i] = nb2int(u[i]);
   inv_lift(q[0], q[1], q[2], q[3]);
   inv_cast<4>(f, q, emax, shift);
+}
+
+// The same as a straight line, for blocks that no budget cuts. What a block ends with need not be found: its planes below the
+// last one are read from whatever follows it and masked off. False (f is not written) where the loop above has to do it:
+// more than three windows or seven planes with n < 3, more than 23 leading zero planes, a code past the 96 bits held.
+GCOW_HD bool decode_code_1d(float* f, const ZfpParams& p, const uint32_t* tab, const uint32_t* words, uint32_t pos, int shift) {
+  const uint32_t* const w = words + (pos >> 5);
+  const uint32_t o = pos & 31u, w1 = w[1], w2 = w[2];
+  uint32_t x0 = window32(w[0], w1, o), x1 = window32(w1, w2, o), x2 = window32(w2, w[3], o);
+  const uint32_t head = x0;
+  if (!(head & 1u)) {
+    f[0] = f[1] = f[2] = f[3] = 0;
+    return true;
+  }
+  const uint32_t e8 = (head >> 1) & 0xffu;                   // emax + 127
+  const uint32_t prec = block_precision((int)e8 - kEBias, p.maxprec, p.minexp, 1), planes = prec < 32u ? prec : 32u;
+  auto skip = [&](uint32_t n) {                            // n < 32
+    x0 = window32(x0, x1, n);
+    x1 = window32(x1, x2, n);
+    x2 >>= n;
+  };
+  skip(kHeaderBits);
+  const uint32_t z = (uint32_t)ctz32(x0 | 0x1000000u);
+  if (planes > z + 23u) return false;                      // of which more than sixteen would be verbatim
+  skip(z);
+  uint32_t U = 0, gone = z, row = 0, used = kHeaderBits + z;
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    if (c == 0 || (row != 0x3000u && gone < planes)) {
+      const DecWindow d = *reinterpret_cast<const DecWindow*>(reinterpret_cast<const char*>(tab) + row + 8u * (x0 & 511u));
+      const uint32_t n = (d.meta >> 8) & 15u, len = d.meta & 31u;
+      U = (U << n) | d.u;
+      gone += n;
+      used += len;
+      skip(len);
+      row = d.meta & 0x3000u;
+    }
+  }
+  const int rest = (int)(planes - gone);                     // verbatim planes; below 0: read too far, which the mask undoes
+  if (!((row == 0x3000u || rest <= 0) && gone - z <= 7u && gone <= 31u && z < 24u && rest <= 16 && (int)used + 4 * rest <= 96)) return false;
+  const uint32_t* const nib = tab + kDecNibbles;
+  const uint32_t W = ((nib[x0 & 255u] * 4u + nib[(x0 >> 8) & 255u]) * 4u + nib[(x0 >> 16) & 255u]) * 4u + nib[x0 >> 24];
+  const uint32_t m = gone < 24u ? pow2_factor(24u - gone) : 1u, r = gone < 24u ? 0u : gone - 24u;
+  uint32_t u[4];
+  u[0] = shr_sat(byte_perm_sx(W, U, 0xcc40) * m, r); u[1] = shr_sat(byte_perm_sx(W, U, 0xdd51) * m, r);
+  u[2] = shr_sat(byte_perm_sx(W, U, 0xee62) * m, r); u[3] = shr_sat(byte_perm_sx(W, U, 0xff73) * m, r);
+  if (rest > 8) {                                          // gone < 24
+    const uint32_t k = 24u - gone;
+    uint32_t V = (nib[x1 & 255u] * 4u + nib[(x1 >> 8) & 255u]) * 16u;
+    if (rest > 12) V += nib[(x1 >> 16) & 255u] * 4u + nib[x1 >> 24];
+    u[0] |= shr_sat(V << 24, 32u - k); u[1] |= shr_sat((V & 0xff00u) << 16, 32u - k);
+    u[2] |= shr_sat((V & 0xff0000u) << 8, 32u - k); u[3] |= shr_sat(V & 0xff000000u, 32u - k);
+  }
+  const uint32_t mask = ~shr_sat(0xffffffffu, planes);
+  int32_t q[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) q[i] = nb2int(u[i] & mask);
+  inv_lift(q[0], q[1], q[2], q[3]);
+  const int ef = (int)e8 - 30 - shift;                     // a normal float unless the block is tiny
+  const float scale = (ef >= 1 && ef <= 254) ? bits_f32((uint32_t)ef << 23) : pow2f((int)e8 - kEBias - 30 - shift);
+#pragma unroll
+  for (int i = 0; i < 4; i++) f[i] = scale * (float)q[i];
+  return true;
 }
 
 // One plane of 16 coefficients whose code the budget cuts: bit by bit. A one-bit that is pending where the bits end is placed.

@@ -1,18 +1,19 @@
 // Tile kernels of the ZFP codec (sm_100a): every mode the one-store fixed-rate 1-D kernels do not cover - 2-D in any
 // mode, fixed accuracy / precision, odd rates.
 //
-// Encode: a warp takes 32 * kPer consecutive blocks, codes each into a slot in shared memory (tile_coder.cuh), prefix-sums
-// the lengths and packs the slots into one bit string in shared memory.
-//   * Fixed rate: the string's place in the stream is known and word aligned, so the warp writes it there: one launch, no
-//     scratch, no barrier.
-//   * Variable rate: the warp writes its string, its length and its blocks' lengths (16 bits each) to scratch, all
-//     coalesced, and the CTA its total; a second kernel adds up the totals before its share of the tiles and moves the
-//     strings into place, shifted, together with the blocks' bit offsets. A word that two strings share is written by
-//     the later one, which reads the earlier one's last 32 bits (a string that is followed by another has at least 32
-//     bits, one per block). The strings are a fraction of the input and mostly still in L2, so this costs little, and
-//     nothing waits: with the lengths passed on inside one kernel (decoupled look-back) the polling of a thousand CTAs
-//     and the wait of every tile for its predecessors took longer than the coding itself (1-D, 25.6 M values at
-//     tolerance 1e-6: 226 to 343 us for that kernel).
+// Encode: a warp takes 32 * kPer consecutive blocks.
+//   * Fixed rate: every block is coded into a slot in shared memory (tile_coder.cuh). Blocks of whole words: every lane stores its
+//     block where it belongs, 16 bytes at a time. Other rates: the warp packs its slots into one bit string, whose place in
+//     the stream is known and word aligned. One launch, no scratch.
+//   * Variable rate: the warp's blocks grow into one bit string in shared memory, 32 at a time (StringBuilder), and leave as a
+//     part of ONE string per tile (a CTA's 256 * kPer blocks), shifted by the length of the warps before it; a word that two
+//     warps share is written by the later one, which takes the earlier one's last 32 bits from shared memory (a string that
+//     is followed by another has at least 32 bits, one per block). Every block's offset within its warp's string (16 bits)
+//     and every warp's within the tile go to scratch with it, all coalesced. A second kernel adds up the tiles' lengths
+//     before its share of them and moves their strings into place the same way, together with the blocks' bit offsets.
+//     Nothing waits: with the lengths passed on inside one kernel (decoupled look-back) the polling of a thousand CTAs and the
+//     wait of every tile for its predecessors took longer than the coding itself (1-D, 25.6 M values at tolerance 1e-6:
+//     226 to 343 us for that kernel).
 //
 // Decode: a warp copies the segment of the stream that holds its 32 * kPer blocks into shared memory, coalesced, and each
 // lane reads its blocks from there.
@@ -22,15 +23,16 @@
 #include <stdint.h>
 #include <atomic>
 #include "tile_coder.cuh"
+#include "../ops/pdl.cuh"
 
 namespace gcow {
 
 constexpr int kTileThreads = 256, kTileWarps = kTileThreads / 32;
-// Blocks per lane: a 1-D block is little work, so four per lane make the steps per string (scan, copy) a small share; a 2-D
-// block is sixteen values and up to 17 words of slot, so one.
-template <int DIM> struct TileShape {
-  static constexpr int kPer = DIM == 1 ? 4 : 1, kWarpBlocks = 32 * kPer, kBlocks = kTileThreads * kPer;
-};
+// Blocks per lane, kPer. A 1-D block is little work, so four per lane make the steps per string (copy, totals) a small share -
+// but one per lane where four would leave SMs without a CTA, since a lane's blocks follow one another. A 2-D block is
+// sixteen values and up to 17 words of slot, so one.
+constexpr uint64_t kWideBlocks = 148ull * 4 * kTileThreads;   // more than this: four per lane
+inline int tile_per(uint64_t blocks, int dim) { return dim == 1 && blocks > kWideBlocks ? 4 : 1; }
 
 __device__ const TwinTable d_twin{};
 __device__ const RunTable d_run{};
@@ -39,8 +41,9 @@ struct TileArgs {
   uint64_t nx, ny, blocks;
   uint32_t bx, tiles;             // blocks per row of blocks (2-D); tiles
   uint32_t slot_words, warp_words;  // encode: words per slot, per packed string; decode: window capacity, window pitch
-  uint32_t pitch;                 // encode at variable rate: words from one string to the next in scratch
+  uint32_t pitch;                 // encode at variable rate: words from one tile's string to the next in scratch
   ZfpParams p;
+  int wide;                       // encode, kDirect: blocks of whole 16 bytes at an aligned address
   int vec;                        // 2-D: values per load that the row pitch and the base address allow (4, 2 or 1); 1-D: 4 or 1
 };
 
@@ -146,12 +149,12 @@ __device__ __forceinline__ void tile_store_2d(const float* f, float* __restrict_
       if (x0 + x < a.nx && y0 + y < a.ny) dst[y * a.nx + x] = f[4 * y + x];
 }
 
-// Scratch of the variable-rate encoder: the warps' strings, their lengths, the tiles' lengths, the blocks' lengths.
+// Scratch of the variable-rate encoder: the tiles' strings and lengths, the warps' offsets in them, the blocks' in their warp's.
 struct TileStrings {
   uint32_t* strings;
-  uint32_t* unit_bits;
   uint32_t* tile_bits;
-  uint16_t* lens;
+  uint32_t* warp_at;
+  uint16_t* block_at;
 };
 
 // The stream ends with this string: its open word, and zeros up to a 64-bit boundary.
@@ -165,34 +168,166 @@ __device__ __forceinline__ void close_stream(uint32_t* __restrict__ out, const u
   }
 }
 
-template <int DIM, bool FIXED, bool BUDGET>
+// The last 32 bits of a string of at least 32.
+__device__ __forceinline__ uint32_t last_bits(const uint32_t* string, uint32_t bits) {
+  const uint32_t* const q = string + ((bits - 32) >> 5);
+  return bits & 31u ? __funnelshift_r(q[0], q[1], bits) : q[0];
+}
+
+// The words of w, zero past the code, to bit `at` of a zeroed string.
+template <int NW>
+__device__ __forceinline__ void put_bits(uint32_t* string, uint32_t at, const uint32_t (&w)[NW]) {
+  uint32_t* const dst = string + (at >> 5);
+  uint32_t below = 0;
+#pragma unroll
+  for (int i = 0; i <= NW; i++) {
+    const uint32_t here = i < NW ? w[i < NW ? i : 0] : 0u, v = __funnelshift_l(below, here, at);
+    if (v) atomicOr(dst + i, v);
+    below = here;
+  }
+}
+
+// A warp's string as it grows, 32 blocks (one per lane, in order) at a time. Words are stored once, whole: a word that two
+// blocks share is stored by the later one, which gets the earlier one's last bits by a shuffle; `carry` holds the last,
+// open word of the string so far. That takes blocks of 32 to 128 bits (a shorter one could share its word with two
+// others); any other group of blocks is put together by atomic operations on zeroed words.
+struct StringBuilder {
+  uint32_t* string;
+  uint32_t at, carry;          // bits so far; the word they end in (0 where they end on its boundary)
+  __device__ __forceinline__ explicit StringBuilder(uint32_t* s) : string(s), at(0), carry(0) {}
+  // This lane's block: `len` bits with its padding (0: none, behind the last one); w: all of it, zero past its end, if in_w;
+  // put(place) adds the block to zeroed words otherwise. Returns the block's place.
+  template <class Put>
+  __device__ __forceinline__ uint32_t add(int lane, uint32_t len, bool in_w, const uint32_t (&w)[4], Put&& put) {
+    uint32_t x = len;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+      if (lane >= d) x += y;
+    }
+    const uint32_t place = at + x - len, end = at + __shfl_sync(0xffffffffu, x, 31), o = place & 31u;
+    if (__all_sync(0xffffffffu, in_w && len - 32u <= 96u)) {
+      const uint32_t n = (o + len) >> 5;                   // words that end in this block: 1 to 4
+      const uint32_t w0 = w[0] << o, w1 = __funnelshift_l(w[0], w[1], o), w2 = __funnelshift_l(w[1], w[2], o),
+                     w3 = __funnelshift_l(w[2], w[3], o), w4 = __funnelshift_l(w[3], 0u, o);
+      const uint32_t open = n == 1 ? w1 : n == 2 ? w2 : n == 3 ? w3 : w4;
+      uint32_t below = __shfl_up_sync(0xffffffffu, open, 1);
+      if (lane == 0) below = carry;
+      carry = __shfl_sync(0xffffffffu, open, 31);
+      uint32_t* const dst = string + (place >> 5);
+      dst[0] = w0 | below;
+      if (n > 1) dst[1] = w1;
+      if (n > 2) dst[2] = w2;
+      if (n > 3) dst[3] = w3;
+    } else {
+      for (uint32_t i = (at >> 5) + lane; i <= end >> 5; i += 32) string[i] = i == at >> 5 ? carry : 0u;
+      __syncwarp();
+      put(place);
+      __syncwarp();
+      carry = string[end >> 5];
+      __syncwarp();
+    }
+    at = end;
+    return place;
+  }
+  // The open word joins the others; the lanes may read the string.
+  __device__ __forceinline__ void close(int lane) {
+    if (lane == 0 && (at & 31u)) string[at >> 5] = carry;
+    __syncwarp();
+  }
+};
+
+enum TileMode { kVariable, kPacked, kDirect };              // variable rate; fixed rate; fixed rate in whole words
+
+template <int DIM, int PER, TileMode MODE, bool BUDGET>
 __global__ void __launch_bounds__(kTileThreads)
 encode_tiles_kernel(const float* __restrict__ in, const TileArgs a, uint32_t* __restrict__ out, uint64_t* __restrict__ block_bits,
                     const TileStrings st, const uint16_t* __restrict__ enc_tab, const uint32_t* __restrict__ pair_tab) {
-  constexpr int kPer = TileShape<DIM>::kPer, WB = TileShape<DIM>::kWarpBlocks, NB = TileShape<DIM>::kBlocks;
+  constexpr int WB = 32 * PER, NB = kTileThreads * PER;
   constexpr int kTabWords = DIM == 1 ? kEncPairTabSize : kTwinTabSize;
+  constexpr int SW = MODE == kVariable ? 32 : WB;           // variable rate: a slot per lane, used again for its next block
   extern __shared__ __align__(16) uint32_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // table | per warp: slots [slot_words][WB], lengths [WB], packed string [warp_words]
+  // table | per warp: slots [slot_words][SW], packed string [warp_words] (none for kDirect)
   uint32_t* const tab = smem;
-  uint32_t* const slots = smem + kTabWords + warp * (a.slot_words * WB + WB + a.warp_words);
-  uint32_t* const lens = slots + a.slot_words * WB;
-  uint32_t* const packed = lens + WB;
-  __shared__ uint32_t s_total[2][kTileWarps];               // alternating: a warp can be one tile ahead of the sum
+  uint32_t* const slots = smem + kTabWords + warp * (a.slot_words * SW + a.warp_words);
+  uint32_t* const packed = slots + a.slot_words * SW;
+  __shared__ uint32_t s_total[2][kTileWarps], s_last[2][kTileWarps];   // alternating: a warp can be one tile ahead of the others
 
+  pdl_trigger();                                            // the kernel that moves the strings may set itself up
   if (DIM == 1) {
     for (int i = tid; i < kEncPairTabSize / 4; i += kTileThreads)
       reinterpret_cast<uint4*>(tab)[i] = reinterpret_cast<const uint4*>(pair_tab)[i];
   } else {
     if (tid < kTwinTabSize / 4) reinterpret_cast<uint4*>(tab)[tid] = reinterpret_cast<const uint4*>(d_twin.v)[tid];
   }
+  if (MODE == kPacked)
+    for (uint32_t i = lane; i < a.warp_words / 4; i += 32) reinterpret_cast<uint4*>(packed)[i] = make_uint4(0, 0, 0, 0);
   __syncthreads();
+  pdl_wait();                                               // the tables came under the tail of the stream's last kernel
   int turn = 0;
   for (uint32_t tile = blockIdx.x; tile < a.tiles; tile += gridDim.x, turn ^= 1) {
     const uint64_t b0 = (uint64_t)tile * NB + warp * WB;
     const uint32_t nb = a.blocks > b0 ? (a.blocks - b0 < WB ? (uint32_t)(a.blocks - b0) : WB) : 0;
+    if (MODE == kVariable) {
+      StringBuilder string(packed);
 #pragma unroll 1
-    for (int j = 0; j < kPer; j++) {
+      for (int j = 0; j < PER; j++) {
+        const uint32_t i = lane + 32 * j;
+        const bool there = i < nb;
+        uint32_t bits = 0, w[4] = {0, 0, 0, 0};
+        bool in_w = false;
+        if (there) {
+          float f[1 << (2 * DIM)];
+          if (DIM == 1) {
+            tile_load_1d(f, in, a, b0 + i);
+            in_w = !BUDGET && encode_code_1d(f, a.p, tab, w, bits);
+            if (!in_w) bits = encode_slot_1d(f, a.p, tab, enc_tab, slots + lane, 32);
+          } else {
+            tile_load_2d(f, in, a, b0 + i);
+            bits = encode_slot_2d<BUDGET>(f, a.p, tab, slots + lane, 32);
+          }
+          if (!in_w && bits <= 128u) {
+            in_w = true;
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) w[k] = 32 * k < bits ? slots[lane + 32 * k] : 0u;
+          }
+        }
+        const uint32_t place = string.add(lane, there && bits < a.p.minbits ? a.p.minbits : bits, in_w, w, [&](uint32_t at) {
+          if (!there) return;
+          if (in_w) put_bits(packed, at, w);
+          else for (uint32_t k = 0; 32 * k < bits; k++) put_bits(packed, at + 32 * k, {slots[lane + 32 * k]});
+        });
+        if (there) st.block_at[b0 + i] = (uint16_t)place;
+      }
+      string.close(lane);
+      const uint32_t total = string.at, words = (total + 31) >> 5;
+      if (lane == 0) {
+        s_total[turn][warp] = total;
+        s_last[turn][warp] = total >= 32 ? last_bits(packed, total) : 0u;
+      }
+      __syncthreads();
+      uint32_t at = 0, all = 0;
+#pragma unroll
+      for (int w = 0; w < kTileWarps; w++) {
+        if (w == warp) at = all;
+        all += s_total[turn][w];
+      }
+      if (tid == 0) st.tile_bits[tile] = all;
+      if (lane == 0 && nb) st.warp_at[(uint64_t)tile * kTileWarps + warp] = at;
+      // whole words up to this string's end (the tile's last string: and the open one)
+      const uint32_t o = at & 31u, prev = at ? s_last[turn][warp - 1] : 0u;
+      const uint32_t n = at + total == all ? (o + total + 31) >> 5 : (o + total) >> 5;
+      uint32_t* const dst = st.strings + (uint64_t)tile * a.pitch + (at >> 5);
+      if (nb)
+        for (uint32_t i = lane; i < n; i += 32) dst[i] = __funnelshift_l(i ? packed[i - 1] : prev, i < words ? packed[i] : 0u, o);
+      __syncwarp();
+      continue;
+    }
+
+    uint32_t lens[PER] = {};                                // the blocks' own lengths, before padding to minbits
+#pragma unroll 1
+    for (int j = 0; j < PER; j++) {
       const uint32_t i = lane + 32 * j;
       uint32_t bits = 0;
       if (i < nb) {
@@ -205,39 +340,40 @@ encode_tiles_kernel(const float* __restrict__ in, const TileArgs a, uint32_t* __
           bits = encode_slot_2d<BUDGET>(f, a.p, tab, slots + i, WB);
         }
       }
-      lens[i] = bits;                                       // the block's own length, before padding to minbits
+#pragma unroll
+      for (int k = 0; k < PER; k++) lens[k] = PER == 1 || k == j ? bits : lens[k];
     }
 
-    // lengths -> offsets within the warp's string
-    uint32_t off[kPer], len[kPer], total = 0;
+    if (MODE == kDirect) {
+      const uint32_t bw = a.p.maxbits >> 5;                 // words per block
 #pragma unroll
-    for (int j = 0; j < kPer; j++) {
-      const uint32_t i = lane + 32 * j;
-      len[j] = lens[i];
-      if (FIXED) {
-        off[j] = i * a.p.maxbits;
-      } else {
-        uint32_t x = len[j];
-        if (i < nb && x < a.p.minbits) x = a.p.minbits;
-        const uint32_t v = x;
-        if (i < nb) st.lens[b0 + i] = (uint16_t)v;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
-          if (lane >= d) x += y;
+      for (int j = 0; j < PER; j++) {
+        const uint32_t i = lane + 32 * j;
+        if (i >= nb) break;
+        const uint32_t* const src = slots + i;
+        uint32_t* const dst = out + (b0 + i) * bw;
+        const uint32_t nw = (lens[j] + 31) >> 5;
+        auto word = [&](uint32_t w) { return w < nw ? src[w * WB] : 0u; };
+        if (a.wide) {
+          for (uint32_t w = 0; w < bw; w += 4) *reinterpret_cast<uint4*>(dst + w) = make_uint4(word(w), word(w + 1), word(w + 2), word(w + 3));
+        } else {
+          for (uint32_t w = 0; w < bw; w++) dst[w] = word(w);
         }
-        off[j] = total + x - v;
-        total += __shfl_sync(0xffffffffu, x, 31);
+        if (block_bits) block_bits[b0 + i] = (b0 + i) * a.p.maxbits;
+        if (b0 + i + 1 == a.blocks) {
+          if (block_bits) block_bits[a.blocks] = a.blocks * a.p.maxbits;
+          if ((a.blocks * bw) & 1u) dst[bw] = 0;            // zeros up to a 64-bit boundary
+        }
       }
+      continue;
     }
-    if (FIXED) total = nb * a.p.maxbits;
-    const uint32_t words = (total + 31) >> 5;
-    for (uint32_t i = lane; i < words / 4 + 1; i += 32) reinterpret_cast<uint4*>(packed)[i] = make_uint4(0, 0, 0, 0);
+
+    const uint32_t total = nb * a.p.maxbits, words = (total + 31) >> 5;
     __syncwarp();
 #pragma unroll
-    for (int j = 0; j < kPer; j++) {
-      const uint32_t nw = (len[j] + 31) >> 5, o = off[j] & 31u;
-      uint32_t* dst = packed + (off[j] >> 5);
+    for (int j = 0; j < PER; j++) {
+      const uint32_t off = (lane + 32 * j) * a.p.maxbits, nw = (lens[j] + 31) >> 5, o = off & 31u;
+      uint32_t* dst = packed + (off >> 5);
       const uint32_t* src = slots + lane + 32 * j;
       uint32_t carry = 0;
 #pragma unroll 1
@@ -250,58 +386,42 @@ encode_tiles_kernel(const float* __restrict__ in, const TileArgs a, uint32_t* __
       if (carry) atomicOr(dst, carry);
     }
     __syncwarp();
-    if (FIXED) {
-      const uint64_t start = b0 * a.p.maxbits;              // a multiple of 32 bits
-      const bool ends = nb && b0 + nb == a.blocks;
-      uint32_t* const dst = out + (start >> 5);
-      for (uint32_t i = lane; i < total >> 5; i += 32) dst[i] = packed[i];
-      if (ends && lane == 0) close_stream(out, packed, start, total, 0);
-      if (block_bits) {
+    const uint64_t start = b0 * a.p.maxbits;                // a multiple of 32 bits
+    const bool ends = nb && b0 + nb == a.blocks;
+    uint32_t* const dst = out + (start >> 5);
+    for (uint32_t i = lane; i < total >> 5; i += 32) dst[i] = packed[i];
+    if (ends && lane == 0) close_stream(out, packed, start, total, 0);
+    if (block_bits) {
 #pragma unroll
-        for (int j = 0; j < kPer; j++) {
-          const uint32_t i = lane + 32 * j;
-          if (i < nb) block_bits[b0 + i] = start + off[j];
-        }
-        if (ends && lane == 0) block_bits[a.blocks] = start + total;
+      for (int j = 0; j < PER; j++) {
+        const uint32_t i = lane + 32 * j;
+        if (i < nb) block_bits[b0 + i] = start + i * a.p.maxbits;
       }
-    } else {
-      const uint64_t unit = (uint64_t)tile * kTileWarps + warp;
-      uint32_t* const dst = st.strings + unit * a.pitch;
-      for (uint32_t i = lane; i < words; i += 32) dst[i] = packed[i];
-      if (lane == 0) {
-        s_total[turn][warp] = total;
-        if (nb) st.unit_bits[unit] = total;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        uint32_t sum = 0;
-#pragma unroll
-        for (int w = 0; w < kTileWarps; w++) sum += s_total[turn][w];
-        st.tile_bits[tile] = sum;
-      }
+      if (ends && lane == 0) block_bits[a.blocks] = start + total;
     }
+    __syncwarp();
+    for (uint32_t i = lane; i < words; i += 32) packed[i] = 0;
     __syncwarp();
   }
 }
 
-// Second kernel of the variable-rate encoder: every CTA takes a contiguous share of the tiles, at most kPlaceUnits strings
-// at a time, whose starts it works out in shared memory first; then every load of a string depends on nothing but that
-// table, and a warp keeps several of them in flight.
-constexpr int kPlaceUnits = 1024;
-
-template <int DIM>
-__global__ void __launch_bounds__(kTileThreads, DIM == 1 ? 4 : 5)
+// Second kernel of the variable-rate encoder: every CTA takes a contiguous share of the tiles, at most kTileThreads of them at a
+// time, whose starts it works out in shared memory first; then nothing depends on anything but that table, and the
+// warps run through the strings at their own pace.
+template <int PER>
+__global__ void __launch_bounds__(kTileThreads)
 place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restrict__ out, uint64_t* __restrict__ block_bits,
                      uint64_t* total_out) {
-  constexpr int kPer = TileShape<DIM>::kPer, WB = TileShape<DIM>::kWarpBlocks;
-  constexpr int kWords = DIM == 1 ? 8 : 3;                  // words per lane and step: a 1-D string is some 200 words, a 2-D one 70
+  constexpr int NB = kTileThreads * PER;
   __shared__ unsigned long long s_sum[kTileWarps];
   __shared__ uint32_t s_warp[kTileWarps];
-  __shared__ uint32_t s_bits[kPlaceUnits];                  // a string's length ...
-  __shared__ uint32_t s_from[kPlaceUnits];                  // ... and start after the first one of the batch
+  __shared__ uint32_t s_bits[kTileThreads];                 // a string's length ...
+  __shared__ uint32_t s_from[kTileThreads];                 // ... and start after the first one of the batch
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t t0 = (uint32_t)((uint64_t)a.tiles * blockIdx.x / gridDim.x);
   const uint32_t t1 = (uint32_t)((uint64_t)a.tiles * (blockIdx.x + 1) / gridDim.x);
+  pdl_trigger();
+  pdl_wait();
   unsigned long long base = 0;
 #pragma unroll 4
   for (uint32_t i = tid; i < t0 / 4; i += kTileThreads) {
@@ -317,19 +437,10 @@ place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restric
 #pragma unroll
   for (int w = 0; w < kTileWarps; w++) base += s_sum[w];
 
-  const uint64_t units = (a.blocks + WB - 1) / WB;
-  const uint64_t u_end = (uint64_t)t1 * kTileWarps < units ? (uint64_t)t1 * kTileWarps : units;
-  for (uint64_t u0 = (uint64_t)t0 * kTileWarps; u0 < u_end; u0 += kPlaceUnits) {
-    const uint32_t nu = u_end - u0 < kPlaceUnits ? (uint32_t)(u_end - u0) : kPlaceUnits;
-    // starts of this batch's strings: four consecutive ones per thread
-    uint32_t v[4], sum = 0;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const uint32_t i = tid * 4 + j;
-      v[j] = i < nu ? st.unit_bits[u0 + i] : 0;
-      sum += v[j];
-    }
-    uint32_t x = sum;
+  for (uint32_t u0 = t0; u0 < t1; u0 += kTileThreads) {
+    const uint32_t nu = t1 - u0 < kTileThreads ? t1 - u0 : kTileThreads;
+    const uint32_t v = tid < nu ? st.tile_bits[u0 + tid] : 0;
+    uint32_t x = v;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
@@ -337,87 +448,60 @@ place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restric
     }
     if (lane == 31) s_warp[warp] = x;
     __syncthreads();
-    uint32_t from = x - sum, all = 0;
+    uint32_t from = x - v, all = 0;
 #pragma unroll
     for (int w = 0; w < kTileWarps; w++) {
       if (w < warp) from += s_warp[w];
       all += s_warp[w];
     }
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      s_bits[tid * 4 + j] = v[j];
-      s_from[tid * 4 + j] = from;
-      from += v[j];
-    }
+    s_bits[tid] = v;
+    s_from[tid] = from;
     __syncthreads();
     // the caller's host thread waits for the stream's length: it gets it before the strings are moved
-    if (total_out && u0 + nu == units && tid == 0) {
+    if (total_out && u0 + nu == a.tiles && tid == 0) {
       *(volatile uint64_t*)total_out = base + all;
       __threadfence_system();
     }
-
-    // The loads of a warp's next string are issued before the current one is written.
-    struct Fetched { uint32_t w[kWords], len[kPer], q0, q1; } cur, nxt;
-    auto fetch = [&](uint32_t k, Fetched& f) {
-      const uint64_t unit = u0 + k, b0 = unit * WB;
-      const uint32_t nb = a.blocks - b0 < WB ? (uint32_t)(a.blocks - b0) : WB, words = (s_bits[k] + 31) >> 5;
-      const uint32_t* const src = st.strings + unit * a.pitch;
-      const uint16_t* const lens = st.lens + b0;
-#pragma unroll
-      for (int j = 0; j < kPer; j++) f.len[j] = lane + 32 * j < nb ? lens[lane + 32 * j] : 0;
-#pragma unroll
-      for (int j = 0; j < kWords; j++) f.w[j] = 32 * j + lane < words ? src[32 * j + lane] : 0u;
-      f.q0 = f.q1 = 0;
-      if (unit) {                                           // the words with the 32 bits before this string
-        const uint32_t pt = k ? s_bits[k - 1] : st.unit_bits[unit - 1];
-        const uint32_t* const q = src - a.pitch + ((pt - 32) >> 5);
-        f.q0 = q[0];
-        f.q1 = pt & 31u ? q[1] : 0u;
-        f.q0 = window32(f.q0, f.q1, pt & 31u);
-      }
-    };
-    if (warp < nu) fetch(warp, cur);
-    for (uint32_t k = warp; k < nu; k += kTileWarps) {
-      if (k + kTileWarps < nu) fetch(k + kTileWarps, nxt);
-      const uint64_t unit = u0 + k, b0 = unit * WB, start = base + s_from[k];
-      const uint32_t nb = a.blocks - b0 < WB ? (uint32_t)(a.blocks - b0) : WB, total = s_bits[k];
-      const uint32_t* const src = st.strings + unit * a.pitch;
+#pragma unroll 1
+    for (uint32_t k = 0; k < nu; k++) {
+      const uint32_t tile = u0 + k, total = s_bits[k];
+      const uint64_t start = base + s_from[k];
+      const uint32_t* const src = st.strings + (uint64_t)tile * a.pitch;
       const uint32_t o = (uint32_t)(start & 31u), words = (total + 31) >> 5, full = (o + total) >> 5;
       uint32_t* const dst = out + (start >> 5);
-      uint32_t last = cur.q0;                               // the word before the next chunk
+      uint32_t prev = 0;
+      if (tid == 0 && tile) prev = last_bits(src - a.pitch, k ? s_bits[k - 1] : st.tile_bits[tile - 1]);
+      const uint64_t b0 = (uint64_t)tile * NB;
+      // all of a thread's loads ahead of its stores
+      uint32_t at[PER];
 #pragma unroll
-      for (int j = 0; j < kWords; j++) {
-        const uint32_t i = 32 * j + lane;
-        uint32_t below = __shfl_up_sync(0xffffffffu, cur.w[j], 1);
-        if (lane == 0) below = last;
-        last = __shfl_sync(0xffffffffu, cur.w[j], 31);
-        if (i < full) dst[i] = __funnelshift_l(below, cur.w[j], o);
+      for (int j = 0; j < PER; j++) {
+        const uint64_t b = b0 + tid + j * kTileThreads;
+        at[j] = b < a.blocks ? st.warp_at[(uint64_t)tile * kTileWarps + (tid + j * kTileThreads) / (32 * PER)] + st.block_at[b] : 0u;
       }
+      constexpr int kWords = 2 * PER;                       // a step's words per thread
 #pragma unroll 1
-      for (uint32_t i0 = 32 * kWords; i0 < full; i0 += 32) {  // a string longer than most
-        const uint32_t i = i0 + lane, w = i < words ? src[i] : 0u;
-        uint32_t below = __shfl_up_sync(0xffffffffu, w, 1);
-        if (lane == 0) below = last;
-        last = __shfl_sync(0xffffffffu, w, 31);
-        if (i < full) dst[i] = __funnelshift_l(below, w, o);
-      }
-      uint64_t at = start;
+      for (uint32_t i = tid; i < full; i += kWords * kTileThreads) {
+        uint32_t below[kWords], here[kWords];
 #pragma unroll
-      for (int j = 0; j < kPer; j++) {
-        uint32_t y = cur.len[j];
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const uint32_t z = __shfl_up_sync(0xffffffffu, y, d);
-          if (lane >= d) y += z;
+        for (int j = 0; j < kWords; j++) {
+          const uint32_t k = i + j * kTileThreads;
+          below[j] = k == 0 ? prev : k - 1 < words ? src[k - 1] : 0u;
+          here[j] = k < words ? src[k] : 0u;
         }
-        if (lane + 32 * j < nb) block_bits[b0 + lane + 32 * j] = at + y - cur.len[j];
-        at += __shfl_sync(0xffffffffu, y, 31);
+#pragma unroll
+        for (int j = 0; j < kWords; j++)
+          if (i + j * kTileThreads < full) dst[i + j * kTileThreads] = __funnelshift_l(below[j], here[j], o);
       }
-      if (b0 + nb == a.blocks && lane == 0) {
+#pragma unroll
+      for (int j = 0; j < PER; j++) {
+        const uint64_t b = b0 + tid + j * kTileThreads;
+        if (b < a.blocks) block_bits[b] = start + at[j];
+      }
+      if (tile + 1 == a.tiles && tid == 0) {
         block_bits[a.blocks] = start + total;
-        close_stream(out, src, start, total, cur.q0);
+        close_stream(out, src, start, total, prev);
       }
-      cur = nxt;
     }
     base += all;
     __syncthreads();
@@ -427,16 +511,17 @@ place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restric
 // 1-D tables in shared memory: the lean coder's windows and nibble pairs, and one plane per lookup.
 // Before, with one plane per lookup throughout and a bit-matrix transpose per eight planes, 25.6 M values took: noise at
 // tolerance 1e-6 121 us (now 101), at 1e-3 95 (93), at 6 bits/value 117 (97); a random walk at 1e-6 218 (138).
-template <int DIM, bool BUDGET>
+template <int DIM, int PER, bool BUDGET>
 __global__ void __launch_bounds__(kTileThreads)
 decode_tiles_kernel(const uint32_t* __restrict__ in, float* __restrict__ out, const TileArgs a,
                     const uint64_t* __restrict__ block_bits, int shift, const uint16_t* __restrict__ plane_tab, const uint32_t* __restrict__ loop_tab) {
-  constexpr int kPer = TileShape<DIM>::kPer, WB = TileShape<DIM>::kWarpBlocks, NB = TileShape<DIM>::kBlocks;
+  constexpr int kPer = PER, WB = 32 * PER, NB = kTileThreads * PER;
   constexpr int kTabWords = DIM == 1 ? kTileDecTab1 : kRunTabSize;
   extern __shared__ __align__(16) uint32_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t* const words = smem + kTabWords + warp * a.warp_words;
   const uint32_t cap = a.slot_words;
+  pdl_trigger();
   if (DIM == 1) {
     for (int i = tid; i < 384; i += kTileThreads) reinterpret_cast<DecWindow*>(smem + kTileRows)[i] = make_tile_row(plane_tab, i);
     for (int i = tid; i < kDecTiny / 4; i += kTileThreads)   // windows and nibble pairs
@@ -445,6 +530,7 @@ decode_tiles_kernel(const uint32_t* __restrict__ in, float* __restrict__ out, co
     for (int i = tid; i < kRunTabSize / 4; i += kTileThreads) reinterpret_cast<uint4*>(smem)[i] = reinterpret_cast<const uint4*>(d_run.v)[i];
   }
   __syncthreads();
+  pdl_wait();
   for (uint32_t tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
     const uint64_t b0 = (uint64_t)tile * NB + warp * WB;
     if (b0 >= a.blocks) return;                             // tiles only grow
@@ -473,7 +559,7 @@ decode_tiles_kernel(const uint32_t* __restrict__ in, float* __restrict__ out, co
       const uint32_t pos = rel < (uint64_t)cap * 32 ? (uint32_t)rel : cap * 32;
       float f[1 << (2 * DIM)];
       if (DIM == 1) {
-        decode_window_1d(f, a.p, smem, plane_tab, words, pos, shift);
+        if (BUDGET || !decode_code_1d(f, a.p, smem, words, pos, shift)) decode_window_1d(f, a.p, smem, plane_tab, words, pos, shift);
         tile_store_1d(f, out, a, b0 + i);
       } else {
         decode_window_2d<BUDGET>(f, a.p, smem, words, pos, shift);
@@ -491,14 +577,13 @@ extern "C" int gcow_codec_tables4(const void** etab, const void** dtab, const vo
 
 namespace {
 
-template <int DIM> constexpr int blocks_per_tile() { return TileShape<DIM>::kBlocks; }
-
 TileArgs tile_args(const void* values, uint64_t nx, uint64_t ny, const ZfpParams& p, uint64_t blocks, int dim) {
   TileArgs a;
   a.nx = nx; a.ny = ny; a.blocks = blocks; a.p = p;
   a.bx = dim == 2 ? (uint32_t)((nx + 3) / 4) : 1;
   a.slot_words = a.warp_words = a.pitch = 0;
-  const uint64_t per = dim == 1 ? blocks_per_tile<1>() : blocks_per_tile<2>();
+  a.wide = 0;
+  const uint64_t per = (uint64_t)kTileThreads * tile_per(blocks, dim);
   a.tiles = (uint32_t)((blocks + per - 1) / per);
   const uintptr_t base = (uintptr_t)values;
   if (dim == 1) a.vec = (base & 15) == 0 ? 4 : 1;
@@ -507,42 +592,47 @@ TileArgs tile_args(const void* values, uint64_t nx, uint64_t ny, const ZfpParams
 }
 
 // Words of a warp's packed string or window.
-uint32_t warp_words_for(const ZfpParams& p, int dim) {
-  const uint32_t wb = dim == 1 ? TileShape<1>::kWarpBlocks : TileShape<2>::kWarpBlocks;
-  return (wb * max_block_bits(p, dim) + 31) / 32;
+uint32_t warp_words_for(const ZfpParams& p, uint64_t blocks, int dim) {
+  return tile_per(blocks, dim) * max_block_bits(p, dim);     // 32 blocks per unit of it
 }
-struct TileScratch { uint64_t strings, unit_bits, tile_bits, lens, bytes; };   // byte offsets
+struct TileScratch { uint64_t strings, warp_at, tile_bits, block_at, bytes; };   // byte offsets
 TileScratch tile_scratch(const ZfpParams& p, uint64_t blocks, int dim) {
-  const uint64_t wb = dim == 1 ? TileShape<1>::kWarpBlocks : TileShape<2>::kWarpBlocks;
-  const uint64_t units = (blocks + wb - 1) / wb, tiles = (units + kTileWarps - 1) / kTileWarps;
+  const uint64_t per = (uint64_t)kTileThreads * tile_per(blocks, dim), tiles = (blocks + per - 1) / per;
+  const uint64_t wb = per / kTileWarps, warps = (blocks + wb - 1) / wb;
   TileScratch t;
   t.tile_bits = 0;                                            // first: read 16 bytes at a time
   t.strings = (tiles * 4 + 15) & ~15ull;
-  t.unit_bits = t.strings + (blocks * max_block_bits(p, dim) + 31) / 32 * 4;
-  t.lens = t.unit_bits + units * 4;
-  t.bytes = t.lens + blocks * 2 + 16;                         // 16: the base is rounded up
+  t.warp_at = t.strings + (blocks * max_block_bits(p, dim) + 31) / 32 * 4;
+  t.block_at = t.warp_at + warps * 4;
+  t.bytes = t.block_at + blocks * 2 + 16;                     // 16: the base is rounded up
   return t;
 }
 constexpr uint32_t kPackedPad = 4;                            // the word after the string, and whole 16-byte rows
 constexpr uint32_t kReadAhead = kTileMaxBlockBits / 32 + 8;   // a block never reads further than this past its start
 uint32_t round4(uint32_t v) { return (v + 3) & ~3u; }
 
+// CTAs of a launch whose CTAs go through the tiles in steps of the grid: four times as many as are resident at once, by what
+// registers, threads and shared memory allow. A number between two multiples of that leaves the GPU nearly empty at the end
+// (2-D encoder, five per SM fit, six launched: a sixth of the work ran at one CTA per SM). Why four is said below.
 template <auto kKernel>
 int grid_of(uint32_t smem, uint32_t tiles, int* err) {
-  static std::atomic<uint64_t> allowed{0};                  // one bit per device: the large dynamic allocation is permitted
-  int dev = 0;
+  static std::atomic<int> held[64];                         // by device: CTAs per SM that registers and threads allow, 0: not asked yet
+  int dev = 0, most = 0;
   *err = (int)cudaGetDevice(&dev);
   if (*err) return 0;
-  if (dev >= 64 || !((allowed.load(std::memory_order_relaxed) >> dev) & 1)) {
+  if (dev < 64) most = held[dev].load(std::memory_order_relaxed);
+  if (!most) {
     *err = (int)cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (!*err) *err = (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&most, kKernel, kTileThreads, 0);
     if (*err) return 0;
-    if (dev < 64) allowed.fetch_or(1ull << dev, std::memory_order_relaxed);
+    if (most < 1) most = 1;
+    if (dev < 64) held[dev].store(most, std::memory_order_relaxed);
   }
-  // 228 KB of shared memory and 2048 threads per SM; more CTAs than fit would only queue
-  uint32_t per_sm = (228u * 1024) / (smem + 1024);
-  if (per_sm > 2048 / kTileThreads) per_sm = 2048 / kTileThreads;
-  if (per_sm < 1) per_sm = 1;
-  const uint32_t g = 148 * per_sm;
+  const int fit = (int)(228u * 1024 / (smem + 1280));       // shared memory of an SM; 1280: the system's 1 KB and static arrays
+  // Four CTAs per place: with one, every place takes the same number of tiles, and the last round of 25.6 M values at tolerance
+  // 1e-6 (7.03 tiles a place) stood almost empty: round trip 233 us, with two 216, three 212, four 212, eight 214; a 7654 x 7654
+  // field at 1e-3 297, 288, 284, 281, 279.
+  const uint32_t g = 4u * 148u * (uint32_t)(fit < 1 ? 1 : fit < most ? fit : most);
   return (int)(tiles < g ? tiles : g);
 }
 
@@ -620,32 +710,43 @@ int gcow_encode_tiles(const float* in, uint64_t nx, uint64_t ny, const int32_t* 
   const void *et, *dt, *pt, *lt;
   if (int rc = gcow_codec_tables4(&et, &dt, &pt, &lt)) return rc;
   TileArgs a = tile_args(in, nx, ny, p, blocks, dim);
+  const int per = tile_per(blocks, dim);
+  const bool cuts = tile_budget_cuts(p, dim);
+  const TileMode mode = !fixed ? kVariable : p.maxbits % 32 ? kPacked : kDirect;
   a.slot_words = tile_slot_words(p, dim);
-  a.warp_words = round4(warp_words_for(p, dim) + kPackedPad);
-  const uint32_t wb = dim == 1 ? TileShape<1>::kWarpBlocks : TileShape<2>::kWarpBlocks;
-  const uint32_t smem = ((dim == 1 ? kEncPairTabSize : kTwinTabSize) + kTileWarps * (a.slot_words * wb + wb + a.warp_words)) * 4;
+  a.warp_words = mode == kDirect ? 0 : round4(warp_words_for(p, blocks, dim) + kPackedPad);
+  a.wide = p.maxbits % 128 == 0 && ((uintptr_t)out & 15) == 0;
+  const uint32_t slots = mode == kVariable ? 32 : 32 * per;
+  const uint32_t smem = ((dim == 1 ? kEncPairTabSize : kTwinTabSize) + kTileWarps * (a.slot_words * slots + a.warp_words)) * 4;
   const TileScratch ts = tile_scratch(p, blocks, dim);
   char* const sp = (char*)(((uintptr_t)scratch + 15) & ~(uintptr_t)15);
-  a.pitch = wb / 32 * max_block_bits(p, dim);
+  a.pitch = kTileWarps * per * max_block_bits(p, dim);
   TileStrings st = {};
-  if (!fixed) st = {(uint32_t*)(sp + ts.strings), (uint32_t*)(sp + ts.unit_bits), (uint32_t*)(sp + ts.tile_bits), (uint16_t*)(sp + ts.lens)};
+  if (!fixed) st = {(uint32_t*)(sp + ts.strings), (uint32_t*)(sp + ts.tile_bits), (uint32_t*)(sp + ts.warp_at), (uint16_t*)(sp + ts.block_at)};
   int err = 0;
-#define GCOW_ENCODE(D, F, B)                                                                                   \
+#define GCOW_ENCODE(D, P, F, B)                                                                                \
   do {                                                                                                         \
-    const int g = grid_of<&encode_tiles_kernel<D, F, B>>(smem, a.tiles, &err);                                 \
+    const int g = grid_of<&encode_tiles_kernel<D, P, F, B>>(smem, a.tiles, &err);                              \
     if (err) return err;                                                                                       \
-    encode_tiles_kernel<D, F, B><<<g, kTileThreads, smem, s>>>(in, a, (uint32_t*)out, block_bits, st,         \
-                                                               (const uint16_t*)et, (const uint32_t*)pt);      \
+    launch_dependent(encode_tiles_kernel<D, P, F, B>, dim3(g), dim3(kTileThreads), smem, s, in, a, (uint32_t*)out, block_bits, st, \
+                     (const uint16_t*)et, (const uint32_t*)pt);                                                \
   } while (0)
-  const bool cuts = tile_budget_cuts(p, dim);
-  if (dim == 1) { if (fixed) GCOW_ENCODE(1, true, true); else GCOW_ENCODE(1, false, true); }
-  else if (fixed) { if (cuts) GCOW_ENCODE(2, true, true); else GCOW_ENCODE(2, true, false); }
-  else { if (cuts) GCOW_ENCODE(2, false, true); else GCOW_ENCODE(2, false, false); }
+#define GCOW_ENCODE_MODE(D, P, B)                                     \
+  do {                                                                \
+    if (mode == kVariable) GCOW_ENCODE(D, P, kVariable, B);           \
+    else if (mode == kPacked) GCOW_ENCODE(D, P, kPacked, B);          \
+    else GCOW_ENCODE(D, P, kDirect, B);                               \
+  } while (0)
+  if (dim == 1 && mode == kVariable && !cuts) { if (per == 4) GCOW_ENCODE(1, 4, kVariable, false); else GCOW_ENCODE(1, 1, kVariable, false); }
+  else if (dim == 1) { if (per == 4) GCOW_ENCODE_MODE(1, 4, true); else GCOW_ENCODE_MODE(1, 1, true); }
+  else if (cuts) GCOW_ENCODE_MODE(2, 1, true);
+  else GCOW_ENCODE_MODE(2, 1, false);
+#undef GCOW_ENCODE_MODE
 #undef GCOW_ENCODE
   if (!fixed) {
-    const uint32_t most = 148 * (dim == 1 ? 4 : 5), g = a.tiles < most ? a.tiles : most;
-    if (dim == 1) place_strings_kernel<1><<<g, kTileThreads, 0, s>>>(st, a, (uint32_t*)out, block_bits, total_out);
-    else place_strings_kernel<2><<<g, kTileThreads, 0, s>>>(st, a, (uint32_t*)out, block_bits, total_out);
+    const uint32_t most = 148 * 8, g = a.tiles < most ? a.tiles : most;
+    if (per == 4) launch_dependent(place_strings_kernel<4>, dim3(g), dim3(kTileThreads), 0, s, st, a, (uint32_t*)out, block_bits, total_out);
+    else launch_dependent(place_strings_kernel<1>, dim3(g), dim3(kTileThreads), 0, s, st, a, (uint32_t*)out, block_bits, total_out);
   }
   return (int)cudaGetLastError();
 }
@@ -664,19 +765,23 @@ int gcow_decode_tiles(const void* in, float* out, uint64_t nx, uint64_t ny, cons
   const void *et, *dt, *pt, *lt;
   if (int rc = gcow_codec_tables4(&et, &dt, &pt, &lt)) return rc;
   TileArgs a = tile_args(out, nx, ny, p, blocks, dim);
-  a.slot_words = warp_words_for(p, dim) + 1;                 // window capacity: one more for the bits before the first block
+  const int per = tile_per(blocks, dim);
+  const bool cuts = tile_budget_cuts(p, dim);
+  a.slot_words = warp_words_for(p, blocks, dim) + 1;                 // window capacity: one more for the bits before the first block
   a.warp_words = round4(a.slot_words + kReadAhead);
   const uint32_t smem = ((dim == 1 ? (uint32_t)kTileDecTab1 : (uint32_t)kRunTabSize) + kTileWarps * a.warp_words) * 4;
   int err = 0;
-#define GCOW_DECODE(D, B)                                                                                      \
+#define GCOW_DECODE(D, P, B)                                                                                      \
   do {                                                                                                         \
-    const int g = grid_of<&decode_tiles_kernel<D, B>>(smem, a.tiles, &err);                                    \
+    const int g = grid_of<&decode_tiles_kernel<D, P, B>>(smem, a.tiles, &err);                                 \
     if (err) return err;                                                                                       \
-    decode_tiles_kernel<D, B><<<g, kTileThreads, smem, s>>>((const uint32_t*)in, out, a, block_bits, shift, (const uint16_t*)dt, (const uint32_t*)lt); \
+    launch_dependent(decode_tiles_kernel<D, P, B>, dim3(g), dim3(kTileThreads), smem, s, (const uint32_t*)in, out, a, block_bits, shift, \
+                     (const uint16_t*)dt, (const uint32_t*)lt);                                                \
   } while (0)
-  if (dim == 1) GCOW_DECODE(1, true);
-  else if (tile_budget_cuts(p, 2)) GCOW_DECODE(2, true);
-  else GCOW_DECODE(2, false);
+  if (dim == 1 && per == 4) { if (cuts) GCOW_DECODE(1, 4, true); else GCOW_DECODE(1, 4, false); }
+  else if (dim == 1) { if (cuts) GCOW_DECODE(1, 1, true); else GCOW_DECODE(1, 1, false); }
+  else if (cuts) GCOW_DECODE(2, 1, true);
+  else GCOW_DECODE(2, 1, false);
 #undef GCOW_DECODE
   return (int)cudaGetLastError();
 }

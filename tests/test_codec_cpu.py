@@ -437,7 +437,7 @@ def test_lean_coders_under_the_accuracy_rule(bits, tol):
 
 
 @pytest.mark.parametrize("maxprec", [1, 3, 4, 8, 9, 16, 17, 31, 32])
-@pytest.mark.parametrize("maxbits", [9, 10, 17, 18, 31, 64, 105, 148])
+@pytest.mark.parametrize("maxbits", [9, 10, 17, 18, 31, 64, 105, 148])   # 148: no budget, the straight line too
 def test_window_decoder_of_the_tiles(maxprec, maxbits):
     """The decoder of the 1-D tile kernel and the plane-by-plane one on arbitrary bits (which cut planes and runs at
     every place), at every limit of planes and budget."""
@@ -494,6 +494,28 @@ def test_roundtrip_without_a_code(bits):
         x = np.ascontiguousarray(x, dtype=np.float32)
         assert lib.gcow_roundtrip_check(x.ctypes.data, n, bits, C.byref(left)) == 0, name
         assert name != "noise" or left.value < n // 500
+
+
+@pytest.mark.parametrize("par", [ZfpParams(1, 16658, 64, e) for e in (-1074, -40, -20, -10, 0)] + [ZfpParams(1, 16658, q, -1074) for q in (1, 2, 7, 8, 9, 15, 16, 17, 24, 25, 32)]
+                         + [ZfpParams(1, 40, 64, -20), ZfpParams(30, 16658, 64, -10), ZfpParams(1, 16658, 0, -1074)], ids=str)
+def test_1d_encoder_of_the_tiles(par):
+    """The register form of the 1-D tile encoder and the plane-by-plane one, and what the former leaves to the serial form: noise
+    only beyond sixteen verbatim planes, smooth data beyond sixteen planes with n < 3, special values."""
+    rng = np.random.default_rng(par.maxprec)
+    n = 20000
+    noise = rng.standard_normal((n, 4)).astype(np.float32)
+    scale = np.exp2(rng.integers(-28, 3, (n, 1))).astype(np.float32)
+    odd = noise.copy()
+    odd[::3, 1] = np.inf
+    odd[1::3, 2] = np.nan
+    odd[2::3] *= np.float32(1e-40)
+    left = C.c_uint64()
+    for name, x in dict(noise=noise * 1e-3, smooth=1 + noise * scale, same=np.repeat(noise[:, :1], 4, 1), sparse=np.where(noise > 1, noise, 0), zeros=noise * 0,
+                        magnitudes=noise * np.exp2(rng.integers(-140, 120, (n, 4))), odd=odd).items():
+        x = np.ascontiguousarray(x, dtype=np.float32)
+        assert lib.gcow_tile_1d_check(x.ctypes.data, n, par.as_c(), C.byref(left)) == 0, name
+        if par.maxbits > 144 and (name == "zeros" or name == "noise" and (par.maxprec <= 24 or par.minexp >= -20)):
+            assert left.value == 0, name
 
 
 def test_generic_scratch_holds_either_layout():

@@ -197,6 +197,24 @@ def test_tile_kernels_at_edges(dim, sizes, how):
                 assert torch.equal(a.view(torch.int32), b.view(torch.int32)), sz
 
 
+@pytest.mark.parametrize("blocks", [151552, 151553, 151552 + 1024, 148 * 6 * 4 * 1024 + 1025])
+@pytest.mark.parametrize("how", [dict(tolerance=1e-6), dict(tolerance=1e-2), dict(precision=2), dict(rate=6), dict(rate=8)])
+def test_tile_kernels_with_four_blocks_per_lane(blocks, how):
+    """The last size with one block per lane and the first ones with four, the first with more tiles than CTAs; strings whose
+    words belong to one block, to two, and (runs of 1-bit blocks) to many."""
+    n = 4 * blocks - 1
+    rng = np.random.default_rng(blocks)
+    x = (rng.standard_normal(n) * 1e-2).astype(np.float32)
+    x[n // 3: n // 2] = 0                                    # runs of 1-bit blocks, and some among the others
+    x[n // 2: n // 2 + 40_000: 7] = 0
+    x[-4000:] *= np.float32(1e-36)                           # denormals
+    x[5000::70_001] = np.inf
+    cpu = g.compress(torch.from_numpy(x), **how)
+    gpu = g.compress(dev(x), **how)
+    assert gpu.nbytes == cpu.nbytes and torch.equal(gpu.stream.cpu(), cpu.stream)
+    assert torch.equal(g.decompress(gpu).cpu().view(torch.int32), g.decompress(cpu).view(torch.int32))
+
+
 @pytest.mark.parametrize("rate", [2.25, 2.5, 2.75, 3])
 def test_decode_of_short_blocks(rate):
     """Blocks of 9 to 11 bits go to the kernel without staging, 12 bits and streams that are not word aligned to the tiles."""
