@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "zfp_block.cuh"
+#include "../ops/pdl.cuh"
 
 namespace gcow {
 
@@ -114,8 +115,10 @@ encode_1d_fixed_kernel(const float* __restrict__ in, uint64_t n, void* __restric
                        const uint16_t* __restrict__ tab, const uint32_t* __restrict__ pair_tab) {
   constexpr int NW = CodeIO<BITS>::NW;
   __shared__ __align__(16) uint32_t epair[kEncPairTabSize];
-  load_pair_table(epair, pair_tab);
+  pdl_trigger();
+  load_pair_table(epair, pair_tab);                          // under the tail of the stream's last kernel, like the launch itself
   __syncthreads();
+  pdl_wait();
   const LeanTables lt = {tab, nullptr, epair, nullptr};      // the plane-by-plane table is read from global memory (rare path)
   const uint64_t blocks = num_blocks_1d(n), stride = (uint64_t)gridDim.x * kRateThreads;
   if (blockIdx.x == 0 && threadIdx.x < pad_words16)          // the stream's last 64-bit word
@@ -154,8 +157,10 @@ decode_1d_fixed_kernel(const void* __restrict__ in, float* __restrict__ out, uin
                        int aligned, const uint16_t* __restrict__ tab, const uint32_t* __restrict__ loop_tab) {
   constexpr int NW = CodeIO<BITS>::NW;
   __shared__ __align__(16) uint32_t dloop[kDecLoopTabSize];
+  pdl_trigger();
   load_loop_table(dloop, loop_tab);
   __syncthreads();
+  pdl_wait();
   const LeanTables lt = {nullptr, tab, nullptr, dloop};      // the plane-by-plane table is read from global memory (rare path)
   const uint64_t blocks = num_blocks_1d(n), stride = (uint64_t)gridDim.x * kRateThreads;
   uint64_t b = (uint64_t)blockIdx.x * kRateThreads + threadIdx.x;
@@ -600,10 +605,10 @@ static int launch_encode_1d(const float* in, uint64_t n, int maxbits, void* out,
   const uint32_t* pt = (const uint32_t*)ptp;
   const int over = (int)(blocks * (uint64_t)maxbits % 64), pw = pad && over ? (64 - over) / 16 : 0;
   switch (maxbits) {
-    case 16: encode_1d_fixed_kernel<16><<<g, kRateThreads, 0, s>>>(in, n, out, aligned, pw, et, pt); break;
-    case 32: encode_1d_fixed_kernel<32><<<g, kRateThreads, 0, s>>>(in, n, out, aligned, pw, et, pt); break;
-    case 64: encode_1d_fixed_kernel<64><<<g, kRateThreads, 0, s>>>(in, n, out, aligned, pw, et, pt); break;
-    case 128: encode_1d_fixed_kernel<128><<<g, kRateThreads, 0, s>>>(in, n, out, aligned, pw, et, pt); break;
+    case 16: launch_dependent(encode_1d_fixed_kernel<16>, dim3(g), dim3(kRateThreads), 0, s, in, n, out, aligned, pw, et, pt); break;
+    case 32: launch_dependent(encode_1d_fixed_kernel<32>, dim3(g), dim3(kRateThreads), 0, s, in, n, out, aligned, pw, et, pt); break;
+    case 64: launch_dependent(encode_1d_fixed_kernel<64>, dim3(g), dim3(kRateThreads), 0, s, in, n, out, aligned, pw, et, pt); break;
+    case 128: launch_dependent(encode_1d_fixed_kernel<128>, dim3(g), dim3(kRateThreads), 0, s, in, n, out, aligned, pw, et, pt); break;
     default: return -1;
   }
   return (int)cudaGetLastError();
@@ -630,10 +635,10 @@ int gcow_decode_1d_fixed(const void* in, float* out, uint64_t n, int maxbits, in
   const uint32_t* lt = (const uint32_t*)ltp;
   const uint16_t* dt = (const uint16_t*)dtp;
   switch (maxbits) {
-    case 16: decode_1d_fixed_kernel<16><<<g, kRateThreads, 0, s>>>(in, out, n, shift, aligned, dt, lt); break;
-    case 32: decode_1d_fixed_kernel<32><<<g, kRateThreads, 0, s>>>(in, out, n, shift, aligned, dt, lt); break;
-    case 64: decode_1d_fixed_kernel<64><<<g, kRateThreads, 0, s>>>(in, out, n, shift, aligned, dt, lt); break;
-    case 128: decode_1d_fixed_kernel<128><<<g, kRateThreads, 0, s>>>(in, out, n, shift, aligned, dt, lt); break;
+    case 16: launch_dependent(decode_1d_fixed_kernel<16>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt); break;
+    case 32: launch_dependent(decode_1d_fixed_kernel<32>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt); break;
+    case 64: launch_dependent(decode_1d_fixed_kernel<64>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt); break;
+    case 128: launch_dependent(decode_1d_fixed_kernel<128>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt); break;
     default: return -1;
   }
   return (int)cudaGetLastError();
