@@ -27,6 +27,26 @@ def test_layernorm_fwd_bwd():
         assert (gb - b.grad).abs().max().item() < 0.02 * b.grad.abs().max().item() + 1e-2
 
 
+@pytest.mark.parametrize("H", [8, 248, 256, 264, 520, 776, 1024, 1032])
+@pytest.mark.parametrize("rows", [1, 5, 4001])
+def test_layernorm_rows_in_registers(H, rows):
+    """Widths around each number of register chunks and the last one with any; fewer rows than warps and several per warp."""
+    from gcow_b200.ops import kernels as K
+    torch.manual_seed(H + rows)
+    x = (torch.randn(rows, H, device="cuda") * 2 + 3).bfloat16()
+    g, b = torch.randn(H, device="cuda"), torch.randn(H, device="cuda")
+    y = K.layernorm(x, g, b, 1e-12)
+    xd = x.double()
+    r = (xd.var(1, unbiased=False, keepdim=True) + 1e-12).rsqrt()
+    n = (xd - xd.mean(1, keepdim=True)) * r
+    ref = n * g.double() + b.double()
+    # bf16 rounds to 2^-9; the mean of H fp32 values of size up to 12 is off by less than 12 (H + 5) 2^-24, which counts once for
+    # every value and once for the deviation
+    bound = 2.0 ** -8 * ref.abs() + 12 * (H + 5) * 2.0 ** -24 * r * (1 + n.abs()) * g.double().abs() + 1e-6
+    assert bool(((y.double() - ref).abs() <= bound).all())
+
+
+
 def test_gelu_fwd_bwd():
     from gcow_b200.ops import kernels as K
     x = (torch.randn(4096, 1024, device="cuda") * 2).requires_grad_(True)
