@@ -163,10 +163,6 @@ template <bool FWD> struct Shape {
   static constexpr int THREADS = FWD ? 384 : 512, REGS = FWD ? 168 : 128, ROW = FWD ? 208 : 184, ISSUE = FWD ? 88 : 72;
   static_assert(2 * ROW + (THREADS / 128 - 2) * ISSUE == THREADS / 128 * REGS && THREADS * REGS <= 65536, "setmaxnreg.inc waits for registers that must exist");
 };
-// In step, both tiles want the exponential units at the same time and leave them idle at the same time: B starts this late.
-__device__ __forceinline__ void stagger(int x) {
-  if (x) for (const long long from = clock64(); clock64() - from < 1200;) {}
-}
 template <bool FWD> __device__ __forceinline__ void regs_issue() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Shape<FWD>::ISSUE)); }
 template <bool FWD> __device__ __forceinline__ void regs_row() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Shape<FWD>::ROW)); }
 
@@ -321,7 +317,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     uint8_t* const stage = sO + warp * (32 * 128);           // the warp's 32 rows
     bool ok = true;
-    stagger(x);
     for (int u = u0; u < u1 && ok; u++) {
       const Unit un = unit_at(u, mode, tiles, heads);
       if (x == 1 && !un.both) continue;
@@ -677,7 +672,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     uint8_t* const stage = sO + warp * kStageWarpBytes;
     bool ok = true;
-    stagger(x);
     const uint64_t sl = tc::pack2(p.scale_log2, p.scale_log2), sc = tc::pack2(p.scale, p.scale);
     for (int u = u0, n = 0; u < u1 && ok; u++, n++) {
       const Unit un = unit_at(u, mode, tiles, heads);
