@@ -743,6 +743,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
               unpack2(mul2(mul2(tc::pack2(o[2], o[3]), add2(tc::pack2(__uint_as_float(dp[c][e + 2]), __uint_as_float(dp[c][e + 3])), d1)), sc), a, b);
               dk[c * 16 + e / 2 + 1] = pack2(a, b);
             }
+          if (!KV && i == nb - 1 && p.S < nb * STEP) {       // keys that do not exist: their score of 0 may be far above the row's
+            const int valid = (p.S - i * STEP) >> 1;         // others, their P beyond fp32
+#pragma unroll
+            for (int e = 0; e < 32; e++) if (e >= valid) dk[e] = 0;
+          }
           if (i) {                                           // the last block's P and dS have been read
             if (!(ok = wait_all(kAcc + x, 43))) break;
             tc_fence_after();

@@ -116,3 +116,32 @@ def test_attention_when_the_row_maximum_moves_between_key_blocks(S, order):
     assert _rel(o, (w @ v).permute(0, 2, 1, 3).reshape(5, S, 128)) < 2 ** -8
     dv = w.transpose(-1, -2) @ go.double().view(5, S, 2, 64).permute(0, 2, 1, 3)
     assert _rel(qkv.grad[:, :, 2], dv.permute(0, 2, 1, 3)) < 2 ** -8
+
+
+@pytest.mark.parametrize("S", [72, 200, 376, 504])
+def test_attention_of_rows_far_below_zero(S):
+    """A shift of a row's scores does not change its softmax. A component that all keys have puts every scaled score near -150:
+    against such a row's log-sum-exp, the zero score of a key that does not exist would be a probability beyond fp32."""
+    from gcow_b200.ops import kernels as K
+    torch.manual_seed(S)
+    B, H = 3, 2
+    qkv = torch.randn(B, S, 3, H, 64, device="cuda")
+    qkv[:, :, 0, :, 0] = 40
+    qkv[:, :, 1, :, 0] = -30
+    qkv = qkv.bfloat16().requires_grad_(True)
+    o = K.fused_attention(qkv)
+    go = torch.randn_like(o)
+    o.backward(go)
+    K.check_errors()
+    q, k, v = (qkv.detach().double()[:, :, i].permute(0, 2, 1, 3) for i in range(3))
+    d = go.double().view(B, S, H, 64).permute(0, 2, 1, 3)
+    p = torch.softmax(q @ k.transpose(-1, -2) / 8, -1)
+    ref = p @ v
+    ds = p * (d @ v.transpose(-1, -2) - (d * ref).sum(-1, keepdim=True)) / 8
+    # P, dS and every result are rounded to bf16 (2^-9 each); so is the output, whose error comes into dS by way of delta
+    e = ds.abs() + p * (d.abs() * ref.abs()).sum(-1, keepdim=True) / 8
+    got = [o.detach().view(B, S, H, 64)] + [qkv.grad[:, :, i] for i in range(3)]
+    want = [(ref, p @ v.abs()), (ds @ k, e @ k.abs()), (ds.transpose(-1, -2) @ q, e.transpose(-1, -2) @ q.abs()),
+            (p.transpose(-1, -2) @ d, p.transpose(-1, -2) @ d.abs())]
+    for x, (r, size) in zip(got, want):
+        assert bool(((x.double().permute(0, 2, 1, 3) - r).abs() <= 2.0 ** -8 * (size + r.abs())).all())
