@@ -121,6 +121,10 @@ inline void* raw(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr;
 inline Tensor bf16_rows(const Tensor& t) {                  // contiguous bf16, copied only where it is not
   return (t.scalar_type() == at::kBFloat16 ? t : t.to(at::kBFloat16)).contiguous();
 }
+inline Tensor bf16_rows16(const Tensor& t) {                // and from a 16-byte boundary on, as the tensor maps want it
+  const Tensor r = bf16_rows(t);
+  return (uintptr_t)r.data_ptr() & 15 ? r.clone(at::MemoryFormat::Contiguous) : r;
+}
 inline Tensor float_vector(const Tensor& t) {
   return !t.defined() ? t : (t.scalar_type() == at::kFloat ? t : t.to(at::kFloat)).contiguous();
 }
@@ -613,7 +617,7 @@ struct FusedAttentionNode : LayerNode {                     // input: qkv
     const Tensor &q = had[0], &o = had[1], &lse = had[2];
     const On on(q);
     const int B = (int)q.size(0), S = (int)q.size(1), H = (int)q.size(3), D = (int)q.size(4);
-    const Tensor g = bf16_rows(in[0]);
+    const Tensor g = bf16_rows16(in[0]);
     Tensor dqkv = at::empty_like(q);
     const Tensor delta = empty({B, H, S}, at::kFloat, q);
     check(gcow_attention_bwd(q.data_ptr(), o.data_ptr(), g.data_ptr(), f32(lse), f32(delta), dqkv.data_ptr(), B, S, H, D, scale, on.error,
@@ -638,7 +642,7 @@ PyObject* fused_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) { 
     Below below;
     const On on(qkv);
     const int64_t B = qkv.size(0), S = qkv.size(1), H = qkv.size(3), D = qkv.size(4);
-    const Tensor q = bf16_rows(qkv);
+    const Tensor q = bf16_rows16(qkv);
     out = empty({B, S, H * D}, at::kBFloat16, q);
     const Tensor lse = empty({B, H, S}, at::kFloat, q);
     check(gcow_attention_fwd(q.data_ptr(), out.data_ptr(), f32(lse), (int)B, (int)S, (int)H, (int)D, (float)scale, on.error, on.stream),

@@ -145,3 +145,23 @@ def test_attention_of_rows_far_below_zero(S):
             (p.transpose(-1, -2) @ d, p.transpose(-1, -2) @ d.abs())]
     for x, (r, size) in zip(got, want):
         assert bool(((x.double().permute(0, 2, 1, 3) - r).abs() <= 2.0 ** -8 * (size + r.abs())).all())
+
+
+@pytest.mark.parametrize("S", [72, 128])
+def test_attention_of_tensors_at_odd_addresses(S):
+    """Contiguous projections and gradients that do not start on 16 bytes are copied, not refused."""
+    from gcow_b200.ops import nn as gnn
+    torch.manual_seed(S)
+    x = torch.randn(2, S, 3, 2, 64, device="cuda").bfloat16()
+    go = torch.randn(2, S, 128, device="cuda").bfloat16()
+
+    def run(qkv, g):
+        qkv = qkv.requires_grad_(True)
+        o = gnn.attention(qkv)
+        o.backward(g)
+        return o.detach(), qkv.grad
+
+    def odd(t):
+        return torch.cat((t.new_zeros(1), t.reshape(-1)))[1:].view(t.shape)
+    for a, b in zip(run(x.clone(), go), run(odd(x), odd(go))):
+        assert torch.equal(a, b)
