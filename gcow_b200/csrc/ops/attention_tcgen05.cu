@@ -491,11 +491,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
 
   if (tid == 0) {
     // 4: the warps of a tile, 8: all row warps, 32: the warp that fetches statistics; a sequence that two tiles share is free
-    // when both have used it, a tile's operands when each warp that reads them has
+    // when both have used it, a tile's operands when each warp that reads them has. For dK/dV tile B's score warp counts beside
+    // its accumulator warp: where there is no tile B neither waits for the other, and a block refilled before one of
+    // them has looked would be a phase that it misses.
     for (int i = 0; i < kBwdBars; i++) {
       const int pair = i & ~1;
       mbar_init(&bs->bar[i], pair == kSGone || pair == kReady ? 4 : pair == kStatFree ? 8 : pair == kStatFull ? 32
-                             : (KV && pair == kAFree) || (i >= kBFree && i < kStatFull && mode == kPair) ? 2 : 1);
+                             : i >= kBFree && i < kStatFull && mode == kPair ? (KV ? 3 : 2) : KV && pair == kAFree ? 2 : 1);
     }
     for (int i = 0; i < 4; i++) mbar_init(&bs->drain[i], 1);
     bs->abort = 0;
@@ -571,11 +573,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
 #pragma unroll 1
             for (int i = 0; i < tiles && ok; i++) {          // each warp waits for what it waits for in the other units
               if (scores) wait(kBFull + i, 32);
-              if (scores != KV) {
-                wait(kBFull + 4 + i, 32);
-                if (ok && lane == 0) mbar_arrive(&bs->bar[kBFree + i]);
-                __syncwarp();
-              }
+              if (scores != KV) wait(kBFull + 4 + i, 32);
+              if (ok && lane == 0) mbar_arrive(&bs->bar[kBFree + i]);
+              __syncwarp();
             }
           continue;
         }
@@ -587,6 +587,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
             if (!(i & 1)) {
               wait(kBFull + sl, 34);
               if (!KV) wait(kBFull + 4 + sl, 34);
+              if (KV && x && mode == kPair && ok && lane == 0) mbar_arrive(&bs->bar[kBFree + sl]);   // it is in use until the accumulators' products
             }
             if (held) wait(kSGone + x, 35);
             held = true;

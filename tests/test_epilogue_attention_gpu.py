@@ -76,9 +76,9 @@ def test_attention(B, S, H):
         assert _rel(qkv.grad[:, :, i], r.grad[:, :, i]) < 2 ** -8
 
 
-@pytest.mark.parametrize("B,S,H", [(99, 128, 3), (331, 128, 1), (120, 384, 2), (80, 512, 2), (75, 256, 4)])
+@pytest.mark.parametrize("B,S,H", [(99, 128, 3), (331, 128, 1), (120, 384, 2), (80, 512, 2), (75, 256, 4), (148, 264, 6), (37, 384, 28)])
 def test_attention_with_several_units_per_cta(B, S, H):
-    """Two tiles per unit (of one head, of two heads, the last one alone) and more units than SMs."""
+    """Two tiles per unit (of one head, of two heads, the last one alone, in long turns with pairs) and more units than SMs."""
     test_attention(B, S, H)
 
 
