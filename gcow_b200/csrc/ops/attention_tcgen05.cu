@@ -1,7 +1,7 @@
 // Fused multi-head self-attention on the 5th-generation tensor cores (sm_100a), head dimension 64, 72 to 512 positions (a
 // multiple of 8), no mask, no dropout: forward and backward.
 //
-// All three kernels read the packed projection qkv [B][S][3][H][64] (bf16) in place through 4-D tensor maps {d, h, s, b} - a
+// The kernels read the packed projection qkv [B][S][3][H][64] (bf16) in place through 4-D tensor maps {d, h, s, b} - a
 // box is 128 sequence positions of one head, 128-byte rows with the 128-byte swizzle - and write the context / gradients in
 // the layouts the neighbouring GEMMs use ([B][S][H][64] and [B][S][3][H][64]), so no transposed copy of Q, K or V exists.
 //
@@ -121,7 +121,7 @@ __device__ __forceinline__ Unit unit_at(int u, int mode, int tiles, int heads) {
 //
 // B 32, S 512, 16 heads: forward 123 us with one tile in flight and the probabilities through shared memory, now 67 (0.51
 // PFLOP/s; the 134 M exponentials take 29 at 16 a clock and SM); backward 327, now 225 (delta 15, the rest 0.57 PFLOP/s;
-// 251 with one issuing warp per tile in the backward pass, 242 before dQ could start beside dK/dV). One sequence of 512:
+// 251 with one issuing warp per tile in the backward pass, 242 with dQ behind dK/dV). One sequence of 512:
 // backward 35 us, now 30.
 //
 // What the issuing warps do per product decides the pace. As code of one thread alone, with the descriptors worked out where
@@ -471,10 +471,8 @@ struct BwdBars {
 // KV = false: a tile is 128 queries, the loop runs over blocks of 64 keys: S = Q K^T, dP = dO V^T, dQ += dS K.
 // a1, a2: the tile's operands (K, V or Q, dO); b1, b2: those of the whole sequence (Q, dO or K, V); to1, to2: dV, dK or -, dQ.
 template <bool KV>
-__global__ void __launch_bounds__(Shape<false>::THREADS, 1)
-attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__ CUtensorMap ta2, const __grid_constant__ CUtensorMap tb1,
-                const __grid_constant__ CUtensorMap tb2, const __grid_constant__ CUtensorMap to1, const __grid_constant__ CUtensorMap to2,
-                const Params p, int units, int mode) {
+__device__ __forceinline__ void attn_bwd_body(const CUtensorMap& ta1, const CUtensorMap& ta2, const CUtensorMap& tb1, const CUtensorMap& tb2,
+                                              const CUtensorMap& to1, const CUtensorMap& to2, const Params& p, int units, int mode, int cta, int ctas) {
   constexpr int STEP = 64, STEP_BYTES = STEP * D * 2;
   extern __shared__ uint8_t raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
@@ -486,7 +484,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
   BwdBars* const bs = reinterpret_cast<BwdBars*>(stats + 4 * MAX_S);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // warp: uniform
   const int tiles = (p.S + TILE - 1) / TILE, heads = p.B * p.H;
-  const int u0 = (int)((long long)units * blockIdx.x / gridDim.x), u1 = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
+  const int u0 = (int)((long long)units * cta / ctas), u1 = (int)((long long)units * (cta + 1) / ctas);
   const int nb = (p.S + STEP - 1) / STEP;
 
   if (tid == 0) {
@@ -508,9 +506,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bs->tmem_base;
-  // The two kernels read the same and write apart, so dQ need not wait for dK/dV: that one lets it start when what both read is
-  // there. A grid that leaves SMs idle, and the end of every grid, is filled so. dQ ends only after dK/dV, for what follows it.
-  if (KV) pdl_wait();
+  pdl_wait();
   pdl_trigger();
   // Columns of a tile: S 64, dP 64, two accumulators of 64. P and dS (32 each, bf16) take dP's place once it has been read; with
   // one accumulator dS has a place of its own, and dP can be refilled at once.
@@ -791,7 +787,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap ta1, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_free_all(tmem);
-  if (!KV) pdl_wait();
+}
+
+// Both in one launch, dK/dV on the first half of the CTAs, dQ on the other: they read the same and write apart, so neither waits
+// for the other. A grid that leaves SMs idle, and the end of dK/dV, is filled with dQ's CTAs.
+__global__ void __launch_bounds__(Shape<false>::THREADS, 1)
+attn_bwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
+                const __grid_constant__ CUtensorMap tdo, const __grid_constant__ CUtensorMap tdq, const __grid_constant__ CUtensorMap tdk,
+                const __grid_constant__ CUtensorMap tdv, const Params p, int units, int mode) {
+  const int ctas = (int)gridDim.x / 2, cta = (int)blockIdx.x;
+  if (cta < ctas) attn_bwd_body<true>(tk, tv, tq, tdo, tdv, tdk, p, units, mode, cta, ctas);
+  else attn_bwd_body<false>(tq, tdo, tk, tv, tdq, tdq, p, units, mode, cta - ctas, ctas);
 }
 
 // ------------------------------------------------------------------------------ host side
@@ -822,7 +828,7 @@ constexpr size_t kBwdSmem = TILE_BYTES * 13 + MAX_S * 16 + sizeof(BwdBars) + 102
 static_assert(kFwdSmem <= 227 * 1024 && kBwdSmem <= 227 * 1024, "one CTA per SM");
 
 // Two tiles per CTA share the sequence's operands, and each keeps the arithmetic units busy while the other one waits for a
-// product; where there are no more tiles than SMs (two kernels share them in the backward pass) each has an SM to itself.
+// product; where there are no more tiles than SMs (dK/dV and dQ share them in the backward pass) each has an SM to itself.
 static int plan_units(int B, int S, int H, int sms, int* mode, int* units) {
   const long long heads = (long long)B * H, tiles = (S + TILE - 1) / TILE;
   *mode = heads * tiles <= sms ? kSingle : tiles == 1 ? kHeads : kPair;
@@ -842,8 +848,7 @@ static void set_attrs() {
   static std::once_flag once;
   std::call_once(once, [] {
     cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwdSmem);
-    cudaFuncSetAttribute(attn_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwdSmem);
-    cudaFuncSetAttribute(attn_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwdSmem);
+    cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwdSmem);
   });
 }
 
@@ -894,9 +899,8 @@ int gcow_attention_bwd(const void* qkv, const void* out, const void* dout, const
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.error = error;
   const size_t rows = (size_t)B * S * H;
   gcow::launch_dependent(attn_delta_kernel, dim3((unsigned)((rows * 8 + 255) / 256)), dim3(256), 0, st, (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, delta, B, S, H);
-  const dim3 grid(units < 148 ? units : 148);
-  gcow::launch_dependent(attn_bwd_kernel<true>, grid, dim3(Shape<false>::THREADS), kBwdSmem, st, in[1], in[2], in[0], in[3], dv, dk, p, units, mode);
-  gcow::launch_dependent(attn_bwd_kernel<false>, grid, dim3(Shape<false>::THREADS), kBwdSmem, st, in[0], in[3], in[1], in[2], dq, dq, p, units, mode);
+  gcow::launch_dependent(attn_bwd_kernel, dim3(2 * (units < 148 ? units : 148)), dim3(Shape<false>::THREADS), kBwdSmem, st, in[0], in[1], in[2], in[3],
+                         dq, dk, dv, p, units, mode);
   return (int)cudaGetLastError();
 }
 

@@ -622,7 +622,7 @@ struct FusedAttentionNode : LayerNode {                     // input: qkv
     const Tensor delta = empty({B, H, S}, at::kFloat, q);
     check(gcow_attention_bwd(q.data_ptr(), o.data_ptr(), g.data_ptr(), f32(lse), f32(delta), dqkv.data_ptr(), B, S, H, D, scale, on.error,
                              on.stream), "gcow_attention_bwd");
-    g_launches += 3;
+    g_launches += 2;
     out[0] = std::move(dqkv);
     return out;
   }
