@@ -50,12 +50,12 @@ __device__ __forceinline__ void load_loop_table(uint32_t* dloop, const uint32_t*
 }
 
 // Load block b of a 1-D array of n floats (tail block padded).
-__device__ __forceinline__ void load_block_1d(float* f, const float* __restrict__ in, uint64_t n,
+__device__ __forceinline__ void load_block_1d(float* f, const float* in, uint64_t n,
                                               uint64_t b, bool aligned) {
   uint64_t x0 = 4 * b;
   if (x0 + 4 <= n) {
     if (aligned) {
-      float4 v = __ldg(reinterpret_cast<const float4*>(in) + b);
+      float4 v = reinterpret_cast<const float4*>(in)[b];
       f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
     } else {
       f[0] = in[x0]; f[1] = in[x0 + 1]; f[2] = in[x0 + 2]; f[3] = in[x0 + 3];
@@ -111,7 +111,7 @@ constexpr int kEncodeCtas = 3, kDecodeCtas = 4;
 
 template <int BITS>
 __global__ void __launch_bounds__(kRateThreads, kEncodeCtas)
-encode_1d_fixed_kernel(const float* __restrict__ in, uint64_t n, void* __restrict__ out, int aligned, int pad_words16,
+encode_1d_fixed_kernel(const float* in, uint64_t n, void* __restrict__ out, int aligned, int pad_words16,
                        const uint16_t* __restrict__ tab, const uint32_t* __restrict__ pair_tab) {
   constexpr int NW = CodeIO<BITS>::NW;
   __shared__ __align__(16) uint32_t epair[kEncPairTabSize];
@@ -131,7 +131,7 @@ encode_1d_fixed_kernel(const float* __restrict__ in, uint64_t n, void* __restric
     bool ok[kAhead];
 #pragma unroll
     for (int i = 0; i < kAhead; i++) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(in) + b + i * stride);
+      const float4 v = reinterpret_cast<const float4*>(in)[b + i * stride];
       f[i][0] = v.x; f[i][1] = v.y; f[i][2] = v.z; f[i][3] = v.w;
     }
 #pragma unroll
@@ -153,7 +153,7 @@ encode_1d_fixed_kernel(const float* __restrict__ in, uint64_t n, void* __restric
 
 template <int BITS>
 __global__ void __launch_bounds__(kRateThreads, 2)      // 32 registers without being forced; forced, 95 instead of 91 us
-decode_1d_fixed_kernel(const void* __restrict__ in, float* __restrict__ out, uint64_t n, int shift,
+decode_1d_fixed_kernel(const void* in, float* __restrict__ out, uint64_t n, int shift,
                        int aligned, const uint16_t* __restrict__ tab, const uint32_t* __restrict__ loop_tab) {
   constexpr int NW = CodeIO<BITS>::NW;
   __shared__ __align__(16) uint32_t dloop[kDecLoopTabSize];

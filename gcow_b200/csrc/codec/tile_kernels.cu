@@ -47,15 +47,15 @@ struct TileArgs {
   int vec;                        // 2-D: values per load that the row pitch and the base address allow (4, 2 or 1); 1-D: 4 or 1
 };
 
-__device__ __forceinline__ void tile_load_1d(float* f, const float* __restrict__ in, const TileArgs& a, uint64_t b) {
+__device__ __forceinline__ void tile_load_1d(float* f, const float* in, const TileArgs& a, uint64_t b) {
   const uint64_t x0 = 4 * b;
   if (x0 + 4 <= a.nx) {
     if (a.vec == 4) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(in) + b);
+      const float4 v = reinterpret_cast<const float4*>(in)[b];
       f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
     } else {
 #pragma unroll
-      for (int i = 0; i < 4; i++) f[i] = __ldg(in + x0 + i);
+      for (int i = 0; i < 4; i++) f[i] = in[x0 + i];
     }
   } else {
     const uint32_t c = (uint32_t)(a.nx - x0);
@@ -77,7 +77,7 @@ __device__ __forceinline__ void tile_store_1d(const float* f, float* __restrict_
     for (uint64_t i = 0; x0 + i < a.nx; i++) out[x0 + i] = f[i];
   }
 }
-__device__ __forceinline__ void tile_load_2d(float* f, const float* __restrict__ in, const TileArgs& a, uint64_t b) {
+__device__ __forceinline__ void tile_load_2d(float* f, const float* in, const TileArgs& a, uint64_t b) {
   const uint64_t by = a.blocks <= 0xffffffffull ? (uint64_t)((uint32_t)b / a.bx) : b / a.bx;
   const uint64_t x0 = 4 * (b - by * a.bx), y0 = 4 * by;
   const float* src = in + y0 * a.nx + x0;
@@ -85,21 +85,21 @@ __device__ __forceinline__ void tile_load_2d(float* f, const float* __restrict__
     if (a.vec == 4) {
 #pragma unroll
       for (int y = 0; y < 4; y++) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(src + y * a.nx));
+        const float4 v = *reinterpret_cast<const float4*>(src + y * a.nx);
         f[4 * y] = v.x; f[4 * y + 1] = v.y; f[4 * y + 2] = v.z; f[4 * y + 3] = v.w;
       }
     } else if (a.vec == 2) {
 #pragma unroll
       for (int y = 0; y < 4; y++) {
-        const float2 v = __ldg(reinterpret_cast<const float2*>(src + y * a.nx));
-        const float2 w = __ldg(reinterpret_cast<const float2*>(src + y * a.nx + 2));
+        const float2 v = *reinterpret_cast<const float2*>(src + y * a.nx);
+        const float2 w = *reinterpret_cast<const float2*>(src + y * a.nx + 2);
         f[4 * y] = v.x; f[4 * y + 1] = v.y; f[4 * y + 2] = w.x; f[4 * y + 3] = w.y;
       }
     } else {
 #pragma unroll
       for (int y = 0; y < 4; y++)
 #pragma unroll
-        for (int x = 0; x < 4; x++) f[4 * y + x] = __ldg(src + y * a.nx + x);
+        for (int x = 0; x < 4; x++) f[4 * y + x] = src[y * a.nx + x];
     }
     return;
   }
@@ -241,7 +241,7 @@ enum TileMode { kVariable, kPacked, kDirect };              // variable rate; fi
 
 template <int DIM, int PER, TileMode MODE, bool BUDGET>
 __global__ void __launch_bounds__(kTileThreads)
-encode_tiles_kernel(const float* __restrict__ in, const TileArgs a, uint32_t* __restrict__ out, uint64_t* __restrict__ block_bits,
+encode_tiles_kernel(const float* in, const TileArgs a, uint32_t* __restrict__ out, uint64_t* __restrict__ block_bits,
                     const TileStrings st, const uint16_t* __restrict__ enc_tab, const uint32_t* __restrict__ pair_tab) {
   constexpr int WB = 32 * PER, NB = kTileThreads * PER;
   constexpr int kTabWords = DIM == 1 ? kEncPairTabSize : kTwinTabSize;
@@ -513,8 +513,8 @@ place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restric
 // tolerance 1e-6 121 us (now 101), at 1e-3 95 (93), at 6 bits/value 117 (97); a random walk at 1e-6 218 (138).
 template <int DIM, int PER, bool BUDGET>
 __global__ void __launch_bounds__(kTileThreads)
-decode_tiles_kernel(const uint32_t* __restrict__ in, float* __restrict__ out, const TileArgs a,
-                    const uint64_t* __restrict__ block_bits, int shift, const uint16_t* __restrict__ plane_tab, const uint32_t* __restrict__ loop_tab) {
+decode_tiles_kernel(const uint32_t* in, float* __restrict__ out, const TileArgs a,
+                    const uint64_t* block_bits, int shift, const uint16_t* __restrict__ plane_tab, const uint32_t* __restrict__ loop_tab) {
   constexpr int kPer = PER, WB = 32 * PER, NB = kTileThreads * PER;
   constexpr int kTabWords = DIM == 1 ? kTileDecTab1 : kRunTabSize;
   extern __shared__ __align__(16) uint32_t smem[];
@@ -548,7 +548,7 @@ decode_tiles_kernel(const uint32_t* __restrict__ in, float* __restrict__ out, co
     const uint32_t* const src = in + w0;
     __syncwarp();
 #pragma unroll 4
-    for (uint32_t i = lane; i < nw; i += 32) words[i] = __ldg(src + i);
+    for (uint32_t i = lane; i < nw; i += 32) words[i] = src[i];
     if (lane < 4) words[nw + lane] = 0;
     __syncwarp();
 #pragma unroll 1

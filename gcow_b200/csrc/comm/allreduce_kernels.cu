@@ -168,7 +168,7 @@ template <> struct Code<128> {
   static __device__ __forceinline__ void ld(const void* base, uint64_t b, uint32_t (&w)[4]) { uint4 v = __ldcg((const uint4*)base + b); w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w; }
 };
 
-__device__ __forceinline__ void load_block(float* f, const float* __restrict__ in, uint64_t n, uint64_t gb, bool aligned) {
+__device__ __forceinline__ void load_block(float* f, const float* in, uint64_t n, uint64_t gb, bool aligned) {
   uint64_t x0 = 4 * gb;
   if (x0 + 4 <= n) {
     if (aligned) { float4 v = reinterpret_cast<const float4*>(in)[gb]; f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w; }

@@ -430,7 +430,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
 
 // delta[b][h][s] = sum_d dO[b][s][h][d] * O[b][s][h][d]; eight lanes per row, so that a warp reads whole lines (262 144
 // rows: 15 us, one thread per row took 24).
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ go,
+__global__ void attn_delta_kernel(const __nv_bfloat16* o, const __nv_bfloat16* go,
                                   float* __restrict__ delta, int B, int S, int H) {
   pdl_trigger();
   pdl_wait();

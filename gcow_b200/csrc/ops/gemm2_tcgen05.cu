@@ -292,12 +292,12 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           if (wide_bias) {                                 // n is a multiple of 32
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
-              const float4 b = __ldg(reinterpret_cast<const float4*>(p.bias + n + j));
+              const float4 b = *reinterpret_cast<const float4*>(p.bias + n + j);
               v[j] += b.x; v[j + 1] += b.y; v[j + 2] += b.z; v[j + 3] += b.w;
             }
           } else {
 #pragma unroll
-            for (int j = 0; j < 32; j++) v[j] += __ldg(p.bias + n + j);
+            for (int j = 0; j < 32; j++) v[j] += p.bias[n + j];
           }
         }
         if (p.flags & kAuxOut) warp_store_rows_bf16(stg, lane, v, p.aux, off, row_ok);

@@ -89,7 +89,7 @@ layernorm_fwd_kernel(const bf16* __restrict__ x, const float* __restrict__ gamma
 // the warp (16384 x 1024: 19.3 us, now 16.8; 67 MB take 10).
 template <int CH>
 __global__ void __launch_bounds__(128)
-layernorm_fwd_rows_kernel(const bf16* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
+layernorm_fwd_rows_kernel(const bf16* x, const float* gamma, const float* beta,
                           bf16* __restrict__ y, float* __restrict__ mean, float* __restrict__ rstd, int rows, int H, float eps) {
   pdl_wait();
   pdl_trigger();
