@@ -86,9 +86,10 @@ layernorm_fwd_kernel(const bf16* __restrict__ x, const float* __restrict__ gamma
 
 // The same for H <= 256 * CH: a row stays in registers (CH chunks of 8 values per lane) and the next one is on its way while
 // this one is worked on. The form above reads a row three times, each time behind a reduction across
-// the warp (16384 x 1024: 19.3 us, now 16.8; 67 MB take 10).
+// the warp (16384 x 1024: 16.8 us, now 14.6; 67 MB take 10).
+template <int CH> constexpr int kRowCtas = CH == 1 ? 10 : CH == 2 ? 9 : CH == 3 ? 8 : 6;   // CTAs per SM, as the registers allow: the grid
 template <int CH>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, kRowCtas<CH>)
 layernorm_fwd_rows_kernel(const bf16* x, const float* gamma, const float* beta,
                           bf16* __restrict__ y, float* __restrict__ mean, float* __restrict__ rstd, int rows, int H, float eps) {
   pdl_wait();
@@ -524,16 +525,17 @@ extern "C" {
 int gcow_layernorm_fwd(const void* x, const float* gamma, const float* beta, void* y, float* mean, float* rstd,
                        int rows, int H, float eps, void* stream) {
   if (H % 8 || rows <= 0) return -1;
-  int grid = (rows + 3) / 4;
-  const int most = 148 * (H <= 1024 ? 6 : 16);              // six CTAs of the row kernel are resident
-  if (grid > most) grid = most;
-#define GCOW_LN_FWD(K) gcow::launch_dependent(K, dim3(grid), dim3(128), 0, (cudaStream_t)stream, (const bf16*)x, gamma, beta, (bf16*)y, mean, rstd, rows, H, eps)
+  const int want = (rows + 3) / 4;
+#define GCOW_LN_FWD(K, CTAS) gcow::launch_dependent(K, dim3(want < 148 * (CTAS) ? want : 148 * (CTAS)), dim3(128), 0, (cudaStream_t)stream, \
+                                                    (const bf16*)x, gamma, beta, (bf16*)y, mean, rstd, rows, H, eps)
+  // As many CTAs as are resident: with six for every width, which is the widest rows' number, 65536 x 128 took 22.7 us (now 14.6), x
+  // 256 25.1 (16.1), x 512 38.8 (28.0), x 768 51.0 (39.5); x 1024 51.6 as before.
   switch ((H + 255) / 256) {
-    case 1: GCOW_LN_FWD(layernorm_fwd_rows_kernel<1>); break;
-    case 2: GCOW_LN_FWD(layernorm_fwd_rows_kernel<2>); break;
-    case 3: GCOW_LN_FWD(layernorm_fwd_rows_kernel<3>); break;
-    case 4: GCOW_LN_FWD(layernorm_fwd_rows_kernel<4>); break;
-    default: GCOW_LN_FWD(layernorm_fwd_kernel); break;
+    case 1: GCOW_LN_FWD(layernorm_fwd_rows_kernel<1>, kRowCtas<1>); break;
+    case 2: GCOW_LN_FWD(layernorm_fwd_rows_kernel<2>, kRowCtas<2>); break;
+    case 3: GCOW_LN_FWD(layernorm_fwd_rows_kernel<3>, kRowCtas<3>); break;
+    case 4: GCOW_LN_FWD(layernorm_fwd_rows_kernel<4>, kRowCtas<4>); break;
+    default: GCOW_LN_FWD(layernorm_fwd_kernel, 16); break;
   }
 #undef GCOW_LN_FWD
   return (int)cudaGetLastError();

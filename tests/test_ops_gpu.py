@@ -28,7 +28,7 @@ def test_layernorm_fwd_bwd():
 
 
 @pytest.mark.parametrize("H", [8, 248, 256, 264, 520, 776, 1024, 1032])
-@pytest.mark.parametrize("rows", [1, 5, 4001])
+@pytest.mark.parametrize("rows", [1, 5, 4001, 13001])
 def test_layernorm_rows_in_registers(H, rows):
     """Widths around each number of register chunks and the last one with any; fewer rows than warps and several per warp."""
     from gcow_b200.ops import kernels as K
@@ -44,7 +44,6 @@ def test_layernorm_rows_in_registers(H, rows):
     # every value and once for the deviation
     bound = 2.0 ** -8 * ref.abs() + 12 * (H + 5) * 2.0 ** -24 * r * (1 + n.abs()) * g.double().abs() + 1e-6
     assert bool(((y.double() - ref).abs() <= bound).all())
-
 
 
 def test_gelu_fwd_bwd():
