@@ -215,6 +215,22 @@ def test_tile_kernels_with_four_blocks_per_lane(blocks, how):
     assert torch.equal(g.decompress(gpu).cpu().view(torch.int32), g.decompress(cpu).view(torch.int32))
 
 
+@pytest.mark.parametrize("n", [4 * 300, 4 * 151552 + 7, 4 * 148 * 6 * 4 * 1024 * 2 + 40_001])
+@pytest.mark.parametrize("how", [dict(tolerance=1e-6), dict(tolerance=1e-3), dict(precision=8), dict(precision=16)])
+def test_1d_tiles_of_data_that_changes(n, how):
+    """Noise, values near 1, denormals and zeros in turn, in stretches that end inside a group of 32 blocks and in long ones: warps that
+    stop trying the straight line and ones that do not, on one tile and on several."""
+    rng = np.random.default_rng(n)
+    x = (rng.standard_normal(n) * 1e-3).astype(np.float32)
+    turn = np.arange(n) // 1999 % 4
+    turn[n // 2:] = np.arange(n - n // 2) // 400_003 % 4
+    x = np.select([turn == 1, turn == 2, turn == 3], [1 + x * np.float32(1e-3), x * np.float32(1e-37), x * 0], x).astype(np.float32)
+    cpu = g.compress(torch.from_numpy(x), **how)
+    gpu = g.compress(dev(x), **how)
+    assert gpu.nbytes == cpu.nbytes and torch.equal(gpu.stream.cpu(), cpu.stream)
+    assert torch.equal(g.decompress(gpu).cpu().view(torch.int32), g.decompress(cpu).view(torch.int32))
+
+
 @pytest.mark.parametrize("rate", [2.25, 2.5, 2.75, 3])
 def test_decode_of_short_blocks(rate):
     """Blocks of 9 to 11 bits go to the kernel without staging, 12 bits and streams that are not word aligned to the tiles."""
