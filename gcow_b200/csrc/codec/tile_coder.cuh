@@ -263,19 +263,24 @@ GCOW_HD bool encode_code_1d(const float* f, const ZfpParams& p, const uint32_t* 
   const uint32_t mb = f32_bits(fmaxf(fmaxf(fabsf(f[0]), fabsf(f[1])), fmaxf(fabsf(f[2]), fabsf(f[3])))), ex = mb >> 23;
   const float scale = bits_f32(0x8d800000u - (mb & 0xff800000u));   // 2^(30 - emax), emax = ex - 126; used with 29 <= ex <= 254
   const float p0 = scale * f[0], p1 = scale * f[1], p2 = scale * f[2], p3 = scale * f[3];
+  const uint32_t prec = block_precision((int)ex - 126, p.maxprec, p.minexp, 1), planes = prec < 32u ? prec : 32u;
+  if (planes == 0 || mb == 0) {                             // the block is a single 0 bit
+    w[0] = w[1] = w[2] = w[3] = 0;
+    length = 1;
+    return true;
+  }
   bool ok = ex - 29u <= 225u && fabsf((p0 + p1) + (p2 + p3)) < 8.0e9f;              // the sum: a NaN member
   int32_t q[4];
 #if defined(__CUDA_ARCH__)
   q[0] = __float2int_rz(p0); q[1] = __float2int_rz(p1); q[2] = __float2int_rz(p2); q[3] = __float2int_rz(p3);
 #else
-  if (ok) { q[0] = (int32_t)p0; q[1] = (int32_t)p1; q[2] = (int32_t)p2; q[3] = (int32_t)p3; }
-  else q[0] = q[1] = q[2] = q[3] = 0;                                               // out of range for this conversion
+  if (!ok) return false;                                    // out of range for this conversion
+  q[0] = (int32_t)p0; q[1] = (int32_t)p1; q[2] = (int32_t)p2; q[3] = (int32_t)p3;
 #endif
   fwd_lift(q[0], q[1], q[2], q[3]);
   uint32_t u[4];
 #pragma unroll
   for (int i = 0; i < 4; i++) u[i] = int2nb(q[i]);
-  const uint32_t prec = block_precision((int)ex - 126, p.maxprec, p.minexp, 1), planes = prec < 32u ? prec : 32u;
   const uint32_t mm = u[0] | u[1] | u[2] | u[3];
   uint32_t z = mm ? clz32(mm) : 32u;
   if (z > planes) z = planes;
@@ -302,13 +307,12 @@ GCOW_HD bool encode_code_1d(const float* f, const ZfpParams& p, const uint32_t* 
   uint32_t lo, hi, bits;
   uint32_t prev = planes8(z, first, 0, lo, hi, bits);
   const uint32_t s = kHeaderBits + z;
-  const bool none = planes == 0 || mb == 0;                 // the block is a single 0 bit
-  w[0] = none ? 0u : (2u * ex + 3u) | (lo << (s & 31u));    // flag bit + biased exponent (emax + 127 = ex + 1)
-  w[1] = none ? 0u : funnel_l(lo, hi, s);
-  w[2] = none ? 0u : funnel_l0(hi, s & 31u);
+  w[0] = (2u * ex + 3u) | (lo << (s & 31u));                // flag bit + biased exponent (emax + 127 = ex + 1)
+  w[1] = funnel_l(lo, hi, s);
+  w[2] = funnel_l0(hi, s & 31u);
   w[3] = 0;
-  length = none ? 1u : s + bits;
-  uint32_t k = 24u - z, rest = none ? 0u : left - first;    // planes k-1 .. k-rest remain
+  length = s + bits;
+  uint32_t k = 24u - z, rest = left - first;                // planes k-1 .. k-rest remain
   if (rest && ((prev >> 8) & 0xffu) < 3u) {
     const uint32_t next = rest < 8u ? rest : 8u;
     prev = planes8(z + 8u, next, prev & 0xff00u, lo, hi, bits);
@@ -324,7 +328,7 @@ GCOW_HD bool encode_code_1d(const float* f, const ZfpParams& p, const uint32_t* 
     append64(w, length, t0, t1);
     length += 4u * rest;
   }
-  return (ok && rest <= 16u && length <= 128u) || none;
+  return ok && rest <= 16u && length <= 128u;
 }
 
 // -------------------------------------------------------- 16 x 16 bit transposition

@@ -231,6 +231,23 @@ def test_1d_tiles_of_data_that_changes(n, how):
     assert torch.equal(g.decompress(gpu).cpu().view(torch.int32), g.decompress(cpu).view(torch.int32))
 
 
+@pytest.mark.parametrize("dim", [1, 2])
+def test_tiles_of_zeros(dim):
+    """Groups of one-bit blocks: nothing else, behind strings that end at every bit of a word, and a last group of fewer than 32."""
+    per = 4 if dim == 1 else 16
+    for blocks in (1, 31, 32, 33, 64, 255, 257, 5000, 151_553 + 77):
+        x = np.zeros((blocks, per), np.float32)
+        for lead in (0, 1, 7):
+            x[:] = 0
+            if lead:                                         # a code of another length ahead of each warp's groups of zeros
+                x[::161] = np.random.default_rng(blocks + lead).standard_normal((len(x[::161]), per)) * 10.0 ** -lead
+            f = x.reshape(-1) if dim == 1 else np.ascontiguousarray(x.reshape(blocks, 4, 4).transpose(1, 0, 2).reshape(4, -1))
+            cpu = g.compress(torch.from_numpy(f), dim=dim, tolerance=1e-9)
+            gpu = g.compress(dev(f), dim=dim, tolerance=1e-9)
+            assert gpu.nbytes == cpu.nbytes and torch.equal(gpu.stream.cpu(), cpu.stream)
+            assert torch.equal(g.decompress(gpu).cpu(), torch.from_numpy(f).new_tensor(g.decompress(cpu).numpy()))
+
+
 @pytest.mark.parametrize("rate", [2.25, 2.5, 2.75, 3])
 def test_decode_of_short_blocks(rate):
     """Blocks of 9 to 11 bits go to the kernel without staging, 12 bits and streams that are not word aligned to the tiles."""
