@@ -80,6 +80,7 @@ def test_single_rank_round_trip_of_a_long_bucket(rate, blocks):
     x[:n // 4] = np.cumsum(x[:n // 4])
     x[n // 4:n // 3:5] = 0
     x[n // 3:n // 2] = 0
+    x[n // 3:n // 2:9] = -0.0
     x[n // 2::4099] = np.inf
     x[n // 2 + 1::4097] = np.nan
     x[-n // 8:] += 1
