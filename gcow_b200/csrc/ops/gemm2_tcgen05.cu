@@ -50,6 +50,7 @@ struct Params {
   int M, N, K, ldc, flags;
   int whole, items;        // items of work: `whole` 256 x 256 tiles (of every slice), then halves of 256 x 128
   int slice_blocks;        // stages per slice of the reduction
+  int halves;              // weight gradient, an item per pair at most: a slice's two halves have an accumulator each
   size_t slice_stride;     // elements from one slice's result to the next
   uint32_t* error;
 };
@@ -201,10 +202,11 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         const uint32_t acc = t & 1, aphase = (t >> 1) & 1;
         if (!(ok = wait(&sm->tmem_empty[acc], aphase ^ 1, 2))) break;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const int second = A_MN && p.halves ? (it.kb0 + it.kb1 + 1) / 2 : it.kb1;    // from this stage on in the other accumulator
         for (int kb = it.kb0; kb < it.kb1; kb++) {
           if (!(ok = wait(&sm->full[s], phase, 3))) break;
           tc_fence_after();
+          const uint32_t d_tmem = tmem_base + acc * BN + (A_MN && kb >= second ? BN : 0);
           const uint32_t sa = smem_u32(base + s * STAGE_BYTES), sb = sa + OPER_BYTES;
           const uint32_t eb0 = map_to_cta(smem_u32(&sm->empty[s]), 0), eb1 = map_to_cta(smem_u32(&sm->empty[s]), 1);
           if (lane == 0) {
@@ -214,7 +216,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
               // MN-major: 16 K-rows of 128 bytes per step, 128 rows contiguous within a column group
               const uint64_t da = A_MN ? smem_desc_mn_sw128_16k(sa + k * 2048) : smem_desc_sw128(sa + (k >> 2) * CHUNK_BYTES + in);
               const uint64_t db = B_MN ? smem_desc_mn_sw128_16k(sb + k * 2048) : smem_desc_sw128(sb + (k >> 2) * chunk_b + in);
-              tc_mma_pair(d_tmem, da, db, idesc, kb != it.kb0 || k);
+              tc_mma_pair(d_tmem, da, db, idesc, (kb != it.kb0 && (!A_MN || kb != second)) || k);
             }
             tc_commit_pair(eb0);
             tc_commit_pair(eb1);
@@ -281,6 +283,13 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
         for (int j = 0; j < 32; j++) v[j] = __uint_as_float(r[j]);
         if constexpr (A_MN) {                              // a weight gradient, fp32
+          if (p.halves && it.kb1 - it.kb0 > 1) {
+            uint32_t other[32];
+            tc_ld32(taddr + BN + c * 32, other);
+            tc_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 32; j++) v[j] += __uint_as_float(other[j]);
+          }
           if (row_ok) {
             float* const o = reinterpret_cast<float*>(p.C) + it.slice * p.slice_stride + off;
 #pragma unroll
@@ -486,21 +495,38 @@ int gcow_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
   return launch(kernel, wide ? Epilogue<true>::THREADS : Epilogue<false>::THREADS, max_pairs, ma, mb, mh, p, stream);
 }
 
+// How many slabs of equal length the one-CTA kernel's weight gradient cuts K rows into for an M x N result: it doubles while
+// the tiles still fit one wave of 148 CTAs and a slab keeps at least 512 rows.
+int gcow_wgrad_slabs(int64_t M, int64_t N, int64_t K) {
+  const int64_t tiles = ((M + 127) / 128) * ((N + 255) / 256);
+  int s = 1;
+  while (s < 64 && tiles * s * 2 <= 148 && K % (2 * s) == 0 && (K / (2 * s)) % 64 == 0 && K / (2 * s) >= 512) s *= 2;
+  return s;
+}
+
 // How many slices of the reduction gcow_gemm2_wgrad cuts an M x N result over K rows into; 0: not taken (an operand narrower
-// than a tile, or no cluster launches). Fewer tiles than pairs leave the others idle, and every further slice costs a pass
-// over an M x N partial result: the count that a model of the two puts lowest, in stages of 128 rows (0.83 us). 16384
-// rows to 1024 x 4096 122 -> 113 us, 4096 x 1024 116 -> 104, 1024 x 1024 48 -> 45; 50176 rows to 1024 x 256 40 -> 37, 12544 to 2048 x 512 38 -> 34.
+// than a tile, or no cluster launches). Fewer tiles than pairs leave the others idle, and slices cost a pass over their M x N
+// partial results: the count that a model of the two puts lowest, in us, fitted to 1024 to 50176 rows and results of 256 x 256 to
+// 4096 x 1024 with 1 to 64 slices: 8 + 0.71 per stage of 128 rows, 1.5 for a further round of tiles, and for the ordered sum 1.8 + 0.003 s^2 +
+// (4.5 + 0.35 s) per million elements. 3000 rows to 768 x 3072: one slice 26.2 us, two 31.2; 6144 to 768 x 768 six 23.6, eight 21.6; 16384 to
+// 1024 x 4096 one 100 (one-CTA kernel 113), to 768 x 3072 two 69 (75).
+// No accumulator takes more stages than one of the slabs above: the tensor core cuts the running sum at every step, and the error
+// grows with the number of steps (relative 2-norm, noise: 512 rows 4.7e-7, 1024 1.0e-6, 4096 4.4e-6). Where every pair has one
+// item at most, its slice is shared by two accumulators: 1024 rows to 1024 x 1024 in one slice 14.2 us, in two slices 17.3, on
+// the one-CTA kernel in two slabs 18.8.
 int gcow_gemm2_wgrad_slices(int M, int N, int K) {
   const int max_pairs = gcow_gemm2_max_pairs();
   if (max_pairs <= 0 || M < 256 || N < 256 || M % 64 || N % 64 || K < 1024) return 0;
   const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  const int kblocks = (K + BK - 1) / BK;
+  const int kblocks = (K + BK - 1) / BK, slab = K / gcow_wgrad_slabs(M, N, K), longest = (slab + BK - 1) / BK;
   int best = 1;
   double least = 1e30;
-  for (int s = 1; s <= 64 && kblocks / s >= 4; s++) {
+  for (int s = 1; s <= 64 && kblocks / s >= 2; s++) {
     const int per = (kblocks + s - 1) / s;
-    if ((s - 1) * per >= kblocks) continue;                  // an empty slice
-    const double cost = (double)((tiles * s + max_pairs - 1) / max_pairs) * (per + 6) + (s > 1 ? s * (double)M * N * 8 / 5e6 / 0.83 : 0.0);
+    if ((s - 1) * per >= kblocks || (tiles * s <= max_pairs ? (per + 1) / 2 : per) > longest) continue;   // an empty slice; one too long
+    const long long rounds = (tiles * s + max_pairs - 1) / max_pairs;
+    const double cost = 8.0 + (double)rounds * per * 0.71 + (double)(rounds - 1) * 1.5 +
+                        (s > 1 ? 1.8 + 0.003 * s * s + (double)M * N * 1e-6 * (4.5 + 0.35 * s) : 0.0);
     if (cost < least) { least = cost; best = s; }
   }
   return best;
@@ -524,6 +550,7 @@ int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, int M, int N, i
   if ((slices - 1) * p.slice_blocks >= kblocks) return -2;   // an empty slice would leave its part unwritten
   p.whole = p.items = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * slices;
   p.slice_stride = (size_t)M * N;
+  p.halves = p.items <= max_pairs;
   return launch(gemm2_bf16_kernel<true, true, false, false>, Epilogue<false>::THREADS, max_pairs, ma, mb, mb, p, stream);
 }
 

@@ -24,6 +24,7 @@
 
 extern "C" {
 int gcow_gemm2_max_pairs();
+int gcow_wgrad_slabs(int64_t M, int64_t N, int64_t K);
 int gcow_gemm2_wgrad_slices(int M, int N, int K);
 int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, int M, int N, int K, int lda, int ldb, int slices, uint32_t* error,
                      void* stream);
@@ -221,8 +222,8 @@ Tensor add_parts(const Tensor& part, int64_t parts, c10::IntArrayRef shape, Tens
 }
 
 // dW[N,K] = g^T x, fp32, for g [M,N] and x [M,K], both stored with the reduction dimension M outermost. The result has few tiles
-// while M is long, so the rows are cut into `s` slabs that run as one batched launch and whose products are added in order: `s`
-// doubles while the tiles still fit one wave of 148 CTAs and a slab keeps at least 512 rows.
+// while M is long, so the rows are cut into slices whose products are added in order: on CTA pairs in one launch, else as
+// slabs of one batched launch.
 Tensor wgrad(const Tensor& g, const Tensor& x, const Tensor& out, const On& on) {
   TORCH_CHECK(g.dim() == 2 && x.dim() == 2 && g.size(0) == x.size(0) && g.scalar_type() == at::kBFloat16 && x.scalar_type() == at::kBFloat16 &&
               g.stride(1) == 1 && x.stride(1) == 1, "wgrad: expected two bf16 matrices with contiguous rows, as many in each");
@@ -240,9 +241,7 @@ Tensor wgrad(const Tensor& g, const Tensor& x, const Tensor& out, const On& on) 
     g_launches++;
     return slices > 1 ? add_parts(to, slices, {N, K}, out, on) : out.defined() ? out : to.view({N, K});
   }
-  const int64_t tiles = ((N + 127) / 128) * ((K + 255) / 256);
-  int64_t s = 1;
-  while (s < 64 && tiles * s * 2 <= 148 && M % (2 * s) == 0 && (M / (2 * s)) % 64 == 0 && M / (2 * s) >= 512) s *= 2;
+  const int64_t s = gcow_wgrad_slabs(N, K, M);
   if (s == 1 || g.stride(0) != N || x.stride(0) != K) {
     GemmOpts o;
     o.a_t = o.b_t = o.out_f32 = true;

@@ -134,6 +134,28 @@ def test_wgrad_on_pairs_at_the_edges(M, N, K):
     assert y.data_ptr() == out.data_ptr()
 
 
+def test_wgrad_slices_are_no_longer_than_slabs():
+    """The tensor core's running sum loses a little at every step, so a slice of the rows on CTA pairs has no more stages of 128 than
+    a slab of the one-CTA route, which doubles the slabs while the tiles fit 148 CTAs and 512 rows are left - twice as
+    many where each pair has one item, whose two halves have an accumulator each."""
+    from gcow_b200 import _native
+    lib = _native.cuda()
+    if lib.gcow_gemm2_wgrad_slices(256, 256, 1024) <= 0:
+        pytest.skip("clusters of two CTAs cannot be scheduled here")
+    for rows in (1024, 1088, 1152, 1192, 2048, 3000, 3136, 4096, 8192, 12544, 16384, 50176, 1 << 17):
+        for n in (256, 320, 512, 768, 1024, 2304, 4096):
+            for k in (256, 768, 1024, 2048, 3072, 4096):
+                slabs = 1
+                while (slabs < 64 and -(-n // 128) * -(-k // 256) * slabs * 2 <= 148 and rows % (2 * slabs) == 0
+                       and rows // (2 * slabs) % 64 == 0 and rows // (2 * slabs) >= 512):
+                    slabs *= 2
+                slices, stages = lib.gcow_gemm2_wgrad_slices(n, k, rows), -(-rows // 128)
+                items = -(-n // 256) * -(-k // 256) * slices
+                run = -(-stages // slices)
+                run = (run + 1) // 2 if items <= lib.gcow_gemm2_max_pairs() else run
+                assert slices >= 1 and run <= -(-(rows // slabs) // 128), (rows, n, k)
+
+
 @pytest.mark.parametrize("M,N,K", [(1024, 512, 256), (2048, 1024, 1024), (1100, 288, 192), (4096, 4096, 64)])
 def test_pair_gemm_matches_fp32_reference(M, N, K, monkeypatch):
     """The CTA-pair kernel (cta_group::2) incl. ragged edges, a K that is not a whole stage, and every epilogue."""
