@@ -531,7 +531,8 @@ place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restric
 
 // 1-D tables in shared memory: the lean coder's windows and nibble pairs, and one plane per lookup.
 // Before, with one plane per lookup throughout and a bit-matrix transpose per eight planes, 25.6 M values took: noise at
-// tolerance 1e-6 121 us (now 101), at 1e-3 95 (93), at 6 bits/value 117 (97); a random walk at 1e-6 218 (138).
+// tolerance 1e-6 121 us, with windows 101, with the straight line first 81; at 1e-3 95, 93, 70; at 6 bits/value 117, 97, 84; a
+// random walk at 1e-6 218, 144, 135.
 template <int DIM, int PER, bool BUDGET>
 __global__ void __launch_bounds__(kTileThreads)
 decode_tiles_kernel(const uint32_t* in, float* __restrict__ out, const TileArgs a,
@@ -674,8 +675,8 @@ int gcow_tile_usable(const int32_t* params, uint64_t blocks, int dim) {
   return max_block_bits(p, dim) <= limit && blocks <= 0xffffffffull * 64 ? 1 : 0;
 }
 
-// Scratch of gcow_encode_tiles in bytes: 0 at fixed rate; else the strings (as many words as the longest possible stream),
-// a length per string and per tile, and 16 bits per block.
+// Scratch of gcow_encode_tiles in bytes: 0 at fixed rate; else a length per tile, the tiles' strings (as many words as the longest
+// possible stream), an offset per warp and one of 16 bits per block.
 uint64_t gcow_encode_tiles_scratch_bytes(const int32_t* params, uint64_t blocks, int dim) {
   if (params[0] == params[1]) return 0;
   const ZfpParams p = {(uint32_t)params[0], (uint32_t)params[1], (uint32_t)params[2], params[3]};

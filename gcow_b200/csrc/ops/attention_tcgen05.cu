@@ -120,9 +120,9 @@ __device__ __forceinline__ Unit unit_at(int u, int mode, int tiles, int heads) {
 // The barriers of a CTA are numbered, and a role keeps the parities it waits for next in one word.
 //
 // B 32, S 512, 16 heads: forward 123 us with one tile in flight and the probabilities through shared memory, now 67 (0.51
-// PFLOP/s; the 134 M exponentials take 29 at 16 a clock and SM); backward 327, now 225 (delta 15, the rest 0.57 PFLOP/s;
-// 251 with one issuing warp per tile in the backward pass, 242 with dQ behind dK/dV). One sequence of 512:
-// backward 35 us, now 30.
+// PFLOP/s; the 134 M exponentials take 29 at 16 a clock and SM); backward 327, now 233 (delta 15, the rest 0.55 PFLOP/s;
+// 251 with one issuing warp per tile in the backward pass, 242 with dQ behind dK/dV, 231 as a launch of its own beside it).
+// One head of 512: backward 24.8 us.
 //
 // What the issuing warps do per product decides the pace. As code of one thread alone, with the descriptors worked out where
 // they are used, a step of four to eight MMAs took it 1500 cycles (forward, B 32, S 512, 16 heads: 131 us): every operand of

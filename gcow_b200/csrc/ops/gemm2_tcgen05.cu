@@ -40,10 +40,10 @@ constexpr int STAGES = 3;
 template <bool WIDE> struct Epilogue { static constexpr int WARPS = WIDE ? 16 : 8, THREADS = 64 + 32 * WARPS; };
 constexpr uint32_t TMEM_COLS = 512;
 
-enum Flags : int { kOutF32 = 1, kBias = 2, kGelu = 4, kResidual = 8, kAuxOut = 32, kGeluGrad = 64 };
+enum Flags : int { kBias = 2, kGelu = 4, kResidual = 8, kAuxOut = 32, kGeluGrad = 64 };
 
 struct Params {
-  __nv_bfloat16* C;        // float* with kOutF32
+  __nv_bfloat16* C;        // float* of a weight gradient
   const float* bias;
   const __nv_bfloat16* residual;
   __nv_bfloat16* aux;
@@ -544,7 +544,7 @@ int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, int M, int N, i
   if (rc) return rc;
   Params p = {};
   p.C = (__nv_bfloat16*)parts;
-  p.M = M; p.N = N; p.K = K; p.ldc = N; p.flags = kOutF32; p.error = error;
+  p.M = M; p.N = N; p.K = K; p.ldc = N; p.error = error;
   const int kblocks = (K + BK - 1) / BK;
   p.slice_blocks = (kblocks + slices - 1) / slices;
   if ((slices - 1) * p.slice_blocks >= kblocks) return -2;   // an empty slice would leave its part unwritten

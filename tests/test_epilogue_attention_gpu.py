@@ -52,9 +52,9 @@ def test_gelu_of_special_values():
     assert math.isnan(K.gemm_bf16(x, torch.eye(64, device="cuda", dtype=torch.bfloat16), gelu=True)[0, 0].item())
 
 
-@pytest.mark.parametrize("B,S,H", [(37, 512, 1), (149, 128, 1), (25, 256, 3), (25, 384, 2), (38, 512, 1)])
+@pytest.mark.parametrize("B,S,H", [(74, 128, 1), (75, 128, 1), (37, 256, 1), (38, 256, 1), (37, 512, 1), (148, 128, 1), (149, 128, 1), (25, 256, 3), (25, 384, 2), (38, 512, 1)])
 def test_attention_on_either_side_of_a_full_gpu(B, S, H):
-    """As below, with 148 CTAs (the last grid with long steps in the backward kernels) and a few more."""
+    """As below, with 74 and 148 tiles, the most that have a CTA each in the backward and the forward kernels, and a few more."""
     test_attention(B, S, H)
 
 
@@ -99,8 +99,8 @@ def test_attention_of_sequences_that_end_inside_a_tile(B, S, H):
 @pytest.mark.parametrize("S", [256, 512])
 @pytest.mark.parametrize("order", [1, -1])
 def test_attention_when_the_row_maximum_moves_between_key_blocks(S, order):
-    """Keys that grow, or shrink, by a factor of four per 128 positions: the forward pass follows the row maximum by more than
-    the margin it allows itself, or never. Two roundings to bf16, as above."""
+    """Keys that grow, or shrink, by a factor of four per 128 positions: the forward pass rescales at every block of keys, or
+    never. Two roundings to bf16, as above."""
     from gcow_b200.ops import kernels as K
     torch.manual_seed(S)
     qkv = torch.randn(5, S, 3, 2, 64, device="cuda")
