@@ -1164,7 +1164,8 @@ GCOW_HD void decode_block_1d_lean(float* f, const LeanTables& t, const uint32_t 
 //   C - 4 k,  C = (top_0 + 1) + (top_1 + 1) + (top_2 + 1) + #{i < 3: highest bit of coefficient i == top_i} + 32,
 // for every k <= top_2, and the bits that are left over (fewer than four) are the lowest coefficients' bits of plane k - 1.
 // No table, no branch.
-// False (f is not written) where the cut falls at or above top_2, or the exponent or a member is out of the ordinary.
+// False (f is not written) where the cut falls into plane top_2 or above it (roundtrip_block_1d_cut), or the exponent or a member is out
+// of the ordinary.
 template <int BITS>
 GCOW_HD bool roundtrip_block_1d_try(float* f) {
   constexpr int P = BITS - (int)kHeaderBits;
@@ -1202,6 +1203,62 @@ GCOW_HD bool roundtrip_block_1d_try(float* f) {
   for (int i = 0; i < 4; i++) q[i] = nb2int(u[i] & (i < 3 && i < a ? more : whole));
   inv_lift(q[0], q[1], q[2], q[3]);
   if (!ok) return false;
+  const float back = bits_f32((ex - 29u) << 23);              // 2^(emax - 30)
+#pragma unroll
+  for (int i = 0; i < 4; i++) f[i] = back * (float)q[i];
+  return true;
+}
+
+// The blocks of an ordinary exponent that the function above leaves, smooth ones mostly: the cut falls into a plane that starts with n < 3.
+// The planes 31..k cost
+//   sum over i < 3 of max(top_i + 1 - k, 0)  +  #{i < 3: highest bit of coefficient i == top_i >= k}  +  32 - k,
+// and plane k - 1 is read again as the decoder would read what is left of the budget: n verbatim bits, then tests and runs, a one-bit
+// that is pending where the bits end included. False where that function's `ordinary` is.
+template <int BITS>
+GCOW_HD bool roundtrip_block_1d_cut(float* f) {
+  constexpr int P = BITS - (int)kHeaderBits;
+  const uint32_t mb = f32_bits(fmaxf(fmaxf(fabsf(f[0]), fabsf(f[1])), fmaxf(fabsf(f[2]), fabsf(f[3]))));
+  const uint32_t ex = mb >> 23;
+  const float scale = bits_f32(0x8d800000u - (mb & 0xff800000u));
+  const float p0 = scale * f[0], p1 = scale * f[1], p2 = scale * f[2], p3 = scale * f[3];
+  if (!(ex - 30u <= 224u && fabsf((p0 + p1) + (p2 + p3)) < 8.0e9f)) return false;
+  int32_t q[4] = {(int32_t)p0, (int32_t)p1, (int32_t)p2, (int32_t)p3};
+  fwd_lift(q[0], q[1], q[2], q[3]);
+  uint32_t u[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) u[i] = int2nb(q[i]);
+  const uint32_t m2 = u[2] | u[3], m1 = m2 | u[1], m0 = m1 | u[0];
+  const int t0 = 31 - (m0 ? (int)clz32(m0) : 32), t1 = 31 - (m1 ? (int)clz32(m1) : 32), t2 = 31 - (m2 ? (int)clz32(m2) : 32);
+  const int o0 = u[0] > (m0 ^ u[0]) ? t0 : -1, o1 = u[1] > (m1 ^ u[1]) ? t1 : -1, o2 = u[2] > (m2 ^ u[2]) ? t2 : -1;
+  auto cost = [&](int k) {
+    return (t0 >= k ? t0 + 1 - k : 0) + (t1 >= k ? t1 + 1 - k : 0) + (t2 >= k ? t2 + 1 - k : 0) + (o0 >= k) + (o1 >= k) + (o2 >= k) + 32 - k;
+  };
+  int k = t2 + 1;                                             // a cut below that is the closed form's
+  while (cost(k) > P) k++;
+  const uint32_t whole = shl_sat(0xffffffffu, (uint32_t)k);
+  uint32_t more = 0;                                          // coefficients that have a one in plane k - 1, as far as it is read
+  if (k > 0) {
+    int a = P - cost(k);
+    const int pl = k - 1;
+    int n = (t0 > pl) + (t1 > pl) + (t2 > pl);                // coefficient 3 has its top at t2 at most
+    const uint32_t x = ((u[0] >> pl) & 1u) | ((u[1] >> pl) & 1u) << 1 | ((u[2] >> pl) & 1u) << 2 | ((u[3] >> pl) & 1u) << 3;
+    const int m = a < n ? a : n;
+    more = x & ((1u << m) - 1u);
+    a -= m;
+    while (a > 0 && n < 4) {
+      a--;
+      if (!(x >> n)) break;
+      while (a > 0 && n < 3) {
+        a--;
+        if ((x >> n) & 1u) break;
+        n++;
+      }
+      more |= 1u << n++;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++) q[i] = nb2int((u[i] & whole) | shl_sat((more >> i) & 1u, (uint32_t)(k - 1)));
+  inv_lift(q[0], q[1], q[2], q[3]);
   const float back = bits_f32((ex - 29u) << 23);              // 2^(emax - 30)
 #pragma unroll
   for (int i = 0; i < 4; i++) f[i] = back * (float)q[i];

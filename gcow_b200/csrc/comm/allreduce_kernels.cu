@@ -420,33 +420,73 @@ allreduce_fused_kernel(const ArArgs a) {
 
 // ------------------------------------------------- one rank: the lossy round trip alone
 // A single rank's one-shot call is y = D(E(x)), one block at a time: no peer, so no slot, flag or wait, and no reason for a
-// resident grid. The kernel reads the bucket once and writes it once, over the whole GPU, and makes the code only for the
-// blocks that roundtrip_block_1d_try leaves (and at 4 bits/value, where half of all noise is cut before n = 3). Two blocks per
-// thread are in flight, as in the stand-alone coders. 6.5 M values at 8 bits/value: the resident kernel on its default 32 CTAs
-// 350 us, both coders in registers 24.6; 1.6 M values at 16 bits/value: both coders 14.0 us, now 5.2.
+// resident grid. The bucket is read once and written once, over the whole GPU, and no code is made: what decoding it would give is
+// worked out by roundtrip_block_1d_try, or by roundtrip_block_1d_cut where the cut falls into the block's first planes (6 blocks of noise
+// in 10^4 at 8 bits/value, nearly all of smooth data). Only a block of a tiny, huge or non-finite maximum goes through both coders, with
+// their tables read from global memory: loading them into every CTA's shared memory took a tenth of the kernel. Four blocks per thread
+// are in flight, bound by integer work and memory in about equal parts: us at 6.5 M / 33 M values of noise, both coders' tables in
+// shared memory and two blocks in flight -> now: 8 bits/value 16.9 -> 12.8 / 59.6 -> 51.2, 16 13.9 -> 12.4 / 53.8 -> 51.3; 1 M 7 either way. 6.5 M values
+// near 1: 8 bits 70 -> 37, 16 bits 158 -> 22. Six blocks in flight (64 registers, four CTAs per SM): 15.0 / 57.4.
+constexpr int kTripAhead = 4, kTripCtas = 6;
 template <int BITS>
-__device__ __forceinline__ bool roundtrip_try(float* f, const LeanTables& lt) {
-  if (BITS > 16) return roundtrip_block_1d_try<BITS>(f);
-  uint32_t w[Code<BITS>::NW];
-  float d[4];
-  if (!encode_block_1d_try<BITS>(f, lt, w, 0) || !decode_block_1d_try<BITS>(d, lt, w, 0, 0)) return false;
+__global__ void __launch_bounds__(kArThreads, kTripCtas)
+roundtrip_kernel(const ArArgs a) {
+  pdl_trigger();
+  pdl_wait();
+  const LeanTables lt = {a.enc_table, a.dec_table, a.pair_table, a.loop_table};
+  const bool aligned = (((uintptr_t)a.in | (uintptr_t)a.out) & 15) == 0;
+  const uint64_t blocks = (a.n + 3) / 4, stride = (uint64_t)gridDim.x * kArThreads, whole = aligned ? a.n / 4 : 0;
+  auto rest = [&](float* f) {
+    if (f[0] == 0 && f[1] == 0 && f[2] == 0 && f[3] == 0) {   // what is left most often
+      f[0] = f[1] = f[2] = f[3] = 0;
+    } else if (!roundtrip_block_1d_cut<BITS>(f)) {
+      uint32_t w[Code<BITS>::NW];
+      encode_block_1d_rest<BITS>(f, lt, w);
+      decode_block_1d_rest<BITS>(f, lt, w, 0, 0);
+    }
+  };
+  auto trip = [&](uint64_t b, uint64_t end) {                 // blocks b, b + stride, .. of those below `end`
+    float f[kTripAhead][4];
+    bool ok[kTripAhead];
 #pragma unroll
-  for (int i = 0; i < 4; i++) f[i] = d[i];
-  return true;
-}
-template <int BITS>
-__device__ __forceinline__ void roundtrip_rest(float* f, const LeanTables& lt) {
-  if (f[0] == 0 && f[1] == 0 && f[2] == 0 && f[3] == 0) {   // what is left most often; half of all blocks, 4 bits/value: 19.3 -> 12.5 us
-    f[0] = f[1] = f[2] = f[3] = 0;
-    return;
+    for (int i = 0; i < kTripAhead; i++) {
+      const float4 v = b + i * stride < end ? reinterpret_cast<const float4*>(a.in)[b + i * stride] : make_float4(0, 0, 0, 0);
+      f[i][0] = v.x; f[i][1] = v.y; f[i][2] = v.z; f[i][3] = v.w;
+    }
+#pragma unroll
+    for (int i = 0; i < kTripAhead; i++) ok[i] = roundtrip_block_1d_try<BITS>(f[i]);
+#pragma unroll
+    for (int i = 0; i < kTripAhead; i++) {
+      if (b + i * stride >= end) break;
+      if (!ok[i]) rest(f[i]);
+      if (a.postscale != 1.0f) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) f[i][j] *= a.postscale;
+      }
+      reinterpret_cast<float4*>(a.out)[b + i * stride] = make_float4(f[i][0], f[i][1], f[i][2], f[i][3]);
+    }
+  };
+  uint64_t b = (uint64_t)blockIdx.x * kArThreads + threadIdx.x;
+  for (; b + (kTripAhead - 1) * stride < whole; b += kTripAhead * stride) trip(b, ~0ull);
+  if (b < whole) trip(b, whole);
+  // the array's end, or all of one at an odd address
+  for (b = whole + (uint64_t)blockIdx.x * kArThreads + threadIdx.x; b < blocks; b += stride) {
+    float f[4];
+    load_block(f, a.in, a.n, b, false);
+    if (!roundtrip_block_1d_try<BITS>(f)) rest(f);
+    if (a.postscale != 1.0f) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) f[i] *= a.postscale;
+    }
+    store_block(f, a.out, a.n, b, false);
   }
-  uint32_t w[Code<BITS>::NW];
-  encode_block_1d_lean<BITS>(f, lt, w);
-  decode_block_1d_lean<BITS>(f, lt, w, 0);
 }
+
+// The same through both coders: at 4 bits/value, where half of all noise is cut before n = 3 and two lookups make the code, and with
+// error feedback. Two blocks per thread are in flight, as in the stand-alone coders.
 template <int BITS>
 __global__ void __launch_bounds__(kArThreads)
-roundtrip_kernel(const ArArgs a) {
+roundtrip_coded_kernel(const ArArgs a) {
   constexpr int kAhead = 2;
   __shared__ __align__(16) uint32_t epair[kEncPairTabSize];
   __shared__ __align__(16) uint32_t dloop[kDecLoopTabSize];
@@ -460,6 +500,23 @@ roundtrip_kernel(const ArArgs a) {
   const LeanTables lt = {a.enc_table, a.dec_table, epair, dloop};
   const bool in_al = ((uintptr_t)a.in & 15) == 0, out_al = ((uintptr_t)a.out & 15) == 0;
   const uint64_t blocks = (a.n + 3) / 4, stride = (uint64_t)gridDim.x * kArThreads;
+  auto attempt = [&](float* f) {
+    uint32_t w[Code<BITS>::NW];
+    float d[4];
+    if (!encode_block_1d_try<BITS>(f, lt, w, 0) || !decode_block_1d_try<BITS>(d, lt, w, 0, 0)) return false;
+#pragma unroll
+    for (int i = 0; i < 4; i++) f[i] = d[i];
+    return true;
+  };
+  auto rest = [&](float* f) {
+    if (f[0] == 0 && f[1] == 0 && f[2] == 0 && f[3] == 0) {   // what is left most often; half of all blocks: 19.3 -> 12.5 us
+      f[0] = f[1] = f[2] = f[3] = 0;
+      return;
+    }
+    uint32_t w[Code<BITS>::NW];
+    encode_block_1d_lean<BITS>(f, lt, w);
+    decode_block_1d_lean<BITS>(f, lt, w, 0);
+  };
   uint64_t b = (uint64_t)blockIdx.x * kArThreads + threadIdx.x;
   const uint64_t whole = in_al && out_al && !a.residual ? a.n / 4 : 0;
   for (; b + (kAhead - 1) * stride < whole; b += kAhead * stride) {
@@ -471,10 +528,10 @@ roundtrip_kernel(const ArArgs a) {
       f[i][0] = v.x; f[i][1] = v.y; f[i][2] = v.z; f[i][3] = v.w;
     }
 #pragma unroll
-    for (int i = 0; i < kAhead; i++) ok[i] = roundtrip_try<BITS>(f[i], lt);
+    for (int i = 0; i < kAhead; i++) ok[i] = attempt(f[i]);
 #pragma unroll
     for (int i = 0; i < kAhead; i++) {
-      if (!ok[i]) roundtrip_rest<BITS>(f[i], lt);
+      if (!ok[i]) rest(f[i]);
       if (a.postscale != 1.0f) {
 #pragma unroll
         for (int j = 0; j < 4; j++) f[i][j] *= a.postscale;
@@ -489,8 +546,8 @@ roundtrip_kernel(const ArArgs a) {
       uint32_t w[Code<BITS>::NW];
       encode_with_feedback<BITS, Code<BITS>::NW>(f, a, b, lt, w);
       decode_block_1d_lean<BITS>(f, lt, w, 0);
-    } else if (!roundtrip_try<BITS>(f, lt)) {
-      roundtrip_rest<BITS>(f, lt);
+    } else if (!attempt(f)) {
+      rest(f);
     }
     if (a.postscale != 1.0f) {
 #pragma unroll
@@ -811,10 +868,24 @@ static int ar_launch_impl(const float* in, float* out, uint64_t n, int rank, int
     return (int)cudaGetLastError();
   }
   if (world == 1 && variant == kOneShot && !stamps) {
-    const uint64_t want = ((n + 3) / 4 + kArThreads - 1) / kArThreads;
-    const int g = (int)(want < 148 * 8 ? want : 148 * 8);
+    const uint64_t want = ((n + 3) / 4 + kArThreads - 1) / kArThreads;   // a block per thread
+    if (residual || bits == 16) {
+      const int g = (int)(want < 148 * 8 ? want : 148 * 8);
+      switch (bits) {
+        case 16: launch_dependent(roundtrip_coded_kernel<16>, dim3(g), dim3(kArThreads), 0, s, a); break;
+        case 32: launch_dependent(roundtrip_coded_kernel<32>, dim3(g), dim3(kArThreads), 0, s, a); break;
+        case 64: launch_dependent(roundtrip_coded_kernel<64>, dim3(g), dim3(kArThreads), 0, s, a); break;
+        case 128: launch_dependent(roundtrip_coded_kernel<128>, dim3(g), dim3(kArThreads), 0, s, a); break;
+        default: return -1;
+      }
+      return (int)cudaGetLastError();
+    }
+    // As many CTAs as are resident (fewer threads of four blocks each took 11.6 instead of 9.1 us for 3 M values at 8 bits), then more, of
+    // four blocks per thread, which the GPU hands out as others end.
+    const uint64_t resident = 148 * kTripCtas, few = want < resident ? want : resident, many = (want + kTripAhead - 1) / kTripAhead;
+    const uint64_t most = 1u << 30;
+    const unsigned g = (unsigned)(many > few ? (many < most ? many : most) : few);
     switch (bits) {
-      case 16: launch_dependent(roundtrip_kernel<16>, dim3(g), dim3(kArThreads), 0, s, a); break;
       case 32: launch_dependent(roundtrip_kernel<32>, dim3(g), dim3(kArThreads), 0, s, a); break;
       case 64: launch_dependent(roundtrip_kernel<64>, dim3(g), dim3(kArThreads), 0, s, a); break;
       case 128: launch_dependent(roundtrip_kernel<128>, dim3(g), dim3(kArThreads), 0, s, a); break;

@@ -92,6 +92,28 @@ def test_single_rank_round_trip_of_a_long_bucket(rate, blocks):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("rate", [8, 16, 32])
+@pytest.mark.parametrize("blocks", [148 * 6 * 256, 148 * 6 * 256 + 1, 3 * 148 * 6 * 256 + 77, 4 * 148 * 6 * 256 - 1, 4 * 148 * 6 * 256 + 1025])
+def test_single_rank_round_trip_without_a_code(rate, blocks):
+    """The kernel that makes no code, around the sizes where its grid is full and where a thread has four blocks: data that the bit
+    budget cuts in every plane, a tail that is no whole block, and the same at an address that is no multiple of 16."""
+    n = 4 * blocks - 2
+    rng = np.random.default_rng(blocks)
+    x = gen(blocks, n)
+    x += np.repeat(np.exp2(rng.integers(-24, 2, n // 1024 + 1)), 1024)[:n].astype(np.float32)
+    x[::4097] = np.nan
+    x[1::8193] *= 1e-36
+    want = allreduce_oracle(x[None], ZfpParams.from_rate(rate, 1), "oneshot", 0)
+    ar = CompressedAllReduce(n, GcowConfig(rate=rate))
+    buf = torch.empty(n + 1, device="cuda")
+    for off in (0, 1):
+        t = buf[off:off + n].copy_(torch.from_numpy(x))
+        y = ar(t).cpu().numpy()
+        assert np.array_equal(y.view(np.uint32), want.view(np.uint32))
+    ar.check()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("cap,tol", [(4, 1e-2), (8, 1e-3), (16, 1e-6), (32, 1e-4)])
 def test_accuracy_mode_single_rank_equals_oracle(cap, tol):
     """Fixed accuracy with a bit cap (the sparse variant): bit-exact against the host model at the same four codec
