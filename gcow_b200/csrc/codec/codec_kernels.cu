@@ -105,9 +105,18 @@ template <> struct CodeIO<128> {
 // blocks that leave the straight line, and the array's end, are seen to one by one. CTAs of 512 threads: half as many
 // copies of the tables as with 256, which is what a vector of a million values feels.
 constexpr int kRateThreads = 512, kAhead = 2;
-// CTAs per SM, as the registers allow, which is also the grid: encoding 67 M values at 8 bits/value takes 80 us with two,
-// 76 us with three.
-constexpr int kEncodeCtas = 3, kDecodeCtas = 4;
+// CTAs per SM, as the registers allow: encoding 67 M values at 8 bits/value takes 80 us with two, 76 us with three.
+constexpr int kEncodeCtas = 3;
+constexpr int decode_ctas(int bits) { return bits <= 32 ? 4 : 3; }
+// Grid: the resident CTAs; twice as many where a thread would have kLong blocks or more, since an SM whose CTAs are through early is
+// then given others. Once, twice: 67 M values at 8 bits/value 68.7, 68.2 us (encoding), 81.0, 80.0; 16 bits/value 104.1, 101.8 and 112.0, 108.2;
+// at 4 bits/value decoding is slower for it (53.1, 54.1), and so is most of 17 M values (19.7, 20.9 encoding at 8 bits/value).
+constexpr uint64_t kLong = 32;
+static int rate_grid(uint64_t blocks, int ctas, bool twice) {
+  const uint64_t resident = 148ull * ctas, want = (blocks + kRateThreads - 1) / kRateThreads;
+  const uint64_t g = twice && blocks >= kLong * resident * kRateThreads ? 2 * resident : resident;
+  return (int)(want < g ? want : g);
+}
 
 template <int BITS>
 __global__ void __launch_bounds__(kRateThreads, kEncodeCtas)
@@ -152,7 +161,7 @@ encode_1d_fixed_kernel(const float* in, uint64_t n, void* __restrict__ out, int 
 }
 
 template <int BITS>
-__global__ void __launch_bounds__(kRateThreads, 2)      // 32 registers without being forced; forced, 95 instead of 91 us
+__global__ void __launch_bounds__(kRateThreads, BITS == 16 ? 4 : 2)   // 32 bits: 32 registers without being forced; forced, 95 instead of 91 us
 decode_1d_fixed_kernel(const void* in, float* __restrict__ out, uint64_t n, int shift,
                        int aligned, const uint16_t* __restrict__ tab, const uint32_t* __restrict__ loop_tab) {
   constexpr int NW = CodeIO<BITS>::NW;
@@ -598,7 +607,7 @@ static int launch_encode_1d(const float* in, uint64_t n, int maxbits, void* out,
   uint64_t blocks = num_blocks_1d(n);
   if (!blocks) return 0;
   int aligned = ((uintptr_t)in & 15) == 0;
-  int g = grid_for(blocks, kRateThreads, 148 * kEncodeCtas);
+  const int g = rate_grid(blocks, kEncodeCtas, true);
   const void *etp, *dtp, *ptp, *ltp;
   if (int rc = gcow_codec_tables4(&etp, &dtp, &ptp, &ltp)) return rc;
   const uint16_t* et = (const uint16_t*)etp;
@@ -629,7 +638,7 @@ int gcow_decode_1d_fixed(const void* in, float* out, uint64_t n, int maxbits, in
   uint64_t blocks = num_blocks_1d(n);
   if (!blocks) return 0;
   int aligned = ((uintptr_t)out & 15) == 0;
-  int g = grid_for(blocks, kRateThreads, 148 * kDecodeCtas);
+  const int g = rate_grid(blocks, decode_ctas(maxbits), maxbits > 16);
   const void *etp, *dtp, *ptp, *ltp;
   if (int rc = gcow_codec_tables4(&etp, &dtp, &ptp, &ltp)) return rc;
   const uint32_t* lt = (const uint32_t*)ltp;

@@ -260,7 +260,8 @@ GCOW_HD void append64(uint32_t (&w)[4], uint32_t at, uint32_t lo, uint32_t hi) {
 // serial form above has to do it: a non-finite or tiny maximum, a NaN member, more than sixteen planes with n < 3 or
 // sixteen verbatim ones, a code of more than 128 bits. No budget: the block's code must not reach maxbits.
 GCOW_HD bool encode_code_1d(const float* f, const ZfpParams& p, const uint32_t* epair, uint32_t (&w)[4], uint32_t& length) {
-  const uint32_t mb = f32_bits(fmaxf(fmaxf(fabsf(f[0]), fabsf(f[1])), fmaxf(fabsf(f[2]), fabsf(f[3])))), ex = mb >> 23;
+  bool ok;
+  const uint32_t mb = block_max_bits(f, 29, ok), ex = mb >> 23;
   const float scale = bits_f32(0x8d800000u - (mb & 0xff800000u));   // 2^(30 - emax), emax = ex - 126; used with 29 <= ex <= 254
   const float p0 = scale * f[0], p1 = scale * f[1], p2 = scale * f[2], p3 = scale * f[3];
   const uint32_t prec = block_precision((int)ex - 126, p.maxprec, p.minexp, 1), planes = prec < 32u ? prec : 32u;
@@ -269,7 +270,6 @@ GCOW_HD bool encode_code_1d(const float* f, const ZfpParams& p, const uint32_t* 
     length = 1;
     return true;
   }
-  bool ok = ex - 29u <= 225u && fabsf((p0 + p1) + (p2 + p3)) < 8.0e9f;              // the sum: a NaN member
   int32_t q[4];
 #if defined(__CUDA_ARCH__)
   q[0] = __float2int_rz(p0); q[1] = __float2int_rz(p1); q[2] = __float2int_rz(p2); q[3] = __float2int_rz(p3);
@@ -462,7 +462,7 @@ constexpr int kTileRows = kDecTiny, kTileDecTab1 = kTileRows + 3 * 128 * 2;
 // Entry i (0..383) of the one-plane rows, from the decoder's budget table.
 GCOW_HD DecWindow make_tile_row(const uint16_t* dtab, uint32_t i) {
   const uint32_t e = dtab[((i >> 7) * 8 + 7) * 128 + (i & 127)], n = e >> 7;
-  return {spread_nibble(e & 15u), ((e >> 4) & 7u) | (1u << 8) | ((n < 3 ? n : 3u) << 12)};
+  return {spread_nibble(e & 15u), 1u | (n < 3 ? (n + 1) << 12 : 0u) | ((e >> 4) & 7u) << 16};
 }
 GCOW_HD void decode_window_1d(float* f, const ZfpParams& p, const uint32_t* tab, const uint16_t* dtab, const uint32_t* words,
                               uint32_t pos, int shift) {
@@ -484,19 +484,19 @@ GCOW_HD void decode_window_1d(float* f, const ZfpParams& p, const uint32_t* tab,
   bits -= z;
   const uint32_t* const nib = tab + kDecNibbles;
   uint32_t u[4] = {0, 0, 0, 0};
-  uint32_t U = 0, held = 0, gone = z, row = 0;             // planes in U; planes above the next one; min(n, 3) * 4096
+  uint32_t U = 0, held = 0, gone = z, row = 0x1000;        // planes in U; planes above the next one; (n + 1) * 4096, 0 once n >= 3
   auto flush = [&]() {                                     // U to its place: the planes down to 32 - gone
     const uint32_t m = pow2_factor(32u - gone);
     u[0] += (U & 0xffu) * m; u[1] += ((U >> 8) & 0xffu) * m; u[2] += ((U >> 16) & 0xffu) * m; u[3] += (U >> 24) * m;
     U = held = 0;
   };
-  while (row != 0x3000u && gone < planes && bits) {
+  while (row && gone < planes && bits) {
     if (held > 3) flush();                                 // at most seven planes: the tail wants the bytes' top bits clear
     const bool wide = planes - gone >= 4 && bits >= 9;     // a window holds at most four planes and nine bits
     if (wide || bits >= 7) {
-      const uint32_t v = src.peek(), at = wide ? row + 8u * (v & 511u) : kTileRows * 4u + (row >> 2) + 8u * (v & 127u);
+      const uint32_t v = src.peek(), at = wide ? row - 0x1000u + 8u * (v & 511u) : kTileRows * 4u + ((row - 0x1000u) >> 2) + 8u * (v & 127u);
       const DecWindow d = *reinterpret_cast<const DecWindow*>(reinterpret_cast<const char*>(tab) + at);
-      const uint32_t n = (d.meta >> 8) & 15u, used = d.meta & 31u;
+      const uint32_t n = d.meta & 15u, used = d.meta >> 16;
       U = (U << n) | d.u;
       held += n;
       gone += n;
@@ -504,13 +504,13 @@ GCOW_HD void decode_window_1d(float* f, const ZfpParams& p, const uint32_t* tab,
       bits -= used;
       row = d.meta & 0x3000u;
     } else {                                               // the budget may end inside this plane
-      const uint32_t e = dtab[(((row >> 12) * 8 + bits) << 7) + (src.peek() & low_mask32(bits))], used = (e >> 4) & 7u, n = e >> 7;
+      const uint32_t e = dtab[((((row >> 12) - 1u) * 8 + bits) << 7) + (src.peek() & low_mask32(bits))], used = (e >> 4) & 7u, n = e >> 7;
       U = 2 * U + (nib[e & 15u] >> 1);
       held++;
       gone++;
       src.skip(used);
       bits -= used;
-      row = (n < 3 ? n : 3u) << 12;
+      row = n < 3 ? (n + 1) << 12 : 0u;
     }
   }
   // A nibble cut by the budget after its first three bits: with n == 3 the missing bit is a group test that reads as 0,
@@ -562,23 +562,22 @@ GCOW_HD bool decode_code_1d(float* f, const ZfpParams& p, const uint32_t* tab, c
   };
   skip(kHeaderBits);
   const uint32_t z = (uint32_t)ctz32(x0 | 0x1000000u);
-  if (planes > z + 23u) return false;                      // of which more than sixteen would be verbatim
+  if (planes > z + 23u || shift < -29) return false;       // more than sixteen verbatim; 2^(emax - 30 - shift) may be infinite
   skip(z);
-  uint32_t U = 0, gone = z, row = 0, used = kHeaderBits + z;
+  uint32_t U = 0, row = 0x1000, sum = (kHeaderBits + z) << 16; // the sum as in decode_block_1d_try
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    if (c == 0 || (row != 0x3000u && gone < planes)) {
-      const DecWindow d = *reinterpret_cast<const DecWindow*>(reinterpret_cast<const char*>(tab) + row + 8u * (x0 & 511u));
-      const uint32_t n = (d.meta >> 8) & 15u, len = d.meta & 31u;
-      U = (U << n) | d.u;
-      gone += n;
-      used += len;
-      skip(len);
+    if (c == 0 || (row && z + (sum & 0xffu) < planes)) {
+      const DecWindow d = *reinterpret_cast<const DecWindow*>(reinterpret_cast<const char*>(tab) + (row - 0x1000u) + 8u * (x0 & 511u));
+      U = c ? funnel_l(0u, U, d.meta) | d.u : d.u;
       row = d.meta & 0x3000u;
+      sum += d.meta;
+      skip(d.meta >> 16);
     }
   }
-  const int rest = (int)(planes - gone);                     // verbatim planes; below 0: read too far, which the mask undoes
-  if (!((row == 0x3000u || rest <= 0) && gone - z <= 7u && gone <= 31u && z < 24u && rest <= 16 && (int)used + 4 * rest <= 96)) return false;
+  const uint32_t gone = z + (sum & 0xffu);
+  const int rest = (int)(planes - gone), used = (int)(sum >> 16);   // verbatim planes; below 0: read too far, which the mask undoes
+  if (!((!row || rest <= 0) && (sum & 0xffu) <= 7u && z < 24u && rest <= 16 && used + 4 * rest <= 96)) return false;
   const uint32_t* const nib = tab + kDecNibbles;
   const uint32_t W = ((nib[x0 & 255u] * 4u + nib[(x0 >> 8) & 255u]) * 4u + nib[(x0 >> 16) & 255u]) * 4u + nib[x0 >> 24];
   const uint32_t m = gone < 24u ? pow2_factor(24u - gone) : 1u, r = gone < 24u ? 0u : gone - 24u;
@@ -598,7 +597,7 @@ GCOW_HD bool decode_code_1d(float* f, const ZfpParams& p, const uint32_t* tab, c
   for (int i = 0; i < 4; i++) q[i] = nb2int(u[i] & mask);
   inv_lift(q[0], q[1], q[2], q[3]);
   const int ef = (int)e8 - 30 - shift;                     // a normal float unless the block is tiny
-  const float scale = (ef >= 1 && ef <= 254) ? bits_f32((uint32_t)ef << 23) : pow2f((int)e8 - kEBias - 30 - shift);
+  const float scale = bits_f32(ef >= 1 ? (uint32_t)ef << 23 : shl_sat(1u, (uint32_t)(ef + 22)));
 #pragma unroll
   for (int i = 0; i < 4; i++) f[i] = scale * (float)q[i];
   return true;

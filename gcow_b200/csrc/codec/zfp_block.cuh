@@ -133,6 +133,36 @@ GCOW_HD void inv_lift(int32_t& x_, int32_t& y_, int32_t& z_, int32_t& w_) {
   x_ = (int32_t)x; y_ = (int32_t)y; z_ = (int32_t)z; w_ = (int32_t)w;
 }
 
+// a + b on the FMA pipe: a times 1, which the compiler cannot know it is. The fixed-rate straight lines below fill the integer ALU (half
+// the issue rate) twice as full as that pipe; with their sums moved there 67 M values at 8 bits/value take 68.7 instead of 70.3 us
+// (encoding) and 81.0 instead of 83.1. The tile coders, which have other work for it, get slower by 1 to 3 %.
+GCOW_HD uint32_t add_fma(uint32_t a, uint32_t b) {
+#if defined(__CUDA_ARCH__)
+  return a * blockDim.z + b;
+#else
+  return a + b;
+#endif
+}
+// The two lifts and the negabinary maps with it.
+GCOW_HD void fwd_lift_fma(int32_t& x_, int32_t& y_, int32_t& z_, int32_t& w_) {
+  uint32_t x = (uint32_t)x_, y = (uint32_t)y_, z = (uint32_t)z_, w = (uint32_t)w_;
+  x = asr1(add_fma(x, w)); w -= x;
+  z = asr1(add_fma(z, y)); y -= z;
+  x = asr1(add_fma(x, z)); z -= x;
+  w = asr1(add_fma(w, y)); y -= w;
+  w = add_fma(w, asr1(y)); y -= asr1(w);
+  x_ = (int32_t)x; y_ = (int32_t)y; z_ = (int32_t)z; w_ = (int32_t)w;
+}
+GCOW_HD void inv_lift_fma(int32_t& x_, int32_t& y_, int32_t& z_, int32_t& w_) {
+  uint32_t x = (uint32_t)x_, y = (uint32_t)y_, z = (uint32_t)z_, w = (uint32_t)w_, t;
+  y = add_fma(y, asr1(w)); w -= asr1(y);
+  t = w; w -= y; y = add_fma(y, t);                          // (y, w) = (y + w, 2 w - (y + w)), and so on
+  t = x; x -= z; z = add_fma(z, t);
+  t = z; z -= y; y = add_fma(y, t);
+  t = x; x -= w; w = add_fma(w, t);
+  x_ = (int32_t)x; y_ = (int32_t)y; z_ = (int32_t)z; w_ = (int32_t)w;
+}
+
 template <int DIM> struct Xform;
 template <> struct Xform<1> {
   static GCOW_HD void fwd(int32_t* q) { fwd_lift(q[0], q[1], q[2], q[3]); }
@@ -161,6 +191,8 @@ template <> struct Xform<2> {
 
 GCOW_HD uint32_t int2nb(int32_t x) { return ((uint32_t)x + kNbMask) ^ kNbMask; }
 GCOW_HD int32_t nb2int(uint32_t u) { return (int32_t)((u ^ kNbMask) - kNbMask); }
+GCOW_HD uint32_t int2nb_fma(int32_t x) { return add_fma((uint32_t)x, kNbMask) ^ kNbMask; }
+GCOW_HD int32_t nb2int_fma(uint32_t u) { return (int32_t)add_fma(u ^ kNbMask, 0u - kNbMask); }
 
 template <int DIM>
 GCOW_HD void fwd_reorder(uint32_t* u, const int32_t* q) {
@@ -805,9 +837,12 @@ inline void build_codec_tables(uint16_t* etab, uint16_t* dtab_budget) {
 //    needs a transpose either.
 //
 // Both are bound by the integer ALU (half the issue rate), so sums of shifted fields are
-// multiplications by powers of two, which run on the FMA pipe. Measured at 67 M values
+// multiplications by powers of two, which run on the FMA pipe, and so do half of the lifts' sums. Measured at 67 M values
 // and 8 bits/value: encoding 104.7 -> 76.3 us (155 -> 101 instructions per warp of
-// blocks), decoding 135.8 -> 90.9 us (212 -> 132).
+// blocks), decoding 135.8 -> 90.9 us (212 -> 132). Instructions are what bounds both (input that is in the L2 takes the same time per
+// value, and so does input fetched ahead into shared memory): with a NaN seen in the maximum instead of a sum, the windows'
+// counts in one register, checked in one operation, and sums on the FMA pipe 73.9 -> 67.7 and 88.4 -> 79.5; at 16 bits/value 106.4 ->
+// 101.8 and 118.1 -> 109.2, 32 bits/value 200 -> 190 and 222 -> 207.
 //
 // Inputs the fast path does not cover (a non-finite or vanishing block maximum, a NaN
 // member, data so smooth that eight planes - in the decoder, three lookups - do not reach
@@ -890,6 +925,23 @@ GCOW_HD uint32_t shr_sat(uint32_t v, uint32_t s) {   // v >> s, 0 for s >= 32
 #endif
 }
 
+// Bits of a block's largest magnitude, and whether the straight lines below take the block: its exponent is in lowest..254 and no member
+// is a NaN. On the device a NaN comes through the maximum (exponent 255), which saves adding the members up to see one.
+GCOW_HD uint32_t block_max_bits(const float* f, uint32_t lowest, bool& ordinary) {
+#if defined(__CUDA_ARCH__)
+  float a, b;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(a) : "f"(fabsf(f[0])), "f"(fabsf(f[1])));
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(b) : "f"(fabsf(f[2])), "f"(fabsf(f[3])));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(a) : "f"(b));
+  const uint32_t mb = f32_bits(a);
+#else
+  const bool nan = f[0] != f[0] || f[1] != f[1] || f[2] != f[2] || f[3] != f[3];
+  const uint32_t mb = nan ? 0x7fffffffu : f32_bits(fmaxf(fmaxf(fabsf(f[0]), fabsf(f[1])), fmaxf(fabsf(f[2]), fabsf(f[3]))));
+#endif
+  ordinary = (mb >> 23) - lowest <= 254u - lowest;
+  return mb;
+}
+
 // BITS bits held in registers, addressed by bit position.
 template <int NW> struct BitBuf;
 template <> struct BitBuf<1> {
@@ -937,8 +989,9 @@ template <> struct BitBuf<4> {
 
 // Decoder tables, one array of words:
 //  * windows: two words at byte offset n * 4096 + 8 * (next nine bits), n = 0..2: the planes that end within the nine bits
-//    and start with n < 3, at most four. First word: byte i = coefficient i's bits, last plane lowest. Second word: bits
-//    used | planes << 8 | min(n', 3) << 12 - masked with 0x3000 the row offset of the next lookup.
+//    and start with n < 3, at most four. First word: byte i = coefficient i's bits, last plane lowest. Second word: planes |
+//    (n' < 3 ? n' + 1 : 0) << 12 | bits used << 16, so that a shift by it is one by the planes, its sum over the windows holds both
+//    counts, and masked with 0x3000 it is 0 at the end, else the next lookup's row (one row further on).
 //  * nibbles: at kDecNibbles + v, the two verbatim planes v as two bits per byte, first plane higher.
 //  * tiny: at kDecTiny + v, the whole of a block with seven payload bits v: byte i = the top eight planes of coefficient i.
 constexpr int kDecNibbles = 3 * 512 * 2, kDecTiny = kDecNibbles + 256, kDecLoopTabSize = kDecTiny + 128;
@@ -958,6 +1011,8 @@ GCOW_HD uint32_t make_dec_loop_entry(uint32_t i) {
   }
   if (i >= (uint32_t)kDecNibbles) return (spread_nibble(i & 15u) << 1) | spread_nibble(((i - kDecNibbles) >> 4) & 15u);
   uint32_t n = i >> 10, v = (i >> 1) & 511u, used = 0, planes = 0, u = 0;
+  // No plane follows the leading zero ones: the block's bits are at their end (the first plane behind those holds a one).
+  if (n == 0 && !(v & 1u)) return 0;
   while (n < 3 && planes < 4) {
     const uint32_t e = make_dec_budget_entry(n, 7, v & 127u), len = (e >> 4) & 7u;
     if (used + len > 9) break;
@@ -967,7 +1022,7 @@ GCOW_HD uint32_t make_dec_loop_entry(uint32_t i) {
     planes++;
     n = e >> 7;
   }
-  return i & 1u ? used | (planes << 8) | ((n < 3 ? n : 3u) << 12) : u;
+  return i & 1u ? planes | (n < 3 ? (n + 1) << 12 : 0u) | used << 16 : u;
 }
 
 struct alignas(8) DecWindow { uint32_t u, meta; };
@@ -983,12 +1038,12 @@ struct LeanTables {
 template <int BITS>
 GCOW_HD bool encode_block_1d_try(const float* f, const LeanTables& t, uint32_t (&w)[(BITS + 31) / 32], uint32_t kmin) {
   constexpr int NW = (BITS + 31) / 32;
-  const uint32_t mb = f32_bits(fmaxf(fmaxf(fabsf(f[0]), fabsf(f[1])), fmaxf(fabsf(f[2]), fabsf(f[3]))));
+  bool finite;
+  const uint32_t mb = block_max_bits(f, 29, finite);
   const uint32_t ex = mb >> 23;
   // 2^(30 - emax), emax = ex - 126; only used with 29 <= ex <= 254
   const float scale = bits_f32(0x8d800000u - (mb & 0xff800000u));
   const float p0 = scale * f[0], p1 = scale * f[1], p2 = scale * f[2], p3 = scale * f[3];
-  const bool finite = ex - 29u <= 225u && fabsf((p0 + p1) + (p2 + p3)) < 8.0e9f;       // the sum: a NaN member
   int32_t q[4];
 #if defined(__CUDA_ARCH__)
   q[0] = __float2int_rz(p0); q[1] = __float2int_rz(p1); q[2] = __float2int_rz(p2); q[3] = __float2int_rz(p3);
@@ -996,13 +1051,12 @@ GCOW_HD bool encode_block_1d_try(const float* f, const LeanTables& t, uint32_t (
   if (!finite) return false;                                  // out of range for this conversion
   q[0] = (int32_t)p0; q[1] = (int32_t)p1; q[2] = (int32_t)p2; q[3] = (int32_t)p3;
 #endif
-  fwd_lift(q[0], q[1], q[2], q[3]);
+  fwd_lift_fma(q[0], q[1], q[2], q[3]);
   uint32_t u[4];
 #pragma unroll
-  for (int i = 0; i < 4; i++) u[i] = int2nb(q[i]);
+  for (int i = 0; i < 4; i++) u[i] = int2nb_fma(q[i]);
   const uint32_t mm = u[0] | u[1] | u[2] | u[3];
-  uint32_t z = mm ? clz32(mm) : 32u;
-  if (z > 24) z = 24;                                         // further zero planes go through the table (one 0 bit each)
+  uint32_t z = clz32(mm | 0x80u);                             // at most 24: further zero planes go through the table (one 0 bit each)
   // pairs of planes through the table: 16-bit blocks have seven payload bits, always exceeded by four planes; 64-bit
   // blocks take sixteen planes, which fill the 55 bits on anything but smooth data
   constexpr int kPairs = BITS == 16 ? 2 : BITS == 64 ? 8 : 4;
@@ -1048,7 +1102,8 @@ GCOW_HD bool encode_block_1d_try(const float* f, const LeanTables& t, uint32_t (
     buf.store(w);
   }
   if (BITS < 32 * NW) w[NW - 1] &= low_mask32(BITS - 32 * (NW - 1));
-  return finite && (pos >= (uint32_t)BITS || k <= (int)kmin);
+  // 16 and 32 bits: the first planes fill them wherever z has reached its limit
+  return finite && (pos >= (uint32_t)BITS || ((BITS > 32 || kmin > 0) && k <= (int)kmin));
 }
 // The blocks encode_block_1d_try leaves: zeros, a member or maximum out of its range, very smooth data.
 template <int BITS>
@@ -1085,26 +1140,31 @@ GCOW_HD bool decode_block_1d_try(float* f, const LeanTables& t, const uint32_t (
     const uint32_t lead = buf.peek(kHeaderBits);
     const uint32_t z = kPayload < 32 ? (uint32_t)ctz32(lead | (1u << (kPayload < 32 ? kPayload : 0)))
                                      : (lead ? (uint32_t)ctz32(lead) : 32u);
-    uint32_t pos = kHeaderBits + z;
     // planes with n < 3, whole ones only: on noise at 8 bits/value one lookup does for 86.6 % of the blocks, two for 99.3 %, three
     // for all but one in 10^6; 6 blocks in 10^4 end in a plane that the budget cuts and are left
     const char* const win = reinterpret_cast<const char*>(t.dloop);
-    uint32_t U = 0, gone = z, row = 0;                         // gone: planes above the next one
+    uint32_t sum = (kHeaderBits + z) << 16;                    // of the windows' second words: planes in the low byte, position in the third
+    DecWindow d = *reinterpret_cast<const DecWindow*>(win + 8u * (buf.peek(kHeaderBits + z) & 511u));
+    uint32_t U = d.u, row = d.meta & 0x3000u;
+    sum += d.meta;
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      if (c == 0 || (row != 0x3000u && pos < (uint32_t)BITS)) {
-        const DecWindow d = *reinterpret_cast<const DecWindow*>(win + row + 8u * (buf.peek(pos) & 511u));
-        const uint32_t n = (d.meta >> 8) & 15u;
-        U = (U << n) | d.u;
-        gone += n;
-        pos += d.meta & 31u;
+    for (int c = 1; c < 3; c++) {
+      if (row) {
+        d = *reinterpret_cast<const DecWindow*>(win + (row - 0x1000u) + 8u * (buf.peek((sum >> 16) & 0xffu) & 511u));
+        U = funnel_l(0u, U, d.meta) | d.u;
         row = d.meta & 0x3000u;
+        sum += d.meta;
       }
     }
+    uint32_t pos = (sum >> 16) & 0xffu;
+    const uint32_t gone = z + (sum & 0xffu);                   // planes above the next one
     // Left for the definition path: a plane that the budget cuts (the zeros past the end completed it), still n < 3, more
     // than seven planes (U's bytes), planes below the last one (BITS >= 64 only: 23 payload bits hold no more than 23 planes).
-    whole = whole && pos <= (uint32_t)BITS && (row == 0x3000u || pos == (uint32_t)BITS || gone + kmin >= 32u) && gone - z <= 7u &&
-            (NW == 1 || gone <= 31u);
+    // A count's limit is passed where bit 7 of its byte is set after adding what lacks.
+    constexpr uint32_t kLimits = (127u - 7u) | (BITS < 127 ? 127u - BITS : 0u) << 16;
+    const uint32_t over = ((sum + kLimits) & 0x00800080u) | row | (~w[0] & 1u);
+    whole = over == 0 && (NW == 1 || gone <= 31u);
+    if (kmin) whole = (w[0] & 1u) && pos <= (uint32_t)BITS && (!row || gone + kmin >= 32u) && (sum & 0xffu) <= 7u && (NW == 1 || gone <= 31u);
     // the rest of the block is verbatim nibbles; bits past its end read as 0
     const uint32_t* const nib = t.dloop + kDecNibbles;
     const uint32_t tail = buf.peek(pos);
@@ -1135,12 +1195,20 @@ GCOW_HD bool decode_block_1d_try(float* f, const LeanTables& t, const uint32_t (
     }
   }
   int32_t q[4];
+  const int ef = (int)e8 - 30 - shift;                         // 2^(emax - 30 - shift): a normal float unless the block is tiny
+  float scale;
+  if (BITS == 16) {                                            // bound by memory: the plain forms
 #pragma unroll
-  for (int i = 0; i < 4; i++) q[i] = nb2int(u[i] & planemask);
-  inv_lift(q[0], q[1], q[2], q[3]);
-  // 2^(emax - 30 - shift): a normal float unless the block is tiny
-  const int ef = (int)e8 - 30 - shift;
-  const float scale = (ef >= 1 && ef <= 254) ? bits_f32((uint32_t)ef << 23) : pow2f((int)e8 - kEBias - 30 - shift);
+    for (int i = 0; i < 4; i++) q[i] = nb2int(u[i] & planemask);
+    inv_lift(q[0], q[1], q[2], q[3]);
+    scale = (ef >= 1 && ef <= 254) ? bits_f32((uint32_t)ef << 23) : pow2f(ef - 127);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; i++) q[i] = nb2int_fma(u[i] & planemask);
+    inv_lift_fma(q[0], q[1], q[2], q[3]);
+    scale = bits_f32(ef >= 1 ? (uint32_t)ef << 23 : shl_sat(1u, (uint32_t)(ef + 22)));
+    whole = whole && shift >= -29;                             // else it may be infinite
+  }
 #pragma unroll
   for (int i = 0; i < 4; i++) f[i] = scale * (float)q[i];
   return whole;
@@ -1169,11 +1237,11 @@ GCOW_HD void decode_block_1d_lean(float* f, const LeanTables& t, const uint32_t 
 template <int BITS>
 GCOW_HD bool roundtrip_block_1d_try(float* f) {
   constexpr int P = BITS - (int)kHeaderBits;
-  const uint32_t mb = f32_bits(fmaxf(fmaxf(fabsf(f[0]), fabsf(f[1])), fmaxf(fabsf(f[2]), fabsf(f[3]))));
+  bool ordinary;
+  const uint32_t mb = block_max_bits(f, 30, ordinary);
   const uint32_t ex = mb >> 23;                               // emax = ex - 126
   const float scale = bits_f32(0x8d800000u - (mb & 0xff800000u));   // 2^(30 - emax)
   const float p0 = scale * f[0], p1 = scale * f[1], p2 = scale * f[2], p3 = scale * f[3];
-  const bool ordinary = ex - 30u <= 224u && fabsf((p0 + p1) + (p2 + p3)) < 8.0e9f;     // the sum: a NaN member
   int32_t q[4];
 #if defined(__CUDA_ARCH__)
   q[0] = __float2int_rz(p0); q[1] = __float2int_rz(p1); q[2] = __float2int_rz(p2); q[3] = __float2int_rz(p3);
@@ -1181,10 +1249,10 @@ GCOW_HD bool roundtrip_block_1d_try(float* f) {
   if (!ordinary) return false;                                // out of range for this conversion
   q[0] = (int32_t)p0; q[1] = (int32_t)p1; q[2] = (int32_t)p2; q[3] = (int32_t)p3;
 #endif
-  fwd_lift(q[0], q[1], q[2], q[3]);
+  fwd_lift_fma(q[0], q[1], q[2], q[3]);
   uint32_t u[4];
 #pragma unroll
-  for (int i = 0; i < 4; i++) u[i] = int2nb(q[i]);
+  for (int i = 0; i < 4; i++) u[i] = int2nb_fma(q[i]);
   const uint32_t m2 = u[2] | u[3], m1 = m2 | u[1], m0 = m1 | u[0];
   const bool low = m2 != 0;                                   // top_2 exists
 #if defined(__CUDA_ARCH__)
@@ -1200,8 +1268,8 @@ GCOW_HD bool roundtrip_block_1d_try(float* f) {
   const bool ok = ordinary && low && k <= 31 - l2;
   const uint32_t whole = shl_sat(0xffffffffu, (uint32_t)k), more = k > 0 ? whole | shl_sat(1u, (uint32_t)(k - 1)) : whole;
 #pragma unroll
-  for (int i = 0; i < 4; i++) q[i] = nb2int(u[i] & (i < 3 && i < a ? more : whole));
-  inv_lift(q[0], q[1], q[2], q[3]);
+  for (int i = 0; i < 4; i++) q[i] = nb2int_fma(u[i] & (i < 3 && i < a ? more : whole));
+  inv_lift_fma(q[0], q[1], q[2], q[3]);
   if (!ok) return false;
   const float back = bits_f32((ex - 29u) << 23);              // 2^(emax - 30)
 #pragma unroll
@@ -1217,11 +1285,12 @@ GCOW_HD bool roundtrip_block_1d_try(float* f) {
 template <int BITS>
 GCOW_HD bool roundtrip_block_1d_cut(float* f) {
   constexpr int P = BITS - (int)kHeaderBits;
-  const uint32_t mb = f32_bits(fmaxf(fmaxf(fabsf(f[0]), fabsf(f[1])), fmaxf(fabsf(f[2]), fabsf(f[3]))));
+  bool ordinary;
+  const uint32_t mb = block_max_bits(f, 30, ordinary);
+  if (!ordinary) return false;
   const uint32_t ex = mb >> 23;
   const float scale = bits_f32(0x8d800000u - (mb & 0xff800000u));
   const float p0 = scale * f[0], p1 = scale * f[1], p2 = scale * f[2], p3 = scale * f[3];
-  if (!(ex - 30u <= 224u && fabsf((p0 + p1) + (p2 + p3)) < 8.0e9f)) return false;
   int32_t q[4] = {(int32_t)p0, (int32_t)p1, (int32_t)p2, (int32_t)p3};
   fwd_lift(q[0], q[1], q[2], q[3]);
   uint32_t u[4];

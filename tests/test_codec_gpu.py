@@ -284,3 +284,21 @@ def test_variable_rate_result_on_another_stream(dim, how):
         torch.cuda.synchronize()
         assert torch.equal(stream, c.stream) and torch.equal(index, c.index) and torch.equal(y, g.decompress(c))
         assert c.nbytes == (int(index[-1]) + 63) // 64 * 8
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rate", [4, 8, 16, 32])
+def test_long_vectors_equal_their_pieces(rate):
+    """Vectors long enough for the larger grid of the fixed-rate kernels, against the same values in pieces, which are short."""
+    n = 4 * (32 * 148 * 4 * 512 + 777) + 3
+    x = torch.randn(n, device="cuda", generator=torch.Generator("cuda").manual_seed(rate)) * 1e-3
+    x[::4099] = float("nan")
+    x[n // 3:n // 2] += 1
+    x[n // 2:n // 2 + 100000] = 0
+    x[-n // 5::9] *= 1e-36
+    c = g.compress(x, rate=rate)
+    piece = 1 << 22
+    parts = [g.compress(x[i:i + piece], rate=rate) for i in range(0, n, piece)]
+    assert torch.equal(c.stream, torch.cat([p.stream for p in parts]))
+    y = g.decompress(c)
+    assert torch.equal(y.view(torch.int32), torch.cat([g.decompress(p) for p in parts]).view(torch.int32))
