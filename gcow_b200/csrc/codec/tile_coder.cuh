@@ -149,14 +149,11 @@ GCOW_HD uint32_t finish_slot(const SlotWriter& s, uint32_t* slot, uint32_t strid
 }
 
 // Cast of a block to integers relative to 2^(emax - 30). The clamping conversion (values out
-// of range, NaN) is only needed with a non-finite member or a vanishing maximum.
+// of range, NaN) is only needed where the block is not ordinary: a non-finite member or a vanishing maximum.
 template <int N>
-GCOW_HD void cast_block(int32_t* q, const float* f, int emax) {
+GCOW_HD void cast_block(int32_t* q, const float* f, int emax, bool ordinary) {
   const float scale = pow2f(30 - emax);
-  float s = 0;
-#pragma unroll
-  for (int i = 0; i < N; i++) s += scale * f[i];
-  if (emax >= -97 && fabsf(s) < (float)N * 2.0e9f) {       // false for NaN and infinity
+  if (ordinary) {
 #pragma unroll
     for (int i = 0; i < N; i++) {
 #if defined(__CUDA_ARCH__)
@@ -177,6 +174,12 @@ GCOW_HD int block_emax_fmax(const float* f) {              // block_emax with th
   for (int i = 0; i < N; i++) m = fmaxf(m, fabsf(f[i]));
   return scalar_exponent(m);
 }
+// The exponent of a block's largest magnitude (emax), NaN members skipped, and whether the plain conversion serves.
+template <int N>
+GCOW_HD int block_exponent(const float* f, bool& ordinary) {
+  const uint32_t mb = block_max_bits<N>(f, 29, ordinary);    // scale * f is below 2^31 and the scale a normal float
+  return ordinary ? (int)(mb >> 23) - 126 : block_emax_fmax<N>(f);
+}
 
 // ------------------------------------------------------------------- 1-D encoder
 // The planes below the leading all-zero ones are coded two per lookup for the first eight, a
@@ -184,13 +187,14 @@ GCOW_HD int block_emax_fmax(const float* f) {              // block_emax with th
 // zero plane minus that plane's own zero bits), and verbatim nibbles follow once n >= 3.
 GCOW_HD uint32_t encode_slot_1d(const float* f, const ZfpParams& p, const uint32_t* epair, const uint16_t* etab,
                                 uint32_t* slot, uint32_t stride) {
-  const int emax = block_emax_fmax<4>(f);
+  bool ordinary;
+  const int emax = block_exponent<4>(f, ordinary);
   const uint32_t prec = block_precision(emax, p.maxprec, p.minexp, 1);
   const uint32_t biased = prec ? (uint32_t)(emax + kEBias) : 0;
   if (!biased) { *slot = 0; return 1; }
   int32_t q[4];
   uint32_t u[4];
-  cast_block<4>(q, f, emax);
+  cast_block<4>(q, f, emax, ordinary);
   fwd_lift(q[0], q[1], q[2], q[3]);
 #pragma unroll
   for (int i = 0; i < 4; i++) u[i] = int2nb(q[i]);
@@ -261,7 +265,7 @@ GCOW_HD void append64(uint32_t (&w)[4], uint32_t at, uint32_t lo, uint32_t hi) {
 // sixteen verbatim ones, a code of more than 128 bits. No budget: the block's code must not reach maxbits.
 GCOW_HD bool encode_code_1d(const float* f, const ZfpParams& p, const uint32_t* epair, uint32_t (&w)[4], uint32_t& length) {
   bool ok;
-  const uint32_t mb = block_max_bits(f, 29, ok), ex = mb >> 23;
+  const uint32_t mb = block_max_bits<4>(f, 29, ok), ex = mb >> 23;
   const float scale = bits_f32(0x8d800000u - (mb & 0xff800000u));   // 2^(30 - emax), emax = ex - 126; used with 29 <= ex <= 254
   const float p0 = scale * f[0], p1 = scale * f[1], p2 = scale * f[2], p3 = scale * f[3];
   const uint32_t prec = block_precision((int)ex - 126, p.maxprec, p.minexp, 1), planes = prec < 32u ? prec : 32u;
@@ -373,13 +377,14 @@ GCOW_HD void transpose16_inv(uint32_t* w) {
 // 30 -> 23 and 38 -> 25.
 template <bool kBudget>
 GCOW_HD uint32_t encode_slot_2d(const float* f, const ZfpParams& p, const uint32_t* twin, uint32_t* slot, uint32_t stride) {
-  const int emax = block_emax_fmax<16>(f);
+  bool ordinary;
+  const int emax = block_exponent<16>(f, ordinary);
   const uint32_t prec = block_precision(emax, p.maxprec, p.minexp, 2);
   const uint32_t biased = prec ? (uint32_t)(emax + kEBias) : 0;
   if (!biased) { *slot = 0; return 1; }
   int32_t q[16];
   uint32_t u[16];
-  cast_block<16>(q, f, emax);
+  cast_block<16>(q, f, emax, ordinary);
   Xform<2>::fwd(q);
   fwd_reorder<2>(u, q);
   uint32_t others = 0;

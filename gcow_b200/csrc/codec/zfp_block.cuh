@@ -83,6 +83,24 @@ GCOW_HD int scalar_exponent(float m) {
   return (int)ex - 126;
 }
 
+// Bits of a block's largest magnitude, a NaN's (exponent 255) where a member is one: on the device it comes through the maximum, which
+// saves adding the members up to see one. `ordinary`: the exponent is in lowest..254.
+template <int N>
+GCOW_HD uint32_t block_max_bits(const float* f, uint32_t lowest, bool& ordinary) {
+#if defined(__CUDA_ARCH__)
+  float m = fabsf(f[0]);
+#pragma unroll
+  for (int i = 1; i + 1 < N; i += 2) asm("max.NaN.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(fabsf(f[i])), "f"(fabsf(f[i + 1])));
+  if (N % 2 == 0) asm("max.NaN.f32 %0, %0, %1;" : "+f"(m) : "f"(fabsf(f[N - 1])));
+  const uint32_t mb = f32_bits(m);
+#else
+  uint32_t mb = 0;                                           // magnitudes compare as their bits do
+  for (int i = 0; i < N; i++) mb = mb < (f32_bits(f[i]) & 0x7fffffffu) ? f32_bits(f[i]) & 0x7fffffffu : mb;
+#endif
+  ordinary = (mb >> 23) - lowest <= 254u - lowest;
+  return mb;
+}
+
 template <int N>
 GCOW_HD int block_emax(const float* f) {
   float m = 0;
@@ -925,23 +943,6 @@ GCOW_HD uint32_t shr_sat(uint32_t v, uint32_t s) {   // v >> s, 0 for s >= 32
 #endif
 }
 
-// Bits of a block's largest magnitude, and whether the straight lines below take the block: its exponent is in lowest..254 and no member
-// is a NaN. On the device a NaN comes through the maximum (exponent 255), which saves adding the members up to see one.
-GCOW_HD uint32_t block_max_bits(const float* f, uint32_t lowest, bool& ordinary) {
-#if defined(__CUDA_ARCH__)
-  float a, b;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(a) : "f"(fabsf(f[0])), "f"(fabsf(f[1])));
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(b) : "f"(fabsf(f[2])), "f"(fabsf(f[3])));
-  asm("max.NaN.f32 %0, %0, %1;" : "+f"(a) : "f"(b));
-  const uint32_t mb = f32_bits(a);
-#else
-  const bool nan = f[0] != f[0] || f[1] != f[1] || f[2] != f[2] || f[3] != f[3];
-  const uint32_t mb = nan ? 0x7fffffffu : f32_bits(fmaxf(fmaxf(fabsf(f[0]), fabsf(f[1])), fmaxf(fabsf(f[2]), fabsf(f[3]))));
-#endif
-  ordinary = (mb >> 23) - lowest <= 254u - lowest;
-  return mb;
-}
-
 // BITS bits held in registers, addressed by bit position.
 template <int NW> struct BitBuf;
 template <> struct BitBuf<1> {
@@ -1039,7 +1040,7 @@ template <int BITS>
 GCOW_HD bool encode_block_1d_try(const float* f, const LeanTables& t, uint32_t (&w)[(BITS + 31) / 32], uint32_t kmin) {
   constexpr int NW = (BITS + 31) / 32;
   bool finite;
-  const uint32_t mb = block_max_bits(f, 29, finite);
+  const uint32_t mb = block_max_bits<4>(f, 29, finite);
   const uint32_t ex = mb >> 23;
   // 2^(30 - emax), emax = ex - 126; only used with 29 <= ex <= 254
   const float scale = bits_f32(0x8d800000u - (mb & 0xff800000u));
@@ -1238,7 +1239,7 @@ template <int BITS>
 GCOW_HD bool roundtrip_block_1d_try(float* f) {
   constexpr int P = BITS - (int)kHeaderBits;
   bool ordinary;
-  const uint32_t mb = block_max_bits(f, 30, ordinary);
+  const uint32_t mb = block_max_bits<4>(f, 30, ordinary);
   const uint32_t ex = mb >> 23;                               // emax = ex - 126
   const float scale = bits_f32(0x8d800000u - (mb & 0xff800000u));   // 2^(30 - emax)
   const float p0 = scale * f[0], p1 = scale * f[1], p2 = scale * f[2], p3 = scale * f[3];
@@ -1286,7 +1287,7 @@ template <int BITS>
 GCOW_HD bool roundtrip_block_1d_cut(float* f) {
   constexpr int P = BITS - (int)kHeaderBits;
   bool ordinary;
-  const uint32_t mb = block_max_bits(f, 30, ordinary);
+  const uint32_t mb = block_max_bits<4>(f, 30, ordinary);
   if (!ordinary) return false;
   const uint32_t ex = mb >> 23;
   const float scale = bits_f32(0x8d800000u - (mb & 0xff800000u));
