@@ -221,7 +221,9 @@ finalize_bwd_kernel(const float* __restrict__ part, int parts, int C, float* __r
   dbeta[c] = (float)s; dgamma[c] = (float)q;
 }
 
-// ---- backward sweep 2: dx = gamma*rstd * (g - dbeta/R - xhat*dgamma/R)
+// ---- backward sweep 2: dx = gamma*rstd * (g - dbeta/R - xhat*dgamma/R). From the last row to the first: sweep 1 has just read the last
+// ones, which the L2 still holds, and what reads dx next finds its first rows there. Backward of 256 x 128 x 28 x 28: 57.8 -> 55.4 us, x 2048 x
+// 7 x 7 62.8 -> 60.7, x 64 x 56 x 56 102.3 -> 100.7, x 256 x 56 x 56 as before. (The forward's second sweep backwards: 33.5 -> 38.2 us.)
 __global__ void __launch_bounds__(kThreads)
 bwd_dx_kernel(const bf16* __restrict__ dy, const uint8_t* __restrict__ mask, const bf16* __restrict__ x,
               const float* __restrict__ gamma, const float* __restrict__ mean, const float* __restrict__ rstd,
@@ -241,7 +243,7 @@ bwd_dx_kernel(const bf16* __restrict__ dy, const uint8_t* __restrict__ mask, con
     k2[i] = dgamma[c] * invR;
   }
 #pragma unroll 4
-  for (int64_t r = (int64_t)blockIdx.x * rstep + r0; r < R; r += (int64_t)gridDim.x * rstep) {
+  for (int64_t r = R - 1 - (int64_t)blockIdx.x * rstep - r0; r >= 0; r -= (int64_t)gridDim.x * rstep) {
     const int64_t off = r * C + g * 8;
     float gv[8], xv[8];
     load8(dy + off, gv);

@@ -7,6 +7,7 @@
 //
 // The reference's models get these from ATen/cuDNN through PyTorch
 // (hw/models/resenet.py:12-22,80-89; cross-entropy at hw/models/train_imagenet.py:249).
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -500,6 +501,55 @@ colsum_partial8_kernel(const bf16* __restrict__ g, float* __restrict__ part, int
   }
 }
 
+// Few rows, one launch: a cluster of eight CTAs takes 64 columns, an eighth of the rows each; 16-byte loads (8 columns per thread, 32
+// row lanes per CTA), folded through shared memory, then CTA r adds up columns 8 r .. 8 r + 7 of all eight in their order. Bound by latency,
+// of which a second launch is the larger part: 2048 x 128 5.1 -> 3.4 us, x 768 5.4 -> 3.5, x 3072 6.1 -> 5.0, 3072 x 1024 5.3 -> 4.4. With more
+// rows a CTA has too many to itself (16384 x 1024 9.6 -> 17.6): those stay with the two kernels above.
+constexpr int kSumCols = 64, kSumCtas = 8, kSumLanes = 32, kSumRows = 4096;
+__global__ void __cluster_dims__(1, kSumCtas, 1) __launch_bounds__(256)
+colsum_cluster_kernel(const bf16* g, float* __restrict__ out, int rows, int cols, int ld) {
+  __shared__ float red[kSumLanes][kSumCols + 4], quarter[4][kSumCols], sum[kSumCols];
+  pdl_trigger();
+  pdl_wait();
+  const int tid = threadIdx.x, cg = tid & 7, rl = tid >> 3;      // column group (8 columns), row lane
+  const int c = blockIdx.x * kSumCols + cg * 8;
+  const int r0 = (int)((int64_t)rows * blockIdx.y / kSumCtas), r1 = (int)((int64_t)rows * (blockIdx.y + 1) / kSumCtas);
+  float acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) acc[j] = 0.0f;
+  if (c < cols) {
+#pragma unroll 8
+    for (int r = r0 + rl; r < r1; r += kSumLanes) {
+      const uint4 v = *reinterpret_cast<const uint4*>(g + (size_t)r * ld + c);
+      const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+      for (int e = 0; e < 4; e++) { const float2 f = __bfloat1622float2(b[e]); acc[2 * e] += f.x; acc[2 * e + 1] += f.y; }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; j++) red[rl][cg * 8 + j] = acc[j];
+  __syncthreads();
+  {
+    const int col = tid & (kSumCols - 1), q = tid / kSumCols;
+    float s = 0.0f;
+#pragma unroll
+    for (int l = 0; l < kSumLanes / 4; l++) s += red[q * (kSumLanes / 4) + l][col];   // fixed order
+    quarter[q][col] = s;
+  }
+  __syncthreads();
+  if (tid < kSumCols) sum[tid] = (quarter[0][tid] + quarter[1][tid]) + (quarter[2][tid] + quarter[3][tid]);
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  cluster.sync();
+  const int mine = (int)blockIdx.y * 8 + tid, col = blockIdx.x * kSumCols + mine;
+  if (tid < 8 && col < cols) {
+    float s = 0.0f;
+#pragma unroll
+    for (int k = 0; k < kSumCtas; k++) s += cluster.map_shared_rank(sum, k)[mine];
+    out[col] = s;
+  }
+  cluster.sync();                                                // the others' sums are read until here
+}
+
 // ------------------------------------------------------- image normalisation
 // uint8 NHWC [n, 3] pixels -> bf16 NHWC padded to `cpad` channels (extra channels 0):
 // y = (x - mean_c) / std_c with mean/std given in 0..255 units.
@@ -616,8 +666,17 @@ int gcow_softmax_bwd(const void* dp, const void* p, void* ds, int64_t rows, int 
 // Column sums of a bf16 [rows, cols] matrix (ld even, cols even) into fp32 out[cols];
 // `part` must hold gcow_colsum_parts(rows) * cols floats.
 int gcow_colsum_parts(int rows) { int p = (rows + 127) / 128; return p < 128 ? (p < 1 ? 1 : p) : 128; }
+// Kernels that gcow_colsum launches: one (`part` is not used), or the partial sums and their reduction.
+int gcow_colsum_launches(const void* g, int rows, int cols, int ld) {
+  return rows <= kSumRows && cols % 8 == 0 && ld % 8 == 0 && ((uintptr_t)g & 15) == 0 ? 1 : 2;
+}
 int gcow_colsum(const void* g, float* part, float* out, int rows, int cols, int ld, void* stream) {
   if (cols % 2 || ld % 2 || rows <= 0) return -1;
+  if (gcow_colsum_launches(g, rows, cols, ld) == 1) {
+    gcow::launch_dependent(colsum_cluster_kernel, dim3((cols + kSumCols - 1) / kSumCols, kSumCtas), dim3(256), 0, (cudaStream_t)stream,
+                           (const bf16*)g, out, rows, cols, ld);
+    return (int)cudaGetLastError();
+  }
   const int parts = gcow_colsum_parts(rows);
   const int rows_per = (rows + parts - 1) / parts;
   if (cols % 8 == 0 && ld % 8 == 0 && ((uintptr_t)g & 15) == 0) {

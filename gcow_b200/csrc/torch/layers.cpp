@@ -39,6 +39,7 @@ int gcow_gemm_bf16_batched(const void* A, const void* B, void* C, int M, int N, 
                            int flags, uint32_t* error, int a_mn, int b_mn, int tile_rows, void* stream);
 int gcow_reduce_partials(const float* part, float* out, int parts, int64_t n, void* stream);
 int gcow_colsum_parts(int rows);
+int gcow_colsum_launches(const void* g, int rows, int cols, int ld);
 int gcow_colsum(const void* g, float* part, float* out, int rows, int cols, int ld, void* stream);
 int gcow_layernorm_fwd(const void* x, const float* gamma, const float* beta, void* y, float* mean, float* rstd, int rows, int H,
                        float eps, void* stream);
@@ -261,9 +262,10 @@ Tensor colsum(const Tensor& g, const On& on) {
   const int64_t rows = g.size(0), cols = g.size(1);
   if (cols % 2 || g.stride(1) != 1 || g.stride(0) % 2) return g.to(at::kFloat).sum(0);
   TORCH_CHECK(g.dim() == 2 && g.scalar_type() == at::kBFloat16, "colsum: expected a bf16 matrix");
-  const Tensor part = empty({gcow_colsum_parts((int)rows) * cols}, at::kFloat, g), out = empty({cols}, at::kFloat, g);
+  const int launches = gcow_colsum_launches(g.data_ptr(), (int)rows, (int)cols, (int)g.stride(0));
+  const Tensor part = launches > 1 ? empty({gcow_colsum_parts((int)rows) * cols}, at::kFloat, g) : Tensor(), out = empty({cols}, at::kFloat, g);
   check(gcow_colsum(g.data_ptr(), f32(part), f32(out), (int)rows, (int)cols, (int)g.stride(0), on.stream), "gcow_colsum");
-  g_launches += 2;
+  g_launches += launches;
   return out;
 }
 
