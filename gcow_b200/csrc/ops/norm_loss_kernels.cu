@@ -550,6 +550,22 @@ colsum_cluster_kernel(const bf16* g, float* __restrict__ out, int rows, int cols
   cluster.sync();                                                // the others' sums are read until here
 }
 
+// ------------------------------------------------------------ weights to bf16
+// y = bf16(x), rounded to nearest even. Stands between two dependent kernels where a weight has no bf16 copy; as one of them its launch
+// and start are hidden, and torch's cast took 10 us of the host (1024 -> 512, 1 x 1 and 7 x 7, batch 16: 180 -> 171 us, all host).
+__global__ void __launch_bounds__(256) cast_bf16_kernel(const float* x, bf16* __restrict__ y, size_t n, int wide) {
+  pdl_trigger();
+  pdl_wait();
+  const size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) * 8;
+  if (i + 8 <= n && wide) {
+    const float4 a = reinterpret_cast<const float4*>(x + i)[0], b = reinterpret_cast<const float4*>(x + i)[1];
+    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    store8(y + i, v);
+  } else {
+    for (size_t k = i; k < i + 8 && k < n; k++) y[k] = __float2bfloat16(x[k]);
+  }
+}
+
 // ------------------------------------------------------- image normalisation
 // uint8 NHWC [n, 3] pixels -> bf16 NHWC padded to `cpad` channels (extra channels 0):
 // y = (x - mean_c) / std_c with mean/std given in 0..255 units.
@@ -692,6 +708,15 @@ int gcow_colsum(const void* g, float* part, float* out, int rows, int cols, int 
   else
     gcow::launch_dependent(reduce_partials_kernel, dim3((cols + 255) / 256), dim3(256), 0, (cudaStream_t)stream, (const float*)part, out,
                      parts, cols);
+  return (int)cudaGetLastError();
+}
+
+int gcow_cast_bf16(const float* x, void* y, uint64_t n, void* stream) {
+  if (!n) return 0;
+  const uint64_t ctas = (n + 2047) / 2048;
+  if (ctas > 0x7fffffff) return -1;
+  const int wide = (((uintptr_t)x | (uintptr_t)y) & 15) == 0;
+  gcow::launch_dependent(cast_bf16_kernel, dim3((unsigned)ctas), dim3(256), 0, (cudaStream_t)stream, x, (bf16*)y, (size_t)n, wide);
   return (int)cudaGetLastError();
 }
 
