@@ -821,6 +821,34 @@ int gcow_ar_max_ctas_v(int bits, int variant) {
 }
 int gcow_ar_max_ctas(int bits) { return gcow_ar_max_ctas_v(bits, kTwoShot); }
 
+// One rank's round trip of a.n values from a.in to a.out.
+static int launch_roundtrip(const ArArgs& a, int bits, cudaStream_t stream) {
+  const uint64_t want = ((a.n + 3) / 4 + kArThreads - 1) / kArThreads;   // a block per thread
+  if (a.residual || bits == 16) {
+    const int g = (int)(want < 148 * 8 ? want : 148 * 8);
+    switch (bits) {
+      case 16: launch_dependent(roundtrip_coded_kernel<16>, dim3(g), dim3(kArThreads), 0, stream, a); break;
+      case 32: launch_dependent(roundtrip_coded_kernel<32>, dim3(g), dim3(kArThreads), 0, stream, a); break;
+      case 64: launch_dependent(roundtrip_coded_kernel<64>, dim3(g), dim3(kArThreads), 0, stream, a); break;
+      case 128: launch_dependent(roundtrip_coded_kernel<128>, dim3(g), dim3(kArThreads), 0, stream, a); break;
+      default: return -1;
+    }
+    return (int)cudaGetLastError();
+  }
+  // As many CTAs as are resident (fewer threads of four blocks each took 11.6 instead of 9.1 us for 3 M values at 8 bits), then more, of
+  // four blocks per thread, which the GPU hands out as others end.
+  const uint64_t resident = 148 * kTripCtas, few = want < resident ? want : resident, many = (want + kTripAhead - 1) / kTripAhead;
+  const uint64_t most = 1u << 30;
+  const unsigned g = (unsigned)(many > few ? (many < most ? many : most) : few);
+  switch (bits) {
+    case 32: launch_dependent(roundtrip_kernel<32>, dim3(g), dim3(kArThreads), 0, stream, a); break;
+    case 64: launch_dependent(roundtrip_kernel<64>, dim3(g), dim3(kArThreads), 0, stream, a); break;
+    case 128: launch_dependent(roundtrip_kernel<128>, dim3(g), dim3(kArThreads), 0, stream, a); break;
+    default: return -1;
+  }
+  return (int)cudaGetLastError();
+}
+
 // Launch the fused all-reduce on `stream`. `residual` (n floats, or null) enables error feedback inside the kernel: the
 // encoder sees in + residual, and residual becomes what this rank's code of that sum dropped.
 //   arenas: `world` device pointers (every rank's arena as mapped in this process)
@@ -867,32 +895,7 @@ static int ar_launch_impl(const float* in, float* out, uint64_t n, int rank, int
     }
     return (int)cudaGetLastError();
   }
-  if (world == 1 && variant == kOneShot && !stamps) {
-    const uint64_t want = ((n + 3) / 4 + kArThreads - 1) / kArThreads;   // a block per thread
-    if (residual || bits == 16) {
-      const int g = (int)(want < 148 * 8 ? want : 148 * 8);
-      switch (bits) {
-        case 16: launch_dependent(roundtrip_coded_kernel<16>, dim3(g), dim3(kArThreads), 0, s, a); break;
-        case 32: launch_dependent(roundtrip_coded_kernel<32>, dim3(g), dim3(kArThreads), 0, s, a); break;
-        case 64: launch_dependent(roundtrip_coded_kernel<64>, dim3(g), dim3(kArThreads), 0, s, a); break;
-        case 128: launch_dependent(roundtrip_coded_kernel<128>, dim3(g), dim3(kArThreads), 0, s, a); break;
-        default: return -1;
-      }
-      return (int)cudaGetLastError();
-    }
-    // As many CTAs as are resident (fewer threads of four blocks each took 11.6 instead of 9.1 us for 3 M values at 8 bits), then more, of
-    // four blocks per thread, which the GPU hands out as others end.
-    const uint64_t resident = 148 * kTripCtas, few = want < resident ? want : resident, many = (want + kTripAhead - 1) / kTripAhead;
-    const uint64_t most = 1u << 30;
-    const unsigned g = (unsigned)(many > few ? (many < most ? many : most) : few);
-    switch (bits) {
-      case 32: launch_dependent(roundtrip_kernel<32>, dim3(g), dim3(kArThreads), 0, s, a); break;
-      case 64: launch_dependent(roundtrip_kernel<64>, dim3(g), dim3(kArThreads), 0, s, a); break;
-      case 128: launch_dependent(roundtrip_kernel<128>, dim3(g), dim3(kArThreads), 0, s, a); break;
-      default: return -1;
-    }
-    return (int)cudaGetLastError();
-  }
+  if (world == 1 && variant == kOneShot && !stamps) return launch_roundtrip(a, bits, s);
   switch (bits) {
     case 16: allreduce_fused_kernel<16><<<ctas, kArThreads, 0, s>>>(a); break;
     case 32: allreduce_fused_kernel<32><<<ctas, kArThreads, 0, s>>>(a); break;
@@ -928,6 +931,21 @@ int gcow_ar_launch(const float* in, float* out, uint64_t n, int rank, int world,
                    uint32_t* abort_flag, unsigned long long* stamps, void* stream) {
   return gcow_ar_launch_ef(in, out, n, rank, world, variant, bits, ctas, shift, postscale, arenas, mc_arena, region_cap,
                            epoch, timeout_ns, status, abort_flag, stamps, nullptr, stream);
+}
+
+// A one-rank call without error feedback: `out` = D(E(`in`)). Needs no arena, so nothing but the arrays is passed.
+int gcow_ar_roundtrip(const float* in, float* out, uint64_t n, int bits, void* stream) {
+  if (!n) return 0;
+  const void *etp, *dtp, *ptp, *ltp;
+  if (int rc = gcow_codec_tables4(&etp, &dtp, &ptp, &ltp)) return rc;
+  ArArgs a = {};
+  a.in = in; a.out = out; a.n = n;
+  a.postscale = 1.0f;
+  a.enc_table = (const uint16_t*)etp;
+  a.dec_table = (const uint16_t*)dtp;
+  a.pair_table = (const uint32_t*)ptp;
+  a.loop_table = (const uint32_t*)ltp;
+  return launch_roundtrip(a, bits, (cudaStream_t)stream);
 }
 
 // Conditional commit of an out-of-place all-reduce result (see commit_kernel).

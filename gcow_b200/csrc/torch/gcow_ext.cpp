@@ -32,6 +32,7 @@ int gcow_ar_launch_ef(const float* in, float* out, uint64_t n, int rank, int wor
                       float postscale, void* const* arenas, void* mc_arena, uint64_t region_cap, uint32_t epoch,
                       uint64_t timeout_ns, uint32_t* status, uint32_t* abort_flag, unsigned long long* stamps, float* residual,
                       void* stream);
+int gcow_ar_roundtrip(const float* in, float* out, uint64_t n, int bits, void* stream);
 uint64_t gcow_max_stream_bytes(const int32_t* params, uint64_t blocks, int dim);
 int gcow_host_word(uint64_t** word);
 int gcow_wait_host_word(volatile uint64_t* word, void* stream, uint64_t* value);
@@ -192,7 +193,36 @@ PyObject* ar_launch(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
+// ar_roundtrip(x, out or None, stream or None, max_numel, bits) -> whether the call was the plain one and has been launched: one rank, no
+// error feedback, contiguous float32 tensors of one device, as many values as an arena holds at most. What is not plain, mistakes
+// among it, is the caller's.
+PyObject* ar_roundtrip(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(nargs == 5, "ar_roundtrip: bad arguments");
+  if (!THPVariable_Check(args[0]) || !(args[1] == Py_None || THPVariable_Check(args[1]))) Py_RETURN_FALSE;
+  const at::Tensor& x0 = THPVariable_Unpack(args[0]);
+  if (!x0.is_cuda() || x0.scalar_type() != at::kFloat || !x0.is_contiguous()) Py_RETURN_FALSE;
+  const at::Tensor& x = gcow_ext::in_memory(x0);
+  const bool own = args[1] == Py_None || args[1] == args[0];
+  if (!own) {
+    const at::Tensor& o = THPVariable_Unpack(args[1]);
+    if (o.device() != x.device() || o.scalar_type() != at::kFloat || !o.is_contiguous() || o.numel() < x.numel()) Py_RETURN_FALSE;
+  }
+  const at::Tensor& out = own ? x : gcow_ext::in_memory(THPVariable_Unpack(args[1]));
+  const int64_t n = x.numel(), most = PyLong_AsLongLong(args[3]);
+  const long bits = PyLong_AsLong(args[4]);
+  const uint64_t given = args[2] == Py_None ? 0 : PyLong_AsUnsignedLongLong(args[2]);
+  if (PyErr_Occurred()) return nullptr;
+  if (n < 1 || n > most) Py_RETURN_FALSE;
+  const c10::cuda::CUDAGuard guard(x.device());
+  void* const stream = args[2] == Py_None ? c10::cuda::getCurrentCUDAStream(x.device().index()).stream() : (void*)given;
+  check(gcow_ar_roundtrip(x.const_data_ptr<float>(), out.mutable_data_ptr<float>(), (uint64_t)n, (int)bits, stream), "gcow_ar_roundtrip");
+  Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef methods[] = {
+    {"ar_roundtrip", (PyCFunction)(void (*)())ar_roundtrip, METH_FASTCALL, nullptr},
     {"ar_launch", (PyCFunction)(void (*)())ar_launch, METH_FASTCALL, nullptr},
     {"compress", (PyCFunction)(void (*)())compress, METH_FASTCALL, nullptr},
     {"decompress", (PyCFunction)(void (*)())decompress, METH_FASTCALL, nullptr},
