@@ -260,10 +260,16 @@ struct StringBuilder {
   }
 };
 
+// CTAs per SM of the 2-D coders: 48 registers, which hold a block without a spill, where the compiler left to itself takes up to 62 and
+// four CTAs fit. 7654 x 7654 at tolerance 1e-3: encoding 153.7 -> 148.4 us, decoding 123.5 -> 115.8; at 1e-1 118.4 -> 112.3 and 72.6 -> 66.2;
+// 2047 x 3001 at 8 bits/value decoding 22.4 -> 21.7. Six (40 registers, 20 to 40 bytes of spills): 161.9, 116.3, 128.1, 63.6. The 1-D
+// coders take 40 to 48 registers by themselves and lose by being told.
+constexpr int kCtas2d = 5;
+
 enum TileMode { kVariable, kPacked, kDirect };              // variable rate; fixed rate; fixed rate in whole words
 
 template <int DIM, int PER, TileMode MODE, bool BUDGET>
-__global__ void __launch_bounds__(kTileThreads)
+__global__ void __launch_bounds__(kTileThreads, DIM == 2 ? kCtas2d : 0)
 encode_tiles_kernel(const float* in, const TileArgs a, uint32_t* __restrict__ out, uint64_t* __restrict__ block_bits,
                     const TileStrings st, const uint16_t* __restrict__ enc_tab, const uint32_t* __restrict__ pair_tab) {
   constexpr int WB = 32 * PER, NB = kTileThreads * PER;
@@ -540,7 +546,7 @@ place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restric
 // tolerance 1e-6 121 us, with windows 101, with the straight line first 81; at 1e-3 95, 93, 70; at 6 bits/value 117, 97, 84; a
 // random walk at 1e-6 218, 144, 135.
 template <int DIM, int PER, bool BUDGET>
-__global__ void __launch_bounds__(kTileThreads)
+__global__ void __launch_bounds__(kTileThreads, DIM == 2 ? kCtas2d : 0)
 decode_tiles_kernel(const uint32_t* in, float* __restrict__ out, const TileArgs a,
                     const uint64_t* block_bits, int shift, const uint16_t* __restrict__ plane_tab, const uint32_t* __restrict__ loop_tab) {
   constexpr int kPer = PER, WB = 32 * PER, NB = kTileThreads * PER;
