@@ -441,8 +441,11 @@ encode_tiles_kernel(const float* in, const TileArgs a, uint32_t* __restrict__ ou
 // Second kernel of the variable-rate encoder: every CTA takes a contiguous share of the tiles, at most kTileThreads of them at a
 // time, whose starts it works out in shared memory first; then nothing depends on anything but that table, and the
 // warps run through the strings at their own pace.
+// Five CTAs per SM with four blocks a lane, where the compiler would take 63 registers for four: encoding 25.6 M values at tolerance 1e-3
+// 114.0 -> 112.5 us, at precision 8 106.9 -> 104.6; six 115.3 and 106.9. With one block a lane eight fit by themselves.
+constexpr int place_ctas(int per) { return per == 4 ? 5 : 8; }
 template <int PER>
-__global__ void __launch_bounds__(kTileThreads)
+__global__ void __launch_bounds__(kTileThreads, PER == 4 ? place_ctas(PER) : 0)
 place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restrict__ out, uint64_t* __restrict__ block_bits,
                      uint64_t* total_out) {
   constexpr int NB = kTileThreads * PER;
@@ -789,7 +792,7 @@ int gcow_encode_tiles(const float* in, uint64_t nx, uint64_t ny, const int32_t* 
 #undef GCOW_ENCODE_MODE
 #undef GCOW_ENCODE
   if (!fixed) {
-    const uint32_t most = 148 * 8, g = a.tiles < most ? a.tiles : most;
+    const uint32_t most = 148 * place_ctas(per), g = a.tiles < most ? a.tiles : most;
     if (per == 4) launch_dependent(place_strings_kernel<4>, dim3(g), dim3(kTileThreads), 0, s, st, a, (uint32_t*)out, block_bits, total_out);
     else launch_dependent(place_strings_kernel<1>, dim3(g), dim3(kTileThreads), 0, s, st, a, (uint32_t*)out, block_bits, total_out);
   }
