@@ -29,6 +29,14 @@ namespace bn {
 
 typedef __nv_bfloat16 bf16;
 constexpr int kThreads = 256;
+// Every sweep over the tensor is launched with at most this many CTAs per SM, and compiled for exactly as many: the sweeps are bound by how
+// many loads are in flight, so each thread gets the registers (80) that keep several rows' loads outstanding. Which operands a sweep has (a
+// residual, a second gradient, a ReLU and its mask) is a template argument: as run-time conditions inside the unrolled loop they kept each
+// row's loads behind the row before. 256 x 512 x 28 x 28, without the template and the bound -> with both: forward 114 -> 110 us, with ReLU
+// 126 -> 113, with residual and ReLU 165 -> 138; backward 192 -> 187, 250 -> 193 and 260 -> 221 us, with a second gradient 315 -> 253.
+// The bound at 4 CTAs or the grid at 6 made the backward slower (55 -> 61..64 us for 256 x 128 x 28 x 28). Rows unrolled: as many as the 80
+// registers hold, measured at 2, 3, 4, 6 and 8.
+constexpr int kSweepCtas = 3;
 
 __device__ __forceinline__ void load8(const bf16* p, float (&v)[8]) {
   uint4 u = *reinterpret_cast<const uint4*>(p);
@@ -64,13 +72,13 @@ __device__ __forceinline__ void cta_fold(const float (&a)[8], const float (&b)[8
 }
 
 // ---- forward statistics: partial sum(x), sum(x^2)
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, kSweepCtas)
 stats_kernel(const bf16* __restrict__ x, float* __restrict__ part, int64_t R, int C) {
   pdl_trigger();
   pdl_wait();       // launched under the tail of the kernel that writes x
   const int groups = C / 8, g = threadIdx.x % groups, r0 = threadIdx.x / groups, rstep = kThreads / groups;
   float s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll 4
+#pragma unroll 8
   for (int64_t r = (int64_t)blockIdx.x * rstep + r0; r < R; r += (int64_t)gridDim.x * rstep) {
     float v[8];
     load8(x + r * C + g * 8, v);
@@ -135,73 +143,75 @@ __global__ void affine_from_stats_kernel(const float* __restrict__ gamma, const 
   scale[c] = sc; shift[c] = beta[c] - mean_in[c] * sc;
 }
 
-// ---- normalise: y = x*scale + shift (+ residual) (ReLU)
-__global__ void __launch_bounds__(kThreads)
+// ---- normalise: y = x*scale + shift (+ residual when ADD) (ReLU when RELU, its outcome to the mask when RELU is 2)
+template <bool ADD, int RELU>
+__global__ void __launch_bounds__(kThreads, kSweepCtas)
 apply_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residual, bf16* __restrict__ y,
              uint8_t* __restrict__ mask, const float* __restrict__ scale, const float* __restrict__ shift, int64_t R,
-             int C, int relu) {
+             int C) {
   pdl_wait();
   pdl_trigger();    // the consumer of y may set itself up meanwhile
   const int groups = C / 8, g = threadIdx.x % groups, r0 = threadIdx.x / groups, rstep = kThreads / groups;
   float sc[8], sh[8];
 #pragma unroll
   for (int i = 0; i < 8; i++) { sc[i] = scale[g * 8 + i]; sh[i] = shift[g * 8 + i]; }
-#pragma unroll 4
+#pragma unroll (ADD ? 3 : RELU ? 4 : 8)
   for (int64_t r = (int64_t)blockIdx.x * rstep + r0; r < R; r += (int64_t)gridDim.x * rstep) {
     const int64_t off = r * C + g * 8;
     float v[8];
     load8(x + off, v);
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = v[i] * sc[i] + sh[i];
-    if (residual) {
+    if (ADD) {
       float w[8];
       load8(residual + off, w);
 #pragma unroll
       for (int i = 0; i < 8; i++) v[i] += w[i];
     }
-    if (relu) {
+    if (RELU) {
       uint32_t bits = 0;
 #pragma unroll
       for (int i = 0; i < 8; i++) { bits |= (v[i] > 0.0f ? 1u : 0u) << i; v[i] = fmaxf(v[i], 0.0f); }
-      if (mask) mask[r * groups + g] = (uint8_t)bits;      // bit i: channel g*8+i passed the ReLU
+      if (RELU == 2) mask[r * groups + g] = (uint8_t)bits;      // bit i: channel g*8+i passed the ReLU
     }
     store8(y + off, v);
   }
 }
 
-// ---- backward sweep 1: partial sum(g), sum(g*xhat); g = dy (+ dy2) masked by (y > 0) when relu.
-// dy2 (nullable) is a second gradient of the same output (the output feeds two consumers): adding it here saves
+// ---- backward sweep 1: partial sum(g), sum(g*xhat); g = dy (+ dy2) masked by (y > 0) when RELU.
+// dy2 is a second gradient of the same output (the output feeds two consumers): adding it here saves
 // the separate addition kernel and its three passes over the tensor.
-// When gmask_out is given, the masked gradient is written there (the residual branch's gradient).
-__global__ void __launch_bounds__(kThreads)
+// The masked gradient is written to gmask_out when OUT (the residual branch's gradient). TWO: there is a dy2, RELU: there is a mask.
+template <bool TWO, bool RELU, bool OUT>
+__global__ void __launch_bounds__(kThreads, kSweepCtas)
 bwd_reduce_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ dy2, const uint8_t* __restrict__ mask,
                   const bf16* __restrict__ x,
                   const float* __restrict__ mean, const float* __restrict__ rstd, bf16* __restrict__ gmask_out,
-                  float* __restrict__ part, int64_t R, int C, int relu) {
+                  float* __restrict__ part, int64_t R, int C) {
   pdl_trigger();
   pdl_wait();
   const int groups = C / 8, g = threadIdx.x % groups, r0 = threadIdx.x / groups, rstep = kThreads / groups;
   float mu[8], rs[8], s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
   for (int i = 0; i < 8; i++) { mu[i] = mean[g * 8 + i]; rs[i] = rstd[g * 8 + i]; }
-#pragma unroll 4
+#pragma unroll (OUT && !TWO ? 3 : 4)
   for (int64_t r = (int64_t)blockIdx.x * rstep + r0; r < R; r += (int64_t)gridDim.x * rstep) {
     const int64_t off = r * C + g * 8;
     float gv[8], xv[8];
     load8(dy + off, gv);
     load8(x + off, xv);
-    if (dy2) {
+    if (TWO) {
       float w[8];
       load8(dy2 + off, w);
 #pragma unroll
       for (int i = 0; i < 8; i++) gv[i] += w[i];
     }
-    if (relu) {
+    if (RELU) {
       const uint32_t bits = mask[r * groups + g];
 #pragma unroll
       for (int i = 0; i < 8; i++) gv[i] = (bits >> i) & 1u ? gv[i] : 0.0f;
     }
-    if (gmask_out) store8(gmask_out + off, gv);
+    if (OUT) store8(gmask_out + off, gv);
 #pragma unroll
     for (int i = 0; i < 8; i++) { s[i] += gv[i]; q[i] += gv[i] * (xv[i] - mu[i]) * rs[i]; }
   }
@@ -223,12 +233,13 @@ finalize_bwd_kernel(const float* __restrict__ part, int parts, int C, float* __r
 
 // ---- backward sweep 2: dx = gamma*rstd * (g - dbeta/R - xhat*dgamma/R). From the last row to the first: sweep 1 has just read the last
 // ones, which the L2 still holds, and what reads dx next finds its first rows there. Backward of 256 x 128 x 28 x 28: 57.8 -> 55.4 us, x 2048 x
-// 7 x 7 62.8 -> 60.7, x 64 x 56 x 56 102.3 -> 100.7, x 256 x 56 x 56 as before. (The forward's second sweep backwards: 33.5 -> 38.2 us.)
-__global__ void __launch_bounds__(kThreads)
+// 7 x 7 62.8 -> 60.7, x 64 x 56 x 56 102.3 -> 100.7, x 256 x 56 x 56 as before, all before the
+// registers that kSweepCtas gives. (The forward's second sweep backwards: 33.5 -> 38.2 us.)
+template <bool RELU>
+__global__ void __launch_bounds__(kThreads, kSweepCtas)
 bwd_dx_kernel(const bf16* __restrict__ dy, const uint8_t* __restrict__ mask, const bf16* __restrict__ x,
               const float* __restrict__ gamma, const float* __restrict__ mean, const float* __restrict__ rstd,
-              const float* __restrict__ dgamma, const float* __restrict__ dbeta, bf16* __restrict__ dx, int64_t R, int C,
-              int relu) {
+              const float* __restrict__ dgamma, const float* __restrict__ dbeta, bf16* __restrict__ dx, int64_t R, int C) {
   pdl_wait();
   pdl_trigger();
   const int groups = C / 8, g = threadIdx.x % groups, r0 = threadIdx.x / groups, rstep = kThreads / groups;
@@ -248,7 +259,7 @@ bwd_dx_kernel(const bf16* __restrict__ dy, const uint8_t* __restrict__ mask, con
     float gv[8], xv[8];
     load8(dy + off, gv);
     load8(x + off, xv);
-    if (relu) {
+    if (RELU) {
       const uint32_t bits = mask[r * groups + g];
 #pragma unroll
       for (int i = 0; i < 8; i++) gv[i] = (bits >> i) & 1u ? gv[i] : 0.0f;
@@ -259,10 +270,22 @@ bwd_dx_kernel(const bf16* __restrict__ dy, const uint8_t* __restrict__ mask, con
   }
 }
 
+// the form of a sweep for the operands that a call has
+inline auto apply_for(const void* residual, const void* mask, int relu) {
+  const int form = relu ? (mask ? 2 : 1) : 0;
+  if (residual) return form == 2 ? apply_kernel<true, 2> : form == 1 ? apply_kernel<true, 1> : apply_kernel<true, 0>;
+  return form == 2 ? apply_kernel<false, 2> : form == 1 ? apply_kernel<false, 1> : apply_kernel<false, 0>;
+}
+inline auto bwd_reduce_for(const void* dy2, const void* dres, int relu) {
+  if (dy2) return relu ? bwd_reduce_kernel<true, true, true> : bwd_reduce_kernel<true, false, true>;
+  if (dres) return relu ? bwd_reduce_kernel<false, true, true> : bwd_reduce_kernel<false, false, true>;
+  return relu ? bwd_reduce_kernel<false, true, false> : bwd_reduce_kernel<false, false, false>;
+}
+
 inline int grid_for(int64_t R, int C) {
   const int rstep = kThreads / (C / 8);
   int64_t g = (R + rstep - 1) / rstep;
-  if (g > 148 * 3) g = 148 * 3;
+  if (g > 148 * kSweepCtas) g = 148 * kSweepCtas;
   return (int)(g < 1 ? 1 : g);
 }
 inline bool shape_ok(int C) { return C % 8 == 0 && C >= 8 && C <= 2048 && kThreads % (C / 8) == 0; }
@@ -290,8 +313,8 @@ int gcow_bn_fwd_train(const void* x, const void* residual, void* y, void* mask, 
   gcow::launch_dependent(stats_kernel, dim3(g), dim3(kThreads), 0, s, (const bf16*)x, part, R, C);
   gcow::launch_dependent(finalize_fwd_kernel, dim3((C + kFinX - 1) / kFinX), dim3(kFinX, kFinY), 0, s, part, g, C, R, eps, momentum, gamma,
                    beta, mean, rstd, scale, shift, run_mean, run_var);
-  gcow::launch_dependent(apply_kernel, dim3(g), dim3(kThreads), 0, s, (const bf16*)x, (const bf16*)residual, (bf16*)y, (uint8_t*)mask,
-                   (const float*)scale, (const float*)shift, R, C, relu);
+  gcow::launch_dependent(apply_for(residual, mask, relu), dim3(g), dim3(kThreads), 0, s, (const bf16*)x, (const bf16*)residual, (bf16*)y, (uint8_t*)mask,
+                   (const float*)scale, (const float*)shift, R, C);
   return (int)cudaGetLastError();
 }
 
@@ -302,7 +325,7 @@ int gcow_bn_fwd_eval(const void* x, const void* residual, void* y, const float* 
   if (!shape_ok(C) || R <= 0) return -1;
   cudaStream_t s = (cudaStream_t)stream;
   affine_from_stats_kernel<<<(C + 127) / 128, 128, 0, s>>>(gamma, beta, run_mean, run_var, eps, C, scratch, scratch + C);
-  apply_kernel<<<grid_for(R, C), kThreads, 0, s>>>((const bf16*)x, (const bf16*)residual, (bf16*)y, nullptr, scratch, scratch + C, R, C, relu);
+  apply_for(residual, nullptr, relu)<<<grid_for(R, C), kThreads, 0, s>>>((const bf16*)x, (const bf16*)residual, (bf16*)y, nullptr, scratch, scratch + C, R, C);
   return (int)cudaGetLastError();
 }
 
@@ -317,12 +340,12 @@ int gcow_bn_bwd3(const void* dy, const void* dy2, const void* mask, const void* 
   cudaStream_t s = (cudaStream_t)stream;
   const int g = grid_for(R, C);
   const float *mean = stats, *rstd = stats + C;
-  gcow::launch_dependent(bwd_reduce_kernel, dim3(g), dim3(kThreads), 0, s, (const bf16*)dy, (const bf16*)dy2, (const uint8_t*)mask,
-                         (const bf16*)x, mean, rstd, (bf16*)dres, part, R, C, relu);
+  gcow::launch_dependent(bwd_reduce_for(dy2, dres, relu), dim3(g), dim3(kThreads), 0, s, (const bf16*)dy, (const bf16*)dy2, (const uint8_t*)mask,
+                         (const bf16*)x, mean, rstd, (bf16*)dres, part, R, C);
   gcow::launch_dependent(finalize_bwd_kernel, dim3((C + kFinX - 1) / kFinX), dim3(kFinX, kFinY), 0, s, (const float*)part, g, C, dgamma, dbeta);
   // the second sweep applies the mask again, or reads the masked gradient if it was written
-  gcow::launch_dependent(bwd_dx_kernel, dim3(g), dim3(kThreads), 0, s, (const bf16*)(dres ? dres : dy), (const uint8_t*)mask, (const bf16*)x,
-                   gamma, mean, rstd, (const float*)dgamma, (const float*)dbeta, (bf16*)dx, R, C, dres ? 0 : relu);
+  gcow::launch_dependent(!dres && relu ? bwd_dx_kernel<true> : bwd_dx_kernel<false>, dim3(g), dim3(kThreads), 0, s, (const bf16*)(dres ? dres : dy), (const uint8_t*)mask, (const bf16*)x,
+                   gamma, mean, rstd, (const float*)dgamma, (const float*)dbeta, (bf16*)dx, R, C);
   return (int)cudaGetLastError();
 }
 

@@ -457,6 +457,46 @@ def test_batchnorm_fork_adds_the_two_gradients_in_the_kernel():
     assert (x.grad.float() - xf.grad).abs().max().item() / xf.grad.abs().max().item() < 3e-2
 
 
+@pytest.mark.parametrize("N,C,H,W", [(5, 8, 1, 1), (2, 64, 3, 5), (11, 2048, 17, 19), (1, 1024, 60, 37), (3, 256, 60, 59)])
+@pytest.mark.parametrize("res,relu,fork", [(a, b, c) for a in (False, True) for b in (False, True) for c in (False, True)])
+def test_batchnorm_every_form_of_the_sweeps(N, C, H, W, res, relu, fork):
+    """Every combination of operands has its own kernels, each with several rows in flight: fewer rows than one CTA takes, fewer than the
+    grid, just under and over 2, 3, 4 and 8 rows a thread. Against float64. A bf16 result is off by half a unit in its last place
+    (2**-9 of it), a masked gradient that was written out carries the same into dx; the rest is fp32 sums."""
+    from gcow_b200.ops import nn as gnn, set_backend
+    set_backend("own")
+    torch.manual_seed(C + H)
+    mk = lambda: torch.randn(N, C, H, W, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last)
+    x0, r0, w1, w2 = mk(), mk(), mk(), mk()
+    bn = gnn.BatchNorm2d(C).cuda()
+    with torch.no_grad():
+        bn.weight.uniform_(0.5, 1.5); bn.bias.uniform_(-0.3, 0.3)
+    x, r = x0.clone().requires_grad_(True), (r0.clone().requires_grad_(True) if res else None)
+    out = bn(x, residual=r, relu=relu, fork=fork)
+    ys, ws = (list(out), [w1, w2]) if fork else ([out], [w1])
+    torch.autograd.backward(ys, ws)
+
+    col = lambda v: v.double().view(1, C, 1, 1)
+    R, xd, ga = N * H * W, x0.double(), col(bn.weight.detach())
+    mean, var = xd.mean((0, 2, 3), keepdim=True), xd.var((0, 2, 3), unbiased=False, keepdim=True)
+    rstd = 1 / (var + bn.eps).sqrt()
+    xh = (xd - mean) * rstd
+    z = xh * ga + col(bn.bias.detach()) + (r0.double() if res else 0)
+    y = ys[0].detach().double()
+    want = z.clamp(min=0) if relu else z
+    assert ((y - want).abs() <= 2**-8 * want.abs() + 1e-4).all()
+    g = sum(w.double() for w in ws)
+    if relu:
+        g = torch.where(y > 0, g, torch.zeros_like(g))
+    if res:
+        assert ((r.grad.double() - g).abs() <= 2**-8 * g.abs()).all()
+    db, dg = g.sum((0, 2, 3)), (g * xh).sum((0, 2, 3))
+    assert ((bn.bias.grad.double() - db).abs() <= 1e-5 * g.abs().sum((0, 2, 3)) + 1e-5).all()
+    assert ((bn.weight.grad.double() - dg).abs() <= 1e-5 * (g * xh).abs().sum((0, 2, 3)) + 1e-5).all()
+    dx = ga * rstd * (g - col(db) / R - xh * col(dg) / R)
+    assert ((x.grad.double() - dx).abs() <= 2**-8 * (dx.abs() + ga * rstd * g.abs()) + 1e-4 * ga * rstd).all()
+
+
 def test_batchnorm_counts_training_steps_lazily():
     """num_batches_tracked is counted on the host by the own path and lands in the tensor when the state is saved,
     when PyTorch's own path runs, and not twice."""
