@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include "pdl.cuh"
+#include <atomic>
 #include <stdint.h>
 
 namespace gcow {
@@ -144,101 +145,138 @@ layernorm_fwd_rows_kernel(const bf16* x, const float* gamma, const float* beta,
   }
 }
 
-// dx per row; per-CTA partial sums of dgamma/dbeta go to part[blockIdx.x][2][H].
-// A lane always works on the same columns (lane*8 + 256*k), so its dgamma/dbeta
-// contributions stay in registers across all rows of the warp (CH = H/256 chunks of
-// 8 columns, CH <= 4) and touch shared memory once at the end; wider rows (CH == 0)
-// accumulate in shared memory.
-template <int CH>
-__global__ void __launch_bounds__(128, CH > 0 ? 3 : 1)
+// LayerNorm backward: dx per row; per-CTA partial sums of dgamma/dbeta go to part[blockIdx.x][2][H].
+// Rows of up to 1024 columns, H <= 256 * CH. A warp takes a row; a lane always works on the same columns (lane * 8 + 256 * k), so its
+// dgamma/dbeta contributions stay in registers over all its rows and touch shared memory once at the end. The next row is on its way into
+// shared memory (cp.async; each lane fetches and reads its own 16-byte pieces, so nothing has to be synchronised) while this one is worked
+// on. What bounds it is how many rows an SM has in flight: with the next row in registers it was 12 warps (168 registers at 1024 columns,
+// some of them spilled), now 16. Two rows ahead are slower (26.7 against 25.6 us at 16384 x 1024).
+// T threads a CTA, 512 / T CTAs per SM: with 512 threads the SM's partial sums are added up before they are written, with 128 few rows spread
+// over more SMs. Both passes together, against the rows in registers: 16384 x 1024 36.7 -> 24.9 us (100 MB take 15.4), x 768 22.6 -> 20.4,
+// x 512 19.0 -> 16.0, x 256 13.3 -> 11.1, 2048 x 1024 12.9 -> 8.7, 512 x 1024 8.7 -> 7.2.
+constexpr int kLnWide = 512, kLnNarrow = 128;
+__device__ __forceinline__ void copy16(void* smem, const void* g) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(g) : "memory");
+}
+template <int CH, int T> constexpr size_t kLnBwdSmem = (size_t)CH * (256 * 4 + 2 * 2 * T * 16);      // gamma, two rows' x and dy of every lane
+template <int CH, int T>
+__global__ void __launch_bounds__(T, 512 / T)
+layernorm_bwd_rows_kernel(const bf16* dy, const bf16* x, const float* gamma, const float* mean, const float* rstd, bf16* __restrict__ dx,
+                          float* __restrict__ part, int rows, int H) {
+  pdl_trigger();
+  pdl_wait();
+  extern __shared__ __align__(16) float sm[];          // gamma [256 * CH], the rows on their way; in the end [warps][2][H]
+  constexpr int kWarps = T / 32;
+  static_assert(kLnBwdSmem<CH, T> >= (size_t)kWarps * 2 * 256 * CH * 4, "the warps' sums lie over the gamma copy and the rows");
+  uint4* const ring = reinterpret_cast<uint4*>(sm + 256 * CH) + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, stride = gridDim.x * kWarps;
+  auto fetch = [&](int row, int slot) {
+    if (row < rows) {
+      const bf16* const xr = x + (size_t)row * H;
+      const bf16* const gr = dy + (size_t)row * H;
+#pragma unroll
+      for (int k = 0; k < CH; k++) {
+        const int c = lane * 8 + 256 * k;
+        if (c < H) {
+          copy16(ring + (slot * 2 * CH + 2 * k) * T, xr + c);
+          copy16(ring + (slot * 2 * CH + 2 * k + 1) * T, gr + c);
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  int r = blockIdx.x * kWarps + warp, slot = 0;
+  fetch(r, 0);
+  for (int c = threadIdx.x; c < 256 * CH; c += T) sm[c] = c < H ? gamma[c] : 0.0f;
+  float rg[CH][8], rb[CH][8], next_mu = 0.0f, next_rs = 0.0f;
+#pragma unroll
+  for (int k = 0; k < CH; k++)
+#pragma unroll
+    for (int i = 0; i < 8; i++) { rg[k][i] = 0; rb[k][i] = 0; }
+  if (r < rows) { next_mu = mean[r]; next_rs = rstd[r]; }
+  __syncthreads();
+  for (; r < rows; r += stride, slot ^= 1) {
+    fetch(r + stride, slot ^ 1);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    const float mu = next_mu, rs = next_rs;
+    if (r + stride < rows) { next_mu = mean[r + stride]; next_rs = rstd[r + stride]; }
+    const uint4* const row = ring + slot * 2 * CH * T;
+    float s1 = 0, s2 = 0;
+#pragma unroll
+    for (int k = 0; k < CH; k++) {
+      const int c = lane * 8 + 256 * k;
+      if (c < H) {
+        float xv[8], gv[8], gam[8];
+        unpack8(row[2 * k * T], xv); unpack8(row[(2 * k + 1) * T], gv);
+        *reinterpret_cast<float4*>(gam) = *reinterpret_cast<const float4*>(sm + c);
+        *reinterpret_cast<float4*>(gam + 4) = *reinterpret_cast<const float4*>(sm + c + 4);
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const float xh = (xv[i] - mu) * rs, gg = gv[i] * gam[i];
+          s1 += gg; s2 += gg * xh;
+          rg[k][i] += gv[i] * xh;
+          rb[k][i] += gv[i];
+        }
+      }
+    }
+    s1 = warp_sum(s1) / H; s2 = warp_sum(s2) / H;
+    bf16* const dr = dx + (size_t)r * H;
+    // the row is unpacked again: cheaper than keeping 2 x 8 x CH floats
+#pragma unroll
+    for (int k = 0; k < CH; k++) {
+      const int c = lane * 8 + 256 * k;
+      if (c < H) {
+        float xv[8], gv[8], gam[8], o[8];
+        unpack8(row[2 * k * T], xv); unpack8(row[(2 * k + 1) * T], gv);
+        *reinterpret_cast<float4*>(gam) = *reinterpret_cast<const float4*>(sm + c);
+        *reinterpret_cast<float4*>(gam + 4) = *reinterpret_cast<const float4*>(sm + c + 4);
+#pragma unroll
+        for (int i = 0; i < 8; i++) o[i] = rs * (gv[i] * gam[i] - s1 - (xv[i] - mu) * rs * s2);
+        store8(dr + c, o);
+      }
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();      // every warp is done with the gamma copy and the rows that these sums overwrite
+  float* const dg = sm + (size_t)warp * 2 * H;
+  float* const db = dg + H;
+#pragma unroll
+  for (int k = 0; k < CH; k++)
+#pragma unroll
+    for (int i = 0; i < 8; i += 4) {
+      const int c = lane * 8 + 256 * k + i;
+      if (c < H) {
+        *reinterpret_cast<float4*>(dg + c) = make_float4(rg[k][i], rg[k][i + 1], rg[k][i + 2], rg[k][i + 3]);
+        *reinterpret_cast<float4*>(db + c) = make_float4(rb[k][i], rb[k][i + 1], rb[k][i + 2], rb[k][i + 3]);
+      }
+    }
+  __syncthreads();
+  float* const out = part + (size_t)blockIdx.x * 2 * H;
+  for (int c = threadIdx.x * 4; c < 2 * H; c += T * 4) {
+    float4 t = *reinterpret_cast<const float4*>(sm + c);
+#pragma unroll
+    for (int w = 1; w < kWarps; w++) {
+      const float4 u = *reinterpret_cast<const float4*>(sm + (size_t)w * 2 * H + c);
+      t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
+    }
+    *reinterpret_cast<float4*>(out + c) = t;
+  }
+}
+
+// Wider rows: dgamma/dbeta are summed up in shared memory.
+__global__ void __launch_bounds__(128)
 layernorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const float* __restrict__ gamma,
                      const float* __restrict__ mean, const float* __restrict__ rstd, bf16* __restrict__ dx,
                      float* __restrict__ part, int rows, int H) {
   pdl_trigger();
   pdl_wait();
-  extern __shared__ float sm[];          // [4 warps][2][H]
+  extern __shared__ __align__(16) float sm[];          // [4 warps][2][H]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float* dg = sm + (size_t)warp * 2 * H;
   float* db = dg + H;
-  constexpr int NR = CH > 0 ? CH : 1;
-  float rg[NR][8], rb[NR][8];
-  if (CH > 0) {
-    // gamma lives in shared memory (one copy per CTA): 32 registers less per thread buy a third CTA per SM
-    for (int c = threadIdx.x; c < 256 * NR; c += blockDim.x) sm[c] = c < H ? gamma[c] : 0.0f;
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NR; k++)
-#pragma unroll
-      for (int i = 0; i < 8; i++) { rg[k][i] = 0; rb[k][i] = 0; }
-  } else {
-    for (int c = lane; c < H; c += 32) { dg[c] = 0; db[c] = 0; }
-    __syncwarp();
-  }
-  if (CH > 0) {
-    // One row per warp and turn; the next row's 2 x CH 16-byte loads are issued before this row's arithmetic, so a
-    // warp always has a row in flight (without that the kernel ran at a quarter of the memory roofline: load, reduce
-    // across the warp, store, and only then the next load).
-    const int stride = gridDim.x * 4;
-    int r = blockIdx.x * 4 + warp;
-    uint4 nx[NR], ng[NR];
-    float nmu = 0.0f, nrs = 0.0f;
-    auto fetch = [&](int row) {
-      const bf16* xr = x + (size_t)row * H;
-      const bf16* gr = dy + (size_t)row * H;
-#pragma unroll
-      for (int k = 0; k < NR; k++) {
-        const int c = lane * 8 + 256 * k;
-        if (c < H) {
-          nx[k] = *reinterpret_cast<const uint4*>(xr + c);
-          ng[k] = *reinterpret_cast<const uint4*>(gr + c);
-        }
-      }
-      nmu = mean[row]; nrs = rstd[row];
-    };
-    if (r < rows) fetch(r);
-    for (; r < rows; r += stride) {
-      uint4 cx[NR], cgv[NR];
-#pragma unroll
-      for (int k = 0; k < NR; k++) { cx[k] = nx[k]; cgv[k] = ng[k]; }
-      const float mu = nmu, rs = nrs;
-      if (r + stride < rows) fetch(r + stride);
-      float s1 = 0, s2 = 0;
-#pragma unroll
-      for (int k = 0; k < NR; k++) {
-        const int c = lane * 8 + 256 * k;
-        if (c < H) {
-          float xv[8], gv[8], gam[8];
-          unpack8(cx[k], xv); unpack8(cgv[k], gv);
-          *reinterpret_cast<float4*>(gam) = *reinterpret_cast<const float4*>(sm + c);
-          *reinterpret_cast<float4*>(gam + 4) = *reinterpret_cast<const float4*>(sm + c + 4);
-#pragma unroll
-          for (int i = 0; i < 8; i++) {
-            const float xh = (xv[i] - mu) * rs, gg = gv[i] * gam[i];
-            s1 += gg; s2 += gg * xh;
-            rg[k][i] += gv[i] * xh;
-            rb[k][i] += gv[i];
-          }
-        }
-      }
-      s1 = warp_sum(s1) / H; s2 = warp_sum(s2) / H;
-      bf16* dr = dx + (size_t)r * H;
-      // the row is still in registers as packed bf16: unpacking it again is cheaper than keeping 2 x 8 x CH floats
-#pragma unroll
-      for (int k = 0; k < NR; k++) {
-        const int c = lane * 8 + 256 * k;
-        if (c < H) {
-          float xv[8], gv[8], gam[8], o[8];
-          unpack8(cx[k], xv); unpack8(cgv[k], gv);
-          *reinterpret_cast<float4*>(gam) = *reinterpret_cast<const float4*>(sm + c);
-          *reinterpret_cast<float4*>(gam + 4) = *reinterpret_cast<const float4*>(sm + c + 4);
-#pragma unroll
-          for (int i = 0; i < 8; i++) o[i] = rs * (gv[i] * gam[i] - s1 - (xv[i] - mu) * rs * s2);
-          store8(dr + c, o);
-        }
-      }
-    }
-  }
-  for (int r = blockIdx.x * 4 + warp; CH == 0 && r < rows; r += gridDim.x * 4) {
+  for (int c = lane; c < H; c += 32) { dg[c] = 0; db[c] = 0; }
+  __syncwarp();
+  for (int r = blockIdx.x * 4 + warp; r < rows; r += gridDim.x * 4) {
     const bf16* xr = x + (size_t)r * H;
     const bf16* gr = dy + (size_t)r * H;
     const float mu = mean[r], rs = rstd[r];
@@ -267,16 +305,6 @@ layernorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, co
       store8(dr + c, o);
     }
   }
-  if (CH > 0) {
-    __syncthreads();      // every warp is done with the gamma copy that these sums overwrite
-#pragma unroll
-    for (int k = 0; k < NR; k++)
-#pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const int c = lane * 8 + 256 * k + i;
-        if (c < H) { dg[c] = rg[k][i]; db[c] = rb[k][i]; }
-      }
-  }
   __syncthreads();
   float* out = part + (size_t)blockIdx.x * 2 * H;
   for (int c = threadIdx.x; c < 2 * H; c += blockDim.x)
@@ -294,7 +322,7 @@ __global__ void reduce_partials_kernel(const float* __restrict__ part, float* __
   out[c] = s;
 }
 
-// The same for many partials of a short vector (LayerNorm's 444 x 2H): 32 x 32 threads per 32 columns, thread (cx, py)
+// The same for many partials of a short vector (LayerNorm's 148 to 444 x 2H): 32 x 32 threads per 32 columns, thread (cx, py)
 // adds partials py, py + 32, ..., then the 32 rows are added in a fixed order. One thread per column walking all the
 // partials serially took longer than the LayerNorm backward sweep it follows.
 __global__ void __launch_bounds__(1024)
@@ -607,28 +635,45 @@ int gcow_layernorm_fwd(const void* x, const float* gamma, const float* beta, voi
   return (int)cudaGetLastError();
 }
 
-// Number of partial rows the backward writes; `part` must hold parts * 2 * H floats.
-int gcow_layernorm_bwd_parts(int rows) { int g = (rows + 3) / 4; return g < 148 * 3 ? g : 148 * 3; }   // three CTAs per SM are resident
+// Number of partial rows the backward writes at most; `part` must hold parts * 2 * H floats.
+int gcow_layernorm_bwd_parts(int rows) { int g = (rows + 3) / 4; return g < 148 * 3 ? g : 148 * 3; }
 
 int gcow_layernorm_bwd(const void* dy, const void* x, const float* gamma, const float* mean, const float* rstd,
                        void* dx, float* part, float* dgamma_dbeta, int rows, int H, void* stream) {
   if (H % 8 || rows <= 0 || H > 4096) return -1;
-  const int parts = gcow_layernorm_bwd_parts(rows);
-  const size_t smem = (size_t)8 * H * sizeof(float);
-  static bool attr = false;
-  if (!attr) { cudaFuncSetAttribute(layernorm_bwd_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * 4096 * 4); attr = true; }
-  const int ch = (H + 255) / 256;
-#define GCOW_LN_BWD(CH) gcow::launch_dependent(layernorm_bwd_kernel<CH>, dim3(parts), dim3(128), smem, (cudaStream_t)stream, (const bf16*)dy, (const bf16*)x, gamma, mean, rstd, (bf16*)dx, part, rows, H)
-  switch (ch) {
-    case 1: GCOW_LN_BWD(1); break;
-    case 2: GCOW_LN_BWD(2); break;
-    case 3: GCOW_LN_BWD(3); break;
-    case 4: GCOW_LN_BWD(4); break;
-    default: GCOW_LN_BWD(0); break;
+  const int most = gcow_layernorm_bwd_parts(rows);
+  // 512 threads from where their sums' way through shared memory is less than what fewer partial sums save: 1024 x 1024 7.4 us with 128,
+  // 8.5 with 512; 1280 8.8, 8.5; 2048 9.5, 8.7; the other widths change sides at the same place.
+  const bool wide = rows > 1280;
+  const int fit = (rows + 15) / 16, grid = H > 1024 || !wide ? most : fit < 148 ? fit : 148;
+#define GCOW_LN_BWD(K, T, SMEM) do { \
+    if ((SMEM) > 48 * 1024) { \
+      static std::atomic<bool> allowed[64]; \
+      int dev = 0; \
+      cudaGetDevice(&dev); \
+      if (dev >= 64 || !allowed[dev].load(std::memory_order_acquire)) { \
+        const int e = (int)cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024); \
+        if (e) return e; \
+        if (dev < 64) allowed[dev].store(true, std::memory_order_release); \
+      } \
+    } \
+    gcow::launch_dependent(K, dim3(grid), dim3(T), SMEM, (cudaStream_t)stream, (const bf16*)dy, (const bf16*)x, gamma, mean, rstd, (bf16*)dx, part, rows, H); \
+  } while (0)
+#define GCOW_LN_ROWS(CH) do { \
+    if (wide) GCOW_LN_BWD((layernorm_bwd_rows_kernel<CH, kLnWide>), kLnWide, (kLnBwdSmem<CH, kLnWide>)); \
+    else GCOW_LN_BWD((layernorm_bwd_rows_kernel<CH, kLnNarrow>), kLnNarrow, (kLnBwdSmem<CH, kLnNarrow>)); \
+  } while (0)
+  switch ((H + 255) / 256) {
+    case 1: GCOW_LN_ROWS(1); break;
+    case 2: GCOW_LN_ROWS(2); break;
+    case 3: GCOW_LN_ROWS(3); break;
+    case 4: GCOW_LN_ROWS(4); break;
+    default: GCOW_LN_BWD(layernorm_bwd_kernel, 128, (size_t)8 * H * sizeof(float)); break;
   }
+#undef GCOW_LN_ROWS
 #undef GCOW_LN_BWD
   gcow::launch_dependent(reduce_partials_tall_kernel, dim3((2 * H + 31) / 32), dim3(32, 32), 0, (cudaStream_t)stream, (const float*)part,
-                   dgamma_dbeta, parts, 2 * H);
+                   dgamma_dbeta, grid, 2 * H);
   return (int)cudaGetLastError();
 }
 

@@ -46,6 +46,32 @@ def test_layernorm_rows_in_registers(H, rows):
     assert bool(((y.double() - ref).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("H", [8, 16, 24, 248, 256, 264, 520, 776, 1024, 1032])
+@pytest.mark.parametrize("rows", [1, 5, 1280, 1281, 2400, 5003])
+def test_layernorm_backward_with_a_row_ahead(H, rows):
+    """Each number of column chunks, the narrowest rows, fewer rows than warps, both CTA sizes around the line between them and one to
+    three rows a warp, against float64."""
+    from gcow_b200.ops import kernels as K
+    torch.manual_seed(H * 7 + rows)
+    x = torch.randn(rows, H, device="cuda").bfloat16().requires_grad_(True)
+    g, b = torch.randn(H, device="cuda", requires_grad=True), torch.randn(H, device="cuda", requires_grad=True)
+    dy = torch.randn(rows, H, device="cuda").bfloat16()
+    K.layernorm(x, g, b, 1e-12).backward(dy)
+    xd, d, gd = x.detach().double(), dy.double(), g.detach().double()
+    rs = (xd.var(1, unbiased=False, keepdim=True) + 1e-12).rsqrt()
+    xh = (xd - xd.mean(1, keepdim=True)) * rs
+    gg = d * gd
+    dx = rs * (gg - gg.mean(1, keepdim=True) - xh * (gg * xh).mean(1, keepdim=True))
+    # bf16 rounds to 2^-9. In fp32 the sums over H values, and the mean and deviation behind xh, are off by up to (H + 16) 2^-24 of the
+    # sum of their terms' sizes (values of size up to 6, one more factor rs); the sums over the rows by up to rows * 2^-24 of theirs.
+    eps = 8 * (H + 16) * 2.0 ** -24 * (1 + rs)
+    size = rs * (gg.abs() + gg.abs().mean(1, keepdim=True) + (1 + xh.abs()) * (gg * xh).abs().mean(1, keepdim=True))
+    assert bool(((x.grad.double() - dx).abs() <= 2.0 ** -8 * dx.abs() + eps * size + 1e-6).all())
+    off = (eps + (rows + 64) * 2.0 ** -24) * d.abs() * (1 + xh.abs())
+    assert bool(((g.grad.double() - (d * xh).sum(0)).abs() <= off.sum(0) + 1e-6).all())
+    assert bool(((b.grad.double() - d.sum(0)).abs() <= off.sum(0) + 1e-6).all())
+
+
 def test_gelu_fwd_bwd():
     from gcow_b200.ops import kernels as K
     x = (torch.randn(4096, 1024, device="cuda") * 2).requires_grad_(True)
