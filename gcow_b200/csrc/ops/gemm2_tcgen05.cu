@@ -52,19 +52,21 @@ struct Params {
   int slice_blocks;        // stages per slice of the reduction
   int halves;              // weight gradient, an item per pair at most: a slice's two halves have an accumulator each
   size_t slice_stride;     // elements from one slice's result to the next
+  TileOrder order;
   uint32_t* error;
 };
 
 // An item of work: a tile, or the left or right half of one, over a slice of the reduction.
 struct Item { int m0, n0, kb0, kb1, slice; bool half; };
-template <bool SLICES> __device__ __forceinline__ Item item_at(const Params& p, int i, int tiles_m, int tiles, int kblocks) {
+template <bool SLICES> __device__ __forceinline__ Item item_at(const Params& p, int i, int tiles, int kblocks) {
   Item r;
   r.half = i >= p.whole;
   const int j = r.half ? (i - p.whole) >> 1 : i;
   r.slice = SLICES ? j / tiles : 0;
   const int tile = r.half ? p.whole + j : j - r.slice * tiles;
-  r.m0 = (tile % tiles_m) * BM;
-  r.n0 = (tile / tiles_m) * BN + (r.half ? ((i - p.whole) & 1) * (BN / 2) : 0);
+  p.order.at(tile, r.m0, r.n0);
+  r.m0 *= BM;
+  r.n0 = r.n0 * BN + (r.half ? ((i - p.whole) & 1) * (BN / 2) : 0);
   r.kb0 = SLICES ? r.slice * p.slice_blocks : 0;
   r.kb1 = SLICES && r.kb0 + p.slice_blocks < kblocks ? r.kb0 + p.slice_blocks : kblocks;
   return r;
@@ -166,7 +168,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       uint32_t s = 0, phase = 0;
       bool ok = true;
       for (int i = pair; i < p.items && ok; i += pairs) {
-        const Item it = item_at<A_MN>(p, i, tiles_m, tiles, kblocks);
+        const Item it = item_at<A_MN>(p, i, tiles, kblocks);
         const int m0 = it.m0 + (int)rank * 128, n0 = it.n0 + (int)rank * (it.half ? 64 : 128);
         const CUtensorMap* const map_b = it.half ? &tmap_bh : &tmap_b;
         for (int kb = it.kb0; kb < it.kb1; kb++) {
@@ -197,7 +199,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         return __all_sync(0xffffffffu, mbar_wait_abortable(&sm->abort, bar, parity, p.error, code)) != 0;
       };
       for (int i = pair; i < p.items && ok; i += pairs, t++) {
-        const Item it = item_at<A_MN>(p, i, tiles_m, tiles, kblocks);
+        const Item it = item_at<A_MN>(p, i, tiles, kblocks);
         const uint32_t idesc = idesc0 | ((uint32_t)((it.half ? BN / 2 : BN) >> 3) << 17), chunk_b = it.half ? CHUNK_BYTES / 2 : CHUNK_BYTES;
         const uint32_t acc = t & 1, aphase = (t >> 1) & 1;
         if (!(ok = wait(&sm->tmem_empty[acc], aphase ^ 1, 2))) break;
@@ -247,7 +249,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     uint32_t t = 0;
     bool ok = true;
     for (int i = pair; i < p.items && ok; i += pairs, t++) {
-      const Item it = item_at<A_MN>(p, i, tiles_m, tiles, kblocks);
+      const Item it = item_at<A_MN>(p, i, tiles, kblocks);
       const int m0 = it.m0 + (int)rank * 128, n0 = it.n0;
       const int cols = (it.half ? BN / 2 : BN) / GROUPS, chunks = cols / 32, col0 = (ew / 4) * cols;   // this warp's
       const uint32_t acc = t & 1, aphase = (t >> 1) & 1;
@@ -482,6 +484,7 @@ int gcow_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN), rest = tiles % max_pairs;
   p.whole = rest && 2 * rest <= max_pairs ? tiles - rest : tiles;
   p.items = p.whole + 2 * (tiles - p.whole);
+  p.order = tile_order(M, N, BM, BN);
   CUtensorMap mh = mb;
   if (p.items > p.whole) {
     rc = b_mn ? make_map_mnfold(&mh, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, 1)
@@ -549,6 +552,7 @@ int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, int M, int N, i
   p.slice_blocks = (kblocks + slices - 1) / slices;
   if ((slices - 1) * p.slice_blocks >= kblocks) return -2;   // an empty slice would leave its part unwritten
   p.whole = p.items = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * slices;
+  p.order = tile_order(M, N, BM, BN);
   p.slice_stride = (size_t)M * N;
   p.halves = p.items <= max_pairs;
   return launch(gemm2_bf16_kernel<true, true, false, false>, Epilogue<false>::THREADS, max_pairs, ma, mb, mb, p, stream);

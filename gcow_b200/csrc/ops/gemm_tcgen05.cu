@@ -69,6 +69,7 @@ struct Params {
   uint32_t stage_tx;       // a smaller box: the rest of its tile is never read back); bytes both copies of a stage bring
   int tma_store;           // bf16 C without residual / aux: the epilogue hands 32 x 32 boxes to the TMA (tmap_c is valid)
   long long stride_c;      // elements between consecutive C (and residual) matrices
+  tc::TileOrder order;         // of the tiles of one product
   uint32_t* error;         // device word, set non-zero when a wait gave up
 };
 
@@ -143,7 +144,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         const int bz = tile / tiles_mn, tmn = tile - bz * tiles_mn;
-        const int m0 = (tmn % tiles_m) * BM, n0 = (tmn / tiles_m) * BN;
+        int m0, n0;
+        p.order.at(tmn, m0, n0);
+        m0 *= BM; n0 *= BN;
         for (int kb = 0; kb < kblocks; kb++) {
           if (!(ok = mbar_wait(sm, &sm->empty[s], phase ^ 1, p.error, 1))) break;
           mbar_expect_tx(&sm->full[s], p.stage_tx);
@@ -224,7 +227,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, t++) {
       const int bz = tile / tiles_mn, tmn = tile - bz * tiles_mn;
-      const int m0 = (tmn % tiles_m) * BM, n0 = (tmn / tiles_m) * BN;
+      int m0, n0;
+      p.order.at(tmn, m0, n0);
+      m0 *= BM; n0 *= BN;
       const uint32_t acc0 = HALVES == 1 ? (t & 1) : 0, aphase = HALVES == 1 ? ((t >> 1) & 1) : (t & 1);
       ok = mbar_wait(sm, &sm->tmem_full[acc0], aphase, p.error, 4);
       ok = __all_sync(0xffffffffu, ok);   // the tensor-memory loads below need the whole warp
@@ -586,6 +591,7 @@ static int gemm_launch(const void* A, const void* B, void* C, int M, int N, int 
   Params p;
   p.C = C; p.bias = bias; p.residual = residual; p.aux = aux;
   p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.flags = flags; p.error = error;
+  p.order = tile_order(M, N, bm, BN);
   p.batch = batch; p.stride_c = batch > 1 ? stride_c : 0;
   p.a_merged = a_merged; p.b_merged = b_merged;
   p.a_chunks = a_rows / 64; p.b_chunks = b_rows / 64;

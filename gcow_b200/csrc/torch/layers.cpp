@@ -192,13 +192,14 @@ Tensor gemm(const Tensor& a, const Tensor& b, const GemmOpts& o, const On& on) {
   if (aux.defined()) flags |= o.pre_gelu_out.defined() ? kAuxOut : kGeluGrad;
   const int lda = (int)a.stride(0), ldb = (int)b.stride(0), ldc = (int)out.stride(0);
   // A large product goes to CTA pairs: two SMs per 256 x 256 tile have the one-CTA tile's traffic per flop and an overlapped
-  // epilogue as well. Long reductions with nothing but a bias behind them stay on the one-CTA tile, whose main loop is a little
-  // faster (8192^3 682 us, pairs 730; 16384 x 1024 x 4096 plain 107 and 112, with a residual 137
-  // and 122), and so do those below 512 (the 1x1 convolutions of a ResNet), which the output stream bounds: the one-CTA
+  // epilogue as well (16384 x 1024 x 4096 103 us on the one-CTA tile, 99.7 on pairs; x 768 x 3072 91, 62; 32768 x 1024 x 4096 199, 192;
+  // 4096^3 174, 154). From K = 8192 on, both operands stored [rows][K] and nothing but a bias behind them, the one-CTA tile's main
+  // loop is a little faster (8192^3 860, 936; 16384 x 2048 x 8192 400, 405); with B stored [K][N] it is not (8192^3 915, 882).
+  // Reductions below 512 (the 1x1 convolutions of a ResNet) stay there too: the output stream bounds them, and the one-CTA
   // kernel's TMA stores are 15 to 30 % faster there.
   const bool can_pair = pair_gemm_enabled() && !o.a_t && !(flags & (kOutF32 | kAccumulate)) && !o.max_ctas && !o.tile_rows;
   const bool by_rule = K % 64 == 0 && K >= 512 && N % (o.b_t ? 64 : 32) == 0 && M >= 1024 && N >= 256 && lda % 8 == 0 && ldb % 8 == 0 &&
-                       ldc % 8 == 0 && !(K >= 2048 && ((M + 255) / 256) * ((N + 255) / 256) >= 118 && !(flags & (kGelu | kResidual | kGeluGrad)));
+                       ldc % 8 == 0 && !(K >= 8192 && !o.b_t && ((M + 255) / 256) * ((N + 255) / 256) >= 118 && !(flags & (kGelu | kResidual | kGeluGrad)));
   if (can_pair && (o.pair < 0 ? by_rule : o.pair > 0)) {
     const int err = gcow_gemm2_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, lda, ldb, ldc, f32(o.bias),
                                     raw(o.residual), raw(aux), flags, on.error, o.b_t, on.stream);

@@ -194,3 +194,19 @@ def test_pair_gemm_matches_fp32_reference(M, N, K, monkeypatch):
         K_.check_errors()
         ref3 = _ref(a, b, residual=res)
         assert (y.float() - ref3).abs().max().item() / ref3.abs().max().item() < 2e-2
+
+
+@pytest.mark.parametrize("M,N", [(1030, 264), (1300, 1288), (2305, 520), (260, 2600), (24, 48), (5000, 1000), (21000, 320)])
+def test_every_tile_is_taken_once_in_either_order(M, N, monkeypatch):
+    """Rows of tiles in groups of four and a shorter last group (more rows than columns), whole columns of tiles (fewer), last rounds
+    cut into halves, in all three kernels. The sums are whole numbers of at most 192, which bf16 and any order of addition hold exactly."""
+    from gcow_b200.ops import kernels as K_
+    torch.manual_seed(M + N)
+    a = torch.randint(-1, 2, (M, 192), device="cuda").bfloat16()
+    b = torch.randint(-1, 2, (N, 192), device="cuda").bfloat16()
+    ref = (a.float() @ b.float().t()).bfloat16()
+    for rows in (0, 128, 256):
+        assert torch.equal(K_.gemm_bf16(a, b, tile_rows=rows), ref), rows
+    monkeypatch.setattr(K_, "_pair_gemm", True)
+    assert torch.equal(K_.gemm_bf16(a, b), ref)
+    K_.check_errors()
