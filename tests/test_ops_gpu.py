@@ -72,6 +72,19 @@ def test_layernorm_backward_with_a_row_ahead(H, rows):
     assert bool(((b.grad.double() - d.sum(0)).abs() <= off.sum(0) + 1e-6).all())
 
 
+@pytest.mark.parametrize("parts,n,off", [(1, 262144, 0), (3, 262144, 0), (8, 262148, 0), (9, 262144, 0), (3, 262140, 0), (3, 262146, 0),
+                                         (4, 300000, 1), (5, 1048579, 0), (70, 300, 0)])
+def test_ordered_sums_of_whole_numbers(parts, n, off):
+    """Both sides of every line between the three kernels: length, multiples of four, alignment, number of partials. Sums of whole
+    numbers are exact."""
+    from gcow_b200 import _native
+    part = torch.randint(-1000, 1000, (parts * n + off,), device="cuda").float()[off:]
+    out = torch.full((n + 8,), 7.0, device="cuda")
+    rc = _native.cuda().gcow_reduce_partials(part.data_ptr(), out.data_ptr(), parts, n, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    assert torch.equal(out[:n], part.view(parts, n).sum(0)) and bool((out[n:] == 7).all())
+
+
 def test_gelu_fwd_bwd():
     from gcow_b200.ops import kernels as K
     x = (torch.randn(4096, 1024, device="cuda") * 2).requires_grad_(True)
