@@ -428,32 +428,44 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
   if (warp == 0) tmem_free_all(tmem);
 }
 
-// delta[b][h][s] = sum_d dO[b][s][h][d] * O[b][s][h][d]; eight lanes per row, so that a warp reads whole lines (262 144
-// rows: 15 us, one thread per row took 24).
-__global__ void attn_delta_kernel(const __nv_bfloat16* o, const __nv_bfloat16* go,
-                                  float* __restrict__ delta, int B, int S, int H) {
+// delta[b][h][s] = sum_d dO[b][s][h][d] * O[b][s][h][d]; eight lanes per row, so that a warp reads whole lines, and kDeltaRows rows to a
+// lane, all of whose loads are under way before the first sum. Bound by memory: 262 144 rows (67 MB, 10 us) 15.5 us with one row to a lane
+// and 64-bit divisions for its place, now 12.7.
+constexpr int kDeltaRows = 4;
+__global__ void __launch_bounds__(256)
+attn_delta_kernel(const __nv_bfloat16* o, const __nv_bfloat16* go, float* __restrict__ delta, uint32_t rows, uint32_t S, uint32_t H) {
   pdl_trigger();
   pdl_wait();
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t i = t >> 3, rows = (size_t)B * S * H;                   // over b, s, h
-  const int part = (int)(t & 7);
-  float acc = 0.0f;
-  if (i < rows) {
-    const uint4 x = reinterpret_cast<const uint4*>(o + i * D)[part], y = reinterpret_cast<const uint4*>(go + i * D)[part];
-    const __nv_bfloat162* xb = reinterpret_cast<const __nv_bfloat162*>(&x);
-    const __nv_bfloat162* yb = reinterpret_cast<const __nv_bfloat162*>(&y);
+  const uint32_t first = blockIdx.x * (32 * kDeltaRows) + (threadIdx.x >> 3), part = threadIdx.x & 7;      // rows over b, s, h
+  uint4 x[kDeltaRows], y[kDeltaRows];
+#pragma unroll
+  for (int k = 0; k < kDeltaRows; k++) {
+    const uint32_t i = first + 32 * k;
+    x[k] = y[k] = make_uint4(0, 0, 0, 0);
+    if (i < rows) {
+      x[k] = reinterpret_cast<const uint4*>(o + (size_t)i * D)[part];
+      y[k] = reinterpret_cast<const uint4*>(go + (size_t)i * D)[part];
+    }
+  }
+  float mine = 0.0f;                                   // lane `part` < kDeltaRows stores row `part`
+#pragma unroll
+  for (int k = 0; k < kDeltaRows; k++) {
+    const __nv_bfloat162* xb = reinterpret_cast<const __nv_bfloat162*>(&x[k]);
+    const __nv_bfloat162* yb = reinterpret_cast<const __nv_bfloat162*>(&y[k]);
+    float acc = 0.0f;
 #pragma unroll
     for (int e = 0; e < 4; e++) {
       const float2 a = __bfloat1622float2(xb[e]), c = __bfloat1622float2(yb[e]);
       acc = fmaf(a.x, c.x, fmaf(a.y, c.y, acc));
     }
-  }
 #pragma unroll
-  for (int d = 1; d < 8; d <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
-  if (i < rows && part == 0) {
-    const int h = (int)(i % H);
-    const size_t bs = i / H;
-    delta[((bs / S) * H + h) * S + bs % S] = acc;
+    for (int d = 1; d < 8; d <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+    if ((int)part == k) mine = acc;
+  }
+  const uint32_t i = first + 32 * part;
+  if (part < kDeltaRows && i < rows) {
+    const uint32_t bs = i / H, h = i - bs * H, b = bs / S, at = bs - b * S;
+    delta[((size_t)b * H + h) * S + at] = mine;
   }
 }
 
@@ -897,8 +909,9 @@ int gcow_attention_bwd(const void* qkv, const void* out, const void* dout, const
   Params p = {};
   p.lse = const_cast<float*>(lse); p.delta = delta; p.B = B; p.S = S; p.H = H;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.error = error;
-  const size_t rows = (size_t)B * S * H;
-  gcow::launch_dependent(attn_delta_kernel, dim3((unsigned)((rows * 8 + 255) / 256)), dim3(256), 0, st, (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, delta, B, S, H);
+  const uint32_t rows = (uint32_t)B * S * H;                 // of 128 bytes each in every tensor: far below 2^32 in any memory
+  gcow::launch_dependent(attn_delta_kernel, dim3((unsigned)(((size_t)rows + 32 * kDeltaRows - 1) / (32 * kDeltaRows))), dim3(256), 0, st,
+                         (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, delta, rows, (uint32_t)S, (uint32_t)H);
   gcow::launch_dependent(attn_bwd_kernel, dim3(2 * (units < 148 ? units : 148)), dim3(Shape<false>::THREADS), kBwdSmem, st, in[0], in[1], in[2], in[3],
                          dq, dk, dv, p, units, mode);
   return (int)cudaGetLastError();
