@@ -34,10 +34,13 @@ constexpr int CHUNK_BYTES = 128 * 64 * 2;             // 128 rows x 128 bytes
 constexpr int OPER_BYTES = 2 * CHUNK_BYTES;           // one CTA's half of an operand, one stage
 constexpr int STAGE_BYTES = 2 * OPER_BYTES;           // 64 KB
 constexpr int STAGES = 3;
+// What an epilogue reads besides the accumulator.
+enum Side : int { kNothing = 0, kSum = 1, kArgument = 2 };      // a residual; the argument of a GELU' factor (and perhaps a residual)
 // Epilogue warps: eight, or sixteen for a GELU, whose arithmetic two warps per scheduler leave half of the issue slots to
 // (bias, GELU and its argument kept: 16384 x 4096 x 1024 142 -> 129 us, x 3072 110 -> 97, x 1024 44 -> 36; with a residual
-// sixteen are slower, 144 and 156, and plain 95 and 98).
-template <bool WIDE> struct Epilogue { static constexpr int WARPS = WIDE ? 16 : 8, THREADS = 64 + 32 * WARPS; };
+// sixteen are slower, 144 and 156, and plain 95 and 98). Twelve for a GELU' factor, whose registers sixteen leave no room for: 159 us with
+// eight, 145 with twelve, 192 with sixteen; a residual gains nothing from twelve (106 and 107 at 16384 x 1024 x 4096).
+template <int SIDE, bool WIDE> struct Epilogue { static constexpr int WARPS = WIDE ? 16 : SIDE == kArgument ? 12 : 8, THREADS = 64 + 32 * WARPS; };
 constexpr uint32_t TMEM_COLS = 512;
 
 enum Flags : int { kBias = 2, kGelu = 4, kResidual = 8, kAuxOut = 32, kGeluGrad = 64 };
@@ -122,13 +125,12 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128_16k(uint32_t saddr) {
 }
 
 // B_MN: B is stored [K][N] (the data-gradient product dX = dY * W reads the weight matrix in place); A_MN: A is stored [K][M]
-// (with B_MN the weight gradient, which reads both in place). SIDE: the epilogue reads
-// a residual or the argument of a GELU' factor.
-template <bool A_MN, bool B_MN, bool SIDE, bool WIDE>
-__global__ void __launch_bounds__(Epilogue<WIDE>::THREADS, 1)
+// (with B_MN the weight gradient, which reads both in place). SIDE: what the epilogue reads.
+template <bool A_MN, bool B_MN, int SIDE, bool WIDE>
+__global__ void __launch_bounds__(Epilogue<SIDE, WIDE>::THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   const __grid_constant__ CUtensorMap tmap_bh, const Params p) {
-  constexpr int EPI_WARPS = Epilogue<WIDE>::WARPS;
+  constexpr int EPI_WARPS = Epilogue<SIDE, WIDE>::WARPS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   Smem* sm = reinterpret_cast<Smem*>(base + STAGES * STAGE_BYTES);
@@ -244,28 +246,43 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     const int q = warp & 3, ew = warp - 2;
     constexpr int GROUPS = EPI_WARPS / 4;               // of columns
     const bool wide_bias = ((uintptr_t)p.bias & 15) == 0;
-    [[maybe_unused]] const __nv_bfloat16* const ahead = p.flags & kGeluGrad ? p.aux : p.residual;
+    [[maybe_unused]] const __nv_bfloat16* const ahead = SIDE == kArgument ? p.aux : p.residual;
     uint8_t* stg = stage_base + ew * kStageWarpBytes;
     uint32_t t = 0;
     bool ok = true;
+    // A tile's blocks of 32 columns go to the column groups in order, as evenly as they can. What the epilogue reads besides the
+    // accumulator is fetched one block ahead, the next tile's first block with this one's last: read where it is used, every
+    // block stood for its load's whole latency, and few warps per scheduler cover little of it (16384 x 4096 x 1024 with a residual
+    // 189 -> 144 us, times GELU' 247 -> 151). The first block under the wait for its own tile was no better where the epilogue sets the
+    // pace, and there is none: with the tile before, and one copy of the code per block in the loop below, a residual 132 -> 122 us (x 1024 x
+    // 1024 52 -> 48, 2048 x 768 x 3072 25.5 -> 23.9), GELU' 177 -> 155 (x 3072 x 768 129 -> 114).
+    constexpr bool EVEN = BN / 64 % GROUPS == 0;
+    [[maybe_unused]] auto blocks_before = [](bool half, int group) { return ((half ? BN / 64 : BN / 32) * group + GROUPS - 1) / GROUPS; };
+    [[maybe_unused]] uint4 pf[4];                         // four lanes per row, as the staging helpers have it
+    [[maybe_unused]] auto fetch = [&](int row0, int n) {
+      n += (lane & 3) * 8;
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int row = row0 + j * 8 + (lane >> 2);
+        pf[j] = make_uint4(0, 0, 0, 0);
+        if (n < p.N && row < p.M) pf[j] = *reinterpret_cast<const uint4*>(ahead + (size_t)row * p.ldc + n);
+      }
+    };
+    [[maybe_unused]] auto fetch_first = [&](int i) {
+      if (i >= p.items) return;
+      const Item it = item_at<A_MN>(p, i, tiles, kblocks);
+      fetch(it.m0 + (int)rank * 128 + q * 32, it.n0 + blocks_before(it.half, ew / 4) * 32);
+    };
+    if (SIDE) fetch_first(pair);
     for (int i = pair; i < p.items && ok; i += pairs, t++) {
       const Item it = item_at<A_MN>(p, i, tiles, kblocks);
       const int m0 = it.m0 + (int)rank * 128, n0 = it.n0;
-      const int cols = (it.half ? BN / 2 : BN) / GROUPS, chunks = cols / 32, col0 = (ew / 4) * cols;   // this warp's
+      // this warp's
+      const int cols = (it.half ? BN / 2 : BN) / GROUPS, chunks = EVEN ? cols / 32 : blocks_before(it.half, ew / 4 + 1) - blocks_before(it.half, ew / 4),
+                col0 = EVEN ? (ew / 4) * cols : blocks_before(it.half, ew / 4) * 32;
       const uint32_t acc = t & 1, aphase = (t >> 1) & 1;
       const int mw = m0 + q * 32;                         // the warp's first row
-      // four lanes per row, as the staging helpers have it
-      [[maybe_unused]] uint4 pf[4];
-      [[maybe_unused]] auto fetch = [&](int c) {
-        const int n = n0 + col0 + c * 32 + (lane & 3) * 8;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const int row = mw + j * 8 + (lane >> 2);
-          pf[j] = make_uint4(0, 0, 0, 0);
-          if (c < chunks && n < p.N && row < p.M) pf[j] = *reinterpret_cast<const uint4*>(ahead + (size_t)row * p.ldc + n);
-        }
-      };
-      if (SIDE) fetch(0);
+      [[maybe_unused]] auto fetch_after = [&](int c) { if (c + 1 < chunks) fetch(mw, n0 + col0 + (c + 1) * 32); else fetch_first(i + pairs); };
       ok = mbar_wait_abortable(&sm->abort, &sm->tmem_full[acc], aphase, p.error, 4);
       ok = __all_sync(0xffffffffu, ok);   // the tensor-memory loads below need the whole warp
       if (!ok) break;
@@ -273,13 +290,12 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const int m = m0 + q * 32 + lane;
       const bool row_ok = m < p.M;
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN + col0;
-      // What the epilogue reads besides the accumulator (the GELU's argument, else the residual) is fetched one block of
-      // 32 columns ahead, the first block under the wait for the tile: read where it is used, every block stood for
-      // its load's whole latency, and with two warps per scheduler nothing covered it (16384 x 4096 x 1024: with a
-      // residual 189 -> 144 us, times GELU' 247 -> 151 us, plain 95 us).
       auto process = [&](const uint32_t (&r)[32], int c) {
         const int n = n0 + col0 + c * 32;
-        if (n >= p.N || mw >= p.M) return;                // warp-uniform; the launcher guarantees N % 32 == 0
+        if (n >= p.N || mw >= p.M) {                      // warp-uniform; the launcher guarantees N % 32 == 0
+          if (SIDE) fetch_after(c);
+          return;
+        }
         const size_t off = (size_t)m * p.ldc + n;
         float v[32];
 #pragma unroll
@@ -315,12 +331,12 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         if (p.flags & kGelu) gelu32(v);                    // not together with kGeluGrad
         if (SIDE) {
           warp_place_rows(stg, lane, pf);
-          fetch(c + 1);
+          fetch_after(c);
 #pragma unroll
           for (int k = 0; k < 4; k++) {
             float x[8];
             own_chunk(stg, lane, k, x);
-            if (p.flags & kGeluGrad) {
+            if (SIDE == kArgument) {
               gelu_grad8(v + 8 * k, x);
             } else {
 #pragma unroll
@@ -329,22 +345,33 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
           __syncwarp();
         }
-        if (SIDE && (p.flags & kGeluGrad) && (p.flags & kResidual)) warp_load_rows_bf16<true>(stg, lane, p.residual, off, row_ok, v);
+        if (SIDE == kArgument && (p.flags & kResidual)) warp_load_rows_bf16<true>(stg, lane, p.residual, off, row_ok, v);
         warp_store_rows_bf16(stg, lane, v, p.C, off, row_ok);
       };
-      // tensor-memory loads one block ahead of the arithmetic (sixteen warps hide them from one another)
-      uint32_t ra[32], rb[32];
+      // tensor-memory loads one block ahead of the arithmetic (sixteen warps hide them from one another, and with a side operand the
+      // registers go to the blocks of that fetched ahead)
+      uint32_t ra[32];
       tc_ld32(taddr, ra);
+      if constexpr (SIDE) {
 #pragma unroll 1
-      for (int c = 0; c < chunks; c += 2) {
-        tc_wait_ld();
-        if (!WIDE && c + 1 < chunks) tc_ld32(taddr + (c + 1) * 32, rb);
-        process(ra, c);
-        if (c + 1 < chunks) {
-          if (WIDE) tc_ld32(taddr + (c + 1) * 32, rb);
+        for (int c = 0; c < chunks; c++) {
           tc_wait_ld();
-          if (!WIDE && c + 2 < chunks) tc_ld32(taddr + (c + 2) * 32, ra);
-          process(rb, c + 1);
+          process(ra, c);
+          if (c + 1 < chunks) tc_ld32(taddr + (c + 1) * 32, ra);
+        }
+      } else {
+        uint32_t rb[32];
+#pragma unroll 1
+        for (int c = 0; c < chunks; c += 2) {
+          tc_wait_ld();
+          if (!WIDE && c + 1 < chunks) tc_ld32(taddr + (c + 1) * 32, rb);
+          process(ra, c);
+          if (c + 1 < chunks) {
+            if (WIDE) tc_ld32(taddr + (c + 1) * 32, rb);
+            tc_wait_ld();
+            if (!WIDE && c + 2 < chunks) tc_ld32(taddr + (c + 2) * 32, ra);
+            process(rb, c + 1);
+          }
         }
       }
       // this CTA's half of the accumulator has been read out: tell the MMA thread in CTA 0
@@ -395,12 +422,13 @@ static int make_map_mnfold(CUtensorMap* map, const void* ptr, uint64_t K, uint64
 }
 
 using KernelFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, Params);
-constexpr size_t kSmemBytes = (size_t)STAGES * STAGE_BYTES + sizeof(Smem) + 16 + (size_t)Epilogue<true>::WARPS * kStageWarpBytes + 1024;
+constexpr size_t kSmemBytes = (size_t)STAGES * STAGE_BYTES + sizeof(Smem) + 16 + (size_t)Epilogue<kNothing, true>::WARPS * kStageWarpBytes + 1024;
 
-static KernelFn pick(bool b_mn, bool side, bool wide) {
-  if (side) return b_mn ? gemm2_bf16_kernel<false, true, true, false> : gemm2_bf16_kernel<false, false, true, false>;
-  if (wide) return b_mn ? gemm2_bf16_kernel<false, true, false, true> : gemm2_bf16_kernel<false, false, false, true>;
-  return b_mn ? gemm2_bf16_kernel<false, true, false, false> : gemm2_bf16_kernel<false, false, false, false>;
+static KernelFn pick(bool b_mn, int side, bool wide) {
+  if (side == kArgument) return b_mn ? gemm2_bf16_kernel<false, true, kArgument, false> : gemm2_bf16_kernel<false, false, kArgument, false>;
+  if (side == kSum) return b_mn ? gemm2_bf16_kernel<false, true, kSum, false> : gemm2_bf16_kernel<false, false, kSum, false>;
+  if (wide) return b_mn ? gemm2_bf16_kernel<false, true, kNothing, true> : gemm2_bf16_kernel<false, false, kNothing, true>;
+  return b_mn ? gemm2_bf16_kernel<false, true, kNothing, false> : gemm2_bf16_kernel<false, false, kNothing, false>;
 }
 
 static int launch(KernelFn kernel, int threads, int max_pairs, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mh,
@@ -433,8 +461,9 @@ int gcow_gemm2_max_pairs() {
   static std::once_flag once;
   static int pairs = 0;
   std::call_once(once, [] {
-    for (const KernelFn kernel : {pick(false, false, false), pick(false, true, false), pick(false, false, true), pick(true, false, false),
-                                  pick(true, true, false), pick(true, false, true), (KernelFn)gemm2_bf16_kernel<true, true, false, false>}) {
+    for (const KernelFn kernel : {pick(false, kNothing, false), pick(false, kNothing, true), pick(false, kSum, false), pick(false, kArgument, false),
+                                  pick(true, kNothing, false), pick(true, kNothing, true), pick(true, kSum, false), pick(true, kArgument, false),
+                                  (KernelFn)gemm2_bf16_kernel<true, true, kNothing, false>}) {
       if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes) != cudaSuccess) {
         cudaGetLastError();
         return;
@@ -442,14 +471,14 @@ int gcow_gemm2_max_pairs() {
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2, 1, 1);
-    cfg.blockDim = dim3(Epilogue<true>::THREADS, 1, 1);
+    cfg.blockDim = dim3(Epilogue<kNothing, true>::THREADS, 1, 1);
     cfg.dynamicSmemBytes = kSmemBytes;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
     cfg.attrs = &attr; cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm2_bf16_kernel<false, false, false, true>, &cfg) == cudaSuccess) pairs = n;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm2_bf16_kernel<false, false, kNothing, true>, &cfg) == cudaSuccess) pairs = n;
     else cudaGetLastError();
   });
   return pairs;
@@ -493,9 +522,10 @@ int gcow_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
   }
   // Its own instance for launches that read nothing besides the accumulator: the blocks fetched ahead cost registers, for
   // which the epilogue spilled (16384 x 4096 x 1024: plain 100 -> 95 us, bias 106 -> 97).
-  const bool side = flags & (kResidual | kGeluGrad), wide = !side && (flags & kGelu);
-  const KernelFn kernel = pick(b_mn, side, wide);
-  return launch(kernel, wide ? Epilogue<true>::THREADS : Epilogue<false>::THREADS, max_pairs, ma, mb, mh, p, stream);
+  const int side = flags & kGeluGrad ? kArgument : flags & kResidual ? kSum : kNothing;
+  const bool wide = !side && (flags & kGelu);
+  const int threads = wide ? Epilogue<kNothing, true>::THREADS : side == kArgument ? Epilogue<kArgument, false>::THREADS : Epilogue<kSum, false>::THREADS;
+  return launch(pick(b_mn, side, wide), threads, max_pairs, ma, mb, mh, p, stream);
 }
 
 // How many slabs of equal length the one-CTA kernel's weight gradient cuts K rows into for an M x N result: it doubles while
@@ -555,7 +585,7 @@ int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, int M, int N, i
   p.order = tile_order(M, N, BM, BN);
   p.slice_stride = (size_t)M * N;
   p.halves = p.items <= max_pairs;
-  return launch(gemm2_bf16_kernel<true, true, false, false>, Epilogue<false>::THREADS, max_pairs, ma, mb, mb, p, stream);
+  return launch(gemm2_bf16_kernel<true, true, kNothing, false>, Epilogue<kNothing, false>::THREADS, max_pairs, ma, mb, mb, p, stream);
 }
 
 }  // extern "C"

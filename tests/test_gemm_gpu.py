@@ -210,3 +210,28 @@ def test_every_tile_is_taken_once_in_either_order(M, N, monkeypatch):
     monkeypatch.setattr(K_, "_pair_gemm", True)
     assert torch.equal(K_.gemm_bf16(a, b), ref)
     K_.check_errors()
+
+
+@pytest.mark.parametrize("M,N,K", [(1024, 256, 64), (1100, 1120, 192), (2100, 544, 576), (9500, 1024, 64), (19000, 512, 128), (40000, 64 * 9, 64)])
+def test_pair_gemm_side_operands_of_whole_numbers(M, N, K, monkeypatch):
+    """The side operand is fetched a block ahead, also across tiles, and twelve warps share eight or four blocks of columns: one tile per
+    pair and several, halves in the last round, ragged edges. Residuals: whole numbers, exact. GELU': against float64, its argument
+    the same bf16 numbers; the product is exact, so that what is left is bf16's rounding and the factor's approximation."""
+    from gcow_b200.ops import kernels as K_
+    monkeypatch.setattr(K_, "_pair_gemm", True)
+    torch.manual_seed(M + N + K)
+    a, b = torch.randint(-1, 2, (M, K), device="cuda").bfloat16(), torch.randint(-1, 2, (N, K), device="cuda").bfloat16()
+    res = torch.randint(-8, 9, (M, N), device="cuda").bfloat16()
+    prod = a.double() @ b.double().t()
+    assert torch.equal(K_.gemm_bf16(a, b, residual=res), (prod + res.double()).bfloat16())
+    x = (torch.randn(M, N, device="cuda") * 2).bfloat16()
+    xd = x.double()
+    factor = 0.5 * (1 + torch.erf(xd / 2 ** 0.5)) + xd * torch.exp(-0.5 * xd * xd) / (2 * 3.141592653589793) ** 0.5
+    for r in (None, res):
+        want = prod * factor + (r.double() if r is not None else 0)
+        got = K_.gemm_bf16(a, b, gelu_grad_of=x, residual=r).double()
+        # the approximation of Phi is good to 1.5e-7, its fp32 evaluation to a few 2^-24; |product| is at most K
+        assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6 * prod.abs() + 1e-30).all())
+    if N % 64 == 0:
+        assert torch.equal(K_.gemm_bf16(a, b.t().contiguous(), b_t=True, residual=res), (prod + res.double()).bfloat16())
+    K_.check_errors()
