@@ -264,12 +264,15 @@ struct StringBuilder {
 // four CTAs fit. 7654 x 7654 at tolerance 1e-3: encoding 153.7 -> 148.4 us, decoding 123.5 -> 115.8; at 1e-1 118.4 -> 112.3 and 72.6 -> 66.2;
 // 2047 x 3001 at 8 bits/value decoding 22.4 -> 21.7. Six (40 registers, 20 to 40 bytes of spills): 161.9, 116.3, 128.1, 63.6. The 1-D
 // coders take 40 to 48 registers by themselves and lose by being told.
+// Where four CTAs per SM hold all tiles at once the unbounded instance stays: more places than that only let some SMs take more tiles than
+// others (1500 x 1500: 1e-3 13.4 and 7.9 us unbounded, 14.4 and 8.7 bounded, 16 bits/value decoding 13.4 and 15.0; 2000 x 2000:
+// 17.7 and 12.2, 17.6 and 11.9).
 constexpr int kCtas2d = 5;
 
 enum TileMode { kVariable, kPacked, kDirect };              // variable rate; fixed rate; fixed rate in whole words
 
-template <int DIM, int PER, TileMode MODE, bool BUDGET>
-__global__ void __launch_bounds__(kTileThreads, DIM == 2 ? kCtas2d : 0)
+template <int DIM, int PER, TileMode MODE, bool BUDGET, int CTAS>
+__global__ void __launch_bounds__(kTileThreads, CTAS)
 encode_tiles_kernel(const float* in, const TileArgs a, uint32_t* __restrict__ out, uint64_t* __restrict__ block_bits,
                     const TileStrings st, const uint16_t* __restrict__ enc_tab, const uint32_t* __restrict__ pair_tab) {
   constexpr int WB = 32 * PER, NB = kTileThreads * PER;
@@ -548,8 +551,8 @@ place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restric
 // Before, with one plane per lookup throughout and a bit-matrix transpose per eight planes, 25.6 M values took: noise at
 // tolerance 1e-6 121 us, with windows 101, with the straight line first 81; at 1e-3 95, 93, 70; at 6 bits/value 117, 97, 84; a
 // random walk at 1e-6 218, 144, 135.
-template <int DIM, int PER, bool BUDGET>
-__global__ void __launch_bounds__(kTileThreads, DIM == 2 ? kCtas2d : 0)
+template <int DIM, int PER, bool BUDGET, int CTAS>
+__global__ void __launch_bounds__(kTileThreads, CTAS)
 decode_tiles_kernel(const uint32_t* in, float* __restrict__ out, const TileArgs a,
                     const uint64_t* block_bits, int shift, const uint16_t* __restrict__ plane_tab, const uint32_t* __restrict__ loop_tab) {
   constexpr int kPer = PER, WB = 32 * PER, NB = kTileThreads * PER;
@@ -772,23 +775,24 @@ int gcow_encode_tiles(const float* in, uint64_t nx, uint64_t ny, const int32_t* 
   TileStrings st = {};
   if (!fixed) st = {(uint32_t*)(sp + ts.strings), (uint32_t*)(sp + ts.tile_bits), (uint32_t*)(sp + ts.warp_at), (uint16_t*)(sp + ts.block_at)};
   int err = 0;
-#define GCOW_ENCODE(D, P, F, B)                                                                                \
+#define GCOW_ENCODE(D, P, F, B, C)                                                                                \
   do {                                                                                                         \
-    const int g = grid_of<&encode_tiles_kernel<D, P, F, B>>(smem, a.tiles, &err);                              \
+    const int g = grid_of<&encode_tiles_kernel<D, P, F, B, C>>(smem, a.tiles, &err);                              \
     if (err) return err;                                                                                       \
-    launch_dependent(encode_tiles_kernel<D, P, F, B>, dim3(g), dim3(kTileThreads), smem, s, in, a, (uint32_t*)out, block_bits, st, \
+    launch_dependent(encode_tiles_kernel<D, P, F, B, C>, dim3(g), dim3(kTileThreads), smem, s, in, a, (uint32_t*)out, block_bits, st, \
                      (const uint16_t*)et, (const uint32_t*)pt);                                                \
   } while (0)
-#define GCOW_ENCODE_MODE(D, P, B)                                     \
+#define GCOW_ENCODE_MODE(D, P, B, C)                                    \
   do {                                                                \
-    if (mode == kVariable) GCOW_ENCODE(D, P, kVariable, B);           \
-    else if (mode == kPacked) GCOW_ENCODE(D, P, kPacked, B);          \
-    else GCOW_ENCODE(D, P, kDirect, B);                               \
+    if (mode == kVariable) GCOW_ENCODE(D, P, kVariable, B, C);           \
+    else if (mode == kPacked) GCOW_ENCODE(D, P, kPacked, B, C);          \
+    else GCOW_ENCODE(D, P, kDirect, B, C);                               \
   } while (0)
-  if (dim == 1 && mode == kVariable && !cuts) { if (per == 4) GCOW_ENCODE(1, 4, kVariable, false); else GCOW_ENCODE(1, 1, kVariable, false); }
-  else if (dim == 1) { if (per == 4) GCOW_ENCODE_MODE(1, 4, true); else GCOW_ENCODE_MODE(1, 1, true); }
-  else if (cuts) GCOW_ENCODE_MODE(2, 1, true);
-  else GCOW_ENCODE_MODE(2, 1, false);
+  if (dim == 1 && mode == kVariable && !cuts) { if (per == 4) GCOW_ENCODE(1, 4, kVariable, false, 0); else GCOW_ENCODE(1, 1, kVariable, false, 0); }
+  else if (dim == 1) { if (per == 4) GCOW_ENCODE_MODE(1, 4, true, 0); else GCOW_ENCODE_MODE(1, 1, true, 0); }
+  else if (a.tiles > 4 * 148) { if (cuts) GCOW_ENCODE_MODE(2, 1, true, kCtas2d); else GCOW_ENCODE_MODE(2, 1, false, kCtas2d); }
+  else if (cuts) GCOW_ENCODE_MODE(2, 1, true, 0);
+  else GCOW_ENCODE_MODE(2, 1, false, 0);
 #undef GCOW_ENCODE_MODE
 #undef GCOW_ENCODE
   if (!fixed) {
@@ -819,17 +823,18 @@ int gcow_decode_tiles(const void* in, float* out, uint64_t nx, uint64_t ny, cons
   a.warp_words = round4(a.slot_words + kReadAhead);
   const uint32_t smem = ((dim == 1 ? (uint32_t)kTileDecTab1 : (uint32_t)kRunTabSize) + kTileWarps * a.warp_words) * 4;
   int err = 0;
-#define GCOW_DECODE(D, P, B)                                                                                      \
+#define GCOW_DECODE(D, P, B, C)                                                                                      \
   do {                                                                                                         \
-    const int g = grid_of<&decode_tiles_kernel<D, P, B>>(smem, a.tiles, &err);                                 \
+    const int g = grid_of<&decode_tiles_kernel<D, P, B, C>>(smem, a.tiles, &err);                                 \
     if (err) return err;                                                                                       \
-    launch_dependent(decode_tiles_kernel<D, P, B>, dim3(g), dim3(kTileThreads), smem, s, (const uint32_t*)in, out, a, block_bits, shift, \
+    launch_dependent(decode_tiles_kernel<D, P, B, C>, dim3(g), dim3(kTileThreads), smem, s, (const uint32_t*)in, out, a, block_bits, shift, \
                      (const uint16_t*)dt, (const uint32_t*)lt);                                                \
   } while (0)
-  if (dim == 1 && per == 4) { if (cuts) GCOW_DECODE(1, 4, true); else GCOW_DECODE(1, 4, false); }
-  else if (dim == 1) { if (cuts) GCOW_DECODE(1, 1, true); else GCOW_DECODE(1, 1, false); }
-  else if (cuts) GCOW_DECODE(2, 1, true);
-  else GCOW_DECODE(2, 1, false);
+  if (dim == 1 && per == 4) { if (cuts) GCOW_DECODE(1, 4, true, 0); else GCOW_DECODE(1, 4, false, 0); }
+  else if (dim == 1) { if (cuts) GCOW_DECODE(1, 1, true, 0); else GCOW_DECODE(1, 1, false, 0); }
+  else if (a.tiles > 4 * 148) { if (cuts) GCOW_DECODE(2, 1, true, kCtas2d); else GCOW_DECODE(2, 1, false, kCtas2d); }
+  else if (cuts) GCOW_DECODE(2, 1, true, 0);
+  else GCOW_DECODE(2, 1, false, 0);
 #undef GCOW_DECODE
   return (int)cudaGetLastError();
 }

@@ -215,6 +215,18 @@ def test_tile_kernels_with_four_blocks_per_lane(blocks, how):
     assert torch.equal(g.decompress(gpu).cpu().view(torch.int32), g.decompress(cpu).view(torch.int32))
 
 
+@pytest.mark.parametrize("tiles", [591, 592, 593])
+@pytest.mark.parametrize("how", [dict(tolerance=1e-3), dict(precision=16), dict(rate=8), dict(rate=9), dict(rate=16)])
+def test_2d_tiles_around_the_line_between_instances(tiles, how):
+    """Four tiles of 256 blocks per SM, one less and one more, against the CPU codec."""
+    ny, nx = 4 * 256 - 1, 4 * tiles - 3
+    y, x = np.mgrid[0:ny, 0:nx].astype(np.float32) * np.float32(1e-3)
+    f = (np.exp(-(x * x + y * y)) + np.random.default_rng(tiles).standard_normal((ny, nx)) * 1e-4).astype(np.float32)
+    cpu, gpu = g.compress(torch.from_numpy(f), **how), g.compress(dev(f), **how)
+    assert gpu.nbytes == cpu.nbytes and torch.equal(gpu.stream.cpu(), cpu.stream)
+    assert torch.equal(g.decompress(gpu).cpu().view(torch.int32), g.decompress(cpu).view(torch.int32))
+
+
 @pytest.mark.parametrize("n", [4 * 300, 4 * 151552 + 7, 4 * 148 * 6 * 4 * 1024 * 2 + 40_001])
 @pytest.mark.parametrize("how", [dict(tolerance=1e-6), dict(tolerance=1e-3), dict(precision=8), dict(precision=16)])
 def test_1d_tiles_of_data_that_changes(n, how):
