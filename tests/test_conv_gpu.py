@@ -298,3 +298,30 @@ def test_resnet50_step_sends_no_convolution_to_cudnn(monkeypatch):
     big = torch.empty(256, 64, 56, 56, device="meta")
     assert K._onebyone_on_igemm(big) and not K._onebyone_on_igemm(x)
     assert all(p.grad is not None and torch.isfinite(p.grad).all() for p in net.parameters())
+
+
+@pytest.mark.parametrize("Co,kh,kw,Ci,off", [(64, 3, 3, 64, 0), (128, 1, 1, 64, 0), (65, 3, 1, 63, 0), (66, 1, 5, 130, 0), (8, 3, 3, 7, 1), (130, 2, 2, 66, 1)])
+def test_turned_filters(Co, kh, kw, Ci, off):
+    """Whole pieces of 64 x 64 channels and cut ones, odd channel counts and odd addresses: [Ci][kh][kw][Co] with the taps reversed."""
+    from gcow_b200 import _native
+    w = torch.randn(Co * kh * kw * Ci + off, device="cuda").bfloat16()[off:]
+    out = torch.full((w.numel() + off + 8,), 7.0, device="cuda").bfloat16()[off:]
+    rc = _native.cuda().gcow_conv_flip_weights(w.data_ptr(), out.data_ptr(), Co, kh, kw, Ci, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    ref = w.view(Co, kh, kw, Ci).flip(1, 2).permute(3, 1, 2, 0).contiguous().view(-1)
+    assert torch.equal(out[:ref.numel()], ref) and bool((out[ref.numel():] == 7).all())
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 2047, 2048, 2049, 70001])
+@pytest.mark.parametrize("off", [0, 1])
+def test_cast_to_bf16(n, off):
+    """Ends inside a thread's eight values and inside a CTA's 2048, unaligned addresses, and every kind of value: the bits of torch's cast."""
+    import ctypes
+    from gcow_b200 import _native
+    x = torch.randn(n + off, device="cuda")[off:]
+    odd = torch.tensor([float("inf"), -float("inf"), 3.4e38, 1e-45, -0.0, 1.00390625, 1.01171875], device="cuda")[:n]
+    x[:odd.numel()] = odd
+    out = torch.full((n + off + 8,), 7.0, device="cuda").bfloat16()[off:]
+    p = ctypes.c_void_p
+    assert _native.cuda().gcow_cast_bf16(p(x.data_ptr()), p(out.data_ptr()), ctypes.c_uint64(n), p(torch.cuda.current_stream().cuda_stream)) == 0
+    assert torch.equal(out[:n].view(torch.int16), x.bfloat16().view(torch.int16)) and bool((out[n:] == 7).all())
