@@ -121,14 +121,14 @@ static int rate_grid(uint64_t blocks, int ctas, bool twice) {
 template <int BITS>
 __global__ void __launch_bounds__(kRateThreads, kEncodeCtas)
 encode_1d_fixed_kernel(const float* in, uint64_t n, void* __restrict__ out, int aligned, int pad_words16,
-                       const uint16_t* __restrict__ tab, const uint32_t* __restrict__ pair_tab) {
+                       const uint16_t* __restrict__ tab, const uint32_t* __restrict__ pair_tab, uint32_t one) {
   constexpr int NW = CodeIO<BITS>::NW;
   __shared__ __align__(16) uint32_t epair[kEncPairTabSize];
   pdl_trigger();
   load_pair_table(epair, pair_tab);                          // under the tail of the stream's last kernel, like the launch itself
   __syncthreads();
   pdl_wait();
-  const LeanTables lt = {tab, nullptr, epair, nullptr};      // the plane-by-plane table is read from global memory (rare path)
+  const LeanTables lt = {tab, nullptr, epair, nullptr, one};      // the plane-by-plane table is read from global memory (rare path)
   const uint64_t blocks = num_blocks_1d(n), stride = (uint64_t)gridDim.x * kRateThreads;
   if (blockIdx.x == 0 && threadIdx.x < pad_words16)          // the stream's last 64-bit word
     reinterpret_cast<uint16_t*>(out)[blocks * (BITS / 16) + threadIdx.x] = 0;
@@ -163,14 +163,14 @@ encode_1d_fixed_kernel(const float* in, uint64_t n, void* __restrict__ out, int 
 template <int BITS>
 __global__ void __launch_bounds__(kRateThreads, BITS == 16 ? 4 : 2)   // 32 bits: 32 registers without being forced; forced, 95 instead of 91 us
 decode_1d_fixed_kernel(const void* in, float* __restrict__ out, uint64_t n, int shift,
-                       int aligned, const uint16_t* __restrict__ tab, const uint32_t* __restrict__ loop_tab) {
+                       int aligned, const uint16_t* __restrict__ tab, const uint32_t* __restrict__ loop_tab, uint32_t one) {
   constexpr int NW = CodeIO<BITS>::NW;
   __shared__ __align__(16) uint32_t dloop[kDecLoopTabSize];
   pdl_trigger();
   load_loop_table(dloop, loop_tab);
   __syncthreads();
   pdl_wait();
-  const LeanTables lt = {nullptr, tab, nullptr, dloop};      // the plane-by-plane table is read from global memory (rare path)
+  const LeanTables lt = {nullptr, tab, nullptr, dloop, one};      // the plane-by-plane table is read from global memory (rare path)
   const uint64_t blocks = num_blocks_1d(n), stride = (uint64_t)gridDim.x * kRateThreads;
   uint64_t b = (uint64_t)blockIdx.x * kRateThreads + threadIdx.x;
   const uint64_t whole = aligned ? n / 4 : 0;
@@ -614,10 +614,10 @@ static int launch_encode_1d(const float* in, uint64_t n, int maxbits, void* out,
   const uint32_t* pt = (const uint32_t*)ptp;
   const int over = (int)(blocks * (uint64_t)maxbits % 64), pw = pad && over ? (64 - over) / 16 : 0;
   switch (maxbits) {
-    case 16: launch_dependent(encode_1d_fixed_kernel<16>, dim3(g), dim3(kRateThreads), 0, s, in, n, out, aligned, pw, et, pt); break;
-    case 32: launch_dependent(encode_1d_fixed_kernel<32>, dim3(g), dim3(kRateThreads), 0, s, in, n, out, aligned, pw, et, pt); break;
-    case 64: launch_dependent(encode_1d_fixed_kernel<64>, dim3(g), dim3(kRateThreads), 0, s, in, n, out, aligned, pw, et, pt); break;
-    case 128: launch_dependent(encode_1d_fixed_kernel<128>, dim3(g), dim3(kRateThreads), 0, s, in, n, out, aligned, pw, et, pt); break;
+    case 16: launch_dependent(encode_1d_fixed_kernel<16>, dim3(g), dim3(kRateThreads), 0, s, in, n, out, aligned, pw, et, pt, 1u); break;
+    case 32: launch_dependent(encode_1d_fixed_kernel<32>, dim3(g), dim3(kRateThreads), 0, s, in, n, out, aligned, pw, et, pt, 1u); break;
+    case 64: launch_dependent(encode_1d_fixed_kernel<64>, dim3(g), dim3(kRateThreads), 0, s, in, n, out, aligned, pw, et, pt, 1u); break;
+    case 128: launch_dependent(encode_1d_fixed_kernel<128>, dim3(g), dim3(kRateThreads), 0, s, in, n, out, aligned, pw, et, pt, 1u); break;
     default: return -1;
   }
   return (int)cudaGetLastError();
@@ -644,10 +644,10 @@ int gcow_decode_1d_fixed(const void* in, float* out, uint64_t n, int maxbits, in
   const uint32_t* lt = (const uint32_t*)ltp;
   const uint16_t* dt = (const uint16_t*)dtp;
   switch (maxbits) {
-    case 16: launch_dependent(decode_1d_fixed_kernel<16>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt); break;
-    case 32: launch_dependent(decode_1d_fixed_kernel<32>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt); break;
-    case 64: launch_dependent(decode_1d_fixed_kernel<64>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt); break;
-    case 128: launch_dependent(decode_1d_fixed_kernel<128>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt); break;
+    case 16: launch_dependent(decode_1d_fixed_kernel<16>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt, 1u); break;
+    case 32: launch_dependent(decode_1d_fixed_kernel<32>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt, 1u); break;
+    case 64: launch_dependent(decode_1d_fixed_kernel<64>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt, 1u); break;
+    case 128: launch_dependent(decode_1d_fixed_kernel<128>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt, 1u); break;
     default: return -1;
   }
   return (int)cudaGetLastError();

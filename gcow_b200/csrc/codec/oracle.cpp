@@ -447,7 +447,7 @@ struct HostLeanTables {
     gcow::build_codec_tables(etab.data(), btab.data());
     gcow::build_pair_table(epair.data());
     gcow::build_dec_loop_table(dloop.data());
-    t.etab = etab.data(); t.dtab = btab.data(); t.epair = epair.data(); t.dloop = dloop.data();
+    t.etab = etab.data(); t.dtab = btab.data(); t.epair = epair.data(); t.dloop = dloop.data(); t.one = 1;
   }
 };
 const gcow::LeanTables& host_lean_tables() {
@@ -610,9 +610,9 @@ int64_t gcow_roundtrip_check(const float* values, uint64_t blocks, int bits, uin
     memcpy(got, f, 16);
     bool ok;
     switch (bits) {
-      case 32: ok = gcow::roundtrip_block_1d_try<32>(got) || gcow::roundtrip_block_1d_cut<32>(got); break;
-      case 64: ok = gcow::roundtrip_block_1d_try<64>(got) || gcow::roundtrip_block_1d_cut<64>(got); break;
-      case 128: ok = gcow::roundtrip_block_1d_try<128>(got) || gcow::roundtrip_block_1d_cut<128>(got); break;
+      case 32: ok = gcow::roundtrip_block_1d_try<32>(got, 1) || gcow::roundtrip_block_1d_cut<32>(got); break;
+      case 64: ok = gcow::roundtrip_block_1d_try<64>(got, 1) || gcow::roundtrip_block_1d_cut<64>(got); break;
+      case 128: ok = gcow::roundtrip_block_1d_try<128>(got, 1) || gcow::roundtrip_block_1d_cut<128>(got); break;
       default: return -1;
     }
     if (ok) bad += memcmp(want, got, 16) != 0; else ++*left;

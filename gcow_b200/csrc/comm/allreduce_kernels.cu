@@ -59,6 +59,7 @@ struct ArArgs {
   int minexp;                 // sparse variant: smallest bit-plane exponent kept (fixed-accuracy rule)
   unsigned long long* wire;   // sparse variant: += codes this rank stored into other ranks' memory, or nullptr
   ArLayout L;
+  uint32_t one = 1;           // see add_fma
 };
 
 // ------------------------------------------------------------- primitives
@@ -230,7 +231,7 @@ allreduce_fused_kernel(const ArArgs a) {
   if (threadIdx.x == 0) s_ok = 1;
   __syncthreads();
   // the plane-by-plane tables serve the rare blocks that leave the fast path and stay in global memory
-  const LeanTables lt = {a.enc_table, a.dec_table, epair, dloop};
+  const LeanTables lt = {a.enc_table, a.dec_table, epair, dloop, a.one};
 
   const int P = a.world, r = a.rank, cta = blockIdx.x, tid = threadIdx.x;
   const ArLayout& L = a.L;
@@ -433,7 +434,7 @@ __global__ void __launch_bounds__(kArThreads, kTripCtas)
 roundtrip_kernel(const ArArgs a) {
   pdl_trigger();
   pdl_wait();
-  const LeanTables lt = {a.enc_table, a.dec_table, a.pair_table, a.loop_table};
+  const LeanTables lt = {a.enc_table, a.dec_table, a.pair_table, a.loop_table, a.one};
   const bool aligned = (((uintptr_t)a.in | (uintptr_t)a.out) & 15) == 0;
   const uint64_t blocks = (a.n + 3) / 4, stride = (uint64_t)gridDim.x * kArThreads, whole = aligned ? a.n / 4 : 0;
   auto rest = [&](float* f) {
@@ -454,7 +455,7 @@ roundtrip_kernel(const ArArgs a) {
       f[i][0] = v.x; f[i][1] = v.y; f[i][2] = v.z; f[i][3] = v.w;
     }
 #pragma unroll
-    for (int i = 0; i < kTripAhead; i++) ok[i] = roundtrip_block_1d_try<BITS>(f[i]);
+    for (int i = 0; i < kTripAhead; i++) ok[i] = roundtrip_block_1d_try<BITS>(f[i], a.one);
 #pragma unroll
     for (int i = 0; i < kTripAhead; i++) {
       if (b + i * stride >= end) break;
@@ -473,7 +474,7 @@ roundtrip_kernel(const ArArgs a) {
   for (b = whole + (uint64_t)blockIdx.x * kArThreads + threadIdx.x; b < blocks; b += stride) {
     float f[4];
     load_block(f, a.in, a.n, b, false);
-    if (!roundtrip_block_1d_try<BITS>(f)) rest(f);
+    if (!roundtrip_block_1d_try<BITS>(f, a.one)) rest(f);
     if (a.postscale != 1.0f) {
 #pragma unroll
       for (int i = 0; i < 4; i++) f[i] *= a.postscale;
@@ -497,7 +498,7 @@ roundtrip_coded_kernel(const ArArgs a) {
   __syncthreads();
   pdl_trigger();
   pdl_wait();
-  const LeanTables lt = {a.enc_table, a.dec_table, epair, dloop};
+  const LeanTables lt = {a.enc_table, a.dec_table, epair, dloop, a.one};
   const bool in_al = ((uintptr_t)a.in & 15) == 0, out_al = ((uintptr_t)a.out & 15) == 0;
   const uint64_t blocks = (a.n + 3) / 4, stride = (uint64_t)gridDim.x * kArThreads;
   auto attempt = [&](float* f) {
@@ -603,7 +604,7 @@ allreduce_sparse_kernel(const ArArgs a) {
     reinterpret_cast<uint4*>(epair)[i] = reinterpret_cast<const uint4*>(a.pair_table)[i];
   if (threadIdx.x == 0) s_ok = 1;
   __syncthreads();
-  const LeanTables lt = {a.enc_table, a.dec_table, epair, dloop};
+  const LeanTables lt = {a.enc_table, a.dec_table, epair, dloop, a.one};
 
   const int P = a.world, r = a.rank, cta = blockIdx.x, tid = threadIdx.x;
   const ArLayout& L = a.L;

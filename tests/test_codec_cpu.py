@@ -3,6 +3,8 @@ oracle vs the header's fast formulation vs the reference build, round trips."""
 import ctypes as C
 import math
 import os
+import re
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -474,6 +476,15 @@ def test_2d_coders_of_the_tiles(par):
     for skip in (0, 5, 31):
         w[1:, 0] |= np.uint32(1 << skip)                        # blocks that are not empty
         assert lib.gcow_tile_2d_check(None, w.ctypes.data, n, w.shape[1], skip, par.as_c()) == 0
+
+
+@pytest.mark.parametrize("header", ["zfp_block.cuh", "tile_coder.cuh"])
+def test_functions_of_a_block_know_nothing_of_the_launch(header):
+    """A block's code is the same from a launch of any shape: the functions shared by host and kernels use no built-in index or size
+    of a launch (the sums on the FMA pipe once took their 1 from blockDim.z)."""
+    src = (Path(__file__).parent.parent / "gcow_b200" / "csrc" / "codec" / header).read_text()
+    code = re.sub(r"//[^\n]*", "", src)
+    assert not re.findall(r"\b(?:blockDim|gridDim|blockIdx|threadIdx|warpSize)\b", code)
 
 
 @pytest.mark.parametrize("bits", [32, 64, 128])
