@@ -428,8 +428,11 @@ allreduce_fused_kernel(const ArArgs a) {
 // are in flight, bound by integer work and memory in about equal parts: us at 6.5 M / 33 M values of noise, both coders' tables in
 // shared memory and two blocks in flight -> now: 8 bits/value 16.9 -> 12.8 / 59.6 -> 51.2, 16 13.9 -> 12.4 / 53.8 -> 51.3; 1 M 7 either way. 6.5 M values
 // near 1: 8 bits 70 -> 37, 16 bits 158 -> 22. Six blocks in flight (64 registers, four CTAs per SM): 15.0 / 57.4.
+// EACH: there is a thread for every block (up to 909 312 values), which then works on that one alone and not on one of four, of which three are
+// empty: 262 144 values at 8 / 16 / 32 bits/value 3.6 -> 2.1 / 1.9 / 1.9 us (through both coders 4.3, 2.4, 2.3), 900 000 values 4.5 -> 2.5 / 2.2 / 2.2,
+// 1000 values 1.8 -> 1.3. With a second block for some, 1 M values, four at a time take 4.3.
 constexpr int kTripAhead = 4, kTripCtas = 6;
-template <int BITS>
+template <int BITS, bool EACH>
 __global__ void __launch_bounds__(kArThreads, kTripCtas)
 roundtrip_kernel(const ArArgs a) {
   pdl_trigger();
@@ -446,6 +449,21 @@ roundtrip_kernel(const ArArgs a) {
       decode_block_1d_rest<BITS>(f, lt, w, 0, 0);
     }
   };
+  auto one = [&](uint64_t b, bool al) {
+    float f[4];
+    load_block(f, a.in, a.n, b, al);
+    if (!roundtrip_block_1d_try<BITS>(f, a.one)) rest(f);
+    if (a.postscale != 1.0f) {
+#pragma unroll
+      for (int i = 0; i < 4; i++) f[i] *= a.postscale;
+    }
+    store_block(f, a.out, a.n, b, al);
+  };
+  const uint64_t first = (uint64_t)blockIdx.x * kArThreads + threadIdx.x;
+  if constexpr (EACH) {
+    if (first < blocks) one(first, aligned);
+    return;
+  }
   auto trip = [&](uint64_t b, uint64_t end) {                 // blocks b, b + stride, .. of those below `end`
     float f[kTripAhead][4];
     bool ok[kTripAhead];
@@ -467,20 +485,10 @@ roundtrip_kernel(const ArArgs a) {
       reinterpret_cast<float4*>(a.out)[b + i * stride] = make_float4(f[i][0], f[i][1], f[i][2], f[i][3]);
     }
   };
-  uint64_t b = (uint64_t)blockIdx.x * kArThreads + threadIdx.x;
+  uint64_t b = first;
   for (; b + (kTripAhead - 1) * stride < whole; b += kTripAhead * stride) trip(b, ~0ull);
   if (b < whole) trip(b, whole);
-  // the array's end, or all of one at an odd address
-  for (b = whole + (uint64_t)blockIdx.x * kArThreads + threadIdx.x; b < blocks; b += stride) {
-    float f[4];
-    load_block(f, a.in, a.n, b, false);
-    if (!roundtrip_block_1d_try<BITS>(f, a.one)) rest(f);
-    if (a.postscale != 1.0f) {
-#pragma unroll
-      for (int i = 0; i < 4; i++) f[i] *= a.postscale;
-    }
-    store_block(f, a.out, a.n, b, false);
-  }
+  for (b = whole + first; b < blocks; b += stride) one(b, false);        // the array's end, or all of one at an odd address
 }
 
 // The same through both coders: at 4 bits/value, where half of all noise is cut before n = 3 and two lookups make the code, and with
@@ -840,11 +848,12 @@ static int launch_roundtrip(const ArArgs& a, int bits, cudaStream_t stream) {
   // four blocks per thread, which the GPU hands out as others end.
   const uint64_t resident = 148 * kTripCtas, few = want < resident ? want : resident, many = (want + kTripAhead - 1) / kTripAhead;
   const uint64_t most = 1u << 30;
+  const bool each = want <= resident;                         // a thread for every block
   const unsigned g = (unsigned)(many > few ? (many < most ? many : most) : few);
   switch (bits) {
-    case 32: launch_dependent(roundtrip_kernel<32>, dim3(g), dim3(kArThreads), 0, stream, a); break;
-    case 64: launch_dependent(roundtrip_kernel<64>, dim3(g), dim3(kArThreads), 0, stream, a); break;
-    case 128: launch_dependent(roundtrip_kernel<128>, dim3(g), dim3(kArThreads), 0, stream, a); break;
+    case 32: launch_dependent(each ? roundtrip_kernel<32, true> : roundtrip_kernel<32, false>, dim3(g), dim3(kArThreads), 0, stream, a); break;
+    case 64: launch_dependent(each ? roundtrip_kernel<64, true> : roundtrip_kernel<64, false>, dim3(g), dim3(kArThreads), 0, stream, a); break;
+    case 128: launch_dependent(each ? roundtrip_kernel<128, true> : roundtrip_kernel<128, false>, dim3(g), dim3(kArThreads), 0, stream, a); break;
     default: return -1;
   }
   return (int)cudaGetLastError();

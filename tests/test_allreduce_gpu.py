@@ -93,7 +93,7 @@ def test_single_rank_round_trip_of_a_long_bucket(rate, blocks):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("rate", [8, 16, 32])
-@pytest.mark.parametrize("blocks", [148 * 6 * 256, 148 * 6 * 256 + 1, 3 * 148 * 6 * 256 + 77, 4 * 148 * 6 * 256 - 1, 4 * 148 * 6 * 256 + 1025])
+@pytest.mark.parametrize("blocks", [1, 255, 257, 65536, 148 * 6 * 256 - 1, 148 * 6 * 256, 148 * 6 * 256 + 1, 3 * 148 * 6 * 256 + 77, 4 * 148 * 6 * 256 - 1, 4 * 148 * 6 * 256 + 1025])
 def test_single_rank_round_trip_without_a_code(rate, blocks):
     """The kernel that makes no code, around the sizes where its grid is full and where a thread has four blocks: data that the bit
     budget cuts in every plane, a tail that is no whole block, and the same at an address that is no multiple of 16."""
