@@ -548,9 +548,11 @@ colsum_partial8_kernel(const bf16* __restrict__ g, float* __restrict__ part, int
 
 // Few rows, one launch: a cluster of eight CTAs takes 64 columns, an eighth of the rows each; 16-byte loads (8 columns per thread, 32
 // row lanes per CTA), folded through shared memory, then CTA r adds up columns 8 r .. 8 r + 7 of all eight in their order. Bound by latency,
-// of which a second launch is the larger part: 2048 x 128 5.1 -> 3.4 us, x 768 5.4 -> 3.5, x 3072 6.1 -> 5.0, 3072 x 1024 5.3 -> 4.4. With more
-// rows a CTA has too many to itself (16384 x 1024 9.6 -> 17.6): those stay with the two kernels above.
-constexpr int kSumCols = 64, kSumCtas = 8, kSumLanes = 32, kSumRows = 4096;
+// of which a second launch is the larger part. The lines (us, the two kernels above -> this one): with more rows a CTA has too many to itself,
+// 4096 x 768 4.9 -> 3.6, 4096 x 3072 8.8 -> 7.4, 5120 x 1024 5.9 -> 5.6, 5120 x 3072 9.7 both, 7168 x 1024 8.9 -> 9.4, 8192 x 1024 8.1 -> 9.5; with more
+// columns the clusters are not all resident, 256 x 6144 4.3 -> 3.6, 2048 x 6144 8.5 -> 6.9, 4096 x 6144 11.2 -> 10.3, but 256 x 8192 4.3 -> 5.7,
+// 2048 x 8192 9.2 -> 11.0, 64 x 30528 3.3 -> 12.8. Within them this one is faster but for a few (3584 x 4096 8.8 -> 9.4).
+constexpr int kSumCols = 64, kSumCtas = 8, kSumLanes = 32, kSumMostRows = 4096, kSumMostCols = 6144;
 __global__ void __cluster_dims__(1, kSumCtas, 1) __launch_bounds__(256)
 colsum_cluster_kernel(const bf16* g, float* __restrict__ out, int rows, int cols, int ld) {
   __shared__ float red[kSumLanes][kSumCols + 4], quarter[4][kSumCols], sum[kSumCols];
@@ -750,7 +752,7 @@ int gcow_softmax_bwd(const void* dp, const void* p, void* ds, int64_t rows, int 
 int gcow_colsum_parts(int rows) { int p = (rows + 127) / 128; return p < 128 ? (p < 1 ? 1 : p) : 128; }
 // Kernels that gcow_colsum launches: one (`part` is not used), or the partial sums and their reduction.
 int gcow_colsum_launches(const void* g, int rows, int cols, int ld) {
-  return rows <= kSumRows && cols % 8 == 0 && ld % 8 == 0 && ((uintptr_t)g & 15) == 0 ? 1 : 2;
+  return rows <= kSumMostRows && cols <= kSumMostCols && cols % 8 == 0 && ld % 8 == 0 && ((uintptr_t)g & 15) == 0 ? 1 : 2;
 }
 int gcow_colsum(const void* g, float* part, float* out, int rows, int cols, int ld, void* stream) {
   if (cols % 2 || ld % 2 || rows <= 0) return -1;

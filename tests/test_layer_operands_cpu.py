@@ -88,3 +88,14 @@ def test_tensors_without_memory_are_refused(ext):
                  lambda: ext.ar_launch(f, f, None, 0, 64, None, *[0] * 6, 1.0, *[0] * 7)):
         with pytest.raises(RuntimeError, match="FakeTensor"):
             call()
+
+
+@pytest.mark.parametrize("rows,cols,ld,at,launches", [(64, 6144, 6144, 0, 1), (64, 6152, 6152, 0, 2), (64, 30528, 30528, 0, 2), (4096, 3072, 3072, 0, 1),
+                                                      (4097, 3072, 3072, 0, 2), (64, 60, 64, 0, 2), (64, 64, 68, 0, 2), (64, 64, 64, 8, 2)])
+def test_column_sums_take_one_launch_where_that_is_faster(ext, rows, cols, ld, at, launches):
+    """Both sides of each line: rows, columns (whose clusters have to be resident together), multiples of eight, alignment."""
+    import ctypes as C
+    from gcow_b200 import _native
+    f = _native.cuda().gcow_colsum_launches
+    f.restype, f.argtypes = C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_int]
+    assert f(4096 + at, rows, cols, ld) == launches

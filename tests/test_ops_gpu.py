@@ -118,9 +118,9 @@ def test_softmax_xent_loss_and_grad():
 
 
 @pytest.mark.parametrize("rows", [1, 7, 255, 257, 4096, 4097])
-@pytest.mark.parametrize("cols,ld", [(8, 8), (64, 64), (72, 80), (1000, 1000)])
+@pytest.mark.parametrize("cols,ld", [(8, 8), (64, 64), (72, 80), (1000, 1000), (6144, 6144), (6152, 6152)])
 def test_colsum_of_whole_numbers(rows, cols, ld):
-    """The one-launch sum (up to 4096 rows) and the two kernels behind it: whole numbers of at most 8, whose sums fp32 holds exactly."""
+    """The one-launch sum (up to 4096 rows of 6144 columns) and the two kernels behind it: whole numbers of at most 8, whose sums fp32 holds exactly."""
     from gcow_b200.ops import kernels as K
     g = torch.randint(-8, 9, (rows, ld), device="cuda").to(torch.bfloat16)[:, :cols]
     assert torch.equal(K.colsum(g), g.double().sum(0).float())
