@@ -513,7 +513,7 @@ int gcow_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN), rest = tiles % max_pairs;
   p.whole = rest && 2 * rest <= max_pairs ? tiles - rest : tiles;
   p.items = p.whole + 2 * (tiles - p.whole);
-  p.order = tile_order(M, N, BM, BN);
+  p.order = tile_order(M, N, K, BM, BN);
   CUtensorMap mh = mb;
   if (p.items > p.whole) {
     rc = b_mn ? make_map_mnfold(&mh, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, 1)
@@ -582,7 +582,7 @@ int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, int M, int N, i
   p.slice_blocks = (kblocks + slices - 1) / slices;
   if ((slices - 1) * p.slice_blocks >= kblocks) return -2;   // an empty slice would leave its part unwritten
   p.whole = p.items = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * slices;
-  p.order = tile_order(M, N, BM, BN);
+  p.order = tile_order(M, N, K, BM, BN);
   p.slice_stride = (size_t)M * N;
   p.halves = p.items <= max_pairs;
   return launch(gemm2_bf16_kernel<true, true, kNothing, false>, Epilogue<kNothing, false>::THREADS, max_pairs, ma, mb, mb, p, stream);

@@ -591,7 +591,7 @@ static int gemm_launch(const void* A, const void* B, void* C, int M, int N, int 
   Params p;
   p.C = C; p.bias = bias; p.residual = residual; p.aux = aux;
   p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.flags = flags; p.error = error;
-  p.order = tile_order(M, N, bm, BN);
+  p.order = tile_order(M, N, K, bm, BN);
   p.batch = batch; p.stride_c = batch > 1 ? stride_c : 0;
   p.a_merged = a_merged; p.b_merged = b_merged;
   p.a_chunks = a_rows / 64; p.b_chunks = b_rows / 64;

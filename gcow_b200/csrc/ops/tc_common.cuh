@@ -256,12 +256,18 @@ __device__ __forceinline__ void warp_load_rows_bf16(uint8_t* stg, int lane, cons
   __syncwarp();
 }
 
-// The order in which a persistent GEMM takes its output tiles: `group` rows of tiles together, column by column. With as many rows of A as of
-// B or more, groups of 4: what is worked on at one time then needs few rows of A and all of a narrow B, and A, where it is larger than the
-// L2, comes from memory once and not once for every column of tiles. With fewer rows of A it is A that is kept, and a column is done from top
-// to bottom. Pair kernel, column by column -> groups of 4: 16384 x 1024 x 4096 plain 119.7 -> 99.7 us, with a residual 122.6 -> 105,
-// x 768 x 3072 69.5 -> 62, 32768 x 1024 x 4096 241 -> 192, 16384 x 4096 x 1024 (A fits) 98.7 -> 96.5; groups of 2, 8 and 16 within 2 % of 4.
-// The other way round, 4096 x 16384 x 4096: 406 column by column, 449 in groups; the one-CTA kernel at 16384 x 30528 x 1024 994 and 1056.
+// The order in which a persistent GEMM takes its output tiles: `group` rows of tiles together, column by column. Groups of 4 need few rows of A
+// and all of B at one time, so that an A larger than the L2 comes from memory once and not once for every column of tiles; column by column
+// it is a column of B and all of A. Groups are taken where A has as many rows as B or more, unless the result's rows are long and the
+// reduction is short (and A has not 2.5 times as many rows): what a group writes, 1024 rows of the result, then displaces B before the next
+// group reads it again.
+// Pair kernel, column by column -> groups, us: 16384 x 1024 x 4096 114.8 -> 101.7, x 2048 x 8192 419 -> 379, x 4096 x 1024 105.6 -> 101.9,
+// x 8192 x 1024 216 -> 213, x 12288 x 1024 319 -> 324, x 16384 x 512 237 -> 243, x 16384 x 1024 418 -> 430, x 16384 x 2048 805 -> 800,
+// x 16384 x 3072 1314 -> 1195; 32768 x 12288 x 1024 657 -> 652, x 16384 x 512 454 -> 475, x 30528 x 768 1225 -> 1268, x 30528 x 1024 1591 -> 1627,
+// x 30528 x 1536 2314 -> 2365, x 30528 x 2048 3404 -> 3175; 65536 x 16384 x 1024 1932 -> 1851. The one-CTA kernel has its lines at the same
+// places (32768 x 30528 x 1024 2090 -> 2214, x 2048 5 % faster). Groups of 2, 8 and 16 are within 2 % of 4. With fewer rows than B it is
+// A that is kept (4096 x 16384 x 4096: 406 column by column, 449 in groups). Under the power limit the same kernel's times drift by 1 to
+// 4 % at the largest of these, and from run to run by more: the two sides of a pair belong together, pairs do not compare.
 struct TileOrder {
   int tiles_m, group, group_tiles;
   __device__ __forceinline__ void at(int tile, int& m, int& n) const {
@@ -270,8 +276,9 @@ struct TileOrder {
     m = first + in - n * high;
   }
 };
-inline TileOrder tile_order(int M, int N, int tile_m, int tile_n) {
-  const int tiles_m = (M + tile_m - 1) / tile_m, group = M >= N && tiles_m > 4 ? 4 : tiles_m;
+inline TileOrder tile_order(int M, int N, int K, int tile_m, int tile_n) {
+  const bool groups = M >= N && (N <= 8192 || K >= 2048 || 2ll * M >= 5ll * N);
+  const int tiles_m = (M + tile_m - 1) / tile_m, group = groups && tiles_m > 4 ? 4 : tiles_m;
   return {tiles_m, group, group * ((N + tile_n - 1) / tile_n)};
 }
 
