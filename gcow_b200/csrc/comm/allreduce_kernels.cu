@@ -491,10 +491,13 @@ roundtrip_kernel(const ArArgs a) {
   for (b = whole + first; b < blocks; b += stride) one(b, false);        // the array's end, or all of one at an odd address
 }
 
-// The same through both coders: at 4 bits/value, where half of all noise is cut before n = 3 and two lookups make the code, and with
-// error feedback. Two blocks per thread are in flight, as in the stand-alone coders.
-template <int BITS>
-__global__ void __launch_bounds__(kArThreads)
+// The same through both coders: with error feedback (FEEDBACK), a block at a time, and without at 4 bits/value, where half of all noise is cut
+// before n = 3 and two lookups make the code; there two blocks per thread are in flight, as in the stand-alone coders.
+// CTAs per SM: left to itself the compiler takes 40 registers for feedback at 4 bits/value (6.5 M values 24.0 us, with the 32 of eight CTAs 19.1), and at
+// 32 bits/value 40, which do not hold its two codes (33 M values 357 us, with up to 64 332).
+constexpr int coded_ctas(int bits) { return bits == 16 ? 8 : bits == 128 ? 4 : 0; }
+template <int BITS, bool FEEDBACK>
+__global__ void __launch_bounds__(kArThreads, coded_ctas(BITS))
 roundtrip_coded_kernel(const ArArgs a) {
   constexpr int kAhead = 2;
   __shared__ __align__(16) uint32_t epair[kEncPairTabSize];
@@ -509,7 +512,7 @@ roundtrip_coded_kernel(const ArArgs a) {
   const LeanTables lt = {a.enc_table, a.dec_table, epair, dloop, a.one};
   const bool in_al = ((uintptr_t)a.in & 15) == 0, out_al = ((uintptr_t)a.out & 15) == 0;
   const uint64_t blocks = (a.n + 3) / 4, stride = (uint64_t)gridDim.x * kArThreads;
-  auto attempt = [&](float* f) {
+  [[maybe_unused]] auto attempt = [&](float* f) {
     uint32_t w[Code<BITS>::NW];
     float d[4];
     if (!encode_block_1d_try<BITS>(f, lt, w, 0) || !decode_block_1d_try<BITS>(d, lt, w, 0, 0)) return false;
@@ -517,7 +520,7 @@ roundtrip_coded_kernel(const ArArgs a) {
     for (int i = 0; i < 4; i++) f[i] = d[i];
     return true;
   };
-  auto rest = [&](float* f) {
+  [[maybe_unused]] auto rest = [&](float* f) {
     if (f[0] == 0 && f[1] == 0 && f[2] == 0 && f[3] == 0) {   // what is left most often; half of all blocks: 19.3 -> 12.5 us
       f[0] = f[1] = f[2] = f[3] = 0;
       return;
@@ -527,31 +530,33 @@ roundtrip_coded_kernel(const ArArgs a) {
     decode_block_1d_lean<BITS>(f, lt, w, 0);
   };
   uint64_t b = (uint64_t)blockIdx.x * kArThreads + threadIdx.x;
-  const uint64_t whole = in_al && out_al && !a.residual ? a.n / 4 : 0;
-  for (; b + (kAhead - 1) * stride < whole; b += kAhead * stride) {
-    float f[kAhead][4];
-    bool ok[kAhead];
+  if constexpr (!FEEDBACK) {
+    const uint64_t whole = in_al && out_al ? a.n / 4 : 0;
+    for (; b + (kAhead - 1) * stride < whole; b += kAhead * stride) {
+      float f[kAhead][4];
+      bool ok[kAhead];
 #pragma unroll
-    for (int i = 0; i < kAhead; i++) {
-      const float4 v = reinterpret_cast<const float4*>(a.in)[b + i * stride];
-      f[i][0] = v.x; f[i][1] = v.y; f[i][2] = v.z; f[i][3] = v.w;
-    }
-#pragma unroll
-    for (int i = 0; i < kAhead; i++) ok[i] = attempt(f[i]);
-#pragma unroll
-    for (int i = 0; i < kAhead; i++) {
-      if (!ok[i]) rest(f[i]);
-      if (a.postscale != 1.0f) {
-#pragma unroll
-        for (int j = 0; j < 4; j++) f[i][j] *= a.postscale;
+      for (int i = 0; i < kAhead; i++) {
+        const float4 v = reinterpret_cast<const float4*>(a.in)[b + i * stride];
+        f[i][0] = v.x; f[i][1] = v.y; f[i][2] = v.z; f[i][3] = v.w;
       }
-      reinterpret_cast<float4*>(a.out)[b + i * stride] = make_float4(f[i][0], f[i][1], f[i][2], f[i][3]);
+#pragma unroll
+      for (int i = 0; i < kAhead; i++) ok[i] = attempt(f[i]);
+#pragma unroll
+      for (int i = 0; i < kAhead; i++) {
+        if (!ok[i]) rest(f[i]);
+        if (a.postscale != 1.0f) {
+#pragma unroll
+          for (int j = 0; j < 4; j++) f[i][j] *= a.postscale;
+        }
+        reinterpret_cast<float4*>(a.out)[b + i * stride] = make_float4(f[i][0], f[i][1], f[i][2], f[i][3]);
+      }
     }
   }
   for (; b < blocks; b += stride) {
     float f[4];
     load_block(f, a.in, a.n, b, in_al);
-    if (a.residual) {
+    if constexpr (FEEDBACK) {
       uint32_t w[Code<BITS>::NW];
       encode_with_feedback<BITS, Code<BITS>::NW>(f, a, b, lt, w);
       decode_block_1d_lean<BITS>(f, lt, w, 0);
@@ -835,11 +840,12 @@ static int launch_roundtrip(const ArArgs& a, int bits, cudaStream_t stream) {
   const uint64_t want = ((a.n + 3) / 4 + kArThreads - 1) / kArThreads;   // a block per thread
   if (a.residual || bits == 16) {
     const int g = (int)(want < 148 * 8 ? want : 148 * 8);
-    switch (bits) {
-      case 16: launch_dependent(roundtrip_coded_kernel<16>, dim3(g), dim3(kArThreads), 0, stream, a); break;
-      case 32: launch_dependent(roundtrip_coded_kernel<32>, dim3(g), dim3(kArThreads), 0, stream, a); break;
-      case 64: launch_dependent(roundtrip_coded_kernel<64>, dim3(g), dim3(kArThreads), 0, stream, a); break;
-      case 128: launch_dependent(roundtrip_coded_kernel<128>, dim3(g), dim3(kArThreads), 0, stream, a); break;
+    if (!a.residual) launch_dependent(roundtrip_coded_kernel<16, false>, dim3(g), dim3(kArThreads), 0, stream, a);
+    else switch (bits) {
+      case 16: launch_dependent(roundtrip_coded_kernel<16, true>, dim3(g), dim3(kArThreads), 0, stream, a); break;
+      case 32: launch_dependent(roundtrip_coded_kernel<32, true>, dim3(g), dim3(kArThreads), 0, stream, a); break;
+      case 64: launch_dependent(roundtrip_coded_kernel<64, true>, dim3(g), dim3(kArThreads), 0, stream, a); break;
+      case 128: launch_dependent(roundtrip_coded_kernel<128, true>, dim3(g), dim3(kArThreads), 0, stream, a); break;
       default: return -1;
     }
     return (int)cudaGetLastError();
