@@ -1105,12 +1105,12 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
 constexpr int kTurn = 64;
 __global__ void __launch_bounds__(256)
 turn_weights_kernel(const __nv_bfloat16* w, __nv_bfloat16* __restrict__ out, int Co, int kh, int kw, int Ci, int phases,
-                    int pairs) {
+                    int pairs, int ci_from, int tap_from) {
   __shared__ __nv_bfloat16 tile[kTurn][kTurn + 2];
   pdl_trigger();
   pdl_wait();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, co0 = blockIdx.x * kTurn, ci0 = blockIdx.y * kTurn;
-  const int tap = blockIdx.z, r = tap / kw, s = tap % kw;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, co0 = blockIdx.x * kTurn, ci0 = ci_from + blockIdx.y * kTurn;
+  const int tap = tap_from + blockIdx.z, r = tap / kw, s = tap % kw;
 #pragma unroll
   for (int k = 0; k < kTurn; k += 8) {
     const int co = co0 + k + warp, ci = ci0 + 2 * lane;
@@ -1147,8 +1147,14 @@ turn_weights_kernel(const __nv_bfloat16* w, __nv_bfloat16* __restrict__ out, int
 // ------------------------------------------------------------------- host side
 static void turn_weights(const void* w, void* out, int Co, int kh, int kw, int Ci, int phases, void* stream) {
   const int pairs = Co % 2 == 0 && Ci % 2 == 0 && (((uintptr_t)w | (uintptr_t)out) & 3) == 0;
-  launch_dependent(turn_weights_kernel, dim3((Co + kTurn - 1) / kTurn, (Ci + kTurn - 1) / kTurn, kh * kw), dim3(256), 0, (cudaStream_t)stream,
-                   (const __nv_bfloat16*)w, (__nv_bfloat16*)out, Co, kh, kw, Ci, phases, pairs);
+  // one launch, unless the filter has more taps or channels than a grid's second and third dimension have CTAs
+  constexpr int kMost = 65535;
+  for (int tap = 0; tap < kh * kw; tap += kMost)
+    for (long long ci = 0; ci < Ci; ci += (long long)kMost * kTurn) {
+      const int tiles = (int)((Ci - ci + kTurn - 1) / kTurn), taps = kh * kw - tap;
+      launch_dependent(turn_weights_kernel, dim3((Co + kTurn - 1) / kTurn, tiles < kMost ? tiles : kMost, taps < kMost ? taps : kMost), dim3(256), 0,
+                       (cudaStream_t)stream, (const __nv_bfloat16*)w, (__nv_bfloat16*)out, Co, kh, kw, Ci, phases, pairs, (int)ci, tap);
+    }
 }
 // bf16 NHWC tensor as {C, W, H, N}; box = 64 channels x bw x bh x bn pixels.
 // chunks > 0: five dimensions {64, W, H, N, C / 64}, the box also spans `chunks` 64-channel groups,

@@ -300,9 +300,11 @@ def test_resnet50_step_sends_no_convolution_to_cudnn(monkeypatch):
     assert all(p.grad is not None and torch.isfinite(p.grad).all() for p in net.parameters())
 
 
-@pytest.mark.parametrize("Co,kh,kw,Ci,off", [(64, 3, 3, 64, 0), (128, 1, 1, 64, 0), (65, 3, 1, 63, 0), (66, 1, 5, 130, 0), (8, 3, 3, 7, 1), (130, 2, 2, 66, 1)])
+@pytest.mark.parametrize("Co,kh,kw,Ci,off", [(64, 3, 3, 64, 0), (128, 1, 1, 64, 0), (65, 3, 1, 63, 0), (66, 1, 5, 130, 0), (8, 3, 3, 7, 1), (130, 2, 2, 66, 1),
+                                               (8, 257, 256, 8, 0), (2, 1, 1, 64 * 65536 + 2, 0)])
 def test_turned_filters(Co, kh, kw, Ci, off):
-    """Whole pieces of 64 x 64 channels and cut ones, odd channel counts and odd addresses: [Ci][kh][kw][Co] with the taps reversed."""
+    """Whole pieces of 64 x 64 channels and cut ones, odd channel counts and odd addresses, more taps and more channels than a grid's
+    second or third dimension has CTAs: [Ci][kh][kw][Co] with the taps reversed."""
     from gcow_b200 import _native
     w = torch.randn(Co * kh * kw * Ci + off, device="cuda").bfloat16()[off:]
     out = torch.full((w.numel() + off + 8,), 7.0, device="cuda").bfloat16()[off:]
