@@ -252,6 +252,7 @@ layernorm_bwd_rows_kernel(const bf16* dy, const bf16* x, const float* gamma, con
     }
   __syncthreads();
   float* const out = part + (size_t)blockIdx.x * 2 * H;
+  const bool wide = ((uintptr_t)part & 15) == 0;       // 2 H is a multiple of 16
   for (int c = threadIdx.x * 4; c < 2 * H; c += T * 4) {
     float4 t = *reinterpret_cast<const float4*>(sm + c);
 #pragma unroll
@@ -259,7 +260,11 @@ layernorm_bwd_rows_kernel(const bf16* dy, const bf16* x, const float* gamma, con
       const float4 u = *reinterpret_cast<const float4*>(sm + (size_t)w * 2 * H + c);
       t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
     }
-    *reinterpret_cast<float4*>(out + c) = t;
+    if (wide) {
+      *reinterpret_cast<float4*>(out + c) = t;
+    } else {
+      out[c] = t.x; out[c + 1] = t.y; out[c + 2] = t.z; out[c + 3] = t.w;
+    }
   }
 }
 

@@ -72,6 +72,27 @@ def test_layernorm_backward_with_a_row_ahead(H, rows):
     assert bool(((b.grad.double() - d.sum(0)).abs() <= off.sum(0) + 1e-6).all())
 
 
+@pytest.mark.parametrize("rows", [5, 1281])
+@pytest.mark.parametrize("H", [24, 1024])
+def test_layernorm_backward_with_partial_sums_at_any_address(H, rows):
+    """The partial sums of gamma's and beta's gradients at an address that is a multiple of 4 alone: the same bits, nothing beside them."""
+    from gcow_b200 import _native
+    lib, S = _native.cuda(), torch.cuda.current_stream().cuda_stream
+    torch.manual_seed(H + rows)
+    dy, x = (torch.randn(rows, H, device="cuda").bfloat16() for _ in range(2))
+    gamma, mean, rstd = torch.randn(H, device="cuda"), x.float().mean(1), 1 / x.float().std(1)
+    parts = lib.gcow_layernorm_bwd_parts(rows)
+    got = []
+    for off in (0, 1):
+        part = torch.full((parts * 2 * H + 16,), 7.0, device="cuda")
+        dx, dgb = torch.empty_like(x), torch.empty(2 * H, device="cuda")
+        assert lib.gcow_layernorm_bwd(dy.data_ptr(), x.data_ptr(), gamma.data_ptr(), mean.data_ptr(), rstd.data_ptr(), dx.data_ptr(),
+                                      part[off:].data_ptr(), dgb.data_ptr(), rows, H, S) == 0
+        assert bool((part[:off] == 7).all()) and bool((part[off + parts * 2 * H:] == 7).all())
+        got.append((dx, dgb))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
 @pytest.mark.parametrize("parts,n,off", [(1, 262144, 0), (3, 262144, 0), (8, 262148, 0), (9, 262144, 0), (3, 262140, 0), (3, 262146, 0),
                                          (4, 300000, 1), (5, 1048579, 0), (70, 300, 0)])
 def test_ordered_sums_of_whole_numbers(parts, n, off):
