@@ -1106,7 +1106,7 @@ constexpr int kTurn = 64;
 __global__ void __launch_bounds__(256)
 turn_weights_kernel(const __nv_bfloat16* w, __nv_bfloat16* __restrict__ out, int Co, int kh, int kw, int Ci, int phases,
                     int pairs, int ci_from, int tap_from) {
-  __shared__ __nv_bfloat16 tile[kTurn][kTurn + 2];
+  __shared__ __align__(4) __nv_bfloat16 tile[kTurn][kTurn + 2];        // written in pairs
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, co0 = blockIdx.x * kTurn, ci0 = ci_from + blockIdx.y * kTurn;
