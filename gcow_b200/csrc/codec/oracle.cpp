@@ -592,6 +592,14 @@ int64_t gcow_lean_accuracy_check(const float* data, uint64_t n, int bits, int mi
   return bad;
 }
 
+// The tile kernels' rows of blocks against a division: how many of the `n` blocks, each below 2^31, get another row of `bx` blocks.
+int64_t gcow_row_division_check(uint32_t bx, const uint32_t* blocks, uint64_t n) {
+  const gcow::RowDivision d = gcow::row_division(bx);
+  int64_t bad = 0;
+  for (uint64_t i = 0; i < n; i++) bad += gcow::row_of_block(blocks[i], d) != blocks[i] / bx;
+  return bad;
+}
+
 // The round trip that makes no code against encode_block / decode_block at `bits` bits per block: the number of blocks
 // whose values differ; *left receives how many of them it leaves to the coders. -1: bits not covered.
 int64_t gcow_roundtrip_check(const float* values, uint64_t blocks, int bits, uint64_t* left) {

@@ -53,7 +53,7 @@ struct TileArgs {
   uint32_t pitch;                 // encode at variable rate: words from one tile's string to the next in scratch
   ZfpParams p;
   int wide;                       // encode, kDirect: blocks of whole 16 bytes at an aligned address
-  uint32_t div_mul, div_shift;    // 2-D: b / bx = umulhi(2 b, div_mul) >> div_shift for blocks below 2^31
+  RowDivision row;                // 2-D: by bx
   int vec;                        // 2-D: values per load that the row pitch and the base address allow (4, 2 or 1); 1-D: 4 or 1
 };
 
@@ -87,10 +87,8 @@ __device__ __forceinline__ void tile_store_1d(const float* f, float* __restrict_
     for (uint64_t i = 0; x0 + i < a.nx; i++) out[x0 + i] = f[i];
   }
 }
-// The row of blocks that block b is in. A division by a number the compiler does not know is some twenty instructions, of about 850 a
-// block takes.
 __device__ __forceinline__ uint64_t block_row(const TileArgs& a, uint64_t b) {
-  return a.blocks <= 0x80000000ull ? (uint64_t)(__umulhi(2u * (uint32_t)b, a.div_mul) >> a.div_shift) : b / a.bx;
+  return a.blocks <= 0x80000000ull ? (uint64_t)row_of_block((uint32_t)b, a.row) : b / a.bx;
 }
 __device__ __forceinline__ void tile_load_2d(float* f, const float* in, const TileArgs& a, uint64_t b) {
   const uint64_t by = block_row(a, b);
@@ -628,12 +626,7 @@ TileArgs tile_args(const void* values, uint64_t nx, uint64_t ny, const ZfpParams
   a.bx = dim == 2 ? (uint32_t)((nx + 3) / 4) : 1;
   a.slot_words = a.warp_words = a.pitch = 0;
   a.wide = 0;
-  // With 2^(s - 1) < bx <= 2^s, mul = floor(2^(31 + s) / bx) + 1 fits 32 bits and b mul / 2^(31 + s) exceeds b / bx by at most b / 2^(31 + s),
-  // which for b < 2^31 is less than 1 / bx: the quotient is exact.
-  uint32_t s = 0;
-  while ((1ull << s) < a.bx) s++;
-  a.div_mul = (uint32_t)((1ull << (31 + s)) / a.bx + 1);
-  a.div_shift = s;
+  a.row = row_division(a.bx);
   const uint64_t per = (uint64_t)kTileThreads * tile_per(blocks, dim);
   a.tiles = (uint32_t)((blocks + per - 1) / per);
   const uintptr_t base = (uintptr_t)values;
