@@ -601,10 +601,12 @@ int64_t gcow_row_division_check(uint32_t bx, const uint32_t* blocks, uint64_t n)
 }
 
 // The round trip that makes no code against encode_block / decode_block at `bits` bits per block: the number of blocks
-// whose values differ; *left receives how many of them it leaves to the coders. -1: bits not covered.
-int64_t gcow_roundtrip_check(const float* values, uint64_t blocks, int bits, uint64_t* left) {
+// whose values differ. *left receives how many blocks the closed form leaves to the one that cuts in the first planes, *coded (or null) how many
+// that one leaves to the coders. -1: bits not covered.
+int64_t gcow_roundtrip_check2(const float* values, uint64_t blocks, int bits, uint64_t* left, uint64_t* coded) {
   const ZfpParams p = {(uint32_t)bits, (uint32_t)bits, 64, -1074};
   int64_t bad = 0;
+  uint64_t open = 0;
   *left = 0;
   for (uint64_t b = 0; b < blocks; b++) {
     const float* f = values + 4 * b;
@@ -616,16 +618,22 @@ int64_t gcow_roundtrip_check(const float* values, uint64_t blocks, int bits, uin
     float want[4], got[4];
     gcow::decode_block<1>(want, p, src, 0);
     memcpy(got, f, 16);
-    bool ok;
+    bool closed, cut = false;
     switch (bits) {
-      case 32: ok = gcow::roundtrip_block_1d_try<32>(got, 1) || gcow::roundtrip_block_1d_cut<32>(got); break;
-      case 64: ok = gcow::roundtrip_block_1d_try<64>(got, 1) || gcow::roundtrip_block_1d_cut<64>(got); break;
-      case 128: ok = gcow::roundtrip_block_1d_try<128>(got, 1) || gcow::roundtrip_block_1d_cut<128>(got); break;
+      case 32: closed = gcow::roundtrip_block_1d_try<32>(got, 1); if (!closed) cut = gcow::roundtrip_block_1d_cut<32>(got); break;
+      case 64: closed = gcow::roundtrip_block_1d_try<64>(got, 1); if (!closed) cut = gcow::roundtrip_block_1d_cut<64>(got); break;
+      case 128: closed = gcow::roundtrip_block_1d_try<128>(got, 1); if (!closed) cut = gcow::roundtrip_block_1d_cut<128>(got); break;
       default: return -1;
     }
-    if (ok) bad += memcmp(want, got, 16) != 0; else ++*left;
+    bad += memcmp(closed || cut ? want : f, got, 16) != 0;     // what both leave has to be as it was
+    *left += !closed;
+    open += !closed && !cut;
   }
+  if (coded) *coded = open;
   return bad;
+}
+int64_t gcow_roundtrip_check(const float* values, uint64_t blocks, int bits, uint64_t* left) {
+  return gcow_roundtrip_check2(values, blocks, bits, left, nullptr);
 }
 
 int gcow_fast1d_compress(const float* data, uint64_t n, const int32_t* params, void* out) {

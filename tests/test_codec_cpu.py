@@ -505,7 +505,8 @@ def test_rows_of_blocks_without_a_division(kind):
 @pytest.mark.parametrize("bits", [32, 64, 128])
 def test_roundtrip_without_a_code(bits):
     """D(E(x)) in closed form against the coders, on data that is cut everywhere (inside a nibble, at the plane that brings the
-    third coefficient in, not at all) and on what it has to leave to them."""
+    third coefficient in, not at all) and on what it has to leave to them. The closed form takes nearly all noise, and what it leaves
+    goes to the cut one unless the block's largest exponent is out of the ordinary, which only the coders take."""
     rng = np.random.default_rng(bits)
     n = 100000
     noise = rng.standard_normal((n, 4))
@@ -513,12 +514,14 @@ def test_roundtrip_without_a_code(bits):
     odd[::3, 1] = np.inf
     odd[1::3, 2] = np.nan
     odd[2::3] *= 1e-40
-    left = C.c_uint64()
+    left, coded = C.c_uint64(), C.c_uint64()
     for name, x in dict(noise=noise * 1e-3, smooth=1 + noise * np.exp2(rng.integers(-28, 3, (n, 1))), uneven=noise * np.exp2(-rng.integers(0, 26, (n, 4))),
                         magnitudes=noise * np.exp2(rng.integers(-140, 120, (n, 1))), sparse=np.where(noise > 1, noise, 0), zeros=noise * 0,
                         same=np.repeat(noise[:, :1], 4, 1), odd=odd).items():
         x = np.ascontiguousarray(x, dtype=np.float32)
-        assert lib.gcow_roundtrip_check(x.ctypes.data, n, bits, C.byref(left)) == 0, name
+        assert lib.gcow_roundtrip_check2(x.ctypes.data, n, bits, C.byref(left), C.byref(coded)) == 0, name
+        exponent = ((x.view(np.uint32) & 0x7fffffff) >> 23).max(1)
+        assert coded.value == int(((exponent < 30) | (exponent > 254)).sum()), name
         assert name != "noise" or left.value < n // 500
 
 
