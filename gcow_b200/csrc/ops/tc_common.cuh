@@ -256,18 +256,19 @@ __device__ __forceinline__ void warp_load_rows_bf16(uint8_t* stg, int lane, cons
   __syncwarp();
 }
 
-// The order in which a persistent GEMM takes its output tiles: `group` rows of tiles together, column by column. Groups of 4 need few rows of A
-// and all of B at one time, so that an A larger than the L2 comes from memory once and not once for every column of tiles; column by column
-// it is a column of B and all of A. Groups are taken where A has as many rows as B or more, unless the result's rows are long and the
-// reduction is short (and A has not 2.5 times as many rows): what a group writes, 1024 rows of the result, then displaces B before the next
-// group reads it again.
-// Pair kernel, column by column -> groups, us: 16384 x 1024 x 4096 114.8 -> 101.7, x 2048 x 8192 419 -> 379, x 4096 x 1024 105.6 -> 101.9,
-// x 8192 x 1024 216 -> 213, x 12288 x 1024 319 -> 324, x 16384 x 512 237 -> 243, x 16384 x 1024 418 -> 430, x 16384 x 2048 805 -> 800,
-// x 16384 x 3072 1314 -> 1195; 32768 x 12288 x 1024 657 -> 652, x 16384 x 512 454 -> 475, x 30528 x 768 1225 -> 1268, x 30528 x 1024 1591 -> 1627,
-// x 30528 x 1536 2314 -> 2365, x 30528 x 2048 3404 -> 3175; 65536 x 16384 x 1024 1932 -> 1851. The one-CTA kernel has its lines at the same
-// places (32768 x 30528 x 1024 2090 -> 2214, x 2048 5 % faster). Groups of 2, 8 and 16 are within 2 % of 4. With fewer rows than B it is
-// A that is kept (4096 x 16384 x 4096: 406 column by column, 449 in groups). Under the power limit the same kernel's times drift by 1 to
-// 4 % at the largest of these, and from run to run by more: the two sides of a pair belong together, pairs do not compare.
+// The order in which a persistent GEMM takes its output tiles: `group` rows of tiles together, column by column. In groups of 4 the L2 has to
+// hold B and the 1024 rows of the result that are being written, and A comes from memory once; column by column it has to hold A and a
+// column of the result, and B comes once. Groups are taken where A has as many rows as B or more, unless only A's share fits: it is below
+// 77 MB, B's above 64 MB and above 5/4 of it. Pair kernel by itself, single launches, column by column -> groups, us (the shares in MB):
+//   groups: 16384 x 4096 x 1024 101.4 -> 98.3 (42, 17), x 8192 x 1024 192.5 -> 188.9 (42, 34), x 12288 x 1024 287.7 -> 289.8 (42, 50),
+//   x 16384 x 2304 917 -> 878 (84, 109), 28672 x 16384 x 1024 737 -> 700 (73, 67), 32768 x 16384 x 512 460.8 -> 455.6 (50, 50),
+//   x 12288 x 768 494.6 -> 459.8 (67, 44), x 30528 x 1024 1653 -> 1604 (84, 125), x 30528 x 2048 3347 -> 3070, 65536 x 16384 x 1024 1997 -> 1635,
+//   30720 x 30528 x 1024 1487 -> 1485 and, back to back, 1768 -> 1722 (79, 125);
+//   columns: 16384 x 16384 x 1024 384 -> 395 (42, 67), x 2048 781 -> 788 (75, 101), 20480 x 16384 x 1024 495.6 -> 497.8 (52, 67),
+//   30720 x 30528 x 768 1142 -> 1174 (63, 109), 32768 x 30528 x 768 1256 -> 1258 (67, 109).
+// Back to back, under the power limit, the differences are the same or larger (16384 x 1024 x 4096 119.7 -> 99.7, 32768 x 30528 x 2048 4310 -> 3546);
+// launches of different kernels in turn show other ones, since each inherits what the one before it left of the power limit. Groups of 2, 8
+// and 16 are within 2 % of 4. With fewer rows than B it is A that is kept (4096 x 16384 x 4096: 406 column by column, 449 in groups).
 struct TileOrder {
   int tiles_m, group, group_tiles;
   __device__ __forceinline__ void at(int tile, int& m, int& n) const {
@@ -277,7 +278,8 @@ struct TileOrder {
   }
 };
 inline TileOrder tile_order(int M, int N, int K, int tile_m, int tile_n) {
-  const bool groups = M >= N && (N <= 8192 || K >= 2048 || 2ll * M >= 5ll * N);
+  const double mb = 1e-6, share_a = mb * M * (2.0 * K + 512), share_b = mb * N * (2.0 * K + 2048);
+  const bool groups = M >= N && !(share_a < 77 && share_b > 64 && share_b > 1.25 * share_a);
   const int tiles_m = (M + tile_m - 1) / tile_m, group = groups && tiles_m > 4 ? 4 : tiles_m;
   return {tiles_m, group, group * ((N + tile_n - 1) / tile_n)};
 }
