@@ -192,14 +192,23 @@ Tensor gemm(const Tensor& a, const Tensor& b, const GemmOpts& o, const On& on) {
   if (aux.defined()) flags |= o.pre_gelu_out.defined() ? kAuxOut : kGeluGrad;
   const int lda = (int)a.stride(0), ldb = (int)b.stride(0), ldc = (int)out.stride(0);
   // A large product goes to CTA pairs: two SMs per 256 x 256 tile have the one-CTA tile's traffic per flop and an overlapped
-  // epilogue as well (16384 x 1024 x 4096 103 us on the one-CTA tile, 99.7 on pairs; x 768 x 3072 91, 62; 32768 x 1024 x 4096 199, 192;
-  // 4096^3 174, 154). From K = 8192 on, both operands stored [rows][K] and nothing but a bias behind them, the one-CTA tile's main
-  // loop is a little faster (8192^3 860, 936; 16384 x 2048 x 8192 400, 405); with B stored [K][N] it is not (8192^3 915, 882).
+  // epilogue as well. Where nothing but a bias follows, the one-CTA tile's main loop is the faster one the longer the reduction, so the pairs
+  // need the finer rounds that they come with (74 tiles at twice the pace instead of 148). `even`: they have none. One-CTA tile, pairs, each
+  // by itself, us, single launches / back to back:
+  //   pairs: 16384 x 1024 x 4096 107.6, 100.4 / 116.3, 116.7; x 768 x 3072 79.9, 63.5 / 80.9, 69.7; 4096^3 106.5, 99.3 / 112.4, 110.2;
+  //   4096 x 8192 x 5120 243.7, 217.1 / 276, 254; 16384 x 2048 x 8192 377, 358 / 435, 433; even, 8192 x 8192 x 4096 363, 367 / 432, 425; with at most
+  //   two rounds, 16384 x 1024 x 6144 152, 144 / 170, 171;
+  //   one-CTA: even, 8192 x 8192 x 5120 451, 469 / 535, 533, x 6144 543, 569 / 639, 652, x 8192 713, 770 / 843, 875; 4096 x 4096 x 8192 194.6, 192.5 / 220, 227;
+  //   a single round, 2048 x 4096 x 4096 57, 57 / 56.0, 57.5.
   // Reductions below 512 (the 1x1 convolutions of a ResNet) stay there too: the output stream bounds them, and the one-CTA
   // kernel's TMA stores are 15 to 30 % faster there.
   const bool can_pair = pair_gemm_enabled() && !o.a_t && !(flags & (kOutF32 | kAccumulate)) && !o.max_ctas && !o.tile_rows;
+  const int64_t tiles = ((M + 255) / 256) * ((N + 255) / 256);
+  const bool even = 2 * ((tiles + 147) / 148) <= (tiles + 73) / 74;
+  const bool one_cta = !(flags & (kGelu | kResidual | kGeluGrad)) && tiles >= 118 && even &&
+                       (K >= 8192 || (K > 4096 && tiles > 296) || (K >= 2048 && tiles <= 148));
   const bool by_rule = K % 64 == 0 && K >= 512 && N % (o.b_t ? 64 : 32) == 0 && M >= 1024 && N >= 256 && lda % 8 == 0 && ldb % 8 == 0 &&
-                       ldc % 8 == 0 && !(K >= 8192 && !o.b_t && ((M + 255) / 256) * ((N + 255) / 256) >= 118 && !(flags & (kGelu | kResidual | kGeluGrad)));
+                       ldc % 8 == 0 && !one_cta;
   if (can_pair && (o.pair < 0 ? by_rule : o.pair > 0)) {
     const int err = gcow_gemm2_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, lda, ldb, ldc, f32(o.bias),
                                     raw(o.residual), raw(aux), flags, on.error, o.b_t, on.stream);
