@@ -48,7 +48,7 @@ def cpu() -> C.CDLL:
             _proto(lib, "gcow_roundtrip_check", C.c_int64, ptr, u64, C.c_int, ptr)
             _proto(lib, "gcow_roundtrip_check2", C.c_int64, ptr, u64, C.c_int, ptr, ptr)
             _proto(lib, "gcow_tile_1d_check", C.c_int64, ptr, u64, ptr, ptr)
-            _proto(lib, "gcow_row_division_check", C.c_int64, C.c_uint32, ptr, u64)
+            _proto(lib, "gcow_divisor_check", C.c_int64, C.c_uint32, ptr, u64)
             _proto(lib, "gcow_tile_2d_check", C.c_int64, ptr, ptr, u64, u32, u32, ptr)
             _proto(lib, "gcow_lean_accuracy_check", C.c_int64, ptr, u64, i32, i32, ptr)
             _proto(lib, "gcow_stage_emax", i32, ptr, i32, i32)

@@ -592,11 +592,12 @@ int64_t gcow_lean_accuracy_check(const float* data, uint64_t n, int bits, int mi
   return bad;
 }
 
-// The tile kernels' rows of blocks against a division: how many of the `n` blocks, each below 2^31, get another row of `bx` blocks.
-int64_t gcow_row_division_check(uint32_t bx, const uint32_t* blocks, uint64_t n) {
-  const gcow::RowDivision d = gcow::row_division(bx);
+// The multiplication that stands for a division by `d` (rows of blocks, tiles of a product): how many of the `n` numbers, each below 2^31,
+// it divides otherwise.
+int64_t gcow_divisor_check(uint32_t d, const uint32_t* numbers, uint64_t n) {
+  const gcow::Divisor by = gcow::divisor(d);
   int64_t bad = 0;
-  for (uint64_t i = 0; i < n; i++) bad += gcow::row_of_block(blocks[i], d) != blocks[i] / bx;
+  for (uint64_t i = 0; i < n; i++) bad += by.under(numbers[i]) != numbers[i] / d;
   return bad;
 }
 

@@ -13,6 +13,7 @@
 //   is the last coefficient the final two bits are not sent (implied).
 // (sw/src/encode.c:279-339 is the serial form: group tests and unary runs.)
 #pragma once
+#include "../divisor.h"
 #include "zfp_block.cuh"
 
 namespace gcow {
@@ -33,24 +34,6 @@ inline uint32_t tile_slot_words(const ZfpParams& p, int dim) {
 inline bool tile_budget_cuts(const ZfpParams& p, int dim) {
   const uint32_t n = dim == 1 ? 4 : 16, prec = p.maxprec < 32 ? p.maxprec : 32;
   return kHeaderBits + (n - 1) + n * prec > p.maxbits;
-}
-
-// The row of a 2-D array's blocks that a block is in, b / bx with bx blocks to a row, for b below 2^31. A division by a number the
-// compiler does not know is some twenty instructions, of about 850 a block takes.
-// With 2^(s - 1) < bx <= 2^s, mul = floor(2^(31 + s) / bx) + 1 fits 32 bits and b mul / 2^(31 + s) exceeds b / bx by at most b / 2^(31 + s),
-// which for b < 2^31 is less than 1 / bx: the quotient is exact.
-struct RowDivision { uint32_t mul, shift; };
-inline RowDivision row_division(uint32_t bx) {
-  uint32_t s = 0;
-  while ((1ull << s) < bx) s++;
-  return {(uint32_t)((1ull << (31 + s)) / bx + 1), s};
-}
-GCOW_HD uint32_t row_of_block(uint32_t b, const RowDivision& d) {
-#if defined(__CUDA_ARCH__)
-  return __umulhi(2u * b, d.mul) >> d.shift;
-#else
-  return (uint32_t)((2ull * b * d.mul) >> 32) >> d.shift;
-#endif
 }
 
 // A rest's ones doubled, a byte at a time: entry v = the byte with every one-bit doubled, its length << 16.

@@ -53,7 +53,7 @@ struct TileArgs {
   uint32_t pitch;                 // encode at variable rate: words from one tile's string to the next in scratch
   ZfpParams p;
   int wide;                       // encode, kDirect: blocks of whole 16 bytes at an aligned address
-  RowDivision row;                // 2-D: by bx
+  Divisor row;                    // 2-D: by bx
   int vec;                        // 2-D: values per load that the row pitch and the base address allow (4, 2 or 1); 1-D: 4 or 1
 };
 
@@ -87,8 +87,10 @@ __device__ __forceinline__ void tile_store_1d(const float* f, float* __restrict_
     for (uint64_t i = 0; x0 + i < a.nx; i++) out[x0 + i] = f[i];
   }
 }
+// The row of blocks that block b is in. A division by a number the compiler does not know is some twenty instructions, of about 850 a
+// block takes.
 __device__ __forceinline__ uint64_t block_row(const TileArgs& a, uint64_t b) {
-  return a.blocks <= 0x80000000ull ? (uint64_t)row_of_block((uint32_t)b, a.row) : b / a.bx;
+  return a.blocks <= 0x80000000ull ? (uint64_t)a.row.under((uint32_t)b) : b / a.bx;
 }
 __device__ __forceinline__ void tile_load_2d(float* f, const float* in, const TileArgs& a, uint64_t b) {
   const uint64_t by = block_row(a, b);
@@ -626,7 +628,7 @@ TileArgs tile_args(const void* values, uint64_t nx, uint64_t ny, const ZfpParams
   a.bx = dim == 2 ? (uint32_t)((nx + 3) / 4) : 1;
   a.slot_words = a.warp_words = a.pitch = 0;
   a.wide = 0;
-  a.row = row_division(a.bx);
+  a.row = divisor(a.bx);
   const uint64_t per = (uint64_t)kTileThreads * tile_per(blocks, dim);
   a.tiles = (uint32_t)((blocks + per - 1) / per);
   const uintptr_t base = (uintptr_t)values;

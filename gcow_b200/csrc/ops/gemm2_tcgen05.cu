@@ -55,19 +55,19 @@ struct Params {
   int slice_blocks;        // stages per slice of the reduction
   int halves;              // weight gradient, an item per pair at most: a slice's two halves have an accumulator each
   size_t slice_stride;     // elements from one slice's result to the next
-  TileOrder order;
+  QuickTileOrder order;
   uint32_t* error;
 };
 
 // An item of work: a tile, or the left or right half of one, over a slice of the reduction.
 struct Item { int m0, n0, kb0, kb1, slice; bool half; };
-template <bool SLICES> __device__ __forceinline__ Item item_at(const Params& p, int i, int tiles, int kblocks) {
+template <bool SLICES, bool DIVIDE> __device__ __forceinline__ Item item_at(const Params& p, int i, int tiles, int kblocks) {
   Item r;
   r.half = i >= p.whole;
   const int j = r.half ? (i - p.whole) >> 1 : i;
   r.slice = SLICES ? j / tiles : 0;
   const int tile = r.half ? p.whole + j : j - r.slice * tiles;
-  p.order.at(tile, r.m0, r.n0);
+  if (DIVIDE) p.order.order.at(tile, r.m0, r.n0); else p.order.at(tile, r.m0, r.n0);
   r.m0 *= BM;
   r.n0 = r.n0 * BN + (r.half ? ((i - p.whole) & 1) * (BN / 2) : 0);
   r.kb0 = SLICES ? r.slice * p.slice_blocks : 0;
@@ -170,7 +170,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       uint32_t s = 0, phase = 0;
       bool ok = true;
       for (int i = pair; i < p.items && ok; i += pairs) {
-        const Item it = item_at<A_MN>(p, i, tiles, kblocks);
+        const Item it = item_at<A_MN, SIDE == kArgument>(p, i, tiles, kblocks);
         const int m0 = it.m0 + (int)rank * 128, n0 = it.n0 + (int)rank * (it.half ? 64 : 128);
         const CUtensorMap* const map_b = it.half ? &tmap_bh : &tmap_b;
         for (int kb = it.kb0; kb < it.kb1; kb++) {
@@ -201,7 +201,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         return __all_sync(0xffffffffu, mbar_wait_abortable(&sm->abort, bar, parity, p.error, code)) != 0;
       };
       for (int i = pair; i < p.items && ok; i += pairs, t++) {
-        const Item it = item_at<A_MN>(p, i, tiles, kblocks);
+        const Item it = item_at<A_MN, SIDE == kArgument>(p, i, tiles, kblocks);
         const uint32_t idesc = idesc0 | ((uint32_t)((it.half ? BN / 2 : BN) >> 3) << 17), chunk_b = it.half ? CHUNK_BYTES / 2 : CHUNK_BYTES;
         const uint32_t acc = t & 1, aphase = (t >> 1) & 1;
         if (!(ok = wait(&sm->tmem_empty[acc], aphase ^ 1, 2))) break;
@@ -270,12 +270,17 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     };
     [[maybe_unused]] auto fetch_first = [&](int i) {
       if (i >= p.items) return;
-      const Item it = item_at<A_MN>(p, i, tiles, kblocks);
+      const Item it = item_at<A_MN, SIDE == kArgument>(p, i, tiles, kblocks);
       fetch(it.m0 + (int)rank * 128 + q * 32, it.n0 + blocks_before(it.half, ew / 4) * 32);
     };
     if (SIDE) fetch_first(pair);
+    // The next item's place is worked out before this one's wait, but for a GELU' factor, whose registers are full. A GELU after
+    // 4096 x 768 x 768 12.7 -> 12.4 us (12.2 before the tiles came in groups), 16384 x 512 x 512 16.4 -> 15.7 (15.5), 8192 x 3072 x 768 38.2 -> 37.3 (37.5).
+    constexpr bool AHEAD = SIDE != kArgument;
+    [[maybe_unused]] Item next = item_at<A_MN, SIDE == kArgument>(p, pair, tiles, kblocks);
     for (int i = pair; i < p.items && ok; i += pairs, t++) {
-      const Item it = item_at<A_MN>(p, i, tiles, kblocks);
+      const Item it = AHEAD ? next : item_at<A_MN, SIDE == kArgument>(p, i, tiles, kblocks);
+      if (AHEAD && i + pairs < p.items) next = item_at<A_MN, SIDE == kArgument>(p, i + pairs, tiles, kblocks);
       const int m0 = it.m0 + (int)rank * 128, n0 = it.n0;
       // this warp's
       const int cols = (it.half ? BN / 2 : BN) / GROUPS, chunks = EVEN ? cols / 32 : blocks_before(it.half, ew / 4 + 1) - blocks_before(it.half, ew / 4),
@@ -513,7 +518,7 @@ int gcow_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN), rest = tiles % max_pairs;
   p.whole = rest && 2 * rest <= max_pairs ? tiles - rest : tiles;
   p.items = p.whole + 2 * (tiles - p.whole);
-  p.order = tile_order(M, N, K, BM, BN);
+  p.order = quick(tile_order(M, N, K, BM, BN));
   CUtensorMap mh = mb;
   if (p.items > p.whole) {
     rc = b_mn ? make_map_mnfold(&mh, B, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, 1)
@@ -582,7 +587,7 @@ int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, int M, int N, i
   p.slice_blocks = (kblocks + slices - 1) / slices;
   if ((slices - 1) * p.slice_blocks >= kblocks) return -2;   // an empty slice would leave its part unwritten
   p.whole = p.items = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * slices;
-  p.order = tile_order(M, N, K, BM, BN);
+  p.order = quick(tile_order(M, N, K, BM, BN));
   p.slice_stride = (size_t)M * N;
   p.halves = p.items <= max_pairs;
   return launch(gemm2_bf16_kernel<true, true, kNothing, false>, Epilogue<kNothing, false>::THREADS, max_pairs, ma, mb, mb, p, stream);

@@ -488,9 +488,9 @@ def test_functions_of_a_block_know_nothing_of_the_launch(header):
 
 
 @pytest.mark.parametrize("kind", ["powers of two and their neighbours", "small", "any"])
-def test_rows_of_blocks_without_a_division(kind):
-    """The 2-D tile kernels' row of a block, a multiplication, against the division: every width at both sides of many multiples and at
-    the last blocks, as far as 2^31 - 1."""
+def test_multiplications_that_stand_for_divisions(kind):
+    """The row of a block in the 2-D tile kernels and the place of a tile in the GEMMs, against the division: every divisor at both sides
+    of many multiples and at the last numbers, as far as 2^31 - 1."""
     rng = np.random.default_rng(len(kind))
     widths = {"powers of two and their neighbours": [w for s in range(32) for w in ((1 << s) - 1, 1 << s, (1 << s) + 1) if 1 <= w <= 1 << 31],
               "small": range(1, 600), "any": np.exp(rng.uniform(np.log(600), np.log(2.0 ** 31), 600)).astype(np.uint64)}[kind]
@@ -499,7 +499,7 @@ def test_rows_of_blocks_without_a_division(kind):
         k = np.unique(np.concatenate([np.arange(1, 40), rng.integers(1, last // w + 2, 200), last // w - np.arange(40)]).astype(np.int64))
         b = np.concatenate([k * w - 1, k * w, rng.integers(0, last + 1, 100), [0, last - 1, last]])
         b = np.ascontiguousarray(b[(b >= 0) & (b <= last)], dtype=np.uint32)
-        assert lib.gcow_row_division_check(w, b.ctypes.data, b.size) == 0, w
+        assert lib.gcow_divisor_check(w, b.ctypes.data, b.size) == 0, w
 
 
 @pytest.mark.parametrize("bits", [32, 64, 128])
