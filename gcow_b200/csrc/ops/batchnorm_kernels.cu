@@ -144,7 +144,9 @@ __global__ void affine_from_stats_kernel(const float* __restrict__ gamma, const 
 }
 
 // ---- normalise: y = x*scale + shift (+ residual when ADD) (ReLU when RELU, its outcome to the mask when RELU is 2)
-template <bool ADD, int RELU>
+// ROWS: how many are unrolled. Behind the statistics, whose last rows the L2 still holds, eight without other operands; where x comes from
+// memory (inference) four: 256 x 64 x 56 x 56 38.0 -> 36.5 us, 32 x 1024 x 14 x 14 7.9 -> 7.3; training with four 256 x 128 x 28 x 28 31.3 -> 32.9.
+template <bool ADD, int RELU, int ROWS = ADD ? 3 : RELU ? 4 : 8>
 __global__ void __launch_bounds__(kThreads, kSweepCtas)
 apply_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residual, bf16* __restrict__ y,
              uint8_t* __restrict__ mask, const float* __restrict__ scale, const float* __restrict__ shift, int64_t R,
@@ -155,7 +157,7 @@ apply_kernel(const bf16* __restrict__ x, const bf16* __restrict__ residual, bf16
   float sc[8], sh[8];
 #pragma unroll
   for (int i = 0; i < 8; i++) { sc[i] = scale[g * 8 + i]; sh[i] = shift[g * 8 + i]; }
-#pragma unroll (ADD ? 3 : RELU ? 4 : 8)
+#pragma unroll ROWS
   for (int64_t r = (int64_t)blockIdx.x * rstep + r0; r < R; r += (int64_t)gridDim.x * rstep) {
     const int64_t off = r * C + g * 8;
     float v[8];
@@ -325,7 +327,8 @@ int gcow_bn_fwd_eval(const void* x, const void* residual, void* y, const float* 
   if (!shape_ok(C) || R <= 0) return -1;
   cudaStream_t s = (cudaStream_t)stream;
   affine_from_stats_kernel<<<(C + 127) / 128, 128, 0, s>>>(gamma, beta, run_mean, run_var, eps, C, scratch, scratch + C);
-  apply_for(residual, nullptr, relu)<<<grid_for(R, C), kThreads, 0, s>>>((const bf16*)x, (const bf16*)residual, (bf16*)y, nullptr, scratch, scratch + C, R, C);
+  const auto kernel = residual || relu ? apply_for(residual, nullptr, relu) : apply_kernel<false, 0, 4>;
+  kernel<<<grid_for(R, C), kThreads, 0, s>>>((const bf16*)x, (const bf16*)residual, (bf16*)y, nullptr, scratch, scratch + C, R, C);
   return (int)cudaGetLastError();
 }
 

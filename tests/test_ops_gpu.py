@@ -555,6 +555,11 @@ def test_batchnorm_every_form_of_the_sweeps(N, C, H, W, res, relu, fork):
     assert ((bn.weight.grad.double() - dg).abs() <= 1e-5 * (g * xh).abs().sum((0, 2, 3)) + 1e-5).all()
     dx = ga * rstd * (g - col(db) / R - xh * col(dg) / R)
     assert ((x.grad.double() - dx).abs() <= 2**-8 * (dx.abs() + ga * rstd * g.abs()) + 1e-4 * ga * rstd).all()
+    if not fork:                                             # inference: the same sweep, without a mask
+        bn.eval()
+        z = (xd - col(bn.running_mean)) / (col(bn.running_var) + bn.eps).sqrt() * ga + col(bn.bias.detach()) + (r0.double() if res else 0)
+        want = z.clamp(min=0) if relu else z
+        assert ((bn(x0, residual=r0 if res else None, relu=relu).double() - want).abs() <= 2**-8 * want.abs() + 1e-4).all()
 
 
 def test_batchnorm_counts_training_steps_lazily():
