@@ -429,9 +429,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
 }
 
 // delta[b][h][s] = sum_d dO[b][s][h][d] * O[b][s][h][d]; eight lanes per row, so that a warp reads whole lines, and kDeltaRows rows to a
-// lane, all of whose loads are under way before the first sum. Bound by memory: 262 144 rows (67 MB, 10 us) 15.5 us with one row to a lane
-// and 64-bit divisions for its place, now 12.7.
-constexpr int kDeltaRows = 4;
+// lane, all of whose loads are under way before the first sum. Bound by memory. With one row and 64-bit divisions for its place, two rows, four
+// rows to a lane, the whole backward takes: 32 x 512 x 16 heads 240.4, 238.2, 238.4 us; 8 x 512 x 16 74.0, 73.3, 75.5; 2 x 512 x 16 30.0, 30.3, 31.0;
+// 1 x 128 x 2 9.8, 9.6, 10.0: with four, few rows are too few CTAs.
+constexpr int kDeltaRows = 2;
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* o, const __nv_bfloat16* go, float* __restrict__ delta, uint32_t rows, uint32_t S, uint32_t H) {
   pdl_trigger();
