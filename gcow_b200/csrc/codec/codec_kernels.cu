@@ -163,14 +163,14 @@ encode_1d_fixed_kernel(const float* in, uint64_t n, void* __restrict__ out, int 
 template <int BITS>
 __global__ void __launch_bounds__(kRateThreads, BITS == 16 ? 4 : 2)   // 32 bits: 32 registers without being forced; forced, 95 instead of 91 us
 decode_1d_fixed_kernel(const void* in, float* __restrict__ out, uint64_t n, int shift,
-                       int aligned, const uint16_t* __restrict__ tab, const uint32_t* __restrict__ loop_tab, uint32_t one) {
+                       int aligned, const uint16_t* __restrict__ tab, const uint32_t* __restrict__ loop_tab) {
   constexpr int NW = CodeIO<BITS>::NW;
   __shared__ __align__(16) uint32_t dloop[kDecLoopTabSize];
   pdl_trigger();
   load_loop_table(dloop, loop_tab);
   __syncthreads();
   pdl_wait();
-  const LeanTables lt = {nullptr, tab, nullptr, dloop, one};      // the plane-by-plane table is read from global memory (rare path)
+  const LeanTables lt = {nullptr, tab, nullptr, dloop, 0};      // the plane-by-plane table is read from global memory (rare path)
   const uint64_t blocks = num_blocks_1d(n), stride = (uint64_t)gridDim.x * kRateThreads;
   uint64_t b = (uint64_t)blockIdx.x * kRateThreads + threadIdx.x;
   const uint64_t whole = aligned ? n / 4 : 0;
@@ -644,10 +644,10 @@ int gcow_decode_1d_fixed(const void* in, float* out, uint64_t n, int maxbits, in
   const uint32_t* lt = (const uint32_t*)ltp;
   const uint16_t* dt = (const uint16_t*)dtp;
   switch (maxbits) {
-    case 16: launch_dependent(decode_1d_fixed_kernel<16>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt, 1u); break;
-    case 32: launch_dependent(decode_1d_fixed_kernel<32>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt, 1u); break;
-    case 64: launch_dependent(decode_1d_fixed_kernel<64>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt, 1u); break;
-    case 128: launch_dependent(decode_1d_fixed_kernel<128>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt, 1u); break;
+    case 16: launch_dependent(decode_1d_fixed_kernel<16>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt); break;
+    case 32: launch_dependent(decode_1d_fixed_kernel<32>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt); break;
+    case 64: launch_dependent(decode_1d_fixed_kernel<64>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt); break;
+    case 128: launch_dependent(decode_1d_fixed_kernel<128>, dim3(g), dim3(kRateThreads), 0, s, in, out, n, shift, aligned, dt, lt); break;
     default: return -1;
   }
   return (int)cudaGetLastError();

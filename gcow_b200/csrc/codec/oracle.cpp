@@ -621,9 +621,9 @@ int64_t gcow_roundtrip_check2(const float* values, uint64_t blocks, int bits, ui
     memcpy(got, f, 16);
     bool closed, cut = false;
     switch (bits) {
-      case 32: closed = gcow::roundtrip_block_1d_try<32>(got, 1); if (!closed) cut = gcow::roundtrip_block_1d_cut<32>(got); break;
-      case 64: closed = gcow::roundtrip_block_1d_try<64>(got, 1); if (!closed) cut = gcow::roundtrip_block_1d_cut<64>(got); break;
-      case 128: closed = gcow::roundtrip_block_1d_try<128>(got, 1); if (!closed) cut = gcow::roundtrip_block_1d_cut<128>(got); break;
+      case 32: closed = gcow::roundtrip_block_1d_try<32>(got); if (!closed) cut = gcow::roundtrip_block_1d_cut<32>(got); break;
+      case 64: closed = gcow::roundtrip_block_1d_try<64>(got); if (!closed) cut = gcow::roundtrip_block_1d_cut<64>(got); break;
+      case 128: closed = gcow::roundtrip_block_1d_try<128>(got); if (!closed) cut = gcow::roundtrip_block_1d_cut<128>(got); break;
       default: return -1;
     }
     bad += memcmp(closed || cut ? want : f, got, 16) != 0;     // what both leave has to be as it was

@@ -151,12 +151,25 @@ GCOW_HD void inv_lift(int32_t& x_, int32_t& y_, int32_t& z_, int32_t& w_) {
   x_ = (int32_t)x; y_ = (int32_t)y; z_ = (int32_t)z; w_ = (int32_t)w;
 }
 
-// a + b on the FMA pipe: a times `one`, a 1 that the compiler cannot know, which a kernel takes from its arguments. The fixed-rate straight
-// lines below fill the integer ALU (half the issue rate) twice as full as that pipe; with their sums moved there 67 M values at 8 bits/value
-// take 68.7 instead of 70.3 us (encoding) and 81.0 instead of 83.1. The tile coders, which have other work for it, get slower by 1 to 3 %.
-// (A 1 in constant memory instead of among the arguments: 0.2 to 0.4 us more per launch, 1000 values encoded 1.1 -> 1.5 us.)
+// The inverse lift of the straight lines below, which keeps a sum and a difference where the one above shifts: (y, w) becomes
+// (y + w, 2 w - (y + w)).
+GCOW_HD void inv_lift_sums(int32_t& x_, int32_t& y_, int32_t& z_, int32_t& w_) {
+  uint32_t x = (uint32_t)x_, y = (uint32_t)y_, z = (uint32_t)z_, w = (uint32_t)w_, t;
+  y += asr1(w); w -= asr1(y);
+  t = w; w -= y; y += t;
+  t = x; x -= z; z += t;
+  t = z; z -= y; y += t;
+  t = x; x -= w; w += t;
+  x_ = (int32_t)x; y_ = (int32_t)y; z_ = (int32_t)z; w_ = (int32_t)w;
+}
+
+// a + b on the FMA pipe: a times `one`, a 1 that the compiler cannot know, which a kernel takes from its arguments. The fixed-rate encoder's
+// straight line fills the integer ALU (half the issue rate) twice as full as that pipe; with its sums moved there 67 M values at 8 bits/value
+// take 67.9 instead of 68.9 us. The decoder and the one-rank round trip gain nothing (79.9 with, 78.8 without; 33 M values 48.9, 48.8), the
+// tile coders, which have other work for that pipe, lose 1 to 3 %. (A 1 in constant memory instead of among the arguments: 0.2 to 0.4 us more
+// per launch, 1000 values encoded 1.1 -> 1.5 us.)
 GCOW_HD uint32_t add_fma(uint32_t a, uint32_t b, uint32_t one) { return a * one + b; }
-// The two lifts and the negabinary maps with it.
+// The forward lift and the negabinary map with it.
 GCOW_HD void fwd_lift_fma(int32_t& x_, int32_t& y_, int32_t& z_, int32_t& w_, uint32_t one) {
   uint32_t x = (uint32_t)x_, y = (uint32_t)y_, z = (uint32_t)z_, w = (uint32_t)w_;
   x = asr1(add_fma(x, w, one)); w -= x;
@@ -164,15 +177,6 @@ GCOW_HD void fwd_lift_fma(int32_t& x_, int32_t& y_, int32_t& z_, int32_t& w_, ui
   x = asr1(add_fma(x, z, one)); z -= x;
   w = asr1(add_fma(w, y, one)); y -= w;
   w = add_fma(w, asr1(y), one); y -= asr1(w);
-  x_ = (int32_t)x; y_ = (int32_t)y; z_ = (int32_t)z; w_ = (int32_t)w;
-}
-GCOW_HD void inv_lift_fma(int32_t& x_, int32_t& y_, int32_t& z_, int32_t& w_, uint32_t one) {
-  uint32_t x = (uint32_t)x_, y = (uint32_t)y_, z = (uint32_t)z_, w = (uint32_t)w_, t;
-  y = add_fma(y, asr1(w), one); w -= asr1(y);
-  t = w; w -= y; y = add_fma(y, t, one);                     // (y, w) = (y + w, 2 w - (y + w)), and so on
-  t = x; x -= z; z = add_fma(z, t, one);
-  t = z; z -= y; y = add_fma(y, t, one);
-  t = x; x -= w; w = add_fma(w, t, one);
   x_ = (int32_t)x; y_ = (int32_t)y; z_ = (int32_t)z; w_ = (int32_t)w;
 }
 
@@ -205,7 +209,6 @@ template <> struct Xform<2> {
 GCOW_HD uint32_t int2nb(int32_t x) { return ((uint32_t)x + kNbMask) ^ kNbMask; }
 GCOW_HD int32_t nb2int(uint32_t u) { return (int32_t)((u ^ kNbMask) - kNbMask); }
 GCOW_HD uint32_t int2nb_fma(int32_t x, uint32_t one) { return add_fma((uint32_t)x, kNbMask, one) ^ kNbMask; }
-GCOW_HD int32_t nb2int_fma(uint32_t u, uint32_t one) { return (int32_t)add_fma(u ^ kNbMask, 0u - kNbMask, one); }
 
 template <int DIM>
 GCOW_HD void fwd_reorder(uint32_t* u, const int32_t* q) {
@@ -1027,7 +1030,7 @@ struct LeanTables {
   const uint16_t* dtab;    // kDecBudgetTabSize: budget-aware, one plane per lookup (definition path, likewise)
   const uint32_t* epair;   // kEncPairTabSize: two planes per lookup
   const uint32_t* dloop;   // kDecLoopTabSize, 8-byte aligned: decoder windows, nibble pairs, tiny blocks
-  uint32_t one;            // 1, from the kernel's arguments (add_fma)
+  uint32_t one;            // encoder: 1, from the kernel's arguments (add_fma)
 };
 
 // The straight-line part of the encoder: true when w holds the block's code. Without branches up to 64 bits, so that a
@@ -1194,15 +1197,13 @@ GCOW_HD bool decode_block_1d_try(float* f, const LeanTables& t, const uint32_t (
   int32_t q[4];
   const int ef = (int)e8 - 30 - shift;                         // 2^(emax - 30 - shift): a normal float unless the block is tiny
   float scale;
-  if (BITS == 16) {                                            // bound by memory: the plain forms
 #pragma unroll
-    for (int i = 0; i < 4; i++) q[i] = nb2int(u[i] & planemask);
+  for (int i = 0; i < 4; i++) q[i] = nb2int(u[i] & planemask);
+  if (BITS == 16) {                                            // bound by memory
     inv_lift(q[0], q[1], q[2], q[3]);
     scale = (ef >= 1 && ef <= 254) ? bits_f32((uint32_t)ef << 23) : pow2f(ef - 127);
   } else {
-#pragma unroll
-    for (int i = 0; i < 4; i++) q[i] = nb2int_fma(u[i] & planemask, t.one);
-    inv_lift_fma(q[0], q[1], q[2], q[3], t.one);
+    inv_lift_sums(q[0], q[1], q[2], q[3]);
     scale = bits_f32(ef >= 1 ? (uint32_t)ef << 23 : shl_sat(1u, (uint32_t)(ef + 22)));
     whole = whole && shift >= -29;                             // else it may be infinite
   }
@@ -1232,7 +1233,7 @@ GCOW_HD void decode_block_1d_lean(float* f, const LeanTables& t, const uint32_t 
 // False (f is not written) where the cut falls into plane top_2 or above it (roundtrip_block_1d_cut), or the exponent or a member is out
 // of the ordinary.
 template <int BITS>
-GCOW_HD bool roundtrip_block_1d_try(float* f, uint32_t one) {
+GCOW_HD bool roundtrip_block_1d_try(float* f) {
   constexpr int P = BITS - (int)kHeaderBits;
   bool ordinary;
   const uint32_t mb = block_max_bits<4>(f, 30, ordinary);
@@ -1246,10 +1247,10 @@ GCOW_HD bool roundtrip_block_1d_try(float* f, uint32_t one) {
   if (!ordinary) return false;                                // out of range for this conversion
   q[0] = (int32_t)p0; q[1] = (int32_t)p1; q[2] = (int32_t)p2; q[3] = (int32_t)p3;
 #endif
-  fwd_lift_fma(q[0], q[1], q[2], q[3], one);
+  fwd_lift(q[0], q[1], q[2], q[3]);
   uint32_t u[4];
 #pragma unroll
-  for (int i = 0; i < 4; i++) u[i] = int2nb_fma(q[i], one);
+  for (int i = 0; i < 4; i++) u[i] = int2nb(q[i]);
   const uint32_t m2 = u[2] | u[3], m1 = m2 | u[1], m0 = m1 | u[0];
   const bool low = m2 != 0;                                   // top_2 exists
 #if defined(__CUDA_ARCH__)
@@ -1265,8 +1266,8 @@ GCOW_HD bool roundtrip_block_1d_try(float* f, uint32_t one) {
   const bool ok = ordinary && low && k <= 31 - l2;
   const uint32_t whole = shl_sat(0xffffffffu, (uint32_t)k), more = k > 0 ? whole | shl_sat(1u, (uint32_t)(k - 1)) : whole;
 #pragma unroll
-  for (int i = 0; i < 4; i++) q[i] = nb2int_fma(u[i] & (i < 3 && i < a ? more : whole), one);
-  inv_lift_fma(q[0], q[1], q[2], q[3], one);
+  for (int i = 0; i < 4; i++) q[i] = nb2int(u[i] & (i < 3 && i < a ? more : whole));
+  inv_lift_sums(q[0], q[1], q[2], q[3]);
   if (!ok) return false;
   const float back = bits_f32((ex - 29u) << 23);              // 2^(emax - 30)
 #pragma unroll

@@ -452,7 +452,7 @@ roundtrip_kernel(const ArArgs a) {
   auto one = [&](uint64_t b, bool al) {
     float f[4];
     load_block(f, a.in, a.n, b, al);
-    if (!roundtrip_block_1d_try<BITS>(f, a.one)) rest(f);
+    if (!roundtrip_block_1d_try<BITS>(f)) rest(f);
     if (a.postscale != 1.0f) {
 #pragma unroll
       for (int i = 0; i < 4; i++) f[i] *= a.postscale;
@@ -473,7 +473,7 @@ roundtrip_kernel(const ArArgs a) {
       f[i][0] = v.x; f[i][1] = v.y; f[i][2] = v.z; f[i][3] = v.w;
     }
 #pragma unroll
-    for (int i = 0; i < kTripAhead; i++) ok[i] = roundtrip_block_1d_try<BITS>(f[i], a.one);
+    for (int i = 0; i < kTripAhead; i++) ok[i] = roundtrip_block_1d_try<BITS>(f[i]);
 #pragma unroll
     for (int i = 0; i < kTripAhead; i++) {
       if (b + i * stride >= end) break;
