@@ -105,12 +105,14 @@ template <> struct CodeIO<128> {
 // blocks that leave the straight line, and the array's end, are seen to one by one. CTAs of 512 threads: half as many
 // copies of the tables as with 256, which is what a vector of a million values feels.
 constexpr int kRateThreads = 512, kAhead = 2;
-// CTAs per SM, as the registers allow: encoding 67 M values at 8 bits/value takes 80 us with two, 76 us with three.
+// CTAs per SM, as the registers allow: with two, encoding 67 M values at 8 bits/value takes 77.6 instead of 67.9 us, 6.55 M at 16 17.7 instead
+// of 13.9.
 constexpr int kEncodeCtas = 3;
 constexpr int decode_ctas(int bits) { return bits <= 32 ? 4 : 3; }
 // Grid: the resident CTAs; twice as many where a thread would have kLong blocks or more, since an SM whose CTAs are through early is
-// then given others. Once, twice: 67 M values at 8 bits/value 68.7, 68.2 us (encoding), 81.0, 80.0; 16 bits/value 104.1, 101.8 and 112.0, 108.2;
-// at 4 bits/value decoding is slower for it (53.1, 54.1), and so is most of 17 M values (19.7, 20.9 encoding at 8 bits/value).
+// then given others. Once, twice, us: encoding at 16 bits/value 26 M values (29 blocks a thread) 42.9 both, 32 M (35) 52.2, 51.5, 67 M 104.0, 101.5; at 8
+// 26 M 28.3, 29.0, 32 M 34.5, 34.9, 67 M 68.1, 67.8, 134 M 131.8, 129.9. Decoding at 16 bits/value 22 M 41.0, 41.4, 26 M 46.5 both, 32 M 57.1, 56.1, 67 M 111.9,
+// 109.2; at 8 36 M (30) 45.6 both, 45 M (37) 56.0, 55.8, 134 M 154, 152; at 4 it gains nothing (134 M 104.9, 104.8).
 constexpr uint64_t kLong = 32;
 static int rate_grid(uint64_t blocks, int ctas, bool twice) {
   const uint64_t resident = 148ull * ctas, want = (blocks + kRateThreads - 1) / kRateThreads;
@@ -161,7 +163,7 @@ encode_1d_fixed_kernel(const float* in, uint64_t n, void* __restrict__ out, int 
 }
 
 template <int BITS>
-__global__ void __launch_bounds__(kRateThreads, BITS == 16 ? 4 : 2)   // 32 bits: 32 registers without being forced; forced, 95 instead of 91 us
+__global__ void __launch_bounds__(kRateThreads, BITS == 16 ? 4 : 2)   // 32 bits: 32 registers without being forced; forced, 82.3 instead of 79.9 us
 decode_1d_fixed_kernel(const void* in, float* __restrict__ out, uint64_t n, int shift,
                        int aligned, const uint16_t* __restrict__ tab, const uint32_t* __restrict__ loop_tab) {
   constexpr int NW = CodeIO<BITS>::NW;

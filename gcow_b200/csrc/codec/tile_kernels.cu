@@ -266,7 +266,8 @@ struct StringBuilder {
 // coders take 40 to 48 registers by themselves and lose by being told.
 // Where four CTAs per SM hold all tiles at once the unbounded instance stays: more places than that only let some SMs take more tiles than
 // others (1500 x 1500: 1e-3 13.4 and 7.9 us unbounded, 14.4 and 8.7 bounded, 16 bits/value decoding 13.4 and 15.0; 2000 x 2000:
-// 17.7 and 12.2, 17.6 and 11.9).
+// 17.7 and 12.2, 17.6 and 11.9; just above the line, 1600 x 1600, decoding at 4 bits/value is slower bounded, 11.3 and 12.0, at 16 bits/value, 1e-3 and 1e-1
+// faster, 15.0 and 14.4, 8.3 and 7.8, 4.9 and 4.0).
 constexpr int kCtas2d = 5;
 
 enum TileMode { kVariable, kPacked, kDirect };              // variable rate; fixed rate; fixed rate in whole words

@@ -165,7 +165,7 @@ GCOW_HD void inv_lift_sums(int32_t& x_, int32_t& y_, int32_t& z_, int32_t& w_) {
 
 // a + b on the FMA pipe: a times `one`, a 1 that the compiler cannot know, which a kernel takes from its arguments. The fixed-rate encoder's
 // straight line fills the integer ALU (half the issue rate) twice as full as that pipe; with its sums moved there 67 M values at 8 bits/value
-// take 67.9 instead of 68.9 us. The decoder and the one-rank round trip gain nothing (79.9 with, 78.8 without; 33 M values 48.9, 48.8), the
+// take 67.9 instead of 68.9 us. The decoder and the one-rank round trip gain nothing (80.3 with, 79.2 without; 33 M values 48.9 both), the
 // tile coders, which have other work for that pipe, lose 1 to 3 %. (A 1 in constant memory instead of among the arguments: 0.2 to 0.4 us more
 // per launch, 1000 values encoded 1.1 -> 1.5 us.)
 GCOW_HD uint32_t add_fma(uint32_t a, uint32_t b, uint32_t one) { return a * one + b; }
@@ -852,13 +852,10 @@ inline void build_codec_tables(uint16_t* etab, uint16_t* dtab_budget) {
 //    per lookup. Both tables deliver coefficient i's bits in byte i, so neither part
 //    needs a transpose either.
 //
-// Both are bound by the integer ALU (half the issue rate), so sums of shifted fields are
-// multiplications by powers of two, which run on the FMA pipe, and so do half of the lifts' sums. Measured at 67 M values
-// and 8 bits/value: encoding 104.7 -> 76.3 us (155 -> 101 instructions per warp of
-// blocks), decoding 135.8 -> 90.9 us (212 -> 132). Instructions are what bounds both (input that is in the L2 takes the same time per
-// value, and so does input fetched ahead into shared memory): with a NaN seen in the maximum instead of a sum, the windows'
-// counts in one register, checked in one operation, and sums on the FMA pipe 73.9 -> 67.7 and 88.4 -> 79.5; at 16 bits/value 106.4 ->
-// 101.8 and 118.1 -> 109.2, 32 bits/value 200 -> 190 and 222 -> 207.
+// Both are bound by the integer ALU (half the issue rate), so sums of shifted fields are multiplications by powers of two, which run on
+// the FMA pipe, and so do half of the encoder's lift's sums. A NaN is seen in the maximum, and the decoder keeps the windows' counts in one
+// register, checked in one operation. 67 M values take 67.9 us to encode at 8 bits/value, 102 at 16, 191 at 32, and 79.2, 109 and 207 to
+// decode (copying the bytes: 51, 61 and 82): input that is in the L2, or fetched ahead into shared memory, takes the same time per value.
 //
 // Inputs the fast path does not cover (a non-finite or vanishing block maximum, a NaN
 // member, data so smooth that eight planes - in the decoder, three lookups - do not reach

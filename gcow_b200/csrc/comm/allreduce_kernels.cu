@@ -426,8 +426,8 @@ allreduce_fused_kernel(const ArArgs a) {
 // in 10^4 at 8 bits/value, nearly all of smooth data). Only a block of a tiny, huge or non-finite maximum goes through both coders, with
 // their tables read from global memory: loading them into every CTA's shared memory took a tenth of the kernel. Four blocks per thread
 // are in flight, bound by integer work and memory in about equal parts: us at 6.5 M / 33 M values of noise, both coders' tables in
-// shared memory and two blocks in flight -> now: 8 bits/value 16.9 -> 12.8 / 59.6 -> 51.2, 16 13.9 -> 12.4 / 53.8 -> 51.3; 1 M 7 either way. 6.5 M values
-// near 1: 8 bits 70 -> 37, 16 bits 158 -> 22. Six blocks in flight (64 registers, four CTAs per SM): 15.0 / 57.4.
+// shared memory and two blocks in flight -> now: 8 bits/value 16.9 -> 12.0 / 59.4 -> 48.9, 16 13.8 -> 11.9 / 53.8 -> 49.6, 32 13.8 -> 11.3 / 54.0 -> 47.0;
+// 6.5 M values near 1: 8 bits 72.5 -> 24.6, 16 bits 20.9 -> 11.9. Six blocks in flight (64 registers, four CTAs per SM): 8 bits 14.5 / 56.8.
 // EACH: there is a thread for every block (up to 909 312 values), which then works on that one alone and not on one of four, of which three are
 // empty: 262 144 values at 8 / 16 / 32 bits/value 3.6 -> 2.1 / 1.9 / 1.9 us (through both coders 4.3, 2.4, 2.3), 900 000 values 4.5 -> 2.5 / 2.2 / 2.2,
 // 1000 values 1.8 -> 1.3. With a second block for some, 1 M values, four at a time take 4.3.

@@ -36,10 +36,9 @@ constexpr int STAGE_BYTES = 2 * OPER_BYTES;           // 64 KB
 constexpr int STAGES = 3;
 // What an epilogue reads besides the accumulator.
 enum Side : int { kNothing = 0, kSum = 1, kArgument = 2 };      // a residual; the argument of a GELU' factor (and perhaps a residual)
-// Epilogue warps: eight, or sixteen for a GELU, whose arithmetic two warps per scheduler leave half of the issue slots to
-// (bias, GELU and its argument kept: 16384 x 4096 x 1024 142 -> 129 us, x 3072 110 -> 97, x 1024 44 -> 36; with a residual
-// sixteen are slower, 144 and 156, and plain 95 and 98). Twelve for a GELU' factor, whose registers sixteen leave no room for: 159 us with
-// eight, 145 with twelve, 192 with sixteen; a residual gains nothing from twelve (106 and 107 at 16384 x 1024 x 4096).
+// Epilogue warps: eight, or sixteen for a GELU, whose arithmetic two warps per scheduler leave half of the issue slots to (bias, GELU and its
+// argument kept, eight, sixteen: 16384 x 4096 x 1024 142, 129 us, x 3072 110, 97, x 1024 44, 36). Twelve for a GELU' factor, whose registers
+// sixteen leave no room for: 16384 x 4096 x 1024 139 us with eight, 133 with twelve, 164 with sixteen. A residual takes 121 with eight, 133 with twelve.
 template <int SIDE, bool WIDE> struct Epilogue { static constexpr int WARPS = WIDE ? 16 : SIDE == kArgument ? 12 : 8, THREADS = 64 + 32 * WARPS; };
 constexpr uint32_t TMEM_COLS = 512;
 
@@ -251,11 +250,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     uint32_t t = 0;
     bool ok = true;
     // A tile's blocks of 32 columns go to the column groups in order, as evenly as they can. What the epilogue reads besides the
-    // accumulator is fetched one block ahead, the next tile's first block with this one's last: read where it is used, every
-    // block stood for its load's whole latency, and few warps per scheduler cover little of it (16384 x 4096 x 1024 with a residual
-    // 189 -> 144 us, times GELU' 247 -> 151). The first block under the wait for its own tile was no better where the epilogue sets the
-    // pace, and there is none: with the tile before, and one copy of the code per block in the loop below, a residual 132 -> 122 us (x 1024 x
-    // 1024 52 -> 48, 2048 x 768 x 3072 25.5 -> 23.9), GELU' 177 -> 155 (x 3072 x 768 129 -> 114).
+    // accumulator is fetched one block ahead, the next tile's first block with this one's last: read where it is used, every block would
+    // stand for its load's whole latency, of which few warps per scheduler cover little. With the first block under the wait for its own
+    // tile, which is none where the epilogue sets the pace, and two copies of the code, 16384 x 4096 x 1024 took 145 us with a bias and a residual
+    // and 154 with GELU', now 121 and 133; x 1024 x 1024 49 and 52, now 41 and 45 (single launches).
     constexpr bool EVEN = BN / 64 % GROUPS == 0;
     [[maybe_unused]] auto blocks_before = [](bool half, int group) { return ((half ? BN / 64 : BN / 32) * group + GROUPS - 1) / GROUPS; };
     [[maybe_unused]] uint4 pf[4];                         // four lanes per row, as the staging helpers have it

@@ -150,10 +150,10 @@ layernorm_fwd_rows_kernel(const bf16* x, const float* gamma, const float* beta,
 // dgamma/dbeta contributions stay in registers over all its rows and touch shared memory once at the end. The next row is on its way into
 // shared memory (cp.async; each lane fetches and reads its own 16-byte pieces, so nothing has to be synchronised) while this one is worked
 // on. What bounds it is how many rows an SM has in flight: with the next row in registers it was 12 warps (168 registers at 1024 columns,
-// some of them spilled), now 16. Two rows ahead are slower (26.7 against 25.6 us at 16384 x 1024).
+// some of them spilled), now 16. Two rows ahead are 4 % slower at 16384 x 1024.
 // T threads a CTA, 512 / T CTAs per SM: with 512 threads the SM's partial sums are added up before they are written, with 128 few rows spread
-// over more SMs. Both passes together, against the rows in registers: 16384 x 1024 36.7 -> 24.9 us (100 MB take 15.4), x 768 22.6 -> 20.4,
-// x 512 19.0 -> 16.0, x 256 13.3 -> 11.1, 2048 x 1024 12.9 -> 8.7, 512 x 1024 8.7 -> 7.2.
+// over more SMs. Both passes together, against the rows in registers: 16384 x 1024 36.1 -> 24.7 us (100 MB take 15.4), x 768 23.1 -> 20.3,
+// x 512 18.6 -> 15.6, x 256 13.5 -> 10.7, 2048 x 1024 12.7 -> 8.5, 512 x 1024 8.1 -> 6.7.
 constexpr int kLnWide = 512, kLnNarrow = 128;
 __device__ __forceinline__ void copy16(void* smem, const void* g) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(g) : "memory");

@@ -292,12 +292,13 @@ PyObject* attr(PyObject* o, PyObject* name) {
   return v;
 }
 
-// A weight in bf16, in its own element order.
+// A weight in bf16, in its own element order. Not counted in g_launches: whether a layer needs it depends on whether an optimiser keeps the
+// copy, or which types torch casts, and the count is of the layers' own work.
 Tensor cast_bf16(const Tensor& d) {
   if (d.scalar_type() != at::kFloat || !d.is_non_overlapping_and_dense()) return d.to(at::kBFloat16);
   const Tensor out = at::detail::empty_strided_cuda(d.sizes(), d.strides(), at::TensorOptions(d.device()).dtype(at::kBFloat16));
   check(gcow_cast_bf16((const float*)d.const_data_ptr(), out.mutable_data_ptr(), (uint64_t)d.numel(),
-                       c10::cuda::getCurrentCUDAStream(d.device().index()).stream()), "gcow_cast_bf16");   // not among the counted launches, as torch's cast was not
+                       c10::cuda::getCurrentCUDAStream(d.device().index()).stream()), "gcow_cast_bf16");
   return out;
 }
 

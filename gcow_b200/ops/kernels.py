@@ -14,7 +14,8 @@ _err_words: dict = {}
 
 
 def launch_count() -> int:
-    """How many compute kernels of this library were launched through this module and the extension module's layers."""
+    """How many compute kernels of this library were launched through this module and the extension module's layers: the layers'
+    products, sweeps and sums. A weight's cast to bf16, where no optimiser keeps a copy, is not among them."""
     return _launches + (_native._ext.launches() if _native._ext is not None else 0)
 
 
