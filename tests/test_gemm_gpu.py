@@ -213,6 +213,24 @@ def test_every_tile_is_taken_once_in_either_order(M, N, monkeypatch):
     K_.check_errors()
 
 
+@pytest.mark.parametrize("M,N,K", [(2816, 2816, 2048), (3072, 3200, 2048), (5120, 5120, 4096), (5120, 5120, 4160), (4352, 4608, 4160), (4096, 4352, 4160),
+                                   (2816, 2816, 8192), (4352, 4608, 8192)])
+@pytest.mark.parametrize("b_t", [False, True])
+def test_long_reductions_on_either_kernel(M, N, K, b_t):
+    """Both sides of the lines between the pair and the one-CTA kernel for long plain reductions: a single round of tiles, as many rounds on
+    either, finer ones on pairs, and their lengths. Sums of whole numbers are exact in fp32 and rounded once."""
+    from gcow_b200.ops import kernels as K_
+    torch.manual_seed(M + K)
+    a = torch.randint(-1, 2, (M, K), device="cuda").bfloat16()
+    b = torch.randint(-1, 2, (K, N) if b_t else (N, K), device="cuda").bfloat16()
+    bias = torch.randint(-9, 10, (N,), device="cuda").float()
+    got = K_.gemm_bf16(a, b, bias=bias, b_t=b_t)
+    assert torch.equal(got, K_.gemm_bf16(a, b, bias=bias, b_t=b_t, tile_rows=256))
+    rows = slice(M // 2, M // 2 + 64)
+    assert torch.equal(got[rows], (a[rows].double() @ (b if b_t else b.t()).double() + bias.double()).float().bfloat16())
+    K_.check_errors()
+
+
 @pytest.mark.parametrize("M,N,K", [(1024, 256, 64), (1100, 1120, 192), (2100, 544, 576), (9500, 1024, 64), (19000, 512, 128), (40000, 64 * 9, 64)])
 def test_pair_gemm_side_operands_of_whole_numbers(M, N, K, monkeypatch):
     """The side operand is fetched a block ahead, also across tiles, and twelve warps share eight or four blocks of columns: one tile per
