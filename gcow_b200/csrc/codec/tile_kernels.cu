@@ -444,23 +444,29 @@ encode_tiles_kernel(const float* in, const TileArgs a, uint32_t* __restrict__ ou
 
 // Second kernel of the variable-rate encoder: every CTA takes a contiguous share of the tiles, at most kTileThreads of them at a
 // time, whose starts it works out in shared memory first; then nothing depends on anything but that table, and the
-// warps run through the strings at their own pace.
-// Five CTAs per SM with four blocks a lane, where the compiler would take 63 registers for four: encoding 25.6 M values at tolerance 1e-3
-// 114.0 -> 112.5 us, at precision 8 106.9 -> 104.6; six 115.3 and 106.9. With one block a lane eight fit by themselves.
-constexpr int place_ctas(int per) { return per == 4 ? 5 : 8; }
-template <int PER>
-__global__ void __launch_bounds__(kTileThreads, PER == 4 ? place_ctas(PER) : 0)
+// warps run through the strings at their own pace, each with parts of PART blocks and as large a share of their tile's words.
+// Bound by latency and by the bytes: a part is a few loads in a row, all of them ahead of the stores, and most of a small array's time is the
+// wait for the coder and the sum of the tiles before. With the whole CTA on one tile (154 instructions a warp for some 40 words and
+// 32 offsets, now a fifth of that) both kernels took, us, 7654 x 7654 at tolerance 1e-3 148.6, now 142, at 1e-1 112.6, now 102.4; 510 x 510 9.3, now
+// 8.8; 25.6 M values at tolerance 1e-6 132.7, now 129.7, at 1e-3 112.6, now 109.7. Six CTAs per SM with 128 blocks of four
+// a lane 131 and 114.4, four 134.7 and 115.7, with 64 blocks 142 and 122.
+// The next kernel is let in once the tiles before are added up: with 244 tiles a decoder that came at the start found the SMs unevenly
+// taken (1 M values at tolerance 1e-3, encoder and decoder 26.5 us, now 20.5; 510 x 510 14.5, now 13.4); at the very end, 7654 x 7654 at 1e-1
+// 103.2 instead of 102.2 and 1000 values 10.5 instead of 8.9.
+constexpr int kPlaceCtas = 5;
+template <int PER, int PART>
+__global__ void __launch_bounds__(kTileThreads, kPlaceCtas)
 place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restrict__ out, uint64_t* __restrict__ block_bits,
                      uint64_t* total_out) {
-  constexpr int NB = kTileThreads * PER;
+  constexpr int NB = kTileThreads * PER, kParts = NB / PART, kWords = PER == 4 ? 8 : 4;
   __shared__ unsigned long long s_sum[kTileWarps];
   __shared__ uint32_t s_warp[kTileWarps];
   __shared__ uint32_t s_bits[kTileThreads];                 // a string's length ...
   __shared__ uint32_t s_from[kTileThreads];                 // ... and start after the first one of the batch
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool wide = ((uintptr_t)block_bits & 15) == 0;
   const uint32_t t0 = (uint32_t)((uint64_t)a.tiles * blockIdx.x / gridDim.x);
   const uint32_t t1 = (uint32_t)((uint64_t)a.tiles * (blockIdx.x + 1) / gridDim.x);
-  pdl_trigger();
   pdl_wait();
   unsigned long long base = 0;
 #pragma unroll 4
@@ -476,6 +482,7 @@ place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restric
   base = 0;
 #pragma unroll
   for (int w = 0; w < kTileWarps; w++) base += s_sum[w];
+  pdl_trigger();
 
   for (uint32_t u0 = t0; u0 < t1; u0 += kTileThreads) {
     const uint32_t nu = t1 - u0 < kTileThreads ? t1 - u0 : kTileThreads;
@@ -503,42 +510,54 @@ place_strings_kernel(const TileStrings st, const TileArgs a, uint32_t* __restric
       __threadfence_system();
     }
 #pragma unroll 1
-    for (uint32_t k = 0; k < nu; k++) {
-      const uint32_t tile = u0 + k, total = s_bits[k];
+    for (uint32_t item = warp; item < nu * kParts; item += kTileWarps) {
+      const uint32_t k = item / kParts, part = item % kParts, tile = u0 + k, total = s_bits[k];
       const uint64_t start = base + s_from[k];
       const uint32_t* const src = st.strings + (uint64_t)tile * a.pitch;
-      const uint32_t o = (uint32_t)(start & 31u), words = (total + 31) >> 5, full = (o + total) >> 5;
+      const uint32_t o = (uint32_t)(start & 31u), full = (o + total) >> 5;   // at most the string's words
       uint32_t* const dst = out + (start >> 5);
-      uint32_t prev = 0;
-      if (tid == 0 && tile) prev = last_bits(src - a.pitch, k ? s_bits[k - 1] : st.tile_bits[tile - 1]);
-      const uint64_t b0 = (uint64_t)tile * NB;
-      // all of a thread's loads ahead of its stores
-      uint32_t at[PER];
+      // the offsets of two blocks a lane at a time, ahead of the words, and all of them ahead of their stores
+      constexpr int kPairs = (PART + 63) / 64;
+      const uint64_t b0 = (uint64_t)tile * NB + part * PART + 2 * lane, b1 = PART < 64 && lane >= PART / 2 ? 0 : a.blocks;
+      uint32_t at[kPairs], from[kPairs];
 #pragma unroll
-      for (int j = 0; j < PER; j++) {
-        const uint64_t b = b0 + tid + j * kTileThreads;
-        at[j] = b < a.blocks ? st.warp_at[(uint64_t)tile * kTileWarps + (tid + j * kTileThreads) / (32 * PER)] + st.block_at[b] : 0u;
+      for (int j = 0; j < kPairs; j++) {
+        const uint64_t b = b0 + 64 * j;
+        at[j] = b + 1 < b1 ? *reinterpret_cast<const uint32_t*>(st.block_at + b) : b < b1 ? st.block_at[b] : 0u;
+        from[j] = b < b1 ? st.warp_at[(uint64_t)tile * kTileWarps + (part * PART + 64 * j + 2 * lane) / (32 * PER)] : 0u;
       }
-      constexpr int kWords = 2 * PER;                       // a step's words per thread
+      const uint32_t each = (full + 32 * kParts - 1) / (32 * kParts) * 32, i0 = part * each, i1 = i0 + each < full ? i0 + each : full;
+      uint32_t prev = 0;                                    // the word before this part's first
+      if (part == 0) {
+        if (tile) prev = last_bits(src - a.pitch, k ? s_bits[k - 1] : st.tile_bits[tile - 1]);
+      } else if (i0 < i1) {
+        prev = src[i0 - 1];
+      }
+      uint32_t carry = prev;
 #pragma unroll 1
-      for (uint32_t i = tid; i < full; i += kWords * kTileThreads) {
-        uint32_t below[kWords], here[kWords];
+      for (uint32_t i = i0 + lane; i - lane < i1; i += 32 * kWords) {
+        uint32_t here[kWords];
+#pragma unroll
+        for (int j = 0; j < kWords; j++) here[j] = i + 32 * j < i1 ? src[i + 32 * j] : 0u;
 #pragma unroll
         for (int j = 0; j < kWords; j++) {
-          const uint32_t k = i + j * kTileThreads;
-          below[j] = k == 0 ? prev : k - 1 < words ? src[k - 1] : 0u;
-          here[j] = k < words ? src[k] : 0u;
+          uint32_t below = __shfl_up_sync(0xffffffffu, here[j], 1);
+          if (lane == 0) below = carry;
+          carry = __shfl_sync(0xffffffffu, here[j], 31);
+          if (i + 32 * j < i1) dst[i + 32 * j] = __funnelshift_l(below, here[j], o);
         }
-#pragma unroll
-        for (int j = 0; j < kWords; j++)
-          if (i + j * kTileThreads < full) dst[i + j * kTileThreads] = __funnelshift_l(below[j], here[j], o);
       }
 #pragma unroll
-      for (int j = 0; j < PER; j++) {
-        const uint64_t b = b0 + tid + j * kTileThreads;
-        if (b < a.blocks) block_bits[b] = start + at[j];
+      for (int j = 0; j < kPairs; j++) {
+        const uint64_t b = b0 + 64 * j, first = start + from[j] + (at[j] & 0xffffu), second = start + from[j] + (at[j] >> 16);
+        if (wide && b + 1 < b1) {
+          *reinterpret_cast<ulonglong2*>(block_bits + b) = make_ulonglong2(first, second);
+        } else {
+          if (b < b1) block_bits[b] = first;
+          if (b + 1 < b1) block_bits[b + 1] = second;
+        }
       }
-      if (tile + 1 == a.tiles && tid == 0) {
+      if (tile + 1 == a.tiles && part == 0 && lane == 0) {
         block_bits[a.blocks] = start + total;
         close_stream(out, src, start, total, prev);
       }
@@ -683,6 +702,18 @@ int grid_of(uint32_t smem, uint32_t tiles, int* err) {
   return (int)(tiles < g ? tiles : g);
 }
 
+// The coders' split between L1 and shared memory for the kernel behind them too: an SM whose next kernel wants another one has to run
+// empty first (510 x 510 at tolerance 1e-3 and back 15.0 -> 13.9 us, 100 000 values at 1e-6 11.3 -> 10.3).
+template <auto kKernel>
+int all_shared() {
+  static std::atomic<bool> done[64];                        // by device
+  int dev = 0, err = (int)cudaGetDevice(&dev);
+  if (err || (dev < 64 && done[dev].load(std::memory_order_relaxed))) return err;
+  err = (int)cudaFuncSetAttribute(kKernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  if (!err && dev < 64) done[dev].store(true, std::memory_order_relaxed);
+  return err;
+}
+
 }  // namespace
 
 extern "C" {
@@ -792,9 +823,17 @@ int gcow_encode_tiles(const float* in, uint64_t nx, uint64_t ny, const int32_t* 
 #undef GCOW_ENCODE_MODE
 #undef GCOW_ENCODE
   if (!fixed) {
-    const uint32_t most = 148 * place_ctas(per), g = a.tiles < most ? a.tiles : most;
-    if (per == 4) launch_dependent(place_strings_kernel<4>, dim3(g), dim3(kTileThreads), 0, s, st, a, (uint32_t*)out, block_bits, total_out);
-    else launch_dependent(place_strings_kernel<1>, dim3(g), dim3(kTileThreads), 0, s, st, a, (uint32_t*)out, block_bits, total_out);
+    const uint32_t most = 148 * kPlaceCtas, g = a.tiles < most ? a.tiles : most;
+    // Where every CTA has a tile of its own, one warp to an eighth of it.
+#define GCOW_PLACE(P, N)                                                                                          \
+  do {                                                                                                         \
+    if ((err = all_shared<&place_strings_kernel<P, N>>())) return err;                                         \
+    launch_dependent(place_strings_kernel<P, N>, dim3(g), dim3(kTileThreads), 0, s, st, a, (uint32_t*)out, block_bits, total_out); \
+  } while (0)
+    if (a.tiles > most) { if (per == 4) GCOW_PLACE(4, 256); else GCOW_PLACE(1, 128); }
+    else if (per == 4) GCOW_PLACE(4, 128);
+    else GCOW_PLACE(1, 32);
+#undef GCOW_PLACE
   }
   return (int)cudaGetLastError();
 }

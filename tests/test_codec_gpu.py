@@ -227,6 +227,37 @@ def test_2d_tiles_around_the_line_between_instances(tiles, how):
     assert torch.equal(g.decompress(gpu).cpu().view(torch.int32), g.decompress(cpu).view(torch.int32))
 
 
+@pytest.mark.parametrize("dim,tile", [(1, 256), (1, 1024), (2, 256)])
+@pytest.mark.parametrize("more", [-1, 0, 1])
+def test_strings_of_as_many_tiles_as_ctas(dim, tile, more):
+    """The placing kernel where its CTAs have a tile each and just above, the last tile with one block or one short of all, for an index
+    at a multiple of 16 bytes and of 8 only."""
+    tiles = 740 + more if (dim, tile) != (1, 256) else 592 + more       # 1-D: four blocks a lane from 593 tiles of 256 on
+    blocks = tiles * tile - (tile - 1 if more == 0 else 1)
+    rng = np.random.default_rng(blocks)
+    if dim == 1:
+        x = (rng.standard_normal(4 * blocks) * 1e-3).astype(np.float32)
+        x[:8000] = 0
+    else:
+        x = (rng.standard_normal((4, 4 * blocks)) * 1e-4).astype(np.float32) + np.float32(1) / (1 + np.arange(4 * blocks, dtype=np.float32))
+    p = ZfpParams.from_accuracy(1e-5)
+    cpu = g.compress(torch.from_numpy(x), params=p, dim=dim, return_index=True)
+    lib, d = _native.cuda(), dev(x)
+    lib.gcow_encode_tiles.argtypes = [C.c_void_p, C.c_uint64, C.c_uint64, C.c_void_p] + [C.c_void_p] * 5
+    lib.gcow_encode_tiles_scratch_bytes.argtypes, lib.gcow_encode_tiles_scratch_bytes.restype = [C.c_void_p, C.c_uint64, C.c_int], C.c_uint64
+    par = p.as_c()
+    scratch = torch.empty(lib.gcow_encode_tiles_scratch_bytes(par, blocks, dim), dtype=torch.uint8, device="cuda")
+    for skip in (0, 1):
+        out = torch.full((blocks * 72 + 64,), 255, dtype=torch.uint8, device="cuda")
+        index = torch.full((blocks + 3,), -1, dtype=torch.int64, device="cuda")
+        rc = lib.gcow_encode_tiles(d.data_ptr(), x.shape[-1], 4 if dim == 2 else 0, par, out.data_ptr(), scratch.data_ptr(),
+                                   index.data_ptr() + 8 * skip, None, None)
+        torch.cuda.synchronize()
+        assert rc == 0
+        assert torch.equal(index[skip:skip + blocks + 1].cpu(), cpu.index) and (index[skip + blocks + 1:] == -1).all()
+        assert torch.equal(out[:cpu.nbytes].cpu(), cpu.stream)
+
+
 @pytest.mark.parametrize("n", [4 * 300, 4 * 151552 + 7, 4 * 148 * 6 * 4 * 1024 * 2 + 40_001])
 @pytest.mark.parametrize("how", [dict(tolerance=1e-6), dict(tolerance=1e-3), dict(precision=8), dict(precision=16)])
 def test_1d_tiles_of_data_that_changes(n, how):
