@@ -40,6 +40,9 @@ enum Side : int { kNothing = 0, kSum = 1, kArgument = 2 };      // a residual; t
 // argument kept, eight, sixteen: 16384 x 4096 x 1024 142, 129 us, x 3072 110, 97, x 1024 44, 36). Twelve for a GELU' factor, whose registers
 // sixteen leave no room for: 16384 x 4096 x 1024 139 us with eight, 133 with twelve, 164 with sixteen. A residual takes 121 with eight, 133 with twelve.
 template <int SIDE, bool WIDE> struct Epilogue { static constexpr int WARPS = WIDE ? 16 : SIDE == kArgument ? 12 : 8, THREADS = 64 + 32 * WARPS; };
+// Warps of a weight gradient that add up the columns of A as they pass through shared memory (the bias gradient).
+constexpr int SUM_WARPS = 2;
+template <bool A_MN, int SIDE, bool WIDE> constexpr int kThreads = Epilogue<SIDE, WIDE>::THREADS + (A_MN ? 32 * SUM_WARPS : 0);
 constexpr uint32_t TMEM_COLS = 512;
 
 enum Flags : int { kBias = 2, kGelu = 4, kResidual = 8, kAuxOut = 32, kGeluGrad = 64 };
@@ -54,6 +57,7 @@ struct Params {
   int slice_blocks;        // stages per slice of the reduction
   int halves;              // weight gradient, an item per pair at most: a slice's two halves have an accumulator each
   size_t slice_stride;     // elements from one slice's result to the next
+  float* sums;             // of a weight gradient: [slices * tile columns][M] partial column sums of A, or null
   QuickTileOrder order;
   uint32_t* error;
 };
@@ -75,7 +79,7 @@ template <bool SLICES, bool DIVIDE> __device__ __forceinline__ Item item_at(cons
 }
 
 struct Smem {
-  uint64_t full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], drain;
+  uint64_t full[STAGES], empty[STAGES], landed[STAGES], tmem_full[2], tmem_empty[2], drain;
   uint32_t tmem_base;
   volatile uint32_t abort;
 };
@@ -126,7 +130,7 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128_16k(uint32_t saddr) {
 // B_MN: B is stored [K][N] (the data-gradient product dX = dY * W reads the weight matrix in place); A_MN: A is stored [K][M]
 // (with B_MN the weight gradient, which reads both in place). SIDE: what the epilogue reads.
 template <bool A_MN, bool B_MN, int SIDE, bool WIDE>
-__global__ void __launch_bounds__(Epilogue<SIDE, WIDE>::THREADS, 1)
+__global__ void __launch_bounds__((kThreads<A_MN, SIDE, WIDE>), 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   const __grid_constant__ CUtensorMap tmap_bh, const Params p) {
   constexpr int EPI_WARPS = Epilogue<SIDE, WIDE>::WARPS;
@@ -143,7 +147,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const int kblocks = (p.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; s++) { mbar_init(&sm->full[s], 1); mbar_init(&sm->empty[s], 1); }
+    const uint32_t readers = A_MN && p.sums ? 1 + SUM_WARPS : 1;
+    for (int s = 0; s < STAGES; s++) { mbar_init(&sm->full[s], 1); mbar_init(&sm->empty[s], readers); mbar_init(&sm->landed[s], 1); }
     for (int a = 0; a < 2; a++) { mbar_init(&sm->tmem_full[a], 1); mbar_init(&sm->tmem_empty[a], 2 * EPI_WARPS * 32); }
     mbar_init(&sm->drain, 1);
     sm->abort = 0;
@@ -213,6 +218,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           const uint32_t sa = smem_u32(base + s * STAGE_BYTES), sb = sa + OPER_BYTES;
           const uint32_t eb0 = map_to_cta(smem_u32(&sm->empty[s]), 0), eb1 = map_to_cta(smem_u32(&sm->empty[s]), 1);
           if (lane == 0) {
+            if (A_MN && p.sums) {                             // the warps that add up may read the stage too
+              mbar_arrive_cluster(map_to_cta(smem_u32(&sm->landed[s]), 0));
+              mbar_arrive_cluster(map_to_cta(smem_u32(&sm->landed[s]), 1));
+            }
 #pragma unroll
             for (int k = 0; k < BK / UMMA_K; k++) {
               const uint32_t in = (k & 3) * 32;                               // 64-wide chunk, then 32 bytes per K step
@@ -238,6 +247,67 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       if (lane == 0) {
         tc_commit_pair(map_to_cta(smem_u32(&sm->drain), 0));
         for (uint32_t it = 0; it < kSpinLimit; it++) if (mbar_try_wait(&sm->drain, 0)) break;
+      }
+    }
+  } else if (A_MN && warp >= 2 + EPI_WARPS) {
+    // ------------------------------------------------- column sums of A (both CTAs, own 128 columns), where they are wanted
+    // The tiles of one row have the same part of A in shared memory, so tile column j takes every tiles_n-th group of four rows of a stage from
+    // the j-th on. A warp takes 64 columns, a lane 8 of them in one row of each group, which come from two of a row's 16-byte chunks in turn
+    // (128-byte swizzle). It adds up 16 rows or a few more, up to four such sums, and those, so that no chain is long.
+    // A stage's MMAs take longer than a share of its sums, so nothing waits for these. The product alone, with the column sums as kernels of their
+    // own, with these, us, each with its ordered sums: 16384 rows to 3072 x 1024 85.9, 107.6, 86.5; to 4096 x 1024 99.4, 130.6, 101.5; to 768 x 768
+    // 29.7, 39.1, 30.2; 1024 rows to 768 x 768 17.0, 19.6, 18.7; 16384 to 256 x 256, where a tile has all groups to itself, 14.6, 21.2, 18.6. Whole
+    // stages in turn instead of groups of rows held a stage for longer than its MMAs: 16384 rows to 4096 x 1024 122.
+    if (p.sums) {
+      const int w = warp - 2 - EPI_WARPS, row = lane >> 3, chunk = lane & 7;
+      const uint8_t* const mine = base + w * 16384 + row * 128;
+      const int even = (chunk ^ row) * 16, odd = 512 + (chunk ^ (row + 4)) * 16;
+      uint32_t s = 0, phase = 0;
+      bool ok = true;
+      for (int i = pair; i < p.items && ok; i += pairs) {
+        const Item it = item_at<A_MN, SIDE == kArgument>(p, i, tiles, kblocks);
+        const int first = it.n0 / BN;
+        int rows = 0, held = 0;
+        float sum[8] = {}, some[8] = {}, v[8] = {};
+        for (int kb = it.kb0; kb < it.kb1; kb++) {
+          ok = __all_sync(0xffffffffu, mbar_wait_abortable(&sm->abort, &sm->landed[s], phase, p.error, 5)) != 0;
+          if (!ok) break;
+          const uint8_t* const at = mine + s * STAGE_BYTES;
+#pragma unroll 4
+          for (int r = first; r < 32; r += tiles_n) {
+            const uint4 x = *reinterpret_cast<const uint4*>(at + (r >> 1) * 1024 + (r & 1 ? odd : even));
+            const uint32_t y[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) { v[2 * j] += __uint_as_float(y[j] << 16); v[2 * j + 1] += __uint_as_float(y[j] & 0xffff0000u); }
+            rows++;
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm->empty[s]);
+          if (rows >= 16) {
+#pragma unroll
+            for (int j = 0; j < 8; j++) { some[j] += v[j]; v[j] = 0.0f; }
+            rows = 0;
+            if (++held == 4) {
+#pragma unroll
+              for (int j = 0; j < 8; j++) { sum[j] += some[j]; some[j] = 0.0f; }
+              held = 0;
+            }
+          }
+          if (++s == STAGES) { s = 0; phase ^= 1; }
+        }
+        if (!ok) break;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          sum[j] += some[j] + v[j];
+#pragma unroll
+          for (int d = 8; d < 32; d *= 2) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], d);
+        }
+        const int m = it.m0 + (int)rank * 128 + w * 64 + chunk * 8;
+        if (lane < 8 && m < p.M) {                            // M is a multiple of 64
+          float* const to = p.sums + (size_t)(it.slice * tiles_n + it.n0 / BN) * p.M + m;
+          *reinterpret_cast<float4*>(to) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+          *reinterpret_cast<float4*>(to + 4) = make_float4(sum[4], sum[5], sum[6], sum[7]);
+        }
       }
     }
   } else {
@@ -568,10 +638,15 @@ int gcow_gemm2_wgrad_slices(int M, int N, int K) {
   return best;
 }
 
+// Partial column sums per slice that gcow_gemm2_wgrad leaves for a result of N columns.
+int gcow_gemm2_wgrad_sums(int N) { return (N + BN - 1) / BN; }
+
 // parts[slice][M][N] fp32 = A^T B over the slice's rows, A [K][M], B [K][N] bf16 with contiguous rows: the weight gradient of a
-// linear layer. `slices` as gcow_gemm2_wgrad_slices has it.
-int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, int M, int N, int K, int lda, int ldb, int slices, uint32_t* error, void* stream) {
-  if (M <= 0 || N <= 0 || K <= 0 || slices <= 0 || M % 64 || N % 64 || lda % 8 || ldb % 8 || ((uintptr_t)parts & 15)) return -2;
+// linear layer. `slices` as gcow_gemm2_wgrad_slices has it. sums (or null): [slices * gcow_gemm2_wgrad_sums(N)][M] fp32, which add up to the
+// column sums of A, the bias gradient.
+int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, float* sums, int M, int N, int K, int lda, int ldb, int slices, uint32_t* error,
+                     void* stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || slices <= 0 || M % 64 || N % 64 || lda % 8 || ldb % 8 || (((uintptr_t)parts | (uintptr_t)sums) & 15)) return -2;
   const int max_pairs = gcow_gemm2_max_pairs();
   if (max_pairs <= 0) return -2;
   CUtensorMap ma, mb;
@@ -588,7 +663,8 @@ int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, int M, int N, i
   p.order = quick(tile_order(M, N, K, BM, BN));
   p.slice_stride = (size_t)M * N;
   p.halves = p.items <= max_pairs;
-  return launch(gemm2_bf16_kernel<true, true, kNothing, false>, Epilogue<kNothing, false>::THREADS, max_pairs, ma, mb, mb, p, stream);
+  p.sums = sums;
+  return launch(gemm2_bf16_kernel<true, true, kNothing, false>, kThreads<true, kNothing, false>, max_pairs, ma, mb, mb, p, stream);
 }
 
 }  // extern "C"

@@ -602,6 +602,40 @@ colsum_cluster_kernel(const bf16* g, float* __restrict__ out, int rows, int cols
   cluster.sync();                                                // the others' sums are read until here
 }
 
+// Both of a linear layer's sums in one launch, each in the order that it has by itself: the first CTAs four columns of the weight gradient a
+// thread, the others 32 columns of the bias gradient each, 8 threads to a column.
+__global__ void __launch_bounds__(256)
+reduce_weight_bias_kernel(const float4* part, float4* __restrict__ out, int parts, int n4, const float* bias_part, float* __restrict__ bias_out,
+                          int bias_parts, int bias_n, unsigned first) {
+  pdl_wait();
+  pdl_trigger();
+  if (blockIdx.x < first) {
+    const int c = blockIdx.x * 256 + threadIdx.x;
+    if (c >= n4) return;
+    float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+    for (int p = 0; p < parts; p++) {
+      const float4 v = part[(size_t)p * n4 + c];
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    out[c] = s;
+    return;
+  }
+  __shared__ float sm[8][33];
+  const int cx = threadIdx.x & 31, py = threadIdx.x >> 5, c = (blockIdx.x - first) * 32 + cx;
+  float s = 0;
+  if (c < bias_n)
+    for (int p = py; p < bias_parts; p += 8) s += bias_part[(size_t)p * bias_n + c];
+  sm[py][cx] = s;
+  __syncthreads();
+  if (py == 0 && c < bias_n) {
+    float t = 0;
+#pragma unroll
+    for (int j = 0; j < 8; j++) t += sm[j][cx];
+    bias_out[c] = t;
+  }
+}
+
 // ------------------------------------------------------------ weights to bf16
 // y = bf16(x), rounded to nearest even. Stands between two dependent kernels where a weight has no bf16 copy; as one of them its launch
 // and start are hidden, and torch's cast took 10 us of the host (1024 -> 512, 1 x 1 and 7 x 7, batch 16: 180 -> 171 us, all host).
@@ -754,6 +788,16 @@ int gcow_softmax_bwd(const void* dp, const void* p, void* ds, int64_t rows, int 
 
 // Column sums of a bf16 [rows, cols] matrix (ld even, cols even) into fp32 out[cols];
 // `part` must hold gcow_colsum_parts(rows) * cols floats.
+// Both sums of partial results of a linear layer: a weight gradient of n elements (parts 0: there is none to add up) and a bias
+// gradient of bias_n. n a multiple of 4, part and out at multiples of 16 bytes.
+int gcow_reduce_weight_bias(const float* part, float* out, int parts, int64_t n, const float* bias_part, float* bias_out, int bias_parts,
+                            int bias_n, void* stream) {
+  if (parts < 0 || bias_parts <= 0 || bias_n <= 0 || n < 0 || n > 0x7fffffff || n % 4 || (((uintptr_t)part | (uintptr_t)out) & 15)) return -1;
+  const unsigned first = parts ? (unsigned)((n / 4 + 255) / 256) : 0;
+  gcow::launch_dependent(reduce_weight_bias_kernel, dim3(first + (unsigned)((bias_n + 31) / 32)), dim3(256), 0, (cudaStream_t)stream,
+                         (const float4*)part, (float4*)out, parts, (int)(n / 4), bias_part, bias_out, bias_parts, bias_n, first);
+  return (int)cudaGetLastError();
+}
 int gcow_colsum_parts(int rows) { int p = (rows + 127) / 128; return p < 128 ? (p < 1 ? 1 : p) : 128; }
 // Kernels that gcow_colsum launches: one (`part` is not used), or the partial sums and their reduction.
 int gcow_colsum_launches(const void* g, int rows, int cols, int ld) {

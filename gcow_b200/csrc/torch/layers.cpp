@@ -26,8 +26,9 @@ extern "C" {
 int gcow_gemm2_max_pairs();
 int gcow_wgrad_slabs(int64_t M, int64_t N, int64_t K);
 int gcow_gemm2_wgrad_slices(int M, int N, int K);
-int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, int M, int N, int K, int lda, int ldb, int slices, uint32_t* error,
-                     void* stream);
+int gcow_gemm2_wgrad_sums(int N);
+int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, float* sums, int M, int N, int K, int lda, int ldb, int slices,
+                     uint32_t* error, void* stream);
 int gcow_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, const float* bias,
                     const void* residual, void* aux, int flags, uint32_t* error, int b_mn, void* stream);
 int gcow_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, const float* bias,
@@ -38,6 +39,8 @@ int gcow_gemm_bf16_batched(const void* A, const void* B, void* C, int M, int N, 
                            long long stride_a, long long stride_b, long long stride_c, const float* bias, const void* residual,
                            int flags, uint32_t* error, int a_mn, int b_mn, int tile_rows, void* stream);
 int gcow_reduce_partials(const float* part, float* out, int parts, int64_t n, void* stream);
+int gcow_reduce_weight_bias(const float* part, float* out, int parts, int64_t n, const float* bias_part, float* bias_out, int bias_parts,
+                            int bias_n, void* stream);
 int gcow_colsum_parts(int rows);
 int gcow_colsum_launches(const void* g, int rows, int cols, int ld);
 int gcow_colsum(const void* g, float* part, float* out, int rows, int cols, int ld, void* stream);
@@ -235,8 +238,8 @@ Tensor add_parts(const Tensor& part, int64_t parts, c10::IntArrayRef shape, Tens
 
 // dW[N,K] = g^T x, fp32, for g [M,N] and x [M,K], both stored with the reduction dimension M outermost. The result has few tiles
 // while M is long, so the rows are cut into slices whose products are added in order: on CTA pairs in one launch, else as
-// slabs of one batched launch.
-Tensor wgrad(const Tensor& g, const Tensor& x, const Tensor& out, const On& on) {
+// slabs of one batched launch. With `bias` CTA pairs add up the columns of g as they pass (*bias: the result, which stays undefined otherwise).
+Tensor wgrad(const Tensor& g, const Tensor& x, const Tensor& out, const On& on, Tensor* bias = nullptr) {
   TORCH_CHECK(g.dim() == 2 && x.dim() == 2 && g.size(0) == x.size(0) && g.scalar_type() == at::kBFloat16 && x.scalar_type() == at::kBFloat16 &&
               g.stride(1) == 1 && x.stride(1) == 1, "wgrad: expected two bf16 matrices with contiguous rows, as many in each");
   const int64_t M = g.size(0), N = g.size(1), K = x.size(1);
@@ -248,9 +251,19 @@ Tensor wgrad(const Tensor& g, const Tensor& x, const Tensor& out, const On& on) 
                          ? gcow_gemm2_wgrad_slices((int)N, (int)K, (int)M) : 0;
   if (slices > 0) {                                          // CTA pairs, which cut the rows themselves
     const Tensor to = slices == 1 && out.defined() ? out : empty({slices, N, K}, at::kFloat, g);
-    check(gcow_gemm2_wgrad(g.data_ptr(), x.data_ptr(), f32(to), (int)N, (int)K, (int)M, (int)g.stride(0), (int)x.stride(0), slices, on.error, on.stream),
-          "gcow_gemm2_wgrad");
+    const int64_t bias_parts = bias ? slices * gcow_gemm2_wgrad_sums((int)K) : 0;
+    const Tensor sums = bias ? empty({bias_parts, N}, at::kFloat, g) : Tensor();
+    check(gcow_gemm2_wgrad(g.data_ptr(), x.data_ptr(), f32(to), f32(sums), (int)N, (int)K, (int)M, (int)g.stride(0), (int)x.stride(0), slices,
+                           on.error, on.stream), "gcow_gemm2_wgrad");
     g_launches++;
+    if (bias) {                                              // N and K are multiples of 64
+      const Tensor dw = slices > 1 && !out.defined() ? empty({N, K}, at::kFloat, g) : out;
+      *bias = empty({N}, at::kFloat, g);
+      check(gcow_reduce_weight_bias(f32(to), slices > 1 ? f32(dw) : nullptr, slices > 1 ? slices : 0, N * K, f32(sums), f32(*bias), (int)bias_parts,
+                                    (int)N, on.stream), "gcow_reduce_weight_bias");
+      g_launches++;
+      return slices > 1 || out.defined() ? dw : to.view({N, K});
+    }
     return slices > 1 ? add_parts(to, slices, {N, K}, out, on) : out.defined() ? out : to.view({N, K});
   }
   const int64_t s = gcow_wgrad_slabs(N, K, M);
@@ -434,12 +447,15 @@ inline std::vector<int64_t> with_last(const Tensor& x, int64_t last) {
   return s;
 }
 
-// dW of a linear layer: into the trainer's target where there is one, else a new tensor.
-Tensor linear_wgrad(const Target& t, const Tensor& g, const Tensor& x, const On& on) {
-  Tensor result;
-  const Tensor flat = target_matrix(t, g.size(1), x.size(1), 16, &result);
-  if (flat.defined()) { wgrad(g, x, flat, on); return result; }
-  return wgrad(g, x, Tensor(), on);
+// The gradients of a linear layer's weight, into the trainer's target where there is one, else a new tensor, and of its bias, as far as they are
+// wanted.
+void linear_wgrad(const Target& t, const Tensor& g, const Tensor& x, bool want_weight, bool want_bias, Tensor* weight, Tensor* bias, const On& on) {
+  if (want_weight) {
+    Tensor result;
+    const Tensor flat = target_matrix(t, g.size(1), x.size(1), 16, &result), dw = wgrad(g, x, flat, on, want_bias ? bias : nullptr);
+    *weight = flat.defined() ? result : dw;
+  }
+  if (want_bias && !bias->defined()) *bias = colsum(g, on);
 }
 
 // ---------------------------------------------------------------------- linear layers
@@ -461,8 +477,7 @@ struct LinearNode : LayerNode {                             // inputs: x, w, b, 
       gemm(g, wb, o, on);
       out[0] = std::move(full);
     }
-    if (wants(1)) out[1] = linear_wgrad(target[0], g, xb, on);
-    if (has_bias && wants(2)) out[2] = colsum(g, on);
+    linear_wgrad(target[0], g, xb, wants(1), has_bias && wants(2), &out[1], &out[2], on);
     if (has_res && wants(3)) out[3] = in[0];
     return out;
   }
@@ -516,8 +531,7 @@ struct FfnNode : LayerNode {                                // inputs: x, w1, b1
     o.b_t = true;
     o.gelu_grad_of = pre;
     const Tensor dpre = gemm(g, w2b, o, on);                // (g W2) * GELU'(pre)
-    if (wants(3)) out[3] = linear_wgrad(target[1], g, act, on);
-    if (wants(4)) out[4] = colsum(g, on);
+    linear_wgrad(target[1], g, act, wants(3), wants(4), &out[3], &out[4], on);
     if (wants(0)) {
       Tensor full = empty(shape, at::kBFloat16, g);
       GemmOpts q;
@@ -527,8 +541,7 @@ struct FfnNode : LayerNode {                                // inputs: x, w1, b1
       gemm(dpre, w1b, q, on);
       out[0] = std::move(full);
     }
-    if (wants(1)) out[1] = linear_wgrad(target[0], dpre, xb, on);
-    if (wants(2)) out[2] = colsum(dpre, on);
+    linear_wgrad(target[0], dpre, xb, wants(1), wants(2), &out[1], &out[2], on);
     return out;
   }
 };

@@ -133,6 +133,28 @@ def test_wgrad_on_pairs_at_the_edges(M, N, K):
     assert y.data_ptr() == out.data_ptr()
 
 
+@pytest.mark.parametrize("M,N,K", [(1024, 256, 256), (1192, 320, 448), (1100, 256, 768), (5000, 1024, 1280), (40000, 256, 320), (2048, 512, 4096),
+                                   (1500, 256, 8192), (1024, 256, 8448), (16384, 3072, 1024), (4096, 4096, 1024)])
+def test_bias_gradient_beside_the_weight_gradient(M, N, K):
+    """Column sums taken while the weight gradient's tiles pass: one tile column that has all rows of a stage to itself up to more tile columns
+    than a stage has groups of four rows, tiles that overhang, rows that end inside a stage, one slice, two accumulators, several."""
+    from gcow_b200 import _native
+    from gcow_b200.ops import kernels as K_
+    if _native.cuda().gcow_gemm2_wgrad_slices(N, K, M) <= 0:
+        pytest.skip("clusters of two CTAs cannot be scheduled here")
+    torch.manual_seed(M + N + K)
+    # whole numbers, so that a sum below 2^24 is exact in any order
+    g, x = (torch.randint(-2, 3, (M, n), device="cuda").bfloat16() for n in (N, K))
+    w = torch.zeros(N, K, device="cuda", requires_grad=True)
+    b = torch.zeros(N, device="cuda", requires_grad=True)
+    for _ in range(2):                                      # results of the second pass do not depend on the first
+        w.grad = b.grad = None
+        K_.linear(x, w, b).backward(g)
+        K_.check_errors()
+        assert torch.equal(b.grad.double(), g.double().sum(0))
+        assert torch.equal(w.grad.double(), g.double().t() @ x.double())
+
+
 def test_wgrad_slices_are_no_longer_than_slabs():
     """The tensor core's running sum loses a little at every step, so a slice of the rows on CTA pairs has no more stages of 128 than
     a slab of the one-CTA route, which doubles the slabs while the tiles fit 148 CTAs and 512 rows are left - twice as
