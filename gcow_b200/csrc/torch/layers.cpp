@@ -459,7 +459,7 @@ void linear_wgrad(const Target& t, const Tensor& g, const Tensor& x, bool want_w
 }
 
 // ---------------------------------------------------------------------- linear layers
-struct LinearNode : LayerNode {                             // inputs: x, w, b, residual
+struct LinearNode : LayerNode {                             // inputs: x, w, b, residual; outputs: y and, forked, x again
   std::vector<int64_t> x_shape;
   bool has_bias = false, has_res = false;
   std::string name() const override { return "GcowLinearBackward"; }
@@ -467,10 +467,16 @@ struct LinearNode : LayerNode {                             // inputs: x, w, b, 
     variable_list out(4);
     const Tensor &xb = had[0], &wb = had[1];
     const On on(xb);
+    const Tensor other = in.size() > 1 ? in[1] : Tensor();  // x's other gradient
+    if (!in[0].defined()) {
+      if (wants(0)) out[0] = other;
+      return out;
+    }
     const Tensor g = rows_of(in[0]);
-    if (wants(0)) {                                         // dx[M,K] = g[M,N] W[N,K]: W is stored [reduction N][K]
+    if (wants(0)) {                                         // dx[M,K] = g[M,N] W[N,K] (+ other): W is stored [reduction N][K]
       GemmOpts o;
       o.b_t = true;
+      if (other.defined()) o.residual = as_rows(bf16_rows16(other));
       o.out = empty(x_shape, at::kBFloat16, g);
       Tensor full = o.out;
       o.out = as_rows(full);
@@ -484,10 +490,14 @@ struct LinearNode : LayerNode {                             // inputs: x, w, b, 
 };
 
 // linear(x, w, b or None, residual or None): x W^T + b (+ residual, in the epilogue)
+// linear(x, w, b or None, None, True): that and a second tensor on x's memory, for the other consumer of a bf16 x. The two gradients then come
+// to this layer's node, and the data gradient's epilogue adds the other one; autograd would add them with a kernel of its own.
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  TORCH_CHECK(nargs == 4, "linear: bad arguments");
+  TORCH_CHECK(nargs == 4 || nargs == 5, "linear: bad arguments");
   const Tensor x = need(args[0]), w = need(args[1]), b = arg(args[2]), r = arg(args[3]);
+  const bool fork = nargs == 5 && PyObject_IsTrue(args[4]) == 1;
+  TORCH_CHECK(!fork || (!r.defined() && x.scalar_type() == at::kBFloat16), "linear: the second result goes with a bf16 input and no residual");
   TORCH_CHECK(x.dim() >= 1, "linear: the input has no dimensions");
   on_device_of(x, {&w, &b, &r});
   dims("linear: the weight", w, 2);
@@ -514,6 +524,18 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
       node->has_res = r.defined();
       node->target[0] = {take_grad_view(args[1]), w};
     }
+  }
+  if (fork) {
+    Tensor again = x.variable_data();                       // the same memory, no autograd view of x
+    if (node) {
+      torch::autograd::set_history(out, node);
+      torch::autograd::set_history(again, node);
+    }
+    PyObject *y = THPVariable_Wrap(std::move(out)), *z = THPVariable_Wrap(std::move(again));
+    PyObject* pair = y && z ? PyTuple_Pack(2, y, z) : nullptr;
+    Py_XDECREF(y);
+    Py_XDECREF(z);
+    return pair;
   }
   return finish(std::move(out), node);
   END_HANDLE_TH_ERRORS

@@ -41,7 +41,8 @@ class BertLayer(nn.Module):
 
     def forward(self, x):                      # x: [B, S, H]
         B, S, H = x.shape
-        qkv = self.qkv(x).view(B, S, 3, self.heads, H // self.heads)
+        qkv, x = gnn.linear_fork(x, self.qkv)
+        qkv = qkv.view(B, S, 3, self.heads, H // self.heads)
         ctx = gnn.attention(qkv)               # [B, S, H]
         x = self.ln1(gnn.linear_residual(ctx, self.proj, x))
         return self.ln2(gnn.ffn_residual(x, self.fc1, self.fc2))

@@ -293,6 +293,11 @@ def linear(x, w, b):
     return _PaddedLinearFn.apply(x, w, b)
 
 
+def linear_fork(x, w, b):
+    """x W^T + b and x again for its other consumer, whose gradient the data gradient's epilogue adds."""
+    return _layers().linear(x, w, b, None, True)
+
+
 def _stream(dev):
     return torch._C._cuda_getCurrentRawStream(dev.index if dev.index is not None else torch.cuda.current_device())
 

@@ -30,6 +30,18 @@ def linear_residual(x: torch.Tensor, lin: nn.Linear, residual: torch.Tensor) -> 
     return residual + linear(x, lin.weight, lin.bias)
 
 
+def linear_fork(x: torch.Tensor, lin: nn.Linear):
+    """``(lin(x), x)`` where x has another consumer, such as a residual branch. On the own backend x comes back as a second
+    result of the layer, so that its two gradients meet in the epilogue of the data-gradient GEMM. Modules with hooks or
+    a forward of their own are called as they are, and so is everything while a trace is taken."""
+    if (backend.get_backend() == "own" and type(lin) is Linear and x.dtype == torch.bfloat16 and x.requires_grad and torch.is_grad_enabled()
+            and lin.out_features % 8 == 0 and K.gemm_usable(x, lin.weight) and torch._C._get_tracing_state() is None
+            and not (lin._forward_hooks or lin._forward_pre_hooks or lin._backward_hooks or lin._backward_pre_hooks or "forward" in lin.__dict__
+                     or nn.modules.module._has_any_global_hook())):
+        return K.linear_fork(x, lin.weight, lin.bias)
+    return lin(x), x
+
+
 def ffn_residual(x: torch.Tensor, fc1: nn.Linear, fc2: nn.Linear) -> torch.Tensor:
     """``x + fc2(gelu(fc1(x)))`` - the transformer feed-forward block. On the own backend bias, GELU, its
     gradient and both residual additions run inside the epilogues of the four GEMMs involved."""

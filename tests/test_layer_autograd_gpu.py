@@ -111,6 +111,35 @@ def test_wrong_arguments_are_refused():
         K.linear_residual(x, w, None, torch.zeros(32, 64, device="cuda"))
 
 
+@pytest.mark.parametrize("rows,n,k", [(2 * 64, 64, 128), (1024, 768, 256), (1192, 320, 448)])
+def test_forked_linear(rows, n, k):
+    """Both gradients of the input, one of them, and a second gradient that is no contiguous matrix; hooks keep the module's own call."""
+    from gcow_b200.ops import kernels as K
+    from gcow_b200.ops import nn as gnn
+    torch.manual_seed(rows)
+    lin = gnn.Linear(k, n).cuda()
+    x = torch.randn(rows, k, device="cuda").bfloat16().requires_grad_(True)
+    gy, gz = torch.randn(rows, n, device="cuda").bfloat16(), torch.randn(k, rows, device="cuda").bfloat16().t()
+    y, z = gnn.linear_fork(x, lin)
+    assert z is not x and z.data_ptr() == x.data_ptr() and torch.equal(y, K.linear(x, lin.weight, lin.bias))
+    got = torch.autograd.grad((y, z), (x, lin.weight, lin.bias), (gy, gz), retain_graph=True)
+    want = torch.autograd.grad(K.linear(x, lin.weight, lin.bias), (x, lin.weight, lin.bias), gy)
+    exact = gy.double() @ lin.weight.detach().bfloat16().double() + gz.double()
+    # fp32 sums of k products and one bf16 rounding (2^-9 of the value; the sums' part is far below)
+    assert ((got[0].double() - exact).abs() <= exact.abs() * 2.0 ** -8 + 1e-4 * exact.abs().max()).all()
+    assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+    assert torch.equal(torch.autograd.grad(y, x, gy, retain_graph=True)[0], want[0])
+    assert torch.equal(torch.autograd.grad(z, x, gz)[0], gz)
+    seen = []
+    handle = lin.register_forward_hook(lambda m, i, o: seen.append(o.shape))
+    y, z = gnn.linear_fork(x, lin)
+    handle.remove()
+    assert z is x and seen == [y.shape]
+    y, z = gnn.linear_fork(x.detach(), lin)
+    assert z.grad_fn is None and y.grad_fn is not None
+    K.check_errors()
+
+
 def _grads(net, x, run):
     y = run(x)
     y.backward(torch.ones_like(y))
