@@ -15,8 +15,12 @@
 //
 // The reference's ResNet uses nn.BatchNorm2d + ReLU + add as separate ATen /
 // cuDNN operators (hw/models/resenet.py:12-22,28-40,80-89).
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+
+#include <atomic>
+#include <type_traits>
 
 #include "pdl.cuh"
 #include <stdlib.h>
@@ -272,6 +276,213 @@ bwd_dx_kernel(const bf16* __restrict__ dy, const uint8_t* __restrict__ mask, con
   }
 }
 
+// ------------------------------------------------------------------ one launch: a cluster takes CH channels
+// Tensors that the shared memory of the clusters holds: a CTA reads its share of the rows of its cluster's channels once, keeps them, and
+// the cluster adds up its sums through distributed shared memory, so the second sweep reads shared memory and there is nothing between the sweeps
+// but a cluster barrier. The three launches spend most of a small tensor's time on their starts and ends and read it twice. Bound by latency up to a
+// few MB, then by a row's 32 or 64 bytes per CTA and by the waves' phases, which load, wait and store alike. The rule is at held_plan.
+constexpr int kHeldThreads = 512, kHeldWarps = kHeldThreads / 32, kHeldBytes = 104 * 1024;
+
+__device__ __forceinline__ void unpack8(const uint4& u, float (&v)[8]) {
+  const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+  for (int i = 0; i < 4; i++) { const float2 f = __bfloat1622float2(b[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
+}
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+  uint4 u;
+  __nv_bfloat162* b = reinterpret_cast<__nv_bfloat162*>(&u);
+#pragma unroll
+  for (int i = 0; i < 4; i++) b[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+  return u;
+}
+// The sums of a cluster's channels: a thread's of its 8, over the warp, the CTA and, in double, the cluster's CTAs, always in the same order.
+// Thread c < CH has channel c's. The other CTAs' `mine` is read until the barrier that this arrives at completes.
+template <int CH>
+__device__ __forceinline__ void cluster_fold(cooperative_groups::cluster_group& cluster, float (&s)[8], float (&q)[8], float (&fold)[kHeldWarps][CH / 8][16],
+                                             float (&mine)[2][CH], double& s_out, double& q_out) {
+  constexpr int CHUNKS = CH / 8;
+  const int tid = threadIdx.x, lane = tid & 31;
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+#pragma unroll
+    for (int d = CHUNKS; d < 32; d *= 2) { s[i] += __shfl_xor_sync(0xffffffffu, s[i], d); q[i] += __shfl_xor_sync(0xffffffffu, q[i], d); }
+  if (lane < CHUNKS) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) { fold[tid >> 5][lane][i] = s[i]; fold[tid >> 5][lane][8 + i] = q[i]; }
+  }
+  __syncthreads();
+  if (tid < 2 * CH) {
+    const int k = tid / CH, c = tid % CH;
+    float a = 0;
+#pragma unroll
+    for (int w = 0; w < kHeldWarps; w++) a += fold[w][c >> 3][k * 8 + (c & 7)];
+    mine[k][c] = a;
+  }
+  cluster.sync();
+  s_out = q_out = 0;
+  if (tid < CH) {
+    const int size = (int)cluster.num_blocks();
+    for (int j = 0; j < size; j++) {
+      const float* const other = cluster.map_shared_rank(&mine[0][0], j);
+      s_out += other[tid];
+      q_out += other[CH + tid];
+    }
+  }
+}
+
+template <int CH, bool ADD, int RELU>
+__global__ void __launch_bounds__(kHeldThreads, 2)
+held_fwd_kernel(const bf16* x, const bf16* residual, bf16* __restrict__ y, uint8_t* __restrict__ mask, const float* gamma, const float* beta,
+                float* __restrict__ stats, float* run_mean, float* run_var, int R, int C, float eps, float momentum) {
+  constexpr int CHUNKS = CH / 8, LANES = kHeldThreads / CHUNKS;
+  extern __shared__ uint4 held[];                           // [rows][CHUNKS]
+  __shared__ float fold[kHeldWarps][CHUNKS][16], mine[2][CH], affine[2][CH];
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int size = (int)cluster.num_blocks(), rank = (int)cluster.block_rank(), tid = threadIdx.x, chunk = tid % CHUNKS, row = tid / CHUNKS;
+  const int c0 = (int)(blockIdx.x / size) * CH, rows = (int)((int64_t)R * (rank + 1) / size - (int64_t)R * rank / size);
+  const size_t at = ((int64_t)R * rank / size) * C + c0 + chunk * 8;
+  float s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  pdl_wait();
+#pragma unroll 4
+  for (int r = row; r < rows; r += LANES) {
+    const uint4 u = *reinterpret_cast<const uint4*>(x + at + (size_t)r * C);
+    held[r * CHUNKS + chunk] = u;
+    float v[8];
+    unpack8(u, v);
+#pragma unroll
+    for (int i = 0; i < 8; i++) { s[i] += v[i]; q[i] += v[i] * v[i]; }
+  }
+  double sum, sq;
+  cluster_fold<CH>(cluster, s, q, fold, mine, sum, sq);
+  if (tid < CH) {
+    const int c = c0 + tid;
+    const double mu = sum / (double)R;
+    double var = sq / (double)R - mu * mu;
+    if (var < 0) var = 0;
+    const float rs = rsqrtf((float)var + eps), sc = gamma[c] * rs, sh = beta[c] - (float)mu * sc;
+    affine[0][tid] = sc; affine[1][tid] = sh;
+    if (rank == 0) {
+      stats[c] = (float)mu; stats[C + c] = rs; stats[2 * C + c] = sc; stats[3 * C + c] = sh;
+      if (run_mean) {
+        const double unbiased = R > 1 ? var * (double)R / (double)(R - 1) : var;
+        run_mean[c] = (1.0f - momentum) * run_mean[c] + momentum * (float)mu;
+        run_var[c] = (1.0f - momentum) * run_var[c] + momentum * (float)unbiased;
+      }
+    }
+  }
+  cluster.barrier_arrive();
+  __syncthreads();
+  pdl_trigger();
+  float sc[8], sh[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) { sc[i] = affine[0][chunk * 8 + i]; sh[i] = affine[1][chunk * 8 + i]; }
+#pragma unroll 4
+  for (int r = row; r - row < rows; r += LANES) {
+    const bool there = r < rows;
+    float v[8];
+    if (there) {
+      unpack8(held[r * CHUNKS + chunk], v);
+#pragma unroll
+      for (int i = 0; i < 8; i++) v[i] = v[i] * sc[i] + sh[i];
+      if (ADD) {
+        float w[8];
+        load8(residual + at + (size_t)r * C, w);
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] += w[i];
+      }
+    }
+    if (RELU) {
+      uint32_t bits = 0;
+      if (there) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) { bits |= (v[i] > 0.0f ? 1u : 0u) << i; v[i] = fmaxf(v[i], 0.0f); }
+      }
+      if (RELU == 2) {                                      // a row's bytes together
+        bits <<= 8 * chunk;
+#pragma unroll
+        for (int d = 1; d < CHUNKS; d *= 2) bits |= __shfl_xor_sync(0xffffffffu, bits, d);
+        if (there && chunk == 0) {
+          uint8_t* const m = mask + (at + (size_t)r * C) / 8;
+          if (CHUNKS == 4) *reinterpret_cast<uint32_t*>(m) = bits; else *reinterpret_cast<uint16_t*>(m) = (uint16_t)bits;
+        }
+      }
+    }
+    if (there) *reinterpret_cast<uint4*>(y + at + (size_t)r * C) = pack8(v);
+  }
+  cluster.barrier_wait();
+}
+
+template <int CH, bool TWO, bool RELU, bool OUT>
+__global__ void __launch_bounds__(kHeldThreads, 2)
+held_bwd_kernel(const bf16* dy, const bf16* dy2, const uint8_t* mask, const bf16* x, const float* gamma, const float* stats, bf16* __restrict__ dx,
+                bf16* __restrict__ gmask_out, float* __restrict__ dgamma, float* __restrict__ dbeta, int R, int C, int most) {
+  constexpr int CHUNKS = CH / 8, LANES = kHeldThreads / CHUNKS;
+  extern __shared__ uint4 held[];                           // the masked gradient and x: [most][CHUNKS] each
+  __shared__ float fold[kHeldWarps][CHUNKS][16], mine[2][CH], affine[2][CH];
+  uint4* const held_x = held + most * CHUNKS;
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int size = (int)cluster.num_blocks(), rank = (int)cluster.block_rank(), tid = threadIdx.x, chunk = tid % CHUNKS, row = tid / CHUNKS;
+  const int c0 = (int)(blockIdx.x / size) * CH, rows = (int)((int64_t)R * (rank + 1) / size - (int64_t)R * rank / size);
+  const size_t at = ((int64_t)R * rank / size) * C + c0 + chunk * 8;
+  float mu[8], rs[8], s[8] = {0, 0, 0, 0, 0, 0, 0, 0}, q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  pdl_wait();
+#pragma unroll
+  for (int i = 0; i < 8; i++) { mu[i] = stats[c0 + chunk * 8 + i]; rs[i] = stats[C + c0 + chunk * 8 + i]; }
+#pragma unroll (TWO ? 2 : 4)
+  for (int r = row; r < rows; r += LANES) {
+    const size_t off = at + (size_t)r * C;
+    uint4 gu = *reinterpret_cast<const uint4*>(dy + off);
+    const uint4 xu = *reinterpret_cast<const uint4*>(x + off);
+    held_x[r * CHUNKS + chunk] = xu;
+    float gv[8], xv[8];
+    unpack8(gu, gv);
+    unpack8(xu, xv);
+    if (TWO) {
+      float w[8];
+      load8(dy2 + off, w);
+#pragma unroll
+      for (int i = 0; i < 8; i++) gv[i] += w[i];
+    }
+    if (RELU) {
+      const uint32_t bits = mask[off / 8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) gv[i] = (bits >> i) & 1u ? gv[i] : 0.0f;
+    }
+    if (TWO || RELU) gu = pack8(gv);
+    if (OUT) *reinterpret_cast<uint4*>(gmask_out + off) = gu;
+    held[r * CHUNKS + chunk] = gu;
+#pragma unroll
+    for (int i = 0; i < 8; i++) { s[i] += gv[i]; q[i] += gv[i] * (xv[i] - mu[i]) * rs[i]; }
+  }
+  double sum, dot;
+  cluster_fold<CH>(cluster, s, q, fold, mine, sum, dot);
+  if (tid < CH) {
+    affine[0][tid] = (float)sum; affine[1][tid] = (float)dot;
+    if (rank == 0) { dbeta[c0 + tid] = (float)sum; dgamma[c0 + tid] = (float)dot; }
+  }
+  cluster.barrier_arrive();
+  __syncthreads();
+  pdl_trigger();
+  float k0[8], k1[8], k2[8];
+  const float invR = 1.0f / (float)R;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    k0[i] = gamma[c0 + chunk * 8 + i] * rs[i];
+    k1[i] = affine[0][chunk * 8 + i] * invR;
+    k2[i] = affine[1][chunk * 8 + i] * invR;
+  }
+#pragma unroll 4
+  for (int r = row; r < rows; r += LANES) {
+    float gv[8], xv[8];
+    unpack8(held[r * CHUNKS + chunk], gv);
+    unpack8(held_x[r * CHUNKS + chunk], xv);
+#pragma unroll
+    for (int i = 0; i < 8; i++) gv[i] = k0[i] * (gv[i] - k1[i] - (xv[i] - mu[i]) * rs[i] * k2[i]);
+    *reinterpret_cast<uint4*>(dx + at + (size_t)r * C) = pack8(gv);
+  }
+  cluster.barrier_wait();
+}
+
 // the form of a sweep for the operands that a call has
 inline auto apply_for(const void* residual, const void* mask, int relu) {
   const int form = relu ? (mask ? 2 : 1) : 0;
@@ -290,6 +501,90 @@ inline int grid_for(int64_t R, int C) {
   if (g > 148 * kSweepCtas) g = 148 * kSweepCtas;
   return (int)(g < 1 ? 1 : g);
 }
+// Whether clusters of sixteen CTAs can be scheduled on the device (more than a program may count on).
+inline bool wide_clusters() {
+  static std::atomic<int> held[64];                         // by device: 0 not asked yet, 1 no, 2 yes
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return false;
+  int v = held[dev].load(std::memory_order_relaxed);
+  if (!v) {
+    const auto kernel = held_bwd_kernel<32, true, true, true>;
+    int n = 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(16); cfg.blockDim = dim3(kHeldThreads); cfg.dynamicSmemBytes = kHeldBytes;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 16; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeldBytes) == cudaSuccess &&
+                    cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0;
+    if (!ok) cudaGetLastError();
+    held[dev].store(v = ok ? 2 : 1, std::memory_order_relaxed);
+  }
+  return v == 2;
+}
+
+// How a call that holds `tensors` tensors of R x C is laid out: `ch` channels to a cluster (0: it takes the three launches), `cluster` CTAs, bytes
+// per CTA. extra: it reads or writes another tensor besides (a residual, a second gradient, the residual's gradient).
+// All clusters are resident at once, with 64 CTAs at least to fetch for, and small clusters before large ones: sixteen CTAs have to find room in
+// one part of the GPU, so of those no more than 128. Shares of 52 KB leave two CTAs on an SM room to work while the other one waits. us, three launches, one:
+// forward and backward of 784 x 2048 12.2, 6.0 and 16.2, 6.0; 3136 x 512 10.8, 6.0 and 14.6, 7.8; 12544 x 128 9.8, 6.4 and 11.5, 8.7; 3136 x 2048
+// 19.7, 10.2 and 23.8, 17.5; forward of 12544 x 512 18.2, 13.6, with ReLU and residual 18.1, 19.7. Outside: forward of 25088 x 256 with
+// ReLU 17.6, 18.4, of 50176 x 256 22.3, 29.6, backward of 12544 x 512 22.2, 22.7, of 12544 x 1024 33.2, 41.8, of 6272 x 1024 with all operands 25.2, 25.6.
+struct HeldPlan { int ch, cluster; size_t bytes; };
+constexpr int kHeldFew = 52 * 1024;
+inline HeldPlan held_plan(int64_t R, int C, int tensors, bool extra) {
+  if (R > 0x7fffffff) return {0, 0, 0};
+  for (const int most : {kHeldFew, kHeldBytes}) {
+    if (most == kHeldBytes && extra) break;
+    for (const int ch : {32, 16}) {
+      if (C % ch || (ch == 16 && most == kHeldBytes)) continue;
+      for (int cluster = 1; cluster <= 16; cluster *= 2) {
+        const int64_t ctas = (int64_t)C / ch * cluster, bytes = (R + cluster - 1) / cluster * ch * 2 * tensors;
+        const int many = cluster < 16 ? 296 : most == kHeldBytes && tensors == 1 ? 64 : 128;
+        if (ctas >= 64 && ctas <= many && bytes <= (ch == 16 && extra ? 40 * 1024 : most) && (cluster < 16 || wide_clusters()))
+          return {ch, cluster, (size_t)bytes};
+      }
+    }
+  }
+  return {0, 0, 0};
+}
+template <class... K, class... A> cudaError_t launch_ex(const cudaLaunchConfig_t& cfg, void (*kernel)(K...), A... args) {
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+template <auto kKernel, class... A>
+int launch_held(const HeldPlan& p, int C, cudaStream_t s, A... args) {
+  static std::atomic<bool> done[64];                        // by device
+  int dev = 0, e = (int)cudaGetDevice(&dev);
+  if (!e && (dev >= 64 || !done[dev].load(std::memory_order_relaxed))) {
+    e = (int)cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeldBytes);
+    if (!e) e = (int)cudaFuncSetAttribute(kKernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (!e && dev < 64) done[dev].store(true, std::memory_order_relaxed);
+  }
+  if (e) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(C / p.ch * p.cluster); cfg.blockDim = dim3(kHeldThreads); cfg.dynamicSmemBytes = p.bytes; cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  static const bool pdl = [] { const char* v = getenv("GCOW_PDL"); return !(v && v[0] == '0'); }();
+  cfg.attrs = attr; cfg.numAttrs = pdl ? 2 : 1;
+  return (int)launch_ex(cfg, kKernel, args...);
+}
+template <int CH, class... A> int held_fwd(bool add, int form, const HeldPlan& p, int C, cudaStream_t s, A... args) {   // form: as RELU
+  if (add) return form == 2 ? launch_held<held_fwd_kernel<CH, true, 2>>(p, C, s, args...) : form == 1 ? launch_held<held_fwd_kernel<CH, true, 1>>(p, C, s, args...)
+                                                                                                  : launch_held<held_fwd_kernel<CH, true, 0>>(p, C, s, args...);
+  return form == 2 ? launch_held<held_fwd_kernel<CH, false, 2>>(p, C, s, args...) : form == 1 ? launch_held<held_fwd_kernel<CH, false, 1>>(p, C, s, args...)
+                                                                                              : launch_held<held_fwd_kernel<CH, false, 0>>(p, C, s, args...);
+}
+template <int CH, class... A> int held_bwd(bool two, bool out, bool relu, const HeldPlan& p, int C, cudaStream_t s, A... args) {
+  if (two) return relu ? launch_held<held_bwd_kernel<CH, true, true, true>>(p, C, s, args...) : launch_held<held_bwd_kernel<CH, true, false, true>>(p, C, s, args...);
+  if (out) return relu ? launch_held<held_bwd_kernel<CH, false, true, true>>(p, C, s, args...) : launch_held<held_bwd_kernel<CH, false, false, true>>(p, C, s, args...);
+  return relu ? launch_held<held_bwd_kernel<CH, false, true, false>>(p, C, s, args...) : launch_held<held_bwd_kernel<CH, false, false, false>>(p, C, s, args...);
+}
 inline bool shape_ok(int C) { return C % 8 == 0 && C >= 8 && C <= 2048 && kThreads % (C / 8) == 0; }
 
 }  // namespace bn
@@ -300,9 +595,12 @@ using namespace gcow::bn;
 extern "C" {
 
 int gcow_bn_supported(int C) { return shape_ok(C) ? 1 : 0; }
+// Kernels that a training call launches: one (`part` is not used), or two sweeps with the sums' second half between them.
+// extra: a residual forward, the residual's gradient backward.
+int gcow_bn_launches(int64_t R, int C, int backward, int extra) { return shape_ok(C) && held_plan(R, C, backward ? 2 : 1, extra != 0).ch ? 1 : 3; }
 int gcow_bn_parts(int64_t R, int C) { return shape_ok(C) ? grid_for(R, C) : 0; }
 
-// Training forward. part: gcow_bn_parts * 2 * C floats of scratch. stats: 4*C floats out
+// Training forward. part: gcow_bn_parts * 2 * C floats of scratch, or null where gcow_bn_launches says 1 (and mask is at a multiple of 4 bytes). stats: 4*C floats out
 // (mean, rstd, scale, shift). run_mean/run_var may be null. mask: R*C/8 bytes out (ReLU
 // outcome, one bit per element), required when relu != 0 and a backward pass will follow.
 int gcow_bn_fwd_train(const void* x, const void* residual, void* y, void* mask, const float* gamma, const float* beta,
@@ -310,6 +608,16 @@ int gcow_bn_fwd_train(const void* x, const void* residual, void* y, void* mask, 
                       float momentum, int relu, void* stream) {
   if (!shape_ok(C) || R <= 0) return -1;
   cudaStream_t s = (cudaStream_t)stream;
+  const HeldPlan plan = held_plan(R, C, 1, residual != nullptr);
+  if (plan.ch && ((uintptr_t)mask & 3) == 0) {
+    const int form = relu ? (mask ? 2 : 1) : 0;
+    auto run = [&](auto ch) {
+      return held_fwd<ch.value>(residual != nullptr, form, plan, C, s, (const bf16*)x, (const bf16*)residual, (bf16*)y, (uint8_t*)mask, gamma, beta, stats,
+                                run_mean, run_var, (int)R, C, eps, momentum);
+    };
+    return plan.ch == 32 ? run(std::integral_constant<int, 32>()) : run(std::integral_constant<int, 16>());
+  }
+  if (!part) return -1;
   const int g = grid_for(R, C);
   float *mean = stats, *rstd = stats + C, *scale = stats + 2 * C, *shift = stats + 3 * C;
   gcow::launch_dependent(stats_kernel, dim3(g), dim3(kThreads), 0, s, (const bf16*)x, part, R, C);
@@ -341,6 +649,15 @@ int gcow_bn_bwd3(const void* dy, const void* dy2, const void* mask, const void* 
                  void* dx, void* dres, float* dgamma, float* dbeta, float* part, int64_t R, int C, int relu, void* stream) {
   if (!shape_ok(C) || R <= 0 || (dy2 && !dres)) return -1;
   cudaStream_t s = (cudaStream_t)stream;
+  const HeldPlan plan = held_plan(R, C, 2, dres != nullptr);
+  if (plan.ch) {
+    auto run = [&](auto ch) {
+      return held_bwd<ch.value>(dy2 != nullptr, dres != nullptr, relu != 0, plan, C, s, (const bf16*)dy, (const bf16*)dy2, (const uint8_t*)mask, (const bf16*)x,
+                                gamma, stats, (bf16*)dx, (bf16*)dres, dgamma, dbeta, (int)R, C, (int)((R + plan.cluster - 1) / plan.cluster));
+    };
+    return plan.ch == 32 ? run(std::integral_constant<int, 32>()) : run(std::integral_constant<int, 16>());
+  }
+  if (!part) return -1;
   const int g = grid_for(R, C);
   const float *mean = stats, *rstd = stats + C;
   gcow::launch_dependent(bwd_reduce_for(dy2, dres, relu), dim3(g), dim3(kThreads), 0, s, (const bf16*)dy, (const bf16*)dy2, (const uint8_t*)mask,

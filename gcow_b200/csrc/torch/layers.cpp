@@ -56,6 +56,7 @@ int gcow_attention_bwd(const void* qkv, const void* out, const void* dout, const
 int gcow_softmax_fwd(const void* x, void* y, int64_t rows, int S, float scale, void* stream);
 int gcow_softmax_bwd(const void* dp, const void* p, void* ds, int64_t rows, int S, float scale, void* stream);
 int gcow_bn_parts(int64_t R, int C);
+int gcow_bn_launches(int64_t R, int C, int backward, int extra);
 int gcow_bn_fwd_train(const void* x, const void* residual, void* y, void* mask, const float* gamma, const float* beta, float* run_mean,
                       float* run_var, float* stats, float* part, int64_t R, int C, float eps, float momentum, int relu, void* stream);
 int gcow_bn_bwd3(const void* dy, const void* dy2, const void* mask, const void* x, const float* gamma, const float* stats, void* dx,
@@ -1005,7 +1006,8 @@ struct BatchNormNode : LayerNode {                          // inputs: x, gamma,
     // the masked (summed) gradient: the residual input's gradient, and what the second sweep reads
     Tensor dres;
     if (has_res || gy2.defined()) dres = empty_nhwc(x.size(0), C, x.size(2), x.size(3), x);
-    const Tensor part = empty({(int64_t)gcow_bn_parts(R, (int)C) * 2 * C}, at::kFloat, x);
+    const int launches = gcow_bn_launches(R, (int)C, 1, dres.defined());
+    const Tensor part = launches > 1 ? empty({(int64_t)gcow_bn_parts(R, (int)C) * 2 * C}, at::kFloat, x) : Tensor();
     // dgamma and dbeta go straight into the two parameters' gradient tensors when the trainer pointed at them
     Tensor dgamma, dbeta, flat_g = target_matrix(target[0], 1, C, 4, &dgamma), flat_b;
     if (flat_g.defined()) flat_b = target_matrix(target[1], 1, C, 4, &dbeta);
@@ -1022,7 +1024,7 @@ struct BatchNormNode : LayerNode {                          // inputs: x, gamma,
     }
     check(gcow_bn_bwd3(gy.data_ptr(), raw(gy2), raw(mask), x.data_ptr(), f32(g32), f32(stats), dx.data_ptr(), raw(dres), pg, pb, f32(part),
                        R, (int)C, relu, on.stream), "gcow_bn_bwd3");
-    g_launches += 3;
+    g_launches += launches;
     out[0] = std::move(dx);
     out[1] = flat_b.defined() ? dgamma : dgamma.to(ptype);
     out[2] = flat_b.defined() ? dbeta : dbeta.to(ptype);
@@ -1058,12 +1060,14 @@ PyObject* batchnorm_act(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const On on(x);
     const int64_t C = x.size(1), R = x.size(0) * x.size(2) * x.size(3);
     y = empty_nhwc(x.size(0), C, x.size(2), x.size(3), x);
-    const Tensor stats = empty({4 * C}, at::kFloat, x), part = empty({(int64_t)gcow_bn_parts(R, (int)C) * 2 * C}, at::kFloat, x);
+    const int launches = gcow_bn_launches(R, (int)C, 0, res.defined());
+    const Tensor stats = empty({4 * C}, at::kFloat, x),
+                 part = launches > 1 ? empty({(int64_t)gcow_bn_parts(R, (int)C) * 2 * C}, at::kFloat, x) : Tensor();
     const Tensor g32 = float_vector(gamma), b32 = float_vector(beta);
     const Tensor mask = relu ? empty({R * C / 8}, at::kByte, x) : Tensor();
     check(gcow_bn_fwd_train(x.data_ptr(), raw(res), y.data_ptr(), raw(mask), f32(g32), f32(b32), f32(rm), f32(rv), f32(stats), f32(part), R,
                             (int)C, (float)eps, (float)momentum, relu, on.stream), "gcow_bn_fwd_train");
-    g_launches += 3;
+    g_launches += launches;
     if (node) {                                             // the ReLU bit mask stands in for y in the backward
       node->kept[0].set(x);
       node->kept[1].set(g32);

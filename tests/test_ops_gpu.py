@@ -1,4 +1,6 @@
 """Own training kernels against fp32 PyTorch references of the same op."""
+import ctypes as C_
+
 import pytest
 import torch
 import torch.nn.functional as F
@@ -560,6 +562,29 @@ def test_batchnorm_every_form_of_the_sweeps(N, C, H, W, res, relu, fork):
         z = (xd - col(bn.running_mean)) / (col(bn.running_var) + bn.eps).sqrt() * ga + col(bn.bias.detach()) + (r0.double() if res else 0)
         want = z.clamp(min=0) if relu else z
         assert ((bn(x0, residual=r0 if res else None, relu=relu).double() - want).abs() <= 2**-8 * want.abs() + 1e-4).all()
+
+
+# Fewer rows than CTAs in a cluster, one CTA a cluster, clusters of 2 to 16, channels by 32 and by 16, shares of rows that differ by one, shares just
+# within 52 KB and 104 KB and just beyond
+@pytest.mark.parametrize("N,C,H,W", [(1, 64, 1, 3), (1, 2048, 1, 1), (3, 2048, 7, 7), (17, 512, 7, 7), (13, 1024, 9, 11), (1, 128, 111, 113), (1, 128, 111, 121),
+                                     (1, 256, 107, 61), (1, 64, 101, 259), (1, 2048, 61, 109), (1, 2048, 33, 50)])
+@pytest.mark.parametrize("res,relu,fork", [(False, False, False), (False, True, False), (True, True, True), (True, False, False), (True, True, False), (False, True, True)])
+def test_batchnorm_of_tensors_held_in_shared_memory(N, C, H, W, res, relu, fork):
+    """The one-launch form against float64, its running statistics, and which form a shape takes."""
+    from gcow_b200 import _native
+    from gcow_b200.ops import nn as gnn
+    R, lib = N * H * W, _native.cuda()
+    lib.gcow_bn_launches.argtypes = [C_.c_int64, C_.c_int, C_.c_int, C_.c_int]
+    assert lib.gcow_bn_launches(R, C, 0, 0) == 1 or (N, C, H, W) in ((1, 256, 107, 61), (1, 2048, 61, 109))
+    test_batchnorm_every_form_of_the_sweeps(N, C, H, W, res, relu, fork)
+    x = torch.randn(N, C, H, W, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last)
+    bn = gnn.BatchNorm2d(C).cuda()
+    for _ in range(2):                                       # the second call finds the first one's sums in shared memory
+        bn(x, residual=x if res else None, relu=relu)
+    xd = x.double()
+    mean, var = xd.mean((0, 2, 3)), xd.var((0, 2, 3), unbiased=R > 1)
+    assert torch.allclose(bn.running_mean.double(), 0.19 * mean, rtol=1e-5, atol=1e-6)
+    assert torch.allclose(bn.running_var.double(), 0.81 + 0.19 * var, rtol=1e-5, atol=1e-6)
 
 
 def test_batchnorm_counts_training_steps_lazily():
