@@ -1196,7 +1196,7 @@ static int make_map_2d(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_
 // Pixel box bw x bh x bn covering a W x H x N grid with the fewest wasted rows.
 // `exact` != 0: the box must hold exactly `rows` pixels (wgrad: 64); else at most `rows`.
 // Ties go to the longer contiguous run (larger bw, then bh). Returns the fraction of fetched rows that are pixels.
-static double pick_box(int W, int H, int N, int rows, int exact, int* obw, int* obh, int* obn) {
+static double search_box(int W, int H, int N, int rows, int exact, int* obw, int* obh, int* obn) {
   double best = -1.0, best_eff = 0.0;
   *obw = 1; *obh = 1; *obn = rows > 256 ? 256 : rows;
   for (int bw = 1; bw <= rows && bw <= 256; bw++) {
@@ -1215,6 +1215,20 @@ static double pick_box(int W, int H, int N, int rows, int exact, int* obw, int* 
     }
   }
   return best_eff;
+}
+
+// The same from the thread's last searches. One takes 2 to 5 us of the host, a layer's forward and backward pass ask eight times (twenty with stride
+// 2), and a network's layers for the same few extents in every step: conv + BatchNorm of 256 channels at 14 x 14, 16 images, 171 -> 162 us, of 128 channels at 56 x 56 with stride 2, 40 images, 246 -> 191.
+static double pick_box(int W, int H, int N, int rows, int exact, int* obw, int* obh, int* obn) {
+  struct Found { int W, H, N, rows, exact, bw, bh, bn; double eff; };
+  static thread_local Found last[128];                      // zeros: no extents are
+  Found& f = last[((unsigned)W * 31u + (unsigned)H * 17u + (unsigned)N * 5u + (unsigned)rows / 64u * 3u + (unsigned)exact) % 128u];
+  if (f.W != W || f.H != H || f.N != N || f.rows != rows || f.exact != exact) {
+    f = {W, H, N, rows, exact, 0, 0, 0, 0.0};
+    f.eff = search_box(W, H, N, rows, exact, &f.bw, &f.bh, &f.bn);
+  }
+  *obw = f.bw; *obh = f.bh; *obn = f.bn;
+  return f.eff;
 }
 
 static size_t smem_for(int halves, int bn_cols, int stages) {
