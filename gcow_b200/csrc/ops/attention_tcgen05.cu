@@ -210,6 +210,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
 
   if (warp >= 8) {
     regs_issue<true>();
+    const bool one = elect_one();
     Phases ph;
     bool ok = true;
     auto wait = [&](int i, uint32_t code) {
@@ -232,7 +233,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
           if ((issued >> full) & 1u) wait(empty, 21);
           if (!ok) break;
           const int b = bh / p.H, h = bh - b * p.H;
-          if (lane == 0) {
+          if (one) {
             mbar_expect_tx(&bs->bar[full], TILE_BYTES);
             tma_load_4d(smem_u32(dst), is_q ? &tq : is_v ? &tv : &tk, smem_u32(&bs->bar[full]), 0, h, row, b);
           }
@@ -257,7 +258,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
             for (int i = 0; i < 2 * blocks && ok; i++) {
               const int op = i < blocks ? i : 4 + i - blocks;
               wait(kKvFull + op, 22);
-              if (ok && lane == 0) mbar_arrive(&bs->bar[kKvFree + op]);
+              if (ok && one) mbar_arrive(&bs->bar[kKvFree + op]);
               __syncwarp();
             }
           continue;
@@ -271,7 +272,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
           if (!ok) return;
           tc_fence_after();
           const uint64_t db = dk + i * (uint64_t)(TILE_BYTES >> 4);
-          if (lane == 0) {
+          if (one) {
 #pragma unroll
             for (int k = 0; k < 4; k++) tc_mma(col_s(x), dq + 2 * k, db + 2 * k, id_qk, k != 0);
             tc_commit(&bs->bar[kSFull + x]);
@@ -292,7 +293,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
           if (!ok) break;
           tc_fence_after();
           const uint64_t db = dv + i * (uint64_t)(TILE_BYTES >> 4);
-          if (lane == 0) {
+          if (one) {
 #pragma unroll
             for (int k = 0; k < 8; k++) tc_mma_ts(col_o(x), col_p(x) + 8 * k, db + (2048 >> 4) * k, id_pv, k != 0 || j != 1);
             tc_commit(&bs->bar[kPv + x]);
@@ -301,7 +302,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ 
           __syncwarp();
         }
       }
-      if (lane == 0) drain(&bs->bar[kFwdDrain + x]);
+      if (one) drain(&bs->bar[kFwdDrain + x]);
     }
   } else {
     // ---- softmax and output: one query per thread
@@ -528,6 +529,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& ta1, const CUte
 
   if (warp >= 8) {
     regs_issue<false>();
+    const bool one = elect_one();
     Phases ph;
     bool ok = true;
     auto wait = [&](int i, uint32_t code) {
@@ -552,7 +554,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& ta1, const CUte
           if (!ok) break;
           const int b = bh / p.H, h = bh - b * p.H;
           const bool arms = !is_a || !which;                 // one barrier for both operands of a tile
-          if (lane == 0) {
+          if (one) {
             if (arms) mbar_expect_tx(&bs->bar[full], is_a ? 2 * TILE_BYTES : TILE_BYTES);
             tma_load_4d(smem_u32(dst), is_a ? (which ? &ta2 : &ta1) : (which ? &tb2 : &tb1), smem_u32(&bs->bar[full]), 0, h, row, b);
           }
@@ -583,7 +585,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& ta1, const CUte
             for (int i = 0; i < tiles && ok; i++) {          // each warp waits for what it waits for in the other units
               if (scores) wait(kBFull + i, 32);
               if (scores != KV) wait(kBFull + 4 + i, 32);
-              if (ok && lane == 0) mbar_arrive(&bs->bar[kBFree + i]);
+              if (ok && one) mbar_arrive(&bs->bar[kBFree + i]);
               __syncwarp();
             }
           continue;
@@ -596,14 +598,14 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& ta1, const CUte
             if (!(i & 1)) {
               wait(kBFull + sl, 34);
               if (!KV) wait(kBFull + 4 + sl, 34);
-              if (KV && x && mode == kPair && ok && lane == 0) mbar_arrive(&bs->bar[kBFree + sl]);   // it is in use until the accumulators' products
+              if (KV && x && mode == kPair && ok && one) mbar_arrive(&bs->bar[kBFree + sl]);   // it is in use until the accumulators' products
             }
             if (held) wait(kSGone + x, 35);
             held = true;
             if (!ok) break;
             tc_fence_after();
             const uint64_t b1 = db1 + i * kStep, b2 = db2 + i * kStep;
-            if (lane == 0) {
+            if (one) {
 #pragma unroll
               for (int k = 0; k < 4; k++) {
                 tc_mma(tm, da1 + 2 * k, b1 + 2 * k, id_s, k != 0);
@@ -624,7 +626,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& ta1, const CUte
               wait(kReady + x, 37);
               if (!ok) break;
               tc_fence_after();
-              if (lane == 0) {
+              if (one) {
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
                   if (KV) tc_mma_ts(tm + ACC1, tm + P_AT + 8 * k, b2 + (2048 >> 4) * k, id_acc, k != 0 || i != 1);
@@ -640,7 +642,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& ta1, const CUte
               if (!ok) break;
               tc_fence_after();
               const uint64_t b2 = db2 + i * kStep;
-              if (lane == 0) {
+              if (one) {
 #pragma unroll
                 for (int k = 0; k < 4; k++) tc_mma(tm + DP, da2 + 2 * k, b2 + 2 * k, id_s, k != 0);
                 tc_commit(&bs->bar[kDpAt + x]);
@@ -651,7 +653,7 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& ta1, const CUte
           }
         }
       }
-      if (lane == 0) drain(&bs->drain[warp - 8]);
+      if (one) drain(&bs->drain[warp - 8]);
     } else if (KV && warp == 13) {                           // ---- statistics of the queries
       for (int u = u0, n = 0; u < u1 && ok; u++, n++) {
         const Unit un = unit_at(u, mode, tiles, heads);

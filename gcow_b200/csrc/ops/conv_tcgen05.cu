@@ -97,7 +97,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   // per-warp staging buffers of the epilogue, 16-byte aligned behind the barriers
   uint8_t* stage_base = reinterpret_cast<uint8_t*>(((uintptr_t)(sm + 1) + 15) & ~(uintptr_t)15);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp: uniform
   const int taps = p.kh * p.kw;
   const int cchunks = p.Ci / BK;
   const int pix_tiles = p.tiles_w * p.tiles_h * p.tiles_n;
@@ -146,7 +146,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t s = 0, phase = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
@@ -204,7 +204,7 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       // instruction descriptor: fp32 accumulate, bf16 x bf16, operand major-ness, N = bn_cols, M = 128
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)WGRAD << 15) | ((uint32_t)WGRAD << 16) |
                              ((uint32_t)(p.bn_cols >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
@@ -475,7 +475,7 @@ conv_ws_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   uint8_t* stage0 = base + WS_W_BYTES;
   WsSmem* sm = reinterpret_cast<WsSmem*>(stage0 + p.stages * p.stage_bytes);
   uint8_t* stage_base = reinterpret_cast<uint8_t*>(((uintptr_t)(sm + 1) + 15) & ~(uintptr_t)15);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp: uniform
   const int num_tiles = p.N * p.tiles_h;
   const int STAGES = p.stages;
 
@@ -499,7 +499,7 @@ conv_ws_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(&sm->wfull, (uint32_t)WS_W_BYTES);
       for (int tap = 0; tap < WS_TAPS; tap++)
         tma_load_2d(smem_u32(base + tap * 8192), &map_w, smem_u32(&sm->wfull), tap * 64, 0);
@@ -518,7 +518,7 @@ conv_ws_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.nslots >> 3) << 17) | ((64u >> 4) << 24);
       bool ok = mbar_wait_abortable(&sm->abort, &sm->wfull, 0, p.error, 5);
       tc_fence_after();
@@ -654,7 +654,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   uint8_t* bring = base + p.a_stages * a_stage_bytes;
   HaloSmem* sm = reinterpret_cast<HaloSmem*>(bring + p.b_stages * HALO_B_BYTES);
   uint8_t* stage_base = reinterpret_cast<uint8_t*>(((uintptr_t)(sm + 1) + 15) & ~(uintptr_t)15);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp: uniform
   const int num_tiles = p.N * p.tiles_h;
 
   if (threadIdx.x == 0) {
@@ -677,7 +677,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t a_tx = (uint32_t)(cchunks * p.pitch * (p.rows + 2)) * 128u;
       uint32_t sa = 0, pa = 0, sb = 0, pb = 0;
       bool ok = true;
@@ -708,7 +708,7 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.nslots >> 3) << 17) | ((128u >> 4) << 24);
       uint32_t sa = 0, pa = 0, sb = 0, pb = 0, t = 0;
       bool ok = true;
@@ -845,7 +845,7 @@ conv_wgrad_ws_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   WsSmem* sm = reinterpret_cast<WsSmem*>(base + WG_STAGES * WG_STAGE_BYTES);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp: uniform
   const int first = blockIdx.x * p.per;
   int last = first + p.per;
   if (last > p.num_tiles) last = p.num_tiles;
@@ -875,7 +875,7 @@ conv_wgrad_ws_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t s = 0, phase = 0;
       bool ok = true;
       for (int tile = first; tile < last && ok; tile++) {
@@ -892,7 +892,7 @@ conv_wgrad_ws_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       // fp32 accumulate, bf16 x bf16, both operands MN-major, N = 192, M = 128
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((192u >> 3) << 17) | ((128u >> 4) << 24);
       uint32_t s = 0, phase = 0, acc = 0;
@@ -976,7 +976,7 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
   uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int stage_bytes = 2 * p.x_chunk_bytes + 2 * p.dy_chunk_bytes;
   WsSmem* sm = reinterpret_cast<WsSmem*>(base + WG_STAGES * stage_bytes);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp: uniform
   const int first = blockIdx.x * p.per;
   int last = first + p.per;
   if (last > p.num_tiles) last = p.num_tiles;
@@ -1012,7 +1012,7 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t tx = 2u * (uint32_t)x_box + 2u * (uint32_t)(p.P * p.R * 128);
       uint32_t s = 0, phase = 0;
       bool ok = true;
@@ -1033,7 +1033,7 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((192u >> 3) << 17) | ((128u >> 4) << 24);
       const int ksteps = p.P * p.R / 16;
       uint32_t s = 0, phase = 0, acc = 0;

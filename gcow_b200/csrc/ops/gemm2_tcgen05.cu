@@ -51,13 +51,13 @@ struct Params {
   __nv_bfloat16* C;        // float* of a weight gradient
   const float* bias;
   const __nv_bfloat16* residual;
-  __nv_bfloat16* aux;
+  __nv_bfloat16* aux;      // float* of a weight gradient: [slices * tile columns][M] partial column sums of A, or null. (A field of their own
+                           // moves the others, and the epilogues spill: 16384 x 4096 x 1024 with a bias and a residual 133 -> 137 us.)
   int M, N, K, ldc, flags;
   int whole, items;        // items of work: `whole` 256 x 256 tiles (of every slice), then halves of 256 x 128
   int slice_blocks;        // stages per slice of the reduction
   int halves;              // weight gradient, an item per pair at most: a slice's two halves have an accumulator each
   size_t slice_stride;     // elements from one slice's result to the next
-  float* sums;             // of a weight gradient: [slices * tile columns][M] partial column sums of A, or null
   QuickTileOrder order;
   uint32_t* error;
 };
@@ -147,7 +147,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const int kblocks = (p.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
-    const uint32_t readers = A_MN && p.sums ? 1 + SUM_WARPS : 1;
+    const uint32_t readers = A_MN && p.aux ? 1 + SUM_WARPS : 1;
     for (int s = 0; s < STAGES; s++) { mbar_init(&sm->full[s], 1); mbar_init(&sm->empty[s], readers); mbar_init(&sm->landed[s], 1); }
     for (int a = 0; a < 2; a++) { mbar_init(&sm->tmem_full[a], 1); mbar_init(&sm->tmem_empty[a], 2 * EPI_WARPS * 32); }
     mbar_init(&sm->drain, 1);
@@ -170,7 +170,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t s = 0, phase = 0;
       bool ok = true;
       for (int i = pair; i < p.items && ok; i += pairs) {
@@ -197,6 +197,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer (CTA 0 only)
     if (rank == 0) {                                    // the warp keeps together, so that every operand is uniform; one lane issues
+      const bool one = elect_one();
       // instruction descriptor: fp32 accumulate, bf16 x bf16, operand major-ness, M 256 (128 rows per CTA), N 256 or 128
       const uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)A_MN << 15) | ((uint32_t)B_MN << 16) | ((uint32_t)(BM >> 4) << 24);
       uint32_t s = 0, phase = 0, t = 0;
@@ -217,8 +218,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           const uint32_t d_tmem = tmem_base + acc * BN + (A_MN && kb >= second ? BN : 0);
           const uint32_t sa = smem_u32(base + s * STAGE_BYTES), sb = sa + OPER_BYTES;
           const uint32_t eb0 = map_to_cta(smem_u32(&sm->empty[s]), 0), eb1 = map_to_cta(smem_u32(&sm->empty[s]), 1);
-          if (lane == 0) {
-            if (A_MN && p.sums) {                             // the warps that add up may read the stage too
+          if (one) {
+            if (A_MN && p.aux) {                              // the warps that add up may read the stage too
               mbar_arrive_cluster(map_to_cta(smem_u32(&sm->landed[s]), 0));
               mbar_arrive_cluster(map_to_cta(smem_u32(&sm->landed[s]), 1));
             }
@@ -236,7 +237,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           __syncwarp();
           if (++s == STAGES) { s = 0; phase ^= 1; }
         }
-        if (ok && lane == 0) {
+        if (ok && one) {
           const uint32_t fb = smem_u32(&sm->tmem_full[acc]);
           tc_commit_pair(map_to_cta(fb, 0));
           tc_commit_pair(map_to_cta(fb, 1));
@@ -244,7 +245,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         __syncwarp();
       }
       // drain: everything issued by this thread has finished before tensor memory is freed
-      if (lane == 0) {
+      if (one) {
         tc_commit_pair(map_to_cta(smem_u32(&sm->drain), 0));
         for (uint32_t it = 0; it < kSpinLimit; it++) if (mbar_try_wait(&sm->drain, 0)) break;
       }
@@ -258,7 +259,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     // own, with these, us, each with its ordered sums: 16384 rows to 3072 x 1024 85.9, 107.6, 86.5; to 4096 x 1024 99.4, 130.6, 101.5; to 768 x 768
     // 29.7, 39.1, 30.2; 1024 rows to 768 x 768 17.0, 19.6, 18.7; 16384 to 256 x 256, where a tile has all groups to itself, 14.6, 21.2, 18.6. Whole
     // stages in turn instead of groups of rows held a stage for longer than its MMAs: 16384 rows to 4096 x 1024 122.
-    if (p.sums) {
+    if (p.aux) {
       const int w = warp - 2 - EPI_WARPS, row = lane >> 3, chunk = lane & 7;
       const uint8_t* const mine = base + w * 16384 + row * 128;
       const int even = (chunk ^ row) * 16, odd = 512 + (chunk ^ (row + 4)) * 16;
@@ -304,7 +305,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         }
         const int m = it.m0 + (int)rank * 128 + w * 64 + chunk * 8;
         if (lane < 8 && m < p.M) {                            // M is a multiple of 64
-          float* const to = p.sums + (size_t)(it.slice * tiles_n + it.n0 / BN) * p.M + m;
+          float* const to = reinterpret_cast<float*>(p.aux) + (size_t)(it.slice * tiles_n + it.n0 / BN) * p.M + m;
           *reinterpret_cast<float4*>(to) = make_float4(sum[0], sum[1], sum[2], sum[3]);
           *reinterpret_cast<float4*>(to + 4) = make_float4(sum[4], sum[5], sum[6], sum[7]);
         }
@@ -663,7 +664,7 @@ int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, float* sums, in
   p.order = quick(tile_order(M, N, K, BM, BN));
   p.slice_stride = (size_t)M * N;
   p.halves = p.items <= max_pairs;
-  p.sums = sums;
+  p.aux = (__nv_bfloat16*)sums;
   return launch(gemm2_bf16_kernel<true, true, kNothing, false>, kThreads<true, kNothing, false>, max_pairs, ma, mb, mb, p, stream);
 }
 

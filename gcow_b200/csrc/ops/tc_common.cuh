@@ -17,6 +17,16 @@ constexpr uint32_t kSpinLimit = 1u << 26;   // polls before a wait gives up
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// True in one lane of the warp, which has to be converged. What a warp issues for all of its lanes - MMAs, commits, tensor copies - takes its
+// operands from uniform registers. Behind `lane == 0` the compiler has to assume several lanes with operands of their own and goes through them;
+// behind this it knows that there is one. Four MMAs and the sums for their descriptors take a warp 447 cycles there and 281 here (M128 N64,
+// whose MMAs take 128). Asked once per role: the same lane has to issue MMAs and the commits that track them.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
