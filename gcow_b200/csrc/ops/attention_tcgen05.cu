@@ -662,11 +662,22 @@ __device__ __forceinline__ void attn_bwd_body(const CUtensorMap& ta1, const CUte
         float* const st = stats + (n & 1) * 2 * MAX_S;
         // kHeads: one head's rows per 128. A query that does not exist has no probabilities (its rows of Q and dO are zeros).
         const int rows = mode == kHeads ? (un.both ? 2 * TILE : TILE) : tiles * TILE;
-        for (int r = lane; r < rows; r += 32) {
-          const int head = mode == kHeads ? un.bh[r >> 7] : un.bh[0], q = mode == kHeads ? r & (TILE - 1) : r;
-          const bool there = q < p.S;
-          st[r] = there ? -p.lse[(size_t)head * p.S + q] : -INFINITY;
-          st[MAX_S + r] = there ? -p.delta[(size_t)head * p.S + q] : 0.0f;
+        // Eight rows a lane under way at a time: one after the other they took longer than a unit, which waited for them.
+#pragma unroll 1
+        for (int r0 = lane; r0 < rows; r0 += 8 * 32) {
+          float l[8], d[8];
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            const int r = r0 + 32 * j, q = mode == kHeads ? r & (TILE - 1) : r;
+            const size_t at = (size_t)(mode == kHeads && r >= TILE ? un.bh[1] : un.bh[0]) * p.S + q;
+            l[j] = INFINITY;
+            d[j] = 0.0f;
+            if (r < rows && q < p.S) { l[j] = p.lse[at]; d[j] = p.delta[at]; }
+          }
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            if (r0 + 32 * j < rows) { st[r0 + 32 * j] = -l[j]; st[MAX_S + r0 + 32 * j] = -d[j]; }
+          }
         }
         mbar_arrive(&bs->bar[kStatFull + (n & 1)]);
       }
