@@ -622,10 +622,11 @@ conv_ws_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
 // ---------------------------------------------------------------------------------------------------------
 // Halo-tile forward for Ci -> 128 channels, 3x3, stride 1, padding 1 (Ci a multiple of 64): the same idea as the
 // weight-stationary kernel with the filter streamed instead of resident. The 128 output channels are the MMA's M,
-// the pixel slots (rows x (W + 2), rounded up to 16) its N. Per tile one halo box per 64-channel chunk of the input
-// (all chunks on one barrier) serves the nine taps; the filter tiles [128][64] of (chunk, tap) run through a ring
-// of their own. Against the general kernel (a 32 KB pixel box per tap and chunk) the pixel traffic from L2 falls
-// ninefold; the filter traffic per tile is the same.
+// the pixel slots (rows x (W + 2), rounded up to 16) its N. One halo box per 64-channel chunk of a tile's input serves the
+// nine taps; the filter pieces [128][64] of (chunk, tap) run through a ring of their own. Against the general kernel (a 32 KB
+// pixel box per tap and chunk) the pixel traffic from L2 falls ninefold; the filter traffic per tile is the same.
+// 128 -> 128 channels at 28 x 28, 256 images: 448 of 556 cycles per piece are its MMAs (M128 N224); with whole tiles' input in two stages and three
+// pieces in the ring 50.3 us, with three chunks and six pieces 46.9.
 struct HaloParams {
   __nv_bfloat16* out;   // [N, H, W, 128]
   const float* bias;
@@ -633,12 +634,12 @@ struct HaloParams {
   int pitch, rows, tiles_h;
   int nslots;           // N of the MMA: rows * pitch rounded up to 16
   int chunk_bytes;      // shared-memory region of one 64-channel chunk of a tile (1024-byte multiple)
-  int a_stages, b_stages;
+  int a_slots, b_stages;  // chunks of input and filter pieces in shared memory
   uint32_t* error;
 };
 
 struct HaloSmem {
-  uint64_t a_full[2], a_empty[2], b_full[8], b_empty[8], tmem_full[2], tmem_empty[2], drain;
+  uint64_t a_full[3], a_empty[3], b_full[8], b_empty[8], tmem_full[2], tmem_empty[2], drain;
   uint32_t tmem_base;
   volatile uint32_t abort;
 };
@@ -650,15 +651,14 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int cchunks = p.Ci / 64;
-  const int a_stage_bytes = cchunks * p.chunk_bytes;
-  uint8_t* bring = base + p.a_stages * a_stage_bytes;
+  uint8_t* bring = base + p.a_slots * p.chunk_bytes;
   HaloSmem* sm = reinterpret_cast<HaloSmem*>(bring + p.b_stages * HALO_B_BYTES);
   uint8_t* stage_base = reinterpret_cast<uint8_t*>(((uintptr_t)(sm + 1) + 15) & ~(uintptr_t)15);
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp: uniform
   const int num_tiles = p.N * p.tiles_h;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < 2; s++) { mbar_init(&sm->a_full[s], 1); mbar_init(&sm->a_empty[s], 1); }
+    for (int s = 0; s < 3; s++) { mbar_init(&sm->a_full[s], 1); mbar_init(&sm->a_empty[s], 1); }
     for (int s = 0; s < 8; s++) { mbar_init(&sm->b_full[s], 1); mbar_init(&sm->b_empty[s], 1); }
     for (int a = 0; a < 2; a++) { mbar_init(&sm->tmem_full[a], 1); mbar_init(&sm->tmem_empty[a], EPI_WARPS * 32); }
     mbar_init(&sm->drain, 1);
@@ -678,26 +678,27 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 
   if (warp == 0) {
     if (elect_one()) {
-      const uint32_t a_tx = (uint32_t)(cchunks * p.pitch * (p.rows + 2)) * 128u;
+      const uint32_t a_tx = (uint32_t)(p.pitch * (p.rows + 2)) * 128u;
       uint32_t sa = 0, pa = 0, sb = 0, pb = 0;
+      int tile_a = blockIdx.x, c_a = 0, visit = 0, due = 0, j = 0;   // the chunk to load next, and the piece that it goes before
       bool ok = true;
-      auto load_a = [&](int tile) {
-        const int n = tile / p.tiles_h, h0 = (tile - n * p.tiles_h) * p.rows;
+      // The first chunks go before the first pieces, a later one when its slot has just been left: the ring's pieces are taken in order, so where
+      // a piece can be loaded, the MMAs of the one b_stages before are done.
+      auto load_a = [&]() {
+        const int n = tile_a / p.tiles_h, h0 = (tile_a - n * p.tiles_h) * p.rows;
         if (!(ok = mbar_wait_abortable(&sm->abort, &sm->a_empty[sa], pa ^ 1, p.error, 1))) return;
         mbar_expect_tx(&sm->a_full[sa], a_tx);
-        for (int c = 0; c < cchunks; c++)
-          tma_load_4d(smem_u32(base + sa * a_stage_bytes + c * p.chunk_bytes), &map_x, smem_u32(&sm->a_full[sa]), c * 64, -1,
-                      h0 - 1, n);
-        if (++sa == (uint32_t)p.a_stages) { sa = 0; pa ^= 1; }
+        tma_load_4d(smem_u32(base + sa * p.chunk_bytes), &map_x, smem_u32(&sm->a_full[sa]), c_a * 64, -1, h0 - 1, n);
+        if (++sa == (uint32_t)p.a_slots) { sa = 0; pa ^= 1; }
+        if (++c_a == cchunks) { c_a = 0; tile_a += gridDim.x; }
+        visit++;
+        due = tile_a >= num_tiles ? 0x7fffffff : visit < p.a_slots ? visit * 6 : (visit - p.a_slots + 1) * WS_TAPS + p.b_stages;
       };
-      // the pixel tile of the next tile is requested in the middle of this tile's filter tiles
-      if (blockIdx.x < num_tiles) load_a(blockIdx.x);
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        for (int kb = 0; kb < cchunks * WS_TAPS && ok; kb++) {
-          // once the ring has wrapped within this tile the previous tile's MMAs are done and its pixel stage is free
-          if (kb == p.b_stages && tile + (int)gridDim.x < num_tiles) { load_a(tile + gridDim.x); if (!ok) break; }
+        for (int kb = 0; kb < cchunks * WS_TAPS; kb++, j++) {
+          if (j >= due) load_a();
           const int c = kb / WS_TAPS, tap = kb - c * WS_TAPS;
-          if (!(ok = mbar_wait_abortable(&sm->abort, &sm->b_empty[sb], pb ^ 1, p.error, 6))) break;
+          if (!ok || !(ok = mbar_wait_abortable(&sm->abort, &sm->b_empty[sb], pb ^ 1, p.error, 6))) break;
           mbar_expect_tx(&sm->b_full[sb], (uint32_t)HALO_B_BYTES);
           tma_load_2d(smem_u32(bring + sb * HALO_B_BYTES), &map_w, smem_u32(&sm->b_full[sb]), tap * p.Ci + c * 64, 0);
           if (++sb == (uint32_t)p.b_stages) { sb = 0; pb ^= 1; }
@@ -710,31 +711,34 @@ conv_halo_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   } else if (warp == 1) {
     if (elect_one()) {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.nslots >> 3) << 17) | ((128u >> 4) << 24);
+      const uint64_t ring = smem_desc_sw128(smem_u32(bring)), chunks = smem_desc_sw128(smem_u32(base));
       uint32_t sa = 0, pa = 0, sb = 0, pb = 0, t = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, t++) {
         const uint32_t buf = t & 1, use = t >> 1;
-        if (!(ok = mbar_wait_abortable(&sm->abort, &sm->a_full[sa], pa, p.error, 3))) break;
         if (!(ok = mbar_wait_abortable(&sm->abort, &sm->tmem_empty[buf], (use & 1) ^ 1, p.error, 2))) break;
-        tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * 256;
-        for (int kb = 0; kb < cchunks * WS_TAPS && ok; kb++) {
-          const int c = kb / WS_TAPS, tap = kb - c * WS_TAPS;
-          const int r = tap / 3, sx = tap - 3 * r;
-          if (!(ok = mbar_wait_abortable(&sm->abort, &sm->b_full[sb], pb, p.error, 7))) break;
-          tc_fence_after();
-          const uint64_t da = smem_desc_sw128(smem_u32(bring + sb * HALO_B_BYTES));
-          const uint64_t db = smem_desc_sw128(smem_u32(base + sa * a_stage_bytes + c * p.chunk_bytes) +
-                                              (uint32_t)(r * p.pitch + sx) * 128u);
+        for (int c = 0; c < cchunks && ok; c++) {
+          if (!(ok = mbar_wait_abortable(&sm->abort, &sm->a_full[sa], pa, p.error, 3))) break;
+          uint64_t db = chunks + sa * ((uint32_t)p.chunk_bytes >> 4);
+#pragma unroll 1
+          for (int r = 0; r < 3 && ok; r++, db += (uint32_t)p.pitch * 8) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; k++) tc_mma(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-          tc_commit(&sm->b_empty[sb]);
-          if (++sb == (uint32_t)p.b_stages) { sb = 0; pb ^= 1; }
+            for (int x = 0; x < 3; x++) {
+              if (!(ok = mbar_wait_abortable(&sm->abort, &sm->b_full[sb], pb, p.error, 7))) break;
+              tc_fence_after();
+              const uint64_t da = ring + sb * (HALO_B_BYTES >> 4);
+#pragma unroll
+              for (int k = 0; k < BK / UMMA_K; k++) tc_mma(d_tmem, da + 2 * k, db + 8 * x + 2 * k, idesc, (c | r | x | k) != 0);
+              tc_commit(&sm->b_empty[sb]);
+              if (++sb == (uint32_t)p.b_stages) { sb = 0; pb ^= 1; }
+            }
+          }
+          if (!ok) break;
+          tc_commit(&sm->a_empty[sa]);
+          if (++sa == (uint32_t)p.a_slots) { sa = 0; pa ^= 1; }
         }
-        if (!ok) break;
-        tc_commit(&sm->a_empty[sa]);
-        tc_commit(&sm->tmem_full[buf]);
-        if (++sa == (uint32_t)p.a_stages) { sa = 0; pa ^= 1; }
+        if (ok) tc_commit(&sm->tmem_full[buf]);
       }
       tc_commit(&sm->drain);
       for (uint32_t it = 0; it < kSpinLimit; it++) if (mbar_try_wait(&sm->drain, 0)) break;
@@ -965,7 +969,7 @@ struct WgHaloParams {
   int N, H, W, Ci, Co;
   int P, R;             // slot pitch, image rows per tile
   int tiles_h, num_tiles, per;
-  int x_chunk_bytes, dy_chunk_bytes;
+  int x_chunk_bytes, dy_chunk_bytes, stages;
   uint32_t* error;
 };
 
@@ -975,17 +979,17 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int stage_bytes = 2 * p.x_chunk_bytes + 2 * p.dy_chunk_bytes;
-  WsSmem* sm = reinterpret_cast<WsSmem*>(base + WG_STAGES * stage_bytes);
+  WsSmem* sm = reinterpret_cast<WsSmem*>(base + p.stages * stage_bytes);
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp: uniform
   const int first = blockIdx.x * p.per;
   int last = first + p.per;
   if (last > p.num_tiles) last = p.num_tiles;
   const int frow = blockIdx.y % 3;                // filter row of this CTA,
   const int cig = (blockIdx.y / 3) % (p.Ci / 128), cog = blockIdx.y / 3 / (p.Ci / 128);   // its 128 input and output channels
-  const int x_box = p.P * (p.R + 2) * 128;        // bytes of one X box; the bytes behind it up to x_chunk_bytes are zero
+  const int x_box = p.P * p.R * 128;              // bytes of one X box; the bytes behind it up to x_chunk_bytes are zero
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < WG_STAGES; s++) { mbar_init(&sm->full[s], 1); mbar_init(&sm->empty[s], 1); }
+    for (int s = 0; s < p.stages; s++) { mbar_init(&sm->full[s], 1); mbar_init(&sm->empty[s], 1); }
     mbar_init(&sm->tmem_full[0], 1);
     mbar_init(&sm->drain, 1);
     sm->abort = 0;
@@ -998,7 +1002,7 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
   // the last taps read a few slots behind each X box against zero dY: those bytes must hold finite numbers
   {
     const int pad16 = (p.x_chunk_bytes - x_box) / 16;
-    for (int i = threadIdx.x; i < WG_STAGES * 2 * pad16; i += blockDim.x) {
+    for (int i = threadIdx.x; i < p.stages * 2 * pad16; i += blockDim.x) {
       const int region = i / pad16, j = i - region * pad16;
       *reinterpret_cast<uint4*>(base + (region / 2) * stage_bytes + (region % 2) * p.x_chunk_bytes + x_box + j * 16) = make_uint4(0, 0, 0, 0);
     }
@@ -1023,10 +1027,10 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
         uint8_t* st = base + s * stage_bytes;
         const uint32_t bar = smem_u32(&sm->full[s]);
         for (int c = 0; c < 2; c++) {
-          tma_load_4d(smem_u32(st + c * p.x_chunk_bytes), &map_x, bar, cig * 128 + c * 64, -1, h0 - 1, n);
+          tma_load_4d(smem_u32(st + c * p.x_chunk_bytes), &map_x, bar, cig * 128 + c * 64, -1, h0 - 1 + frow, n);
           tma_load_4d(smem_u32(st + 2 * p.x_chunk_bytes + c * p.dy_chunk_bytes), &map_dy, bar, cog * 128 + c * 64, 0, h0, n);
         }
-        if (++s == WG_STAGES) { s = 0; phase ^= 1; }
+        if (++s == (uint32_t)p.stages) { s = 0; phase ^= 1; }
       }
       if (!ok) {
         for (int i = 0; i < 1000; i++) __nanosleep(1000);
@@ -1042,17 +1046,16 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
         if (!(ok = mbar_wait_abortable(&sm->abort, &sm->full[s], phase, p.error, 3))) break;
         tc_fence_after();
         const uint32_t xs = smem_u32(base + s * stage_bytes), ds = xs + 2 * p.x_chunk_bytes;
+        uint64_t da = smem_desc_mn_lbo(ds, (uint32_t)p.dy_chunk_bytes), d0 = smem_desc_mn_lbo(xs, 128u), d1 = smem_desc_mn_lbo(xs + p.x_chunk_bytes, 128u);
 #pragma unroll 1
         for (int k = 0; k < ksteps; k++) {
-          const uint32_t off = (uint32_t)k * 16u * 128u;
-          const uint64_t da = smem_desc_mn_lbo(ds + off, (uint32_t)p.dy_chunk_bytes);
-          const uint32_t xo = off + (uint32_t)(frow * p.P) * 128u;
-          tc_mma(tmem_base, da, smem_desc_mn_lbo(xs + xo, 128u), idesc, acc);
-          tc_mma(tmem_base + 192, da, smem_desc_mn_lbo(xs + p.x_chunk_bytes + xo, 128u), idesc, acc);
+          tc_mma(tmem_base, da, d0, idesc, acc);
+          tc_mma(tmem_base + 192, da, d1, idesc, acc);
           acc = 1;
+          da += 16 * 128 / 16; d0 += 16 * 128 / 16; d1 += 16 * 128 / 16;   // the next 16 slots
         }
         tc_commit(&sm->empty[s]);
-        if (++s == WG_STAGES) { s = 0; phase ^= 1; }
+        if (++s == (uint32_t)p.stages) { s = 0; phase ^= 1; }
       }
       if (ok) tc_commit(&sm->tmem_full[0]);
       tc_commit(&sm->drain);
@@ -1428,10 +1431,11 @@ static bool halo_plan(int N, int H, int W, int Ci, HaloParams* p) {
   if (best < 0) return false;
   p->tiles_h = (H + p->rows - 1) / p->rows;
   p->chunk_bytes = ((p->nslots + 2 * p->pitch + 2) * 128 + 1023) & ~1023;
-  p->a_stages = 2;
-  const int fixed = 1024 + (int)sizeof(HaloSmem) + 16 + EPI_WARPS * kStageWarpBytes;
-  const int left = kWsSmemMax - fixed - p->a_stages * (Ci / 64) * p->chunk_bytes;
-  p->b_stages = left / HALO_B_BYTES;
+  const int fixed = 1024 + (int)sizeof(HaloSmem) + 16 + EPI_WARPS * kStageWarpBytes, left = kWsSmemMax - fixed;
+  if ((left - 2 * (Ci / 64) * p->chunk_bytes) / HALO_B_BYTES < 3) return false;   // what two whole tiles' input left room for is what it takes
+  // Three chunks of a tile of two or more, the third one the next tile's first; what a fourth would take goes to the filter's ring.
+  p->a_slots = Ci > 64 ? 3 : 2;
+  p->b_stages = (left - p->a_slots * p->chunk_bytes) / HALO_B_BYTES;
   if (p->b_stages > 8) p->b_stages = 8;
   return p->b_stages >= 3;
 }
@@ -1455,7 +1459,7 @@ int gcow_conv_fwd_halo(const void* x, const void* w, void* y, const float* bias,
   if (rc) return rc;
   const long long tiles = (long long)N * p.tiles_h;
   const int grid = (int)(tiles < sms ? tiles : sms);
-  const size_t smem = 1024 + (size_t)p.a_stages * (Ci / 64) * p.chunk_bytes + (size_t)p.b_stages * HALO_B_BYTES +
+  const size_t smem = 1024 + (size_t)p.a_slots * p.chunk_bytes + (size_t)p.b_stages * HALO_B_BYTES +
                       sizeof(HaloSmem) + 16 + EPI_WARPS * kStageWarpBytes;
   gcow::launch_dependent(conv_halo_kernel, dim3(grid), dim3(THREADS), smem, (cudaStream_t)stream, mx, mw, p);
   return (int)cudaGetLastError();
@@ -1507,8 +1511,10 @@ static int wgrad_halo_plan(int N, int H, int W, int Ci, int Co, WgHaloParams* p)
   int groups = device_sms() / per_tile;
   if (groups < 1) groups = 1;
   p->per = (int)((tiles + groups - 1) / groups);
-  p->x_chunk_bytes = (p->P * (p->R + 2) * 128 + 256 + 1023) & ~1023;
+  p->x_chunk_bytes = (p->P * p->R * 128 + 256 + 1023) & ~1023;
   p->dy_chunk_bytes = p->P * p->R * 128;
+  p->stages = (kWsSmemMax - 1024 - (int)sizeof(WsSmem) - 64) / (2 * (p->x_chunk_bytes + p->dy_chunk_bytes));
+  if (p->stages > MAX_STAGES / 2) p->stages = MAX_STAGES / 2;
   return (int)((tiles + p->per - 1) / p->per);
 }
 
@@ -1526,11 +1532,11 @@ int gcow_conv_wgrad_halo(const void* dy, const void* x, float* part, int N, int 
   if (split <= 0 || ((uintptr_t)part & 15)) return -1;
   p.part = part; p.error = error;
   CUtensorMap mx, md;
-  int rc = make_map_nhwc(&mx, x, (uint64_t)N, (uint64_t)H, (uint64_t)W, (uint64_t)Ci, (uint32_t)p.P, (uint32_t)(p.R + 2), 1, 0);
+  int rc = make_map_nhwc(&mx, x, (uint64_t)N, (uint64_t)H, (uint64_t)W, (uint64_t)Ci, (uint32_t)p.P, (uint32_t)p.R, 1, 0);
   if (rc) return rc;
   rc = make_map_nhwc(&md, dy, (uint64_t)N, (uint64_t)H, (uint64_t)W, (uint64_t)Co, (uint32_t)p.P, (uint32_t)p.R, 1, 0);
   if (rc) return rc;
-  const size_t smem = 1024 + (size_t)WG_STAGES * (2 * p.x_chunk_bytes + 2 * p.dy_chunk_bytes) + sizeof(WsSmem) + 64;
+  const size_t smem = 1024 + (size_t)p.stages * (2 * p.x_chunk_bytes + 2 * p.dy_chunk_bytes) + sizeof(WsSmem) + 64;
   if (smem > (size_t)kWsSmemMax) return -1;
   gcow::launch_dependent(conv_wgrad_halo_kernel, dim3(split, 3 * (Ci / 128) * (Co / 128)), dim3(THREADS), smem, (cudaStream_t)stream, mx, md, p);
   return (int)cudaGetLastError();
