@@ -365,18 +365,17 @@ conv_igemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                                  row_off + n, row_ok);
             return;
           }
+          if (WGRAD && n + 32 <= n_limit) {
+            const size_t first = __shfl_sync(0xffffffffu, (unsigned long long)row_off, 0);
+            warp_store_rows_f32_halves(stage_base + ew * kStageWarpBytes, lane, r, reinterpret_cast<float*>(p.out) + first + n, (size_t)(col_groups * BK),
+                                       __popc(__ballot_sync(0xffffffffu, row_ok)));
+            return;
+          }
           if (row_ok && n < n_limit) {
             if (WGRAD) {
               float* C = reinterpret_cast<float*>(p.out) + row_off + n;
-              if (n + 32 <= n_limit) {
 #pragma unroll
-                for (int j = 0; j < 32; j += 4)
-                  *reinterpret_cast<float4*>(C + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
-                                                                  __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-              } else {
-#pragma unroll
-                for (int j = 0; j < 32; j++) if (n + j < n_limit) C[j] = __uint_as_float(r[j]);
-              }
+              for (int j = 0; j < 32; j++) if (n + j < n_limit) C[j] = __uint_as_float(r[j]);
             } else {
               float v[32];
 #pragma unroll
@@ -927,20 +926,16 @@ conv_wgrad_ws_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     ok = __all_sync(0xffffffffu, ok);
     if (ok && !(half == 1 && q >= 2)) {
       tc_fence_after();
-      const int row = q * 32 + lane;
-      const int co = row & 63;
-      const int r = half == 1 ? 2 : (row < 64 ? 1 : 0);        // filter row of this accumulator half
-      float* dst = p.part + ((size_t)blockIdx.x * 64 + co) * 576 + r * 192;
+      const int r = half == 1 ? 2 : (q < 2 ? 1 : 0);           // filter row of this accumulator half
+      float* dst = p.part + ((size_t)blockIdx.x * 64 + (q & 1) * 32) * 576 + r * 192;
+      uint8_t* const stg = base + ew * 4096;                  // the stages: every copy has landed and been read
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + half * 192;
 #pragma unroll 1
       for (int c = 0; c < 6; c++) {
         uint32_t v[32];
         tc_ld32(taddr + c * 32, v);
         tc_wait_ld();
-#pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(dst + c * 32 + j) = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
-                                                                     __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+        warp_store_rows_f32(stg, lane, v, dst + c * 32, 576, 32);
       }
     }
   }
@@ -1067,20 +1062,16 @@ conv_wgrad_halo_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
     ok = __all_sync(0xffffffffu, ok);
     if (ok) {
       tc_fence_after();
-      const int co = q * 32 + lane;
       // column c * 32 + j of this half is tap s = (c * 32 + j) / 64, input channel cig * 128 + half * 64 + (c * 32 + j) % 64
-      float* dst = p.part + ((size_t)blockIdx.x * p.Co + cog * 128 + co) * (size_t)(9 * p.Ci) + (size_t)frow * 3 * p.Ci + cig * 128 + half * 64;
+      float* dst = p.part + ((size_t)blockIdx.x * p.Co + cog * 128 + q * 32) * (size_t)(9 * p.Ci) + (size_t)frow * 3 * p.Ci + cig * 128 + half * 64;
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + half * 192;
+      uint8_t* const stg = base + ew * 4096;                  // the stages: every copy has landed and been read
 #pragma unroll 1
       for (int c = 0; c < 6; c++) {
         uint32_t v[32];
         tc_ld32(taddr + c * 32, v);
         tc_wait_ld();
-        float* o = dst + (c >> 1) * p.Ci + (c & 1) * 32;
-#pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(o + j) = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
-                                                          __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+        warp_store_rows_f32(stg, lane, v, dst + (c >> 1) * p.Ci + (c & 1) * 32, (size_t)(9 * p.Ci), 32);
       }
     }
   }

@@ -382,11 +382,11 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
             for (int j = 0; j < 32; j++) v[j] += __uint_as_float(other[j]);
           }
-          if (row_ok) {
-            float* const o = reinterpret_cast<float*>(p.C) + it.slice * p.slice_stride + off;
+          uint32_t o[32];
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-          }
+          for (int j = 0; j < 32; j++) o[j] = __float_as_uint(v[j]);
+          warp_store_rows_f32(stage_base + ew * 4096, lane, o, reinterpret_cast<float*>(p.C) + it.slice * p.slice_stride + (size_t)mw * p.ldc + n, p.ldc,
+                              p.M - mw);
           return;
         }
         if (p.flags & kBias) {

@@ -302,6 +302,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             warp_store_rows_bf16(stg, lane, v, reinterpret_cast<__nv_bfloat16*>(p.C), off, row_ok);
             return;
           }
+          const int mw = m0 + h * 128 + q * 32;
+          if ((p.flags & (kOutF32 | kBias | kGelu | kResidual | kAccumulate)) == kOutF32 && n + 32 <= p.N && mw < p.M) {   // a weight gradient
+            warp_store_rows_f32(stage_base + ew * 2 * kStageWarpBytes, lane, r, reinterpret_cast<float*>(p.C) + (size_t)bz * (size_t)p.stride_c + (size_t)mw * p.ldc + n,
+                                (size_t)p.ldc, p.M - mw);
+            return;
+          }
           if (m < p.M && n < p.N) {
             float v[32];
 #pragma unroll

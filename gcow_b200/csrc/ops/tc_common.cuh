@@ -222,6 +222,41 @@ __device__ __forceinline__ void warp_store_rows_bf16(uint8_t* stg, int lane, con
   __syncwarp();
 }
 
+// A warp's 32 x 32 fp32 block, a row per lane in r, to rows `ld` floats apart from `to` on, eight lanes a row, so that every store covers whole
+// 128-byte rows; `rows` of them exist. stg: 4 KB of the warp's own. A row per lane stored by its own lane is 32 lines an instruction and half
+// sectors.
+__device__ __forceinline__ void warp_store_rows_f32(uint8_t* stg, int lane, const uint32_t (&r)[32], float* to, size_t ld, int rows) {
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    *reinterpret_cast<uint4*>(stg + lane * 128 + ((k ^ (lane & 7)) << 4)) = make_uint4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int it = 0; it < 8; it++) {
+    const int row = it * 4 + (lane >> 3);
+    const uint4 x = *reinterpret_cast<const uint4*>(stg + row * 128 + (((lane & 7) ^ (row & 7)) << 4));
+    if (row < rows) *reinterpret_cast<uint4*>(to + (size_t)row * ld + (lane & 7) * 4) = x;
+  }
+}
+
+// The same with 2 KB, 16 columns and four lanes a row at a time.
+__device__ __forceinline__ void warp_store_rows_f32_halves(uint8_t* stg, int lane, const uint32_t (&r)[32], float* to, size_t ld, int rows) {
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      *reinterpret_cast<uint4*>(stg + stage_offset(lane, k)) = make_uint4(r[16 * h + 4 * k], r[16 * h + 4 * k + 1], r[16 * h + 4 * k + 2], r[16 * h + 4 * k + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int it = 0; it < 4; it++) {
+      const int row = it * 8 + (lane >> 2);
+      const uint4 x = *reinterpret_cast<const uint4*>(stg + stage_offset(row, lane & 3));
+      if (row < rows) *reinterpret_cast<uint4*>(to + (size_t)row * ld + h * 16 + (lane & 3) * 4) = x;
+    }
+  }
+}
+
 // A block that was fetched four lanes per row (row it * 8 + lane / 4, chunk lane & 3, in x[it]) into the staging buffer,
 // from where own_chunk() reads eight columns of the lane's own row. __syncwarp() after the last read.
 __device__ __forceinline__ void warp_place_rows(uint8_t* stg, int lane, const uint4 (&x)[4]) {
