@@ -92,37 +92,59 @@ stats_kernel(const bf16* __restrict__ x, float* __restrict__ part, int64_t R, in
   cta_fold(s, q, C, part);
 }
 
-// Sum the per-CTA partials of 32 channels with a 32 x 8 thread block: thread (cx, py)
-// adds partials py, py+8, ... of channel c (coalesced across cx), then the 8 rows are
-// added in a fixed order, so the result does not depend on scheduling.
-constexpr int kFinX = 32, kFinY = 32;
-__device__ __forceinline__ void fold_partials(const float* __restrict__ part, int parts, int C, int c, double& s_out,
-                                              double& q_out) {
-  __shared__ double sm_s[kFinY][kFinX + 1], sm_q[kFinY][kFinX + 1];
-  const int cx = threadIdx.x, py = threadIdx.y;
-  double s = 0, q = 0;   // the variance is a difference of two large sums: fold in double
-  if (c < C)
-    for (int p = py; p < parts; p += kFinY) { s += part[(size_t)p * 2 * C + c]; q += part[(size_t)p * 2 * C + C + c]; }
-  sm_s[py][cx] = s; sm_q[py][cx] = q;
+// The sums of the CTAs' partials for 8 channels (a sector of each partial), in double precision: a variance is a difference of two large sums.
+// Thread (channel, row) adds partials row, row + 128, ... with the loads of a turn all on their way before the first addition (partials past
+// the end count as zeros). Then a warp's four rows are added by shuffles and the warps' sums by the first warp, each in an order of its
+// own, so the result does not depend on scheduling. Returns true in the 8 threads that hold the channels' sums.
+// Bound by latency: the launch, one trip to the L2 (three sweep CTAs an SM leave at most 444 partials) and the fold. With 32 channels a CTA, four
+// trips and every thread repeating the last fold in double precision, forward of 256 x 128 x 28 x 28 31.2 us, now 29.5, x 64 x 56 x 56 55.8, 54.7,
+// 16 x 64 x 56 x 56 10.8, 9.2; backward 52.6, 51.9, the same, 12.3, 11.6. Fewer threads and more trips are slower: 512 threads in turns of 7 30.3, 256
+// 32.7, 128 35.4. Two CTAs of 32 registers fit on an SM: at 50 registers 256 x 2048 x 7 x 7, which has 256 CTAs here, takes 37.8 us instead of 33.3.
+constexpr int kFinX = 8, kFinY = 128, kFinThreads = kFinX * kFinY, kFinWarps = kFinThreads / 32;
+__device__ __forceinline__ bool fold_partials(const float* __restrict__ part, int parts, int C, int c, double& s, double& q) {
+  constexpr int TURN = 4;
+  __shared__ double sm[2][kFinWarps][kFinX];
+  const int row = threadIdx.x / kFinX, lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  s = 0; q = 0;
+#pragma unroll 1
+  for (int p0 = row; p0 < parts; p0 += TURN * kFinY) {
+    float a[TURN], b[TURN];
+#pragma unroll
+    for (int j = 0; j < TURN; j++) {
+      const float* from = part + (size_t)(p0 + j * kFinY) * 2 * C + c;
+      const bool there = p0 + j * kFinY < parts;
+      a[j] = there ? from[0] : 0.0f; b[j] = there ? from[C] : 0.0f;
+    }
+#pragma unroll
+    for (int j = 0; j < TURN; j++) { s += a[j]; q += b[j]; }
+  }
+  auto rows = [](double v) {      // the four rows of a warp, to all of its lanes
+#pragma unroll
+    for (int m = kFinX; m < 32; m *= 2) v += __shfl_xor_sync(~0u, v, m);
+    return v;
+  };
+  s = rows(s); q = rows(q);
+  if (lane < kFinX) { sm[0][warp][lane] = s; sm[1][warp][lane] = q; }
   __syncthreads();
+  if (warp != 0) return false;
   s = 0; q = 0;
 #pragma unroll
-  for (int j = 0; j < kFinY; j++) { s += sm_s[j][cx]; q += sm_q[j][cx]; }
-  s_out = s; q_out = q;
+  for (int j = lane / kFinX; j < kFinWarps; j += 32 / kFinX) { s += sm[0][j][lane % kFinX]; q += sm[1][j][lane % kFinX]; }
+  s = rows(s); q = rows(q);
+  return lane < kFinX;
 }
 
 // ---- finalize forward: mean/rstd, scale/shift, running statistics
-__global__ void __launch_bounds__(kFinX * kFinY)
+__global__ void __launch_bounds__(kFinThreads, 2048 / kFinThreads)
 finalize_fwd_kernel(const float* __restrict__ part, int parts, int C, int64_t R, float eps, float momentum,
                     const float* __restrict__ gamma, const float* __restrict__ beta,
                     float* __restrict__ mean, float* __restrict__ rstd, float* __restrict__ scale,
                     float* __restrict__ shift, float* __restrict__ run_mean, float* __restrict__ run_var) {
   pdl_wait();
   pdl_trigger();
-  const int c = blockIdx.x * kFinX + threadIdx.x;
+  const int c = blockIdx.x * kFinX + threadIdx.x % kFinX;      // C is a multiple of kFinX
   double s, q;
-  fold_partials(part, parts, C, c, s, q);
-  if (c >= C || threadIdx.y != 0) return;
+  if (!fold_partials(part, parts, C, c, s, q)) return;
   const double mu = s / (double)R;
   double var = q / (double)R - mu * mu;
   if (var < 0) var = 0;
@@ -225,15 +247,14 @@ bwd_reduce_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ dy2, con
 }
 
 // ---- finalize backward: dbeta = sum g, dgamma = sum g*xhat (fixed order)
-__global__ void __launch_bounds__(kFinX * kFinY)
+__global__ void __launch_bounds__(kFinThreads, 2048 / kFinThreads)
 finalize_bwd_kernel(const float* __restrict__ part, int parts, int C, float* __restrict__ dgamma,
                     float* __restrict__ dbeta) {
   pdl_wait();
   pdl_trigger();
-  const int c = blockIdx.x * kFinX + threadIdx.x;
+  const int c = blockIdx.x * kFinX + threadIdx.x % kFinX;      // C is a multiple of kFinX
   double s, q;
-  fold_partials(part, parts, C, c, s, q);
-  if (c >= C || threadIdx.y != 0) return;
+  if (!fold_partials(part, parts, C, c, s, q)) return;
   dbeta[c] = (float)s; dgamma[c] = (float)q;
 }
 
@@ -621,7 +642,7 @@ int gcow_bn_fwd_train(const void* x, const void* residual, void* y, void* mask, 
   const int g = grid_for(R, C);
   float *mean = stats, *rstd = stats + C, *scale = stats + 2 * C, *shift = stats + 3 * C;
   gcow::launch_dependent(stats_kernel, dim3(g), dim3(kThreads), 0, s, (const bf16*)x, part, R, C);
-  gcow::launch_dependent(finalize_fwd_kernel, dim3((C + kFinX - 1) / kFinX), dim3(kFinX, kFinY), 0, s, part, g, C, R, eps, momentum, gamma,
+  gcow::launch_dependent(finalize_fwd_kernel, dim3(C / kFinX), dim3(kFinThreads), 0, s, part, g, C, R, eps, momentum, gamma,
                    beta, mean, rstd, scale, shift, run_mean, run_var);
   gcow::launch_dependent(apply_for(residual, mask, relu), dim3(g), dim3(kThreads), 0, s, (const bf16*)x, (const bf16*)residual, (bf16*)y, (uint8_t*)mask,
                    (const float*)scale, (const float*)shift, R, C);
@@ -662,7 +683,7 @@ int gcow_bn_bwd3(const void* dy, const void* dy2, const void* mask, const void* 
   const float *mean = stats, *rstd = stats + C;
   gcow::launch_dependent(bwd_reduce_for(dy2, dres, relu), dim3(g), dim3(kThreads), 0, s, (const bf16*)dy, (const bf16*)dy2, (const uint8_t*)mask,
                          (const bf16*)x, mean, rstd, (bf16*)dres, part, R, C);
-  gcow::launch_dependent(finalize_bwd_kernel, dim3((C + kFinX - 1) / kFinX), dim3(kFinX, kFinY), 0, s, (const float*)part, g, C, dgamma, dbeta);
+  gcow::launch_dependent(finalize_bwd_kernel, dim3(C / kFinX), dim3(kFinThreads), 0, s, (const float*)part, g, C, dgamma, dbeta);
   // the second sweep applies the mask again, or reads the masked gradient if it was written
   gcow::launch_dependent(!dres && relu ? bwd_dx_kernel<true> : bwd_dx_kernel<false>, dim3(g), dim3(kThreads), 0, s, (const bf16*)(dres ? dres : dy), (const uint8_t*)mask, (const bf16*)x,
                    gamma, mean, rstd, (const float*)dgamma, (const float*)dbeta, (bf16*)dx, R, C);

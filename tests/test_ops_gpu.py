@@ -564,6 +564,12 @@ def test_batchnorm_every_form_of_the_sweeps(N, C, H, W, res, relu, fork):
         assert ((bn(x0, residual=r0 if res else None, relu=relu).double() - want).abs() <= 2**-8 * want.abs() + 1e-4).all()
 
 
+@pytest.mark.parametrize("parts", [1, 2, 127, 129, 385, 443])
+def test_batchnorm_sums_of_any_number_of_partials(parts):
+    """The sums' second half takes 128 partials at a time, four times a turn: fewer, just more, just more than three, and nearly as many as the sweeps leave."""
+    test_batchnorm_every_form_of_the_sweeps(1, 8, 1, parts * 256 - 3, False, True, False)     # 8 channels: 256 rows a partial
+
+
 # Fewer rows than CTAs in a cluster, one CTA a cluster, clusters of 2 to 16, channels by 32 and by 16, shares of rows that differ by one, shares just
 # within 52 KB and 104 KB and just beyond
 @pytest.mark.parametrize("N,C,H,W", [(1, 64, 1, 3), (1, 2048, 1, 1), (3, 2048, 7, 7), (17, 512, 7, 7), (13, 1024, 9, 11), (1, 128, 111, 113), (1, 128, 111, 121),
