@@ -36,13 +36,14 @@ constexpr int STAGE_BYTES = 2 * OPER_BYTES;           // 64 KB
 constexpr int STAGES = 3;
 // What an epilogue reads besides the accumulator.
 enum Side : int { kNothing = 0, kSum = 1, kArgument = 2 };      // a residual; the argument of a GELU' factor (and perhaps a residual)
-// Epilogue warps: eight, or sixteen for a GELU, whose arithmetic two warps per scheduler leave half of the issue slots to (bias, GELU and its
-// argument kept, eight, sixteen: 16384 x 4096 x 1024 142, 129 us, x 3072 110, 97, x 1024 44, 36). Twelve for a GELU' factor, whose registers
-// sixteen leave no room for: 16384 x 4096 x 1024 139 us with eight, 133 with twelve, 164 with sixteen. A residual takes 121 with eight, 133 with twelve.
-template <int SIDE, bool WIDE> struct Epilogue { static constexpr int WARPS = WIDE ? 16 : SIDE == kArgument ? 12 : 8, THREADS = 64 + 32 * WARPS; };
+// Epilogue warps: eight, or sixteen where two per scheduler leave half of the issue slots to waiting: for a GELU (bias, GELU and its argument kept, eight,
+// sixteen: 16384 x 4096 x 1024 142, 129 us, x 3072 110, 97, x 1024 44, 36) and for a side operand (a residual 115, 108, with a bias 160, 119; 4096 x
+// 768 x 768 11.3, 10.4 and 13.3, 11.4).
+template <int SIDE, bool WIDE> struct Epilogue { static constexpr int WARPS = WIDE || SIDE ? 16 : 8, THREADS = 64 + 32 * WARPS; };
 // Warps of a weight gradient that add up the columns of A as they pass through shared memory (the bias gradient).
 constexpr int SUM_WARPS = 2;
 template <bool A_MN, int SIDE, bool WIDE> constexpr int kThreads = Epilogue<SIDE, WIDE>::THREADS + (A_MN ? 32 * SUM_WARPS : 0);
+static_assert(Epilogue<kSum, false>::THREADS == Epilogue<kArgument, false>::THREADS && Epilogue<kSum, false>::THREADS == Epilogue<kNothing, true>::THREADS, "one launch shape");
 constexpr uint32_t TMEM_COLS = 512;
 
 enum Flags : int { kBias = 2, kGelu = 4, kResidual = 8, kAuxOut = 32, kGeluGrad = 64 };
@@ -64,13 +65,13 @@ struct Params {
 
 // An item of work: a tile, or the left or right half of one, over a slice of the reduction.
 struct Item { int m0, n0, kb0, kb1, slice; bool half; };
-template <bool SLICES, bool DIVIDE> __device__ __forceinline__ Item item_at(const Params& p, int i, int tiles, int kblocks) {
+template <bool SLICES> __device__ __forceinline__ Item item_at(const Params& p, int i, int tiles, int kblocks) {
   Item r;
   r.half = i >= p.whole;
   const int j = r.half ? (i - p.whole) >> 1 : i;
   r.slice = SLICES ? j / tiles : 0;
   const int tile = r.half ? p.whole + j : j - r.slice * tiles;
-  if (DIVIDE) p.order.order.at(tile, r.m0, r.n0); else p.order.at(tile, r.m0, r.n0);
+  p.order.at(tile, r.m0, r.n0);
   r.m0 *= BM;
   r.n0 = r.n0 * BN + (r.half ? ((i - p.whole) & 1) * (BN / 2) : 0);
   r.kb0 = SLICES ? r.slice * p.slice_blocks : 0;
@@ -78,8 +79,28 @@ template <bool SLICES, bool DIVIDE> __device__ __forceinline__ Item item_at(cons
   return r;
 }
 
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+  uint4 o;
+  __nv_bfloat162* const b = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+  for (int e = 0; e < 4; e++) b[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+  return o;
+}
+__device__ __forceinline__ void add8(float (&v)[8], const uint4& x) {
+  const __nv_bfloat162* const b = reinterpret_cast<const __nv_bfloat162*>(&x);
+#pragma unroll
+  for (int e = 0; e < 4; e++) { const float2 f = __bfloat1622float2(b[e]); v[2 * e] += f.x; v[2 * e + 1] += f.y; }
+}
+
 struct Smem {
-  uint64_t full[STAGES], empty[STAGES], landed[STAGES], tmem_full[2], tmem_empty[2], drain;
+  uint64_t full[STAGES], empty[STAGES], landed[STAGES], tmem_full[2], tmem_empty[2], drain, side[16];
   uint32_t tmem_base;
   volatile uint32_t abort;
 };
@@ -132,12 +153,13 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128_16k(uint32_t saddr) {
 template <bool A_MN, bool B_MN, int SIDE, bool WIDE>
 __global__ void __launch_bounds__((kThreads<A_MN, SIDE, WIDE>), 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                  const __grid_constant__ CUtensorMap tmap_bh, const Params p) {
+                  const __grid_constant__ CUtensorMap tmap_bh, const Params p, const __grid_constant__ CUtensorMap tmap_side,
+                  const __grid_constant__ CUtensorMap tmap_c) {
   constexpr int EPI_WARPS = Epilogue<SIDE, WIDE>::WARPS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   Smem* sm = reinterpret_cast<Smem*>(base + STAGES * STAGE_BYTES);
-  uint8_t* stage_base = reinterpret_cast<uint8_t*>(((uintptr_t)(sm + 1) + 15) & ~(uintptr_t)15);
+  uint8_t* stage_base = reinterpret_cast<uint8_t*>(((uintptr_t)(sm + 1) + 511) & ~(uintptr_t)511);
 
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp: uniform
   const uint32_t rank = cluster_rank();               // 0: issues the MMAs and owns full / tmem_empty
@@ -151,6 +173,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     for (int s = 0; s < STAGES; s++) { mbar_init(&sm->full[s], 1); mbar_init(&sm->empty[s], readers); mbar_init(&sm->landed[s], 1); }
     for (int a = 0; a < 2; a++) { mbar_init(&sm->tmem_full[a], 1); mbar_init(&sm->tmem_empty[a], 2 * EPI_WARPS * 32); }
     mbar_init(&sm->drain, 1);
+    if (SIDE) for (int w = 0; w < EPI_WARPS; w++) mbar_init(&sm->side[w], 1);
     sm->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -174,7 +197,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       uint32_t s = 0, phase = 0;
       bool ok = true;
       for (int i = pair; i < p.items && ok; i += pairs) {
-        const Item it = item_at<A_MN, SIDE == kArgument>(p, i, tiles, kblocks);
+        const Item it = item_at<A_MN>(p, i, tiles, kblocks);
         const int m0 = it.m0 + (int)rank * 128, n0 = it.n0 + (int)rank * (it.half ? 64 : 128);
         const CUtensorMap* const map_b = it.half ? &tmap_bh : &tmap_b;
         for (int kb = it.kb0; kb < it.kb1; kb++) {
@@ -206,7 +229,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         return __all_sync(0xffffffffu, mbar_wait_abortable(&sm->abort, bar, parity, p.error, code)) != 0;
       };
       for (int i = pair; i < p.items && ok; i += pairs, t++) {
-        const Item it = item_at<A_MN, SIDE == kArgument>(p, i, tiles, kblocks);
+        const Item it = item_at<A_MN>(p, i, tiles, kblocks);
         const uint32_t idesc = idesc0 | ((uint32_t)((it.half ? BN / 2 : BN) >> 3) << 17), chunk_b = it.half ? CHUNK_BYTES / 2 : CHUNK_BYTES;
         const uint32_t acc = t & 1, aphase = (t >> 1) & 1;
         if (!(ok = wait(&sm->tmem_empty[acc], aphase ^ 1, 2))) break;
@@ -266,7 +289,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       uint32_t s = 0, phase = 0;
       bool ok = true;
       for (int i = pair; i < p.items && ok; i += pairs) {
-        const Item it = item_at<A_MN, SIDE == kArgument>(p, i, tiles, kblocks);
+        const Item it = item_at<A_MN>(p, i, tiles, kblocks);
         const int first = it.n0 / BN;
         int rows = 0, held = 0;
         float sum[8] = {}, some[8] = {}, v[8] = {};
@@ -316,47 +339,43 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     const int q = warp & 3, ew = warp - 2;
     constexpr int GROUPS = EPI_WARPS / 4;               // of columns
     const bool wide_bias = ((uintptr_t)p.bias & 15) == 0;
-    [[maybe_unused]] const __nv_bfloat16* const ahead = SIDE == kArgument ? p.aux : p.residual;
     uint8_t* stg = stage_base + ew * kStageWarpBytes;
     uint32_t t = 0;
     bool ok = true;
-    // A tile's blocks of 32 columns go to the column groups in order, as evenly as they can. What the epilogue reads besides the
-    // accumulator is fetched one block ahead, the next tile's first block with this one's last: read where it is used, every block would
-    // stand for its load's whole latency, of which few warps per scheduler cover little. With the first block under the wait for its own
-    // tile, which is none where the epilogue sets the pace, and two copies of the code, 16384 x 4096 x 1024 took 145 us with a bias and a residual
-    // and 154 with GELU', now 121 and 133; x 1024 x 1024 49 and 52, now 41 and 45 (single launches).
-    constexpr bool EVEN = BN / 64 % GROUPS == 0;
-    [[maybe_unused]] auto blocks_before = [](bool half, int group) { return ((half ? BN / 64 : BN / 32) * group + GROUPS - 1) / GROUPS; };
-    [[maybe_unused]] uint4 pf[4];                         // four lanes per row, as the staging helpers have it
-    [[maybe_unused]] auto fetch = [&](int row0, int n) {
-      n += (lane & 3) * 8;
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int row = row0 + j * 8 + (lane >> 2);
-        pf[j] = make_uint4(0, 0, 0, 0);
-        if (n < p.N && row < p.M) pf[j] = *reinterpret_cast<const uint4*>(ahead + (size_t)row * p.ldc + n);
+    // What the epilogue reads besides the accumulator comes by the TMA, a warp's 32 x 32 block into its staging buffer, where each lane takes its row
+    // and puts the result's in its place, from where the TMA fetches it. The next block, or the next tile's first one, is asked for as soon as the
+    // buffer has been read, so it comes under the wait for the accumulator. Bound by a warp's chain of block, arithmetic and store, four to a
+    // scheduler. Read by the lanes themselves a block ahead, which left registers for eight warps (twelve for a GELU' factor), and written by
+    // them, us, now: 16384 x 4096 x 1024 with a residual 115, 110, and a bias 135, 113, GELU' 155, 122, and a residual 240, 147; 16384 x 1024 x 1024 32.7,
+    // 31.0, 38.7, 33.2, 42.1, 35.8, 53.8, 39.7; 4096 x 768 x 768 11.1, 10.4, 12.1, 11.2, 13.9, 12.3, 16.6, 12.7. The results are the same bits.
+    [[maybe_unused]] uint32_t side_phase = 0;
+    [[maybe_unused]] bool side_due = false;               // the block asked for has not been waited for
+    [[maybe_unused]] const bool one = elect_one();
+    [[maybe_unused]] auto ask = [&](int row0, int n) {    // where there is no such block, nobody will wait for it
+      if (n >= p.N || row0 >= p.M) return;
+      if (one) {
+        mbar_expect_tx(&sm->side[ew], kStageWarpBytes);
+        tma_load_2d(smem_u32(stg), &tmap_side, smem_u32(&sm->side[ew]), n, row0);
       }
+      side_due = true;
     };
-    [[maybe_unused]] auto fetch_first = [&](int i) {
+    [[maybe_unused]] auto ask_first = [&](int i) {
       if (i >= p.items) return;
-      const Item it = item_at<A_MN, SIDE == kArgument>(p, i, tiles, kblocks);
-      fetch(it.m0 + (int)rank * 128 + q * 32, it.n0 + blocks_before(it.half, ew / 4) * 32);
+      const Item it = item_at<A_MN>(p, i, tiles, kblocks);
+      ask(it.m0 + (int)rank * 128 + q * 32, it.n0 + (ew / 4) * ((it.half ? BN / 2 : BN) / GROUPS));
     };
-    if (SIDE) fetch_first(pair);
-    // The next item's place is worked out before this one's wait, but for a GELU' factor, whose registers are full. A GELU after
-    // 4096 x 768 x 768 12.7 -> 12.4 us (12.2 before the tiles came in groups), 16384 x 512 x 512 16.4 -> 15.7 (15.5), 8192 x 3072 x 768 38.2 -> 37.3 (37.5).
-    constexpr bool AHEAD = SIDE != kArgument;
-    [[maybe_unused]] Item next = item_at<A_MN, SIDE == kArgument>(p, pair, tiles, kblocks);
+    if (SIDE) ask_first(pair);
+    // The next item's place is worked out before this one's wait. A GELU after 4096 x 768 x 768 12.7 -> 12.4 us (12.2 before the tiles came in
+    // groups), 16384 x 512 x 512 16.4 -> 15.7 (15.5), 8192 x 3072 x 768 38.2 -> 37.3 (37.5).
+    Item next = item_at<A_MN>(p, pair, tiles, kblocks);
     for (int i = pair; i < p.items && ok; i += pairs, t++) {
-      const Item it = AHEAD ? next : item_at<A_MN, SIDE == kArgument>(p, i, tiles, kblocks);
-      if (AHEAD && i + pairs < p.items) next = item_at<A_MN, SIDE == kArgument>(p, i + pairs, tiles, kblocks);
+      const Item it = next;
+      if (i + pairs < p.items) next = item_at<A_MN>(p, i + pairs, tiles, kblocks);
       const int m0 = it.m0 + (int)rank * 128, n0 = it.n0;
       // this warp's
-      const int cols = (it.half ? BN / 2 : BN) / GROUPS, chunks = EVEN ? cols / 32 : blocks_before(it.half, ew / 4 + 1) - blocks_before(it.half, ew / 4),
-                col0 = EVEN ? (ew / 4) * cols : blocks_before(it.half, ew / 4) * 32;
+      const int cols = (it.half ? BN / 2 : BN) / GROUPS, chunks = cols / 32, col0 = (ew / 4) * cols;
       const uint32_t acc = t & 1, aphase = (t >> 1) & 1;
       const int mw = m0 + q * 32;                         // the warp's first row
-      [[maybe_unused]] auto fetch_after = [&](int c) { if (c + 1 < chunks) fetch(mw, n0 + col0 + (c + 1) * 32); else fetch_first(i + pairs); };
       ok = mbar_wait_abortable(&sm->abort, &sm->tmem_full[acc], aphase, p.error, 4);
       ok = __all_sync(0xffffffffu, ok);   // the tensor-memory loads below need the whole warp
       if (!ok) break;
@@ -366,10 +385,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN + col0;
       auto process = [&](const uint32_t (&r)[32], int c) {
         const int n = n0 + col0 + c * 32;
-        if (n >= p.N || mw >= p.M) {                      // warp-uniform; the launcher guarantees N % 32 == 0
-          if (SIDE) fetch_after(c);
-          return;
-        }
+        if (n >= p.N || mw >= p.M) return;                // warp-uniform; the launcher guarantees N % 32 == 0
         const size_t off = (size_t)m * p.ldc + n;
         float v[32];
 #pragma unroll
@@ -402,55 +418,111 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
         }
         if (p.flags & kAuxOut) warp_store_rows_bf16(stg, lane, v, p.aux, off, row_ok);
-        if (p.flags & kGelu) gelu32(v);                    // not together with kGeluGrad
-        if (SIDE) {
-          warp_place_rows(stg, lane, pf);
-          fetch_after(c);
-#pragma unroll
-          for (int k = 0; k < 4; k++) {
-            float x[8];
-            own_chunk(stg, lane, k, x);
-            if (SIDE == kArgument) {
-              gelu_grad8(v + 8 * k, x);
-            } else {
-#pragma unroll
-              for (int e = 0; e < 8; e++) v[8 * k + e] += x[e];
-            }
-          }
-          __syncwarp();
-        }
-        if (SIDE == kArgument && (p.flags & kResidual)) warp_load_rows_bf16<true>(stg, lane, p.residual, off, row_ok, v);
+        if (p.flags & kGelu) gelu(v);                    // not together with kGeluGrad
         warp_store_rows_bf16(stg, lane, v, p.C, off, row_ok);
       };
-      // tensor-memory loads one block ahead of the arithmetic (sixteen warps hide them from one another, and with a side operand the
-      // registers go to the blocks of that fetched ahead)
-      uint32_t ra[32];
-      tc_ld32(taddr, ra);
-      if constexpr (SIDE) {
+      if constexpr (SIDE != kNothing) {
 #pragma unroll 1
         for (int c = 0; c < chunks; c++) {
-          tc_wait_ld();
-          process(ra, c);
-          if (c + 1 < chunks) tc_ld32(taddr + (c + 1) * 32, ra);
-        }
-      } else {
-        uint32_t rb[32];
-#pragma unroll 1
-        for (int c = 0; c < chunks; c += 2) {
-          tc_wait_ld();
-          if (!WIDE && c + 1 < chunks) tc_ld32(taddr + (c + 1) * 32, rb);
-          process(ra, c);
-          if (c + 1 < chunks) {
-            if (WIDE) tc_ld32(taddr + (c + 1) * 32, rb);
-            tc_wait_ld();
-            if (!WIDE && c + 2 < chunks) tc_ld32(taddr + (c + 2) * 32, ra);
-            process(rb, c + 1);
+          const int n = n0 + col0 + c * 32;
+          if (n < p.N && mw < p.M) {                       // warp-uniform; the launcher guarantees N % 32 == 0
+            ok = mbar_wait_abortable(&sm->abort, &sm->side[ew], side_phase, p.error, 5);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            side_phase ^= 1;
+            side_due = false;
+            const size_t off = (size_t)m * p.ldc + n;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              uint32_t r[16];
+              uint4 res[2] = {};
+              if (SIDE == kArgument && (p.flags & kResidual) && row_ok)   // the buffer holds the argument: a lane reads its own row
+#pragma unroll
+                for (int k = 0; k < 2; k++) res[k] = *reinterpret_cast<const uint4*>(p.residual + off + h * 16 + k * 8);
+              tc_ld16(taddr + c * 32 + h * 16, r);
+              float bias[16];                              // a residual: under the wait for the accumulator; no registers for it with a GELU' factor
+              auto add_bias = [&](float* to, int from) {   // eight columns
+                if (wide_bias) {                           // n is a multiple of 32
+#pragma unroll
+                  for (int e = 0; e < 8; e += 4) {
+                    const float4 b = *reinterpret_cast<const float4*>(p.bias + from + e);
+                    to[e] += b.x; to[e + 1] += b.y; to[e + 2] += b.z; to[e + 3] += b.w;
+                  }
+                } else {
+#pragma unroll
+                  for (int e = 0; e < 8; e++) to[e] += p.bias[from + e];
+                }
+              };
+              if constexpr (SIDE == kSum) {
+#pragma unroll
+                for (int e = 0; e < 16; e++) bias[e] = -0.0f;   // added to anything leaves it as it is
+                if (p.flags & kBias) {
+                  add_bias(bias, n + h * 16);
+                  add_bias(bias + 8, n + h * 16 + 8);
+                }
+              }
+              tc_wait_ld();
+#pragma unroll
+              for (int k = 0; k < 2; k++) {
+                const int e0 = h * 16 + k * 8;
+                float v[8], x[8];
+#pragma unroll
+                for (int e = 0; e < 8; e++) v[e] = SIDE == kSum ? __uint_as_float(r[8 * k + e]) + bias[8 * k + e] : __uint_as_float(r[8 * k + e]);
+                if (SIDE == kArgument && (p.flags & kBias)) add_bias(v, n + e0);
+                own_chunk(stg, lane, 2 * h + k, x);
+                if ((p.flags & kAuxOut) && row_ok) *reinterpret_cast<uint4*>(p.aux + off + e0) = pack8(v);
+                if constexpr (SIDE == kArgument) {
+                  gelu_grad8(v, x);
+                  if (p.flags & kResidual) add8(v, res[k]);
+                } else {
+                  if (p.flags & kGelu) gelu(v);
+#pragma unroll
+                  for (int e = 0; e < 8; e++) v[e] += x[e];
+                }
+                *reinterpret_cast<uint4*>(stg + stage_offset(lane, 2 * h + k)) = pack8(v);
+              }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (one) {
+              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+                           ::"l"((uint64_t)&tmap_c), "r"(smem_u32(stg)), "r"(n), "r"(mw) : "memory");   // rows past M are clipped
+              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+              asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            }
           }
+          if (c + 1 < chunks) ask(mw, n + 32); else ask_first(i + pairs);
+          __syncwarp();
+        }
+        if (!ok) break;
+        tc_fence_before();
+        mbar_arrive_cluster(map_to_cta(smem_u32(&sm->tmem_empty[acc]), 0));
+        continue;
+      }
+      // tensor-memory loads one block ahead of the arithmetic (sixteen warps hide them from one another)
+      uint32_t ra[32];
+      tc_ld32(taddr, ra);
+      uint32_t rb[32];
+#pragma unroll 1
+      for (int c = 0; c < chunks; c += 2) {
+        tc_wait_ld();
+        if (!WIDE && c + 1 < chunks) tc_ld32(taddr + (c + 1) * 32, rb);
+        process(ra, c);
+        if (c + 1 < chunks) {
+          if (WIDE) tc_ld32(taddr + (c + 1) * 32, rb);
+          tc_wait_ld();
+          if (!WIDE && c + 2 < chunks) tc_ld32(taddr + (c + 2) * 32, ra);
+          process(rb, c + 1);
         }
       }
       // this CTA's half of the accumulator has been read out: tell the MMA thread in CTA 0
       tc_fence_before();
       mbar_arrive_cluster(map_to_cta(smem_u32(&sm->tmem_empty[acc]), 0));
+    }
+    if (SIDE) {                                            // nothing may be in flight when the CTA ends
+      if (side_due)
+        for (uint32_t it = 0; it < kSpinLimit; it++) if (mbar_try_wait(&sm->side[ew], side_phase)) break;
+      if (one) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
   }
 
@@ -495,8 +567,23 @@ static int make_map_mnfold(CUtensorMap* map, const void* ptr, uint64_t K, uint64
   return r == CUDA_SUCCESS ? 0 : -12;
 }
 
-using KernelFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, Params);
-constexpr size_t kSmemBytes = (size_t)STAGES * STAGE_BYTES + sizeof(Smem) + 16 + (size_t)Epilogue<kNothing, true>::WARPS * kStageWarpBytes + 1024;
+// Row-major matrix [rows][cols] in blocks of 32 x 32 (64-byte rows, the staging buffers' swizzle).
+static int make_map_blocks(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return -10;
+  if (((uintptr_t)ptr & 15) || (ld * 2) % 16 || cols % 32) return -11;
+  cuuint64_t dims[2] = {cols, rows};
+  cuuint64_t strides[1] = {ld * 2};
+  cuuint32_t box[2] = {32, 32};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -12;
+}
+
+using KernelFn = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, Params, CUtensorMap, CUtensorMap);
+static_assert(sizeof(Smem) <= 512, "the staging buffers begin 512 bytes behind the operands");
+constexpr size_t kSmemBytes = (size_t)STAGES * STAGE_BYTES + 512 + (size_t)Epilogue<kNothing, true>::WARPS * kStageWarpBytes + 1024;
 
 static KernelFn pick(bool b_mn, int side, bool wide) {
   if (side == kArgument) return b_mn ? gemm2_bf16_kernel<false, true, kArgument, false> : gemm2_bf16_kernel<false, false, kArgument, false>;
@@ -506,7 +593,7 @@ static KernelFn pick(bool b_mn, int side, bool wide) {
 }
 
 static int launch(KernelFn kernel, int threads, int max_pairs, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mh,
-                  const Params& p, void* stream) {
+                  const Params& p, const CUtensorMap& side, const CUtensorMap& mc, void* stream) {
   const int pairs = p.items < max_pairs ? p.items : max_pairs;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs, 1, 1);
@@ -520,7 +607,7 @@ static int launch(KernelFn kernel, int threads, int max_pairs, const CUtensorMap
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   static const bool pdl = [] { const char* e = getenv("GCOW_PDL"); return !(e && e[0] == '0'); }();
   cfg.attrs = attr; cfg.numAttrs = pdl ? 2 : 1;
-  return (int)cudaLaunchKernelEx(&cfg, kernel, ma, mb, mh, p);
+  return (int)cudaLaunchKernelEx(&cfg, kernel, ma, mb, mh, p, side, mc);
 }
 
 }  // namespace gemm2
@@ -598,8 +685,14 @@ int gcow_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
   // which the epilogue spilled (16384 x 4096 x 1024: plain 100 -> 95 us, bias 106 -> 97).
   const int side = flags & kGeluGrad ? kArgument : flags & kResidual ? kSum : kNothing;
   const bool wide = !side && (flags & kGelu);
-  const int threads = wide ? Epilogue<kNothing, true>::THREADS : side == kArgument ? Epilogue<kArgument, false>::THREADS : Epilogue<kSum, false>::THREADS;
-  return launch(pick(b_mn, side, wide), threads, max_pairs, ma, mb, mh, p, stream);
+  CUtensorMap mside = mb, mc = mb;
+  if (side) {
+    rc = make_map_blocks(&mside, side == kArgument ? aux : residual, (uint64_t)M, (uint64_t)N, (uint64_t)ldc);
+    if (!rc) rc = make_map_blocks(&mc, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc);
+    if (rc) return rc;
+  }
+  const int threads = wide || side ? Epilogue<kSum, false>::THREADS : Epilogue<kNothing, false>::THREADS;
+  return launch(pick(b_mn, side, wide), threads, max_pairs, ma, mb, mh, p, mside, mc, stream);
 }
 
 // How many slabs of equal length the one-CTA kernel's weight gradient cuts K rows into for an M x N result: it doubles while
@@ -665,7 +758,7 @@ int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, float* sums, in
   p.slice_stride = (size_t)M * N;
   p.halves = p.items <= max_pairs;
   p.aux = (__nv_bfloat16*)sums;
-  return launch(gemm2_bf16_kernel<true, true, kNothing, false>, kThreads<true, kNothing, false>, max_pairs, ma, mb, mb, p, stream);
+  return launch(gemm2_bf16_kernel<true, true, kNothing, false>, kThreads<true, kNothing, false>, max_pairs, ma, mb, mb, p, mb, mb, stream);
 }
 
 }  // extern "C"

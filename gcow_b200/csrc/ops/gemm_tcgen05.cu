@@ -255,7 +255,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 #pragma unroll
               for (int j = 0; j < 32; j++) v[j] += __ldg(p.bias + n + j);
             }
-            if (p.flags & kGelu) gelu32(v);
+            if (p.flags & kGelu) gelu(v);
 #pragma unroll
             for (int k = 0; k < 4; k++) {
               uint4 o;
@@ -296,7 +296,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 #pragma unroll
               for (int k = 0; k < 4; k++) gelu_grad8(v + 8 * k, x + 8 * k);
             }
-            if (p.flags & kGelu) gelu32(v);
+            if (p.flags & kGelu) gelu(v);
             if (p.flags & kResidual)
               warp_load_rows_bf16<true>(stg, lane, reinterpret_cast<const __nv_bfloat16*>(p.residual), off, row_ok, v);
             warp_store_rows_bf16(stg, lane, v, reinterpret_cast<__nv_bfloat16*>(p.C), off, row_ok);
@@ -317,7 +317,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
               for (int j = 0; j < 32; j++) if (n + j < p.N) v[j] += __ldg(p.bias + n + j);
             }
             const size_t off = (size_t)bz * (size_t)p.stride_c + (size_t)m * p.ldc + n;
-            if (p.flags & kGelu) gelu32(v);
+            if (p.flags & kGelu) gelu(v);
             if (p.flags & kOutF32) {
               float* C = reinterpret_cast<float*>(p.C) + off;
               const float* R = reinterpret_cast<const float*>(p.residual) + off;

@@ -168,9 +168,9 @@ __device__ __forceinline__ void gelu_parts2(float x0, float x1, uint64_t x, uint
   cdf = pack2(x0 >= 0.0f ? a : q0, x1 >= 0.0f ? b : q1);
 }
 // v = GELU(v)
-__device__ __forceinline__ void gelu32(float (&v)[32]) {
+template <int N> __device__ __forceinline__ void gelu(float (&v)[N]) {
 #pragma unroll
-  for (int j = 0; j < 32; j += 2) {
+  for (int j = 0; j < N; j += 2) {
     const uint64_t x = pack2(v[j], v[j + 1]);
     uint64_t cdf, gauss;
     gelu_parts2(v[j], v[j + 1], x, cdf, gauss);
@@ -257,13 +257,7 @@ __device__ __forceinline__ void warp_store_rows_f32_halves(uint8_t* stg, int lan
   }
 }
 
-// A block that was fetched four lanes per row (row it * 8 + lane / 4, chunk lane & 3, in x[it]) into the staging buffer,
-// from where own_chunk() reads eight columns of the lane's own row. __syncwarp() after the last read.
-__device__ __forceinline__ void warp_place_rows(uint8_t* stg, int lane, const uint4 (&x)[4]) {
-#pragma unroll
-  for (int it = 0; it < 4; it++) *reinterpret_cast<uint4*>(stg + stage_offset(it * 8 + (lane >> 2), lane & 3)) = x[it];
-  __syncwarp();
-}
+// Eight columns of the lane's own row of a block in the staging buffer.
 __device__ __forceinline__ void own_chunk(const uint8_t* stg, int lane, int k, float (&x)[8]) {
   const uint4 y = *reinterpret_cast<const uint4*>(stg + stage_offset(lane, k));
   const __nv_bfloat162* yb = reinterpret_cast<const __nv_bfloat162*>(&y);

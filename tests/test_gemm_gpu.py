@@ -253,9 +253,35 @@ def test_long_reductions_on_either_kernel(M, N, K, b_t):
     K_.check_errors()
 
 
+@pytest.mark.parametrize("M,N,K", [(8, 32, 64), (300, 96, 64), (1100, 1120, 192), (19000, 544, 64)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_pair_gemm_side_operands_with_everything(M, N, K, shift, monkeypatch):
+    """A residual behind bias, kept argument and GELU; bias and residual around a GELU' factor; blocks and rows that do not exist; a bias that vectors
+    cannot read; the result in the residual's place. Products, biases and residuals are whole numbers, so what is left is the approximation of
+    Phi (1.5e-7 and a few 2^-24 of fp32 evaluation, times |argument| or |product|, at most K + 9) and bf16's rounding."""
+    from gcow_b200.ops import kernels as K_
+    monkeypatch.setattr(K_, "_pair_gemm", True)
+    torch.manual_seed(M + N)
+    a, b = torch.randint(-1, 2, (M, K), device="cuda").bfloat16(), torch.randint(-1, 2, (N, K), device="cuda").bfloat16()
+    res, bias = torch.randint(-8, 9, (M, N), device="cuda").bfloat16(), torch.randint(-9, 10, (N + shift,), device="cuda").float()[shift:]
+    z, pre = a.double() @ b.double().t() + bias.double(), torch.empty_like(res)
+    close = lambda got, want, size: bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6 * size + 1e-30).all())
+    cdf = lambda v: 0.5 * torch.erfc(-v / 2 ** 0.5)
+    got = K_.gemm_bf16(a, b, bias=bias, residual=res, gelu=True, pre_gelu_out=pre)
+    assert torch.equal(pre, z.bfloat16()) and close(got, z * cdf(z) + res.double(), z.abs())
+    x = (torch.randn(M, N, device="cuda") * 2).bfloat16()
+    xd = x.double()
+    got = K_.gemm_bf16(a, b, bias=bias, residual=res, gelu_grad_of=x)
+    assert close(got, z * (cdf(xd) + xd * torch.exp(-0.5 * xd * xd) / (2 * 3.141592653589793) ** 0.5) + res.double(), z.abs())
+    own = res.clone()
+    K_.gemm_bf16(a, b, residual=own, out=own, bias=bias)
+    assert torch.equal(own, (z + res.double()).bfloat16())
+    K_.check_errors()
+
+
 @pytest.mark.parametrize("M,N,K", [(1024, 256, 64), (1100, 1120, 192), (2100, 544, 576), (9500, 1024, 64), (19000, 512, 128), (40000, 64 * 9, 64)])
 def test_pair_gemm_side_operands_of_whole_numbers(M, N, K, monkeypatch):
-    """The side operand is fetched a block ahead, also across tiles, and twelve warps share eight or four blocks of columns: one tile per
+    """The side operand is fetched a block ahead, also across tiles, and sixteen warps share eight or four blocks of columns: one tile per
     pair and several, halves in the last round, ragged edges. Residuals: whole numbers, exact. GELU': against float64, its argument
     the same bf16 numbers; the product is exact, so that what is left is bf16's rounding and the factor's approximation."""
     from gcow_b200.ops import kernels as K_
