@@ -86,6 +86,11 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr) : "memory");
 }
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const uint8_t* from, int x, int y) {   // rows past the end are clipped
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+               ::"l"((uint64_t)map), "r"(smem_u32(from)), "r"(x), "r"(y) : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
 __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
   uint4 o;
   __nv_bfloat162* const b = reinterpret_cast<__nv_bfloat162*>(&o);
@@ -365,6 +370,29 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       ask(it.m0 + (int)rank * 128 + q * 32, it.n0 + (ew / 4) * ((it.half ? BN / 2 : BN) / GROUPS));
     };
     if (SIDE) ask_first(pair);
+    // A warp's 32 x 32 results to the matrix of `map`, through the staging buffer that the last store but one (sixteen warps: the last one) has left.
+    // Two passes over the buffer and the lanes' own stores took, us, now: bias, GELU and its argument kept 16384 x 4096 x 1024 142, 124, x 1024 x 1024 38.4,
+    // 33.4, x 512 x 512 18.8, 15.1, 4096 x 768 x 768 13.7, 11.6, bias and GELU 118, 109, 33.7, 30.7, 15.6, 14.1, 12.4, 11.5, a bias 97.9, 93.7, 29.4, 27.1, 13.7,
+    // 11.3, 11.0, 9.8, plain 106, 105, 28.2, 27.9, 11.3, 10.3, 9.6, 8.8. Sixteen warps with one block of the accumulator each: GELU 116, 124; without
+    // a GELU sixteen warps instead of eight and two buffers: bias 112, 122.
+    constexpr int BUFFERS = WIDE ? 1 : 2;
+    [[maybe_unused]] int buffer = 0;
+    [[maybe_unused]] auto emit = [&](const float (&v)[32], const CUtensorMap* map, int n, int row0) {
+      uint8_t* const to = stage_base + (ew * BUFFERS + buffer) * kStageWarpBytes;
+      if (one) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(BUFFERS - 1) : "memory");
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        float u[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++) u[e] = v[8 * k + e];
+        *reinterpret_cast<uint4*>(to + stage_offset(lane, k)) = pack8(u);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (one) tma_store_2d(map, to, n, row0);
+      if (BUFFERS == 2) buffer ^= 1;
+    };
     // The next item's place is worked out before this one's wait. A GELU after 4096 x 768 x 768 12.7 -> 12.4 us (12.2 before the tiles came in
     // groups), 16384 x 512 x 512 16.4 -> 15.7 (15.5), 8192 x 3072 x 768 38.2 -> 37.3 (37.5).
     Item next = item_at<A_MN>(p, pair, tiles, kblocks);
@@ -417,9 +445,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             for (int j = 0; j < 32; j++) v[j] += p.bias[n + j];
           }
         }
-        if (p.flags & kAuxOut) warp_store_rows_bf16(stg, lane, v, p.aux, off, row_ok);
+        if (p.flags & kAuxOut) emit(v, &tmap_side, n, mw);
         if (p.flags & kGelu) gelu(v);                    // not together with kGeluGrad
-        warp_store_rows_bf16(stg, lane, v, p.C, off, row_ok);
+        emit(v, &tmap_c, n, mw);
       };
       if constexpr (SIDE != kNothing) {
 #pragma unroll 1
@@ -485,9 +513,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (one) {
-              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-                           ::"l"((uint64_t)&tmap_c), "r"(smem_u32(stg)), "r"(n), "r"(mw) : "memory");   // rows past M are clipped
-              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+              tma_store_2d(&tmap_c, stg, n, mw);
               asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             }
           }
@@ -519,7 +545,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       tc_fence_before();
       mbar_arrive_cluster(map_to_cta(smem_u32(&sm->tmem_empty[acc]), 0));
     }
-    if (SIDE) {                                            // nothing may be in flight when the CTA ends
+    if (!A_MN) {                                           // nothing may be in flight when the CTA ends
       if (side_due)
         for (uint32_t it = 0; it < kSpinLimit; it++) if (mbar_try_wait(&sm->side[ew], side_phase)) break;
       if (one) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -686,11 +712,10 @@ int gcow_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
   const int side = flags & kGeluGrad ? kArgument : flags & kResidual ? kSum : kNothing;
   const bool wide = !side && (flags & kGelu);
   CUtensorMap mside = mb, mc = mb;
-  if (side) {
-    rc = make_map_blocks(&mside, side == kArgument ? aux : residual, (uint64_t)M, (uint64_t)N, (uint64_t)ldc);
-    if (!rc) rc = make_map_blocks(&mc, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc);
-    if (rc) return rc;
-  }
+  const void* const other = side == kSum ? residual : flags & (kAuxOut | kGeluGrad) ? aux : nullptr;
+  rc = make_map_blocks(&mc, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc);
+  if (!rc && other) rc = make_map_blocks(&mside, other, (uint64_t)M, (uint64_t)N, (uint64_t)ldc);
+  if (rc) return rc;
   const int threads = wide || side ? Epilogue<kSum, false>::THREADS : Epilogue<kNothing, false>::THREADS;
   return launch(pick(b_mn, side, wide), threads, max_pairs, ma, mb, mh, p, mside, mc, stream);
 }
