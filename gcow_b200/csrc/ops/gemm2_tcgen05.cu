@@ -715,7 +715,7 @@ int gcow_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
   const void* const other = side == kSum ? residual : flags & (kAuxOut | kGeluGrad) ? aux : nullptr;
   rc = make_map_blocks(&mc, C, (uint64_t)M, (uint64_t)N, (uint64_t)ldc);
   if (!rc && other) rc = make_map_blocks(&mside, other, (uint64_t)M, (uint64_t)N, (uint64_t)ldc);
-  if (rc) return rc;
+  if (rc) return -2;
   const int threads = wide || side ? Epilogue<kSum, false>::THREADS : Epilogue<kNothing, false>::THREADS;
   return launch(pick(b_mn, side, wide), threads, max_pairs, ma, mb, mh, p, mside, mc, stream);
 }

@@ -204,15 +204,30 @@ Tensor gemm(const Tensor& a, const Tensor& b, const GemmOpts& o, const On& on) {
   //   two rounds, 16384 x 1024 x 6144 152, 144 / 170, 171;
   //   one-CTA: even, 8192 x 8192 x 5120 451, 469 / 535, 533, x 6144 543, 569 / 639, 652, x 8192 713, 770 / 843, 875; 4096 x 4096 x 8192 194.6, 192.5 / 220, 227;
   //   a single round, 2048 x 4096 x 4096 57, 57 / 56.0, 57.5.
-  // Reductions below 512 (the 1x1 convolutions of a ResNet) stay there too: the output stream bounds them, and the one-CTA
-  // kernel's TMA stores are 15 to 30 % faster there.
+  // A single round that leaves pairs idle, short and wide, plain or with a bias, stays there too: 1024 x 4096 x 512 6.9, 7.7, 2048 x 2048 x 768 8.4, 9.1, 4096 x
+  // 768 x 768 8.8, 9.2; from 1536 rows of reduction on, or with 512 columns, the two are even (8192 x 512 x 768 10.5, 10.3).
+  // Shorter, narrower and lower products (K < 512, N < 256, M < 1024; one-CTA tile, pairs in a graph). A residual, a kept argument or a GELU' factor, which
+  // the one-CTA kernel's lanes read and write themselves: pairs from 64 columns on, 1 x 1024 x 1024 with a residual 12.1, 7.1, 300 x 1024 x 1024
+  // 15.4, 7.9, 16384 x 1024 x 256 46.5, 18.0, 200704 x 512 x 128 261, 84; 32 columns 16384 x 32 x 64 5.5, 6.4. Others, whose results leave by the TMA
+  // on both: pairs where a round's tiles are few (a pair fetches twice as much at once: 128 x 1024 x 1024 9.4, 6.6, 1024 x 256 x 64 5.0, 4.4; up to 8
+  // tiles with 64 columns, 24 with 128, 37 with 256) and where there are several rounds of 256 columns (50176 x 1024 x 256 32.7, 28.7, with a bias
+  // 38.0, 33.0; 12544 x 2048 x 256 19.1, 15.9); a single round of more than 37 tiles is one of twice as many CTAs without pairs' start (16384 x 256 x 64 5.2,
+  // 6.2, 4096 x 768 x 256 6.3, 6.6). Plain, 64 columns deep in few rounds 8192 x 1024 x 64 7.0, 7.2, and the longest streams 802816 x 256 x 64 84.4, 90.7,
+  // x 128 100.6, 103.9: on one CTA. A single row of 4096 columns or more is uneven on pairs (x 4096 22.7, 22.5 to 28).
   const bool can_pair = pair_gemm_enabled() && !o.a_t && !(flags & (kOutF32 | kAccumulate)) && !o.max_ctas && !o.tile_rows;
   const int64_t tiles = ((M + 255) / 256) * ((N + 255) / 256);
   const bool even = 2 * ((tiles + 147) / 148) <= (tiles + 73) / 74;
   const bool one_cta = !(flags & (kGelu | kResidual | kGeluGrad)) && tiles >= 118 && even &&
                        (K >= 8192 || (K > 4096 && tiles > 296) || (K >= 2048 && tiles <= 148));
-  const bool by_rule = K % 64 == 0 && K >= 512 && N % (o.b_t ? 64 : 32) == 0 && M >= 1024 && N >= 256 && lda % 8 == 0 && ldb % 8 == 0 &&
-                       ldc % 8 == 0 && !one_cta;
+  const bool fits = K % 64 == 0 && N % (o.b_t ? 64 : 32) == 0 && lda % 8 == 0 && ldb % 8 == 0 && ldc % 8 == 0;
+  const bool bare = !(flags & (kGelu | kResidual | kGeluGrad | kAuxOut)), plain = bare && !(flags & kBias), short_round = tiles > 37 && tiles <= 74;
+  const bool by_rule = fits && (M > 1 || N <= 3072) &&
+                       (K >= 512 && M >= 1024 && N >= 256 ? !one_cta && !(bare && short_round && K <= 768 && N >= 768)
+                        : flags & (kResidual | kGeluGrad | kAuxOut) ? N >= 64
+                        : tiles <= 8                                ? N >= 64
+                        : tiles <= 24                               ? N >= 128
+                        : tiles <= 37                               ? N >= 256 && K >= 128
+                                                                    : !short_round && N >= 256 && !(plain && (M >= 524288 || (K < 128 && tiles <= 148))));
   if (can_pair && (o.pair < 0 ? by_rule : o.pair > 0)) {
     const int err = gcow_gemm2_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, lda, ldb, ldc, f32(o.bias),
                                     raw(o.residual), raw(aux), flags, on.error, o.b_t, on.stream);

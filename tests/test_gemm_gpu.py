@@ -253,6 +253,36 @@ def test_long_reductions_on_either_kernel(M, N, K, b_t):
     K_.check_errors()
 
 
+# Both sides of the lines: rows of 64, 128 and 256 columns, 8, 24, 37, 74 and 148 tiles, 128 and 512 deep, a single low row, rows that are not whole vectors
+@pytest.mark.parametrize("M,N,K", [(1, 256, 512), (7, 32, 64), (2048, 64, 64), (2300, 64, 64), (6144, 128, 128), (6145, 128, 128), (9472, 256, 128), (9473, 256, 64),
+                                   (18944, 256, 64), (18945, 256, 64), (37900, 256, 192), (300, 1024, 768), (1000, 4096, 512), (2048, 2048, 768), (2048, 2048, 832),
+                                   (300, 192, 72), (520, 96, 256)])
+@pytest.mark.parametrize("b_t", [False, True])
+def test_every_form_on_either_side_of_the_dispatch(M, N, K, b_t, monkeypatch):
+    """The kernel that the rule takes against the one-CTA kernel: every epilogue, operands and results with rows apart, the result in the residual's
+    place. Whole numbers, so the sums are exact and rounded once in both; GELU and GELU' have the same arithmetic in both."""
+    from gcow_b200.ops import kernels as K_
+    torch.manual_seed(M + N + K)
+    mk = lambda r, c, lo, hi: torch.randint(lo, hi, (r, c + 8), device="cuda").bfloat16()[:, :c]      # rows apart
+    a, b, res, x = mk(M, K, -1, 2), mk(K, N, -1, 2) if b_t else mk(N, K, -1, 2), mk(M, N, -8, 9), mk(M, N, -3, 4)
+    bias, pre = torch.randint(-9, 10, (N,), device="cuda").float(), {}
+    forms = [dict(), dict(bias=bias), dict(bias=bias, gelu=True), dict(residual=res), dict(bias=bias, residual=res)]
+    if N % 32 == 0:
+        forms += [dict(gelu_grad_of=x), dict(gelu_grad_of=x, residual=res), dict(bias=bias, gelu=True, pre_gelu_out=0), dict(gelu=True, residual=res, pre_gelu_out=0)]
+    for form in forms:
+        got = []
+        for pair in (None, False):
+            monkeypatch.setattr(K_, "_pair_gemm", pair)
+            out, kw = mk(M, N, 0, 1), dict(form)
+            if "pre_gelu_out" in kw:
+                kw["pre_gelu_out"] = mk(M, N, 0, 1)
+            K_.gemm_bf16(a, b, b_t=b_t, out=out, **kw)
+            got.append((out, kw.get("pre_gelu_out")))
+        assert torch.equal(got[0][0], got[1][0]), sorted(form)
+        assert got[0][1] is None or torch.equal(got[0][1], got[1][1])
+    K_.check_errors()
+
+
 @pytest.mark.parametrize("M,N,K", [(8, 32, 64), (300, 96, 64), (1100, 1120, 192), (19000, 544, 64)])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_pair_gemm_side_operands_with_everything(M, N, K, shift, monkeypatch):
