@@ -732,9 +732,11 @@ int gcow_wgrad_slabs(int64_t M, int64_t N, int64_t K) {
 // How many slices of the reduction gcow_gemm2_wgrad cuts an M x N result over K rows into; 0: not taken (an operand narrower
 // than a tile, or no cluster launches). Fewer tiles than pairs leave the others idle, and slices cost a pass over their M x N
 // partial results: the count that a model of the two puts lowest, in us, fitted to 1024 to 50176 rows and results of 256 x 256 to
-// 4096 x 1024 with 1 to 64 slices: 8 + 0.71 per stage of 128 rows, 1.5 for a further round of tiles, and for the ordered sum 1.8 + 0.003 s^2 +
-// (4.5 + 0.35 s) per million elements. 3000 rows to 768 x 3072: one slice 26.2 us, two 31.2; 6144 to 768 x 768 six 23.6, eight 21.6; 16384 to
-// 1024 x 4096 one 100 (one-CTA kernel 113), to 768 x 3072 two 69 (75).
+// 4096 x 4096 with 1 to 64 slices, launches with their sums in a chain: 0.7 per stage of 128 rows, 4 for a further round of tiles, and for the ordered
+// sum 0.0014 s^2 + (1.17 s - 0.8) per million elements, half as much again where the partial results no longer fit the L2. An earlier model, of a
+// slower kernel (0.71, 1.5 a round, 1.8 + 0.003 s^2 + (4.5 + 0.35 s) per million), cut less: 1024 rows to 768 x 768 one slice 12.8 us, four 10.2; 3000 to
+// 2304 x 768 one 22.1, two 17.9; 4096 to 768 x 3072 one 28.1, two 22.0; 8192 to 3072 x 1024 one 47.2, three 45.2; 6144 to 4096 x 4096 still one, 153, two
+// 172. Where it cut more its count stays (8192 to 512 x 512 sixteen 16.7, thirteen 13.8): fewer slices are longer sums.
 // No accumulator takes more stages than one of the slabs above: the tensor core cuts the running sum at every step, and the error
 // grows with the number of steps (relative 2-norm, noise: 512 rows 4.7e-7, 1024 1.0e-6, 4096 4.4e-6). Where every pair has one
 // item at most, its slice is shared by two accumulators: 1024 rows to 1024 x 1024 in one slice 14.2 us, in two slices 17.3, on
@@ -744,17 +746,24 @@ int gcow_gemm2_wgrad_slices(int M, int N, int K) {
   if (max_pairs <= 0 || M < 256 || N < 256 || M % 64 || N % 64 || K < 1024) return 0;
   const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   const int kblocks = (K + BK - 1) / BK, slab = K / gcow_wgrad_slabs(M, N, K), longest = (slab + BK - 1) / BK;
-  int best = 1;
-  double least = 1e30;
-  for (int s = 1; s <= 64 && kblocks / s >= 2; s++) {
-    const int per = (kblocks + s - 1) / s;
-    if ((s - 1) * per >= kblocks || (tiles * s <= max_pairs ? (per + 1) / 2 : per) > longest) continue;   // an empty slice; one too long
-    const long long rounds = (tiles * s + max_pairs - 1) / max_pairs;
-    const double cost = 8.0 + (double)rounds * per * 0.71 + (double)(rounds - 1) * 1.5 +
-                        (s > 1 ? 1.8 + 0.003 * s * s + (double)M * N * 1e-6 * (4.5 + 0.35 * s) : 0.0);
-    if (cost < least) { least = cost; best = s; }
-  }
-  return best;
+  const auto stages = [&](int s) { const int per = (kblocks + s - 1) / s; return tiles * s <= max_pairs ? (per + 1) / 2 : per; };   // per accumulator
+  const auto rounds = [&](int s) { return (double)((tiles * s + max_pairs - 1) / max_pairs); };
+  const auto cheapest = [&](int most, auto cost) {
+    int best = 1;
+    double least = 1e30;
+    for (int s = 1; s <= 64 && kblocks / s >= 2; s++) {
+      const int per = (kblocks + s - 1) / s;
+      if ((s - 1) * per >= kblocks || stages(s) > most) continue;   // an empty slice; one too long
+      const double c = cost(s, rounds(s), (double)per);
+      if (c < least) { least = c; best = s; }
+    }
+    return best;
+  };
+  const double size = (double)M * N * 1e-6;
+  const int before = cheapest(longest, [&](int s, double r, double per) { return r * per * 0.71 + (r - 1) * 1.5 + (s > 1 ? 1.8 + 0.003 * s * s + size * (4.5 + 0.35 * s) : 0.0); });
+  return cheapest(stages(before), [&](int s, double r, double per) {
+    return r * per * 0.7 + (r - 1) * 4.0 + (s > 1 ? 0.0014 * s * s + size * (1.17 * s - 0.8) * (size * s > 24 ? 1.5 : 1.0) : 0.0);
+  });
 }
 
 // Partial column sums per slice that gcow_gemm2_wgrad leaves for a result of N columns.
