@@ -120,15 +120,18 @@ __device__ __forceinline__ Unit unit_at(int u, int mode, int tiles, int heads) {
 // The barriers of a CTA are numbered, and a role keeps the parities it waits for next in one word.
 //
 // B 32, S 512, 16 heads: forward 123 us with one tile in flight and the probabilities through shared memory, now 67 (0.51
-// PFLOP/s; the 134 M exponentials take 29 at 16 a clock and SM); backward 327, now 233 (delta 15, the rest 0.55 PFLOP/s;
-// 251 with one issuing warp per tile in the backward pass, 242 with dQ behind dK/dV, 231 as a launch of its own beside it).
-// One head of 512: backward 24.8 us.
+// PFLOP/s; the 134 M exponentials take 29 at 16 a clock and SM); backward 327, now 211 (delta 12; 233 with the queries' statistics fetched one
+// row a lane and one lane of a diverged warp issuing; before that 251 with one issuing warp per tile in the backward pass, 242 with dQ behind
+// dK/dV, 231 as a launch of its own beside it). One head of 512: backward 24.8, now 16.5 us.
+// Bound by the row warps' chains of load, exponentials and stores, two warps a scheduler (four backward): a block of the forward pass takes one 3900
+// cycles, of which exponentials 1640, epilogue and stores 780, waits for the scores 460, where the exponential unit needs 1024. A quarter of the
+// exponentials as polynomials on the multiply-add pipe: forward 64.7, 65.8, backward 210, 205 but short sequences 2 to 5 % longer.
 //
 // What the issuing warps do per product decides the pace. As code of one thread alone, with the descriptors worked out where
 // they are used, a step of four to eight MMAs took it 1500 cycles (forward, B 32, S 512, 16 heads: 131 us): every operand of
 // an MMA is a uniform register, which a divergent thread has to fill one by one. So the whole warp runs the loop, all its
-// values are uniform, and one lane executes the MMAs, commits and copies alone (95 us). A wait that has nothing to wait for
-// still takes 200 cycles and an MMA 70 to 80, so each tile has a warp of its own.
+// values are uniform, and one elected lane executes the MMAs, commits and copies alone (95 us). A wait that has nothing to wait for
+// still takes 110 cycles and an MMA with its descriptors 70, so each tile has a warp of its own.
 struct Phases {
   uint32_t bits = 0;
   __device__ __forceinline__ uint32_t next(int i) {

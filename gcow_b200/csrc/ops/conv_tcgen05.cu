@@ -27,9 +27,9 @@
 // epilogue warps read them back with tcgen05.ld. No multicast; every wait is bounded and
 // gives up by raising an error word.
 //
-// What sets the speed (measured): a TMA copy costs a few hundred cycles per instruction
-// on top of its bytes, and an M128 x N x K16 MMA takes about as long for N = 64 as for
-// N = 256. So a stage is fetched with as few, as large boxes as possible - the forward
+// What sets the speed (measured): an M128 x N x K16 MMA takes the tensor core 48 cycles at N = 64, 64 at 128 and 128 at 256, so narrow tiles do
+// not fill it, and the issuing warp some 70 cycles with its descriptors; a copy has the issuing lane's time and its own latency besides its
+// bytes. So a stage is fetched with as few, as large boxes as possible - the forward
 // tile is one box of up to 256 pixels (two 128-row accumulators that share the filter
 // tile), the weight gradient folds its 64-channel groups into a fifth box dimension -
 // and the launcher picks the tile from a small cost model of those two effects.
@@ -1255,8 +1255,9 @@ static int stages_for(int halves, int bn_cols) {
   return st;
 }
 
-// Cycles of one reduction step as measured on B200: every TMA copy costs about 220 cycles plus its bytes at
-// about 100 bytes per cycle, every M128 x N x K16 MMA about 128 cycles whatever N; the slower side wins.
+// Cycles of one reduction step, for choosing tiles: a copy 220 plus its bytes at 100 per cycle, an M128 x N x K16 MMA 128 whatever N; the
+// slower side wins. Fitted when one lane of a diverged warp issued both, which made narrow MMAs look as long as wide ones; with elected lanes a
+// step is shorter on both sides; the choices have not been fitted again.
 static double step_cycles(int copies, double bytes, int mmas) {
   const double tma = 220.0 * copies + bytes / 100.0, mma = 128.0 * mmas;
   return tma > mma ? tma : mma;

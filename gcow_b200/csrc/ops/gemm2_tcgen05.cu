@@ -7,7 +7,7 @@
 // each CTA ends up with its 128 rows x 256 columns in its own tensor memory - which leaves room for two
 // accumulators, so the epilogue of a tile overlaps the main loop of the next.
 // A stage holds 128 K-elements: the tensor maps describe an operand as {64, rows, K/64}, so ONE 32 KB box per
-// operand brings both 64-wide K chunks (a TMA copy costs a few hundred cycles per instruction besides its bytes).
+// operand brings both 64-wide K chunks (a copy costs its issue and its latency besides its bytes).
 //
 // Signalling inside the pair (no multicast qualifier anywhere; remote barriers are addressed with mapa):
 //   full[s]       lives in CTA 0; armed by CTA 0's producer with the bytes of both CTAs' copies, which both

@@ -786,8 +786,6 @@ int gcow_softmax_bwd(const void* dp, const void* p, void* ds, int64_t rows, int 
   return (int)cudaGetLastError();
 }
 
-// Column sums of a bf16 [rows, cols] matrix (ld even, cols even) into fp32 out[cols];
-// `part` must hold gcow_colsum_parts(rows) * cols floats.
 // Both sums of partial results of a linear layer: a weight gradient of n elements (parts 0: there is none to add up) and a bias
 // gradient of bias_n. n a multiple of 4, part and out at multiples of 16 bytes.
 int gcow_reduce_weight_bias(const float* part, float* out, int parts, int64_t n, const float* bias_part, float* bias_out, int bias_parts,
@@ -798,6 +796,8 @@ int gcow_reduce_weight_bias(const float* part, float* out, int parts, int64_t n,
                          (const float4*)part, (float4*)out, parts, (int)(n / 4), bias_part, bias_out, bias_parts, bias_n, first);
   return (int)cudaGetLastError();
 }
+// Column sums of a bf16 [rows, cols] matrix (ld even, cols even) into fp32 out[cols];
+// `part` must hold gcow_colsum_parts(rows) * cols floats.
 int gcow_colsum_parts(int rows) { int p = (rows + 127) / 128; return p < 128 ? (p < 1 ? 1 : p) : 128; }
 // Kernels that gcow_colsum launches: one (`part` is not used), or the partial sums and their reduction.
 int gcow_colsum_launches(const void* g, int rows, int cols, int ld) {

@@ -1,7 +1,7 @@
 // The training layers' autograd functions: allocation, routing and launches of the tensor-core, normalisation and attention
 // kernels, forward and backward, without Python between them.
 //
-// One BERT layer is 12 function calls and about 35 launches; as Python autograd functions with ctypes launches that was
+// One BERT layer is 12 function calls and about 25 launches; as Python autograd functions with ctypes launches that was
 // 1.1 ms of host time forward and backward, five times the device time of a small batch. The arithmetic, the kernels and
 // their order are those of the Python functions these replace (ops/kernels.py keeps the less used ones).
 #include "layers.h"
