@@ -32,7 +32,7 @@
 // bytes. So a stage is fetched with as few, as large boxes as possible - the forward
 // tile is one box of up to 256 pixels (two 128-row accumulators that share the filter
 // tile), the weight gradient folds its 64-channel groups into a fifth box dimension -
-// and the launcher picks the tile from a small cost model of those two effects.
+// and the launcher picks the tile from a small model of steps, epilogues and rounds of tiles (fwd_plan).
 //
 // Replaces the cuDNN 3x3 convolutions behind nn.Conv2d in the reference's models
 // (hw/models/resenet.py:14,48-50).
@@ -1255,29 +1255,31 @@ static int stages_for(int halves, int bn_cols) {
   return st;
 }
 
-// Cycles of one reduction step, for choosing tiles: a copy 220 plus its bytes at 100 per cycle, an M128 x N x K16 MMA 128 whatever N; the
-// slower side wins. Fitted when one lane of a diverged warp issued both, which made narrow MMAs look as long as wide ones; with elected lanes a
-// step is shorter on both sides; the choices have not been fitted again.
-static double step_cycles(int copies, double bytes, int mmas) {
-  const double tma = 220.0 * copies + bytes / 100.0, mma = 128.0 * mmas;
-  return tma > mma ? tma : mma;
-}
-
-// One or two 128-row accumulators per forward tile: fewer, larger copies against fewer tiles to spread over the SMs.
-static int fwd_halves(int Wo, int Ho, int N, int tiles_c, int ksteps, int bn_cols, int sms) {
-  double cost[3] = {0, 0, 0};
-  for (int hv = 1; hv <= 2; hv++) {
-    int bw, bh, bn;
-    pick_box(Wo, Ho, N, 128 * hv, 0, &bw, &bh, &bn);
-    const long long tiles = (long long)((Wo + bw - 1) / bw) * ((Ho + bh - 1) / bh) * ((N + bn - 1) / bn) * tiles_c;
-    const long long waves = (tiles + sms - 1) / sms;
-    cost[hv] = (double)waves * ksteps * step_cycles(2, hv * HALF_BYTES + bn_cols * 128.0, 4 * hv);
+// Forward tile: `cols` output channels by one or two accumulators of 128 pixels. A model in us picks it: per round of tiles the longer one of the
+// reduction's steps and the epilogue. A step takes what its latency is where few CTAs run, and what the L2 delivers to all of them where many do
+// (32 KB to each of 148 CTAs in 0.31 us). Two accumulators of 256 channels fill the tensor memory, so their epilogue no longer
+// overlaps the next tile (256 x 28 x 28, 256 -> 512 channels, 1 x 1: 86 us, one 68). Fitted to 48 forward passes and input gradients of batches
+// of 8 to 256; its choice takes 0.6 % longer than the best tile, that of an earlier model of copies and MMAs 9.5 %. us,
+// that one, this one: 8 x 14 x 14, 256 -> 256 15.6, 11.6; 8 x 7 x 7, 512 -> 512 25.4, 18.2; 32 x 14 x 14, 256 -> 256 15.9, 13.1; 100 x 56 x 56, 128 -> 128 stride 2,
+// input gradient 73.4, 61.4; 100 x 28 x 28, 256 -> 512, 1 x 1 41.0, 29.9; 256 x 7 x 7, 1024 -> 2048, 1 x 1 50.0, 45.0.
+struct FwdPlan { int cols, halves, bw, bh, bn; };
+static FwdPlan fwd_plan(int Wo, int Ho, int N, int Co, int ksteps, bool strided, int sms) {
+  struct Tile { int cols, halves; double few, all, epilogue, epilogue_strided; };        // us
+  static constexpr Tile tiles[] = {{64, 1, .355, .355, 1.2, 1.2}, {64, 2, .43, .43, 2.2, 2.2}, {128, 1, .2, .31, 2.2, 3.05}, {128, 2, .35, .47, 4.6, 5.8},
+                                   {256, 1, .33, .42, 3.1, 3.1}, {256, 2, .83, .9, 7.8, 7.8}};
+  FwdPlan best{};
+  double least = 1e30;
+  for (const Tile& t : tiles) {
+    if (Co <= 64 ? t.cols != 64 : t.cols == 64 || (Co <= 128 && t.cols == 256)) continue;
+    FwdPlan q{t.cols, t.halves, 0, 0, 0};
+    pick_box(Wo, Ho, N, 128 * t.halves, 0, &q.bw, &q.bh, &q.bn);
+    const long long n = (long long)((Wo + q.bw - 1) / q.bw) * ((Ho + q.bh - 1) / q.bh) * ((N + q.bn - 1) / q.bn) * ((Co + t.cols - 1) / t.cols);
+    const double shared = n < sms ? t.all * (double)n / sms : t.all, steps = ksteps * (shared > t.few ? shared : t.few);
+    const double tail = strided ? t.epilogue_strided : t.epilogue;
+    const double cost = (double)((n + sms - 1) / sms) * (steps > tail ? steps : tail);
+    if (cost < least) { least = cost; best = q; }
   }
-  // two 256-column accumulators fill the tensor memory: the epilogue no longer overlaps the next tile, and the
-  // 64 KB stages leave a ring of three (measured: 1.45 x the modelled step)
-  if (bn_cols == 256) cost[2] *= 1.45;
-  int halves = cost[2] < cost[1] ? 2 : 1;
-  return halves;
+  return best;
 }
 
 struct WgradPlan { int bw, bh, bn, tiles_w, tiles_h, tiles_n, split, per, b_chunks, halves; };
@@ -1321,11 +1323,9 @@ static int conv_fwd_launch(const void* x, const void* w, void* y, const float* b
   if ((uintptr_t)y & 15) return -1;
   const int sms = device_sms();
   Params p{};
-  p.bn_cols = Co <= 64 ? 64 : (Co <= 128 ? 128 : 256);
-  const int tiles_c = (Co + p.bn_cols - 1) / p.bn_cols;
-  const int ksteps = kh * kw * (Ci / 64);
-  const int halves = fwd_halves(Wo, Ho, N, tiles_c, ksteps, p.bn_cols, sms);
-  pick_box(Wo, Ho, N, 128 * halves, 0, &p.bw, &p.bh, &p.bn);
+  const FwdPlan plan = fwd_plan(Wo, Ho, N, Co, kh * kw * (Ci / 64), out_step > 1, sms);
+  const int halves = plan.halves, tiles_c = (Co + plan.cols - 1) / plan.cols;
+  p.bn_cols = plan.cols; p.bw = plan.bw; p.bh = plan.bh; p.bn = plan.bn;
   p.tiles_w = (Wo + p.bw - 1) / p.bw; p.tiles_h = (Ho + p.bh - 1) / p.bh; p.tiles_n = (N + p.bn - 1) / p.bn;
   p.stages = stages_for(halves, p.bn_cols);
   p.out = y; p.bias = bias; p.N = N; p.H = Ho; p.W = Wo; p.Ci = Ci; p.Co = Co;
@@ -1631,11 +1631,9 @@ int gcow_conv_flip_weights(const void* w, void* wt, int Co, int kh, int kw, int 
 // columns per tile, bw, bh, bn, pipeline stages}. For tests and tuning; needs no GPU.
 void gcow_conv_fwd_plan(int N, int Hin, int Win, int Ci, int Co, int kh, int kw, int pad_h, int pad_w, int sms, int* out) {
   const int Ho = Hin + 2 * pad_h - kh + 1, Wo = Win + 2 * pad_w - kw + 1;
-  const int bn_cols = Co <= 64 ? 64 : (Co <= 128 ? 128 : 256);
-  const int halves = fwd_halves(Wo, Ho, N, (Co + bn_cols - 1) / bn_cols, kh * kw * (Ci / 64), bn_cols, sms);
-  out[0] = halves; out[1] = bn_cols;
-  pick_box(Wo, Ho, N, 128 * halves, 0, &out[2], &out[3], &out[4]);
-  out[5] = stages_for(halves, bn_cols);
+  const FwdPlan plan = fwd_plan(Wo, Ho, N, Co, kh * kw * (Ci / 64), false, sms);
+  out[0] = plan.halves; out[1] = plan.cols; out[2] = plan.bw; out[3] = plan.bh; out[4] = plan.bn;
+  out[5] = stages_for(plan.halves, plan.cols);
 }
 
 // The pixel box chosen for given extents: out = {bw, bh, bn}. For tests of the tiling rule.

@@ -98,6 +98,25 @@ def test_weight_stationary_kernel_serves_the_64_channel_layers_and_agrees_with_t
     assert lib.gcow_conv_wgrad_ws_split(N, H, W) > 1 and lib.gcow_conv_wgrad_ws_split(N, H, 63) == 0
 
 
+# Every forward tile of 256 and more output channels: 128 or 256 channels wide, 128 or 256 pixels, also where the last tile has few channels or pixels
+@pytest.mark.parametrize("N,C,H,W,Co,tile", [(2, 64, 9, 7, 256, (1, 128)), (3, 64, 10, 11, 264, (1, 128)), (40, 64, 28, 28, 320, (2, 128)), (256, 64, 7, 7, 512, (1, 256)),
+                                             (2, 320, 5, 5, 512, (1, 128)), (256, 512, 7, 7, 512, (2, 256))])
+def test_every_forward_tile_of_wide_layers(N, C, H, W, Co, tile):
+    """Against float64 on the same bf16 operands: fp32 sums of 9 C products (2^-24 of the sum of magnitudes a step at most) and bf16's rounding."""
+    import ctypes
+    from gcow_b200.ops import kernels as K
+    plan = (ctypes.c_int * 6)()
+    K._native.cuda().gcow_conv_fwd_plan(N, H, W, C, Co, 3, 3, 1, 1, 148, plan)
+    assert (plan[0], plan[1]) == tile
+    torch.manual_seed(C + Co)
+    x, w, b = _mk(N, C, H, W, Co, 3, 3)
+    got = K.conv_igemm(x, w, b, (1, 1))[:3].double()
+    K.check_errors()
+    conv = lambda f: torch.nn.functional.conv2d(f(x[:3].double()), f(w.bfloat16().double()), f(b.double()), padding=1)
+    want, size = conv(lambda v: v), conv(torch.abs)
+    assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 9 * C * 2.0 ** -24 * size).all())
+
+
 def test_operand_swapped_forward_agrees_with_the_plain_one(monkeypatch):
     import ctypes
     from gcow_b200.ops import kernels as K
