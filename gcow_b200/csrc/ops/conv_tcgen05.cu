@@ -1289,11 +1289,20 @@ static WgradPlan wgrad_plan(int N, int Ho, int Wo, int Ci, int Co, int taps, int
   pick_box(Wo, Ho, N, 64, 1, &q.bw, &q.bh, &q.bn);
   q.tiles_w = (Wo + q.bw - 1) / q.bw; q.tiles_h = (Ho + q.bh - 1) / q.bh; q.tiles_n = (N + q.bn - 1) / q.bn;
   const int chunks = q.tiles_w * q.tiles_h * q.tiles_n;
-  q.halves = Co >= 256 ? 2 : 1;                                 // 256 output rows per tile share each X box
-  const int base = ((Co + 128 * q.halves - 1) / (128 * q.halves)) * ((taps * Ci + 255) / 256);
-  int split = sms / base;                                       // one wave: never more tiles than SMs
-  if (split > (chunks + 7) / 8) split = (chunks + 7) / 8;      // at least 8 pixel boxes per CTA
-  if (split < 1) split = 1;
+  // 256 output rows per tile share each X box; where a small batch leaves few boxes, tiles of 128 rows make twice as many CTAs of them, as long as no sum
+  // gets longer than with 256 rows and eight boxes per CTA at least. us with the ordered sum, before, now: 8 x 14 x 14, 256 -> 256, 3 x 3 16.4, 12.9;
+  // 8 x 7 x 7, 512 -> 512 17.8, 12.1; 8 x 56 x 56, 256 -> 512, 1 x 1 stride 2 17.0, 12.7, 64 -> 64, 1 x 1 13.0, 9.3; from 32 images on as before (with 128
+  // rows there 32 x 14 x 14 20.6, 17.4, but 8 pieces for 13, and 256 x 14 x 14 47, 56).
+  const auto cut = [&](int halves, int boxes) {                 // into one round of tiles at most, with `boxes` pixel boxes per CTA at least
+    const int base = ((Co + 128 * halves - 1) / (128 * halves)) * ((taps * Ci + 255) / 256), most = (chunks + boxes - 1) / boxes;
+    int split = sms / base < most ? sms / base : most;
+    if (split < 1) split = 1;
+    const int per = (chunks + split - 1) / split;
+    return (chunks + per - 1) / per;                            // no empty one
+  };
+  const int together = Co >= 256 ? cut(2, 8) : 0, apart = cut(1, 4);
+  q.halves = apart >= together ? 1 : 2;
+  const int split = q.halves == 2 ? together : apart;
   q.per = (chunks + split - 1) / split;
   q.split = (chunks + q.per - 1) / q.per;                       // no empty split
   const int cchunks = Ci / 64;

@@ -346,3 +346,19 @@ def test_cast_to_bf16(n, off):
     p = ctypes.c_void_p
     assert _native.cuda().gcow_cast_bf16(p(x.data_ptr()), p(out.data_ptr()), ctypes.c_uint64(n), p(torch.cuda.current_stream().cuda_stream)) == 0
     assert torch.equal(out[:n].view(torch.int16), x.bfloat16().view(torch.int16)) and bool((out[n:] == 7).all())
+
+
+# Few pixel boxes: one or two per CTA, 128 rows of the result per tile for 256 and more channels, a last tile that overhangs
+@pytest.mark.parametrize("N,C,H,W,Co,k", [(1, 64, 4, 5, 256, 3), (2, 64, 9, 7, 320, 3), (8, 128, 14, 14, 256, 3), (3, 64, 30, 31, 64, 3), (8, 64, 7, 7, 512, 1)])
+def test_weight_gradients_of_small_batches(N, C, H, W, Co, k, monkeypatch):
+    """Whole numbers: the products' sums are below 2^24 and exact in fp32 in any order."""
+    from gcow_b200.ops import kernels as K
+    for v in ("GCOW_CONV_WS_WGRAD", "GCOW_CONV_HALO"):
+        monkeypatch.setenv(v, "0")
+    torch.manual_seed(N + Co)
+    mk = lambda c: torch.randint(-2, 3, (N, c, H, W), device="cuda").bfloat16().contiguous(memory_format=torch.channels_last)
+    x, gy, w = mk(C), mk(Co), torch.zeros(Co, C, k, k, device="cuda").contiguous(memory_format=torch.channels_last).requires_grad_(True)
+    K.conv_igemm(x, w, None, (k // 2, k // 2)).backward(gy)
+    K.check_errors()
+    want = torch.nn.grad.conv2d_weight(x.double(), w.shape, gy.double(), padding=k // 2)
+    assert torch.equal(w.grad.double(), want)
