@@ -550,9 +550,10 @@ inline bool wide_clusters() {
 // per CTA. extra: it reads or writes another tensor besides (a residual, a second gradient, the residual's gradient).
 // All clusters are resident at once, with 64 CTAs at least to fetch for, and small clusters before large ones: sixteen CTAs have to find room in
 // one part of the GPU, so of those no more than 128. Shares of 52 KB leave two CTAs on an SM room to work while the other one waits. us, three launches, one:
-// forward and backward of 784 x 2048 12.2, 6.0 and 16.2, 6.0; 3136 x 512 10.8, 6.0 and 14.6, 7.8; 12544 x 128 9.8, 6.4 and 11.5, 8.7; 3136 x 2048
-// 19.7, 10.2 and 23.8, 17.5; forward of 12544 x 512 18.2, 13.6, with ReLU and residual 18.1, 19.7. Outside: forward of 25088 x 256 with
-// ReLU 17.6, 18.4, of 50176 x 256 22.3, 29.6, backward of 12544 x 512 22.2, 22.7, of 12544 x 1024 33.2, 41.8, of 6272 x 1024 with all operands 25.2, 25.6.
+// forward and backward of 784 x 2048 11.4, 5.9 and 16.1, 5.9; 3136 x 512 9.6, 6.1 and 14.8, 7.8; 12544 x 128 8.4, 6.4 and 11.2, 8.7; 3136 x 2048
+// 18.6, 10.2 and 24.1, 17.6; forward of 12544 x 512 17.3, 13.9, of 25088 x 128 10.4, 9.8, with ReLU 10.7, 11.2, of 12544 x 256 with ReLU and residual 11.8,
+// 11.9. Outside, before the three launches' sums took one trip: forward of 25088 x 256 with ReLU 17.6, 18.4, of 50176 x 256 22.3, 29.6, backward of 12544 x
+// 512 22.2, 22.7, of 12544 x 1024 33.2, 41.8, of 6272 x 1024 with all operands 25.2, 25.6.
 struct HeldPlan { int ch, cluster; size_t bytes; };
 constexpr int kHeldFew = 52 * 1024;
 inline HeldPlan held_plan(int64_t R, int C, int tensors, bool extra) {
