@@ -12,7 +12,7 @@
 // Signalling inside the pair (no multicast qualifier anywhere; remote barriers are addressed with mapa):
 //   full[s]       lives in CTA 0; armed by CTA 0's producer with the bytes of both CTAs' copies, which both
 //                 complete on it (cp.async.bulk.tensor ... .cta_group::2 with CTA 0's barrier address);
-//   empty[s]      one per CTA; the MMA thread commits to its own and to the peer's;
+//   empty[s]      one per CTA; the MMA thread commits to its own and to the peer's, and the warps of CTA 0 that add up columns arrive on its own;
 //   tmem_full[a]  one per CTA, same; tmem_empty[a] lives in CTA 0, both CTAs' epilogue threads arrive on it.
 // Every wait is bounded; a CTA that gives up raises the error word, and its peer's waits then run out too.
 //
@@ -41,7 +41,7 @@ enum Side : int { kNothing = 0, kSum = 1, kArgument = 2 };      // a residual; t
 // 768 x 768 11.3, 10.4 and 13.3, 11.4).
 template <int SIDE, bool WIDE> struct Epilogue { static constexpr int WARPS = WIDE || SIDE ? 16 : 8, THREADS = 64 + 32 * WARPS; };
 // Warps of a weight gradient that add up the columns of A as they pass through shared memory (the bias gradient).
-constexpr int SUM_WARPS = 2;
+constexpr int SUM_WARPS = 4;
 template <bool A_MN, int SIDE, bool WIDE> constexpr int kThreads = Epilogue<SIDE, WIDE>::THREADS + (A_MN ? 32 * SUM_WARPS : 0);
 static_assert(Epilogue<kSum, false>::THREADS == Epilogue<kArgument, false>::THREADS && Epilogue<kSum, false>::THREADS == Epilogue<kNothing, true>::THREADS, "one launch shape");
 constexpr uint32_t TMEM_COLS = 512;
@@ -65,6 +65,8 @@ struct Params {
 
 // An item of work: a tile, or the left or right half of one, over a slice of the reduction.
 struct Item { int m0, n0, kb0, kb1, slice; bool half; };
+// Which half of a tile's rows a CTA of the pair takes: its own, in a weight gradient's odd tile columns the other one (see the column sums).
+template <bool A_MN> __device__ __forceinline__ int half_of(const Item& it, uint32_t rank) { return (int)rank ^ (A_MN ? it.n0 / BN & 1 : 0); }
 template <bool SLICES> __device__ __forceinline__ Item item_at(const Params& p, int i, int tiles, int kblocks) {
   Item r;
   r.half = i >= p.whole;
@@ -105,7 +107,7 @@ __device__ __forceinline__ void add8(float (&v)[8], const uint4& x) {
 }
 
 struct Smem {
-  uint64_t full[STAGES], empty[STAGES], landed[STAGES], tmem_full[2], tmem_empty[2], drain, side[16];
+  uint64_t full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], drain, side[16];
   uint32_t tmem_base;
   volatile uint32_t abort;
 };
@@ -174,8 +176,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const int kblocks = (p.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
-    const uint32_t readers = A_MN && p.aux ? 1 + SUM_WARPS : 1;
-    for (int s = 0; s < STAGES; s++) { mbar_init(&sm->full[s], 1); mbar_init(&sm->empty[s], readers); mbar_init(&sm->landed[s], 1); }
+    const uint32_t readers = A_MN && p.aux && rank == 0 ? 1 + SUM_WARPS : 1;
+    for (int s = 0; s < STAGES; s++) { mbar_init(&sm->full[s], 1); mbar_init(&sm->empty[s], readers); }
     for (int a = 0; a < 2; a++) { mbar_init(&sm->tmem_full[a], 1); mbar_init(&sm->tmem_empty[a], 2 * EPI_WARPS * 32); }
     mbar_init(&sm->drain, 1);
     if (SIDE) for (int w = 0; w < EPI_WARPS; w++) mbar_init(&sm->side[w], 1);
@@ -203,7 +205,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       bool ok = true;
       for (int i = pair; i < p.items && ok; i += pairs) {
         const Item it = item_at<A_MN>(p, i, tiles, kblocks);
-        const int m0 = it.m0 + (int)rank * 128, n0 = it.n0 + (int)rank * (it.half ? 64 : 128);
+        const int m0 = it.m0 + half_of<A_MN>(it, rank) * 128, n0 = it.n0 + (int)rank * (it.half ? 64 : 128);
         const CUtensorMap* const map_b = it.half ? &tmap_bh : &tmap_b;
         for (int kb = it.kb0; kb < it.kb1; kb++) {
           if (!(ok = mbar_wait_abortable(&sm->abort, &sm->empty[s], phase ^ 1, p.error, 1))) break;
@@ -247,10 +249,6 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           const uint32_t sa = smem_u32(base + s * STAGE_BYTES), sb = sa + OPER_BYTES;
           const uint32_t eb0 = map_to_cta(smem_u32(&sm->empty[s]), 0), eb1 = map_to_cta(smem_u32(&sm->empty[s]), 1);
           if (one) {
-            if (A_MN && p.aux) {                              // the warps that add up may read the stage too
-              mbar_arrive_cluster(map_to_cta(smem_u32(&sm->landed[s]), 0));
-              mbar_arrive_cluster(map_to_cta(smem_u32(&sm->landed[s]), 1));
-            }
 #pragma unroll
             for (int k = 0; k < BK / UMMA_K; k++) {
               const uint32_t in = (k & 3) * 32;                               // 64-wide chunk, then 32 bytes per K step
@@ -279,31 +277,36 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       }
     }
   } else if (A_MN && warp >= 2 + EPI_WARPS) {
-    // ------------------------------------------------- column sums of A (both CTAs, own 128 columns), where they are wanted
-    // The tiles of one row have the same part of A in shared memory, so tile column j takes every tiles_n-th group of four rows of a stage from
-    // the j-th on. A warp takes 64 columns, a lane 8 of them in one row of each group, which come from two of a row's 16-byte chunks in turn
-    // (128-byte swizzle). It adds up 16 rows or a few more, up to four such sums, and those, so that no chain is long.
-    // A stage's MMAs take longer than a share of its sums, so nothing waits for these. The product alone, with the column sums as kernels of their
-    // own, with these, us, each with its ordered sums: 16384 rows to 3072 x 1024 85.9, 107.6, 86.5; to 4096 x 1024 99.4, 130.6, 101.5; to 768 x 768
-    // 29.7, 39.1, 30.2; 1024 rows to 768 x 768 17.0, 19.6, 18.7; 16384 to 256 x 256, where a tile has all groups to itself, 14.6, 21.2, 18.6. Whole
-    // stages in turn instead of groups of rows held a stage for longer than its MMAs: 16384 rows to 4096 x 1024 122.
-    if (p.aux) {
-      const int w = warp - 2 - EPI_WARPS, row = lane >> 3, chunk = lane & 7;
+    // ------------------------------------------------- column sums of A (CTA 0), where they are wanted
+    // Ordinary loads may read what this CTA's own copies brought once full[s], which lives here, has completed. CTA 1 would need its copies' completion
+    // passed on, with a release and an acquire at cluster scope per stage: a BERT layer 1650 us instead of 1520, and in the MMA warp's loop
+    // 1930. So CTA 0 adds up alone. The tiles of one row have the same two halves of A in shared memory; in even tile columns CTA 0 takes the first, in
+    // odd ones the second, and either half's stages are shared by the columns of its parity: of `sharing` columns the j-th takes every
+    // sharing-th group of four rows, in turn by two pairs of warps. A warp takes 64 columns, a lane 8 of them in one row of each group, which come
+    // from two of a row's 16-byte chunks in turn (128-byte swizzle). It adds up 16 rows or a few more, up to four such sums, and those, so that no
+    // chain is long.
+    // A stage's MMAs take longer than a share of its sums, so hardly anything waits for these. The product alone, with the column sums as kernels of
+    // their own, with these, us, each with its ordered sums: 16384 rows to 3072 x 1024 80.9, 103.4, 79.0; to 4096 x 1024 96.1, 122.2, 97.1; to 768 x 768 29.9, 40.6,
+    // 30.8; 1024 rows to 768 x 768 12.4, 15.6, 12.8; 50176 to 512 x 512, where one tile column has all groups of a half, 31.5, 57.9, 35.8. Whole stages in turn
+    // instead of groups of rows held a stage for longer than its MMAs (16384 rows to 4096 x 1024 122). Both CTAs adding up for themselves, with the
+    // order between them left to chance, took 98.3 there and 29.7 for 768 x 768.
+    if (rank == 0 && p.aux) {
+      const int w = (warp - 2 - EPI_WARPS) & 1, turn = (warp - 2 - EPI_WARPS) >> 1, row = lane >> 3, chunk = lane & 7;
       const uint8_t* const mine = base + w * 16384 + row * 128;
       const int even = (chunk ^ row) * 16, odd = 512 + (chunk ^ (row + 4)) * 16;
       uint32_t s = 0, phase = 0;
       bool ok = true;
       for (int i = pair; i < p.items && ok; i += pairs) {
         const Item it = item_at<A_MN>(p, i, tiles, kblocks);
-        const int first = it.n0 / BN;
+        const int column = it.n0 / BN, sharing = (tiles_n + 1 - (column & 1)) / 2, first = (column >> 1) + sharing * turn;
         int rows = 0, held = 0;
         float sum[8] = {}, some[8] = {}, v[8] = {};
         for (int kb = it.kb0; kb < it.kb1; kb++) {
-          ok = __all_sync(0xffffffffu, mbar_wait_abortable(&sm->abort, &sm->landed[s], phase, p.error, 5)) != 0;
+          ok = __all_sync(0xffffffffu, mbar_wait_abortable(&sm->abort, &sm->full[s], phase, p.error, 5)) != 0;
           if (!ok) break;
           const uint8_t* const at = mine + s * STAGE_BYTES;
 #pragma unroll 4
-          for (int r = first; r < 32; r += tiles_n) {
+          for (int r = first; r < 32; r += 2 * sharing) {
             const uint4 x = *reinterpret_cast<const uint4*>(at + (r >> 1) * 1024 + (r & 1 ? odd : even));
             const uint32_t y[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
@@ -331,12 +334,16 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
           for (int d = 8; d < 32; d *= 2) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], d);
         }
-        const int m = it.m0 + (int)rank * 128 + w * 64 + chunk * 8;
+        // Two partial sums of a half per two tile columns. Behind the last of an odd number of columns nobody has the second half's: zeros.
+        const bool alone = column + 1 == tiles_n && !(column & 1);
+        const int m = it.m0 + half_of<A_MN>(it, 0) * 128 + w * 64 + chunk * 8;
+        float* const to = reinterpret_cast<float*>(p.aux) + (size_t)(it.slice * ((tiles_n + 1) & ~1) + (column & ~1) + turn) * p.M + m;
         if (lane < 8 && m < p.M) {                            // M is a multiple of 64
-          float* const to = reinterpret_cast<float*>(p.aux) + (size_t)(it.slice * tiles_n + it.n0 / BN) * p.M + m;
           *reinterpret_cast<float4*>(to) = make_float4(sum[0], sum[1], sum[2], sum[3]);
           *reinterpret_cast<float4*>(to + 4) = make_float4(sum[4], sum[5], sum[6], sum[7]);
         }
+        if (alone && lane < 8 && m + 128 < p.M)
+          *reinterpret_cast<float4*>(to + 128) = *reinterpret_cast<float4*>(to + 132) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
     }
   } else {
@@ -367,7 +374,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     [[maybe_unused]] auto ask_first = [&](int i) {
       if (i >= p.items) return;
       const Item it = item_at<A_MN>(p, i, tiles, kblocks);
-      ask(it.m0 + (int)rank * 128 + q * 32, it.n0 + (ew / 4) * ((it.half ? BN / 2 : BN) / GROUPS));
+      ask(it.m0 + half_of<A_MN>(it, rank) * 128 + q * 32, it.n0 + (ew / 4) * ((it.half ? BN / 2 : BN) / GROUPS));
     };
     if (SIDE) ask_first(pair);
     // A warp's 32 x 32 results to the matrix of `map`, through the staging buffer that the last store but one (sixteen warps: the last one) has left.
@@ -399,7 +406,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     for (int i = pair; i < p.items && ok; i += pairs, t++) {
       const Item it = next;
       if (i + pairs < p.items) next = item_at<A_MN>(p, i + pairs, tiles, kblocks);
-      const int m0 = it.m0 + (int)rank * 128, n0 = it.n0;
+      const int m0 = it.m0 + half_of<A_MN>(it, rank) * 128, n0 = it.n0;
       // this warp's
       const int cols = (it.half ? BN / 2 : BN) / GROUPS, chunks = cols / 32, col0 = (ew / 4) * cols;
       const uint32_t acc = t & 1, aphase = (t >> 1) & 1;
@@ -766,15 +773,15 @@ int gcow_gemm2_wgrad_slices(int M, int N, int K) {
   });
 }
 
-// Partial column sums per slice that gcow_gemm2_wgrad leaves for a result of N columns.
-int gcow_gemm2_wgrad_sums(int N) { return (N + BN - 1) / BN; }
+// Partial column sums per slice that gcow_gemm2_wgrad leaves for a result of N columns; 0: it has none to give, one tile column sees half of A's.
+int gcow_gemm2_wgrad_sums(int N) { return N <= BN ? 0 : ((N + BN - 1) / BN + 1) & ~1; }
 
 // parts[slice][M][N] fp32 = A^T B over the slice's rows, A [K][M], B [K][N] bf16 with contiguous rows: the weight gradient of a
 // linear layer. `slices` as gcow_gemm2_wgrad_slices has it. sums (or null): [slices * gcow_gemm2_wgrad_sums(N)][M] fp32, which add up to the
 // column sums of A, the bias gradient.
 int gcow_gemm2_wgrad(const void* A, const void* B, float* parts, float* sums, int M, int N, int K, int lda, int ldb, int slices, uint32_t* error,
                      void* stream) {
-  if (M <= 0 || N <= 0 || K <= 0 || slices <= 0 || M % 64 || N % 64 || lda % 8 || ldb % 8 || (((uintptr_t)parts | (uintptr_t)sums) & 15)) return -2;
+  if ((sums && N <= BN) || M <= 0 || N <= 0 || K <= 0 || slices <= 0 || M % 64 || N % 64 || lda % 8 || ldb % 8 || (((uintptr_t)parts | (uintptr_t)sums) & 15)) return -2;
   const int max_pairs = gcow_gemm2_max_pairs();
   if (max_pairs <= 0) return -2;
   CUtensorMap ma, mb;

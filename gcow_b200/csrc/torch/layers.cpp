@@ -268,6 +268,7 @@ Tensor wgrad(const Tensor& g, const Tensor& x, const Tensor& out, const On& on, 
   if (slices > 0) {                                          // CTA pairs, which cut the rows themselves
     const Tensor to = slices == 1 && out.defined() ? out : empty({slices, N, K}, at::kFloat, g);
     const int64_t bias_parts = bias ? slices * gcow_gemm2_wgrad_sums((int)K) : 0;
+    if (!bias_parts) bias = nullptr;
     const Tensor sums = bias ? empty({bias_parts, N}, at::kFloat, g) : Tensor();
     check(gcow_gemm2_wgrad(g.data_ptr(), x.data_ptr(), f32(to), f32(sums), (int)N, (int)K, (int)M, (int)g.stride(0), (int)x.stride(0), slices,
                            on.error, on.stream), "gcow_gemm2_wgrad");
