@@ -593,6 +593,29 @@ def test_batchnorm_of_tensors_held_in_shared_memory(N, C, H, W, res, relu, fork)
     assert torch.allclose(bn.running_var.double(), 0.81 + 0.19 * var, rtol=1e-5, atol=1e-6)
 
 
+@pytest.mark.parametrize("N,C,H,W", [(16, 2048, 7, 7), (1, 2048, 33, 50), (1, 128, 111, 113), (1, 64, 101, 259), (1, 256, 107, 61), (64, 512, 7, 7)])
+@pytest.mark.parametrize("mean,low,high", [(10, 4, 15), (100, 64, 127)])
+def test_batchnorm_variance_of_values_far_from_zero(N, C, H, W, mean, low, high):
+    """The variance is what is left of two sums that are 100 and 10000 times as large. With these values, multiples of 2^-5 below 16 and of 2^-1 below 128, every fp32
+    sum of 13 squares, a thread's share, is exact (less than 2^24 units), what lies behind in double is 2^-53 of 10000, and one rounding to fp32 is left."""
+    from gcow_b200 import _native
+    from gcow_b200.ops import nn as gnn
+    lib = _native.cuda()
+    lib.gcow_bn_launches.argtypes = [C_.c_int64, C_.c_int, C_.c_int, C_.c_int]
+    assert lib.gcow_bn_launches(N * H * W, C, 0, 0) == 1
+    torch.manual_seed(C + mean)
+    x = (torch.randn(N, C, H, W, device="cuda") + mean).clamp(low, high).bfloat16().contiguous(memory_format=torch.channels_last)
+    bn = gnn.BatchNorm2d(C, momentum=1.0).cuda()
+    y = bn(x)
+    xd = x.double()
+    want, mu = xd.var((0, 2, 3)), xd.mean((0, 2, 3))
+    assert ((bn.running_var.double() - want).abs() <= 2.0 ** -22 * want).all()
+    assert ((bn.running_mean.double() - mu).abs() <= 2.0 ** -23 * mu).all()
+    # x * scale + shift: two roundings of mean / deviation, and bf16's
+    z = (xd - mu.view(1, C, 1, 1)) / (xd.var((0, 2, 3), unbiased=False) + bn.eps).sqrt().view(1, C, 1, 1)
+    assert ((y.double() - z).abs() <= 2.0 ** -8 * z.abs() + 2.0 ** -21 * mean).all()
+
+
 def test_batchnorm_counts_training_steps_lazily():
     """num_batches_tracked is counted on the host by the own path and lands in the tensor when the state is saved,
     when PyTorch's own path runs, and not twice."""
