@@ -786,16 +786,6 @@ int gcow_softmax_bwd(const void* dp, const void* p, void* ds, int64_t rows, int 
   return (int)cudaGetLastError();
 }
 
-// Both sums of partial results of a linear layer: a weight gradient of n elements (parts 0: there is none to add up) and a bias
-// gradient of bias_n. n a multiple of 4, part and out at multiples of 16 bytes.
-int gcow_reduce_weight_bias(const float* part, float* out, int parts, int64_t n, const float* bias_part, float* bias_out, int bias_parts,
-                            int bias_n, void* stream) {
-  if (parts < 0 || bias_parts <= 0 || bias_n <= 0 || n < 0 || n > 0x7fffffff || n % 4 || (((uintptr_t)part | (uintptr_t)out) & 15)) return -1;
-  const unsigned first = parts ? (unsigned)((n / 4 + 255) / 256) : 0;
-  gcow::launch_dependent(reduce_weight_bias_kernel, dim3(first + (unsigned)((bias_n + 31) / 32)), dim3(256), 0, (cudaStream_t)stream,
-                         (const float4*)part, (float4*)out, parts, (int)(n / 4), bias_part, bias_out, bias_parts, bias_n, first);
-  return (int)cudaGetLastError();
-}
 // Column sums of a bf16 [rows, cols] matrix (ld even, cols even) into fp32 out[cols];
 // `part` must hold gcow_colsum_parts(rows) * cols floats.
 int gcow_colsum_parts(int rows) { int p = (rows + 127) / 128; return p < 128 ? (p < 1 ? 1 : p) : 128; }
@@ -825,6 +815,18 @@ int gcow_colsum(const void* g, float* part, float* out, int rows, int cols, int 
   else
     gcow::launch_dependent(reduce_partials_kernel, dim3((cols + 255) / 256), dim3(256), 0, (cudaStream_t)stream, (const float*)part, out,
                      parts, cols);
+  return (int)cudaGetLastError();
+}
+// Both sums of partial results of a linear layer: a weight gradient of n elements (parts 0: there is none to add up, and n, part and out are not
+// looked at) and a bias gradient of bias_n. n a multiple of 4, part and out at multiples of 16 bytes.
+int gcow_reduce_weight_bias(const float* part, float* out, int parts, int64_t n, const float* bias_part, float* bias_out, int bias_parts,
+                            int bias_n, void* stream) {
+  if (parts < 0 || bias_parts <= 0 || bias_n <= 0) return -1;
+  if (!parts) n = 0;
+  else if (n < 0 || n % 4 || n / 4 > 0x7fffffff - 255 || (((uintptr_t)part | (uintptr_t)out) & 15)) return -1;
+  const unsigned first = (unsigned)((n / 4 + 255) / 256);
+  gcow::launch_dependent(reduce_weight_bias_kernel, dim3(first + (unsigned)((bias_n + 31) / 32)), dim3(256), 0, (cudaStream_t)stream,
+                         (const float4*)part, (float4*)out, parts, (int)(n / 4), bias_part, bias_out, bias_parts, bias_n, first);
   return (int)cudaGetLastError();
 }
 

@@ -276,7 +276,7 @@ Tensor wgrad(const Tensor& g, const Tensor& x, const Tensor& out, const On& on, 
     if (bias) {                                              // N and K are multiples of 64
       const Tensor dw = slices > 1 && !out.defined() ? empty({N, K}, at::kFloat, g) : out;
       *bias = empty({N}, at::kFloat, g);
-      check(gcow_reduce_weight_bias(f32(to), slices > 1 ? f32(dw) : nullptr, slices > 1 ? slices : 0, N * K, f32(sums), f32(*bias), (int)bias_parts,
+      check(gcow_reduce_weight_bias(f32(to), slices > 1 ? f32(dw) : nullptr, slices > 1 ? slices : 0, slices > 1 ? N * K : 0, f32(sums), f32(*bias), (int)bias_parts,
                                     (int)N, on.stream), "gcow_reduce_weight_bias");
       g_launches++;
       return slices > 1 || out.defined() ? dw : to.view({N, K});

@@ -155,6 +155,43 @@ def test_bias_gradient_beside_the_weight_gradient(M, N, K):
         assert torch.equal(w.grad.double(), g.double().t() @ x.double())
 
 
+def test_bias_gradient_beside_weights_of_more_than_two_to_the_31_elements():
+    """A single slice leaves no partial weight gradients to add up, so their number of elements is no limit; as sums of their own they may be
+    as many as 4 (2^31 - 256). Whole numbers, exact in any order."""
+    import ctypes
+    from gcow_b200 import _native
+    from gcow_b200.ops import kernels as K_
+    M, N, K = 1024, 65536, 32768
+    lib = _native.cuda()
+    if lib.gcow_gemm2_wgrad_slices(N, K, M) != 1:
+        pytest.skip("clusters of two CTAs cannot be scheduled here")
+    torch.manual_seed(3)
+    g, x = (torch.randint(-2, 3, (M, n), device="cuda").bfloat16() for n in (N, K))
+    w = torch.zeros(N, K, device="cuda", requires_grad=True)
+    b = torch.zeros(N, device="cuda", requires_grad=True)
+    K_.linear(x, w, b).backward(g)
+    K_.check_errors()
+    assert torch.equal(b.grad.double(), g.double().sum(0))
+    rows = [0, 1, 255, 256, 32767, N - 1]
+    assert torch.equal(w.grad[rows].double(), g[:, rows].double().t() @ x.double())
+    del w, b, g, x
+    torch.cuda.empty_cache()
+    n, p, i64 = 2 ** 31 + 4, ctypes.c_void_p, ctypes.c_int64
+    part, out = torch.empty(2 * n, device="cuda"), torch.empty(n, device="cuda")
+    ends = [0, 1, 2 ** 31 - 1, 2 ** 31, n - 1]
+    part[ends] = torch.arange(1.0, 6.0, device="cuda")
+    part[[n + e for e in ends]] = 10 * torch.arange(1.0, 6.0, device="cuda")
+    bias_part, bias = torch.ones(3, 40, device="cuda"), torch.zeros(40, device="cuda")
+    fn = lambda parts, n, at=0: lib.gcow_reduce_weight_bias(p(part.data_ptr() + at), p(out.data_ptr()), parts, i64(n), p(bias_part.data_ptr()), p(bias.data_ptr()), 3, 40,
+                                                            p(torch.cuda.current_stream().cuda_stream))
+    assert fn(2, n) == 0 and torch.equal(out[ends], 11 * torch.arange(1.0, 6.0, device="cuda")) and bool((bias == 3).all())
+    bias.zero_()
+    assert fn(0, 2 ** 40 + 1, 4) == 0 and bool((bias == 3).all())
+    assert fn(2, 2 ** 33) == -1 and fn(2, 6) == -1 and fn(2, 8, 4) == -1 and fn(-1, 8) == -1
+    del part, out
+    torch.cuda.empty_cache()
+
+
 def test_wgrad_slices_are_no_longer_than_slabs():
     """The tensor core's running sum loses a little at every step, so a slice of the rows on CTA pairs has no more stages of 128 than
     a slab of the one-CTA route, which doubles the slabs while the tiles fit 148 CTAs and 512 rows are left - twice as
