@@ -544,6 +544,7 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   }
   if (fork) {
     Tensor again = x.variable_data();                       // the same memory, no autograd view of x
+    torch::autograd::impl::set_version_counter(again, torch::autograd::impl::version_counter(x));   // a change of it is one of the saved input
     if (node) {
       torch::autograd::set_history(out, node);
       torch::autograd::set_history(again, node);

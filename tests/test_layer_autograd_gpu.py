@@ -140,6 +140,27 @@ def test_forked_linear(rows, n, k):
     K.check_errors()
 
 
+@pytest.mark.parametrize("which", ["x", "again"])
+def test_forked_linear_sees_changes_in_place(which):
+    """Both tensors are the memory that the weight gradient reads, so a change of either between the passes is an error, as with torch's own layers."""
+    from gcow_b200.ops import kernels as K
+    from gcow_b200.ops import nn as gnn
+    lin = gnn.Linear(128, 64).cuda()
+    x = torch.randn(128, 128, device="cuda", requires_grad=True).bfloat16()
+    y, z = gnn.linear_fork(x, lin)
+    assert z._version == x._version
+    with torch.no_grad():
+        (x if which == "x" else z).mul_(2)
+    assert z._version == x._version > 0
+    with pytest.raises(RuntimeError, match="modified (by an )?inplace"):
+        (y.sum() + z.sum()).backward()
+    y, z = gnn.linear_fork(x.detach().requires_grad_(True), lin)
+    z = torch.relu_(z)                                       # with its history
+    with pytest.raises(RuntimeError, match="modified (by an )?inplace"):
+        (y.sum() + z.sum()).backward()
+    K.check_errors()
+
+
 def _grads(net, x, run):
     y = run(x)
     y.backward(torch.ones_like(y))
