@@ -1102,6 +1102,7 @@ PyObject* batchnorm_act(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (fork) {                                             // a second tensor on the same storage (not an autograd view of the first)
       y2 = empty({0}, at::kBFloat16, x);
       y2.set_(y.storage(), y.storage_offset(), y.sizes(), y.strides());
+      torch::autograd::impl::set_version_counter(y2, torch::autograd::impl::version_counter(y));   // a change of either is one of both
     }
   }
   if (node) torch::autograd::set_history(y, node);

@@ -161,6 +161,23 @@ def test_forked_linear_sees_changes_in_place(which):
     K.check_errors()
 
 
+@pytest.mark.parametrize("which", [0, 1])
+def test_forked_batchnorm_sees_changes_in_place(which):
+    """A consumer of one of the two results has saved the memory of both."""
+    from gcow_b200.ops import kernels as K
+    from gcow_b200.ops import nn as gnn
+    bn = gnn.BatchNorm2d(64).cuda()
+    x = torch.randn(4, 64, 9, 9, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last).requires_grad_(True)
+    pair = bn(x, relu=True, fork=True)
+    assert pair[0].data_ptr() == pair[1].data_ptr() and pair[0]._version == pair[1]._version
+    kept = pair[1 - which] ** 2
+    pair[which].add_(1)
+    assert pair[0]._version == pair[1]._version > 0
+    with pytest.raises(RuntimeError, match="modified by an inplace"):
+        kept.sum().backward()
+    K.check_errors()
+
+
 def _grads(net, x, run):
     y = run(x)
     y.backward(torch.ones_like(y))
