@@ -564,26 +564,32 @@ inline bool wide_clusters() {
 }
 
 // How a call that holds `tensors` tensors of R x C is laid out: `ch` channels to a cluster (0: it takes the three launches), `cluster` CTAs, bytes
-// per CTA. extra: it reads or writes another tensor besides (a residual, a second gradient, the residual's gradient).
+// per CTA. extra: it reads or writes another tensor besides (a residual, a second gradient, the residual's gradient); relu: it has one.
 // All clusters are resident at once, with 64 CTAs at least to fetch for, and small clusters before large ones: sixteen CTAs have to find room in
-// one part of the GPU, so of those no more than 128. Shares of 52 KB leave two CTAs on an SM room to work while the other one waits. us, three launches, one:
-// forward and backward of 784 x 2048 11.4, 5.9 and 16.1, 5.9; 3136 x 512 9.6, 6.1 and 14.8, 7.8; 12544 x 128 8.4, 6.4 and 11.2, 8.7; 3136 x 2048
-// 18.6, 10.2 and 24.1, 17.6; forward of 12544 x 512 17.3, 13.9, of 25088 x 128 10.4, 9.8, with ReLU 10.7, 11.2, of 12544 x 256 with ReLU and residual 11.8,
-// 11.9. Outside, before the three launches' sums took one trip: forward of 25088 x 256 with ReLU 17.6, 18.4, of 50176 x 256 22.3, 29.6, backward of 12544 x
-// 512 22.2, 22.7, of 12544 x 1024 33.2, 41.8, of 6272 x 1024 with all operands 25.2, 25.6.
+// one part of the GPU, so of those no more than 128. Shares of 52 KB leave two CTAs on an SM room to work while the other one waits; a forward call
+// that writes a mask or reads a residual has less to win, the less the fewer bytes its rows have in a CTA. us, three launches, one;
+// inside: forward of 784 x 2048 11.4, 5.9, 3328 x 2048 19.0, 10.3, 13312 x 1024 22.9, 21.7, with ReLU 23.7, 22.9, 26624 x 64 with ReLU 8.2, 7.3, 20480 x 128 9.6, 9.4, with residual
+// and ReLU 10976 x 128 8.4, 8.0, 10240 x 256 10.7, 10.0, 9408 x 512 15.3, 14.7, 18000 x 64 7.7, 7.6; backward of 3328 x 2048 24.1, 17.9, with ReLU 25.1, 22.0, 13312 x 256 17.0,
+// 15.4, with ReLU 17.4, 17.3, with all operands 10240 x 128 10.8, 10.8, 5120 x 512 17.1, 11.3.
+// Outside: forward of 26624 x 128 with ReLU 10.9, 11.4, with residual and ReLU 12544 x 128 8.3, 8.6, x 256 11.9, 12.1, 10240 x 512 15.6, 16.8, 20480 x 64 7.6, 7.9, by clusters of 16
+// channels 14000 x 128 8.6, 9.8, 20480 x 128 9.6, 12.0; by more CTAs or larger shares 25088 x 256 16.9, 17.8, x 512 21.4, 27.4, 13312 x 512 backward 22.6, 26.5, with all operands 13312 x 128
+// 11.8, 12.7, 9408 x 512 21.6, 22.3. Some calls there would gain: backward of 2205 x 2048 with all operands 22.3, 13.2 with shares of 104 KB, of 8192 x 512 18.9,
+// 15.9 with 256 CTAs in clusters of sixteen, of 12544 x 64 with residual 9.0, 7.8, forward of 18816 x 256 14.5, 13.8.
+// The backward instances spill up to 156 bytes of their 64 registers, which two CTAs on an SM leave them.
 struct HeldPlan { int ch, cluster; size_t bytes; };
-constexpr int kHeldFew = 52 * 1024;
-inline HeldPlan held_plan(int64_t R, int C, int tensors, bool extra) {
+inline HeldPlan held_plan(int64_t R, int C, int tensors, bool extra, bool relu) {
+  constexpr int KB = 1024;
   if (R > 0x7fffffff) return {0, 0, 0};
-  for (const int most : {kHeldFew, kHeldBytes}) {
+  for (const int most : {52 * KB, kHeldBytes}) {
     if (most == kHeldBytes && extra) break;
     for (const int ch : {32, 16}) {
       if (C % ch || (ch == 16 && most == kHeldBytes)) continue;
-      for (int cluster = 1; cluster <= 16; cluster *= 2) {
+      for (int cluster = 1; cluster <= (most == kHeldBytes && tensors == 1 ? 8 : 16); cluster *= 2) {
         const int64_t ctas = (int64_t)C / ch * cluster, bytes = (R + cluster - 1) / cluster * ch * 2 * tensors;
-        const int many = cluster < 16 ? 296 : most == kHeldBytes && tensors == 1 ? 64 : 128;
-        if (ctas >= 64 && ctas <= many && bytes <= (ch == 16 && extra ? 40 * 1024 : most) && (cluster < 16 || wide_clusters()))
-          return {ch, cluster, (size_t)bytes};
+        const bool wide_forward = cluster == 16 && tensors == 1;
+        const int many = cluster < 16 ? 296 : wide_forward && ch == 16 && extra ? 64 : 128;
+        const int limit = ch == 16 && extra ? (tensors == 1 ? 37 * KB : 40 * KB) : wide_forward && extra ? 44 * KB : wide_forward && ch == 16 && relu && ctas > 64 ? 40 * KB : most;
+        if (ctas >= 64 && ctas <= many && bytes <= limit && (cluster < 16 || wide_clusters())) return {ch, cluster, (size_t)bytes};
       }
     }
   }
@@ -635,8 +641,10 @@ extern "C" {
 
 int gcow_bn_supported(int C) { return shape_ok(C) ? 1 : 0; }
 // Kernels that a training call launches: one (`part` is not used), or two sweeps with the sums' second half between them.
-// extra: a residual forward, the residual's gradient backward.
-int gcow_bn_launches(int64_t R, int C, int backward, int extra) { return shape_ok(C) && held_plan(R, C, backward ? 2 : 1, extra != 0).ch ? 1 : 3; }
+// extra: 1 a residual forward, the residual's gradient backward; 2 a ReLU.
+int gcow_bn_launches(int64_t R, int C, int backward, int extra) {
+  return shape_ok(C) && held_plan(R, C, backward ? 2 : 1, extra & 1, extra & 2).ch ? 1 : 3;
+}
 int gcow_bn_parts(int64_t R, int C) { return shape_ok(C) ? grid_for(R, C) : 0; }
 
 // Training forward. part: gcow_bn_parts * 2 * C floats of scratch, or null where gcow_bn_launches says 1 (and mask is at a multiple of 4 bytes). stats: 4*C floats out
@@ -647,7 +655,7 @@ int gcow_bn_fwd_train(const void* x, const void* residual, void* y, void* mask, 
                       float momentum, int relu, void* stream) {
   if (!shape_ok(C) || R <= 0) return -1;
   cudaStream_t s = (cudaStream_t)stream;
-  const HeldPlan plan = held_plan(R, C, 1, residual != nullptr);
+  const HeldPlan plan = held_plan(R, C, 1, residual != nullptr, relu != 0);
   if (plan.ch && ((uintptr_t)mask & 3) == 0) {
     const int form = relu ? (mask ? 2 : 1) : 0;
     auto run = [&](auto ch) {
@@ -688,7 +696,7 @@ int gcow_bn_bwd3(const void* dy, const void* dy2, const void* mask, const void* 
                  void* dx, void* dres, float* dgamma, float* dbeta, float* part, int64_t R, int C, int relu, void* stream) {
   if (!shape_ok(C) || R <= 0 || (dy2 && !dres)) return -1;
   cudaStream_t s = (cudaStream_t)stream;
-  const HeldPlan plan = held_plan(R, C, 2, dres != nullptr);
+  const HeldPlan plan = held_plan(R, C, 2, dres != nullptr, relu != 0);
   if (plan.ch) {
     auto run = [&](auto ch) {
       return held_bwd<ch.value>(dy2 != nullptr, dres != nullptr, relu != 0, plan, C, s, (const bf16*)dy, (const bf16*)dy2, (const uint8_t*)mask, (const bf16*)x,

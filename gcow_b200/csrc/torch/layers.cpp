@@ -1023,7 +1023,7 @@ struct BatchNormNode : LayerNode {                          // inputs: x, gamma,
     // the masked (summed) gradient: the residual input's gradient, and what the second sweep reads
     Tensor dres;
     if (has_res || gy2.defined()) dres = empty_nhwc(x.size(0), C, x.size(2), x.size(3), x);
-    const int launches = gcow_bn_launches(R, (int)C, 1, dres.defined());
+    const int launches = gcow_bn_launches(R, (int)C, 1, (dres.defined() ? 1 : 0) | (relu ? 2 : 0));
     const Tensor part = launches > 1 ? empty({(int64_t)gcow_bn_parts(R, (int)C) * 2 * C}, at::kFloat, x) : Tensor();
     // dgamma and dbeta go straight into the two parameters' gradient tensors when the trainer pointed at them
     Tensor dgamma, dbeta, flat_g = target_matrix(target[0], 1, C, 4, &dgamma), flat_b;
@@ -1077,7 +1077,7 @@ PyObject* batchnorm_act(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const On on(x);
     const int64_t C = x.size(1), R = x.size(0) * x.size(2) * x.size(3);
     y = empty_nhwc(x.size(0), C, x.size(2), x.size(3), x);
-    const int launches = gcow_bn_launches(R, (int)C, 0, res.defined());
+    const int launches = gcow_bn_launches(R, (int)C, 0, (res.defined() ? 1 : 0) | (relu ? 2 : 0));
     const Tensor stats = empty({4 * C}, at::kFloat, x),
                  part = launches > 1 ? empty({(int64_t)gcow_bn_parts(R, (int)C) * 2 * C}, at::kFloat, x) : Tensor();
     const Tensor g32 = float_vector(gamma), b32 = float_vector(beta);

@@ -593,6 +593,35 @@ def test_batchnorm_of_tensors_held_in_shared_memory(N, C, H, W, res, relu, fork)
     assert torch.allclose(bn.running_var.double(), 0.81 + 0.19 * var, rtol=1e-5, atol=1e-6)
 
 
+# Per channel count the most rows that one launch takes: forward plain, with ReLU, with residual and ReLU, backward without and with another tensor
+@pytest.mark.parametrize("C,lines", [(2048, (6656, 6656, 3328, 3328, 1664)), (1024, (13312, 13312, 6656, 6656, 3328)), (512, (13312, 13312, 9472, 6656, 5120)),
+                                     (256, (13312, 13312, 11264, 13312, 6656)), (128, (26624, 20480, 11264, 13312, 10240)), (64, (26624, 26624, 18944, 13312, 10240)),
+                                     (32, (0, 0, 0, 0, 0))])
+def test_batchnorm_forms_on_either_side_of_their_lines(C, lines):
+    """Which form a call takes and its results against float64, with the most rows that one launch takes and with one more. Values have a mean near 0 and a
+    deviation near 1, so a result is off by bf16's rounding and a few fp32 roundings of numbers up to 5, and a sum by fp32's of its terms (below 2^-20 each)."""
+    from gcow_b200 import _native
+    from gcow_b200.ops import nn as gnn
+    lib = _native.cuda()
+    lib.gcow_bn_launches.argtypes = [C_.c_int64, C_.c_int, C_.c_int, C_.c_int]
+    for (backward, extra), most in zip(((0, 0), (0, 2), (0, 3), (1, 0), (1, 3)), lines):
+        for rows, launches in ((most, 1), (most + 1, 3)) if most else ((100, 3),):
+            assert lib.gcow_bn_launches(rows, C, backward, extra) == launches, (backward, extra, rows)
+            torch.manual_seed(rows)
+            x, r, g = (torch.randn(1, C, rows, 1, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last) for _ in range(3))
+            bn, x = gnn.BatchNorm2d(C, momentum=1.0).cuda(), x.requires_grad_(True)
+            y = bn(x, residual=r.requires_grad_(True) if extra & 1 else None, relu=bool(extra & 2))
+            y.backward(g)
+            xd = x.detach().double()
+            mean, var = xd.mean((0, 2, 3), keepdim=True), xd.var((0, 2, 3), unbiased=False, keepdim=True)
+            xh = (xd - mean) / (var + bn.eps).sqrt()
+            z = xh + (r.detach().double() if extra & 1 else 0)
+            assert ((y.double() - (z.clamp(min=0) if extra & 2 else z)).abs() <= 2.0 ** -8 * z.abs() + 2.0 ** -18).all()
+            gd = torch.where(y > 0, g, torch.zeros_like(g)).double() if extra & 2 else g.double()
+            assert torch.allclose(bn.bias.grad.double(), gd.sum((0, 2, 3)), rtol=0, atol=2.0 ** -20 * rows)
+            assert torch.allclose(bn.weight.grad.double(), (gd * xh).sum((0, 2, 3)), rtol=0, atol=2.0 ** -20 * rows)
+
+
 @pytest.mark.parametrize("N,C,H,W", [(16, 2048, 7, 7), (1, 2048, 33, 50), (1, 128, 111, 113), (1, 64, 101, 259), (1, 256, 107, 61), (64, 512, 7, 7)])
 @pytest.mark.parametrize("mean,low,high", [(10, 4, 15), (100, 64, 127)])
 def test_batchnorm_variance_of_values_far_from_zero(N, C, H, W, mean, low, high):
