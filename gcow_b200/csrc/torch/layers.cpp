@@ -212,8 +212,14 @@ Tensor gemm(const Tensor& a, const Tensor& b, const GemmOpts& o, const On& on) {
   // on both: pairs where a round's tiles are few (a pair fetches twice as much at once: 128 x 1024 x 1024 9.4, 6.6, 1024 x 256 x 64 5.0, 4.4; up to 8
   // tiles with 64 columns, 24 with 128, 37 with 256) and where there are several rounds of 256 columns (50176 x 1024 x 256 32.7, 28.7, with a bias
   // 38.0, 33.0; 12544 x 2048 x 256 19.1, 15.9); a single round of more than 37 tiles is one of twice as many CTAs without pairs' start (16384 x 256 x 64 5.2,
-  // 6.2, 4096 x 768 x 256 6.3, 6.6). Plain, 64 columns deep in few rounds 8192 x 1024 x 64 7.0, 7.2, and the longest streams 802816 x 256 x 64 84.4, 90.7,
-  // x 128 100.6, 103.9: on one CTA. A single row of 4096 columns or more is uneven on pairs (x 4096 22.7, 22.5 to 28).
+  // 6.2, 4096 x 768 x 256 6.3, 6.6). On one CTA: plain, 64 columns deep in few rounds 8192 x 1024 x 64 7.0, 7.2; plain with 524288 rows and more, where the two
+  // are uneven (524288 x 256 x 256 88.1, 90.5, 802816 x 256 x 256 134.9, 140.5, 1204224 x 256 x 128 152, 159, but 602112 x 256 x 256 120.6, 105.0, 802816 x 256 x 128 147, 116, x 64 84.4, 90.7
+  // and 136.6, 125.7 on two days; 401408 x 256 x 256 73.3, 70.5); a single row of 4096 columns or more (x 1024 9.5, 9.8; 8192 x 4096 23.3, 32.5).
+  // Few rows of a wide result (`wide`). Up to 128 rows, and from 257 to 384, half of a pair, or of one pair in two, has no rows, while the one-CTA kernel's tiles
+  // of 128 rows fit: 64 x 30528 x 768 12.1, 15.4, 128 x 50304 x 256 12.0, 13.6, 300 x 50304 x 256 with a bias 20.7, 25.9; where those are one round of CTAs, pairs need two: 300
+  // x 12288 x 4096 32.4, 43.6. Pairs all the same: deep and wide 128 x 50304 x 2048 55, 45, and with a residual, a kept argument or a GELU' factor 64 x 30528 x 768 19.2, 16.5.
+  // Up to 16 rows pairs wait for their short A (less than 64 K elements of it): 2 x 6144 x 4096 27.4, 32.1, 8 x 30528 x 4096 with a residual 55.9, 76.6; 16 x 8192 x 4096
+  // 28.1, 21.5.
   const bool can_pair = pair_gemm_enabled() && !o.a_t && !(flags & (kOutF32 | kAccumulate)) && !o.max_ctas && !o.tile_rows;
   const int64_t tiles = ((M + 255) / 256) * ((N + 255) / 256);
   const bool even = 2 * ((tiles + 147) / 148) <= (tiles + 73) / 74;
@@ -221,13 +227,21 @@ Tensor gemm(const Tensor& a, const Tensor& b, const GemmOpts& o, const On& on) {
                        (K >= 8192 || (K > 4096 && tiles > 296) || (K >= 2048 && tiles <= 148));
   const bool fits = K % 64 == 0 && N % (o.b_t ? 64 : 32) == 0 && lda % 8 == 0 && ldb % 8 == 0 && ldc % 8 == 0;
   const bool bare = !(flags & (kGelu | kResidual | kGeluGrad | kAuxOut)), plain = bare && !(flags & kBias), short_round = tiles > 37 && tiles <= 74;
+  const bool side = flags & (kResidual | kGeluGrad | kAuxOut), low = M <= 128 || (M > 256 && M <= 384);
+  const bool wide = M >= 1024 || tiles <= 16 ? false
+                    : tiles <= 37            ? M <= 16 && M * K < 65536 && (K >= 2048 || (bare && (K >= 512 || tiles > 24)))
+                    : side                   ? M <= 8 || (M * K < 65536 && K >= 1536)
+                    : tiles <= 74            ? false
+                    : M <= 128               ? tiles <= 148 || K < 2048 || M * K < 65536
+                                             : ((M + 127) / 128) * ((N + 255) / 256) <= 148 || (low && K < 2048 && K >= (bare ? 128 : 1024));
   const bool by_rule = fits && (M > 1 || N <= 3072) &&
                        (K >= 512 && M >= 1024 && N >= 256 ? !one_cta && !(bare && short_round && K <= 768 && N >= 768)
-                        : flags & (kResidual | kGeluGrad | kAuxOut) ? N >= 64
-                        : tiles <= 8                                ? N >= 64
-                        : tiles <= 24                               ? N >= 128
-                        : tiles <= 37                               ? N >= 256 && K >= 128
-                                                                    : !short_round && N >= 256 && !(plain && (M >= 524288 || (K < 128 && tiles <= 148))));
+                        : wide                            ? false
+                        : side                            ? N >= 64
+                        : tiles <= 8                      ? N >= 64
+                        : tiles <= 24                     ? N >= 128
+                        : tiles <= 37                     ? N >= 256 && K >= 128
+                                                          : !short_round && N >= 256 && !(plain && (M >= 524288 || (K < 128 && tiles <= 148))));
   if (can_pair && (o.pair < 0 ? by_rule : o.pair > 0)) {
     const int err = gcow_gemm2_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, lda, ldb, ldc, f32(o.bias),
                                     raw(o.residual), raw(aux), flags, on.error, o.b_t, on.stream);

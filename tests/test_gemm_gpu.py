@@ -320,6 +320,13 @@ def test_every_form_on_either_side_of_the_dispatch(M, N, K, b_t, monkeypatch):
     K_.check_errors()
 
 
+# Few rows of a wide result, on both sides of each line: 8, 16, 128 and 384 rows, 16, 37, 74 and 148 tiles, 64 K elements of A
+@pytest.mark.parametrize("M,N,K", [(2, 4096, 512), (16, 4160, 512), (17, 4160, 512), (8, 6208, 64), (8, 9472, 192), (8, 9536, 64), (9, 9536, 64), (16, 9536, 1536), (40, 9536, 1536),
+                                   (128, 19008, 64), (128, 38144, 2048), (129, 19008, 64), (256, 19008, 64), (300, 12288, 64), (300, 19008, 128), (300, 19008, 1024)])
+def test_every_form_of_few_rows_on_either_side_of_the_dispatch(M, N, K, monkeypatch):
+    test_every_form_on_either_side_of_the_dispatch(M, N, K, False, monkeypatch)
+
+
 @pytest.mark.parametrize("M,N,K", [(8, 32, 64), (300, 96, 64), (1100, 1120, 192), (19000, 544, 64)])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_pair_gemm_side_operands_with_everything(M, N, K, shift, monkeypatch):
