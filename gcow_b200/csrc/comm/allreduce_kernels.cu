@@ -425,7 +425,8 @@ allreduce_fused_kernel(const ArArgs a) {
 // worked out by roundtrip_block_1d_try, or by roundtrip_block_1d_cut where the cut falls into the block's first planes (6 blocks of noise
 // in 10^4 at 8 bits/value, nearly all of smooth data). Only a block of a tiny, huge or non-finite maximum goes through both coders, with
 // their tables read from global memory: loading them into every CTA's shared memory took a tenth of the kernel. Four blocks per thread
-// are in flight, bound by integer work and memory in about equal parts: us at 6.5 M / 33 M values of noise, both coders' tables in
+// are in flight, bound by integer work and memory in about equal parts (6.5 M values at 8 bits/value 12.1 us, with input and result in the L2 10.4; a
+// copy of them 10.2 and 5.7): us at 6.5 M / 33 M values of noise, both coders' tables in
 // shared memory and two blocks in flight -> now: 8 bits/value 16.9 -> 12.0 / 59.4 -> 48.9, 16 13.8 -> 11.9 / 53.8 -> 49.6, 32 13.8 -> 11.3 / 54.0 -> 47.0;
 // 6.5 M values near 1: 8 bits 72.5 -> 24.6, 16 bits 20.9 -> 11.9. Six blocks in flight (64 registers, four CTAs per SM): 8 bits 14.5 / 56.8.
 // EACH: there is a thread for every block (up to 909 312 values), which then works on that one alone and not on one of four, of which three are

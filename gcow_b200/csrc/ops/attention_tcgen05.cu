@@ -128,9 +128,8 @@ __device__ __forceinline__ Unit unit_at(int u, int mode, int tiles, int heads) {
 // exponentials as polynomials on the multiply-add pipe: forward 64.7, 65.8, backward 210, 205 but short sequences 2 to 5 % longer.
 //
 // What the issuing warps do per product decides the pace. As code of one thread alone, with the descriptors worked out where
-// they are used, a step of four to eight MMAs took it 1500 cycles (forward, B 32, S 512, 16 heads: 131 us): every operand of
-// an MMA is a uniform register, which a divergent thread has to fill one by one. So the whole warp runs the loop, all its
-// values are uniform, and one elected lane executes the MMAs, commits and copies alone (95 us). A wait that has nothing to wait for
+// they are used, a step of four to eight MMAs took it 1500 cycles (forward, B 32, S 512, 16 heads: 131 us). So the whole warp
+// runs the loop, all its values are uniform, and one elected lane executes the MMAs, commits and copies alone (95 us). A wait that has nothing to wait for
 // still takes 110 cycles and an MMA with its descriptors 70, so each tile has a warp of its own.
 struct Phases {
   uint32_t bits = 0;

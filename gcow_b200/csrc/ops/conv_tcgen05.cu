@@ -953,8 +953,8 @@ conv_wgrad_ws_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
 // ---------------------------------------------------------------------------------------------------------
 // Halo-tile weight gradient for channel counts that are multiples of 128, 3x3, stride 1, padding 1. The scheme of
 // conv_wgrad_ws_kernel with real channels in both halves of M: per tile of R image rows in slots of pitch P (16, 32 or 64) one box of dY per
-// 64 output channels (rows h0 .. h0+R-1, columns 0..P-1) and one box of X per 64 input channels (rows h0-1 .. h0+R,
-// columns -1..P-2); X slot = dY slot + r * P + s. A: dY, M = 128 = the two channel boxes (leading offset = one
+// 64 output channels (rows h0 .. h0+R-1, columns 0..P-1) and one box of X per 64 input channels (the rows of filter row r,
+// h0-1+r .. h0+R-2+r, columns -1..P-2); X slot = dY slot + s. A: dY, M = 128 = the two channel boxes (leading offset = one
 // box); B: X of one channel chunk, N = 192 = the three taps of filter row r (leading offset one slot). The
 // accumulators of one filter row and 128 x 128 channels are 2 x 192 columns, so a CTA serves ONE (filter row, 128 input
 // channels, 128 output channels) group (blockIdx.y) over its range of tiles; the groups re-read the tiles, which are
@@ -1261,7 +1261,8 @@ static int stages_for(int halves, int bn_cols) {
 // overlaps the next tile (256 x 28 x 28, 256 -> 512 channels, 1 x 1: 86 us, one 68). Fitted to 48 forward passes and input gradients of batches
 // of 8 to 256; its choice takes 0.6 % longer than the best tile, that of an earlier model of copies and MMAs 9.5 %. us,
 // that one, this one: 8 x 14 x 14, 256 -> 256 15.6, 11.6; 8 x 7 x 7, 512 -> 512 25.4, 18.2; 32 x 14 x 14, 256 -> 256 15.9, 13.1; 100 x 56 x 56, 128 -> 128 stride 2,
-// input gradient 73.4, 61.4; 100 x 28 x 28, 256 -> 512, 1 x 1 41.0, 29.9; 256 x 7 x 7, 1024 -> 2048, 1 x 1 50.0, 45.0.
+// input gradient 73.4, 61.4; 100 x 28 x 28, 256 -> 512, 1 x 1 41.0, 29.9; 256 x 7 x 7, 1024 -> 2048, 1 x 1 50.0, 45.0. Where it is off: 256 x 7 x 7, 512 -> 512, 3 x 3
+// takes 57.9 as two accumulators of 256 channels, 55.1 as the best tile.
 struct FwdPlan { int cols, halves, bw, bh, bn; };
 static FwdPlan fwd_plan(int Wo, int Ho, int N, int Co, int ksteps, bool strided, int sms) {
   struct Tile { int cols, halves; double few, all, epilogue, epilogue_strided; };        // us
@@ -1291,8 +1292,9 @@ static WgradPlan wgrad_plan(int N, int Ho, int Wo, int Ci, int Co, int taps, int
   const int chunks = q.tiles_w * q.tiles_h * q.tiles_n;
   // 256 output rows per tile share each X box; where a small batch leaves few boxes, tiles of 128 rows make twice as many CTAs of them, as long as no sum
   // gets longer than with 256 rows and eight boxes per CTA at least. us with the ordered sum, before, now: 8 x 14 x 14, 256 -> 256, 3 x 3 16.4, 12.9;
-  // 8 x 7 x 7, 512 -> 512 17.8, 12.1; 8 x 56 x 56, 256 -> 512, 1 x 1 stride 2 17.0, 12.7, 64 -> 64, 1 x 1 13.0, 9.3; from 32 images on as before (with 128
-  // rows there 32 x 14 x 14 20.6, 17.4, but 8 pieces for 13, and 256 x 14 x 14 47, 56).
+  // 8 x 7 x 7, 512 -> 512 17.8, 12.1; 8 x 56 x 56, 256 -> 512, 1 x 1 stride 2 17.0, 12.7, 64 -> 64, 1 x 1 13.0, 9.3. The 3 x 3 and stride-2 layers of a ResNet-50
+  // come to 256 rows again from 32 images on (with 128 there 32 x 14 x 14 20.6, 17.4, but 8 pieces for 13, and 256 x 14 x 14 47, 56), small 1 x 1 ones later: 128 x 7 x 7,
+  // 512 -> 512 in 17 pieces of 128 rows instead of 13 of 256 22.7, 13.3, 40 x 28 x 28, 256 -> 256 25.2, 24.3.
   const auto cut = [&](int halves, int boxes) {                 // into one round of tiles at most, with `boxes` pixel boxes per CTA at least
     const int base = ((Co + 128 * halves - 1) / (128 * halves)) * ((taps * Ci + 255) / 256), most = (chunks + boxes - 1) / boxes;
     int split = sms / base < most ? sms / base : most;
@@ -1433,7 +1435,9 @@ static bool halo_plan(int N, int H, int W, int Ci, HaloParams* p) {
   p->tiles_h = (H + p->rows - 1) / p->rows;
   p->chunk_bytes = ((p->nslots + 2 * p->pitch + 2) * 128 + 1023) & ~1023;
   const int fixed = 1024 + (int)sizeof(HaloSmem) + 16 + EPI_WARPS * kStageWarpBytes, left = kWsSmemMax - fixed;
-  if ((left - 2 * (Ci / 64) * p->chunk_bytes) / HALO_B_BYTES < 3) return false;   // what two whole tiles' input left room for is what it takes
+  // Taken are the widths and channels of which two whole tiles' input would leave room for three filter pieces (128 channels at 28 x 28); the three chunks
+  // held would do for more, which has not been measured against the general kernel.
+  if ((left - 2 * (Ci / 64) * p->chunk_bytes) / HALO_B_BYTES < 3) return false;
   // Three chunks of a tile of two or more, the third one the next tile's first; what a fourth would take goes to the filter's ring.
   p->a_slots = Ci > 64 ? 3 : 2;
   p->b_stages = (left - p->a_slots * p->chunk_bytes) / HALO_B_BYTES;
@@ -1502,7 +1506,7 @@ static int wgrad_halo_plan(int N, int H, int W, int Ci, int Co, WgHaloParams* p)
   if (N <= 0 || H <= 0 || W < 1 || W + 2 > 64 || Ci < 128 || Ci % 128 || Co < 128 || Co % 128) return 0;
   p->N = N; p->H = H; p->W = W; p->Ci = Ci; p->Co = Co;
   p->P = W + 2 <= 16 ? 16 : (W + 2 <= 32 ? 32 : 64);
-  p->R = p->P == 16 ? 7 : (p->P == 32 ? 4 : 2);   // two stages of two X and two dY boxes fit the shared memory
+  p->R = p->P == 16 ? 7 : (p->P == 32 ? 4 : 2);   // three stages of two X and two dY boxes fit the shared memory
   p->tiles_h = (H + p->R - 1) / p->R;
   const long long tiles = (long long)N * p->tiles_h;
   if (tiles > (1ll << 30)) return 0;

@@ -421,7 +421,6 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       auto process = [&](const uint32_t (&r)[32], int c) {
         const int n = n0 + col0 + c * 32;
         if (n >= p.N || mw >= p.M) return;                // warp-uniform; the launcher guarantees N % 32 == 0
-        const size_t off = (size_t)m * p.ldc + n;
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; j++) v[j] = __uint_as_float(r[j]);
@@ -714,8 +713,8 @@ int gcow_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
               : make_map_kfold(&mh, B, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, 64);
     if (rc) return rc;
   }
-  // Its own instance for launches that read nothing besides the accumulator: the blocks fetched ahead cost registers, for
-  // which the epilogue spilled (16384 x 4096 x 1024: plain 100 -> 95 us, bias 106 -> 97).
+  // Its own instance for launches that read nothing besides the accumulator: those hold two of its blocks in registers and two staging buffers a
+  // warp, with eight warps; a side operand comes through the one buffer of each of sixteen.
   const int side = flags & kGeluGrad ? kArgument : flags & kResidual ? kSum : kNothing;
   const bool wide = !side && (flags & kGelu);
   CUtensorMap mside = mb, mc = mb;
@@ -743,7 +742,8 @@ int gcow_wgrad_slabs(int64_t M, int64_t N, int64_t K) {
 // sum 0.0014 s^2 + (1.17 s - 0.8) per million elements, half as much again where the partial results no longer fit the L2. An earlier model, of a
 // slower kernel (0.71, 1.5 a round, 1.8 + 0.003 s^2 + (4.5 + 0.35 s) per million), cut less: 1024 rows to 768 x 768 one slice 12.8 us, four 10.2; 3000 to
 // 2304 x 768 one 22.1, two 17.9; 4096 to 768 x 3072 one 28.1, two 22.0; 8192 to 3072 x 1024 one 47.2, three 45.2; 6144 to 4096 x 4096 still one, 153, two
-// 172. Where it cut more its count stays (8192 to 512 x 512 sixteen 16.7, thirteen 13.8): fewer slices are longer sums.
+// 172. It stays as the bound on a slice: where it cut more its count stays (8192 to 512 x 512 sixteen 16.7, thirteen 13.8), since fewer slices are longer
+// sums, less exact ones than results had.
 // No accumulator takes more stages than one of the slabs above: the tensor core cuts the running sum at every step, and the error
 // grows with the number of steps (relative 2-norm, noise: 512 rows 4.7e-7, 1024 1.0e-6, 4096 4.4e-6). Where every pair has one
 // item at most, its slice is shared by two accumulators: 1024 rows to 1024 x 1024 in one slice 14.2 us, in two slices 17.3, on

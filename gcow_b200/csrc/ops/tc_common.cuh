@@ -17,10 +17,9 @@ constexpr uint32_t kSpinLimit = 1u << 26;   // polls before a wait gives up
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// True in one lane of the warp, which has to be converged. What a warp issues for all of its lanes - MMAs, commits, tensor copies - takes its
-// operands from uniform registers. Behind `lane == 0` the compiler has to assume several lanes with operands of their own and goes through them;
-// behind this it knows that there is one. Four MMAs and the sums for their descriptors take a warp 447 cycles there and 281 here (M128 N64,
-// whose MMAs take 128). Asked once per role: the same lane has to issue MMAs and the commits that track them.
+// True in one lane of the warp, which has to be converged: for what a warp issues for all of its lanes - MMAs, commits, tensor copies. Four MMAs and
+// the sums for their descriptors take a warp 447 cycles behind `lane == 0` and 281 behind this (M128 N64, whose MMAs take 128). Asked once per
+// role: the same lane has to issue MMAs and the commits that track them.
 __device__ __forceinline__ bool elect_one() {
   uint32_t one;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(one));
@@ -324,8 +323,7 @@ struct TileOrder {
   }
 };
 // The same with multiplications for the two divisions, some 30 dependent instructions less, which an epilogue of sixteen warps does not cover
-// (gemm2_tcgen05.cu). Not for kernels whose registers are full: the pair kernel with a GELU' factor takes 14.8 us with it instead of 13.9
-// (4096 x 768 x 768), the one-CTA kernel 99 instead of 85 (802816 x 256 x 64).
+// (gemm2_tcgen05.cu). Not for kernels whose registers are full: the one-CTA kernel takes 99 us with it instead of 85 (802816 x 256 x 64).
 struct QuickTileOrder {
   TileOrder order;
   Divisor by_group_tiles, by_group, by_last;             // by_last: the last group's rows of tiles

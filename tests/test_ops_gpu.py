@@ -571,17 +571,17 @@ def test_batchnorm_sums_of_any_number_of_partials(parts):
 
 
 # Fewer rows than CTAs in a cluster, one CTA a cluster, clusters of 2 to 16, channels by 32 and by 16, shares of rows that differ by one, shares just
-# within 52 KB and 104 KB and just beyond
+# within 52 KB and 104 KB (the lines themselves: test_batchnorm_forms_on_either_side_of_their_lines)
 @pytest.mark.parametrize("N,C,H,W", [(1, 64, 1, 3), (1, 2048, 1, 1), (3, 2048, 7, 7), (17, 512, 7, 7), (13, 1024, 9, 11), (1, 128, 111, 113), (1, 128, 111, 121),
                                      (1, 256, 107, 61), (1, 64, 101, 259), (1, 2048, 61, 109), (1, 2048, 33, 50)])
 @pytest.mark.parametrize("res,relu,fork", [(False, False, False), (False, True, False), (True, True, True), (True, False, False), (True, True, False), (False, True, True)])
 def test_batchnorm_of_tensors_held_in_shared_memory(N, C, H, W, res, relu, fork):
-    """The one-launch form against float64, its running statistics, and which form a shape takes."""
+    """Shapes that take the one-launch form, without other operands at least: against float64, and the running statistics."""
     from gcow_b200 import _native
     from gcow_b200.ops import nn as gnn
     R, lib = N * H * W, _native.cuda()
     lib.gcow_bn_launches.argtypes = [C_.c_int64, C_.c_int, C_.c_int, C_.c_int]
-    assert lib.gcow_bn_launches(R, C, 0, 0) == 1 or (N, C, H, W) in ((1, 256, 107, 61), (1, 2048, 61, 109))
+    assert lib.gcow_bn_launches(R, C, 0, 0) == 1
     test_batchnorm_every_form_of_the_sweeps(N, C, H, W, res, relu, fork)
     x = torch.randn(N, C, H, W, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last)
     bn = gnn.BatchNorm2d(C).cuda()
