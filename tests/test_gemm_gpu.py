@@ -136,8 +136,9 @@ def test_wgrad_on_pairs_at_the_edges(M, N, K):
 @pytest.mark.parametrize("M,N,K", [(1024, 256, 256), (1192, 320, 448), (1100, 256, 768), (5000, 1024, 1280), (40000, 256, 320), (2048, 512, 4096),
                                    (1500, 256, 8192), (1024, 256, 8448), (16384, 3072, 1024), (4096, 4096, 1024)])
 def test_bias_gradient_beside_the_weight_gradient(M, N, K):
-    """Column sums taken while the weight gradient's tiles pass: one tile column that has all rows of a stage to itself up to more tile columns
-    than a stage has groups of four rows, tiles that overhang, rows that end inside a stage, one slice, two accumulators, several."""
+    """Column sums taken while the weight gradient's tiles pass: two tile columns, with a half of all rows to themselves each, up to more than a
+    stage has groups of four rows for, an odd number of them, tiles that overhang, rows that end inside a stage, one slice, two accumulators, several; a single
+    tile column, whose sums have a kernel of their own."""
     from gcow_b200 import _native
     from gcow_b200.ops import kernels as K_
     if _native.cuda().gcow_gemm2_wgrad_slices(N, K, M) <= 0:
